@@ -2,6 +2,7 @@
 // orchestration of one MoE block (see include/dnb200.h for the contract).
 #include <algorithm>
 #include <chrono>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
@@ -379,8 +380,9 @@ static int tc_type(const Layer& L, int first, int last) {
         if (!L.m[i].dev || L.m[i].type != ty) return -1;
     return ty;
 }
-// Tokens from which a chunk or decode batch leaves the one-token kernels for the tensor-core grouped GEMM.
-static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? 16 : c->exact_min_nt; }
+// Tokens from which a chunk or decode batch leaves the mma.sync kernel for the tcgen05 grouped GEMM.
+constexpr int kTcMin = 48;
+static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMin : c->exact_min_nt; }
 
 static bool umma_eligible(const dnb_ctx* c, const Layer& L, int nt) {
     const Model& M = c->model;
@@ -432,6 +434,42 @@ static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const
                           (shared && L.shared_gate_row) ? w.shcoef : nullptr, out);
 }
 
+// Layers that the mma.sync grouped kernel takes (grouped_mma.cu): its five formats, the shared expert like the routed ones.
+static bool mm_eligible(const dnb_ctx* c, const Layer& L) {
+    const Model& M = c->model;
+    if (!c->decode_fast || L.m[0].type != L.m[1].type || !mm_handles(L.m[0].type, M.e) || !mm_handles(L.m[2].type, M.ff)) return false;
+    if (!L.has_shared()) return true;
+    return L.m[3].type == L.m[0].type && L.m[4].type == L.m[1].type && L.m[5].type == L.m[2].type && L.m[3].n_out == M.ff;
+}
+
+// The experts on the mma.sync grouped kernel: tables, gate/up, down, combine.  The shared expert is one more segment.
+static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts, float* out, int parts,
+                           int k = -1, int ne = -1, int with_shared = -1) {
+    const Model& M = c->model;
+    const Layer& L = M.layers[layer];
+    Workspace& w = c->ws;
+    cudaStream_t st = c->stream;
+    if (k < 0) k = M.k;
+    if (ne < 0) ne = M.ne;
+    const bool shared = with_shared < 0 ? L.has_shared() : (with_shared != 0);
+    int rc;
+    if ((rc = launch_route_tables(c, st, sels, nt, k, ne, L, w, shared))) return rc;
+    const int rows = nt * k + (shared ? nt : 0);
+    const int nseg_max = (nt * k < ne ? nt * k : ne) + (shared ? 1 : 0);
+    // experts that nt tokens reach when each picks k of ne at random
+    const int est = std::min(nseg_max, (int)(ne * (1.0 - pow(1.0 - (double)k / ne, nt)) + 1.5));
+    if ((rc = launch_mm(c, st, L.m[0].type, true, parts, w.seg_gu, w.nseg, nseg_max, est, rows, M.e, M.ff, x, M.e, w.row_token, w.act, nullptr,
+                        "mm_gate_up")))
+        return rc;
+    if ((rc = launch_mm(c, st, L.m[2].type, false, parts, w.seg_dn, w.nseg, nseg_max, est, rows, M.ff, M.e, w.act, M.ff, nullptr, w.hrow, nullptr,
+                        "mm_down")))
+        return rc;
+    if (shared && L.shared_gate_row)
+        if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
+    return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
+                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out);
+}
+
 // Router logits of nt rows: the tensor-core kernel from kRouterTcMin tokens, the fp32 kernel below.
 int router_logits(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const Layer& L, float* logits) {
     const Model& M = c->model;
@@ -464,7 +502,8 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out) 
         rc = block_dev_decode(c, layer, h, out, nullptr);
         if (rc != DNB_DECLINED) return rc;
     }
-    if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !umma_eligible(c, L, nt)) {
+    const bool mma = nt > 1 && mm_eligible(c, L) && !umma_eligible(c, L, nt);
+    if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !mma && !umma_eligible(c, L, nt)) {
         rc = block_dev_decode_batch(c, layer, h, nt, out, nullptr);
         if (rc != DNB_DECLINED) return rc;
     }
@@ -480,6 +519,10 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out) 
     const float* x = L.norm_w ? w.xn : h;
     if ((rc = router_topk_dev(c, st, x, nt, L, w.sels, w.wts, nullptr, split_in_prep))) return rc;
     if (umma_eligible(c, L, nt)) return experts_dev_umma(c, layer, x, nt, w.sels, w.wts, out);
+    if (mma) {
+        rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, nt >= 16 && tc_type(L, 0, 3) >= 0 ? 2 : 3);
+        if (rc != DNB_DECLINED) return rc;
+    }
     return experts_dev(c, layer, x, nt, w.sels, w.wts, out);
 }
 
@@ -1075,7 +1118,9 @@ int dnb_moe_experts(dnb_ctx* c, int layer, const float* x, int nt, const int32_t
         if ((rc = launch_prep(c, c->stream, w.hin, nullptr, M.eps, nt, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn,
                               L.m[3].dev, L.m[4].dev, L.m[5].dev)))
             return rc;
-    if ((rc = experts_dev(c, layer, w.hin, nt, w.sels, w.wts, w.out))) return rc;
+    rc = mm_eligible(c, L) ? experts_dev_mma(c, layer, w.hin, nt, w.sels, w.wts, w.out, 3) : DNB_DECLINED;
+    if (rc == DNB_DECLINED) rc = experts_dev(c, layer, w.hin, nt, w.sels, w.wts, w.out);
+    if (rc) return rc;
     DNB_CUDA(cudaMemcpyAsync(w.pinned_out, w.out, bytes, cudaMemcpyDeviceToHost, c->stream));
     DNB_CUDA(nt <= 64 ? wait_short(c->stream) : cudaStreamSynchronize(c->stream));
     if ((rc = finish_checked(c, "moe_experts"))) return rc;
@@ -1451,7 +1496,7 @@ int dnb_moe_stack_dev(dnb_ctx* c, float* h_dev, int nt) {
                 if (rd == DNB_OK) continue;
                 if (rd != DNB_DECLINED) return rd;
             }
-            if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !umma_eligible(c, M.layers[l], nt)) {
+            if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !mm_eligible(c, M.layers[l]) && !umma_eligible(c, M.layers[l], nt)) {
                 const int rd = block_dev_decode_batch(c, l, h_dev, nt, h_dev, h_dev);
                 if (rd == DNB_OK) continue;
                 if (rd != DNB_DECLINED) return rd;

@@ -181,7 +181,7 @@ struct dnb_ctx {
     bool gemv_mma = true;               // one-token IQ3_XXS kernels on mma.sync (gemv_mma.cu, decode_fused.cu) where the shape fits
     bool decode_fused = true;           // gate/up + down of a one-token IQ3_XXS block as one kernel (decode_fused.cu)
     bool decode_routed = true;          // ... with the router folded into the same kernel (one launch per block)
-    int exact_min_nt = 16;              // IQ3_XXS layers: tokens from which a batch takes the exact-weight tcgen05 kernel
+    int exact_min_nt = 48;              // IQ3_XXS layers: tokens from which a batch takes the exact-weight tcgen05 kernel
     bool use_umma = true;               // prefill chunks of Q4_K layers take the tcgen05 grouped GEMM
     void* ep = nullptr;                 // dnb::EpState of the peer-memory expert-parallel path (ep_p2p.cu)
     void* hc = nullptr;                 // dnb::HcState: hyper-connection mix weights and scratch (hc_mix.cu)
@@ -381,6 +381,15 @@ int launch_rows_f16(dnb_ctx* c, cudaStream_t st, const float* x, int ldx, const 
 int launch_grouped_q4k_int(dnb_ctx* c, cudaStream_t st, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
                            int n_in, int n_out, const UmmaMaps* maps, const float* rowscale, float* out_f32,
                            float* const* row_dst = nullptr);
+
+// Grouped dequant matmul for few tokens per expert on mma.sync (grouped_mma.cu): fused = gate/up with silu(g) * u, else one
+// matrix; parts = fp16 numbers per activation (3: all bits of an fp32, 2: 22 bits).  fp32 rows in (row_token names a packed
+// row's input row, null: itself), fp32 packed rows out.  rows, nseg_est: token rows and active segments (an estimate where the
+// device counts them; it only steers the split of the work).  DNB_DECLINED = type or shape not covered, nothing launched.
+bool mm_handles(int type, int n_in);
+int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
+              int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
+              const SegDesc* single, const char* name);
 
 // tcgen05 grouped GEMM of prefill (grouped_umma.cu)
 int umma_make_maps(void* hi, void* lo, uint64_t rows, uint64_t cols, UmmaMaps* out);

@@ -1,0 +1,716 @@
+// Grouped dequant matmul for few tokens per expert: decode batches, short prompts, caller-given selections, single
+// matrices with a few vectors.  Q4_K, Q5_K, Q6_K, Q8_0 and IQ3_XXS on mma.sync.m16n8k16 (fp16, fp32 accumulators).
+//
+// Reference kernels of this role: kernels_seg_k.cu:201-241, kernels_exp_iq_v2.cu:259-319 (one warp per row, fp32 FMA);
+// block layouts kquant.rs:341-887.
+//
+// What bounds a call like this is instructions, not bytes: at HBM speed an SM has about four lane-instructions per weight
+// of a 4-bit format, and an FMA kernel spends two (convert, multiply) per weight AND token.  Here a weight costs its
+// decoding only, whatever the number of tokens:
+//   * a lane turns packed bytes into the fp16 A fragment in registers; the quantised value is an integer and exact
+//     (Q4_K, Q5_K: sc * q <= 63 * 31 = 1953 < 2048, formed by one fp16 fma on the 1024 + q bit pattern; Q6_K: q - 32;
+//     Q8_0: q; IQ3_XXS: the codebook magnitude <= 62 with its sign), so no weight is rounded;
+//   * the scales multiply the fp32 sums of a 256-element block (Q4_K, Q5_K: d; their mins are one more K step of
+//     m against the sub-block sums of the activations), of a 32-element block (Q8_0, IQ3_XXS) or of 16 elements (Q6_K);
+//   * an activation is P fp16 numbers in P columns of B (P = 3 carries the 24 bits of an fp32; P = 2 carries 22 and is
+//     used where a call of this size had 16 before), of the row times a power of two that puts its largest element into
+//     [512, 1024), so that nothing overflows and sub-block sums fit, too;
+//   * K is walked in the order in which the packed bytes yield elements; the activations are staged in that order.
+// A B column costs an mma per 16 weights of a lane's two rows and half a 16-byte shared-memory read.
+//
+// Work: an item is (segment, token tile, block of row groups); a row group is 16 A rows: 16 rows of one matrix, or 8 gate
+// and 8 up rows of the same indices, whose results meet in one lane for silu(g) * u.  A persistent CTA of 16 warps stages
+// an item's activations once; a warp then streams its row groups through a private ring of cp.async stages (one
+// 256-element block of the 16 rows each) without any CTA-wide barrier.  Few row groups for the chip (small models, single
+// matrices): KS warps share a row group, each takes a part of K, and their sums are added in a fixed order.
+// A row's result depends on nothing but the row: not on the tile, the column or the split of the launch.
+#include <algorithm>
+
+#include "dnb_common.cuh"
+#include "formats.cuh"
+#include "tc_ptx.cuh"
+#include "dnb_iq_tables.h"
+
+namespace dnb {
+
+constexpr int kMmWarps = 16;
+constexpr int kMmThreads = kMmWarps * 32;
+constexpr int kMmSegMax = 1088;  // segments of a launch at most
+
+// 256 elements of a row: bytes, 16-byte units of a stage row (blocks that are not 16-byte sized start anywhere in their first
+// unit), and the unit stride of a stage row (chosen so that the eight rows a warp reads at once fall on different banks).
+template <int T> struct Mq;
+template <> struct Mq<T_Q4_K> { static constexpr int BB = 144, UNITS = 9, RS = 144; static constexpr bool ALIGNED = true; };
+template <> struct Mq<T_Q5_K> { static constexpr int BB = 176, UNITS = 11, RS = 176; static constexpr bool ALIGNED = true; };
+template <> struct Mq<T_Q6_K> { static constexpr int BB = 210, UNITS = 14, RS = 240; static constexpr bool ALIGNED = false; };
+template <> struct Mq<T_IQ3_XXS> { static constexpr int BB = 98, UNITS = 7, RS = 112; static constexpr bool ALIGNED = false; };
+template <> struct Mq<T_Q8_0> { static constexpr int BB = 272, UNITS = 17, RS = 272; static constexpr bool ALIGNED = true; };
+
+template <int T> constexpr bool mq_mins = (T == T_Q4_K || T == T_Q5_K);
+
+// IQ3_XXS codebook as fp16 pairs, kLutRep copies (a lane reads copy lane % kLutRep: no bank conflicts).
+struct MmCodebook { uint2 grid[256 * kLutRep]; };
+static __device__ __align__(16) MmCodebook g_mm_codebook;
+static bool g_mm_tables[64] = {false};
+
+static int upload_mm_tables(int device) {
+    if (device < 0 || device >= 64) return DNB_ERR_ARG;
+    if (g_mm_tables[device]) return DNB_OK;
+    static MmCodebook tb;
+    for (int e = 0; e < 256; ++e) {
+        uint32_t h[4];
+        for (int j = 0; j < 4; ++j) h[j] = __half_as_ushort(__float2half((float)((dnb_iq3xxs_grid[e] >> (8 * j)) & 0xFFu)));
+        for (int r = 0; r < kLutRep; ++r) tb.grid[e * kLutRep + r] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+    }
+    DNB_CUDA(cudaMemcpyToSymbol(g_mm_codebook, &tb, sizeof(tb)));
+    g_mm_tables[device] = true;
+    return DNB_OK;
+}
+
+// First element (of 256) of the two groups of four that unit u = 0..7 of lane t takes; `swap`: a group's order is 0, 2, 1, 3.
+template <int T>
+__device__ __forceinline__ void mm_unit_elems(int u, int t, int& e0, int& e1) {
+    if constexpr (mq_mins<T>) {
+        e0 = 64 * t + 4 * u;
+        e1 = e0 + 32;
+    } else if constexpr (T == T_Q6_K) {
+        e0 = (u >> 2) * 128 + (u & 1) * 32 + ((u >> 1) & 1) * 16 + 4 * t;
+        e1 = e0 + 64;
+    } else {
+        e0 = 32 * u + 8 * t;
+        e1 = e0 + 4;
+    }
+}
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f16_z(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ uint32_t h2fma(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2sub(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2mul(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t ld32u(const uint8_t* p) { return ld16(p) | (ld16(p + 2) << 16); }  // 2-byte aligned
+
+// Q4_K / Q5_K: a lane's scales of one row of a block.  s0 / s1: the scale of its even / odd sub-block in both halves,
+// k0 / k1: -1024 * s0 and -64 * s1, mm: the pair of mins.
+struct KScales { float d, dmin; uint32_t s0, s1, k0, k1, mm; };
+__device__ __forceinline__ KScales k_scales(const uint8_t* row, int t) {
+    const uint4 h = *reinterpret_cast<const uint4*>(row);
+    const int sh = 16 * (t & 1);
+    const uint32_t a = h.y >> sh, b = h.z >> sh, c = h.w >> sh;
+    const bool low = t < 2;  // kquant.rs:878-887
+    const uint32_t sc = low ? (a & 0x3f3fu) : ((c & 0x0f0fu) | ((a >> 2) & 0x3030u));
+    const uint32_t mn = low ? (b & 0x3f3fu) : (((c >> 4) & 0x0f0fu) | ((b >> 2) & 0x3030u));
+    KScales r;
+    r.d = h2f((uint16_t)h.x);
+    r.dmin = h2f((uint16_t)(h.x >> 16));
+    r.s0 = h2sub(__byte_perm(sc, 0x64646464u, 0x4040u), 0x64006400u);
+    r.s1 = h2sub(__byte_perm(sc, 0x64646464u, 0x4141u), 0x64006400u);
+    r.k0 = h2mul(r.s0, 0xE400E400u);  // * -1024
+    r.k1 = h2mul(r.s1, 0xD400D400u);  // * -64
+    r.mm = h2sub(__byte_perm(mn, 0x64646464u, 0x4140u), 0x64006400u);
+    return r;
+}
+// Word i of a lane's 32 bytes: low nibbles are the even sub-block, high nibbles the odd one.  hq (Q5_K): the word of fifth
+// bits shifted so that bit 0 of a byte belongs to the low and bit 1 to the high nibble.
+template <bool FIVE>
+__device__ __forceinline__ void k_word(uint32_t w, uint32_t hq, const KScales& s, uint32_t (&p)[4]) {
+    const uint32_t w8 = w >> 8;
+    uint32_t a = (w & 0x000f000fu) | 0x64006400u, b = (w8 & 0x000f000fu) | 0x64006400u;    // 1024 + q
+    uint32_t c = (w & 0x00f000f0u) | 0x54005400u, d = (w8 & 0x00f000f0u) | 0x54005400u;    // 64 + q
+    if constexpr (FIVE) {
+        const uint32_t h8 = hq >> 8;
+        a |= (hq << 4) & 0x00100010u;
+        b |= (h8 << 4) & 0x00100010u;
+        c |= (hq << 7) & 0x01000100u;
+        d |= (h8 << 7) & 0x01000100u;
+    }
+    p[0] = h2fma(a, s.s0, s.k0);
+    p[1] = h2fma(b, s.s0, s.k0);
+    p[2] = h2fma(c, s.s1, s.k1);
+    p[3] = h2fma(d, s.s1, s.k1);
+}
+
+// Eight weights of an IQ3_XXS sub-block as four signed fp16 pairs.
+__device__ __forceinline__ void iq3_pairs_h(const uint2* grid, uint32_t idx, uint32_t code, uint32_t (&p)[4]) {
+    const uint32_t sg = code | ((__popc(code) & 1u) << 7);  // bit 7 makes the number of minus signs even
+    const uint2 g1 = grid[(idx & 0xFFu) * kLutRep], g2 = grid[(idx >> 8) * kLutRep];
+    p[0] = g1.x ^ ((sg * 0x40008000u) & 0x80008000u);
+    p[1] = g1.y ^ ((sg * 0x10002000u) & 0x80008000u);
+    p[2] = g2.x ^ ((sg * 0x04000800u) & 0x80008000u);
+    p[3] = g2.y ^ ((sg * 0x01000200u) & 0x80008000u);
+}
+
+// One 256-element block of 16 rows (this lane: rows `ra` and `rb`) against NT column tiles; bp[i]: the lane's B column of tile
+// i at this block; nt: tiles in use.  acc += scales * sums.
+template <int T, int NT>
+__device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, const uint2* grid, const uint8_t* const (&bp)[NT],
+                                         const uint32_t (&sumw)[NT], int nt, float (&acc)[NT][4]) {
+    if constexpr (mq_mins<T>) {
+        const KScales sa = k_scales(ra, t), sb = k_scales(rb, t);
+        constexpr bool FIVE = T == T_Q5_K;
+        constexpr int QS = FIVE ? 48 : 16;
+        float D[NT][4];
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) D[i][c] = 0.f;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const uint4 qa = *reinterpret_cast<const uint4*>(ra + QS + 32 * t + 16 * half);
+            const uint4 qb = *reinterpret_cast<const uint4*>(rb + QS + 32 * t + 16 * half);
+            uint4 ha = make_uint4(0, 0, 0, 0), hb = ha;
+            if constexpr (FIVE) {
+                ha = *reinterpret_cast<const uint4*>(ra + 16 + 16 * half);
+                hb = *reinterpret_cast<const uint4*>(rb + 16 + 16 * half);
+            }
+            const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
+            const uint32_t fa[4] = {ha.x, ha.y, ha.z, ha.w}, fb[4] = {hb.x, hb.y, hb.z, hb.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t p[4], q[4];
+                k_word<FIVE>(wa[i], fa[i] >> (2 * t), sa, p);
+                k_word<FIVE>(wb[i], fb[i] >> (2 * t), sb, q);
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    if (n < nt) {
+                        const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + (half * 4 + i) * 64);
+                        mma_f16(D[n], p[0], q[0], p[1], q[1], y.x, y.y);
+                        mma_f16(D[n], p[2], q[2], p[3], q[3], y.z, y.w);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            if (n < nt) {
+                float M[4];
+                mma_f16_z(M, sa.mm, sb.mm, 0u, 0u, sumw[n], 0u);
+                acc[n][0] = fmaf(-sa.dmin, M[0], fmaf(sa.d, D[n][0], acc[n][0]));
+                acc[n][1] = fmaf(-sa.dmin, M[1], fmaf(sa.d, D[n][1], acc[n][1]));
+                acc[n][2] = fmaf(-sb.dmin, M[2], fmaf(sb.d, D[n][2], acc[n][2]));
+                acc[n][3] = fmaf(-sb.dmin, M[3], fmaf(sb.d, D[n][3], acc[n][3]));
+            }
+        }
+    } else if constexpr (T == T_IQ3_XXS) {
+        const float da = h2f(ld16(ra)) * 0.25f, db = h2f(ld16(rb)) * 0.25f;
+#pragma unroll 4
+        for (int ib = 0; ib < 8; ++ib) {
+            const uint32_t xa = ld32u(ra + 66 + 4 * ib), xb = ld32u(rb + 66 + 4 * ib);
+            uint32_t p[4], q[4];
+            iq3_pairs_h(grid, ld16(ra + 2 + 8 * ib + 2 * t), (xa >> (7 * t)) & 127u, p);
+            iq3_pairs_h(grid, ld16(rb + 2 + 8 * ib + 2 * t), (xb >> (7 * t)) & 127u, q);
+            // d * (0.5 + s) * 0.5 = (d / 4) * (2 s + 1) (kquant.rs:667)
+            const float fa = fmaf((float)(xa >> 28), da + da, da), fb = fmaf((float)(xb >> 28), db + db, db);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                if (n < nt) {
+                    const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + ib * 64);
+                    float D[4];
+                    mma_f16_z(D, p[0], q[0], p[1], q[1], y.x, y.y);
+                    mma_f16(D, p[2], q[2], p[3], q[3], y.z, y.w);
+                    acc[n][0] = fmaf(fa, D[0], acc[n][0]);
+                    acc[n][1] = fmaf(fa, D[1], acc[n][1]);
+                    acc[n][2] = fmaf(fb, D[2], acc[n][2]);
+                    acc[n][3] = fmaf(fb, D[3], acc[n][3]);
+                }
+            }
+        }
+    } else if constexpr (T == T_Q8_0) {
+        const uint32_t bias = 0x64806480u;  // 1024 + 128
+#pragma unroll 4
+        for (int ib = 0; ib < 8; ++ib) {
+            const float fa = h2f(ld16(ra + 34 * ib)), fb = h2f(ld16(rb + 34 * ib));
+            uint32_t p[4], q[4];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const uint32_t wa = ld32u(ra + 34 * ib + 2 + 8 * t + 4 * v) ^ 0x80808080u;
+                const uint32_t wb = ld32u(rb + 34 * ib + 2 + 8 * t + 4 * v) ^ 0x80808080u;
+                p[2 * v] = h2sub(__byte_perm(wa, 0x64646464u, 0x5140u), bias);
+                p[2 * v + 1] = h2sub(__byte_perm(wa, 0x64646464u, 0x7362u), bias);
+                q[2 * v] = h2sub(__byte_perm(wb, 0x64646464u, 0x5140u), bias);
+                q[2 * v + 1] = h2sub(__byte_perm(wb, 0x64646464u, 0x7362u), bias);
+            }
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                if (n < nt) {
+                    const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + ib * 64);
+                    float D[4];
+                    mma_f16_z(D, p[0], q[0], p[1], q[1], y.x, y.y);
+                    mma_f16(D, p[2], q[2], p[3], q[3], y.z, y.w);
+                    acc[n][0] = fmaf(fa, D[0], acc[n][0]);
+                    acc[n][1] = fmaf(fa, D[1], acc[n][1]);
+                    acc[n][2] = fmaf(fb, D[2], acc[n][2]);
+                    acc[n][3] = fmaf(fb, D[3], acc[n][3]);
+                }
+            }
+        }
+    } else {  // Q6_K: a K step is one 16-element group of one scale
+        const float da = h2f(ld16(ra + 208)), db = h2f(ld16(rb + 208));
+        const uint32_t bias = 0x64206420u;  // 1024 + 32
+#pragma unroll 2
+        for (int g = 0; g < 4; ++g) {  // (half, is)
+            const int half = g >> 1, is = g & 1;
+            const uint32_t ha = ld32u(ra + 128 + 32 * half + 16 * is + 4 * t), hb = ld32u(rb + 128 + 32 * half + 16 * is + 4 * t);
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const uint32_t qa = ld32u(ra + 64 * half + 32 * w + 16 * is + 4 * t), qb = ld32u(rb + 64 * half + 32 * w + 16 * is + 4 * t);
+#pragma unroll
+                for (int hi = 0; hi < 2; ++hi) {
+                    const uint32_t va = ((qa >> (4 * hi)) & 0x0f0f0f0fu) | (((ha >> (2 * w + 4 * hi)) & 0x03030303u) << 4);
+                    const uint32_t vb = ((qb >> (4 * hi)) & 0x0f0f0f0fu) | (((hb >> (2 * w + 4 * hi)) & 0x03030303u) << 4);
+                    const uint32_t p0 = h2sub(__byte_perm(va, 0x64646464u, 0x5140u), bias), p1 = h2sub(__byte_perm(va, 0x64646464u, 0x7362u), bias);
+                    const uint32_t q0 = h2sub(__byte_perm(vb, 0x64646464u, 0x5140u), bias), q1 = h2sub(__byte_perm(vb, 0x64646464u, 0x7362u), bias);
+                    const int sc = 192 + 8 * half + is + 2 * w + 4 * hi;
+                    const float fa = da * (float)(int)*reinterpret_cast<const int8_t*>(ra + sc), fb = db * (float)(int)*reinterpret_cast<const int8_t*>(rb + sc);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        if (n < nt) {
+                            const uint2 y = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 64 + 8 * hi);
+                            float D[4];
+                            mma_f16_z(D, p0, q0, p1, q1, y.x, y.y);
+                            acc[n][0] = fmaf(fa, D[0], acc[n][0]);
+                            acc[n][1] = fmaf(fa, D[1], acc[n][1]);
+                            acc[n][2] = fmaf(fb, D[2], acc[n][2]);
+                            acc[n][3] = fmaf(fb, D[3], acc[n][3]);
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+struct MmArgs {
+    const SegDesc* seg;        // or null: `single`
+    const int32_t* nseg_dev;   // or null: nseg_max segments
+    SegDesc single;
+    int nseg_max;
+    int n_in, n_out, rb;       // rb: bytes of a row
+    const float* x;            // fp32 rows
+    int ldx;
+    const int32_t* row_token;  // packed row -> x row, or null
+    float* out;                // [packed row][n_out]
+    int rpi, rblocks;          // row groups per item, items per (segment, tile)
+    int ks, nst;               // warps that split K, stages of a warp's ring
+    int col_stride;            // bytes between B columns
+};
+
+__device__ __forceinline__ void mm_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Scale of a row: the power of two that puts its largest element into [512, 1024).
+__device__ __forceinline__ float mm_row_scale(uint32_t amax_bits) {
+    const int ex = (int)(amax_bits >> 23);  // biased exponent of the largest |x|
+    const int s = ex == 0 ? 0 : max(-126, min(126, 9 - (ex - 127)));
+    return __uint_as_float((uint32_t)(s + 127) << 23);
+}
+// Two values as P fp16 pairs whose sums are the values (P = 3: every bit of an fp32; P = 2: 22 bits).
+template <int P>
+__device__ __forceinline__ void mm_split(float a, float b, uint32_t (&h)[P]) {
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        const __half2 v = __floats2half2_rn(a, b);
+        h[p] = *reinterpret_cast<const uint32_t*>(&v);
+        if (p + 1 < P) {
+            const float2 f = __half22float2(v);
+            a -= f.x;
+            b -= f.y;
+        }
+    }
+}
+
+template <int T, bool FUSED, int P, int NT>
+__global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
+    using Q = Mq<T>;
+    constexpr int TPT = P == 3 ? 2 : 4;  // tokens of a column tile (P = 3: columns 3 and 7 are copies nobody adds)
+    constexpr int TT = NT * TPT;         // tokens of an item
+    constexpr int STAGE = 16 * Q::RS;
+    extern __shared__ __align__(128) uint8_t smem[];
+    int* pre = reinterpret_cast<int*>(smem);                            // [kMmSegMax + 1] first item of a segment
+    int* wsum = pre + kMmSegMax + 4;                                    // [16]
+    uint32_t* amax = reinterpret_cast<uint32_t*>(wsum + 16);            // [2][16]
+    uint8_t* p0 = smem + ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
+    uint2* book = reinterpret_cast<uint2*>(p0);
+    if constexpr (T == T_IQ3_XXS) p0 += sizeof(MmCodebook);
+    float* red = reinterpret_cast<float*>(p0);                          // [2][16 warps][NT * 4][32] when ks > 1
+    if (A.ks > 1) p0 += 2 * kMmWarps * NT * 4 * 32 * sizeof(float);
+    uint8_t* acts = p0;
+    uint8_t* ring = acts + (size_t)TT * P * A.col_stride;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    ring += (size_t)warp * A.nst * STAGE;
+    if constexpr (T == T_IQ3_XXS) {
+        for (int i = tid; i < (int)(sizeof(MmCodebook) / 16); i += kMmThreads)
+            tcp::cp_async16<false>(reinterpret_cast<uint8_t*>(book) + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_codebook) + 16 * i);
+        tcp::cp_async_commit();
+        tcp::cp_async_wait_all();
+    }
+    if (tid < 32) amax[tid] = 0u;
+    pdl_wait();
+    pdl_launch_dependents();
+
+    // ---- first item of every segment ----
+    const int nseg = A.nseg_dev ? min(*A.nseg_dev, A.nseg_max) : A.nseg_max;
+    {
+        const int per = (nseg + kMmThreads - 1) / kMmThreads;
+        int sum = 0;
+        for (int j = 0; j < per; ++j) {
+            const int s = tid * per + j;
+            if (s < nseg) sum += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT) * A.rblocks;
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        int at = incl - sum;
+        for (int w = 0; w < warp; ++w) at += wsum[w];
+        for (int j = 0; j < per; ++j) {
+            const int s = tid * per + j;
+            if (s < nseg) {
+                pre[s] = at;
+                at += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT) * A.rblocks;
+            }
+        }
+        if (tid == kMmThreads - 1) pre[nseg] = at;
+        __syncthreads();
+    }
+    const int total = pre[nseg];
+    const int nb = A.n_in >> 8;
+    const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
+    const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
+    const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
+    const uint2* grid = book + (lane & (kLutRep - 1));
+    int par = 0;
+
+    for (int item = blockIdx.x; item < total; item += gridDim.x, par ^= 1) {
+        int lo = 0, hi = nseg;  // the segment: pre[lo] <= item < pre[lo + 1]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (pre[mid] <= item) lo = mid; else hi = mid;
+        }
+        const SegDesc sd = A.seg ? A.seg[lo] : A.single;
+        const int rem = item - pre[lo], tile = rem / A.rblocks, rbk = rem - tile * A.rblocks;
+        const int m = min(TT, (int)sd.m - tile * TT);
+        const uint32_t row0 = sd.row0 + tile * TT;
+        const int rg_end = min((rbk + 1) * A.rpi, n_rg);
+        int rg = rbk * A.rpi + slot;
+        const int nrg = rg < rg_end ? (rg_end - rg + nslot - 1) / nslot : 0;
+        const int nstage = nrg * kbn;
+
+        // ---- the warp's weight stream: block pf_b of row group pf_rg goes to ring slot pf_s ----
+        int pf_rg = rg, pf_b = 0, pf_s = 0, pf_n = 0;
+        auto prefetch = [&]() {
+            if (pf_n < nstage) {
+                const uint32_t boff = (uint32_t)(kb0 + pf_b) * Q::BB;
+                uint8_t* dst = ring + pf_s * STAGE;
+                const int r_in = lane >> 3, c = lane & 7;
+                constexpr bool TAIL = Q::ALIGNED && Q::UNITS % 8 == 1;  // one odd unit per row: 16 lanes take it
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int row = FUSED ? pf_rg * 8 + (j & 1) * 4 + r_in : min(pf_rg * 16 + j * 4 + r_in, A.n_out - 1);
+                    const uint8_t* src = ((FUSED && j >= 2) ? sd.wb : sd.wa) + (size_t)row * A.rb + boff;
+                    int units = Q::UNITS;
+                    if constexpr (!Q::ALIGNED) {
+                        const uint32_t off = (uint32_t)(uintptr_t)src & 15u;
+                        src -= off;
+                        units = (int)(off + Q::BB + 15u) >> 4;
+                    }
+                    uint8_t* d = dst + (j * 4 + r_in) * Q::RS;
+#pragma unroll
+                    for (int cc = 0; cc < (TAIL ? Q::UNITS - 1 : Q::UNITS); cc += 8)
+                        if (cc + 8 <= Q::UNITS - (Q::ALIGNED ? 0 : 1) || cc + c < units) tcp::cp_async16(d + (cc + c) * 16, src + (cc + c) * 16);
+                }
+                if constexpr (TAIL) {
+                    if (lane < 16) {
+                        const int row = FUSED ? pf_rg * 8 + (lane & 7) : min(pf_rg * 16 + lane, A.n_out - 1);
+                        const uint8_t* src = ((FUSED && lane >= 8) ? sd.wb : sd.wa) + (size_t)row * A.rb + boff;
+                        tcp::cp_async16(dst + lane * Q::RS + (Q::UNITS - 1) * 16, src + (Q::UNITS - 1) * 16);
+                    }
+                }
+                ++pf_n;
+                if (++pf_b == kbn) { pf_b = 0; pf_rg += nslot; }
+                if (++pf_s == A.nst) pf_s = 0;
+            }
+            tcp::cp_async_commit();
+        };
+        for (int i = 1; i < A.nst; ++i) prefetch();
+
+        // ---- activations: largest element of each row, then the split into P columns ----
+        for (int gi = warp; gi < m * nb; gi += kMmWarps) {  // one 256-element block of one token per warp
+            const int tok = gi / nb, b = gi - tok * nb;
+            const uint32_t pr = row0 + tok;
+            const float* xr = A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256;
+            const float4 v0 = *reinterpret_cast<const float4*>(xr + 4 * lane), v1 = *reinterpret_cast<const float4*>(xr + 128 + 4 * lane);
+            uint32_t mx = max(max(__float_as_uint(fabsf(v0.x)), __float_as_uint(fabsf(v0.y))), max(__float_as_uint(fabsf(v0.z)), __float_as_uint(fabsf(v0.w))));
+            mx = max(mx, max(max(__float_as_uint(fabsf(v1.x)), __float_as_uint(fabsf(v1.y))), max(__float_as_uint(fabsf(v1.z)), __float_as_uint(fabsf(v1.w)))));
+            mx = __reduce_max_sync(0xffffffffu, mx);
+            if (lane == 0) atomicMax(&amax[par * 16 + tok], mx);  // a maximum: any order gives the same
+        }
+        __syncthreads();
+        for (int gi = warp; gi < m * nb; gi += kMmWarps) {
+            const int tok = gi / nb, b = gi - tok * nb;
+            const uint32_t pr = row0 + tok;
+            const float* xr = A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256;
+            const float s = mm_row_scale(amax[par * 16 + tok]);
+            int e0, e1;
+            mm_unit_elems<T>(g, t, e0, e1);  // lane = 4 * unit + quarter
+            float4 v0 = *reinterpret_cast<const float4*>(xr + e0), v1 = *reinterpret_cast<const float4*>(xr + e1);
+            v0.x *= s; v0.y *= s; v0.z *= s; v0.w *= s;
+            v1.x *= s; v1.y *= s; v1.z *= s; v1.w *= s;
+            uint32_t h[4][P];
+            if constexpr (mq_mins<T>) {
+                mm_split<P>(v0.x, v0.z, h[0]);
+                mm_split<P>(v0.y, v0.w, h[1]);
+                mm_split<P>(v1.x, v1.z, h[2]);
+                mm_split<P>(v1.y, v1.w, h[3]);
+            } else {
+                mm_split<P>(v0.x, v0.y, h[0]);
+                mm_split<P>(v0.z, v0.w, h[1]);
+                mm_split<P>(v1.x, v1.y, h[2]);
+                mm_split<P>(v1.z, v1.w, h[3]);
+            }
+            uint8_t* col = acts + (size_t)tok * P * A.col_stride;
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+                *reinterpret_cast<uint4*>(col + (size_t)p * A.col_stride + b * 512 + lane * 16) = make_uint4(h[0][p], h[1][p], h[2][p], h[3][p]);
+            if constexpr (mq_mins<T>) {  // sums of the lane's two sub-blocks, over the eight units
+                float a = (v0.x + v0.y) + (v0.z + v0.w), c = (v1.x + v1.y) + (v1.z + v1.w);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    a += __shfl_xor_sync(0xffffffffu, a, o);
+                    c += __shfl_xor_sync(0xffffffffu, c, o);
+                }
+                uint32_t sp[P];
+                mm_split<P>(a, c, sp);
+                if (g == 0) {
+#pragma unroll
+                    for (int p = 0; p < P; ++p) *reinterpret_cast<uint32_t*>(col + (size_t)p * A.col_stride + A.n_in * 2 + b * 16 + t * 4) = sp[p];
+                }
+            }
+        }
+        if (tid < 16) amax[(par ^ 1) * 16 + tid] = 0u;
+        __syncthreads();
+
+        // ---- the row groups ----
+        const int nt = (m + TPT - 1) / TPT;
+        const uint8_t* colb[NT];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const int tok = min(n * TPT + (P == 3 ? g >> 2 : g >> 1), m - 1), part = P == 3 ? min(g & 3, 2) : g & 1;
+            colb[n] = acts + (size_t)(tok * P + part) * A.col_stride;
+        }
+        float acc[NT][4];
+        int q_s = 0, q_b = 0, round = 0;
+        for (int q = 0; q < nstage; ++q) {
+            if (A.nst == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            else if (A.nst == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 2;" ::: "memory");
+            __syncwarp();  // the stage is complete for every lane, and every lane has left the slot that is filled next
+            prefetch();
+            const uint8_t* st = ring + q_s * STAGE;
+            const uint8_t* ra = st + g * Q::RS;
+            const uint8_t* rb = st + (g + 8) * Q::RS;
+            if constexpr (!Q::ALIGNED) {
+                const uint32_t boff = (uint32_t)(kb0 + q_b) * Q::BB;
+                const uint32_t r0 = FUSED ? rg * 8 + g : min(rg * 16 + g, A.n_out - 1), r1 = FUSED ? r0 : (uint32_t)min(rg * 16 + 8 + g, A.n_out - 1);
+                ra += (r0 * (uint32_t)A.rb + boff) & 15u;
+                rb += (r1 * (uint32_t)A.rb + boff) & 15u;
+            }
+            if (q_b == 0) {
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
+            }
+            const uint8_t* bp[NT];
+            uint32_t sumw[NT];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                bp[n] = colb[n] + (kb0 + q_b) * 512 + t * 16;
+                sumw[n] = 0u;
+                if constexpr (mq_mins<T>) {
+                    if (n < nt) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + A.n_in * 2 + (kb0 + q_b) * 16 + t * 4);
+                }
+            }
+            mm_block<T, NT>(ra, rb, t, grid, bp, sumw, nt, acc);
+            if (++q_s == A.nst) q_s = 0;
+            if (++q_b == kbn) {
+                q_b = 0;
+                bool mine = true;
+                if (A.ks > 1) {  // the warps of the row group meet; the first adds the others' sums in order
+                    float* rp = red + ((size_t)(round & 1) * kMmWarps + warp) * NT * 4 * 32 + lane;
+                    mine = kpart == 0;
+                    if (!mine) {
+#pragma unroll
+                        for (int n = 0; n < NT; ++n)
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) rp[(n * 4 + c) * 32] = acc[n][c];
+                    }
+                    mm_barrier(1 + slot, A.ks * 32);
+                    if (mine) {
+                        for (int k2 = 1; k2 < A.ks; ++k2) {
+                            rp += NT * 4 * 32;
+#pragma unroll
+                            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) acc[n][c] += rp[(n * 4 + c) * 32];
+                        }
+                    }
+                }
+                if (mine) {
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        if (n < nt) {
+                            float a, b;  // this row of both halves of the tile, one token
+                            int tok;
+                            if constexpr (P == 3) {
+                                a = (t & 1) ? acc[n][0] : acc[n][0] + acc[n][1];
+                                b = (t & 1) ? acc[n][2] : acc[n][2] + acc[n][3];
+                                a += __shfl_xor_sync(0xffffffffu, a, 1);
+                                b += __shfl_xor_sync(0xffffffffu, b, 1);
+                                tok = n * TPT + (t >> 1);
+                            } else {
+                                a = acc[n][0] + acc[n][1];
+                                b = acc[n][2] + acc[n][3];
+                                tok = n * TPT + t;
+                            }
+                            if (tok < m) {
+                                const float s = mm_row_scale(amax[par * 16 + tok]);
+                                const float inv = __uint_as_float((254u << 23) - __float_as_uint(s));  // 1 / 2^s: exponent 254 - e
+                                a *= inv;
+                                b *= inv;
+                                float* o = A.out + (size_t)(row0 + tok) * A.n_out;
+                                if constexpr (FUSED) {
+                                    if (P == 2 || !(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
+                                } else {
+                                    const int r = rg * 16 + g;
+                                    if ((P == 2 || !(t & 1)) && r < A.n_out) o[r] = a;
+                                    if ((P == 2 || (t & 1)) && r + 8 < A.n_out) o[r + 8] = b;
+                                }
+                            }
+                        }
+                    }
+                }
+                rg += nslot;
+                ++round;
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // every warp has left the activations
+    }
+}
+
+template <int T, bool FUSED, int P, int NT>
+static int launch_mm_t(dnb_ctx* c, cudaStream_t st, MmArgs A, size_t smem, int grid, const char* name) {
+    auto kern = mm_kernel<T, FUSED, P, NT>;
+    static SmemGrant grant;
+    DNB_CUDA(grant_smem(grant, c->device, kern, smem));
+    ProfScope prof_(c, st, name);
+    DNB_CUDA(launch_k(kern, dim3(grid), dim3(kMmThreads), smem, st, c->use_pdl, A));
+    c->launches++;
+    return DNB_OK;
+}
+
+bool mm_handles(int type, int n_in) {
+    return (type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_Q8_0 || type == T_IQ3_XXS) && n_in % 256 == 0 && n_in > 0;
+}
+
+template <int T>
+static int mm_launch_type(dnb_ctx* c, cudaStream_t st, bool fused, int parts, int nt, MmArgs& A, size_t smem, int grid, const char* name) {
+#define DNB_MM(F, P, N) return launch_mm_t<T, F, P, N>(c, st, A, smem, grid, name)
+    if (parts == 2) {
+        if constexpr (T == T_Q4_K || T == T_IQ3_XXS) {
+            if (fused) { if (nt == 1) DNB_MM(true, 2, 1); DNB_MM(true, 2, 2); }
+            if (nt == 1) DNB_MM(false, 2, 1);
+            DNB_MM(false, 2, 2);
+        }
+        return DNB_DECLINED;
+    }
+    if (fused) { if (nt == 1) DNB_MM(true, 3, 1); if (nt == 2) DNB_MM(true, 3, 2); DNB_MM(true, 3, 4); }
+    if (nt == 1) DNB_MM(false, 3, 1);
+    if (nt == 2) DNB_MM(false, 3, 2);
+    DNB_MM(false, 3, 4);
+#undef DNB_MM
+}
+
+// rows: token rows of the launch in total; nseg_est: segments that will have rows (an estimate when the device counts them).
+int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
+              int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
+              const SegDesc* single, const char* name) {
+    if (!mm_handles(type, n_in) || n_out < 1 || (fused && n_out % 8) || nseg_max < 1 || nseg_max > kMmSegMax || rows < 1) return DNB_DECLINED;
+    if (!seg && !single) return DNB_ERR_ARG;
+    if ((((uintptr_t)x) & 15) || ldx % 4 || (single && ((((uintptr_t)single->wa) & 15) || (fused && (((uintptr_t)single->wb) & 15))))) return DNB_DECLINED;
+    if (type != T_Q4_K && type != T_IQ3_XXS) parts = 3;
+    int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
+    if (rc) return rc;
+    const int bb = type == T_Q4_K ? 144 : type == T_Q5_K ? 176 : type == T_Q6_K ? 210 : type == T_Q8_0 ? 272 : 98;
+    const int rs = type == T_Q4_K ? Mq<T_Q4_K>::RS : type == T_Q5_K ? Mq<T_Q5_K>::RS : type == T_Q6_K ? Mq<T_Q6_K>::RS
+                 : type == T_Q8_0 ? Mq<T_Q8_0>::RS : Mq<T_IQ3_XXS>::RS;
+    MmArgs A = {};
+    A.seg = seg; A.nseg_dev = nseg_dev; A.nseg_max = nseg_max;
+    if (single) A.single = *single;
+    A.n_in = n_in; A.n_out = n_out; A.rb = bb * (n_in / 256);
+    A.x = x; A.ldx = ldx; A.row_token = row_token; A.out = out;
+    // columns 64 bytes apart modulo 128: the two columns a quarter-warp reads together fall on different banks
+    A.col_stride = n_in * 2 + (n_in / 16 + 127) / 128 * 128 + 64;
+    // Column tiles: the fewest that hold an average segment (a wider instance costs registers and shared memory, a narrower
+    // one decodes a segment's weights once more per tile).
+    const int tpt = parts == 3 ? 2 : 4, max_nt = parts == 3 ? 4 : 2;
+    const float avg = (float)rows / (float)std::max(1, nseg_est);
+    int nt = 1;
+    while (nt < max_nt && avg > 0.75f * nt * tpt) nt *= 2;
+    const int n_rg = fused ? n_out / 8 : (n_out + 15) / 16, nb = n_in / 256;
+    const size_t fixed = ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128 + (type == T_IQ3_XXS ? sizeof(MmCodebook) : 0);
+    for (;; nt /= 2) {
+        const int tiles = std::max(nseg_est, (int)((rows + nt * tpt - 1) / (nt * tpt)));
+        // K is split while the row groups do not give every warp of the chip one
+        int ks = 1;
+        while (ks < 8 && ks * 2 <= nb && (long)tiles * n_rg * ks < (long)c->sm_count * kMmWarps) ks *= 2;
+        const int nslot = kMmWarps / ks;
+        // items of one row group per warp, or of several while there are more than four items per SM
+        int per = 1;
+        while ((long)tiles * ((n_rg + nslot * per * 2 - 1) / (nslot * per * 2)) >= 4L * c->sm_count) per *= 2;
+        A.ks = ks;
+        A.rpi = nslot * per;
+        A.rblocks = (n_rg + A.rpi - 1) / A.rpi;
+        const size_t base = fixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 4 * 32 * 4 : 0) + (size_t)nt * tpt * parts * A.col_stride;
+        const size_t stage = (size_t)kMmWarps * 16 * rs, cap = 225 * 1024;
+        for (A.nst = 4; A.nst >= 2 && base + A.nst * stage > cap; --A.nst) {}
+        if (A.nst >= 2) {
+            const size_t smem = base + A.nst * stage;
+            const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, (long)tiles * A.rblocks);
+            switch (type) {
+                case T_Q4_K: return mm_launch_type<T_Q4_K>(c, st, fused, parts, nt, A, smem, grid, name);
+                case T_Q5_K: return mm_launch_type<T_Q5_K>(c, st, fused, parts, nt, A, smem, grid, name);
+                case T_Q6_K: return mm_launch_type<T_Q6_K>(c, st, fused, parts, nt, A, smem, grid, name);
+                case T_Q8_0: return mm_launch_type<T_Q8_0>(c, st, fused, parts, nt, A, smem, grid, name);
+                default: return mm_launch_type<T_IQ3_XXS>(c, st, fused, parts, nt, A, smem, grid, name);
+            }
+        }
+        if (nt == 1) return DNB_DECLINED;
+    }
+}
+
+}  // namespace dnb
