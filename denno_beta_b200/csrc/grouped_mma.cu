@@ -191,7 +191,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                 k_word<FIVE>(wb[i], fb[i] >> (2 * t), sb, q);
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    if (n < nt) {
+                    if (NT == 1 || n < nt) {
                         const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + (half * 4 + i) * 64);
                         mma_f16(D[n], p[0], q[0], p[1], q[1], y.x, y.y);
                         mma_f16(D[n], p[2], q[2], p[3], q[3], y.z, y.w);
@@ -201,7 +201,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
         }
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            if (n < nt) {
+            if (NT == 1 || n < nt) {
                 float M[4];
                 mma_f16_z(M, sa.mm, sb.mm, 0u, 0u, sumw[n], 0u);
                 acc[n][0] = fmaf(-sa.dmin, M[0], fmaf(sa.d, D[n][0], acc[n][0]));
@@ -212,17 +212,30 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
         }
     } else if constexpr (T == T_IQ3_XXS) {
         const float da = h2f(ld16(ra)) * 0.25f, db = h2f(ld16(rb)) * 0.25f;
-#pragma unroll 4
+        // the eight sub-block words of a row as aligned words, shifted into place (a block starts on any even byte)
+        const uint32_t ma = (tcp::s32(ra) + 2u) & 2u, mb = (tcp::s32(rb) + 2u) & 2u;
+        const uint32_t* wa = reinterpret_cast<const uint32_t*>(ra + 66 - ma);
+        const uint32_t* wb = reinterpret_cast<const uint32_t*>(rb + 66 - mb);
+        const uint32_t sa = ma * 8u, sb = mb * 8u;
+        const uint8_t* ia = ra + 2 + 2 * t;
+        const uint8_t* ibp = rb + 2 + 2 * t;
+        const int st = 7 * t;
+        uint32_t la = wa[0], lb = wb[0];
+#pragma unroll
         for (int ib = 0; ib < 8; ++ib) {
-            const uint32_t xa = ld32u(ra + 66 + 4 * ib), xb = ld32u(rb + 66 + 4 * ib);
+            // the ninth word belongs to the row only where the words are shifted
+            const uint32_t na = wa[ib < 7 ? ib + 1 : 7 + (ma >> 1)], nbw = wb[ib < 7 ? ib + 1 : 7 + (mb >> 1)];
+            const uint32_t xa = __funnelshift_r(la, na, sa), xb = __funnelshift_r(lb, nbw, sb);
+            la = na;
+            lb = nbw;
             uint32_t p[4], q[4];
-            iq3_pairs_h(grid, ld16(ra + 2 + 8 * ib + 2 * t), (xa >> (7 * t)) & 127u, p);
-            iq3_pairs_h(grid, ld16(rb + 2 + 8 * ib + 2 * t), (xb >> (7 * t)) & 127u, q);
+            iq3_pairs_h(grid, ld16(ia + 8 * ib), (xa >> st) & 127u, p);
+            iq3_pairs_h(grid, ld16(ibp + 8 * ib), (xb >> st) & 127u, q);
             // d * (0.5 + s) * 0.5 = (d / 4) * (2 s + 1) (kquant.rs:667)
             const float fa = fmaf((float)(xa >> 28), da + da, da), fb = fmaf((float)(xb >> 28), db + db, db);
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                if (n < nt) {
+                if (NT == 1 || n < nt) {
                     const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + ib * 64);
                     float D[4];
                     mma_f16_z(D, p[0], q[0], p[1], q[1], y.x, y.y);
@@ -251,7 +264,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
             }
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                if (n < nt) {
+                if (NT == 1 || n < nt) {
                     const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + ib * 64);
                     float D[4];
                     mma_f16_z(D, p[0], q[0], p[1], q[1], y.x, y.y);
@@ -283,7 +296,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                     const float fa = da * (float)(int)*reinterpret_cast<const int8_t*>(ra + sc), fb = db * (float)(int)*reinterpret_cast<const int8_t*>(rb + sc);
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
-                        if (n < nt) {
+                        if (NT == 1 || n < nt) {
                             const uint2 y = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 64 + 8 * hi);
                             float D[4];
                             mma_f16_z(D, p0, q0, p1, q1, y.x, y.y);
@@ -309,7 +322,6 @@ struct MmArgs {
     int ldx;
     const int32_t* row_token;  // packed row -> x row, or null
     float* out;                // [packed row][n_out]
-    int rpi, rblocks;          // row groups per item, items per (segment, tile)
     int ks, nst;               // warps that split K, stages of a warp's ring
     int col_stride;            // bytes between B columns
 };
@@ -344,7 +356,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     constexpr int TT = NT * TPT;         // tokens of an item
     constexpr int STAGE = 16 * Q::RS;
     extern __shared__ __align__(128) uint8_t smem[];
-    int* pre = reinterpret_cast<int*>(smem);                            // [kMmSegMax + 1] first item of a segment
+    int* pre = reinterpret_cast<int*>(smem);                            // [kMmSegMax + 1] first token tile of a segment
     int* wsum = pre + kMmSegMax + 4;                                    // [16]
     uint32_t* amax = reinterpret_cast<uint32_t*>(wsum + 16);            // [2][16]
     uint8_t* p0 = smem + ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
@@ -367,14 +379,14 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     pdl_wait();
     pdl_launch_dependents();
 
-    // ---- first item of every segment ----
+    // ---- first token tile of every segment ----
     const int nseg = A.nseg_dev ? min(*A.nseg_dev, A.nseg_max) : A.nseg_max;
     {
         const int per = (nseg + kMmThreads - 1) / kMmThreads;
         int sum = 0;
         for (int j = 0; j < per; ++j) {
             const int s = tid * per + j;
-            if (s < nseg) sum += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT) * A.rblocks;
+            if (s < nseg) sum += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT);
         }
         int incl = sum;
 #pragma unroll
@@ -390,67 +402,87 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
             const int s = tid * per + j;
             if (s < nseg) {
                 pre[s] = at;
-                at += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT) * A.rblocks;
+                at += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT);
             }
         }
         if (tid == kMmThreads - 1) pre[nseg] = at;
         __syncthreads();
     }
-    const int total = pre[nseg];
     const int nb = A.n_in >> 8;
     const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
     const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
     const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
     const uint2* grid = book + (lane & (kLutRep - 1));
     int par = 0;
+    // this CTA's share of all (tile, row group) pairs: a range of pairs in a row, so that every CTA gets the same number
+    const long total = (long)pre[nseg] * n_rg;
+    const long at1 = total * (blockIdx.x + 1) / gridDim.x;
 
-    for (int item = blockIdx.x; item < total; item += gridDim.x, par ^= 1) {
-        int lo = 0, hi = nseg;  // the segment: pre[lo] <= item < pre[lo + 1]
+    for (long at = total * blockIdx.x / gridDim.x; at < at1; par ^= 1) {
+        const int gtile = (int)(at / n_rg), rg_begin = (int)(at - (long)gtile * n_rg);
+        const int rg_end = (int)min((long)n_rg, rg_begin + (at1 - at));
+        at += rg_end - rg_begin;
+        int lo = 0, hi = nseg;  // the segment: pre[lo] <= gtile < pre[lo + 1]
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
-            if (pre[mid] <= item) lo = mid; else hi = mid;
+            if (pre[mid] <= gtile) lo = mid; else hi = mid;
         }
         const SegDesc sd = A.seg ? A.seg[lo] : A.single;
-        const int rem = item - pre[lo], tile = rem / A.rblocks, rbk = rem - tile * A.rblocks;
+        const int tile = gtile - pre[lo];
         const int m = min(TT, (int)sd.m - tile * TT);
         const uint32_t row0 = sd.row0 + tile * TT;
-        const int rg_end = min((rbk + 1) * A.rpi, n_rg);
-        int rg = rbk * A.rpi + slot;
+        int rg = rg_begin + slot;
         const int nrg = rg < rg_end ? (rg_end - rg + nslot - 1) / nslot : 0;
         const int nstage = nrg * kbn;
 
-        // ---- the warp's weight stream: block pf_b of row group pf_rg goes to ring slot pf_s ----
+        // ---- the warp's weight stream: the next block of the next row group goes to ring slot pf_s ----
+        // A lane copies unit `lane & 7` (+ 8, 16) of rows lane / 8 + 4 j; a format with one unit over has 16 lanes copy that one.
         int pf_rg = rg, pf_b = 0, pf_s = 0, pf_n = 0;
+        const int r_in = lane >> 3, c16 = (lane & 7) * 16;
+        constexpr bool TAIL = Q::ALIGNED && Q::UNITS % 8 == 1;
+        const uint8_t *sa = nullptr, *sb = nullptr, *stl = nullptr;
+        uint32_t o1 = 4u * A.rb, o2 = 0, o3 = 0;
+        auto point = [&]() {  // row group pf_rg, first block
+            const uint32_t boff = (uint32_t)kb0 * Q::BB;
+            if constexpr (FUSED) {
+                const size_t off = (size_t)(pf_rg * 8 + r_in) * A.rb + boff;
+                sa = sd.wa + off;
+                sb = sd.wb + off;
+                if constexpr (TAIL) stl = (lane < 8 ? sd.wa : sd.wb) + (size_t)(pf_rg * 8 + (lane & 7)) * A.rb + boff + (Q::UNITS - 1) * 16;
+            } else {
+                const int row = pf_rg * 16 + r_in, last = A.n_out - 1;
+                const int r0 = min(row, last);
+                sa = sd.wa + (size_t)r0 * A.rb + boff;
+                o1 = (uint32_t)(min(row + 4, last) - r0) * A.rb;
+                o2 = (uint32_t)(min(row + 8, last) - r0) * A.rb;
+                o3 = (uint32_t)(min(row + 12, last) - r0) * A.rb;
+                if constexpr (TAIL) stl = sd.wa + (size_t)min(pf_rg * 16 + (lane & 15), last) * A.rb + boff + (Q::UNITS - 1) * 16;
+            }
+        };
+        if (nstage > 0) point();
         auto prefetch = [&]() {
             if (pf_n < nstage) {
-                const uint32_t boff = (uint32_t)(kb0 + pf_b) * Q::BB;
-                uint8_t* dst = ring + pf_s * STAGE;
-                const int r_in = lane >> 3, c = lane & 7;
-                constexpr bool TAIL = Q::ALIGNED && Q::UNITS % 8 == 1;  // one odd unit per row: 16 lanes take it
+                uint8_t* dst = ring + pf_s * STAGE + r_in * Q::RS + c16;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int row = FUSED ? pf_rg * 8 + (j & 1) * 4 + r_in : min(pf_rg * 16 + j * 4 + r_in, A.n_out - 1);
-                    const uint8_t* src = ((FUSED && j >= 2) ? sd.wb : sd.wa) + (size_t)row * A.rb + boff;
-                    int units = Q::UNITS;
-                    if constexpr (!Q::ALIGNED) {
-                        const uint32_t off = (uint32_t)(uintptr_t)src & 15u;
-                        src -= off;
-                        units = (int)(off + Q::BB + 15u) >> 4;
-                    }
-                    uint8_t* d = dst + (j * 4 + r_in) * Q::RS;
+                    const uint8_t* src = FUSED ? (j >= 2 ? sb : sa) + ((j & 1) ? o1 : 0u) : sa + (j == 0 ? 0u : j == 1 ? o1 : j == 2 ? o2 : o3);
+                    if constexpr (!Q::ALIGNED) src = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
 #pragma unroll
                     for (int cc = 0; cc < (TAIL ? Q::UNITS - 1 : Q::UNITS); cc += 8)
-                        if (cc + 8 <= Q::UNITS - (Q::ALIGNED ? 0 : 1) || cc + c < units) tcp::cp_async16(d + (cc + c) * 16, src + (cc + c) * 16);
+                        if (cc + 8 <= Q::UNITS || cc * 16 + c16 < Q::UNITS * 16) tcp::cp_async16(dst + j * 4 * Q::RS + cc * 16, src + cc * 16 + c16);
                 }
                 if constexpr (TAIL) {
-                    if (lane < 16) {
-                        const int row = FUSED ? pf_rg * 8 + (lane & 7) : min(pf_rg * 16 + lane, A.n_out - 1);
-                        const uint8_t* src = ((FUSED && lane >= 8) ? sd.wb : sd.wa) + (size_t)row * A.rb + boff;
-                        tcp::cp_async16(dst + lane * Q::RS + (Q::UNITS - 1) * 16, src + (Q::UNITS - 1) * 16);
-                    }
+                    if (lane < 16) tcp::cp_async16(ring + pf_s * STAGE + lane * Q::RS + (Q::UNITS - 1) * 16, stl);
+                    stl += Q::BB;
                 }
                 ++pf_n;
-                if (++pf_b == kbn) { pf_b = 0; pf_rg += nslot; }
+                sa += Q::BB;
+                if constexpr (FUSED) sb += Q::BB;
+                if (++pf_b == kbn) {
+                    pf_b = 0;
+                    pf_rg += nslot;
+                    if (pf_n < nstage) point();
+                }
                 if (++pf_s == A.nst) pf_s = 0;
             }
             tcp::cp_async_commit();
@@ -523,6 +555,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
         }
         float acc[NT][4];
         int q_s = 0, q_b = 0, round = 0;
+        uint32_t offa = 0, offb = 0;  // where a row's block starts (only the position inside 16 bytes matters)
         for (int q = 0; q < nstage; ++q) {
             if (A.nst == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
             else if (A.nst == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -533,10 +566,15 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
             const uint8_t* ra = st + g * Q::RS;
             const uint8_t* rb = st + (g + 8) * Q::RS;
             if constexpr (!Q::ALIGNED) {
-                const uint32_t boff = (uint32_t)(kb0 + q_b) * Q::BB;
-                const uint32_t r0 = FUSED ? rg * 8 + g : min(rg * 16 + g, A.n_out - 1), r1 = FUSED ? r0 : (uint32_t)min(rg * 16 + 8 + g, A.n_out - 1);
-                ra += (r0 * (uint32_t)A.rb + boff) & 15u;
-                rb += (r1 * (uint32_t)A.rb + boff) & 15u;
+                if (q_b == 0) {
+                    const uint32_t r0 = FUSED ? rg * 8 + g : min(rg * 16 + g, A.n_out - 1), r1 = FUSED ? r0 : (uint32_t)min(rg * 16 + 8 + g, A.n_out - 1);
+                    offa = r0 * (uint32_t)A.rb + (uint32_t)kb0 * Q::BB;
+                    offb = r1 * (uint32_t)A.rb + (uint32_t)kb0 * Q::BB;
+                }
+                ra += offa & 15u;
+                rb += offb & 15u;
+                offa += Q::BB;
+                offb += Q::BB;
             }
             if (q_b == 0) {
 #pragma unroll
@@ -582,7 +620,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
                 if (mine) {
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
-                        if (n < nt) {
+                        if (NT == 1 || n < nt) {
                             float a, b;  // this row of both halves of the tile, one token
                             int tok;
                             if constexpr (P == 3) {
@@ -684,23 +722,19 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
     const int n_rg = fused ? n_out / 8 : (n_out + 15) / 16, nb = n_in / 256;
     const size_t fixed = ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128 + (type == T_IQ3_XXS ? sizeof(MmCodebook) : 0);
     for (;; nt /= 2) {
-        const int tiles = std::max(nseg_est, (int)((rows + nt * tpt - 1) / (nt * tpt)));
-        // K is split while the row groups do not give every warp of the chip one
+        const long tiles = std::max(nseg_est, (rows + nt * tpt - 1) / (nt * tpt));
+        // A CTA's row groups go round its slots of `ks` warps; the last round is partly empty, so K is split until there are
+        // about six rounds (at most eight ways: each split costs an exchange of the sums).
+        const long per_cta = tiles * n_rg / c->sm_count;
         int ks = 1;
-        while (ks < 8 && ks * 2 <= nb && (long)tiles * n_rg * ks < (long)c->sm_count * kMmWarps) ks *= 2;
-        const int nslot = kMmWarps / ks;
-        // items of one row group per warp, or of several while there are more than four items per SM
-        int per = 1;
-        while ((long)tiles * ((n_rg + nslot * per * 2 - 1) / (nslot * per * 2)) >= 4L * c->sm_count) per *= 2;
+        while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
         A.ks = ks;
-        A.rpi = nslot * per;
-        A.rblocks = (n_rg + A.rpi - 1) / A.rpi;
         const size_t base = fixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 4 * 32 * 4 : 0) + (size_t)nt * tpt * parts * A.col_stride;
         const size_t stage = (size_t)kMmWarps * 16 * rs, cap = 225 * 1024;
         for (A.nst = 4; A.nst >= 2 && base + A.nst * stage > cap; --A.nst) {}
         if (A.nst >= 2) {
             const size_t smem = base + A.nst * stage;
-            const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, (long)tiles * A.rblocks);
+            const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, std::max<long>(1, tiles * n_rg * ks / kMmWarps));
             switch (type) {
                 case T_Q4_K: return mm_launch_type<T_Q4_K>(c, st, fused, parts, nt, A, smem, grid, name);
                 case T_Q5_K: return mm_launch_type<T_Q5_K>(c, st, fused, parts, nt, A, smem, grid, name);
