@@ -48,8 +48,14 @@ template <> struct Mq<T_Q8_0> { static constexpr int BB = 272, UNITS = 17, RS = 
 
 template <int T> constexpr bool mq_mins = (T == T_Q4_K || T == T_Q5_K);
 
-// IQ3_XXS codebook as fp16 pairs, kLutRep copies (a lane reads copy lane % kLutRep: no bank conflicts).
-struct MmCodebook { uint2 grid[256 * kLutRep]; };
+// IQ3_XXS tables in shared memory, kLutRep copies each (a lane reads copy lane % kLutRep: no bank conflicts).
+//   grid: the codebook as fp16 pairs, 128 bytes from entry to entry
+//   sgn : the eight signs of a 7-bit code (the eighth makes their number even): pair q of the eight weights at bits 15 - q and
+//         31 - q, so that a shift by q and a mask give the sign bits of a pair
+// The tables sit on a 32 KB boundary of the shared-memory address space: an entry's address is a shift and one and-or.
+struct MmCodebook { uint2 grid[256 * kLutRep]; uint32_t sgn[128 * kLutRep]; };
+constexpr uint32_t kMmBookAlign = 32768;
+constexpr uint32_t kMmSmemBase = 1024;  // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
 static __device__ __align__(16) MmCodebook g_mm_codebook;
 static bool g_mm_tables[64] = {false};
 
@@ -61,6 +67,12 @@ static int upload_mm_tables(int device) {
         uint32_t h[4];
         for (int j = 0; j < 4; ++j) h[j] = __half_as_ushort(__float2half((float)((dnb_iq3xxs_grid[e] >> (8 * j)) & 0xFFu)));
         for (int r = 0; r < kLutRep; ++r) tb.grid[e * kLutRep + r] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+    }
+    for (uint32_t code = 0; code < 128; ++code) {
+        const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
+        uint32_t u = 0;
+        for (int q = 0; q < 4; ++q) u |= ((sg >> (2 * q)) & 1u) << (15 - q) | ((sg >> (2 * q + 1)) & 1u) << (31 - q);
+        for (int r = 0; r < kLutRep; ++r) tb.sgn[code * kLutRep + r] = u;
     }
     DNB_CUDA(cudaMemcpyToSymbol(g_mm_codebook, &tb, sizeof(tb)));
     g_mm_tables[device] = true;
@@ -149,20 +161,23 @@ __device__ __forceinline__ void k_word(uint32_t w, uint32_t hq, const KScales& s
     p[3] = h2fma(d, s.s1, s.k1);
 }
 
-// Eight weights of an IQ3_XXS sub-block as four signed fp16 pairs.
-__device__ __forceinline__ void iq3_pairs_h(const uint2* grid, uint32_t idx, uint32_t code, uint32_t (&p)[4]) {
-    const uint32_t sg = code | ((__popc(code) & 1u) << 7);  // bit 7 makes the number of minus signs even
-    const uint2 g1 = grid[(idx & 0xFFu) * kLutRep], g2 = grid[(idx >> 8) * kLutRep];
-    p[0] = g1.x ^ ((sg * 0x40008000u) & 0x80008000u);
-    p[1] = g1.y ^ ((sg * 0x10002000u) & 0x80008000u);
-    p[2] = g2.x ^ ((sg * 0x04000800u) & 0x80008000u);
-    p[3] = g2.y ^ ((sg * 0x01000200u) & 0x80008000u);
+// Eight weights of an IQ3_XXS sub-block as four signed fp16 pairs.  gl, sl: shared addresses of the lane's copies; idx: the two
+// codebook indices; code: the sub-block word rotated so that the quarter's 7-bit sign code starts at bit 6.
+__device__ __forceinline__ void iq3_pairs_h(uint32_t gl, uint32_t sl, uint32_t idx, uint32_t code, uint32_t (&p)[4]) {
+    uint32_t u, g0, g1, g2, g3;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"((code & 0x1fc0u) | sl));  // constant tables: plain asm, free to move
+    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(g0), "=r"(g1) : "r"(((idx << 7) & 0x7f80u) | gl));
+    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(g2), "=r"(g3) : "r"(((idx >> 1) & 0x7f80u) | gl));
+    p[0] = g0 ^ (u & 0x80008000u);
+    p[1] = g1 ^ ((u << 1) & 0x80008000u);
+    p[2] = g2 ^ ((u << 2) & 0x80008000u);
+    p[3] = g3 ^ ((u << 3) & 0x80008000u);
 }
 
 // One 256-element block of 16 rows (this lane: rows `ra` and `rb`) against NT column tiles; bp[i]: the lane's B column of tile
 // i at this block; nt: tiles in use.  acc += scales * sums.
 template <int T, int NT>
-__device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, const uint2* grid, const uint8_t* const (&bp)[NT],
+__device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, uint32_t gl, uint32_t sl, const uint8_t* const (&bp)[NT],
                                          const uint32_t (&sumw)[NT], int nt, float (&acc)[NT][4]) {
     if constexpr (mq_mins<T>) {
         const KScales sa = k_scales(ra, t), sb = k_scales(rb, t);
@@ -219,7 +234,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
         const uint32_t sa = ma * 8u, sb = mb * 8u;
         const uint8_t* ia = ra + 2 + 2 * t;
         const uint8_t* ibp = rb + 2 + 2 * t;
-        const int st = 7 * t;
+        const int st = (7 * t + 26) & 31;
         uint32_t la = wa[0], lb = wb[0];
 #pragma unroll
         for (int ib = 0; ib < 8; ++ib) {
@@ -229,8 +244,8 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
             la = na;
             lb = nbw;
             uint32_t p[4], q[4];
-            iq3_pairs_h(grid, ld16(ia + 8 * ib), (xa >> st) & 127u, p);
-            iq3_pairs_h(grid, ld16(ibp + 8 * ib), (xb >> st) & 127u, q);
+            iq3_pairs_h(gl, sl, ld16(ia + 8 * ib), __funnelshift_r(xa, xa, st), p);
+            iq3_pairs_h(gl, sl, ld16(ibp + 8 * ib), __funnelshift_r(xb, xb, st), q);
             // d * (0.5 + s) * 0.5 = (d / 4) * (2 s + 1) (kquant.rs:667)
             const float fa = fmaf((float)(xa >> 28), da + da, da), fb = fmaf((float)(xb >> 28), db + db, db);
 #pragma unroll
@@ -324,6 +339,8 @@ struct MmArgs {
     float* out;                // [packed row][n_out]
     int ks, nst;               // warps that split K, stages of a warp's ring
     int col_stride;            // bytes between B columns
+    uint32_t smem;             // bytes of dynamic shared memory
+    int* status;
 };
 
 __device__ __forceinline__ void mm_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
@@ -360,18 +377,26 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     int* wsum = pre + kMmSegMax + 4;                                    // [16]
     uint32_t* amax = reinterpret_cast<uint32_t*>(wsum + 16);            // [2][16]
     uint8_t* p0 = smem + ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
-    uint2* book = reinterpret_cast<uint2*>(p0);
-    if constexpr (T == T_IQ3_XXS) p0 += sizeof(MmCodebook);
     float* red = reinterpret_cast<float*>(p0);                          // [2][16 warps][NT * 4][32] when ks > 1
     if (A.ks > 1) p0 += 2 * kMmWarps * NT * 4 * 32 * sizeof(float);
     uint8_t* acts = p0;
-    uint8_t* ring = acts + (size_t)TT * P * A.col_stride;
+    p0 += (size_t)TT * P * A.col_stride;
+    uint8_t* book = p0;
+    if constexpr (T == T_IQ3_XXS) {
+        book += (kMmBookAlign - (tcp::s32(p0) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
+        p0 = book + sizeof(MmCodebook);
+    }
+    uint8_t* ring = p0;
+    if (T == T_IQ3_XXS && (uint32_t)(ring - smem) + kMmWarps * A.nst * STAGE > A.smem) {  // only if shared memory started elsewhere
+        if (threadIdx.x == 0) status_set(A.status, 26);
+        return;
+    }
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     ring += (size_t)warp * A.nst * STAGE;
     if constexpr (T == T_IQ3_XXS) {
         for (int i = tid; i < (int)(sizeof(MmCodebook) / 16); i += kMmThreads)
-            tcp::cp_async16<false>(reinterpret_cast<uint8_t*>(book) + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_codebook) + 16 * i);
+            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_codebook) + 16 * i);
         tcp::cp_async_commit();
         tcp::cp_async_wait_all();
     }
@@ -412,7 +437,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
     const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
     const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
-    const uint2* grid = book + (lane & (kLutRep - 1));
+    const uint32_t gl = tcp::s32(book) + 8 * (lane & (kLutRep - 1)), sl = tcp::s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
     int par = 0;
     // this CTA's share of all (tile, row group) pairs: a range of pairs in a row, so that every CTA gets the same number
     const long total = (long)pre[nseg] * n_rg;
@@ -592,7 +617,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
                     if (n < nt) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + A.n_in * 2 + (kb0 + q_b) * 16 + t * 4);
                 }
             }
-            mm_block<T, NT>(ra, rb, t, grid, bp, sumw, nt, acc);
+            mm_block<T, NT>(ra, rb, t, gl, sl, bp, sumw, nt, acc);
             if (++q_s == A.nst) q_s = 0;
             if (++q_b == kbn) {
                 q_b = 0;
@@ -720,7 +745,7 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
     int nt = 1;
     while (nt < max_nt && avg > 0.75f * nt * tpt) nt *= 2;
     const int n_rg = fused ? n_out / 8 : (n_out + 15) / 16, nb = n_in / 256;
-    const size_t fixed = ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128 + (type == T_IQ3_XXS ? sizeof(MmCodebook) : 0);
+    const size_t fixed = ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
     for (;; nt /= 2) {
         const long tiles = std::max(nseg_est, (rows + nt * tpt - 1) / (nt * tpt));
         // A CTA's row groups go round its slots of `ks` warps; the last round is partly empty, so K is split until there are
@@ -729,11 +754,15 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
         int ks = 1;
         while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
         A.ks = ks;
-        const size_t base = fixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 4 * 32 * 4 : 0) + (size_t)nt * tpt * parts * A.col_stride;
+        size_t base = fixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 4 * 32 * 4 : 0) + (size_t)nt * tpt * parts * A.col_stride;
+        if (type == T_IQ3_XXS)  // the tables behind the activations, on their boundary (dynamic shared memory starts at kMmSmemBase)
+            base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmCodebook);
         const size_t stage = (size_t)kMmWarps * 16 * rs, cap = 225 * 1024;
         for (A.nst = 4; A.nst >= 2 && base + A.nst * stage > cap; --A.nst) {}
         if (A.nst >= 2) {
             const size_t smem = base + A.nst * stage;
+            A.smem = (uint32_t)smem;
+            A.status = c->status;
             const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, std::max<long>(1, tiles * n_rg * ks / kMmWarps));
             switch (type) {
                 case T_Q4_K: return mm_launch_type<T_Q4_K>(c, st, fused, parts, nt, A, smem, grid, name);

@@ -87,6 +87,7 @@ uint64_t dnb_launch_count(dnb_ctx* ctx);
  *   24       expert-parallel decode: a peer's result rows did not arrive
  *   23       grid barrier of the fused one-token kernel
  *   25       the tensor-core router GEMM of a prefill chunk (stage or accumulator barrier)
+ *   26       no wait: the mma.sync grouped kernel found its shared memory laid out otherwise than it asked for
  * What the reference promises for a GPU call that did not complete -- "false: out
  * untouched, the caller recomputes" (cuda.rs:21024-21027, 8785-8788) -- holds here too:
  * every host-buffer entry point reads the word after its stream synchronisation and, when
