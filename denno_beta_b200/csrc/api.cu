@@ -32,8 +32,8 @@ static int dev_alloc(T** p, size_t n) {
 
 static void free_ws(Workspace& w) {
     void* dev[] = {w.act_h, w.xn_perm, w.act_perm, w.xn, w.logits, w.wts, w.act, w.hrow, w.sact, w.sh, w.hin, w.out, w.shcoef, w.sels, w.row_token,
-                   w.pos, w.nseg, w.counts, w.one, w.seg_gu, w.seg_dn, w.seg_sh_gu, w.seg_sh_dn, w.xg_hi, w.xg_lo, w.act_hi, w.act_lo,
-                   w.x3, w.rpart, w.xq_hi, w.xq_lo, w.aq_hi, w.aq_lo, w.xq_scale, w.aq_scale};
+                   w.pos, w.nseg, w.counts, w.one, w.seg_gu, w.seg_dn, w.seg_sh_gu, w.seg_sh_dn, w.op_x, w.op_act,
+                   w.x3, w.rpart};
     for (void* p : dev)
         if (p) cudaFree(p);
     if (w.pinned_in) cudaFreeHost(w.pinned_in);
@@ -86,34 +86,14 @@ static int ensure_ws(dnb_ctx* c, int nt) {
     if ((rc = dev_alloc(&w.seg_dn, nseg_cap))) return rc;
     if ((rc = dev_alloc(&w.seg_sh_gu, 1))) return rc;
     if ((rc = dev_alloc(&w.seg_sh_dn, 1))) return rc;
-    // bf16 hi/lo operand buffers of the tcgen05 path (a few rows of slack so that a
-    // tile that starts near the end stays inside the allocation)
-    const size_t rows_pad = rows + 128;
-    if ((rc = dev_alloc(&w.xg_hi, rows_pad * M.e))) return rc;
-    if ((rc = dev_alloc(&w.xg_lo, rows_pad * M.e))) return rc;
-    if ((rc = dev_alloc(&w.act_hi, rows_pad * M.ff))) return rc;
-    if ((rc = dev_alloc(&w.act_lo, rows_pad * M.ff))) return rc;
-    DNB_CUDA(cudaMemset(w.xg_hi, 0, rows_pad * M.e * 2));
-    DNB_CUDA(cudaMemset(w.xg_lo, 0, rows_pad * M.e * 2));
-    DNB_CUDA(cudaMemset(w.act_hi, 0, rows_pad * M.ff * 2));
-    DNB_CUDA(cudaMemset(w.act_lo, 0, rows_pad * M.ff * 2));
-    w.maps_ok = (M.e % 64 == 0 && M.ff % 64 == 0) &&
-                umma_make_maps(w.xg_hi, w.xg_lo, rows_pad, (uint64_t)M.e, &w.maps_x) == DNB_OK &&
-                umma_make_maps(w.act_hi, w.act_lo, rows_pad, (uint64_t)M.ff, &w.maps_act) == DNB_OK;
-    if (c->q4k_int && w.maps_ok && q4k_int_handles(M.e, M.ff, true) && q4k_int_handles(M.ff, M.e, false)) {
-        const size_t xp = (size_t)M.e + kQ4kIntXcols, ap = (size_t)M.ff + kQ4kIntXcols;
-        if ((rc = dev_alloc(&w.xq_hi, rows_pad * xp))) return rc;
-        if ((rc = dev_alloc(&w.xq_lo, rows_pad * xp))) return rc;
-        if ((rc = dev_alloc(&w.aq_hi, rows_pad * ap))) return rc;
-        if ((rc = dev_alloc(&w.aq_lo, rows_pad * ap))) return rc;
-        if ((rc = dev_alloc(&w.xq_scale, rows_pad))) return rc;
-        if ((rc = dev_alloc(&w.aq_scale, rows_pad))) return rc;
-        DNB_CUDA(cudaMemset(w.xq_hi, 0, rows_pad * xp * 2));  // the padding columns behind the sub-block sums stay zero
-        DNB_CUDA(cudaMemset(w.xq_lo, 0, rows_pad * xp * 2));
-        DNB_CUDA(cudaMemset(w.aq_hi, 0, rows_pad * ap * 2));
-        DNB_CUDA(cudaMemset(w.aq_lo, 0, rows_pad * ap * 2));
-        w.q4k_int_ok = umma_make_maps(w.xq_hi, w.xq_lo, rows_pad, xp, &w.maps_xq) == DNB_OK &&
-                       umma_make_maps(w.aq_hi, w.aq_lo, rows_pad, ap, &w.maps_aq) == DNB_OK;
+    // operand rows of the tcgen05 path (a few rows of slack so that a tile that starts near the end stays inside the allocation)
+    if (M.e % 256 == 0 && M.ff % 256 == 0) {
+        const size_t rows_pad = rows + 64;
+        if ((rc = dev_alloc(&w.op_x, rows_pad * 2 * tc_row_pitch(M.e)))) return rc;
+        if ((rc = dev_alloc(&w.op_act, rows_pad * 2 * tc_row_pitch(M.ff)))) return rc;
+        DNB_CUDA(cudaMemset(w.op_x, 0, rows_pad * 4 * tc_row_pitch(M.e)));
+        DNB_CUDA(cudaMemset(w.op_act, 0, rows_pad * 4 * tc_row_pitch(M.ff)));
+        w.maps_ok = tc_make_maps(w.op_x, rows_pad, M.e, &w.maps_x) == DNB_OK && tc_make_maps(w.op_act, rows_pad, M.ff, &w.maps_act) == DNB_OK;
     }
     if ((rc = router_tc_workspace(c, w, cap, M.ne, M.e))) return rc;
     w.pinned_cap = (size_t)cap * M.e * sizeof(float);
@@ -369,13 +349,11 @@ static int block_dev_decode_batch(dnb_ctx* c, int layer, const float* h, int nt,
                                w.act_perm, nt);
 }
 
-// Prefill chunks of all-Q4_K layers: expert-major packed rows as bf16 hi/lo, grouped
-// GEMMs on tcgen05 (gate/up with the SwiGLU epilogue, then down), weighted combine.
-// The common block format of matrices [first, last) when a tensor-core grouped GEMM takes it
-// (Q4_K: three-product kernel of grouped_umma.cu; IQ3_XXS: exact-weight kernel of grouped_exact.cu), else -1.
+// The common block format of matrices [first, last) when the tcgen05 grouped GEMM (grouped_tc.cu) takes it, else -1.
+static bool tc_type_ok(int ty) { return ty == T_Q4_K || ty == T_IQ3_XXS; }
 static int tc_type(const Layer& L, int first, int last) {
     const int ty = L.m[first].type;
-    if (ty != T_Q4_K && ty != T_IQ3_XXS) return -1;
+    if (!tc_type_ok(ty)) return -1;
     for (int i = first; i < last; ++i)
         if (!L.m[i].dev || L.m[i].type != ty) return -1;
     return ty;
@@ -387,17 +365,17 @@ static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMi
 static bool umma_eligible(const dnb_ctx* c, const Layer& L, int nt) {
     const Model& M = c->model;
     if (!c->use_umma || !c->ws.maps_ok) return false;
-    if (M.e % 256 || M.ff % 256 || M.e % 128 || M.ff % 128) return false;
     const int ty = tc_type(L, 0, 3);
-    if (ty < 0 || nt < tc_min_tokens(c, ty)) return false;
+    if (ty < 0 || nt < tc_min_tokens(c, ty) || !tc_handles(ty, M.e, M.ff, true) || !tc_handles(ty, M.ff, M.e, false)) return false;
     if (L.has_shared()) {  // the shared expert rides in the same launches as one more segment
         if (tc_type(L, 3, 6) != ty || L.m[3].n_out != M.ff) return false;
     }
     return true;
 }
 
+// op_ready: the operand rows of x are in the workspace (written with the RMSNorm).
 static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts,
-                            float* out, int k = -1, int ne = -1, int with_shared = -1) {
+                            float* out, int k = -1, int ne = -1, int with_shared = -1, bool op_ready = false) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
     Workspace& w = c->ws;
@@ -410,24 +388,11 @@ static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const
     const int rows = nt * k + (shared ? nt : 0);
     const int nseg_max = (nt * k < ne ? nt * k : ne) + (shared ? 1 : 0);
     const int ty = L.m[0].type;
-    if (ty == T_Q4_K && c->q4k_int && w.q4k_int_ok) {
-        // integer weights, block scales after the tensor-core sum: fp16 rows in, fp32 activations between the two GEMMs
-        if ((rc = launch_rows_f16(c, st, x, M.e, w.row_token, rows, M.e, w.xq_hi, w.xq_lo, w.xq_scale, "rows_f16_x"))) return rc;
-        if ((rc = launch_grouped_q4k_int(c, st, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, &w.maps_xq, w.xq_scale, w.act))) return rc;
-        if ((rc = launch_rows_f16(c, st, w.act, M.ff, nullptr, rows, M.ff, w.aq_hi, w.aq_lo, w.aq_scale, "rows_f16_act"))) return rc;
-        if ((rc = launch_grouped_q4k_int(c, st, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, &w.maps_aq, w.aq_scale, w.hrow))) return rc;
-        if (shared && L.shared_gate_row)
-            if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
-        return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
-                              (shared && L.shared_gate_row) ? w.shcoef : nullptr, out);
-    }
-    if ((rc = launch_gather_split(c, st, x, M.e, w.row_token, rows, M.e, w.xg_hi, w.xg_lo))) return rc;
-    if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, &w.maps_x, nt, w.act_hi, w.act_lo,
-                                nullptr)))
-        return rc;
-    if ((rc = launch_grouped_tc(c, st, ty, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, &w.maps_act, nt, nullptr, nullptr,
-                                w.hrow)))
-        return rc;
+    if (!op_ready)
+        if ((rc = launch_operand_rows(c, st, ty, x, M.e, nt, M.e, w.op_x, "operand_rows_x"))) return rc;
+    if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, w.op_x, &w.maps_x, w.row_token, w.act))) return rc;
+    if ((rc = launch_operand_rows(c, st, ty, w.act, M.ff, rows, M.ff, w.op_act, "operand_rows_act"))) return rc;
+    if ((rc = launch_grouped_tc(c, st, ty, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, w.op_act, &w.maps_act, nullptr, w.hrow))) return rc;
     if (shared && L.shared_gate_row)
         if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
     return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
@@ -508,9 +473,12 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out) 
         if (rc != DNB_DECLINED) return rc;
     }
     const bool shared = L.has_shared();
-    // the RMSNorm kernel writes the router's operand (three bf16 parts of the normalised rows) in the same pass
-    const bool split_in_prep = L.norm_w && router_tc_eligible(c, L, nt);
-    if (L.norm_w || shared) {
+    // the RMSNorm kernel writes the router's operand (three bf16 parts of the normalised rows) and the experts' in the same pass
+    const bool umma = umma_eligible(c, L, nt), split_in_prep = L.norm_w && router_tc_eligible(c, L, nt), op_in_prep = L.norm_w && umma;
+    if (op_in_prep) {
+        if ((rc = launch_prep_operand(c, st, L.m[0].type, h, L.norm_w, M.eps, nt, M.e, w.xn, split_in_prep ? w.x3 : nullptr, w.x3_part, w.op_x)))
+            return rc;
+    } else if (L.norm_w || shared) {
         if ((rc = launch_prep(c, st, h, L.norm_w, M.eps, nt, M.e, w.xn, shared ? w.seg_sh_gu : nullptr,
                               shared ? w.seg_sh_dn : nullptr, L.m[3].dev, L.m[4].dev, L.m[5].dev,
                               split_in_prep ? w.x3 : nullptr, w.x3_part)))
@@ -518,12 +486,32 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out) 
     }
     const float* x = L.norm_w ? w.xn : h;
     if ((rc = router_topk_dev(c, st, x, nt, L, w.sels, w.wts, nullptr, split_in_prep))) return rc;
-    if (umma_eligible(c, L, nt)) return experts_dev_umma(c, layer, x, nt, w.sels, w.wts, out);
+    if (umma) return experts_dev_umma(c, layer, x, nt, w.sels, w.wts, out, -1, -1, -1, op_in_prep);
     if (mma) {
         rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, nt >= 16 && tc_type(L, 0, 3) >= 0 ? 2 : 3);
         if (rc != DNB_DECLINED) return rc;
     }
     return experts_dev(c, layer, x, nt, w.sels, w.wts, out);
+}
+
+// The shared expert on all rows: one segment, rows in place.
+int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, float* out) {
+    const Model& M = c->model;
+    const Layer& L = M.layers[layer];
+    Workspace& w = c->ws;
+    cudaStream_t st = c->stream;
+    int rc;
+    if ((rc = launch_prep(c, st, x, nullptr, M.eps, rows, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev, L.m[4].dev, L.m[5].dev))) return rc;
+    const int sff = L.m[3].n_out, ty = sff == M.ff ? tc_type(L, 3, 6) : -1;
+    if (c->use_umma && w.maps_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
+        if (!op_ready)
+            if ((rc = launch_operand_rows(c, st, ty, x, M.e, rows, M.e, w.op_x, "operand_rows_x"))) return rc;
+        if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, &w.maps_x, nullptr, w.act))) return rc;
+        if ((rc = launch_operand_rows(c, st, ty, w.act, M.ff, rows, M.ff, w.op_act, "operand_rows_act"))) return rc;
+        return launch_grouped_tc(c, st, ty, false, w.seg_sh_dn, w.one, 1, M.ff, M.e, w.op_act, &w.maps_act, nullptr, out);
+    }
+    if ((rc = launch_seg_matmul(c, st, L.m[3].type, true, w.seg_sh_gu, nullptr, 1, M.e, sff, x, M.e, nullptr, w.sact, rows))) return rc;
+    return launch_seg_matmul(c, st, L.m[5].type, false, w.seg_sh_dn, nullptr, 1, sff, M.e, w.sact, sff, nullptr, out, rows);
 }
 
 }  // namespace dnb
@@ -820,9 +808,7 @@ int dnb_set_tc_min_tokens(dnb_ctx* c, int iq3_xxs_min_tokens) {
 int dnb_set_q4k_int(dnb_ctx* c, int on) {
     if (!c) return DNB_ERR_ARG;
     DNB_CUDA(cudaDeviceSynchronize());
-    drop_graphs(c);
-    if (c->q4k_int != (on != 0)) free_ws(c->ws);  // its operand buffers exist only while it is on: the next call sizes the workspace again
-    c->q4k_int = on != 0;
+    (void)on;  // the one tcgen05 kernel has integer weights
     return DNB_OK;
 }
 
@@ -1190,11 +1176,10 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
     SegDesc* dsd = (SegDesc*)c->gg_seg.p;
     int32_t* dnseg = (int32_t*)((uint8_t*)c->gg_seg.p + (size_t)nseg * sizeof(SegDesc));
     const Model& M = c->model;
-    // Q4_K matrices of the model's own shapes with enough rows go to the tcgen05 grouped GEMM
-    // (the packed rows are split to bf16 hi/lo in the workspace's operand buffers first).
+    // Matrices of the model's own shapes with enough rows per segment go to the tcgen05 grouped GEMM, the others to the mma.sync
+    // kernel (four rows per segment: where decoding a weight once per 32 tokens starts to pay for the 128-row tiles).
     const bool in_e = t.n_in == M.e, in_ff = t.n_in == M.ff;
-    bool umma = c->use_umma && ((t.type == T_Q4_K && row >= 64) || (t.type == T_IQ3_XXS && row >= 16)) && (in_e || in_ff) &&
-                t.n_in % 256 == 0 && t.n_out % 128 == 0;
+    bool umma = c->use_umma && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(t.type, t.n_in, t.n_out, false);
     if (umma) {
         if ((rc = ensure_ws(c, (int)((row + M.k) / (M.k + 1))))) return rc;
         umma = c->ws.maps_ok;
@@ -1204,14 +1189,16 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
     if (umma) {
         Workspace& w = c->ws;
         DNB_CUDA(cudaMemcpyAsync(dnseg, &nseg, sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-        uint16_t* hi = in_e ? w.xg_hi : w.act_hi;
-        uint16_t* lo = in_e ? w.xg_lo : w.act_lo;
-        if ((rc = launch_gather_split(c, c->stream, dx, t.n_in, nullptr, (int)row, t.n_in, hi, lo)) == DNB_OK)
-            rc = launch_grouped_tc(c, c->stream, t.type, false, dsd, dnseg, nseg, t.n_in, t.n_out, in_e ? &w.maps_x : &w.maps_act,
-                                   (int)row, nullptr, nullptr, dout);
+        uint16_t* op = in_e ? w.op_x : w.op_act;
+        if ((rc = launch_operand_rows(c, c->stream, t.type, dx, t.n_in, (int)row, t.n_in, op, "operand_rows_gemm")) == DNB_OK)
+            rc = launch_grouped_tc(c, c->stream, t.type, false, dsd, dnseg, nseg, t.n_in, t.n_out, op, in_e ? &w.maps_x : &w.maps_act, nullptr,
+                                   dout);
     } else {
-        rc = launch_seg_matmul(c, c->stream, t.type, false, dsd, nullptr, nseg, t.n_in, t.n_out, dx, t.n_in, nullptr, dout,
-                               (int)m_max);
+        rc = c->decode_fast ? launch_mm(c, c->stream, t.type, false, tc_type_ok(t.type) && row >= 64 ? 2 : 3, dsd, nullptr, nseg, nseg, (int)row,
+                                        t.n_in, t.n_out, dx, t.n_in, nullptr, dout, nullptr, "mm_grouped")
+                            : DNB_DECLINED;
+        if (rc == DNB_DECLINED)
+            rc = launch_seg_matmul(c, c->stream, t.type, false, dsd, nullptr, nseg, t.n_in, t.n_out, dx, t.n_in, nullptr, dout, (int)m_max);
     }
     if (rc == DNB_OK) {
         cudaError_t e = cudaMemcpyAsync(outs, dout, row * t.n_out * sizeof(float), cudaMemcpyDeviceToHost, c->stream);
@@ -1435,29 +1422,14 @@ int dnb_expert_rows_dev(dnb_ctx* c, int layer, const float* x_rows_dev, const in
     if (rc) return rc;
     Workspace& w = c->ws;
     cudaStream_t st = c->stream;
-    const int ty_routed = use_shared ? -1 : tc_type(L, 0, 3);
-    const int ty_shared = (L.has_shared() && L.m[3].n_out == M.ff) ? tc_type(L, 3, 6) : -1;
-    const bool q4k_routed = ty_routed >= 0, q4k_shared = ty_shared >= 0;
-    const bool umma = c->use_umma && w.maps_ok && rows >= 16 && M.e % 256 == 0 && M.ff % 256 == 0;
+    const bool tc_routed = !use_shared && tc_type(L, 0, 3) >= 0 && tc_handles(L.m[0].type, M.e, M.ff, true) && tc_handles(L.m[2].type, M.ff, M.e, false);
+    const bool umma = c->use_umma && w.maps_ok && rows >= 16;
     if (!use_shared) {
         // every row is one (token, slot): a "chunk" of `rows` tokens with one selected expert each and weight 1
-        if (umma && q4k_routed) return experts_dev_umma(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, 1, M.shard_count, 0);
+        if (umma && tc_routed) return experts_dev_umma(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, 1, M.shard_count, 0);
         return experts_dev(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, 1, M.shard_count, 0);
     }
-    // the shared expert on all rows: one segment, rows in place
-    if ((rc = launch_prep(c, st, x_rows_dev, nullptr, M.eps, rows, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev,
-                          L.m[4].dev, L.m[5].dev)))
-        return rc;
-    const int sff = L.m[3].n_out;
-    if (umma && q4k_shared) {
-        if ((rc = launch_gather_split(c, st, x_rows_dev, M.e, nullptr, rows, M.e, w.xg_hi, w.xg_lo))) return rc;
-        if ((rc = launch_grouped_tc(c, st, ty_shared, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, &w.maps_x, rows, w.act_hi, w.act_lo, nullptr)))
-            return rc;
-        return launch_grouped_tc(c, st, ty_shared, false, w.seg_sh_dn, w.one, 1, M.ff, M.e, &w.maps_act, rows, nullptr, nullptr, h_rows_dev);
-    }
-    if ((rc = launch_seg_matmul(c, st, L.m[3].type, true, w.seg_sh_gu, nullptr, 1, M.e, sff, x_rows_dev, M.e, nullptr, w.sact, rows)))
-        return rc;
-    return launch_seg_matmul(c, st, L.m[5].type, false, w.seg_sh_dn, nullptr, 1, sff, M.e, w.sact, sff, nullptr, h_rows_dev, rows);
+    return shared_rows(c, layer, x_rows_dev, rows, false, h_rows_dev);
 }
 
 int dnb_moe_combine_dev(dnb_ctx* c, int layer, const float* h_slots_dev, const float* wts_dev, const float* shared_dev,

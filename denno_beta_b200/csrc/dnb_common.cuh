@@ -88,8 +88,8 @@ struct Model {
     std::vector<Layer> layers;
 };
 
-struct alignas(64) UmmaMaps {  // eight TMA tensor maps (4 box heights x hi/lo), opaque here
-    unsigned char bytes[8 * 128];
+struct alignas(64) TcMaps {  // four TMA tensor maps of an operand array (grouped_tc.cu), opaque here
+    unsigned char bytes[4 * 128];
 };
 
 struct Workspace {             // device buffers of the MoE pipeline, sized for nt_cap tokens
@@ -101,14 +101,9 @@ struct Workspace {             // device buffers of the MoE pipeline, sized for 
     uint16_t* act_h = nullptr;  // bf16 triples of the fused decode kernel's activations (decode_fused.cu)
     int32_t *sels = nullptr, *row_token = nullptr, *pos = nullptr, *nseg = nullptr, *counts = nullptr, *one = nullptr;
     SegDesc *seg_gu = nullptr, *seg_dn = nullptr, *seg_sh_gu = nullptr, *seg_sh_dn = nullptr;
-    uint16_t *xg_hi = nullptr, *xg_lo = nullptr, *act_hi = nullptr, *act_lo = nullptr;  // bf16 hi/lo packed rows
-    UmmaMaps maps_x, maps_act;
+    uint16_t *op_x = nullptr, *op_act = nullptr;  // operand rows of the tcgen05 grouped GEMM: n_embd and n_ff wide (grouped_tc.cu)
+    TcMaps maps_x, maps_act;
     bool maps_ok = false;
-    // integer-weight Q4_K kernel (grouped_q4k_int.cu): fp16 hi / lo rows with the sub-block sums appended, row scales
-    uint16_t *xq_hi = nullptr, *xq_lo = nullptr, *aq_hi = nullptr, *aq_lo = nullptr;
-    float *xq_scale = nullptr, *aq_scale = nullptr;
-    UmmaMaps maps_xq, maps_aq;
-    bool q4k_int_ok = false;
     uint16_t* x3 = nullptr;    // [3][nt_cap + 128][e]: the chunk's rows as three bf16 parts (router_tc.cu)
     size_t x3_part = 0;        // elements between the parts
     float* rpart = nullptr;    // [K splits][nt][ne]: partial router sums
@@ -174,15 +169,14 @@ struct dnb_ctx {
     unsigned long long* gbar = nullptr; // grid barrier of the fused decode kernel: arrivals of all launches so far
     uint64_t launches = 0;              // kernels launched by this context (bench accounting)
     int gemv_impl = 0;                  // 0 = fast (default), 1 = sequential bit-exact
-    bool q4k_int = false;               // Q4_K chunks on the integer-weight tcgen05 kernel (grouped_q4k_int.cu): more exact, measured slower
     bool router_tc = true;              // router logits of large chunks on the tensor cores (router_tc.cu)
     bool decode_fast = true;            // one-token calls take the bulk-copy GEMV + fused router path
     bool use_pdl = true;                // programmatic dependent launch between the decode kernels
     bool gemv_mma = true;               // one-token IQ3_XXS kernels on mma.sync (gemv_mma.cu, decode_fused.cu) where the shape fits
     bool decode_fused = true;           // gate/up + down of a one-token IQ3_XXS block as one kernel (decode_fused.cu)
     bool decode_routed = true;          // ... with the router folded into the same kernel (one launch per block)
-    int exact_min_nt = 48;              // IQ3_XXS layers: tokens from which a batch takes the exact-weight tcgen05 kernel
-    bool use_umma = true;               // prefill chunks of Q4_K layers take the tcgen05 grouped GEMM
+    int exact_min_nt = 48;              // IQ3_XXS layers: tokens from which a batch takes the tcgen05 kernel
+    bool use_umma = true;               // prefill chunks of Q4_K and IQ3_XXS layers take the tcgen05 grouped GEMM
     void* ep = nullptr;                 // dnb::EpState of the peer-memory expert-parallel path (ep_p2p.cu)
     void* hc = nullptr;                 // dnb::HcState: hyper-connection mix weights and scratch (hc_mix.cu)
     void* epd = nullptr;                // dnb::EpdState of the expert-parallel decode path (ep_decode.cu)
@@ -277,6 +271,9 @@ int launch_rmsnorm(dnb_ctx* c, cudaStream_t st, const float* h, const float* w, 
 int launch_prep(dnb_ctx* c, cudaStream_t st, const float* h, const float* w, float eps, int nt, int e, float* out,
                 SegDesc* sh_gu, SegDesc* sh_dn, const uint8_t* sg, const uint8_t* su, const uint8_t* sdn,
                 uint16_t* x3 = nullptr, size_t x3_part = 0);
+// RMSNorm for a call on the tcgen05 experts: out, x3 (optional) and the operand rows of `type` (grouped_tc.cu) in one pass.
+int launch_prep_operand(dnb_ctx* c, cudaStream_t st, int type, const float* h, const float* w, float eps, int nt, int e, float* out, uint16_t* x3,
+                        size_t x3_part, uint16_t* op);
 int launch_add_inplace(dnb_ctx* c, cudaStream_t st, float* h, const float* d, size_t n);
 int launch_stage_in(dnb_ctx* c, cudaStream_t st, const float* host_pinned, float* dst, size_t n);  // DNB_DECLINED: use a copy
 int launch_stall(dnb_ctx* c, cudaStream_t st, float ms);
@@ -373,15 +370,6 @@ int router_topk_dev(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const L
 // One tensor map: [rows][cols] bf16 row-major, box = 64 columns x box_rows rows, 128-byte swizzle.  map: 128 bytes.
 int tc_make_map(void* map, void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
-// Q4_K grouped GEMM with integer fp16 weights and block scales after the tensor-core sum (grouped_q4k_int.cu)
-constexpr int kQ4kIntXcols = 64;  // sub-block sum columns appended to an activation row
-bool q4k_int_handles(int n_in, int n_out, bool fused);
-int launch_rows_f16(dnb_ctx* c, cudaStream_t st, const float* x, int ldx, const int32_t* row_token, int rows, int K,
-                    uint16_t* hi, uint16_t* lo, float* rowscale, const char* name);
-int launch_grouped_q4k_int(dnb_ctx* c, cudaStream_t st, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
-                           int n_in, int n_out, const UmmaMaps* maps, const float* rowscale, float* out_f32,
-                           float* const* row_dst = nullptr);
-
 // Grouped dequant matmul for few tokens per expert on mma.sync (grouped_mma.cu): fused = gate/up with silu(g) * u, else one
 // matrix; parts = fp16 numbers per activation (3: all bits of an fp32, 2: 22 bits).  fp32 rows in (row_token names a packed
 // row's input row, null: itself), fp32 packed rows out.  rows, nseg_est: token rows and active segments (an estimate where the
@@ -391,21 +379,20 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name);
 
-// tcgen05 grouped GEMM of prefill (grouped_umma.cu)
-int umma_make_maps(void* hi, void* lo, uint64_t rows, uint64_t cols, UmmaMaps* out);
-int launch_gather_split(dnb_ctx* c, cudaStream_t st, const float* x, int ldx, const int32_t* row_token, int rows, int e,
-                        uint16_t* hi, uint16_t* lo);
-int launch_grouped_umma(dnb_ctx* c, cudaStream_t st, bool fused, const SegDesc* seg, const int32_t* nseg_dev,
-                        int nseg_max, int n_in, int n_out, const UmmaMaps* maps, int nt_max, uint16_t* out_hi,
-                        uint16_t* out_lo, float* out_f32, float* const* row_dst = nullptr);
-// grouped_exact.cu: IQ3_XXS with exact bf16 weights and the block scales applied after the tensor-core sum
-int launch_grouped_exact(dnb_ctx* c, cudaStream_t st, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
-                         int n_in, int n_out, const UmmaMaps* maps, uint16_t* out_hi, uint16_t* out_lo, float* out_f32,
-                         float* const* row_dst = nullptr);
-// The tensor-core grouped GEMM of a block format: Q4_K -> launch_grouped_umma, IQ3_XXS -> launch_grouped_exact.
-int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev,
-                      int nseg_max, int n_in, int n_out, const UmmaMaps* maps, int nt_max, uint16_t* out_hi,
-                      uint16_t* out_lo, float* out_f32, float* const* row_dst = nullptr);
+// tcgen05 grouped GEMM of prefill (grouped_tc.cu): Q4_K and IQ3_XXS.  Its activations are operand rows: fp16 hi and lo parts,
+// tc_row_pitch(n_in) numbers each, one after the other.  launch_operand_rows makes them from fp32 rows; rows_dev (optional): the
+// device's count of rows, at most `rows`.
+size_t tc_row_pitch(int n_in);
+int tc_make_maps(void* op, uint64_t rows, int n_in, TcMaps* out);
+bool tc_handles(int type, int n_in, int n_out, bool fused);
+int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, int ldx, int rows, int n_in, uint16_t* op, const char* name,
+                        const int32_t* rows_dev = nullptr);
+// fused: seg[].wa / wb = gate / up, out = silu(g) * u; otherwise seg[].wa.  fp32 packed rows out, or where row_dst says (expert
+// parallel).  row_token: packed row -> operand row (gathered by TMA), null: itself.
+int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
+                      int n_out, const uint16_t* op, const TcMaps* maps, const int32_t* row_token, float* out, float* const* row_dst = nullptr);
+// The shared expert of a layer on `rows` fp32 rows (api.cu); op_ready: their operand rows are in the workspace already.
+int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, float* out);
 int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t* pos, const float* wts, int nt,
                    int k, int e, const float* sh, const float* shcoef, float* out);
 int launch_shared_coef(dnb_ctx* c, cudaStream_t st, const float* x, const float* row, int nt, int e, float* coef);

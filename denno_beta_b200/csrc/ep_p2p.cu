@@ -62,20 +62,10 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* p, uint32_t seq, int p
     return false;
 }
 
-// bf16 hi/lo split of a pair (hi rounded to nearest, lo = the exact remainder truncated):
-// the same arithmetic as the single-GPU gather pass, so the operands are the same bits.
-__device__ __forceinline__ void ep_split2(float a, float b, uint32_t& hi_pair, uint32_t& lo_pair) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    hi_pair = *reinterpret_cast<const uint32_t*>(&h);
-    const float al = a - __uint_as_float(hi_pair << 16), bl = b - __uint_as_float(hi_pair & 0xFFFF0000u);
-    lo_pair = __byte_perm(__float_as_uint(al), __float_as_uint(bl), 0x7632);
-}
-
 struct EpPeers {                 // kernel parameter: every rank's arena as seen from this GPU
     EpArena* arena[kEpMaxWorld];
     int32_t* recv_slot[kEpMaxWorld];
-    uint16_t* xg_hi[kEpMaxWorld];
-    uint16_t* xg_lo[kEpMaxWorld];
+    uint16_t* op[kEpMaxWorld];    // operand rows of the owner's gate/up GEMM
     float* h_slots[kEpMaxWorld];
 };
 
@@ -157,14 +147,14 @@ ep_offsets_kernel(const EpArena* mine, int ne, int n_local, int world, int me, u
     for (int e = tid; e < ne; e += blockDim.x) base[e] = tot[e] + mine_off[e];
 }
 
-// Rows i = t*k+slot, dealt to the CTAs round-robin: split x[t] to bf16 hi/lo and store it as row
-// base[expert] + j of the owner's operand buffers; the last CTA to finish raises the data flag at every
+// Rows i = t*k+slot, dealt to the CTAs round-robin: store token t's operand row (op_bytes, a multiple of 32) as row
+// base[expert] + j of the owner's operand array; the last CTA to finish raises the data flag at every
 // peer.  A CTA walks many rows and fences once at the end: the kernel runs beside the shared expert's
 // GEMM, which leaves room for about one of these CTAs per SM, and with a CTA (and a system-wide fence,
 // i.e. an NVLink round trip) per row the 4,096 rows of a chunk went out at a third of the link rate.
 __global__ void __launch_bounds__(256)
-ep_dispatch_kernel(const float* __restrict__ x, const int32_t* __restrict__ sels, const int32_t* __restrict__ send_row,
-                   const int32_t* __restrict__ base, int k, int e, int n_local, int world, int me, int rows_total,
+ep_dispatch_kernel(const uint16_t* __restrict__ op, size_t op_bytes, const int32_t* __restrict__ sels, const int32_t* __restrict__ send_row,
+                   const int32_t* __restrict__ base, int k, int n_local, int world, int me, int rows_total,
                    int n_rows, uint32_t seq, EpPeers peers, unsigned int* ticket, int* status) {
     const int tid = threadIdx.x;
     for (int i = blockIdx.x; i < n_rows; i += gridDim.x) {
@@ -176,20 +166,9 @@ ep_dispatch_kernel(const float* __restrict__ x, const int32_t* __restrict__ sels
             continue;
         }
         const int d = ex / n_local;
-        const float* xr = x + (size_t)(i / k) * e;
-        uint16_t* hi = peers.xg_hi[d] + r * e;
-        uint16_t* lo = peers.xg_lo[d] + r * e;
-        for (int c = tid * 8; c < e; c += 2048) {  // 16-byte stores: the peer write is NVLink traffic
-            const float4 v = *reinterpret_cast<const float4*>(xr + c);
-            const float4 u = *reinterpret_cast<const float4*>(xr + c + 4);
-            uint32_t h0, l0, h1, l1, h2, l2, h3, l3;
-            ep_split2(v.x, v.y, h0, l0);
-            ep_split2(v.z, v.w, h1, l1);
-            ep_split2(u.x, u.y, h2, l2);
-            ep_split2(u.z, u.w, h3, l3);
-            *reinterpret_cast<uint4*>(hi + c) = make_uint4(h0, h1, h2, h3);
-            *reinterpret_cast<uint4*>(lo + c) = make_uint4(l0, l1, l2, l3);
-        }
+        const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(op) + (size_t)(i / k) * op_bytes);
+        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(peers.op[d]) + r * op_bytes);
+        for (int c = tid; c < (int)(op_bytes / 16); c += 256) dst[c] = src[c];  // 16-byte stores: the peer write is NVLink traffic
         if (tid == 0) peers.recv_slot[d][r] = (me << 24) | i;  // who owns the token, and which (token, slot) row
     }
     __threadfence_system();
@@ -223,7 +202,7 @@ ep_build_kernel(EpArena* mine, const int32_t* __restrict__ recv_slot, int world,
     }
     __syncthreads();
     if (!ok_all) {  // nothing to compute: publish an empty table
-        if (tid == 0) *nseg = 0;
+        if (tid == 0) nseg[0] = nseg[1] = 0;
         return;
     }
     for (int x = tid; x < n_local; x += blockDim.x) {
@@ -236,7 +215,8 @@ ep_build_kernel(EpArena* mine, const int32_t* __restrict__ recv_slot, int world,
         int run = 0, n = 0;
         for (int x = 0; x < n_local; ++x) { first[x] = run; run += tot[x]; n += tot[x] > 0 ? 1 : 0; }
         n_rows = run;
-        *nseg = n;
+        nseg[0] = n;
+        nseg[1] = run;  // rows in all
     }
     __syncthreads();
     for (int x = tid; x < n_local; x += blockDim.x) {
@@ -279,18 +259,19 @@ struct EpState {
     bool loopback = false;         // every peer pointer is the own arena (time-out test): nothing to close
     uint8_t* arena = nullptr;      // this rank's exported allocation
     size_t arena_bytes = 0;
-    size_t off_slot = 0, off_hi = 0, off_lo = 0, off_h = 0;  // layout, identical on every rank
+    size_t off_slot = 0, off_op = 0, off_h = 0;  // layout, identical on every rank
     void* peer_base[kEpMaxWorld] = {nullptr};                // every rank's arena in this process's address space
     EpPeers peers;
     // local-only buffers
     int32_t* send_row = nullptr;
     int32_t* base = nullptr;       // [ne]: where this rank's rows of each expert start at the owner
     float** row_dst = nullptr;
-    uint16_t *act_hi = nullptr, *act_lo = nullptr;
+    float* act = nullptr;
+    uint16_t* op_act = nullptr;
     SegDesc *seg_gu = nullptr, *seg_dn = nullptr;
     int32_t* nseg = nullptr;
     unsigned int* ticket = nullptr;
-    UmmaMaps maps_x, maps_act;
+    TcMaps maps_x, maps_act;
 };
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -300,7 +281,7 @@ void ep_release(dnb_ctx* c) {
     if (!s) return;
     for (int r = 0; r < s->world; ++r)
         if (r != s->rank && s->peer_base[r] && !s->loopback) cudaIpcCloseMemHandle(s->peer_base[r]);
-    void* loc[] = {s->arena, s->send_row, s->base, s->row_dst, s->act_hi, s->act_lo, s->seg_gu, s->seg_dn, s->nseg, s->ticket};
+    void* loc[] = {s->arena, s->send_row, s->base, s->row_dst, s->act, s->op_act, s->seg_gu, s->seg_dn, s->nseg, s->ticket};
     for (void* p : loc)
         if (p) cudaFree(p);
     delete s;
@@ -336,26 +317,23 @@ extern "C" int dnb_ep_init(dnb_ctx* c, int rank, int world, int max_tokens, void
     s->rows_total = world * s->cap;
     const size_t rows_pad = (size_t)s->rows_total + 128;  // a tile that starts near the end stays inside
     s->off_slot = align_up(sizeof(EpArena), 256);
-    s->off_hi = align_up(s->off_slot + (size_t)s->rows_total * 4, 256);
-    s->off_lo = align_up(s->off_hi + rows_pad * M.e * 2, 256);
-    s->off_h = align_up(s->off_lo + rows_pad * M.e * 2, 256);
+    s->off_op = align_up(s->off_slot + (size_t)s->rows_total * 4, 256);
+    s->off_h = align_up(s->off_op + rows_pad * 4 * tc_row_pitch(M.e), 256);
     s->arena_bytes = align_up(s->off_h + (size_t)s->cap * M.e * 4, 256);
     DNB_CUDA(cudaMalloc((void**)&s->arena, s->arena_bytes));
     DNB_CUDA(cudaMemset(s->arena, 0, s->arena_bytes));
     DNB_CUDA(cudaMalloc((void**)&s->send_row, (size_t)s->cap * 4));
     DNB_CUDA(cudaMalloc((void**)&s->base, (size_t)M.ne * 4));
     DNB_CUDA(cudaMalloc((void**)&s->row_dst, (size_t)s->rows_total * sizeof(float*)));
-    DNB_CUDA(cudaMalloc((void**)&s->act_hi, rows_pad * M.ff * 2));
-    DNB_CUDA(cudaMalloc((void**)&s->act_lo, rows_pad * M.ff * 2));
-    DNB_CUDA(cudaMemset(s->act_hi, 0, rows_pad * M.ff * 2));
-    DNB_CUDA(cudaMemset(s->act_lo, 0, rows_pad * M.ff * 2));
+    DNB_CUDA(cudaMalloc((void**)&s->act, rows_pad * M.ff * sizeof(float)));
+    DNB_CUDA(cudaMalloc((void**)&s->op_act, rows_pad * 4 * tc_row_pitch(M.ff)));
+    DNB_CUDA(cudaMemset(s->op_act, 0, rows_pad * 4 * tc_row_pitch(M.ff)));
     DNB_CUDA(cudaMalloc((void**)&s->seg_gu, ((size_t)world * s->n_local + 1) * sizeof(SegDesc)));
     DNB_CUDA(cudaMalloc((void**)&s->seg_dn, ((size_t)world * s->n_local + 1) * sizeof(SegDesc)));
-    DNB_CUDA(cudaMalloc((void**)&s->nseg, 4));
+    DNB_CUDA(cudaMalloc((void**)&s->nseg, 8));
     DNB_CUDA(cudaMalloc((void**)&s->ticket, 4));
     DNB_CUDA(cudaMemset(s->ticket, 0, 4));
-    if (umma_make_maps(s->arena + s->off_hi, s->arena + s->off_lo, rows_pad, (uint64_t)M.e, &s->maps_x) != DNB_OK ||
-        umma_make_maps(s->act_hi, s->act_lo, rows_pad, (uint64_t)M.ff, &s->maps_act) != DNB_OK) {
+    if (tc_make_maps(s->arena + s->off_op, rows_pad, M.e, &s->maps_x) != DNB_OK || tc_make_maps(s->op_act, rows_pad, M.ff, &s->maps_act) != DNB_OK) {
         set_error("ep_init: tensor maps of the operand buffers could not be made");
         return DNB_DECLINED;
     }
@@ -382,8 +360,7 @@ extern "C" int dnb_ep_connect(dnb_ctx* c, const void* handles) {
         uint8_t* b = (uint8_t*)s->peer_base[r];
         s->peers.arena[r] = (EpArena*)b;
         s->peers.recv_slot[r] = (int32_t*)(b + s->off_slot);
-        s->peers.xg_hi[r] = (uint16_t*)(b + s->off_hi);
-        s->peers.xg_lo[r] = (uint16_t*)(b + s->off_lo);
+        s->peers.op[r] = (uint16_t*)(b + s->off_op);
         s->peers.h_slots[r] = (float*)(b + s->off_h);
     }
     s->connected = true;
@@ -402,8 +379,7 @@ extern "C" int dnb_ep_connect_loopback(dnb_ctx* c) {
         s->peer_base[r] = s->arena;
         s->peers.arena[r] = (EpArena*)b;
         s->peers.recv_slot[r] = (int32_t*)(b + s->off_slot);
-        s->peers.xg_hi[r] = (uint16_t*)(b + s->off_hi);
-        s->peers.xg_lo[r] = (uint16_t*)(b + s->off_lo);
+        s->peers.op[r] = (uint16_t*)(b + s->off_op);
         s->peers.h_slots[r] = (float*)(b + s->off_h);
     }
     s->connected = true;
@@ -446,6 +422,7 @@ extern "C" int dnb_ep_block_dev(dnb_ctx* c, int layer, const float* h_dev, int n
         ProfScope p_(c, st, "ep_offsets");
         ep_offsets_kernel<<<1, 1024, 0, st>>>((const EpArena*)s->arena, M.ne, s->n_local, s->world, s->rank, seq, s->base, c->status, c->flag_polls);
     }
+    if ((rc = launch_operand_rows(c, st, L.m[0].type, w.xn, M.e, nt, M.e, w.op_x, "operand_rows_x"))) return rc;
     // The dispatch stores run on the side stream, beside the shared expert of the own tokens
     // on the main one: peer stores over NVLink and a local GEMM do not compete for much.
     DNB_CUDA(cudaEventRecord(c->ev_fork, st));
@@ -454,7 +431,7 @@ extern "C" int dnb_ep_block_dev(dnb_ctx* c, int layer, const float* h_dev, int n
         ProfScope p_(c, c->side, "ep_dispatch");
         const int n_rows = nt * M.k;
         const int ctas = n_rows < 4 * c->sm_count ? n_rows : 4 * c->sm_count;
-        ep_dispatch_kernel<<<ctas, 256, 0, c->side>>>(w.xn, w.sels, s->send_row, s->base, M.k, M.e, s->n_local, s->world,
+        ep_dispatch_kernel<<<ctas, 256, 0, c->side>>>(w.op_x, 4 * tc_row_pitch(M.e), w.sels, s->send_row, s->base, M.k, s->n_local, s->world,
                                                      s->rank, s->rows_total, n_rows, seq, s->peers, s->ticket, c->status);
     }
     DNB_CUDA(cudaEventRecord(c->ev_join, c->side));
@@ -463,7 +440,7 @@ extern "C" int dnb_ep_block_dev(dnb_ctx* c, int layer, const float* h_dev, int n
     // 2. the shared expert of the own tokens while the rows travel
     const bool shared = L.has_shared();
     if (shared)
-        if ((rc = dnb_expert_rows_dev(c, layer, w.xn, nullptr, nt, 1, w.sh))) return rc;
+        if ((rc = shared_rows(c, layer, w.xn, nt, L.m[3].type == L.m[0].type, w.sh))) return rc;
     DNB_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
     // 3. the rows this rank owns: tables, the two grouped GEMMs, results stored at the token owners
     {
@@ -476,11 +453,12 @@ extern "C" int dnb_ep_block_dev(dnb_ctx* c, int layer, const float* h_dev, int n
     c->launches++;
     DNB_CUDA(cudaGetLastError());
     const int nseg_max = s->n_local;
-    if ((rc = launch_grouped_tc(c, st, L.m[0].type, true, s->seg_gu, s->nseg, nseg_max, M.e, M.ff, &s->maps_x, s->rows_total, s->act_hi,
-                                s->act_lo, nullptr)))
+    if ((rc = launch_grouped_tc(c, st, L.m[0].type, true, s->seg_gu, s->nseg, nseg_max, M.e, M.ff, (const uint16_t*)(s->arena + s->off_op), &s->maps_x,
+                                nullptr, s->act)))
         return rc;
-    if ((rc = launch_grouped_tc(c, st, L.m[0].type, false, s->seg_dn, s->nseg, nseg_max, M.ff, M.e, &s->maps_act, s->rows_total, nullptr,
-                                nullptr, nullptr, s->row_dst)))
+    if ((rc = launch_operand_rows(c, st, L.m[0].type, s->act, M.ff, s->rows_total, M.ff, s->op_act, "operand_rows_act", s->nseg + 1))) return rc;
+    if ((rc = launch_grouped_tc(c, st, L.m[0].type, false, s->seg_dn, s->nseg, nseg_max, M.ff, M.e, s->op_act, &s->maps_act, nullptr, nullptr,
+                                s->row_dst)))
         return rc;
     {
         ProfScope p_(c, st, "ep_signal_wait");

@@ -4,6 +4,7 @@
 #include "dnb_common.cuh"
 #include "formats.cuh"
 #include "tc_ptx.cuh"
+#include "operand_rows.cuh"
 
 namespace dnb {
 
@@ -54,9 +55,74 @@ prep_kernel(const float* __restrict__ h, const float* __restrict__ w, float eps,
     }
 }
 
+// The same row, also as the operand row of the tcgen05 experts (operand_rows.cuh; e a multiple of 256): the values are computed in
+// that layout's order, a 256-element block per warp, and read back once the row's largest element is known.
+template <int T>
+__global__ void __launch_bounds__(128)
+prep_operand_kernel(const float* __restrict__ h, const float* __restrict__ w, float eps, int e, float* __restrict__ out, uint16_t* __restrict__ x3,
+                    size_t x3_part, uint16_t* __restrict__ op) {
+    __shared__ float red[4];
+    __shared__ uint32_t redm[4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* xr = h + (size_t)blockIdx.x * e;
+    const float inv = rms_inv_128(xr, e, eps, red);
+    float* o = out + (size_t)blockIdx.x * e;
+    uint16_t* p3 = x3 ? x3 + (size_t)blockIdx.x * e : nullptr;
+    uint32_t mx = 0u;
+    for (int b = 256 * warp; b < e; b += 1024) {
+        int e0, e1;
+        tg::operand_elems<T>(b, lane, e0, e1);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = q ? e1 : e0;
+            float4 v = *reinterpret_cast<const float4*>(xr + i);
+            const float4 nw = *reinterpret_cast<const float4*>(w + i);
+            v.x = __fmul_rn(__fmul_rn(v.x, inv), nw.x);
+            v.y = __fmul_rn(__fmul_rn(v.y, inv), nw.y);
+            v.z = __fmul_rn(__fmul_rn(v.z, inv), nw.z);
+            v.w = __fmul_rn(__fmul_rn(v.w, inv), nw.w);
+            *reinterpret_cast<float4*>(o + i) = v;
+            mx = tg::operand_max(mx, v);
+            if (p3) {
+                ushort4 a, bb, c;
+                tcp::split3_bf16(v.x, a.x, bb.x, c.x);
+                tcp::split3_bf16(v.y, a.y, bb.y, c.y);
+                tcp::split3_bf16(v.z, a.z, bb.z, c.z);
+                tcp::split3_bf16(v.w, a.w, bb.w, c.w);
+                *reinterpret_cast<ushort4*>(p3 + i) = a;
+                *reinterpret_cast<ushort4*>(p3 + x3_part + i) = bb;
+                *reinterpret_cast<ushort4*>(p3 + 2 * x3_part + i) = c;
+            }
+        }
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) redm[warp] = mx;
+    __syncthreads();
+    const float up = tg::operand_scale(max(max(redm[0], redm[1]), max(redm[2], redm[3])));
+    const int pitch = tg::row_pitch(e);
+    uint16_t* hi = op + (size_t)(2 * blockIdx.x) * pitch;
+    for (int b = 256 * warp; b < e; b += 1024) {
+        int e0, e1;
+        tg::operand_elems<T>(b, lane, e0, e1);
+        tg::operand_block<T>(*reinterpret_cast<const float4*>(o + e0), *reinterpret_cast<const float4*>(o + e1), up, b, e, pitch, lane, hi);
+    }
+    if (warp == 3) tg::operand_tail<T>(up, e, pitch, lane, hi);
+}
+
 int launch_rmsnorm(dnb_ctx* c, cudaStream_t st, const float* h, const float* w, float eps, int nt, int e, float* out) {
     ProfScope prof_(c, st, "rmsnorm");
     prep_kernel<<<nt, 128, 0, st>>>(h, w, eps, e, out, nullptr, nullptr, nullptr, nullptr, nullptr, 0u, nullptr, 0);
+    c->launches++;
+    DNB_CUDA(cudaGetLastError());
+    return DNB_OK;
+}
+
+int launch_prep_operand(dnb_ctx* c, cudaStream_t st, int type, const float* h, const float* w, float eps, int nt, int e, float* out, uint16_t* x3,
+                        size_t x3_part, uint16_t* op) {
+    if (e % 256 || (type != T_Q4_K && type != T_IQ3_XXS)) return DNB_DECLINED;
+    ProfScope prof_(c, st, "prep_rmsnorm");
+    auto kern = type == T_Q4_K ? prep_operand_kernel<T_Q4_K> : prep_operand_kernel<T_IQ3_XXS>;
+    kern<<<nt, 128, 0, st>>>(h, w, eps, e, out, x3, x3_part, op);
     c->launches++;
     DNB_CUDA(cudaGetLastError());
     return DNB_OK;
