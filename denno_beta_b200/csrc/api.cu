@@ -93,7 +93,7 @@ static int ensure_ws(dnb_ctx* c, int nt) {
         if ((rc = dev_alloc(&w.op_act, rows_pad * 2 * tc_row_pitch(M.ff)))) return rc;
         DNB_CUDA(cudaMemset(w.op_x, 0, rows_pad * 4 * tc_row_pitch(M.e)));
         DNB_CUDA(cudaMemset(w.op_act, 0, rows_pad * 4 * tc_row_pitch(M.ff)));
-        w.maps_ok = tc_make_maps(w.op_x, rows_pad, M.e, &w.maps_x) == DNB_OK && tc_make_maps(w.op_act, rows_pad, M.ff, &w.maps_act) == DNB_OK;
+        w.op_ok = true;
     }
     if ((rc = router_tc_workspace(c, w, cap, M.ne, M.e))) return rc;
     w.pinned_cap = (size_t)cap * M.e * sizeof(float);
@@ -364,7 +364,7 @@ static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMi
 
 static bool umma_eligible(const dnb_ctx* c, const Layer& L, int nt) {
     const Model& M = c->model;
-    if (!c->use_umma || !c->ws.maps_ok) return false;
+    if (!c->use_umma || !c->ws.op_ok) return false;
     const int ty = tc_type(L, 0, 3);
     if (ty < 0 || nt < tc_min_tokens(c, ty) || !tc_handles(ty, M.e, M.ff, true) || !tc_handles(ty, M.ff, M.e, false)) return false;
     if (L.has_shared()) {  // the shared expert rides in the same launches as one more segment
@@ -390,9 +390,9 @@ static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const
     const int ty = L.m[0].type;
     if (!op_ready)
         if ((rc = launch_operand_rows(c, st, ty, x, M.e, nt, M.e, w.op_x, "operand_rows_x"))) return rc;
-    if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, w.op_x, &w.maps_x, w.row_token, w.act))) return rc;
+    if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, w.op_x, w.row_token, w.act))) return rc;
     if ((rc = launch_operand_rows(c, st, ty, w.act, M.ff, rows, M.ff, w.op_act, "operand_rows_act"))) return rc;
-    if ((rc = launch_grouped_tc(c, st, ty, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, w.op_act, &w.maps_act, nullptr, w.hrow))) return rc;
+    if ((rc = launch_grouped_tc(c, st, ty, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, w.op_act, nullptr, w.hrow))) return rc;
     if (shared && L.shared_gate_row)
         if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
     return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
@@ -503,12 +503,12 @@ int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, 
     int rc;
     if ((rc = launch_prep(c, st, x, nullptr, M.eps, rows, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev, L.m[4].dev, L.m[5].dev))) return rc;
     const int sff = L.m[3].n_out, ty = sff == M.ff ? tc_type(L, 3, 6) : -1;
-    if (c->use_umma && w.maps_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
+    if (c->use_umma && w.op_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
         if (!op_ready)
             if ((rc = launch_operand_rows(c, st, ty, x, M.e, rows, M.e, w.op_x, "operand_rows_x"))) return rc;
-        if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, &w.maps_x, nullptr, w.act))) return rc;
+        if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, nullptr, w.act))) return rc;
         if ((rc = launch_operand_rows(c, st, ty, w.act, M.ff, rows, M.ff, w.op_act, "operand_rows_act"))) return rc;
-        return launch_grouped_tc(c, st, ty, false, w.seg_sh_dn, w.one, 1, M.ff, M.e, w.op_act, &w.maps_act, nullptr, out);
+        return launch_grouped_tc(c, st, ty, false, w.seg_sh_dn, w.one, 1, M.ff, M.e, w.op_act, nullptr, out);
     }
     if ((rc = launch_seg_matmul(c, st, L.m[3].type, true, w.seg_sh_gu, nullptr, 1, M.e, sff, x, M.e, nullptr, w.sact, rows))) return rc;
     return launch_seg_matmul(c, st, L.m[5].type, false, w.seg_sh_dn, nullptr, 1, sff, M.e, w.sact, sff, nullptr, out, rows);
@@ -1182,7 +1182,7 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
     bool umma = c->use_umma && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(t.type, t.n_in, t.n_out, false);
     if (umma) {
         if ((rc = ensure_ws(c, (int)((row + M.k) / (M.k + 1))))) return rc;
-        umma = c->ws.maps_ok;
+        umma = c->ws.op_ok;
     }
     DNB_CUDA(cudaMemcpyAsync(dx, xs, row * t.n_in * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     DNB_CUDA(cudaMemcpyAsync(dsd, sd.data(), nseg * sizeof(SegDesc), cudaMemcpyHostToDevice, c->stream));
@@ -1191,7 +1191,7 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
         DNB_CUDA(cudaMemcpyAsync(dnseg, &nseg, sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
         uint16_t* op = in_e ? w.op_x : w.op_act;
         if ((rc = launch_operand_rows(c, c->stream, t.type, dx, t.n_in, (int)row, t.n_in, op, "operand_rows_gemm")) == DNB_OK)
-            rc = launch_grouped_tc(c, c->stream, t.type, false, dsd, dnseg, nseg, t.n_in, t.n_out, op, in_e ? &w.maps_x : &w.maps_act, nullptr,
+            rc = launch_grouped_tc(c, c->stream, t.type, false, dsd, dnseg, nseg, t.n_in, t.n_out, op, nullptr,
                                    dout);
     } else {
         rc = c->decode_fast ? launch_mm(c, c->stream, t.type, false, tc_type_ok(t.type) && row >= 64 ? 2 : 3, dsd, nullptr, nseg, nseg, (int)row,
@@ -1423,7 +1423,7 @@ int dnb_expert_rows_dev(dnb_ctx* c, int layer, const float* x_rows_dev, const in
     Workspace& w = c->ws;
     cudaStream_t st = c->stream;
     const bool tc_routed = !use_shared && tc_type(L, 0, 3) >= 0 && tc_handles(L.m[0].type, M.e, M.ff, true) && tc_handles(L.m[2].type, M.ff, M.e, false);
-    const bool umma = c->use_umma && w.maps_ok && rows >= 16;
+    const bool umma = c->use_umma && w.op_ok && rows >= 16;
     if (!use_shared) {
         // every row is one (token, slot): a "chunk" of `rows` tokens with one selected expert each and weight 1
         if (umma && tc_routed) return experts_dev_umma(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, 1, M.shard_count, 0);

@@ -88,10 +88,6 @@ struct Model {
     std::vector<Layer> layers;
 };
 
-struct alignas(64) TcMaps {  // four TMA tensor maps of an operand array (grouped_tc.cu), opaque here
-    unsigned char bytes[4 * 128];
-};
-
 struct Workspace {             // device buffers of the MoE pipeline, sized for nt_cap tokens
     int nt_cap = 0;
     float *xn = nullptr, *logits = nullptr, *wts = nullptr, *act = nullptr, *hrow = nullptr, *sact = nullptr,
@@ -102,8 +98,7 @@ struct Workspace {             // device buffers of the MoE pipeline, sized for 
     int32_t *sels = nullptr, *row_token = nullptr, *pos = nullptr, *nseg = nullptr, *counts = nullptr, *one = nullptr;
     SegDesc *seg_gu = nullptr, *seg_dn = nullptr, *seg_sh_gu = nullptr, *seg_sh_dn = nullptr;
     uint16_t *op_x = nullptr, *op_act = nullptr;  // operand rows of the tcgen05 grouped GEMM: n_embd and n_ff wide (grouped_tc.cu)
-    TcMaps maps_x, maps_act;
-    bool maps_ok = false;
+    bool op_ok = false;
     uint16_t* x3 = nullptr;    // [3][nt_cap + 128][e]: the chunk's rows as three bf16 parts (router_tc.cu)
     size_t x3_part = 0;        // elements between the parts
     float* rpart = nullptr;    // [K splits][nt][ne]: partial router sums
@@ -383,14 +378,13 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
 // tc_row_pitch(n_in) numbers each, one after the other.  launch_operand_rows makes them from fp32 rows; rows_dev (optional): the
 // device's count of rows, at most `rows`.
 size_t tc_row_pitch(int n_in);
-int tc_make_maps(void* op, uint64_t rows, int n_in, TcMaps* out);
 bool tc_handles(int type, int n_in, int n_out, bool fused);
 int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, int ldx, int rows, int n_in, uint16_t* op, const char* name,
                         const int32_t* rows_dev = nullptr);
 // fused: seg[].wa / wb = gate / up, out = silu(g) * u; otherwise seg[].wa.  fp32 packed rows out, or where row_dst says (expert
-// parallel).  row_token: packed row -> operand row (gathered by TMA), null: itself.
+// parallel).  row_token: packed row -> operand row, null: itself.
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
-                      int n_out, const uint16_t* op, const TcMaps* maps, const int32_t* row_token, float* out, float* const* row_dst = nullptr);
+                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst = nullptr);
 // The shared expert of a layer on `rows` fp32 rows (api.cu); op_ready: their operand rows are in the workspace already.
 int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, float* out);
 int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t* pos, const float* wts, int nt,

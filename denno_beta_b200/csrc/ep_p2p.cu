@@ -271,7 +271,6 @@ struct EpState {
     SegDesc *seg_gu = nullptr, *seg_dn = nullptr;
     int32_t* nseg = nullptr;
     unsigned int* ticket = nullptr;
-    TcMaps maps_x, maps_act;
 };
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -333,10 +332,6 @@ extern "C" int dnb_ep_init(dnb_ctx* c, int rank, int world, int max_tokens, void
     DNB_CUDA(cudaMalloc((void**)&s->nseg, 8));
     DNB_CUDA(cudaMalloc((void**)&s->ticket, 4));
     DNB_CUDA(cudaMemset(s->ticket, 0, 4));
-    if (tc_make_maps(s->arena + s->off_op, rows_pad, M.e, &s->maps_x) != DNB_OK || tc_make_maps(s->op_act, rows_pad, M.ff, &s->maps_act) != DNB_OK) {
-        set_error("ep_init: tensor maps of the operand buffers could not be made");
-        return DNB_DECLINED;
-    }
     DNB_CUDA(cudaDeviceSynchronize());
     cudaIpcMemHandle_t h;
     DNB_CUDA(cudaIpcGetMemHandle(&h, s->arena));
@@ -453,11 +448,11 @@ extern "C" int dnb_ep_block_dev(dnb_ctx* c, int layer, const float* h_dev, int n
     c->launches++;
     DNB_CUDA(cudaGetLastError());
     const int nseg_max = s->n_local;
-    if ((rc = launch_grouped_tc(c, st, L.m[0].type, true, s->seg_gu, s->nseg, nseg_max, M.e, M.ff, (const uint16_t*)(s->arena + s->off_op), &s->maps_x,
+    if ((rc = launch_grouped_tc(c, st, L.m[0].type, true, s->seg_gu, s->nseg, nseg_max, M.e, M.ff, (const uint16_t*)(s->arena + s->off_op),
                                 nullptr, s->act)))
         return rc;
     if ((rc = launch_operand_rows(c, st, L.m[0].type, s->act, M.ff, s->rows_total, M.ff, s->op_act, "operand_rows_act", s->nseg + 1))) return rc;
-    if ((rc = launch_grouped_tc(c, st, L.m[0].type, false, s->seg_dn, s->nseg, nseg_max, M.ff, M.e, s->op_act, &s->maps_act, nullptr, nullptr,
+    if ((rc = launch_grouped_tc(c, st, L.m[0].type, false, s->seg_dn, s->nseg, nseg_max, M.ff, M.e, s->op_act, nullptr, nullptr,
                                 s->row_dst)))
         return rc;
     {

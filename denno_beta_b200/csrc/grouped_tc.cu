@@ -11,19 +11,21 @@
 // more block of K = sub-blocks: A = -(dmin * m) * 2^10 as fp16 hi and lo, B = X.  An activation is fp16 hi + lo (22 bits) of the
 // row times a power of two that puts its largest element into [512, 1024).
 //
-// What bounds it: per 64-element stage of two 128-row tiles the 16 producer warps issue about 900 instructions (Q4_K; 1.7 per
-// weight) on four schedulers while the tensor core needs 8 MMAs of N = 2 x tokens; decoding and tensor work are of the same
-// size at 32 tokens per tile, so both have to run all the time.  Hence:
-//   * four producer groups of four warps, each on a stage of its own (a thread owns one row of both tiles: a 16-byte piece of
-//     its 128-byte swizzled row goes to a different bank group in each of eight neighbouring lanes), a ring of four or five
-//     stages: a group has the time of three other stages to wait for its bytes, decode and hand over.  (Two groups on a ring
-//     of two or three stages of the same size left the MMA warp without work for half the time.)
-//   * a thread's packed bytes for its next stage are requested before it waits for the ring;
-//   * hi and lo rows of a token are neighbours in memory, in the B tile (N = 2 x tokens) and in TMEM: a weight tile is read
-//     once per K step, and the epilogue adds the pair;
-//   * gate/up reads its tokens through TMA row gathers from the token-major rows: no packed copy of the activations.
-// Warps: 0-7 epilogue (thread = weight row, half of the token columns of both tiles; four TMEM buffers), 8-23 producers,
-// 24 TMA, 25 MMA.  Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
+// What bounds it: a 64-element stage of two 128-row tiles is about 900 warp instructions of decoding (Q4_K; 1.7 per weight) on
+// four schedulers and 8 MMAs of N = 2 x tokens, the same order of time at 32 tokens; everything else has to stay out of the
+// way of both.  Shared memory is the tightest: with A tiles in it (32 KB written and 32 KB read per stage, B read once per tile) a
+// stage took 840 cycles, all of them shared-memory bandwidth.  So A goes from the producers' registers to tensor memory
+// (tcgen05.st, thread = row = lane) and the MMA takes it from there.  One role per warp, each with a ring of its own in front:
+//   * two warps copy packed rows (a 256-element block of all 256 rows: 9 or 7 neighbouring lanes per row) into a raw ring.  (A
+//     thread that fetches its own row's bytes touches 32 cache lines per instruction; that alone took 0.5 us per stage.)
+//   * one warp copies the tokens' hi and lo rows into swizzled B tiles, gathered from the token-major rows: no packed copy of
+//     the activations.  (TMA row gathers took 80 cycles per four rows.)
+//   * four groups of four producer warps, group j decodes the j-th 64 elements of every block, a thread one row of both tiles;
+//     the block's scales go to a small ring.
+//   * the MMA warp; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
+//     once per K step.
+//   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
+// Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -39,21 +41,23 @@ using namespace tcp;
 constexpr int BK = 64;                  // K of a stage: one 128-byte swizzle row of fp16
 constexpr int TILE_M = 128;
 constexpr int NT = 32;                  // tokens of an item
-constexpr int A_TILE = TILE_M * BK * 2; // 16 KB
-constexpr int A_STAGE = 2 * A_TILE;
+constexpr int A_COLS = BK / 2;          // tensor-memory columns of an A tile (two fp16 each)
 constexpr int B_STAGE = 2 * NT * BK * 2;// hi and lo rows: 8 KB
-constexpr int NB = 4;                   // TMEM buffers
+constexpr int NB = 2;                   // accumulator buffers
 constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
-constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS;
-constexpr int W_TMA = EWARPS + PWARPS, W_MMA = W_TMA + 1;
+constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS, RWARPS = 2;
+constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + 1;
 constexpr int NTHREADS = (W_MMA + 1) * 32;
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
+constexpr int ASTAGES = 4, BSTAGES = 6;
+constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + ASTAGES * 2 * A_COLS;
+static_assert(TMEM_COLS == 512, "tensor memory");
+constexpr int SCL = 8;                  // ring of block scales: producers are at most NB + 2 blocks ahead of the epilogue
+constexpr int BDEPTH = 4;               // B stages on their way
 constexpr float kMinScale = 1024.f;     // the mins' A values are scaled up so that the low halves stay normal fp16 numbers
 
 template <int T> constexpr int kBB = T == T_Q4_K ? 144 : 98;
-
-struct Maps { CUtensorMap box[3]; CUtensorMap row; };  // boxes of 16, 32, 64 operand rows; single rows for the gathers
 
 struct Item {
     const uint8_t* pa;  // tile 0, first row
@@ -85,12 +89,11 @@ __device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int
 // Tokens of the B tile: the smallest of 8, 16, 32 that holds the item.
 __device__ __forceinline__ int tile_tokens(int m) { return m <= 8 ? 8 : m <= 16 ? 16 : 32; }
 
-// Stages of an item: K / 64, then those of the mins (Q4_K): with up to 32 sub-blocks one stage holds the hi parts in its first
-// 32 columns and the lo parts in the others (X is stored twice for it); with more, a stage of hi and one of lo per 64.
-__host__ __device__ __forceinline__ int min_stages(int type, int n_in) {
-    const int nsub = n_in / 32;
-    return type != T_Q4_K ? 0 : nsub <= 32 ? 1 : 2 * ((nsub + 63) / 64);
-}
+// An item's stages: for every eight blocks (or the rest) their 64-element stages, then those of the mins (Q4_K): with up to four
+// blocks one stage holds the hi parts of the up to 32 mins in its first 32 columns and the lo parts in the others (the operand row
+// has those sums twice), with more there is a stage of hi and one of lo.
+template <int T> __host__ __device__ __forceinline__ int min_stages(int blocks) { return T != T_Q4_K ? 0 : blocks <= 4 ? 1 : 2; }
+
 struct Args {
     const SegDesc* seg;
     const int32_t* nseg_dev;
@@ -108,151 +111,186 @@ __device__ __forceinline__ uint32_t chunk_off(int r, int c) {  // 16-byte column
 }
 
 // ---- producers: one row of both tiles per thread -------------------------------------------------------------------------
-template <int T> struct Raw;
+template <int T> struct Raw;  // what stage `c` (0..3) of a block needs of a row's packed bytes
 template <> struct Raw<T_Q4_K> {
+    static constexpr int UNITS = 9, RS = 144;
     uint4 h, a, b;
-    __device__ __forceinline__ void load(const uint8_t* row, int c) {
-        const uint8_t* p = row + (c >> 2) * 144;
-        h = __ldg(reinterpret_cast<const uint4*>(p));
-        a = __ldg(reinterpret_cast<const uint4*>(p + 16 + 32 * (c & 3)));
-        b = __ldg(reinterpret_cast<const uint4*>(p + 32 + 32 * (c & 3)));
+    __device__ __forceinline__ void load(const uint8_t* p, int c) {
+        h = *reinterpret_cast<const uint4*>(p);
+        a = *reinterpret_cast<const uint4*>(p + 16 + 32 * c);
+        b = *reinterpret_cast<const uint4*>(p + 32 + 32 * c);
     }
+    __device__ __forceinline__ float scale() const { return h2f((uint16_t)h.x); }
 };
 template <> struct Raw<T_IQ3_XXS> {  // 16 index bytes and two sub-block words from the aligned words around them
+    static constexpr int UNITS = 7, RS = 112;
     uint32_t i[5], x[3];
-    __device__ __forceinline__ void load(const uint8_t* row, int c) {
-        const uint8_t* p = row + (c >> 2) * 98 + 2 + 16 * (c & 3);
-        const uint32_t* wi = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
-        const uint32_t* wx = reinterpret_cast<const uint32_t*>((uintptr_t)(p + 64 - 8 * (c & 3)) & ~(uintptr_t)3);
+    uint32_t d, sh;
+    __device__ __forceinline__ void load(const uint8_t* p, int c) {  // p: the block, on an even address
+        sh = ((s32(p) + 2u) & 2u) * 8u;
+        d = ld16(p);
+        const uint32_t* wi = reinterpret_cast<const uint32_t*>(p + 2 + 16 * c - (sh >> 3));
+        const uint32_t* wx = reinterpret_cast<const uint32_t*>(p + 66 + 8 * c - (sh >> 3));
 #pragma unroll
-        for (int k = 0; k < 5; ++k) i[k] = __ldg(wi + k);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) x[k] = __ldg(wx + k);
+        for (int k = 0; k < 4; ++k) i[k] = wi[k];
+        i[4] = wi[sh ? 4 : 3];  // the word after is the row's only where the words are shifted
+        x[0] = wx[0];
+        x[1] = wx[1];
+        x[2] = wx[sh ? 2 : 1];
     }
+    __device__ __forceinline__ float scale() const { return 0.25f * h2f((uint16_t)d); }
 };
 
-__device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint8_t* tile, int r, uint32_t, uint32_t, const uint8_t*) {
-    const int t = c & 3, sh = 16 * (t & 1);
+// A tile's row of a stage goes to tensor memory in halves of 32 elements: 16 columns.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
+        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
+        "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D (+)= A * B with A in tensor memory.
+__device__ __forceinline__ void mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint32_t taddr, uint32_t, uint32_t) {
+    const int sh = 16 * (c & 1);
     const uint32_t a = R.h.y >> sh, cc = R.h.w >> sh;
-    const uint32_t sc = t < 2 ? (a & 0x3f3fu) : ((cc & 0x0f0fu) | ((a >> 2) & 0x3030u));  // kquant.rs:878-887
+    const uint32_t sc = c < 2 ? (a & 0x3f3fu) : ((cc & 0x0f0fu) | ((a >> 2) & 0x3030u));  // kquant.rs:878-887
     KScales s;
     s.s0 = h2sub(__byte_perm(sc, 0x64646464u, 0x4040u), 0x64006400u);
     s.s1 = h2sub(__byte_perm(sc, 0x64646464u, 0x4141u), 0x64006400u);
     s.k0 = h2mul(s.s0, 0xE400E400u);
     s.k1 = h2mul(s.s1, 0xD400D400u);
-    const uint32_t w[8] = {R.a.x, R.a.y, R.a.z, R.a.w, R.b.x, R.b.y, R.b.z, R.b.w};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        uint32_t p[4];
-        k_word<false>(w[i], 0u, s, p);
-        *reinterpret_cast<uint4*>(tile + chunk_off(r, i)) = make_uint4(p[0], p[1], p[2], p[3]);
+    for (int h = 0; h < 2; ++h) {
+        const uint4 q = h ? R.b : R.a;
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        uint32_t o[16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t p[4];
+            k_word<false>(w[i], 0u, s, p);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[4 * i + j] = p[j];
+        }
+        tmem_st16(taddr + 16 * h, o);
     }
 }
-__device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int c, uint8_t* tile, int r, uint32_t gl, uint32_t sl, const uint8_t* row) {
-    // index bytes and sub-block words of a block share their position within 4 bytes: 98 b + 2 + 16 c and 98 b + 66 + 8 c
-    const uint32_t sh = (uint32_t)((uintptr_t)(row + (c >> 2) * 98 + 2) & 2u) * 8u;
+__device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int, uint32_t taddr, uint32_t gl, uint32_t sl) {
 #pragma unroll
     for (int hb = 0; hb < 2; ++hb) {
-        const uint32_t aux = __funnelshift_r(R.x[hb], R.x[hb + 1], sh);
+        const uint32_t aux = __funnelshift_r(R.x[hb], R.x[hb + 1], R.sh);
         const uint32_t s2 = h2sub((((aux >> 27) & 0x1Eu) | 0x6401u) * 0x10001u, 0x64006400u);  // 2 s + 1 in both halves
+        uint32_t o[16];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint32_t iw = __funnelshift_r(R.i[2 * hb + (q >> 1)], R.i[2 * hb + (q >> 1) + 1], sh) >> (16 * (q & 1));
+            const uint32_t iw = __funnelshift_r(R.i[2 * hb + (q >> 1)], R.i[2 * hb + (q >> 1) + 1], R.sh) >> (16 * (q & 1));
             uint32_t p[4];
             iq3_pairs_h(gl, sl, iw, q == 0 ? aux << 6 : aux >> (7 * q - 6), p);
-            *reinterpret_cast<uint4*>(tile + chunk_off(r, 4 * hb + q)) =
-                make_uint4(h2mul(p[0], s2), h2mul(p[1], s2), h2mul(p[2], s2), h2mul(p[3], s2));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[4 * q + j] = h2mul(p[j], s2);
         }
+        tmem_st16(taddr + 16 * hb, o);
     }
 }
-// Stage u of the mins of one Q4_K row.
-__device__ __forceinline__ void mins_stage(const uint8_t* row, int nsub, int u, uint8_t* tile, int r) {
-    const bool both = nsub <= 32;
-    const int base = both ? 0 : 64 * (u >> 1);
+// Stage u of the mins of one Q4_K row; raw: the row's headers of `blocks` blocks, 16 bytes each.
+__device__ __forceinline__ void mins_stage(const uint8_t* raw, int blocks, int u, uint32_t taddr) {
+    const bool both = blocks <= 4;
 #pragma unroll 1
-    for (int c = 0; c < 8; ++c) {  // eight sub-blocks = one 256-element block per 16-byte column
-        const int part = both ? c >> 2 : u & 1, blk = base / 8 + (both ? c & 3 : c);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (blk * 8 < nsub) {
-            const uint4 h = __ldg(reinterpret_cast<const uint4*>(row + blk * 144));
-            const float dm = -kMinScale * h2f((uint16_t)(h.x >> 16));
-            uint32_t o[4];
+    for (int half = 0; half < 2; ++half) {
+        uint32_t o[16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {  // the eight sub-blocks of a block: four columns
+            const int part = both ? half : u, blk = both ? c : 4 * half + c;
+            const bool live = blk < blocks;
+            const uint4 h = *reinterpret_cast<const uint4*>(raw + 16 * (live ? blk : 0));
+            const float dm = live ? -kMinScale * h2f((uint16_t)(h.x >> 16)) : 0.f;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {  // sub-blocks 2 k, 2 k + 1
                 const int sh = 16 * (k & 1);
                 const uint32_t b = h.z >> sh, d = h.w >> sh;
                 const uint32_t mn = k < 2 ? (b & 0x3f3fu) : (((d >> 4) & 0x0f0fu) | ((b >> 2) & 0x3030u));
-                const float f0 = dm * (float)(mn & 0xffu), f1 = dm * (float)(mn >> 8);
+                const float f0 = dm * (float)(mn & 0xffu), f1 = dm * (float)((mn >> 8) & 0xffu);
                 const __half2 hi = __floats2half2_rn(f0, f1);
                 const float2 hf = __half22float2(hi);
                 const __half2 lo = __floats2half2_rn(f0 - hf.x, f1 - hf.y);
-                o[k] = part ? *reinterpret_cast<const uint32_t*>(&lo) : *reinterpret_cast<const uint32_t*>(&hi);
+                o[4 * c + k] = part ? *reinterpret_cast<const uint32_t*>(&lo) : *reinterpret_cast<const uint32_t*>(&hi);
             }
-            v = make_uint4(o[0], o[1], o[2], o[3]);
         }
-        *reinterpret_cast<uint4*>(tile + chunk_off(r, c)) = v;
+        tmem_st16(taddr + 16 * half, o);
     }
 }
 
 __device__ __forceinline__ float swiglu_fast(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
-__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, int x, int y0, int y1, int y2, int y3, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(
-            s32(dst)),
-        "l"(map), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(s32(bar))
-        : "memory");
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {  // an arrival once this thread's copies so far are complete
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(s32(bar)) : "memory");
 }
+template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Shared memory: [barriers, segment table, items][B stages that fit below the tables][IQ3_XXS tables at a 32 KB boundary][A stages][other B stages]
+// Shared memory: [barriers, segment table, items][block scales][B stages that fit below][IQ3_XXS tables at a 32 KB boundary]
+// [rest of the B ring][raw ring]
 template <int T> struct Layout {
-    static constexpr int STAGES = T == T_Q4_K ? 5 : 4;
-    static constexpr int LOW_B = T == T_Q4_K ? STAGES : 3;   // B stages in front
-    static constexpr int HEAD = ((2 * STAGES + 2 * NB) * 8 + 16 + (kMaxSeg + 1) * 4 + kLocalItems * (int)sizeof(Item) + 1023) / 1024 * 1024;
+    static constexpr int RSTAGES = 3;
+    static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
+    static constexpr int LOW_B = T == T_Q4_K ? BSTAGES : 2;
+    static constexpr int BARS = 3 * ASTAGES + 2 * (BSTAGES + RSTAGES + NB);
+    static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
+    static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
+    static constexpr int TAIL = (BSTAGES - LOW_B) * B_STAGE + RSTAGES * RAW_STAGE;
 };
 
 template <int T, bool PAIR>  // PAIR: both tiles from seg.wa (256 rows, fp32 results); else gate and up rows, silu(g) * u
-__global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A, const __grid_constant__ Maps maps) {
+__global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     using L = Layout<T>;
-    constexpr int STAGES = L::STAGES;
+    using R = Raw<T>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (s32(smem_raw) & 1023u)) & 1023u);
-    uint64_t* full = reinterpret_cast<uint64_t*>(base);
-    uint64_t* empty = full + STAGES;
-    uint64_t* tfull = empty + STAGES;
+    uint64_t* afull = reinterpret_cast<uint64_t*>(base);
+    uint64_t* aempty = afull + ASTAGES;
+    uint64_t* bfull = aempty + 2 * ASTAGES;  // (two per slot, see the producers)
+    uint64_t* bempty = bfull + BSTAGES;
+    uint64_t* rfull = bempty + BSTAGES;
+    uint64_t* rempty = rfull + L::RSTAGES;
+    uint64_t* tfull = rempty + L::RSTAGES;
     uint64_t* tfree = tfull + NB;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfree + NB);
     int* pre = reinterpret_cast<int*>(tmem_slot + 4);  // [nseg + 1] first token tile of a segment
     Item* itab = reinterpret_cast<Item*>((reinterpret_cast<uintptr_t>(pre + kMaxSeg + 1) + 7) & ~(uintptr_t)7);
-    uint8_t* b_low = base + L::HEAD;
+    float* scl = reinterpret_cast<float*>(base + L::HEAD);  // [SCL][2][128]
+    uint8_t* b_low = base + L::LOW;
     uint8_t* p = b_low + L::LOW_B * B_STAGE;
     uint8_t* book = p;
     if constexpr (T == T_IQ3_XXS) {
         book += (kMmBookAlign - (s32(p) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
         p = book + sizeof(MmCodebook);
     }
-    uint8_t* a_base = p;
-    uint8_t* b_high = a_base + STAGES * A_STAGE;
-    if ((uint32_t)(b_high + (STAGES - L::LOW_B) * B_STAGE - smem_raw) > A.smem) {  // only if shared memory started elsewhere
+    uint8_t* b_high = p;
+    uint8_t* raw_base = b_high + (BSTAGES - L::LOW_B) * B_STAGE;
+    if ((uint32_t)(b_high + L::TAIL - smem_raw) > A.smem) {  // only if shared memory started elsewhere
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
     }
     auto b_tile = [&](int st) { return st < L::LOW_B ? b_low + st * B_STAGE : b_high + (st - L::LOW_B) * B_STAGE; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nchunks = A.n_in / BK, nmin = min_stages(T, A.n_in), nch = nchunks + nmin, nblk = A.n_in / 256, nsub = A.n_in / 32;
+    const int nblk = A.n_in / 256;
     const int row_tiles = A.n_out / (PAIR ? 2 * TILE_M : TILE_M);
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) {
-            mb_init(&full[i], 5);   // the four warps of a producer group + the TMA thread's expect_tx
-            mb_init(&empty[i], 1);  // one tcgen05.commit
-        }
-        for (int i = 0; i < NB; ++i) {
-            mb_init(&tfull[i], 1);
-            mb_init(&tfree[i], EWARPS);
-        }
+        for (int i = 0; i < ASTAGES; ++i) mb_init(&afull[i], 4);                                     // a producer group
+        for (int i = 0; i < 2 * ASTAGES; ++i) mb_init(&aempty[i], 1);                                // a commit
+        for (int i = 0; i < BSTAGES; ++i) { mb_init(&bfull[i], 1); mb_init(&bempty[i], 1); }       // the B warp; a commit
+        for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
+        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
         fence_mbarrier_init();
     }
     if constexpr (T == T_IQ3_XXS) {
@@ -261,7 +299,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A, c
         cp_async_commit();
         cp_async_wait_all();
     }
-    if (warp == W_MMA) tmem_alloc<NB * BUF_COLS>(tmem_slot);
+    if (warp == W_MMA) tmem_alloc<TMEM_COLS>(tmem_slot);
     pdl_wait();
     pdl_launch_dependents();
     const int nseg = min(*A.nseg_dev, A.nseg_max);
@@ -301,18 +339,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A, c
         const int quad = warp & 3, hsel = warp >> 2;
         const int r = quad * 32 + lane;
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
-        int buf = 0;
+        int buf = 0, sc = 0;
         uint32_t pb = 0;
-        uint16_t dn[2] = {0, 0};
-        auto fetch_d = [&](const Item& it, int blk) {  // this row's block scale in both tiles
-            dn[0] = __ldg(reinterpret_cast<const uint16_t*>(it.pa + (size_t)r * A.rb + blk * kBB<T>));
-            dn[1] = __ldg(reinterpret_cast<const uint16_t*>(it.pb + (size_t)r * A.rb + blk * kBB<T>));
-        };
-        Item nx = my_items > 0 ? item(0) : Item{};
-        if (my_items > 0) fetch_d(nx, 0);
         for (int k = 0; k < my_items && ok; ++k) {
-            const Item it = nx;
-            if (k + 1 < my_items) nx = item(k + 1);
+            const Item it = item(k);
             const int nte = tile_tokens(it.m), half = nte >> 1;
             float rs = 0.f;  // lane j: what undoes the scaling of token j of this warp's half
             if (lane < half) {
@@ -325,161 +355,270 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A, c
             for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[mt][j] = 0.f;
-            for (int blk = 0; blk < nblk + (nmin ? 1 : 0); ++blk) {
-                float s[2] = {1.f / kMinScale, 1.f / kMinScale};
-                if (blk < nblk) {
-                    constexpr float f = T == T_IQ3_XXS ? 0.25f : 1.f;
-                    s[0] = f * h2f(dn[0]);
-                    s[1] = f * h2f(dn[1]);
-                    if (blk + 1 < nblk) fetch_d(it, blk + 1);
-                    else if (k + 1 < my_items) fetch_d(nx, 0);
-                }
-                ok = warp_all(mb_wait(&tfull[buf], pb, A.status, 3));
-                if (!ok) break;
-                tc_fence_after();
-#pragma unroll
-                for (int mt = 0; mt < 2; ++mt)
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0);
+                for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0); ++b) {  // the last one: the mins
+                    ok = warp_all(mb_wait(&tfull[buf], pb, A.status, 3));
+                    if (!ok) break;
+                    tc_fence_after();
+                    float s[2] = {1.f / kMinScale, 1.f / kMinScale};
+                    if (b < bn) {
+                        s[0] = scl[(sc * 2) * TILE_M + r];
+                        s[1] = scl[(sc * 2 + 1) * TILE_M + r];
+                        sc = (sc + 1) & (SCL - 1);
+                    }
+                    const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * nte);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {  // eight tokens each; 32-token tiles have two per warp
                         if (h == 0 || nte == 32) {
-                            uint32_t v[16];
-                            tmem_ld16(tlane + (uint32_t)(buf * BUF_COLS + mt * 2 * NT + hsel * nte + 16 * h), v);
+                            uint32_t v[2][16];
+                            tmem_ld16(col + 16 * h, v[0]);
+                            tmem_ld16(col + 2 * NT + 16 * h, v[1]);
                             tmem_ld_wait();
+                            if (h == 1 || nte != 32) {  // read: hand the buffer back before the arithmetic
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mb_arrive(&tfree[buf]);
+                            }
 #pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                acc[mt][8 * h + j] = fmaf(s[mt], __uint_as_float(v[2 * j]) + __uint_as_float(v[2 * j + 1]), acc[mt][8 * h + j]);
+                            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                                for (int j = 0; j < 8; ++j)
+                                    acc[mt][8 * h + j] =
+                                        fmaf(s[mt], __uint_as_float(v[mt][2 * j]) + __uint_as_float(v[mt][2 * j + 1]), acc[mt][8 * h + j]);
                         }
                     }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mb_arrive(&tfree[buf]);
-                if (++buf == NB) { buf = 0; pb ^= 1u; }
+                    if (++buf == NB) { buf = 0; pb ^= 1u; }
+                }
             }
             if (!ok) break;
+            const int t0 = hsel * half, cnt = min(half, it.m - t0);
+            float* o = A.out + (size_t)(it.prow + t0) * A.n_out + it.r0 + r;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const float f = __shfl_sync(0xffffffffu, rs, j);
-                const int t = hsel * half + j;
-                if (j < half && t < it.m) {
+                if (j < cnt) {
                     const float a0 = acc[0][j] * f, a1 = acc[1][j] * f;
                     if constexpr (!PAIR) {
-                        A.out[(size_t)(it.prow + t) * A.n_out + it.r0 + r] = swiglu_fast(a0, a1);
+                        *o = swiglu_fast(a0, a1);
                     } else {
-                        // expert parallel: the owner's (token, slot) row
-                        float* o = A.row_dst ? A.row_dst[it.prow + t] + it.r0 + r : A.out + (size_t)(it.prow + t) * A.n_out + it.r0 + r;
-                        o[0] = a0;
-                        o[TILE_M] = a1;
+                        float* d = A.row_dst ? A.row_dst[it.prow + t0 + j] + it.r0 + r : o;  // expert parallel: the owner's (token, slot) row
+                        d[0] = a0;
+                        d[TILE_M] = a1;
+                    }
+                    o += A.n_out;
+                }
+            }
+        }
+    } else if (warp < W_RAW) {
+        // ---------------- producers ----------------
+        const int pw = warp - EWARPS, grp = pw >> 2, r = (pw & 3) * 32 + lane;
+        const uint32_t tlane = tmem_base + A_COL0 + ((uint32_t)((pw & 3) * 32) << 16);
+        const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
+        int rst = 0, sc = 0;
+        uint32_t rph = 0u;
+        // A group's stages are up to six apart and the groups may be a block apart from one another: with one barrier per slot a
+        // group could look at a slot whose last but one stage is still in use and take its parity for the last one's.  Stage q
+        // therefore commits to barrier q mod 2 * ASTAGES, and its slot's next user waits for exactly that commit.
+        int q = grp;               // this group's next stage, mod 2 * ASTAGES
+        uint32_t turn = 0u;        // parity of the turn of that count
+        auto advance = [&](int n) {
+            q += n;
+            while (q >= 2 * ASTAGES) { q -= 2 * ASTAGES; turn ^= 1u; }
+        };
+        auto slot = [&]() { return q < ASTAGES ? q : q - ASTAGES; };
+        auto wait_slot = [&]() {
+            return warp_all(q < ASTAGES ? mb_wait(&aempty[q + ASTAGES], turn ^ 1u, A.status, 2) : mb_wait(&aempty[q - ASTAGES], turn, A.status, 2));
+        };
+        for (int k = 0; k < my_items && ok; ++k) {
+            const Item it = item(k);
+            uint32_t oa = 0, ob = 0;  // where the two rows' blocks start within 16 bytes
+            if constexpr (T == T_IQ3_XXS) {
+                oa = (uint32_t)(uintptr_t)it.pa + (uint32_t)r * A.rb;
+                ob = (uint32_t)(uintptr_t)it.pb + (uint32_t)r * A.rb;
+            }
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0);
+                for (int b = 0; b < bn; ++b) {
+                    ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
+                    if (!ok) break;
+                    const uint8_t* raw = raw_base + rst * L::RAW_STAGE + r * R::RS;
+                    R ra, rb;
+                    ra.load(raw + (oa & 15u), grp);
+                    rb.load(raw + L::RAW_TILE + (ob & 15u), grp);
+                    if constexpr (T == T_IQ3_XXS) { oa += kBB<T>; ob += kBB<T>; }
+                    __syncwarp();
+                    if (lane == 0) mb_arrive(&rempty[rst]);
+                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
+                    if (grp == 0) {
+                        scl[(sc * 2) * TILE_M + r] = ra.scale();
+                        scl[(sc * 2 + 1) * TILE_M + r] = rb.scale();
+                        sc = (sc + 1) & (SCL - 1);
+                    }
+                    ok = wait_slot();
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t ta = tlane + slot() * (2 * A_COLS);
+                    decode_stage(ra, grp, ta, gl, sl);
+                    decode_stage(rb, grp, ta + A_COLS, gl, sl);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mb_arrive(&afull[slot()]);
+                    advance(4);
+                }
+                if (!ok) break;
+                if constexpr (T == T_Q4_K) {  // the mins: group u builds stage u; then every group is `nm` stages on
+                    const int nm = min_stages<T>(bn);
+                    ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
+                    if (!ok) break;
+                    if (grp < nm) {
+                        ok = wait_slot();
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t ta = tlane + slot() * (2 * A_COLS);
+                        const uint8_t* raw = raw_base + rst * L::RAW_STAGE + r * R::RS;
+                        mins_stage(raw, bn, grp, ta);
+                        mins_stage(raw + L::RAW_TILE, bn, grp, ta + A_COLS);
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mb_arrive(&afull[slot()]);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mb_arrive(&rempty[rst]);
+                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
+                    advance(nm);
+                }
+            }
+        }
+    } else if (warp < W_B) {
+        // ---------------- raw rows: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
+        const int rw = warp - W_RAW, c16 = (lane & 7) * 16;
+        int rst = 0;
+        uint32_t rph = 1u;
+        for (int k = 0; k < my_items && ok; ++k) {
+            const Item it = item(k);
+            const uint8_t* tile0 = (rw ? it.pb : it.pa);  // a warp per tile
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0);
+                for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0); ++b) {
+                    ok = warp_all(mb_wait(&rempty[rst], rph, A.status, 8));
+                    if (!ok) break;
+                    uint8_t* dst = raw_base + rst * L::RAW_STAGE + rw * L::RAW_TILE;
+                    if (b < bn) {
+                        const uint8_t* src = tile0 + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
+                        uint8_t* d = dst + (lane >> 3) * R::RS + c16;
+                        const uint32_t step = 4u * A.rb;
+#pragma unroll 8
+                        for (int i = 0; i < TILE_M / 4; ++i, src += step) {
+                            if constexpr (T == T_Q4_K) {
+                                cp_async16(d + i * 4 * R::RS, src + c16);
+                            } else {
+                                const uint8_t* s16 = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
+                                if (c16 < R::UNITS * 16) cp_async16(d + i * 4 * R::RS, s16 + c16);
+                            }
+                        }
+                        if constexpr (T == T_Q4_K) {
+                            const uint8_t* s9 = tile0 + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
+#pragma unroll
+                            for (int i = 0; i < TILE_M / 32; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
+                        }
+                    } else if constexpr (T == T_Q4_K) {  // the headers of the last bn blocks: lane = block lane % 8
+                        const uint8_t* src = tile0 + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + (lane & 7)) * kBB<T>;
+                        if ((lane & 7) < bn) {
+#pragma unroll 8
+                            for (int i = 0; i < TILE_M / 4; ++i) cp_async16(dst + ((lane >> 3) + 4 * i) * R::RS + c16, src + (size_t)(4 * i) * A.rb);
+                        }
+                    }
+                    cp_async_arrive(&rfull[rst]);
+                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
+                }
+            }
+        }
+        cp_async_wait_all();
+    } else if (warp == W_B) {
+        // ---------------- B tiles: rows 2 t, 2 t + 1 = hi and lo of token t; lane = unit lane % 8 of row lane / 8 (+ 4 per step) ----------------
+        int sb = 0, sd = 0, flying = 0;  // next slot, oldest slot on its way, how many are
+        uint32_t bph = 1u;
+        auto land = [&]() {  // the oldest stage on its way is complete: visible to the tensor core
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mb_arrive(&bfull[sd]);
+            if (++sd == BSTAGES) sd = 0;
+            --flying;
+        };
+        const uint16_t* opl = A.op + 8 * (lane & 7);
+        for (int k = 0; k < my_items && ok; ++k) {
+            const Item it = item(k);
+            const int steps = tile_tokens(it.m) / 2;  // 4 rows each
+            uint32_t row[16];  // operand array rows of this lane's B rows
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int br = 4 * i + (lane >> 3), pr = it.prow + min(br >> 1, it.m - 1);
+                row[i] = i < steps ? 2u * (uint32_t)(A.row_token ? A.row_token[pr] : pr) + (br & 1) : 0u;
+            }
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0), nst = 4 * bn + min_stages<T>(bn);
+                for (int c = 0; c < nst; ++c) {
+                    ok = warp_all(mb_wait(&bempty[sb], bph, A.status, 4));
+                    if (!ok) break;
+                    const int col = c < 4 * bn ? b0 * 256 + c * BK : A.n_in + 8 * b0;  // the mins read the sums behind the row
+                    uint8_t* d = b_tile(sb);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (i < steps) cp_async16(d + chunk_off(4 * i + (lane >> 3), lane & 7), opl + (size_t)row[i] * pitch + col);
+                    cp_async_commit();
+                    if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
+                    if (++flying > BDEPTH) {
+                        cp_async_wait_group<BDEPTH>();
+                        land();
                     }
                 }
             }
         }
-    } else if (warp < W_TMA) {
-        // ---------------- producers ----------------
-        const int pw = warp - EWARPS, grp = pw >> 2, r = (pw & 3) * 32 + lane;
-        const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
-        int k = 0, c = grp, st = grp;  // stage number grp, grp + GROUPS, ... -> (item, stage of the item, ring slot)
-        uint32_t ph = 1u;              // parity of the empty barrier to wait for; the first turn of the ring finds it free
-        while (c >= nch && k < my_items) { c -= nch; ++k; }
-        const uint8_t *pa = nullptr, *pb = nullptr;
-        Raw<T> ra, rb;
-        auto aim = [&]() {
-            const Item it = item(k);
-            pa = it.pa + (size_t)r * A.rb;
-            pb = it.pb + (size_t)r * A.rb;
-        };
-        auto fetch = [&]() {
-            if (k < my_items && c < nchunks) {
-                ra.load(pa, c);
-                rb.load(pb, c);
-            }
-        };
-        if (k < my_items) aim();
-        fetch();
-        while (k < my_items) {
-            ok = warp_all(mb_wait(&empty[st], ph, A.status, 2));
-            if (!ok) break;
-            uint8_t* tile = a_base + st * A_STAGE;
-            if (c < nchunks) {
-                decode_stage(ra, c, tile, r, gl, sl, pa);
-                decode_stage(rb, c, tile + A_TILE, r, gl, sl, pb);
-            } else {
-                mins_stage(pa, nsub, c - nchunks, tile, r);
-                mins_stage(pb, nsub, c - nchunks, tile + A_TILE, r);
-            }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) mb_arrive(&full[st]);
-            c += GROUPS;
-            if (c >= nch) {
-                do { c -= nch; ++k; } while (c >= nch && k < my_items);
-                if (k < my_items) aim();
-            }
-            st += GROUPS;
-            if (st >= STAGES) { st -= STAGES; ph ^= 1u; }
-            fetch();
-        }
-    } else if (warp == W_TMA) {
-        // ---------------- TMA: hi and lo rows of the tokens ----------------
-        int st = 0;
-        uint32_t ph = 1u;
-        for (int k = 0; k < my_items && ok; ++k) {
-            const Item it = item(k);
-            const int nte = tile_tokens(it.m), sel = nte == 8 ? 0 : nte == 16 ? 1 : 2;
-            int y0 = 0, y1 = 0;  // gathers: lane l brings tokens 2 l and 2 l + 1
-            if (A.row_token && lane < nte / 2) {
-                y0 = 2 * A.row_token[it.prow + min(2 * lane, it.m - 1)];
-                y1 = 2 * A.row_token[it.prow + min(2 * lane + 1, it.m - 1)];
-            }
-            for (int c = 0; c < nch; ++c) {
-                ok = warp_all(mb_wait(&empty[st], ph, A.status, 4));
-                if (!ok) break;
-                const int u = c - nchunks, col = c < nchunks ? c * BK : A.n_in + 64 * (u >> 1);
-                if (lane == 0) mb_expect_tx(&full[st], (uint32_t)(2 * nte * BK * 2));
-                __syncwarp();
-                if (A.row_token) {
-                    if (lane < nte / 2) tma_gather4(b_tile(st) + lane * 512, &maps.row, col, y0, y0 + 1, y1, y1 + 1, &full[st]);
-                } else if (elect_one()) {
-                    tma_load_2d(b_tile(st), &maps.box[sel], col, 2 * it.prow, &full[st]);
-                }
-                __syncwarp();
-                if (++st == STAGES) { st = 0; ph ^= 1u; }
-            }
-        }
+        cp_async_wait_all();
+        while (flying > 0) land();
     } else {
         // ---------------- MMA issue ----------------
-        int st = 0, buf = 0;
-        uint32_t ph = 0u, pf = 1u;
+        int sa = 0, se = 0, sb = 0, buf = 0;
+        uint32_t aph = 0u, bph = 0u, pf = 1u;
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             const int nte = tile_tokens(it.m);
             const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
-            for (int c = 0; c < nch; ++c) {
-                ok = warp_all(mb_wait(&full[st], ph, A.status, 5));
-                if (!ok) break;
-                const bool first = c < nchunks ? (c & 3) == 0 : c == nchunks;
-                const bool last = c < nchunks ? (c & 3) == 3 : c == nch - 1;
-                if (first) ok = warp_all(mb_wait(&tfree[buf], pf, A.status, 6));
-                if (!ok) break;
-                tc_fence_after();
-                if (elect_one()) {
-                    const uint32_t a_lo = desc_lo(s32(a_base + st * A_STAGE)), b_lo = desc_lo(s32(b_tile(st)));
-                    const uint32_t d0 = tmem_base + (uint32_t)(buf * BUF_COLS);
-                    // a stage of mins uses the K steps that hold sub-blocks (hi and lo halves side by side when both fit)
-                    const int u = c - nchunks;
-                    const int live = c < nchunks ? 4 : nsub <= 32 ? (nsub + 15) / 16 : min(4, (nsub - 64 * (u >> 1) + 15) / 16);
-                    uint32_t acc = first ? 0u : 1u;
-                    for (int ks = 0; ks < 4; ++ks) {
-                        if (c >= nchunks && (nsub <= 32 ? (ks & 1) >= live : ks >= live)) continue;
-                        mma_bf16(d0, desc_of(a_lo + 2u * ks), desc_of(b_lo + 2u * ks), idesc, acc);
-                        mma_bf16(d0 + 2 * NT, desc_of(a_lo + (A_TILE >> 4) + 2u * ks), desc_of(b_lo + 2u * ks), idesc, acc);
-                        acc = 1u;
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0), nst = 4 * bn + min_stages<T>(bn);
+                for (int c = 0; c < nst; ++c) {
+                    const bool mins = c >= 4 * bn, first = mins ? c == 4 * bn : (c & 3) == 0, last = mins ? c == nst - 1 : (c & 3) == 3;
+                    if (first) ok = warp_all(mb_wait(&tfree[buf], pf, A.status, 6));
+                    if (ok) ok = warp_all(mb_wait(&bfull[sb], bph, A.status, 5));
+                    if (ok) ok = warp_all(mb_wait(&afull[sa], aph, A.status, 5));
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(sa * 2 * A_COLS), b_lo = desc_lo(s32(b_tile(sb)));
+                        const uint32_t d0 = tmem_base + (uint32_t)(buf * BUF_COLS);
+                        // a stage of mins: the K steps that hold sub-blocks (hi and lo halves side by side when both fit)
+                        const int live = !mins ? 4 : (bn * 8 + 15) / 16;
+                        uint32_t acc = first ? 0u : 1u;
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks) {
+                            if (mins && (bn <= 4 ? (ks & 1) >= live : ks >= live)) continue;
+                            mma_f16_ta(d0, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
+                            mma_f16_ta(d0 + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
+                            acc = 1u;
+                        }
+                        mma_commit(&aempty[se]);
+                        mma_commit(&bempty[sb]);
+                        if (last) mma_commit(&tfull[buf]);
                     }
-                    mma_commit(&empty[st]);
-                    if (last) mma_commit(&tfull[buf]);
+                    __syncwarp();
+                    if (last && ++buf == NB) { buf = 0; pf ^= 1u; }
+                    if (++sa == ASTAGES) { sa = 0; aph ^= 1u; }
+                    if (++se == 2 * ASTAGES) se = 0;
+                    if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
                 }
-                __syncwarp();
-                if (last && ++buf == NB) { buf = 0; pf ^= 1u; }
-                if (++st == STAGES) { st = 0; ph ^= 1u; }
             }
         }
     }
@@ -487,7 +626,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A, c
     __syncthreads();
     if (warp == W_MMA) {
         tc_fence_after();
-        tmem_free<NB * BUF_COLS>(tmem_base);
+        tmem_free<TMEM_COLS>(tmem_base);
     }
 }
 
@@ -558,16 +697,6 @@ int tc_make_map(void* m, void* base, uint64_t rows, uint64_t cols, uint32_t box_
 
 size_t tc_row_pitch(int n_in) { return (size_t)tg::row_pitch(n_in); }
 
-// Tensor maps over `rows` operand rows (2 * rows map rows of `pitch` fp16).
-int tc_make_maps(void* op, uint64_t rows, int n_in, TcMaps* out) {
-    static_assert(sizeof(TcMaps) == sizeof(tg::Maps), "TcMaps must mirror tg::Maps");
-    tg::Maps* m = reinterpret_cast<tg::Maps*>(out);
-    int rc;
-    for (int i = 0; i < 3; ++i)
-        if ((rc = tc_make_map(&m->box[i], op, 2 * rows, (uint64_t)tg::row_pitch(n_in), 16u << i))) return rc;
-    return tc_make_map(&m->row, op, 2 * rows, (uint64_t)tg::row_pitch(n_in), 1);
-}
-
 int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, int ldx, int rows, int n_in, uint16_t* op, const char* name,
                         const int32_t* rows_dev) {
     if (n_in % 256 || ldx % 4) return DNB_DECLINED;
@@ -583,32 +712,32 @@ bool tc_handles(int type, int n_in, int n_out, bool fused) {
 }
 
 template <int T, bool PAIR>
-static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A, const tg::Maps& M) {
+static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
     using L = tg::Layout<T>;
-    size_t at = kMmSmemBase + L::HEAD + L::LOW_B * tg::B_STAGE;
+    size_t at = kMmSmemBase + L::LOW + L::LOW_B * tg::B_STAGE;
     if (T == T_IQ3_XXS) at = (at + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign + sizeof(MmCodebook);
-    const size_t smem = at + L::STAGES * tg::A_STAGE + (L::STAGES - L::LOW_B) * tg::B_STAGE - kMmSmemBase;
+    const size_t smem = at + L::TAIL - kMmSmemBase;
+    static_assert(L::BARS * 8 + 16 + (tg::kMaxSeg + 1) * 4 + 8 + tg::kLocalItems * sizeof(tg::Item) <= L::HEAD, "head too small");
     A.smem = (uint32_t)smem;
     auto kern = tg::grouped_tc_kernel<T, PAIR>;
     static SmemGrant grant;
     DNB_CUDA(grant_smem(grant, c->device, kern, smem));
     ProfScope prof_(c, st, PAIR ? "tc_down" : "tc_gate_up");
-    DNB_CUDA(launch_k(kern, dim3(c->sm_count), dim3(tg::NTHREADS), smem, st, c->use_pdl, A, M));
+    DNB_CUDA(launch_k(kern, dim3(c->sm_count), dim3(tg::NTHREADS), smem, st, c->use_pdl, A));
     c->launches++;
     return DNB_OK;
 }
 
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
-                      int n_out, const uint16_t* op, const TcMaps* maps, const int32_t* row_token, float* out, float* const* row_dst) {
+                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst) {
     if (!tc_handles(type, n_in, n_out, fused) || nseg_max > tg::kMaxSeg) return DNB_DECLINED;
     int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
     if (rc) return rc;
     tg::Args A = {};
     A.seg = seg; A.nseg_dev = nseg_dev; A.nseg_max = nseg_max; A.n_in = n_in; A.n_out = n_out; A.rb = (int)row_bytes(type, n_in);
     A.op = op; A.row_token = row_token; A.out = out; A.row_dst = row_dst; A.status = c->status;
-    const tg::Maps& M = *reinterpret_cast<const tg::Maps*>(maps);
-    if (type == T_Q4_K) return fused ? launch_tc_t<T_Q4_K, false>(c, st, A, M) : launch_tc_t<T_Q4_K, true>(c, st, A, M);
-    return fused ? launch_tc_t<T_IQ3_XXS, false>(c, st, A, M) : launch_tc_t<T_IQ3_XXS, true>(c, st, A, M);
+    if (type == T_Q4_K) return fused ? launch_tc_t<T_Q4_K, false>(c, st, A) : launch_tc_t<T_Q4_K, true>(c, st, A);
+    return fused ? launch_tc_t<T_IQ3_XXS, false>(c, st, A) : launch_tc_t<T_IQ3_XXS, true>(c, st, A);
 }
 
 }  // namespace dnb

@@ -66,7 +66,7 @@ __device__ __forceinline__ void operand_block(float4 v0, float4 v1, float up, in
             const int at = K + b / 32 + 2 * (lane >> 3);
             *reinterpret_cast<uint32_t*>(hi + at) = sh;
             *reinterpret_cast<uint32_t*>(lo + at) = sl;
-            if (K <= 1024) {  // the stage with both halves of the mins reads the sums twice
+            if (K % 2048 && K % 2048 <= 1024 && b >= K / 2048 * 2048) {  // the stage with both halves of the mins reads the sums twice
                 *reinterpret_cast<uint32_t*>(hi + at + 32) = sh;
                 *reinterpret_cast<uint32_t*>(lo + at + 32) = sl;
             }
@@ -78,9 +78,9 @@ template <int T>
 __device__ __forceinline__ void operand_tail(float up, int K, int pitch, int lane, uint16_t* hi) {
     const int xc = x_cols(K);
     if constexpr (T == T_Q4_K) {
-        const int nsub = K / 32;
-        for (int i = lane; i < xc; i += 32)
-            if (K <= 1024 ? (i & 31) >= nsub : i >= nsub) hi[K + i] = hi[pitch + K + i] = 0;
+        const int nsub = K / 32, g0 = nsub / 64 * 64, rest = nsub - g0;  // the last, partial group of 64
+        for (int i = lane; i < xc - g0; i += 32)
+            if (rest <= 32 ? (i & 31) >= rest : i >= rest) hi[K + g0 + i] = hi[pitch + K + g0 + i] = 0;
     }
     if (lane == 0) *reinterpret_cast<float*>(hi + K + xc) = __uint_as_float((254u << 23) - __float_as_uint(up));  // 1 / up
 }

@@ -81,7 +81,7 @@ uint64_t dnb_launch_count(dnb_ctx* ctx);
  * kernel, the flags of the expert-parallel exchange) are bounded.  A wait that gives up
  * records a code in the context's status word (pinned host memory the device writes):
  *   1        a bulk copy into shared memory never completed
- *   2-6      the tcgen05 grouped GEMM (stage, accumulator or drain barrier)
+ *   2-8      the tcgen05 grouped GEMM (stage, accumulator, drain or raw-row barrier)
  *   20-22    expert-parallel exchange: row out of range / a peer's counts or rows did not
  *            arrive / a peer's results did not arrive
  *   24       expert-parallel decode: a peer's result rows did not arrive
