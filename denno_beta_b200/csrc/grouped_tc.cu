@@ -55,7 +55,8 @@ constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + ASTAGES * 2 * A_COLS;
 static_assert(TMEM_COLS == 512, "tensor memory");
 constexpr int SCL = 8;                  // ring of block scales: producers are at most NB + 2 blocks ahead of the epilogue
 constexpr int BDEPTH = 4;               // B stages on their way
-constexpr float kMinScale = 1024.f;     // the mins' A values are scaled up so that the low halves stay normal fp16 numbers
+constexpr uint32_t kMinScaleH = 0x4C004C00u;  // the mins' A values are 16 times the mins: their low halves then lose nothing that matters
+constexpr float kMinScale = 16.f;             // (2^-28 absolute), and a min may still be as large as 4,000
 
 template <int T> constexpr int kBB = T == T_Q4_K ? 144 : 98;
 
@@ -205,23 +206,20 @@ __device__ __forceinline__ void mins_stage(const uint8_t* raw, int blocks, int u
     const bool both = blocks <= 4;
 #pragma unroll 1
     for (int half = 0; half < 2; ++half) {
+        const bool low = both ? half != 0 : u != 0;
         uint32_t o[16];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {  // the eight sub-blocks of a block: four columns
-            const int part = both ? half : u, blk = both ? c : 4 * half + c;
+            const int blk = both ? c : 4 * half + c;
             const bool live = blk < blocks;
             const uint4 h = *reinterpret_cast<const uint4*>(raw + 16 * (live ? blk : 0));
-            const float dm = live ? -kMinScale * h2f((uint16_t)(h.x >> 16)) : 0.f;
+            const uint32_t dm = live ? h2mul(__byte_perm(h.x, 0u, 0x3232u), kMinScaleH ^ 0x80008000u) : 0u;  // -16 * dmin
+            const uint32_t mn[2] = {h.z & 0x3f3f3f3fu, ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u)};  // kquant.rs:878-887
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {  // sub-blocks 2 k, 2 k + 1
-                const int sh = 16 * (k & 1);
-                const uint32_t b = h.z >> sh, d = h.w >> sh;
-                const uint32_t mn = k < 2 ? (b & 0x3f3fu) : (((d >> 4) & 0x0f0fu) | ((b >> 2) & 0x3030u));
-                const float f0 = dm * (float)(mn & 0xffu), f1 = dm * (float)((mn >> 8) & 0xffu);
-                const __half2 hi = __floats2half2_rn(f0, f1);
-                const float2 hf = __half22float2(hi);
-                const __half2 lo = __floats2half2_rn(f0 - hf.x, f1 - hf.y);
-                o[4 * c + k] = part ? *reinterpret_cast<const uint32_t*>(&lo) : *reinterpret_cast<const uint32_t*>(&hi);
+            for (int k = 0; k < 4; ++k) {  // sub-blocks 2 k, 2 k + 1: dmin * m rounded, or exactly what that left over
+                const uint32_t m2 = h2sub(__byte_perm(mn[k >> 1], 0x64646464u, (k & 1) ? 0x4342u : 0x4140u), 0x64006400u);
+                const uint32_t hi = h2mul(dm, m2);
+                o[4 * c + k] = low ? h2fma(dm, m2, hi ^ 0x80008000u) : hi;
             }
         }
         tmem_st16(taddr + 16 * half, o);
@@ -548,79 +546,90 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             if (++sd == BSTAGES) sd = 0;
             --flying;
         };
-        const uint16_t* opl = A.op + 8 * (lane & 7);
+        const uint32_t sw0 = chunk_off(lane >> 3, lane & 7), sw1 = chunk_off(4 + (lane >> 3), lane & 7);  // rows r and r + 8 swizzle alike
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             const int steps = tile_tokens(it.m) / 2;  // 4 rows each
-            uint32_t row[16];  // operand array rows of this lane's B rows
+            const uint16_t* src[16];  // operand array rows of this lane's B rows
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int br = 4 * i + (lane >> 3), pr = it.prow + min(br >> 1, it.m - 1);
-                row[i] = i < steps ? 2u * (uint32_t)(A.row_token ? A.row_token[pr] : pr) + (br & 1) : 0u;
+                const uint32_t orow = i < steps ? (uint32_t)(A.row_token ? A.row_token[pr] : pr) : 0u;
+                src[i] = A.op + (size_t)(2u * orow + (br & 1)) * pitch + 8 * (lane & 7);
             }
-            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
-                const int bn = min(8, nblk - b0), nst = 4 * bn + min_stages<T>(bn);
-                for (int c = 0; c < nst; ++c) {
-                    ok = warp_all(mb_wait(&bempty[sb], bph, A.status, 4));
-                    if (!ok) break;
-                    const int col = c < 4 * bn ? b0 * 256 + c * BK : A.n_in + 8 * b0;  // the mins read the sums behind the row
-                    uint8_t* d = b_tile(sb);
+            auto stage = [&](int off) {  // off: elements from src
+                ok = warp_all(mb_wait(&bempty[sb], bph, A.status, 4));
+                if (!ok) return;
+                uint8_t* d = b_tile(sb);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (i < steps) cp_async16(d + chunk_off(4 * i + (lane >> 3), lane & 7), opl + (size_t)row[i] * pitch + col);
-                    cp_async_commit();
-                    if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
-                    if (++flying > BDEPTH) {
-                        cp_async_wait_group<BDEPTH>();
-                        land();
-                    }
+                for (int i = 0; i < 16; ++i)
+                    if (i < steps) cp_async16(d + ((i & 1) ? sw1 : sw0) + (i >> 1) * 1024, src[i] + off);
+                cp_async_commit();
+                if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
+                if (++flying > BDEPTH) {
+                    cp_async_wait_group<BDEPTH>();
+                    land();
                 }
+            };
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0);
+                for (int b = 0; b < bn && ok; ++b) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (ok) stage(c * BK);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) src[i] += 256;
+                }
+                const int sums = A.n_in - 256 * (b0 + bn) + 8 * b0;  // the mins read the sums behind the row
+                for (int u = 0; u < min_stages<T>(bn) && ok; ++u) stage(sums);
             }
         }
         cp_async_wait_all();
         while (flying > 0) land();
     } else {
-        // ---------------- MMA issue ----------------
-        int sa = 0, se = 0, sb = 0, buf = 0;
-        uint32_t aph = 0u, bph = 0u, pf = 1u;
-        for (int k = 0; k < my_items && ok; ++k) {
-            const Item it = item(k);
-            const int nte = tile_tokens(it.m);
-            const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
-            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
-                const int bn = min(8, nblk - b0), nst = 4 * bn + min_stages<T>(bn);
-                for (int c = 0; c < nst; ++c) {
-                    const bool mins = c >= 4 * bn, first = mins ? c == 4 * bn : (c & 3) == 0, last = mins ? c == nst - 1 : (c & 3) == 3;
-                    if (first) ok = warp_all(mb_wait(&tfree[buf], pf, A.status, 6));
-                    if (ok) ok = warp_all(mb_wait(&bfull[sb], bph, A.status, 5));
-                    if (ok) ok = warp_all(mb_wait(&afull[sa], aph, A.status, 5));
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(sa * 2 * A_COLS), b_lo = desc_lo(s32(b_tile(sb)));
+        // ---------------- MMA issue: one thread ----------------
+        if (elect_one()) {
+            int sa = 0, se = 0, sb = 0, buf = 0;
+            uint32_t aph = 0u, bph = 0u, pf = 1u;
+            for (int k = 0; k < my_items && ok; ++k) {
+                const Item it = item(k);
+                const int nte = tile_tokens(it.m);
+                const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
+                for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                    const int bn = min(8, nblk - b0);
+                    // one block: `stages` stages of `live` K steps (mins: the K steps that hold sub-blocks; hi and lo side by side when both fit)
+                    auto block = [&](int stages, int live, bool pair) {
+                        ok = mb_wait(&tfree[buf], pf, A.status, 6);
                         const uint32_t d0 = tmem_base + (uint32_t)(buf * BUF_COLS);
-                        // a stage of mins: the K steps that hold sub-blocks (hi and lo halves side by side when both fit)
-                        const int live = !mins ? 4 : (bn * 8 + 15) / 16;
-                        uint32_t acc = first ? 0u : 1u;
+                        uint32_t acc = 0u;
+                        for (int c = 0; c < stages && ok; ++c) {
+                            ok = mb_wait(&bfull[sb], bph, A.status, 5) && mb_wait(&afull[sa], aph, A.status, 5);
+                            if (!ok) break;
+                            tc_fence_after();
+                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(sa * 2 * A_COLS), b_lo = desc_lo(s32(b_tile(sb)));
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            if (mins && (bn <= 4 ? (ks & 1) >= live : ks >= live)) continue;
-                            mma_f16_ta(d0, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
-                            mma_f16_ta(d0 + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
-                            acc = 1u;
+                            for (int ks = 0; ks < 4; ++ks) {
+                                if ((pair ? ks & 1 : ks) >= live) continue;
+                                mma_f16_ta(d0, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
+                                mma_f16_ta(d0 + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
+                                acc = 1u;
+                            }
+                            mma_commit(&aempty[se]);
+                            mma_commit(&bempty[sb]);
+                            if (++sa == ASTAGES) { sa = 0; aph ^= 1u; }
+                            if (++se == 2 * ASTAGES) se = 0;
+                            if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
                         }
-                        mma_commit(&aempty[se]);
-                        mma_commit(&bempty[sb]);
-                        if (last) mma_commit(&tfull[buf]);
-                    }
-                    __syncwarp();
-                    if (last && ++buf == NB) { buf = 0; pf ^= 1u; }
-                    if (++sa == ASTAGES) { sa = 0; aph ^= 1u; }
-                    if (++se == 2 * ASTAGES) se = 0;
-                    if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
+                        if (!ok) return;
+                        mma_commit(&tfull[buf]);
+                        if (++buf == NB) { buf = 0; pf ^= 1u; }
+                    };
+                    for (int b = 0; b < bn && ok; ++b) block(4, 4, false);
+                    if (T == T_Q4_K && ok) block(min_stages<T>(bn), (bn * 8 + 15) / 16, bn <= 4);
                 }
             }
         }
+        __syncwarp();
     }
     tc_fence_before();
     __syncthreads();

@@ -20,18 +20,19 @@ __device__ __forceinline__ void mb_arrive(uint64_t* b) {
 __device__ __forceinline__ void mb_expect_tx(uint64_t* b, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(s32(b)), "r"(bytes) : "memory");
 }
+// One poll sleeps for up to 20 us while the phase is open: a warp that waits leaves its issue slots to the others.
 __device__ __forceinline__ bool mb_try(uint64_t* b, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(s32(b)), "r"(parity)
+        : "r"(s32(b)), "r"(parity), "r"(20000u)
         : "memory");
     return ok != 0;
 }
-// Bounded: after 2^21 polls the wait gives up, records `code` in the status word and returns false.
+// Bounded: after 2^15 polls (half a second or so) the wait gives up, records `code` in the status word and returns false.
 __device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, int* status, int code) {
-    for (int i = 0; i < (1 << 21); ++i)
+    for (int i = 0; i < (1 << 15); ++i)
         if (mb_try(b, parity)) return true;
     status_set(status, code);
     return false;
