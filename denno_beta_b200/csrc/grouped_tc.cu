@@ -16,10 +16,11 @@
 // way of both.  Shared memory is the tightest: with A tiles in it (32 KB written and 32 KB read per stage, B read once per tile) a
 // stage took 840 cycles, all of them shared-memory bandwidth.  So A goes from the producers' registers to tensor memory
 // (tcgen05.st, thread = row = lane) and the MMA takes it from there.  One role per warp, each with a ring of its own in front:
-//   * two warps copy packed rows (a 256-element block of all 256 rows: 9 or 7 neighbouring lanes per row) into a raw ring.  (A
+//   * four warps copy packed rows (a 256-element block of all 256 rows: 9 or 7 neighbouring lanes per row) into a raw ring.  (A
 //     thread that fetches its own row's bytes touches 32 cache lines per instruction; that alone took 0.5 us per stage.)
-//   * one warp copies the tokens' hi and lo rows into swizzled B tiles, gathered from the token-major rows: no packed copy of
-//     the activations.  (TMA row gathers took 80 cycles per four rows.)
+//   * two warps copy the tokens' hi and lo rows into swizzled B tiles, a stage each in turn, gathered from the token-major rows:
+//     no packed copy of the activations.  (TMA row gathers took 80 cycles per four rows; a proxy fence in the copying warp
+//     waits for the copies still on their way, so it is the MMA thread that executes it.)
 //   * four groups of four producer warps, group j decodes the j-th 64 elements of every block, a thread one row of both tiles;
 //     the block's scales go to a small ring.
 //   * the MMA warp; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
@@ -45,16 +46,15 @@ constexpr int A_COLS = BK / 2;          // tensor-memory columns of an A tile (t
 constexpr int B_STAGE = 2 * NT * BK * 2;// hi and lo rows: 8 KB
 constexpr int NB = 2;                   // accumulator buffers
 constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
-constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS, RWARPS = 2;
-constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + 1;
+constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS, RWARPS = 4, BWARPS = 2;
+constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;
 constexpr int NTHREADS = (W_MMA + 1) * 32;
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
-constexpr int ASTAGES = 4, BSTAGES = 6;
-constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + ASTAGES * 2 * A_COLS;
+constexpr int STAGES = 4;               // of the ring that A (tensor memory) and B (shared memory) share
+constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + STAGES * 2 * A_COLS;
 static_assert(TMEM_COLS == 512, "tensor memory");
-constexpr int SCL = 8;                  // ring of block scales: producers are at most NB + 2 blocks ahead of the epilogue
-constexpr int BDEPTH = 4;               // B stages on their way
+constexpr int SCL = 8;                  // ring of block scales: producers are at most NB + 3 blocks ahead of the epilogue
 constexpr uint32_t kMinScaleH = 0x4C004C00u;  // the mins' A values are 16 times the mins: their low halves then lose nothing that matters
 constexpr float kMinScale = 16.f;             // (2^-28 absolute), and a min may still be as large as 4,000
 
@@ -233,16 +233,32 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {  // an arrival 
 }
 template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Shared memory: [barriers, segment table, items][block scales][B stages that fit below][IQ3_XXS tables at a 32 KB boundary]
-// [rest of the B ring][raw ring]
+// Shared memory: [barriers, segment table, items][block scales][two B stages][IQ3_XXS tables at a 32 KB boundary][two B stages][raw ring]
 template <int T> struct Layout {
     static constexpr int RSTAGES = 3;
     static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
-    static constexpr int LOW_B = T == T_Q4_K ? BSTAGES : 2;
-    static constexpr int BARS = 3 * ASTAGES + 2 * (BSTAGES + RSTAGES + NB);
+    static constexpr int LOW_B = 2;
+    static constexpr int BARS = 3 * STAGES + 2 * (RSTAGES + NB);
     static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
     static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
-    static constexpr int TAIL = (BSTAGES - LOW_B) * B_STAGE + RSTAGES * RAW_STAGE;
+    static constexpr int TAIL = (STAGES - LOW_B) * B_STAGE + RSTAGES * RAW_STAGE;
+};
+
+// A stage number as its user sees it.  A group's stages are up to six apart and the groups may be a block apart from one another:
+// with one `empty` barrier per slot a group could look at a slot whose last but one stage is still in use and take its parity for
+// the last one's.  Stage n therefore commits to barrier n mod 2 * STAGES, and its slot's next user waits for exactly that commit.
+struct StageCount {
+    int q;          // stage number mod 2 * STAGES
+    uint32_t turn;  // parity of its turn
+    __device__ __forceinline__ explicit StageCount(int first) : q(first), turn(0u) {}
+    __device__ __forceinline__ void advance(int n) {
+        q += n;
+        if (q >= 2 * STAGES) { q -= 2 * STAGES; turn ^= 1u; }
+    }
+    __device__ __forceinline__ int slot() const { return q & (STAGES - 1); }
+    __device__ __forceinline__ bool wait(uint64_t* empty, int* status, int code) const {  // the stage STAGES earlier is done with its slot
+        return q < STAGES ? mb_wait(&empty[q + STAGES], turn ^ 1u, status, code) : mb_wait(&empty[q - STAGES], turn, status, code);
+    }
 };
 
 template <int T, bool PAIR>  // PAIR: both tiles from seg.wa (256 rows, fp32 results); else gate and up rows, silu(g) * u
@@ -251,11 +267,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     using R = Raw<T>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (s32(smem_raw) & 1023u)) & 1023u);
-    uint64_t* afull = reinterpret_cast<uint64_t*>(base);
-    uint64_t* aempty = afull + ASTAGES;
-    uint64_t* bfull = aempty + 2 * ASTAGES;  // (two per slot, see the producers)
-    uint64_t* bempty = bfull + BSTAGES;
-    uint64_t* rfull = bempty + BSTAGES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(base);
+    uint64_t* empty = full + STAGES;          // two per slot, see the producers
+    uint64_t* rfull = empty + 2 * STAGES;
     uint64_t* rempty = rfull + L::RSTAGES;
     uint64_t* tfull = rempty + L::RSTAGES;
     uint64_t* tfree = tfull + NB;
@@ -271,7 +285,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         p = book + sizeof(MmCodebook);
     }
     uint8_t* b_high = p;
-    uint8_t* raw_base = b_high + (BSTAGES - L::LOW_B) * B_STAGE;
+    uint8_t* raw_base = b_high + (STAGES - L::LOW_B) * B_STAGE;
     if ((uint32_t)(b_high + L::TAIL - smem_raw) > A.smem) {  // only if shared memory started elsewhere
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
@@ -284,9 +298,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < ASTAGES; ++i) mb_init(&afull[i], 4);                                     // a producer group
-        for (int i = 0; i < 2 * ASTAGES; ++i) mb_init(&aempty[i], 1);                                // a commit
-        for (int i = 0; i < BSTAGES; ++i) { mb_init(&bfull[i], 1); mb_init(&bempty[i], 1); }       // the B warp; a commit
+        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 4 + 32);    // a producer group's warps, a B warp's lanes
+        for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], 1);    // a commit
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
         for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
         fence_mbarrier_init();
@@ -339,15 +352,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
         int buf = 0, sc = 0;
         uint32_t pb = 0;
+        auto row_scale = [&](int k) {  // lane j: what undoes the scaling of token j of this warp's half (asked for an item ahead)
+            const Item it = item(k);
+            const int half = tile_tokens(it.m) >> 1, pr = it.prow + min(hsel * half + min(lane, half - 1), it.m - 1);
+            const int orow = A.row_token ? A.row_token[pr] : pr;
+            return *reinterpret_cast<const float*>(A.op + (size_t)(2 * orow) * pitch + scale_col);
+        };
+        float rs_next = my_items > 0 ? row_scale(0) : 0.f;
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             const int nte = tile_tokens(it.m), half = nte >> 1;
-            float rs = 0.f;  // lane j: what undoes the scaling of token j of this warp's half
-            if (lane < half) {
-                const int pr = it.prow + min(hsel * half + lane, it.m - 1);
-                const int orow = A.row_token ? A.row_token[pr] : pr;
-                rs = *reinterpret_cast<const float*>(A.op + (size_t)(2 * orow) * pitch + scale_col);
-            }
+            const float rs = rs_next;
+            rs_next = k + 1 < my_items ? row_scale(k + 1) : 0.f;
             float acc[2][16];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt)
@@ -415,19 +431,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
         int rst = 0, sc = 0;
         uint32_t rph = 0u;
-        // A group's stages are up to six apart and the groups may be a block apart from one another: with one barrier per slot a
-        // group could look at a slot whose last but one stage is still in use and take its parity for the last one's.  Stage q
-        // therefore commits to barrier q mod 2 * ASTAGES, and its slot's next user waits for exactly that commit.
-        int q = grp;               // this group's next stage, mod 2 * ASTAGES
-        uint32_t turn = 0u;        // parity of the turn of that count
-        auto advance = [&](int n) {
-            q += n;
-            while (q >= 2 * ASTAGES) { q -= 2 * ASTAGES; turn ^= 1u; }
-        };
-        auto slot = [&]() { return q < ASTAGES ? q : q - ASTAGES; };
-        auto wait_slot = [&]() {
-            return warp_all(q < ASTAGES ? mb_wait(&aempty[q + ASTAGES], turn ^ 1u, A.status, 2) : mb_wait(&aempty[q - ASTAGES], turn, A.status, 2));
-        };
+        StageCount q(grp);
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             uint32_t oa = 0, ob = 0;  // where the two rows' blocks start within 16 bytes
@@ -453,17 +457,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         scl[(sc * 2 + 1) * TILE_M + r] = rb.scale();
                         sc = (sc + 1) & (SCL - 1);
                     }
-                    ok = wait_slot();
+                    ok = warp_all(q.wait(empty, A.status, 2));
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t ta = tlane + slot() * (2 * A_COLS);
+                    const uint32_t ta = tlane + q.slot() * (2 * A_COLS);
                     decode_stage(ra, grp, ta, gl, sl);
                     decode_stage(rb, grp, ta + A_COLS, gl, sl);
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mb_arrive(&afull[slot()]);
-                    advance(4);
+                    if (lane == 0) mb_arrive(&full[q.slot()]);
+                    q.advance(4);
                 }
                 if (!ok) break;
                 if constexpr (T == T_Q4_K) {  // the mins: group u builds stage u; then every group is `nm` stages on
@@ -471,45 +475,45 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
                     if (!ok) break;
                     if (grp < nm) {
-                        ok = wait_slot();
+                        ok = warp_all(q.wait(empty, A.status, 2));
                         if (!ok) break;
                         tc_fence_after();
-                        const uint32_t ta = tlane + slot() * (2 * A_COLS);
+                        const uint32_t ta = tlane + q.slot() * (2 * A_COLS);
                         const uint8_t* raw = raw_base + rst * L::RAW_STAGE + r * R::RS;
                         mins_stage(raw, bn, grp, ta);
                         mins_stage(raw + L::RAW_TILE, bn, grp, ta + A_COLS);
                         tmem_st_wait();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mb_arrive(&afull[slot()]);
+                        if (lane == 0) mb_arrive(&full[q.slot()]);
                     }
                     __syncwarp();
                     if (lane == 0) mb_arrive(&rempty[rst]);
                     if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
-                    advance(nm);
+                    q.advance(nm);
                 }
             }
         }
     } else if (warp < W_B) {
         // ---------------- raw rows: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
-        const int rw = warp - W_RAW, c16 = (lane & 7) * 16;
+        const int rw = warp - W_RAW, c16 = (lane & 7) * 16, row0 = (rw & 1) * (TILE_M / 2);  // half a tile per warp
         int rst = 0;
         uint32_t rph = 1u;
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
-            const uint8_t* tile0 = (rw ? it.pb : it.pa);  // a warp per tile
+            const uint8_t* half = ((rw & 2) ? it.pb : it.pa) + (size_t)row0 * A.rb;
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
                 for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0); ++b) {
                     ok = warp_all(mb_wait(&rempty[rst], rph, A.status, 8));
                     if (!ok) break;
-                    uint8_t* dst = raw_base + rst * L::RAW_STAGE + rw * L::RAW_TILE;
+                    uint8_t* dst = raw_base + rst * L::RAW_STAGE + ((rw & 2) ? L::RAW_TILE : 0) + row0 * R::RS;
+                    const uint32_t step = 4u * A.rb;
                     if (b < bn) {
-                        const uint8_t* src = tile0 + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
+                        const uint8_t* src = half + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
                         uint8_t* d = dst + (lane >> 3) * R::RS + c16;
-                        const uint32_t step = 4u * A.rb;
-#pragma unroll 8
-                        for (int i = 0; i < TILE_M / 4; ++i, src += step) {
+#pragma unroll
+                        for (int i = 0; i < TILE_M / 8; ++i, src += step) {
                             if constexpr (T == T_Q4_K) {
                                 cp_async16(d + i * 4 * R::RS, src + c16);
                             } else {
@@ -518,15 +522,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                             }
                         }
                         if constexpr (T == T_Q4_K) {
-                            const uint8_t* s9 = tile0 + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
+                            const uint8_t* s9 = half + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
 #pragma unroll
-                            for (int i = 0; i < TILE_M / 32; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
+                            for (int i = 0; i < TILE_M / 64; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
                         }
                     } else if constexpr (T == T_Q4_K) {  // the headers of the last bn blocks: lane = block lane % 8
-                        const uint8_t* src = tile0 + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + (lane & 7)) * kBB<T>;
+                        const uint8_t* src = half + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + (lane & 7)) * kBB<T>;
                         if ((lane & 7) < bn) {
-#pragma unroll 8
-                            for (int i = 0; i < TILE_M / 4; ++i) cp_async16(dst + ((lane >> 3) + 4 * i) * R::RS + c16, src + (size_t)(4 * i) * A.rb);
+#pragma unroll
+                            for (int i = 0; i < TILE_M / 8; ++i, src += step) cp_async16(dst + ((lane >> 3) + 4 * i) * R::RS + c16, src);
                         }
                     }
                     cp_async_arrive(&rfull[rst]);
@@ -535,17 +539,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         cp_async_wait_all();
-    } else if (warp == W_B) {
+    } else if (warp < W_MMA) {
         // ---------------- B tiles: rows 2 t, 2 t + 1 = hi and lo of token t; lane = unit lane % 8 of row lane / 8 (+ 4 per step) ----------------
-        int sb = 0, sd = 0, flying = 0;  // next slot, oldest slot on its way, how many are
-        uint32_t bph = 1u;
-        auto land = [&]() {  // the oldest stage on its way is complete: visible to the tensor core
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) mb_arrive(&bfull[sd]);
-            if (++sd == BSTAGES) sd = 0;
-            --flying;
-        };
+        StageCount q(0);
+        int mine = warp - W_B;  // 0: the next stage is this warp's
         const uint32_t sw0 = chunk_off(lane >> 3, lane & 7), sw1 = chunk_off(4 + (lane >> 3), lane & 7);  // rows r and r + 8 swizzle alike
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
@@ -558,18 +555,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                 src[i] = A.op + (size_t)(2u * orow + (br & 1)) * pitch + 8 * (lane & 7);
             }
             auto stage = [&](int off) {  // off: elements from src
-                ok = warp_all(mb_wait(&bempty[sb], bph, A.status, 4));
-                if (!ok) return;
-                uint8_t* d = b_tile(sb);
+                if (mine == 0) {
+                    ok = warp_all(q.wait(empty, A.status, 4));
+                    if (!ok) return;
+                    uint8_t* d = b_tile(q.slot());
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (i < steps) cp_async16(d + ((i & 1) ? sw1 : sw0) + (i >> 1) * 1024, src[i] + off);
-                cp_async_commit();
-                if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
-                if (++flying > BDEPTH) {
-                    cp_async_wait_group<BDEPTH>();
-                    land();
+                    for (int i = 0; i < 16; ++i)
+                        if (i < steps) cp_async16(d + ((i & 1) ? sw1 : sw0) + (i >> 1) * 1024, src[i] + off);
+                    cp_async_arrive(&full[q.slot()]);
                 }
+                mine ^= 1;
+                q.advance(1);
             };
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
@@ -585,12 +581,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         cp_async_wait_all();
-        while (flying > 0) land();
     } else {
         // ---------------- MMA issue: one thread ----------------
         if (elect_one()) {
-            int sa = 0, se = 0, sb = 0, buf = 0;
-            uint32_t aph = 0u, bph = 0u, pf = 1u;
+            StageCount q(0);
+            int buf = 0;
+            uint32_t pf = 1u;
             for (int k = 0; k < my_items && ok; ++k) {
                 const Item it = item(k);
                 const int nte = tile_tokens(it.m);
@@ -603,10 +599,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         const uint32_t d0 = tmem_base + (uint32_t)(buf * BUF_COLS);
                         uint32_t acc = 0u;
                         for (int c = 0; c < stages && ok; ++c) {
-                            ok = mb_wait(&bfull[sb], bph, A.status, 5) && mb_wait(&afull[sa], aph, A.status, 5);
+                            ok = mb_wait(&full[q.slot()], q.q < STAGES ? 0u : 1u, A.status, 5);  // a slot has two turns in the count
                             if (!ok) break;
-                            tc_fence_after();
-                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(sa * 2 * A_COLS), b_lo = desc_lo(s32(b_tile(sb)));
+                            tc_fence_after();    // A: written to tensor memory by the producers
+                            fence_async_smem();  // B: written to shared memory by the B warps' copies
+                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(q.slot() * 2 * A_COLS), b_lo = desc_lo(s32(b_tile(q.slot())));
 #pragma unroll
                             for (int ks = 0; ks < 4; ++ks) {
                                 if ((pair ? ks & 1 : ks) >= live) continue;
@@ -614,11 +611,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                                 mma_f16_ta(d0 + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
                                 acc = 1u;
                             }
-                            mma_commit(&aempty[se]);
-                            mma_commit(&bempty[sb]);
-                            if (++sa == ASTAGES) { sa = 0; aph ^= 1u; }
-                            if (++se == 2 * ASTAGES) se = 0;
-                            if (++sb == BSTAGES) { sb = 0; bph ^= 1u; }
+                            mma_commit(&empty[q.q]);
+                            q.advance(1);
                         }
                         if (!ok) return;
                         mma_commit(&tfull[buf]);
