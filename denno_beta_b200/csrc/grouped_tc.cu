@@ -30,6 +30,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "dnb_common.cuh"
 #include "tc_ptx.cuh"
 #include "iq3_f16.cuh"
@@ -48,7 +50,11 @@ constexpr int NB = 2;                   // accumulator buffers
 constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
 constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS, RWARPS = 4, BWARPS = 2;
 constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;
-constexpr int NTHREADS = (W_MMA + 1) * 32;
+constexpr int NTHREADS = 1024;          // 32 warps, the last one idle
+// Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
+constexpr int REG_EPI = 112, REG_PROD = 56, REG_RAW = 24, REG_MISC = 40;
+static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
+static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA < 32, "roles fill warpgroups");
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
 constexpr int STAGES = 4;               // of the ring that A (tensor memory) and B (shared memory) share
@@ -110,6 +116,9 @@ struct Args {
 __device__ __forceinline__ uint32_t chunk_off(int r, int c) {  // 16-byte column c of row r in a 128-byte-swizzled tile
     return (uint32_t)r * 128u + (uint32_t)((c ^ (r & 7)) << 4);
 }
+
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ---- producers: one row of both tiles per thread -------------------------------------------------------------------------
 template <int T> struct Raw;  // what stage `c` (0..3) of a block needs of a row's packed bytes
@@ -298,7 +307,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 4 + 32);    // a producer group's warps, a B warp's lanes
+        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 4 + BWARPS * 32);    // a producer group's warps, the B warps' lanes
         for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], 1);    // a commit
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
         for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
@@ -347,6 +356,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
 
     if (warp < EWARPS) {
         // ---------------- epilogue: TMEM lane = weight row ----------------
+        reg_inc<REG_EPI>();
         const int quad = warp & 3, hsel = warp >> 2;
         const int r = quad * 32 + lane;
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -382,26 +392,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         sc = (sc + 1) & (SCL - 1);
                     }
                     const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * nte);
+                    auto drain = [&](auto full_tile) {  // eight tokens a load and tile; 32-token tiles have sixteen per warp
+                        constexpr int H = decltype(full_tile)::value ? 2 : 1;
+                        uint32_t v[2][H][16];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {  // eight tokens each; 32-token tiles have two per warp
-                        if (h == 0 || nte == 32) {
-                            uint32_t v[2][16];
-                            tmem_ld16(col + 16 * h, v[0]);
-                            tmem_ld16(col + 2 * NT + 16 * h, v[1]);
-                            tmem_ld_wait();
-                            if (h == 1 || nte != 32) {  // read: hand the buffer back before the arithmetic
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) mb_arrive(&tfree[buf]);
-                            }
+                        for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-                            for (int mt = 0; mt < 2; ++mt)
+                            for (int h = 0; h < H; ++h) tmem_ld16(col + mt * 2 * NT + 16 * h, v[mt][h]);
+                        tmem_ld_wait();
+                        tc_fence_before();  // read: hand the buffer back before the arithmetic
+                        __syncwarp();
+                        if (lane == 0) mb_arrive(&tfree[buf]);
 #pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    acc[mt][8 * h + j] =
-                                        fmaf(s[mt], __uint_as_float(v[mt][2 * j]) + __uint_as_float(v[mt][2 * j + 1]), acc[mt][8 * h + j]);
-                        }
-                    }
+                        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                            for (int j = 0; j < 8 * H; ++j)
+                                acc[mt][j] = fmaf(s[mt], __uint_as_float(v[mt][j >> 3][2 * (j & 7)]) + __uint_as_float(v[mt][j >> 3][2 * (j & 7) + 1]), acc[mt][j]);
+                    };
+                    if (nte == 32) drain(std::true_type{}); else drain(std::false_type{});
                     if (++buf == NB) { buf = 0; pb ^= 1u; }
                 }
             }
@@ -409,23 +417,32 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             const int t0 = hsel * half, cnt = min(half, it.m - t0);
             float* o = A.out + (size_t)(it.prow + t0) * A.n_out + it.r0 + r;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < 16; ++j) {  // all results first (independent chains), then the stores
                 const float f = __shfl_sync(0xffffffffu, rs, j);
-                if (j < cnt) {
-                    const float a0 = acc[0][j] * f, a1 = acc[1][j] * f;
-                    if constexpr (!PAIR) {
-                        *o = swiglu_fast(a0, a1);
-                    } else {
-                        float* d = A.row_dst ? A.row_dst[it.prow + t0 + j] + it.r0 + r : o;  // expert parallel: the owner's (token, slot) row
-                        d[0] = a0;
-                        d[TILE_M] = a1;
+                acc[0][j] *= f;
+                acc[1][j] *= f;
+                if constexpr (!PAIR) acc[0][j] = swiglu_fast(acc[0][j], acc[1][j]);
+            }
+            if (PAIR && A.row_dst) {  // expert parallel: the owner's (token, slot) row
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (j < cnt) {
+                        float* d = A.row_dst[it.prow + t0 + j] + it.r0 + r;
+                        d[0] = acc[0][j];
+                        d[TILE_M] = acc[1][j];
                     }
-                    o += A.n_out;
-                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j, o += A.n_out)
+                    if (j < cnt) {
+                        o[0] = acc[0][j];
+                        if constexpr (PAIR) o[TILE_M] = acc[1][j];
+                    }
             }
         }
     } else if (warp < W_RAW) {
         // ---------------- producers ----------------
+        reg_dec<REG_PROD>();
         const int pw = warp - EWARPS, grp = pw >> 2, r = (pw & 3) * 32 + lane;
         const uint32_t tlane = tmem_base + A_COL0 + ((uint32_t)((pw & 3) * 32) << 16);
         const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
@@ -445,24 +462,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
                     if (!ok) break;
                     const uint8_t* raw = raw_base + rst * L::RAW_STAGE + r * R::RS;
-                    R ra, rb;
-                    ra.load(raw + (oa & 15u), grp);
-                    rb.load(raw + L::RAW_TILE + (ob & 15u), grp);
-                    if constexpr (T == T_IQ3_XXS) { oa += kBB<T>; ob += kBB<T>; }
-                    __syncwarp();
-                    if (lane == 0) mb_arrive(&rempty[rst]);
-                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
-                    if (grp == 0) {
-                        scl[(sc * 2) * TILE_M + r] = ra.scale();
-                        scl[(sc * 2 + 1) * TILE_M + r] = rb.scale();
-                        sc = (sc + 1) & (SCL - 1);
-                    }
+                    R in;
+                    in.load(raw + (oa & 15u), grp);
+                    if (grp == 0) scl[(sc * 2) * TILE_M + r] = in.scale();
                     ok = warp_all(q.wait(empty, A.status, 2));
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t ta = tlane + q.slot() * (2 * A_COLS);
-                    decode_stage(ra, grp, ta, gl, sl);
-                    decode_stage(rb, grp, ta + A_COLS, gl, sl);
+                    decode_stage(in, grp, ta, gl, sl);
+                    in.load(raw + L::RAW_TILE + (ob & 15u), grp);
+                    if (grp == 0) {
+                        scl[(sc * 2 + 1) * TILE_M + r] = in.scale();
+                        sc = (sc + 1) & (SCL - 1);
+                    }
+                    if constexpr (T == T_IQ3_XXS) { oa += kBB<T>; ob += kBB<T>; }
+                    __syncwarp();
+                    if (lane == 0) mb_arrive(&rempty[rst]);
+                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
+                    decode_stage(in, grp, ta + A_COLS, gl, sl);
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
@@ -495,6 +512,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
     } else if (warp < W_B) {
+        reg_dec<REG_RAW>();
         // ---------------- raw rows: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
         const int rw = warp - W_RAW, c16 = (lane & 7) * 16, row0 = (rw & 1) * (TILE_M / 2);  // half a tile per warp
         int rst = 0;
@@ -539,32 +557,32 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         cp_async_wait_all();
-    } else if (warp < W_MMA) {
-        // ---------------- B tiles: rows 2 t, 2 t + 1 = hi and lo of token t; lane = unit lane % 8 of row lane / 8 (+ 4 per step) ----------------
+    } else {
+        reg_dec<REG_MISC>();
+        if (warp < W_MMA) {
+        // ---------------- B tiles: rows 2 t, 2 t + 1 = hi and lo of token t; lane = unit lane % 8 of row lane / 8 (+ 8 per step, the
+        // other warp takes the four between) ----------------
         StageCount q(0);
-        int mine = warp - W_B;  // 0: the next stage is this warp's
-        const uint32_t sw0 = chunk_off(lane >> 3, lane & 7), sw1 = chunk_off(4 + (lane >> 3), lane & 7);  // rows r and r + 8 swizzle alike
+        const int brow = 4 * (warp - W_B) + (lane >> 3);
+        const uint32_t at = chunk_off(brow, lane & 7);  // rows r and r + 8 swizzle alike
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
-            const int steps = tile_tokens(it.m) / 2;  // 4 rows each
-            const uint16_t* src[16];  // operand array rows of this lane's B rows
+            const int steps = tile_tokens(it.m) / 4;  // 8 rows each
+            const uint16_t* src[8];  // operand array rows of this lane's B rows
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int br = 4 * i + (lane >> 3), pr = it.prow + min(br >> 1, it.m - 1);
+            for (int i = 0; i < 8; ++i) {
+                const int br = 8 * i + brow, pr = it.prow + min(br >> 1, it.m - 1);
                 const uint32_t orow = i < steps ? (uint32_t)(A.row_token ? A.row_token[pr] : pr) : 0u;
                 src[i] = A.op + (size_t)(2u * orow + (br & 1)) * pitch + 8 * (lane & 7);
             }
             auto stage = [&](int off) {  // off: elements from src
-                if (mine == 0) {
-                    ok = warp_all(q.wait(empty, A.status, 4));
-                    if (!ok) return;
-                    uint8_t* d = b_tile(q.slot());
+                ok = warp_all(q.wait(empty, A.status, 4));
+                if (!ok) return;
+                uint8_t* d = b_tile(q.slot()) + at;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (i < steps) cp_async16(d + ((i & 1) ? sw1 : sw0) + (i >> 1) * 1024, src[i] + off);
-                    cp_async_arrive(&full[q.slot()]);
-                }
-                mine ^= 1;
+                for (int i = 0; i < 8; ++i)
+                    if (i < steps) cp_async16(d + i * 1024, src[i] + off);
+                cp_async_arrive(&full[q.slot()]);
                 q.advance(1);
             };
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
@@ -574,14 +592,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     for (int c = 0; c < 4; ++c)
                         if (ok) stage(c * BK);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) src[i] += 256;
+                    for (int i = 0; i < 8; ++i) src[i] += 256;
                 }
                 const int sums = A.n_in - 256 * (b0 + bn) + 8 * b0;  // the mins read the sums behind the row
                 for (int u = 0; u < min_stages<T>(bn) && ok; ++u) stage(sums);
             }
         }
         cp_async_wait_all();
-    } else {
+        } else if (warp == W_MMA) {
         // ---------------- MMA issue: one thread ----------------
         if (elect_one()) {
             StageCount q(0);
@@ -624,6 +642,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         __syncwarp();
+        }
     }
     tc_fence_before();
     __syncthreads();
