@@ -23,7 +23,7 @@
 //     waits for the copies still on their way, so it is the MMA thread that executes it.)
 //   * four groups of four producer warps, group j decodes the j-th 64 elements of every block, a thread one row of both tiles;
 //     the block's scales go to a small ring.
-//   * the MMA warp; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
+//   * two MMA warps, one per tile; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
 //     once per K step.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
 // Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
@@ -49,16 +49,17 @@ constexpr int B_STAGE = 2 * NT * BK * 2;// hi and lo rows: 8 KB
 constexpr int NB = 2;                   // accumulator buffers
 constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
 constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS, RWARPS = 4, BWARPS = 2;
-constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;
-constexpr int NTHREADS = 1024;          // 32 warps, the last one idle
+constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS, MWARPS = 2;
+constexpr int NTHREADS = 1024;          // 32 warps
 // Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
 constexpr int REG_EPI = 112, REG_PROD = 56, REG_RAW = 24, REG_MISC = 40;
 static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
-static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA < 32, "roles fill warpgroups");
+static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA + MWARPS == 32, "roles fill warpgroups");
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
-constexpr int STAGES = 4;               // of the ring that A (tensor memory) and B (shared memory) share
+constexpr int STAGES = 4, BSTAGES = 8;  // rings of A (tensor memory) and of B (shared memory: its copies take over a microsecond)
 constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + STAGES * 2 * A_COLS;
+static_assert(BSTAGES == 2 * STAGES, "a stage number names its B slot");
 static_assert(TMEM_COLS == 512, "tensor memory");
 constexpr int SCL = 8;                  // ring of block scales: producers are at most NB + 3 blocks ahead of the epilogue
 constexpr uint32_t kMinScaleH = 0x4C004C00u;  // the mins' A values are 16 times the mins: their low halves then lose nothing that matters
@@ -242,15 +243,14 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {  // an arrival 
 }
 template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Shared memory: [barriers, segment table, items][block scales][two B stages][IQ3_XXS tables at a 32 KB boundary][two B stages][raw ring]
+// Shared memory: [barriers, segment table, items][block scales][B ring][IQ3_XXS tables at a 32 KB boundary][raw ring]
 template <int T> struct Layout {
     static constexpr int RSTAGES = 3;
     static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
-    static constexpr int LOW_B = 2;
-    static constexpr int BARS = 3 * STAGES + 2 * (RSTAGES + NB);
+    static constexpr int BARS = 3 * STAGES + BSTAGES + 2 * (RSTAGES + NB);
     static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
     static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
-    static constexpr int TAIL = (STAGES - LOW_B) * B_STAGE + RSTAGES * RAW_STAGE;
+    static constexpr int TAIL = RSTAGES * RAW_STAGE;
 };
 
 // A stage number as its user sees it.  A group's stages are up to six apart and the groups may be a block apart from one another:
@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (s32(smem_raw) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(base);
-    uint64_t* empty = full + STAGES;          // two per slot, see the producers
+    uint64_t* bfull = full + STAGES;
+    uint64_t* empty = bfull + BSTAGES;        // one per B slot, two per A slot
     uint64_t* rfull = empty + 2 * STAGES;
     uint64_t* rempty = rfull + L::RSTAGES;
     uint64_t* tfull = rempty + L::RSTAGES;
@@ -286,20 +287,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     int* pre = reinterpret_cast<int*>(tmem_slot + 4);  // [nseg + 1] first token tile of a segment
     Item* itab = reinterpret_cast<Item*>((reinterpret_cast<uintptr_t>(pre + kMaxSeg + 1) + 7) & ~(uintptr_t)7);
     float* scl = reinterpret_cast<float*>(base + L::HEAD);  // [SCL][2][128]
-    uint8_t* b_low = base + L::LOW;
-    uint8_t* p = b_low + L::LOW_B * B_STAGE;
+    uint8_t* b_ring = base + L::LOW;
+    uint8_t* p = b_ring + BSTAGES * B_STAGE;
     uint8_t* book = p;
     if constexpr (T == T_IQ3_XXS) {
         book += (kMmBookAlign - (s32(p) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
         p = book + sizeof(MmCodebook);
     }
-    uint8_t* b_high = p;
-    uint8_t* raw_base = b_high + (STAGES - L::LOW_B) * B_STAGE;
-    if ((uint32_t)(b_high + L::TAIL - smem_raw) > A.smem) {  // only if shared memory started elsewhere
+    uint8_t* raw_base = p;
+    if ((uint32_t)(raw_base + L::TAIL - smem_raw) > A.smem) {  // only if shared memory started elsewhere
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
     }
-    auto b_tile = [&](int st) { return st < L::LOW_B ? b_low + st * B_STAGE : b_high + (st - L::LOW_B) * B_STAGE; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nblk = A.n_in / 256;
@@ -307,10 +306,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 4 + BWARPS * 32);    // a producer group's warps, the B warps' lanes
-        for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], 1);    // a commit
+        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 4);                 // a producer group's warps
+        for (int i = 0; i < BSTAGES; ++i) mb_init(&bfull[i], BWARPS * 32);     // the B warps' lanes
+        for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], MWARPS);       // a commit per tile
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
-        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
+        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], MWARPS); mb_init(&tfree[i], EWARPS); }
         fence_mbarrier_init();
     }
     if constexpr (T == T_IQ3_XXS) {
@@ -576,21 +576,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                 src[i] = A.op + (size_t)(2u * orow + (br & 1)) * pitch + 8 * (lane & 7);
             }
             auto stage = [&](int off) {  // off: elements from src
-                ok = warp_all(q.wait(empty, A.status, 4));
+                ok = warp_all(mb_wait(&empty[q.q], q.turn ^ 1u, A.status, 4));  // BSTAGES stages earlier
                 if (!ok) return;
-                uint8_t* d = b_tile(q.slot()) + at;
+                uint8_t* d = b_ring + q.q * B_STAGE + at;
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (i < steps) cp_async16(d + i * 1024, src[i] + off);
-                cp_async_arrive(&full[q.slot()]);
+                cp_async_arrive(&bfull[q.q]);
                 q.advance(1);
             };
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
                 for (int b = 0; b < bn && ok; ++b) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-                        if (ok) stage(c * BK);
+#pragma unroll 1
+                    for (int c = 0; c < 4 && ok; ++c) stage(c * BK);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) src[i] += 256;
                 }
@@ -599,49 +598,50 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         cp_async_wait_all();
-        } else if (warp == W_MMA) {
-        // ---------------- MMA issue: one thread ----------------
-        if (elect_one()) {
-            StageCount q(0);
-            int buf = 0;
-            uint32_t pf = 1u;
-            for (int k = 0; k < my_items && ok; ++k) {
-                const Item it = item(k);
-                const int nte = tile_tokens(it.m);
-                const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
-                for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
-                    const int bn = min(8, nblk - b0);
-                    // one block: `stages` stages of `live` K steps (mins: the K steps that hold sub-blocks; hi and lo side by side when both fit)
-                    auto block = [&](int stages, int live, bool pair) {
-                        ok = mb_wait(&tfree[buf], pf, A.status, 6);
-                        const uint32_t d0 = tmem_base + (uint32_t)(buf * BUF_COLS);
-                        uint32_t acc = 0u;
-                        for (int c = 0; c < stages && ok; ++c) {
-                            ok = mb_wait(&full[q.slot()], q.q < STAGES ? 0u : 1u, A.status, 5);  // a slot has two turns in the count
-                            if (!ok) break;
-                            tc_fence_after();    // A: written to tensor memory by the producers
-                            fence_async_smem();  // B: written to shared memory by the B warps' copies
-                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(q.slot() * 2 * A_COLS), b_lo = desc_lo(s32(b_tile(q.slot())));
+        } else {
+        // ---------------- MMA issue, a warp per tile ----------------
+        const int mt = warp - W_MMA;
+        const uint32_t d_tile = tmem_base + (uint32_t)(mt * 2 * NT), a_tile = tmem_base + A_COL0 + (uint32_t)(mt * A_COLS), b_lo0 = desc_lo(s32(b_ring));
+        StageCount q(0);
+        int buf = 0;
+        uint32_t pf = 1u;
+        for (int k = 0; k < my_items && ok; ++k) {
+            const int nte = tile_tokens(item(k).m);
+            const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
+            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                const int bn = min(8, nblk - b0);
+                for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0) && ok; ++b) {
+                    // a block's four stages; or those of the mins, whose K steps without sub-blocks are left out (hi and lo side by
+                    // side when both fit into one stage)
+                    const bool mins = b == bn, pair = mins && bn <= 4;
+                    const int stages = mins ? min_stages<T>(bn) : 4, live = mins ? (bn * 8 + 15) / 16 : 4;
+                    ok = warp_all(mb_wait(&tfree[buf], pf, A.status, 6));
+                    for (int c = 0; c < stages && ok; ++c) {
+                        ok = warp_all(mb_wait(&bfull[q.q], q.turn, A.status, 5) && mb_wait(&full[q.slot()], q.q < STAGES ? 0u : 1u, A.status, 5));
+                        if (!ok) break;
+                        tc_fence_after();    // A: written to tensor memory by the producers
+                        fence_async_smem();  // B: written to shared memory by the B warps' copies
+                        if (elect_one()) {
+                            const uint32_t d = d_tile + (uint32_t)(buf * BUF_COLS), ta = a_tile + (uint32_t)(q.slot() * 2 * A_COLS);
+                            const uint32_t b_lo = b_lo0 + (uint32_t)(q.q * (B_STAGE >> 4));
+                            if (live == 4) {
 #pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) {
-                                if ((pair ? ks & 1 : ks) >= live) continue;
-                                mma_f16_ta(d0, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
-                                mma_f16_ta(d0 + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
-                                acc = 1u;
+                                for (int ks = 0; ks < 4; ++ks) mma_f16_ta(d, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, c + ks);
+                            } else {
+#pragma unroll 1
+                                for (int ks = 0; ks < 4; ++ks)
+                                    if ((pair ? ks & 1 : ks) < live) mma_f16_ta(d, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, c + ks);
                             }
                             mma_commit(&empty[q.q]);
-                            q.advance(1);
+                            if (c == stages - 1) mma_commit(&tfull[buf]);
                         }
-                        if (!ok) return;
-                        mma_commit(&tfull[buf]);
-                        if (++buf == NB) { buf = 0; pf ^= 1u; }
-                    };
-                    for (int b = 0; b < bn && ok; ++b) block(4, 4, false);
-                    if (T == T_Q4_K && ok) block(min_stages<T>(bn), (bn * 8 + 15) / 16, bn <= 4);
+                        __syncwarp();
+                        q.advance(1);
+                    }
+                    if (++buf == NB) { buf = 0; pf ^= 1u; }
                 }
             }
         }
-        __syncwarp();
         }
     }
     tc_fence_before();
@@ -736,7 +736,7 @@ bool tc_handles(int type, int n_in, int n_out, bool fused) {
 template <int T, bool PAIR>
 static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
     using L = tg::Layout<T>;
-    size_t at = kMmSmemBase + L::LOW + L::LOW_B * tg::B_STAGE;
+    size_t at = kMmSmemBase + L::LOW + tg::BSTAGES * tg::B_STAGE;
     if (T == T_IQ3_XXS) at = (at + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign + sizeof(MmCodebook);
     const size_t smem = at + L::TAIL - kMmSmemBase;
     static_assert(L::BARS * 8 + 16 + (tg::kMaxSeg + 1) * 4 + 8 + tg::kLocalItems * sizeof(tg::Item) <= L::HEAD, "head too small");
