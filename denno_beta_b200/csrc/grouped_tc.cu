@@ -21,16 +21,15 @@
 //   * two warps copy the tokens' hi and lo rows into swizzled B tiles, a stage each in turn, gathered from the token-major rows:
 //     no packed copy of the activations.  (TMA row gathers took 80 cycles per four rows; a proxy fence in the copying warp
 //     waits for the copies still on their way, so it is the MMA thread that executes it.)
-//   * four groups of four producer warps, group j decodes the j-th 64 elements of every block, a thread one row of both tiles;
-//     the block's scales go to a small ring.
+//   * four groups of four producer warps, (even or odd stages) x (tile), a thread one row: decodes 64 weights into registers, THEN
+//     waits for a ring slot (tensor memory holds only four stages; with the decoding inside its turn-around a stage took 1,100
+//     cycles) and stores them.  The block's scales go to a small ring, its mins to shared memory of the thread's own.
 //   * two MMA warps, one per tile; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
 //     once per K step.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
 // Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
 #include <cuda.h>
 #include <cuda_fp16.h>
-
-#include <type_traits>
 
 #include "dnb_common.cuh"
 #include "tc_ptx.cuh"
@@ -48,11 +47,11 @@ constexpr int A_COLS = BK / 2;          // tensor-memory columns of an A tile (t
 constexpr int B_STAGE = 2 * NT * BK * 2;// hi and lo rows: 8 KB
 constexpr int NB = 2;                   // accumulator buffers
 constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
-constexpr int EWARPS = 8, GROUPS = 4, PWARPS = 4 * GROUPS, RWARPS = 4, BWARPS = 2;
+constexpr int EWARPS = 8, PWARPS = 16, RWARPS = 4, BWARPS = 2;
 constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS, MWARPS = 2;
 constexpr int NTHREADS = 1024;          // 32 warps
 // Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
-constexpr int REG_EPI = 112, REG_PROD = 56, REG_RAW = 24, REG_MISC = 40;
+constexpr int REG_EPI = 96, REG_PROD = 64, REG_RAW = 24, REG_MISC = 40;
 static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
 static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA + MWARPS == 32, "roles fill warpgroups");
 constexpr int kMaxSeg = 1055;
@@ -152,12 +151,14 @@ template <> struct Raw<T_IQ3_XXS> {  // 16 index bytes and two sub-block words f
     __device__ __forceinline__ float scale() const { return 0.25f * h2f((uint16_t)d); }
 };
 
-// A tile's row of a stage goes to tensor memory in halves of 32 elements: 16 columns.
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+// 32 columns of this thread's tensor-memory lane.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
-        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]),
-        "r"(r[13]), "r"(r[14]), "r"(r[15])
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,"
+        "%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+        "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -170,7 +171,7 @@ __device__ __forceinline__ void mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uin
         : "memory");
 }
 
-__device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint32_t taddr, uint32_t, uint32_t) {
+__device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint32_t (&o)[32], uint32_t, uint32_t) {
     const int sh = 16 * (c & 1);
     const uint32_t a = R.h.y >> sh, cc = R.h.w >> sh;
     const uint32_t sc = c < 2 ? (a & 0x3f3fu) : ((cc & 0x0f0fu) | ((a >> 2) & 0x3030u));  // kquant.rs:878-887
@@ -183,56 +184,49 @@ __device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint32
     for (int h = 0; h < 2; ++h) {
         const uint4 q = h ? R.b : R.a;
         const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-        uint32_t o[16];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             uint32_t p[4];
             k_word<false>(w[i], 0u, s, p);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o[4 * i + j] = p[j];
+            for (int j = 0; j < 4; ++j) o[16 * h + 4 * i + j] = p[j];
         }
-        tmem_st16(taddr + 16 * h, o);
     }
 }
-__device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int, uint32_t taddr, uint32_t gl, uint32_t sl) {
+__device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int, uint32_t (&o)[32], uint32_t gl, uint32_t sl) {
 #pragma unroll
     for (int hb = 0; hb < 2; ++hb) {
         const uint32_t aux = __funnelshift_r(R.x[hb], R.x[hb + 1], R.sh);
         const uint32_t s2 = h2sub((((aux >> 27) & 0x1Eu) | 0x6401u) * 0x10001u, 0x64006400u);  // 2 s + 1 in both halves
-        uint32_t o[16];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t iw = __funnelshift_r(R.i[2 * hb + (q >> 1)], R.i[2 * hb + (q >> 1) + 1], R.sh) >> (16 * (q & 1));
             uint32_t p[4];
             iq3_pairs_h(gl, sl, iw, q == 0 ? aux << 6 : aux >> (7 * q - 6), p);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o[4 * q + j] = h2mul(p[j], s2);
+            for (int j = 0; j < 4; ++j) o[16 * hb + 4 * q + j] = h2mul(p[j], s2);
         }
-        tmem_st16(taddr + 16 * hb, o);
     }
 }
-// Stage u of the mins of one Q4_K row; raw: the row's headers of `blocks` blocks, 16 bytes each.
-__device__ __forceinline__ void mins_stage(const uint8_t* raw, int blocks, int u, uint32_t taddr) {
+// Stage u of the mins of one Q4_K row.  mm, dd: the last eight mins bytes of each block's header and its dmin, as the thread saved
+// them (PWARPS * 32 entries from block to block).
+__device__ __forceinline__ void mins_stage(const uint2* mm, const uint16_t* dd, int blocks, int u, uint32_t (&o)[32]) {
     const bool both = blocks <= 4;
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-        const bool low = both ? half != 0 : u != 0;
-        uint32_t o[16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {  // the eight sub-blocks of a block: four columns
-            const int blk = both ? c : 4 * half + c;
-            const bool live = blk < blocks;
-            const uint4 h = *reinterpret_cast<const uint4*>(raw + 16 * (live ? blk : 0));
-            const uint32_t dm = live ? h2mul(__byte_perm(h.x, 0u, 0x3232u), kMinScaleH ^ 0x80008000u) : 0u;  // -16 * dmin
-            const uint32_t mn[2] = {h.z & 0x3f3f3f3fu, ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u)};  // kquant.rs:878-887
+    for (int c = 0; c < 8; ++c) {  // the eight sub-blocks of a block: four columns
+        const bool low = both ? c >= 4 : u != 0;
+        const int blk = both ? c & 3 : c;
+        const bool live = blk < blocks;
+        const uint2 h = mm[(live ? blk : 0) * PWARPS * 32];
+        const uint32_t d = live ? dd[blk * PWARPS * 32] : 0u;
+        const uint32_t dm = h2mul(d * 0x10001u, kMinScaleH ^ 0x80008000u);  // -16 * dmin
+        const uint32_t mn[2] = {h.x & 0x3f3f3f3fu, ((h.y >> 4) & 0x0f0f0f0fu) | ((h.x >> 2) & 0x30303030u)};  // kquant.rs:878-887
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {  // sub-blocks 2 k, 2 k + 1: dmin * m rounded, or exactly what that left over
-                const uint32_t m2 = h2sub(__byte_perm(mn[k >> 1], 0x64646464u, (k & 1) ? 0x4342u : 0x4140u), 0x64006400u);
-                const uint32_t hi = h2mul(dm, m2);
-                o[4 * c + k] = low ? h2fma(dm, m2, hi ^ 0x80008000u) : hi;
-            }
+        for (int k = 0; k < 4; ++k) {  // sub-blocks 2 k, 2 k + 1: dmin * m rounded, or exactly what that left over
+            const uint32_t m2 = h2sub(__byte_perm(mn[k >> 1], 0x64646464u, (k & 1) ? 0x4342u : 0x4140u), 0x64006400u);
+            const uint32_t hi = h2mul(dm, m2);
+            o[4 * c + k] = low ? h2fma(dm, m2, hi ^ 0x80008000u) : hi;
         }
-        tmem_st16(taddr + 16 * half, o);
     }
 }
 
@@ -243,14 +237,15 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {  // an arrival 
 }
 template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Shared memory: [barriers, segment table, items][block scales][B ring][IQ3_XXS tables at a 32 KB boundary][raw ring]
+// Shared memory: [barriers, segment table, items][block scales][B ring][IQ3_XXS tables at a 32 KB boundary][raw ring][Q4_K: mins]
 template <int T> struct Layout {
     static constexpr int RSTAGES = 3;
     static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
     static constexpr int BARS = 3 * STAGES + BSTAGES + 2 * (RSTAGES + NB);
     static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
     static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
-    static constexpr int TAIL = RSTAGES * RAW_STAGE;
+    static constexpr int MINS = T == T_Q4_K ? PWARPS * 32 * 8 * 10 : 0;  // 8 + 2 bytes per block and producer thread
+    static constexpr int TAIL = RSTAGES * RAW_STAGE + MINS;
 };
 
 // A stage number as its user sees it.  A group's stages are up to six apart and the groups may be a block apart from one another:
@@ -306,7 +301,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 4);                 // a producer group's warps
+        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 8);                 // two producer groups' warps, a tile each
         for (int i = 0; i < BSTAGES; ++i) mb_init(&bfull[i], BWARPS * 32);     // the B warps' lanes
         for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], MWARPS);       // a commit per tile
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
@@ -392,24 +387,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         sc = (sc + 1) & (SCL - 1);
                     }
                     const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * nte);
-                    auto drain = [&](auto full_tile) {  // eight tokens a load and tile; 32-token tiles have sixteen per warp
-                        constexpr int H = decltype(full_tile)::value ? 2 : 1;
-                        uint32_t v[2][H][16];
 #pragma unroll
-                        for (int mt = 0; mt < 2; ++mt)
+                    for (int h = 0; h < 2; ++h) {  // eight tokens a load; 32-token tiles have sixteen per warp
+                        if (h == 0 || nte == 32) {
+                            uint32_t v[2][16];
+                            tmem_ld16(col + 16 * h, v[0]);
+                            tmem_ld16(col + 2 * NT + 16 * h, v[1]);
+                            tmem_ld_wait();
+                            if (h == 1 || nte != 32) {  // read: hand the buffer back before the arithmetic
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mb_arrive(&tfree[buf]);
+                            }
 #pragma unroll
-                            for (int h = 0; h < H; ++h) tmem_ld16(col + mt * 2 * NT + 16 * h, v[mt][h]);
-                        tmem_ld_wait();
-                        tc_fence_before();  // read: hand the buffer back before the arithmetic
-                        __syncwarp();
-                        if (lane == 0) mb_arrive(&tfree[buf]);
+                            for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-                        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                            for (int j = 0; j < 8 * H; ++j)
-                                acc[mt][j] = fmaf(s[mt], __uint_as_float(v[mt][j >> 3][2 * (j & 7)]) + __uint_as_float(v[mt][j >> 3][2 * (j & 7) + 1]), acc[mt][j]);
-                    };
-                    if (nte == 32) drain(std::true_type{}); else drain(std::false_type{});
+                                for (int j = 0; j < 8; ++j)
+                                    acc[mt][8 * h + j] =
+                                        fmaf(s[mt], __uint_as_float(v[mt][2 * j]) + __uint_as_float(v[mt][2 * j + 1]), acc[mt][8 * h + j]);
+                        }
+                    }
                     if (++buf == NB) { buf = 0; pb ^= 1u; }
                 }
             }
@@ -443,70 +440,69 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     } else if (warp < W_RAW) {
         // ---------------- producers ----------------
         reg_dec<REG_PROD>();
-        const int pw = warp - EWARPS, grp = pw >> 2, r = (pw & 3) * 32 + lane;
-        const uint32_t tlane = tmem_base + A_COL0 + ((uint32_t)((pw & 3) * 32) << 16);
+        const int pw = warp - EWARPS, odd = pw >> 3, tile = (pw >> 2) & 1, r = (pw & 3) * 32 + lane;
+        const uint32_t tlane = tmem_base + A_COL0 + (uint32_t)(tile * A_COLS) + ((uint32_t)((pw & 3) * 32) << 16);
         const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
+        uint2* mm = reinterpret_cast<uint2*>(raw_base + L::RSTAGES * L::RAW_STAGE) + pw * 32 + lane;
+        uint16_t* dd = reinterpret_cast<uint16_t*>(raw_base + L::RSTAGES * L::RAW_STAGE + PWARPS * 32 * 8 * 8) + pw * 32 + lane;
         int rst = 0, sc = 0;
         uint32_t rph = 0u;
-        StageCount q(grp);
+        StageCount q(odd);
+        auto hand_over = [&](const uint32_t (&o)[32]) {  // into the ring slot of stage q
+            ok = warp_all(q.wait(empty, A.status, 2));
+            if (!ok) return;
+            tc_fence_after();
+            tmem_st32(tlane + q.slot() * (2 * A_COLS), o);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mb_arrive(&full[q.slot()]);
+        };
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
-            uint32_t oa = 0, ob = 0;  // where the two rows' blocks start within 16 bytes
-            if constexpr (T == T_IQ3_XXS) {
-                oa = (uint32_t)(uintptr_t)it.pa + (uint32_t)r * A.rb;
-                ob = (uint32_t)(uintptr_t)it.pb + (uint32_t)r * A.rb;
-            }
+            uint32_t off = 0;  // where the row's block starts within 16 bytes
+            if constexpr (T == T_IQ3_XXS) off = (uint32_t)(uintptr_t)(tile ? it.pb : it.pa) + (uint32_t)r * A.rb;
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
                 for (int b = 0; b < bn; ++b) {
                     ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
                     if (!ok) break;
-                    const uint8_t* raw = raw_base + rst * L::RAW_STAGE + r * R::RS;
-                    R in;
-                    in.load(raw + (oa & 15u), grp);
-                    if (grp == 0) scl[(sc * 2) * TILE_M + r] = in.scale();
-                    ok = warp_all(q.wait(empty, A.status, 2));
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t ta = tlane + q.slot() * (2 * A_COLS);
-                    decode_stage(in, grp, ta, gl, sl);
-                    in.load(raw + L::RAW_TILE + (ob & 15u), grp);
-                    if (grp == 0) {
-                        scl[(sc * 2 + 1) * TILE_M + r] = in.scale();
-                        sc = (sc + 1) & (SCL - 1);
+                    const uint8_t* raw = raw_base + rst * L::RAW_STAGE + tile * L::RAW_TILE + r * R::RS + (off & 15u);
+                    if constexpr (T == T_IQ3_XXS) off += kBB<T>;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        R in;
+                        in.load(raw, odd + 2 * h);
+                        if (h == 0) {
+                            if (!odd) {
+                                scl[(sc * 2 + tile) * TILE_M + r] = in.scale();
+                                sc = (sc + 1) & (SCL - 1);
+                            }
+                            if constexpr (T == T_Q4_K) {
+                                mm[b * PWARPS * 32] = make_uint2(in.h.z, in.h.w);
+                                dd[b * PWARPS * 32] = (uint16_t)(in.h.x >> 16);
+                            }
+                        } else {
+                            __syncwarp();
+                            if (lane == 0) mb_arrive(&rempty[rst]);
+                            if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
+                        }
+                        uint32_t o[32];
+                        decode_stage(in, odd + 2 * h, o, gl, sl);
+                        hand_over(o);
+                        if (!ok) break;
+                        q.advance(2);
                     }
-                    if constexpr (T == T_IQ3_XXS) { oa += kBB<T>; ob += kBB<T>; }
-                    __syncwarp();
-                    if (lane == 0) mb_arrive(&rempty[rst]);
-                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
-                    decode_stage(in, grp, ta + A_COLS, gl, sl);
-                    tmem_st_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mb_arrive(&full[q.slot()]);
-                    q.advance(4);
+                    if (!ok) break;
                 }
                 if (!ok) break;
-                if constexpr (T == T_Q4_K) {  // the mins: group u builds stage u; then every group is `nm` stages on
+                if constexpr (T == T_Q4_K) {
                     const int nm = min_stages<T>(bn);
-                    ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
-                    if (!ok) break;
-                    if (grp < nm) {
-                        ok = warp_all(q.wait(empty, A.status, 2));
-                        if (!ok) break;
-                        tc_fence_after();
-                        const uint32_t ta = tlane + q.slot() * (2 * A_COLS);
-                        const uint8_t* raw = raw_base + rst * L::RAW_STAGE + r * R::RS;
-                        mins_stage(raw, bn, grp, ta);
-                        mins_stage(raw + L::RAW_TILE, bn, grp, ta + A_COLS);
-                        tmem_st_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mb_arrive(&full[q.slot()]);
+                    if (odd < nm) {
+                        uint32_t o[32];
+                        mins_stage(mm, dd, bn, odd, o);
+                        hand_over(o);
                     }
-                    __syncwarp();
-                    if (lane == 0) mb_arrive(&rempty[rst]);
-                    if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
                     q.advance(nm);
                 }
             }
@@ -522,34 +518,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             const uint8_t* half = ((rw & 2) ? it.pb : it.pa) + (size_t)row0 * A.rb;
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
-                for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0); ++b) {
+                for (int b = 0; b < bn; ++b) {
                     ok = warp_all(mb_wait(&rempty[rst], rph, A.status, 8));
                     if (!ok) break;
                     uint8_t* dst = raw_base + rst * L::RAW_STAGE + ((rw & 2) ? L::RAW_TILE : 0) + row0 * R::RS;
                     const uint32_t step = 4u * A.rb;
-                    if (b < bn) {
-                        const uint8_t* src = half + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
-                        uint8_t* d = dst + (lane >> 3) * R::RS + c16;
+                    const uint8_t* src = half + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
+                    uint8_t* d = dst + (lane >> 3) * R::RS + c16;
 #pragma unroll
-                        for (int i = 0; i < TILE_M / 8; ++i, src += step) {
-                            if constexpr (T == T_Q4_K) {
-                                cp_async16(d + i * 4 * R::RS, src + c16);
-                            } else {
-                                const uint8_t* s16 = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
-                                if (c16 < R::UNITS * 16) cp_async16(d + i * 4 * R::RS, s16 + c16);
-                            }
-                        }
+                    for (int i = 0; i < TILE_M / 8; ++i, src += step) {
                         if constexpr (T == T_Q4_K) {
-                            const uint8_t* s9 = half + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
-#pragma unroll
-                            for (int i = 0; i < TILE_M / 64; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
+                            cp_async16(d + i * 4 * R::RS, src + c16);
+                        } else {
+                            const uint8_t* s16 = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
+                            if (c16 < R::UNITS * 16) cp_async16(d + i * 4 * R::RS, s16 + c16);
                         }
-                    } else if constexpr (T == T_Q4_K) {  // the headers of the last bn blocks: lane = block lane % 8
-                        const uint8_t* src = half + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + (lane & 7)) * kBB<T>;
-                        if ((lane & 7) < bn) {
+                    }
+                    if constexpr (T == T_Q4_K) {
+                        const uint8_t* s9 = half + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
 #pragma unroll
-                            for (int i = 0; i < TILE_M / 8; ++i, src += step) cp_async16(dst + ((lane >> 3) + 4 * i) * R::RS + c16, src);
-                        }
+                        for (int i = 0; i < TILE_M / 64; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
                     }
                     cp_async_arrive(&rfull[rst]);
                     if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
