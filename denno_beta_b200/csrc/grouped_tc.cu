@@ -24,7 +24,7 @@
 //   * four groups of four producer warps, (even or odd stages) x (tile), a thread one row: decodes 64 weights into registers, THEN
 //     waits for a ring slot (tensor memory holds only four stages; with the decoding inside its turn-around a stage took 1,100
 //     cycles) and stores them.  The block's scales go to a small ring, its mins to shared memory of the thread's own.
-//   * two MMA warps, one per tile; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
+//   * one MMA thread; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
 //     once per K step.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
 // Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
@@ -48,12 +48,12 @@ constexpr int B_STAGE = 2 * NT * BK * 2;// hi and lo rows: 8 KB
 constexpr int NB = 2;                   // accumulator buffers
 constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
 constexpr int EWARPS = 8, PWARPS = 16, RWARPS = 4, BWARPS = 2;
-constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS, MWARPS = 2;
-constexpr int NTHREADS = 1024;          // 32 warps
+constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;
+constexpr int NTHREADS = 1024;          // 32 warps, the last one idle
 // Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
 constexpr int REG_EPI = 96, REG_PROD = 64, REG_RAW = 24, REG_MISC = 40;
 static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
-static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA + MWARPS == 32, "roles fill warpgroups");
+static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA == 30, "roles fill warpgroups");
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
 constexpr int STAGES = 4, BSTAGES = 8;  // rings of A (tensor memory) and of B (shared memory: its copies take over a microsecond)
@@ -303,9 +303,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     if (tid == 0) {
         for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 8);                 // two producer groups' warps, a tile each
         for (int i = 0; i < BSTAGES; ++i) mb_init(&bfull[i], BWARPS * 32);     // the B warps' lanes
-        for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], MWARPS);       // a commit per tile
+        for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], 1);            // a commit
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
-        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], MWARPS); mb_init(&tfree[i], EWARPS); }
+        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
         fence_mbarrier_init();
     }
     if constexpr (T == T_IQ3_XXS) {
@@ -586,51 +586,49 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         cp_async_wait_all();
-        } else {
-        // ---------------- MMA issue, a warp per tile ----------------
-        const int mt = warp - W_MMA;
-        const uint32_t d_tile = tmem_base + (uint32_t)(mt * 2 * NT), a_tile = tmem_base + A_COL0 + (uint32_t)(mt * A_COLS), b_lo0 = desc_lo(s32(b_ring));
-        StageCount q(0);
-        int buf = 0;
-        uint32_t pf = 1u;
-        for (int k = 0; k < my_items && ok; ++k) {
-            const int nte = tile_tokens(item(k).m);
-            const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
-            for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
-                const int bn = min(8, nblk - b0);
-                for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0) && ok; ++b) {
-                    // a block's four stages; or those of the mins, whose K steps without sub-blocks are left out (hi and lo side by
-                    // side when both fit into one stage)
-                    const bool mins = b == bn, pair = mins && bn <= 4;
-                    const int stages = mins ? min_stages<T>(bn) : 4, live = mins ? (bn * 8 + 15) / 16 : 4;
-                    ok = warp_all(mb_wait(&tfree[buf], pf, A.status, 6));
-                    for (int c = 0; c < stages && ok; ++c) {
-                        ok = warp_all(mb_wait(&bfull[q.q], q.turn, A.status, 5) && mb_wait(&full[q.slot()], q.q < STAGES ? 0u : 1u, A.status, 5));
-                        if (!ok) break;
-                        tc_fence_after();    // A: written to tensor memory by the producers
-                        fence_async_smem();  // B: written to shared memory by the B warps' copies
-                        if (elect_one()) {
-                            const uint32_t d = d_tile + (uint32_t)(buf * BUF_COLS), ta = a_tile + (uint32_t)(q.slot() * 2 * A_COLS);
-                            const uint32_t b_lo = b_lo0 + (uint32_t)(q.q * (B_STAGE >> 4));
-                            if (live == 4) {
+        } else if (warp == W_MMA && elect_one()) {
+            // ---------------- MMA issue: one thread ----------------
+            const uint32_t b_lo0 = desc_lo(s32(b_ring));
+            StageCount q(0);
+            int buf = 0;
+            uint32_t pf = 1u;
+            for (int k = 0; k < my_items && ok; ++k) {
+                const int nte = tile_tokens(item(k).m);
+                const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
+                for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
+                    const int bn = min(8, nblk - b0);
+                    for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0) && ok; ++b) {
+                        // a block's four stages; or those of the mins, whose K steps without sub-blocks are left out (hi and lo side
+                        // by side when both fit into one stage)
+                        const bool mins = b == bn, pair = mins && bn <= 4;
+                        const int stages = mins ? min_stages<T>(bn) : 4, live = mins ? (bn * 8 + 15) / 16 : 4;
+                        ok = mb_wait(&tfree[buf], pf, A.status, 6);
+                        const uint32_t d = tmem_base + (uint32_t)(buf * BUF_COLS);
+                        for (int c = 0; c < stages && ok; ++c) {
+                            ok = mb_wait(&bfull[q.q], q.turn, A.status, 5) && mb_wait(&full[q.slot()], q.q < STAGES ? 0u : 1u, A.status, 5);
+                            if (!ok) break;
+                            tc_fence_after();    // A: written to tensor memory by the producers
+                            fence_async_smem();  // B: written to shared memory by the B warps' copies
+                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(q.slot() * 2 * A_COLS), b_lo = b_lo0 + (uint32_t)(q.q * (B_STAGE >> 4));
+                            uint32_t acc = c == 0 ? 0u : 1u;
 #pragma unroll
-                                for (int ks = 0; ks < 4; ++ks) mma_f16_ta(d, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, c + ks);
-                            } else {
-#pragma unroll 1
-                                for (int ks = 0; ks < 4; ++ks)
-                                    if ((pair ? ks & 1 : ks) < live) mma_f16_ta(d, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, c + ks);
+                            for (int ks = 0; ks < 4; ++ks) {
+                                if ((pair ? ks & 1 : ks) >= live) continue;
+                                mma_f16_ta(d, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
+                                mma_f16_ta(d + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
+                                acc = 1u;
                             }
                             mma_commit(&empty[q.q]);
-                            if (c == stages - 1) mma_commit(&tfull[buf]);
+                            q.advance(1);
                         }
-                        __syncwarp();
-                        q.advance(1);
+                        if (!ok) break;
+                        mma_commit(&tfull[buf]);
+                        if (++buf == NB) { buf = 0; pf ^= 1u; }
                     }
-                    if (++buf == NB) { buf = 0; pf ^= 1u; }
                 }
             }
         }
-        }
+        __syncwarp();
     }
     tc_fence_before();
     __syncthreads();
