@@ -514,6 +514,11 @@ int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, 
     return launch_seg_matmul(c, st, L.m[5].type, false, w.seg_sh_dn, nullptr, 1, sff, M.e, w.sact, sff, nullptr, out, rows);
 }
 
+void forget_graphs(dnb_ctx* c) { drop_graphs(c); }
+bool moe_layer_ready(const dnb_ctx* c, int layer) { return layer_ready(c, layer, true); }
+int enqueue_block(dnb_ctx* c, int layer, const float* h, int nt, float* out) { return block_dev(c, layer, h, nt, out); }
+cudaError_t wait_for_stream(cudaStream_t st) { return wait_short(st); }
+
 }  // namespace dnb
 
 using namespace dnb;

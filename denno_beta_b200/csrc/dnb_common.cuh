@@ -187,6 +187,10 @@ int ensure_workspace(dnb_ctx* c, int nt);  // device buffers of the MoE pipeline
 // Run a launch sequence directly the first time `key` is seen, capture it into a CUDA graph the second time,
 // replay it afterwards (api.cu).
 int graphed(dnb_ctx* c, const GraphKey& key, const std::function<int()>& enqueue);
+void forget_graphs(dnb_ctx* c);                          // captured sequences hold addresses that have changed
+bool moe_layer_ready(const dnb_ctx* c, int layer);
+int enqueue_block(dnb_ctx* c, int layer, const float* h, int nt, float* out);  // one MoE block, not graphed by itself (workspace sized)
+cudaError_t wait_for_stream(cudaStream_t st);            // polls for a while before it blocks
 
 struct ProfScope {
     dnb_ctx* c; cudaStream_t st; cudaEvent_t b = nullptr;
