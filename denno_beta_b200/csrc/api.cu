@@ -847,6 +847,11 @@ static int gemv_dev(dnb_ctx* c, int type, const uint8_t* w, int k, int n, const 
         return DNB_OK;
     }
     const SegDesc sd{w, nullptr, (uint32_t)nvec, 0u};
+    if (c->decode_fast) {
+        int rc = launch_gemv_mma(c, c->stream, type, w, k, n, x, out, nvec);
+        if (rc == DNB_DECLINED) rc = launch_mm(c, c->stream, type, false, 3, nullptr, nullptr, 1, 1, nvec, k, n, x, k, nullptr, out, &sd, "mm_vectors");
+        if (rc != DNB_DECLINED) return rc;
+    }
     if (nvec == 1 && c->decode_fast && (((uintptr_t)w) & 15) == 0) {
         const int rc = launch_seg_gemv_m1(c, c->stream, type, false, true, nullptr, nullptr, 1, k, n, x, k, nullptr, out, &sd,
                                           "gemv_single");
@@ -1426,7 +1431,6 @@ int dnb_expert_rows_dev(dnb_ctx* c, int layer, const float* x_rows_dev, const in
     int rc = ensure_ws(c, rows);
     if (rc) return rc;
     Workspace& w = c->ws;
-    cudaStream_t st = c->stream;
     const bool tc_routed = !use_shared && tc_type(L, 0, 3) >= 0 && tc_handles(L.m[0].type, M.e, M.ff, true) && tc_handles(L.m[2].type, M.ff, M.e, false);
     const bool umma = c->use_umma && w.op_ok && rows >= 16;
     if (!use_shared) {

@@ -378,6 +378,9 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name);
 
+// The same arithmetic for one matrix and one or two vectors, or more where the matrix is small (grouped_mma.cu).
+int launch_gemv_mma(dnb_ctx* c, cudaStream_t st, int type, const uint8_t* w, int k, int n, const float* x, float* out, int nvec);
+
 // tcgen05 grouped GEMM of prefill (grouped_tc.cu): Q4_K and IQ3_XXS.  Its activations are operand rows: fp16 hi and lo parts,
 // tc_row_pitch(n_in) numbers each, one after the other.  launch_operand_rows makes them from fp32 rows; rows_dev (optional): the
 // device's count of rows, at most `rows`.

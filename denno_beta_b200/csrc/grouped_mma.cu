@@ -677,4 +677,255 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
     }
 }
 
+// ---- one matrix, a few vectors ---------------------------------------------------------------------------------------
+// The same arithmetic for the GEMV of a single matrix (cuda.rs:21028 maybe_gpu_gguf_gemv_into).  What bounds it: a 4096 x 4096
+// matrix is 64 KB per SM, so the time is how soon the bytes are asked for and how little follows once the vector is there; a large
+// matrix is bytes or decoding.  Hence CTAs of eight warps, two per SM (the next GEMV's CTAs come in while this one's last are at
+// work); a warp takes every ks-th block of K of 16 rows and asks for its first stages before it waits for the kernel in front of
+// it, whose output the vector may be; it converts its own blocks of the vector, each with a power of two of its own, so that no
+// CTA-wide step stands between vector and math; the warps' partial sums meet once per 16 rows, in a fixed order.
+constexpr int kGvWarps = 8;
+constexpr int kGvPart = 576;  // bytes of a part of a block: 512, its sub-block sums (16), and padding that spreads neighbouring parts over the banks
+
+struct GvArgs {
+    const uint8_t* w;
+    const float* x;      // [tok][k]
+    float* out;          // [tok][n]
+    int k, n, rb, ks, nst;
+    int nvec;            // a grid row takes TOK of them
+    uint32_t smem;
+    int* status;
+};
+
+template <int T, int TOK>
+__global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const GvArgs A) {
+    using Q = Mq<T>;
+    constexpr int STAGE = 16 * Q::RS, XB = TOK * 3 * kGvPart;  // bytes of a converted block
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int nb = A.k >> 8, nslot = kGvWarps / A.ks, slot = warp / A.ks, kw = warp - slot * A.ks;
+    const int kbn = (nb - kw + A.ks - 1) / A.ks, kb_max = (nb + A.ks - 1) / A.ks;  // this warp's blocks: kw, kw + ks, ...
+    float* red = reinterpret_cast<float*>(smem);                                   // [2][8 warps][16 rows][TOK]
+    float* inv = red + 2 * kGvWarps * 16 * TOK + warp * kb_max * TOK;              // [blocks][TOK] what undoes a block's scaling
+    uint8_t* p = smem + ((2 * kGvWarps * 16 * TOK + kGvWarps * kb_max * TOK) * 4 + 127) / 128 * 128;
+    uint8_t* xs = p + (size_t)warp * kb_max * XB;
+    p += (size_t)kGvWarps * kb_max * XB;
+    uint8_t* book = p;
+    if constexpr (T == T_IQ3_XXS) {
+        book += (kMmBookAlign - (tcp::s32(p) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
+        p = book + sizeof(MmCodebook);
+    }
+    if (T == T_IQ3_XXS && (uint32_t)(p - smem) + kGvWarps * A.nst * STAGE > A.smem) {  // only if shared memory started elsewhere
+        if (tid == 0) status_set(A.status, 26);
+        return;
+    }
+    uint8_t* ring = p + (size_t)warp * A.nst * STAGE;
+    const int n_rg = (A.n + 15) / 16, last = A.n - 1, rg_step = gridDim.x * nslot;
+    const int rounds = (n_rg - (int)blockIdx.x * nslot + rg_step - 1) / rg_step;  // of the CTA; a slot's last one may be empty
+    const int rg0 = blockIdx.x * nslot + slot;
+    const int nrg = rg0 < n_rg ? (n_rg - rg0 + rg_step - 1) / rg_step : 0, nstage = nrg * kbn;
+
+    // ---- weight stream (as in mm_kernel) ----
+    int pf_rg = rg0, pf_b = 0, pf_s = 0, pf_n = 0;
+    const int r_in = lane >> 3, c16 = (lane & 7) * 16;
+    constexpr bool TAIL = Q::ALIGNED && Q::UNITS % 8 == 1;
+    const uint8_t *sa = nullptr, *stl = nullptr;
+    uint32_t o1 = 0, o2 = 0, o3 = 0;
+    auto point = [&]() {
+        const int row = pf_rg * 16 + r_in, r0 = min(row, last);
+        sa = A.w + (size_t)r0 * A.rb + (uint32_t)kw * Q::BB;
+        o1 = (uint32_t)(min(row + 4, last) - r0) * A.rb;
+        o2 = (uint32_t)(min(row + 8, last) - r0) * A.rb;
+        o3 = (uint32_t)(min(row + 12, last) - r0) * A.rb;
+        if constexpr (TAIL) stl = A.w + (size_t)min(pf_rg * 16 + (lane & 15), last) * A.rb + (uint32_t)kw * Q::BB + (Q::UNITS - 1) * 16;
+    };
+    if (nstage > 0) point();
+    auto prefetch = [&]() {
+        if (pf_n < nstage) {
+            uint8_t* dst = ring + pf_s * STAGE + r_in * Q::RS + c16;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint8_t* src = sa + (j == 0 ? 0u : j == 1 ? o1 : j == 2 ? o2 : o3);
+                if constexpr (!Q::ALIGNED) src = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
+#pragma unroll
+                for (int cc = 0; cc < (TAIL ? Q::UNITS - 1 : Q::UNITS); cc += 8)
+                    if (cc + 8 <= Q::UNITS || cc * 16 + c16 < Q::UNITS * 16) tcp::cp_async16(dst + j * 4 * Q::RS + cc * 16, src + cc * 16 + c16);
+            }
+            if constexpr (TAIL) {
+                if (lane < 16) tcp::cp_async16(ring + pf_s * STAGE + lane * Q::RS + (Q::UNITS - 1) * 16, stl);
+                stl += A.ks * Q::BB;
+            }
+            ++pf_n;
+            sa += A.ks * Q::BB;
+            if (++pf_b == kbn) {
+                pf_b = 0;
+                pf_rg += rg_step;
+                if (pf_n < nstage) point();
+            }
+            if (++pf_s == A.nst) pf_s = 0;
+        }
+        tcp::cp_async_commit();
+    };
+    for (int i = 1; i < A.nst; ++i) prefetch();
+    if constexpr (T == T_IQ3_XXS) {  // in the last of those groups' shadow: waited for with the first stage
+        for (int i = tid; i < (int)(sizeof(MmCodebook) / 16); i += kGvWarps * 32)
+            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_codebook) + 16 * i);
+        tcp::cp_async_commit();
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+
+    // ---- this warp's blocks of the vectors ----
+    const int v0 = blockIdx.y * TOK;
+    for (int i = 0; i < kbn; ++i) {
+#pragma unroll
+        for (int q = 0; q < TOK; ++q) {
+            const float* xr = A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (kw + i * A.ks) * 256;
+            int e0, e1;
+            mm_unit_elems<T>(g, t, e0, e1);  // lane = 4 * unit + quarter
+            float4 xa = *reinterpret_cast<const float4*>(xr + e0), xb = *reinterpret_cast<const float4*>(xr + e1);
+            uint32_t mx = max(max(__float_as_uint(fabsf(xa.x)), __float_as_uint(fabsf(xa.y))), max(__float_as_uint(fabsf(xa.z)), __float_as_uint(fabsf(xa.w))));
+            mx = max(mx, max(max(__float_as_uint(fabsf(xb.x)), __float_as_uint(fabsf(xb.y))), max(__float_as_uint(fabsf(xb.z)), __float_as_uint(fabsf(xb.w)))));
+            const float s = mm_row_scale(__reduce_max_sync(0xffffffffu, mx));
+            if (lane == 0) inv[i * TOK + q] = __uint_as_float((254u << 23) - __float_as_uint(s));
+            xa.x *= s; xa.y *= s; xa.z *= s; xa.w *= s;
+            xb.x *= s; xb.y *= s; xb.z *= s; xb.w *= s;
+            uint32_t h[4][3];
+            if constexpr (mq_mins<T>) {
+                mm_split<3>(xa.x, xa.z, h[0]);
+                mm_split<3>(xa.y, xa.w, h[1]);
+                mm_split<3>(xb.x, xb.z, h[2]);
+                mm_split<3>(xb.y, xb.w, h[3]);
+            } else {
+                mm_split<3>(xa.x, xa.y, h[0]);
+                mm_split<3>(xa.z, xa.w, h[1]);
+                mm_split<3>(xb.x, xb.y, h[2]);
+                mm_split<3>(xb.z, xb.w, h[3]);
+            }
+            uint8_t* col = xs + i * XB + q * 3 * kGvPart;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) *reinterpret_cast<uint4*>(col + c * kGvPart + lane * 16) = make_uint4(h[0][c], h[1][c], h[2][c], h[3][c]);
+            if constexpr (mq_mins<T>) {
+                float a = (xa.x + xa.y) + (xa.z + xa.w), b = (xb.x + xb.y) + (xb.z + xb.w);
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    a += __shfl_xor_sync(0xffffffffu, a, o);
+                    b += __shfl_xor_sync(0xffffffffu, b, o);
+                }
+                uint32_t sp[3];
+                mm_split<3>(a, b, sp);
+                if (g == 0) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(col + c * kGvPart + 512 + t * 4) = sp[c];
+                }
+            }
+        }
+    }
+    if constexpr (T == T_IQ3_XXS) {  // the tables came in parts from all threads
+        tcp::cp_async_wait_all();
+        __syncthreads();
+    }
+    __syncwarp();
+
+    // ---- the row groups ----
+    const uint32_t gl = tcp::s32(book) + 8 * (lane & (kLutRep - 1)), sl = tcp::s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
+    const uint8_t* colb = xs + ((TOK == 2 ? (g >> 2) : 0) * 3 + min(g & 3, 2)) * kGvPart;
+    int q_s = 0, rg = rg0;
+    for (int rd = 0; rd < rounds; ++rd, rg += rg_step) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        if (rd < nrg) {
+            uint32_t offa = 0, offb = 0;
+            if constexpr (!Q::ALIGNED) {
+                offa = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + g, last) * A.rb + (uint32_t)kw * Q::BB;
+                offb = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + 8 + g, last) * A.rb + (uint32_t)kw * Q::BB;
+            }
+            for (int i = 0; i < kbn; ++i) {
+                if (A.nst == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+                else if (A.nst == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 2;" ::: "memory");
+                __syncwarp();
+                prefetch();
+                const uint8_t* st = ring + q_s * STAGE;
+                const uint8_t *ra = st + g * Q::RS, *rb = st + (g + 8) * Q::RS;
+                if constexpr (!Q::ALIGNED) {
+                    ra += offa & 15u;
+                    rb += offb & 15u;
+                    offa += A.ks * Q::BB;
+                    offb += A.ks * Q::BB;
+                }
+                const uint8_t* const bp[1] = {colb + i * XB + t * 16};
+                const uint32_t sumw[1] = {mq_mins<T> ? *reinterpret_cast<const uint32_t*>(colb + i * XB + 512 + t * 4) : 0u};
+                float c[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+                mm_block<T, 1>(ra, rb, t, gl, sl, bp, sumw, 1, c);
+                const float f = inv[i * TOK + (TOK == 2 ? t >> 1 : 0)];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] = fmaf(f, c[0][j], acc[j]);
+                if (++q_s == A.nst) q_s = 0;
+            }
+        }
+        // columns 0-2 (lanes t = 0, 1) are the first vector's parts, 4-6 (t = 2, 3) the second's
+        float a = (t & 1) ? acc[0] : acc[0] + acc[1], b = (t & 1) ? acc[2] : acc[2] + acc[3];
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        b += __shfl_xor_sync(0xffffffffu, b, 1);
+        float* rp = red + ((rd & 1) * kGvWarps + warp) * 16 * TOK;
+        if ((t >> 1) < TOK) rp[(t >> 1) * 16 + ((t & 1) ? 8 + g : g)] = (t & 1) ? b : a;
+        __syncthreads();  // (two buffers: a warp is at most one round ahead of the sums below)
+        if (tid < nslot * 16 * TOK) {
+            const int sl2 = tid / (16 * TOK), e = tid - sl2 * 16 * TOK, q = e >> 4;
+            const int row = (blockIdx.x * nslot + rd * rg_step + sl2) * 16 + (e & 15);
+            const float* r0 = red + ((rd & 1) * kGvWarps + sl2 * A.ks) * 16 * TOK + e;
+            float v = r0[0];
+            for (int w2 = 1; w2 < A.ks; ++w2) v += r0[w2 * 16 * TOK];
+            if (row < A.n && v0 + q < A.nvec) A.out[(size_t)(v0 + q) * A.n + row] = v;
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+template <int T, int TOK>
+static int launch_gv_t(dnb_ctx* c, cudaStream_t st, GvArgs A) {
+    const int nb = A.k / 256, rs = Mq<T>::RS;
+    int ks = 1;
+    while (ks < kGvWarps && ks * 2 <= nb) ks *= 2;
+    const int kb_max = (nb + ks - 1) / ks;
+    size_t base = ((2 * kGvWarps * 16 * TOK + kGvWarps * kb_max * TOK) * 4 + 127) / 128 * 128 + (size_t)kGvWarps * kb_max * TOK * 3 * kGvPart;
+    if (T == T_IQ3_XXS) base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmCodebook);
+    const size_t stage = (size_t)kGvWarps * 16 * rs, two = 113 * 1024, cap = 225 * 1024;  // two CTAs per SM where they fit
+    A.ks = ks;
+    for (A.nst = 4; A.nst > 2 && base + A.nst * stage > two; --A.nst) {}
+    const size_t smem = base + A.nst * stage;
+    if (smem > cap) return DNB_DECLINED;
+    A.smem = (uint32_t)smem;
+    A.status = c->status;
+    auto kern = gemv_mma_single_kernel<T, TOK>;
+    static SmemGrant grant;
+    DNB_CUDA(grant_smem(grant, c->device, kern, smem));
+    const int nslot = kGvWarps / ks, n_rg = (A.n + 15) / 16;
+    const int room = (smem <= two ? 2 : 1) * c->sm_count, ctas = (n_rg + nslot - 1) / nslot, rows = (A.nvec + TOK - 1) / TOK;
+    // more vectors in grid rows of their own, each decoding the weights again: while they only fill SMs that would idle
+    if (rows > 1 && (long)ctas * rows > room) return DNB_DECLINED;
+    const int grid = std::min(ctas, room);
+    ProfScope prof_(c, st, "gemv_mma");
+    DNB_CUDA(launch_k(kern, dim3(grid, rows), dim3(kGvWarps * 32), smem, st, c->use_pdl, A));
+    c->launches++;
+    return DNB_OK;
+}
+
+int launch_gemv_mma(dnb_ctx* c, cudaStream_t st, int type, const uint8_t* w, int k, int n, const float* x, float* out, int nvec) {
+    if (!mm_handles(type, k) || n < 1 || nvec < 1 || (((uintptr_t)w) & 15) || (((uintptr_t)x) & 15)) return DNB_DECLINED;
+    const int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
+    if (rc) return rc;
+    GvArgs A = {};
+    A.w = w; A.x = x; A.out = out; A.k = k; A.n = n; A.nvec = nvec; A.rb = (int)row_bytes(type, k);
+#define DNB_GV(TT) case TT: return nvec == 1 ? launch_gv_t<TT, 1>(c, st, A) : launch_gv_t<TT, 2>(c, st, A);
+    switch (type) {
+        DNB_GV(T_Q4_K)
+        DNB_GV(T_Q5_K)
+        DNB_GV(T_Q6_K)
+        DNB_GV(T_Q8_0)
+        default: return nvec == 1 ? launch_gv_t<T_IQ3_XXS, 1>(c, st, A) : launch_gv_t<T_IQ3_XXS, 2>(c, st, A);
+    }
+#undef DNB_GV
+}
+
 }  // namespace dnb

@@ -144,7 +144,7 @@ class CudaCtx:
         check(self.lib.dnb_dev_upload(self.h, C.c_void_p(ptr), _p(arr), arr.nbytes))
 
     def dev_copy(self, dst, src, nbytes):
-        check(self.lib.dnb_dev_copy(self.h, C.c_void_p(dst), C.c_void_p(src), nbytes))
+        check(self.lib.dnb_dev_copy(self.h, dst, src, nbytes))
 
     def download(self, ptr, arr):
         check(self.lib.dnb_dev_download(self.h, _p(arr), C.c_void_p(ptr), arr.nbytes))
@@ -159,8 +159,7 @@ class CudaCtx:
         return check(self.lib.dnb_gemv(self.h, uid, _p(x), _p(out)), True)
 
     def gemv_dev(self, ty, w_ptr, k, n, x_ptr, out_ptr, nvec=1):
-        return check(self.lib.dnb_gemv_dev(self.h, ty, C.c_void_p(w_ptr), k, n, C.c_void_p(x_ptr), C.c_void_p(out_ptr),
-                                           nvec), True)
+        return check(self.lib.dnb_gemv_dev(self.h, ty, w_ptr, k, n, x_ptr, out_ptr, nvec), True)
 
     def set_gemv_impl(self, impl):
         check(self.lib.dnb_set_gemv_impl(self.h, impl))
@@ -236,7 +235,7 @@ class CudaCtx:
         return check(self.lib.dnb_moe_block(self.h, layer, hp, nt, op, None, None), True)
 
     def moe_block_dev(self, layer, h_ptr, nt, out_ptr):
-        return check(self.lib.dnb_moe_block_dev(self.h, layer, C.c_void_p(h_ptr), nt, C.c_void_p(out_ptr)), True)
+        return check(self.lib.dnb_moe_block_dev(self.h, layer, h_ptr, nt, out_ptr), True)
 
     def moe_experts(self, layer, x, sels, wts):
         e = self.model["e"]
@@ -339,7 +338,7 @@ class CudaCtx:
         return out
 
     def moe_stack_dev(self, h_ptr, nt):
-        return check(self.lib.dnb_moe_stack_dev(self.h, C.c_void_p(h_ptr), nt), True)
+        return check(self.lib.dnb_moe_stack_dev(self.h, h_ptr, nt), True)
 
 
 # ---- free functions with the reference's names ----------------------------------
