@@ -216,7 +216,7 @@ static bool layer_ready(const dnb_ctx* c, int layer, bool need_router) {
 // [nt][e]; sels/wts on the device.  Writes out[nt][e].  The shared expert's
 // segment descriptors must already have been published by launch_prep.
 static int experts_dev(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts,
-                       float* out, int k = -1, int ne = -1, int with_shared = -1) {
+                       float* out, const float* residual = nullptr, int k = -1, int ne = -1, int with_shared = -1) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
     Workspace& w = c->ws;
@@ -237,10 +237,11 @@ static int experts_dev(dnb_ctx* c, int layer, const float* x, int nt, const int3
                                     nullptr, w.sh, nt)))
             return rc;
         if (L.shared_gate_row)
-            if ((rc = launch_shared_coef(c, c->side, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
+            if ((rc = launch_shared_coef(c, c->side, x, L.shared_gate_row, nt, M.e, w.shcoef, false))) return rc;
         DNB_CUDA(cudaEventRecord(c->ev_join, c->side));
     }
-    if ((rc = launch_route_tables(c, st, sels, nt, k, ne, L, w))) return rc;
+    // beside a forked stream every launch is an ordinary one
+    if ((rc = launch_route_tables(c, st, sels, nt, k, ne, L, w, false, !shared))) return rc;
     const int nseg_max = nt * k < ne ? nt * k : ne;
     if ((rc = launch_seg_matmul(c, st, L.m[0].type, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, x, M.e, w.row_token,
                                 w.act, nt)))
@@ -250,7 +251,7 @@ static int experts_dev(dnb_ctx* c, int layer, const float* x, int nt, const int3
         return rc;
     if (shared) DNB_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
     return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.sh : nullptr,
-                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out);
+                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out, residual, !shared);
 }
 
 // One token: fused router kernel, gate/up GEMV over the k routed experts plus the
@@ -308,9 +309,8 @@ static int block_dev_decode(dnb_ctx* c, int layer, const float* h, float* out, c
         rc = launch_seg_matmul(c, st, L.m[2].type, false, w.seg_dn, nullptr, nseg, M.ff, M.e, w.act, M.ff, nullptr, w.hrow, 1);
     if (rc) return rc;
     if ((rc = launch_combine(c, st, w.hrow, w.pos, w.wts, 1, M.k, M.e, fold ? w.hrow + (size_t)M.k * M.e : nullptr, coef,
-                             residual ? w.out : out)))
+                             out, residual)))
         return rc;
-    if (residual) return launch_add_inplace(c, st, out, w.out, (size_t)M.e);
     return DNB_OK;
 }
 
@@ -375,7 +375,7 @@ static bool umma_eligible(const dnb_ctx* c, const Layer& L, int nt) {
 
 // op_ready: the operand rows of x are in the workspace (written with the RMSNorm).
 static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts,
-                            float* out, int k = -1, int ne = -1, int with_shared = -1, bool op_ready = false) {
+                            float* out, const float* residual = nullptr, int k = -1, int ne = -1, int with_shared = -1, bool op_ready = false) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
     Workspace& w = c->ws;
@@ -396,7 +396,7 @@ static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const
     if (shared && L.shared_gate_row)
         if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
     return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
-                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out);
+                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out, residual);
 }
 
 // Layers that the mma.sync grouped kernel takes (grouped_mma.cu): its five formats, the shared expert like the routed ones.
@@ -409,7 +409,7 @@ static bool mm_eligible(const dnb_ctx* c, const Layer& L) {
 
 // The experts on the mma.sync grouped kernel: tables, gate/up, down, combine.  The shared expert is one more segment.
 static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts, float* out, int parts,
-                           int k = -1, int ne = -1, int with_shared = -1) {
+                           const float* residual = nullptr, int k = -1, int ne = -1, int with_shared = -1, bool tables_ready = false) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
     Workspace& w = c->ws;
@@ -418,7 +418,11 @@ static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const 
     if (ne < 0) ne = M.ne;
     const bool shared = with_shared < 0 ? L.has_shared() : (with_shared != 0);
     int rc;
-    if ((rc = launch_route_tables(c, st, sels, nt, k, ne, L, w, shared))) return rc;
+    if (!tables_ready) {
+        rc = launch_topk_tables(c, st, false, nt, k, ne, M.norm_topk, const_cast<int32_t*>(sels), nullptr, L, w, shared);
+        if (rc == DNB_DECLINED) rc = launch_route_tables(c, st, sels, nt, k, ne, L, w, shared);
+        if (rc) return rc;
+    }
     const int rows = nt * k + (shared ? nt : 0);
     const int nseg_max = (nt * k < ne ? nt * k : ne) + (shared ? 1 : 0);
     // experts that nt tokens reach when each picks k of ne at random
@@ -432,7 +436,7 @@ static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const 
     if (shared && L.shared_gate_row)
         if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
     return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
-                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out);
+                          (shared && L.shared_gate_row) ? w.shcoef : nullptr, out, residual);
 }
 
 // Router logits of nt rows: the tensor-core kernel from kRouterTcMin tokens, the fp32 kernel below.
@@ -457,22 +461,29 @@ int router_topk_dev(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const L
     return launch_topk(c, st, w.logits, nt, M.ne, M.k, M.norm_topk, sels, wts, rowsum);
 }
 
-static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out) {
+static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out, const float* residual = nullptr) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
     Workspace& w = c->ws;
     cudaStream_t st = c->stream;
     int rc;
     if (nt == 1 && c->decode_fast) {
-        rc = block_dev_decode(c, layer, h, out, nullptr);
+        rc = block_dev_decode(c, layer, h, out, residual);
         if (rc != DNB_DECLINED) return rc;
     }
     const bool mma = nt > 1 && mm_eligible(c, L) && !umma_eligible(c, L, nt);
     if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !mma && !umma_eligible(c, L, nt)) {
-        rc = block_dev_decode_batch(c, layer, h, nt, out, nullptr);
+        rc = block_dev_decode_batch(c, layer, h, nt, out, residual);
         if (rc != DNB_DECLINED) return rc;
     }
     const bool shared = L.has_shared();
+    if (mma && !router_tc_eligible(c, L, nt)) {
+        // a decode batch: routing in two launches (route_small.cu), the block in five
+        rc = launch_router_batch(c, st, h, nt, M, L, w);
+        if (rc == DNB_OK) rc = launch_topk_tables(c, st, true, nt, M.k, M.ne, M.norm_topk, w.sels, w.wts, L, w, shared);
+        if (rc == DNB_OK) rc = experts_dev_mma(c, layer, L.norm_w ? w.xn : h, nt, w.sels, w.wts, out, 3, residual, -1, -1, -1, true);
+        if (rc != DNB_DECLINED) return rc;
+    }
     // the RMSNorm kernel writes the router's operand (three bf16 parts of the normalised rows) and the experts' in the same pass
     const bool umma = umma_eligible(c, L, nt), split_in_prep = L.norm_w && router_tc_eligible(c, L, nt), op_in_prep = L.norm_w && umma;
     if (op_in_prep) {
@@ -486,12 +497,12 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out) 
     }
     const float* x = L.norm_w ? w.xn : h;
     if ((rc = router_topk_dev(c, st, x, nt, L, w.sels, w.wts, nullptr, split_in_prep))) return rc;
-    if (umma) return experts_dev_umma(c, layer, x, nt, w.sels, w.wts, out, -1, -1, -1, op_in_prep);
+    if (umma) return experts_dev_umma(c, layer, x, nt, w.sels, w.wts, out, residual, -1, -1, -1, op_in_prep);
     if (mma) {
-        rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, nt >= 16 && tc_type(L, 0, 3) >= 0 ? 2 : 3);
+        rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, nt >= 16 && tc_type(L, 0, 3) >= 0 ? 2 : 3, residual);
         if (rc != DNB_DECLINED) return rc;
     }
-    return experts_dev(c, layer, x, nt, w.sels, w.wts, out);
+    return experts_dev(c, layer, x, nt, w.sels, w.wts, out, residual);
 }
 
 // The shared expert on all rows: one segment, rows in place.
@@ -1106,18 +1117,30 @@ int dnb_moe_experts(dnb_ctx* c, int layer, const float* x, int nt, const int32_t
     memcpy(w.pinned_in, x, bytes);
     memcpy(w.pinned_sels, sels, rows * 4);
     memcpy(w.pinned_wts, wts, rows * 4);
-    DNB_CUDA(cudaMemcpyAsync(w.hin, w.pinned_in, bytes, cudaMemcpyHostToDevice, c->stream));
-    DNB_CUDA(cudaMemcpyAsync(w.sels, w.pinned_sels, rows * 4, cudaMemcpyHostToDevice, c->stream));
-    DNB_CUDA(cudaMemcpyAsync(w.wts, w.pinned_wts, rows * 4, cudaMemcpyHostToDevice, c->stream));
     const Layer& L = M.layers[layer];
-    if (L.has_shared())
-        if ((rc = launch_prep(c, c->stream, w.hin, nullptr, M.eps, nt, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn,
-                              L.m[3].dev, L.m[4].dev, L.m[5].dev)))
-            return rc;
-    rc = mm_eligible(c, L) ? experts_dev_mma(c, layer, w.hin, nt, w.sels, w.wts, w.out, 3) : DNB_DECLINED;
-    if (rc == DNB_DECLINED) rc = experts_dev(c, layer, w.hin, nt, w.sels, w.wts, w.out);
+    rc = run_graphed(c, GraphKey{9, layer, nt, nullptr, nullptr}, [&]() -> int {
+        // A few tokens, as in dnb_moe_block: read by a kernel, the result stored straight into the pinned buffer.
+        const bool direct = nt <= 8;
+        int r = direct ? launch_stage_routed(c, c->stream, w.pinned_in, w.hin, bytes / 4, w.pinned_sels, w.sels, w.pinned_wts, w.wts, rows) : DNB_DECLINED;
+        if (r != DNB_OK && r != DNB_DECLINED) return r;
+        if (r == DNB_DECLINED) {
+            DNB_CUDA(cudaMemcpyAsync(w.hin, w.pinned_in, bytes, cudaMemcpyHostToDevice, c->stream));
+            DNB_CUDA(cudaMemcpyAsync(w.sels, w.pinned_sels, rows * 4, cudaMemcpyHostToDevice, c->stream));
+            DNB_CUDA(cudaMemcpyAsync(w.wts, w.pinned_wts, rows * 4, cudaMemcpyHostToDevice, c->stream));
+        }
+        float* o = direct ? w.pinned_out : w.out;
+        r = mm_eligible(c, L) ? experts_dev_mma(c, layer, w.hin, nt, w.sels, w.wts, o, 3) : DNB_DECLINED;
+        if (r == DNB_DECLINED) {
+            if (L.has_shared())
+                if ((r = launch_prep(c, c->stream, w.hin, nullptr, M.eps, nt, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev, L.m[4].dev, L.m[5].dev)))
+                    return r;
+            r = experts_dev(c, layer, w.hin, nt, w.sels, w.wts, o);
+        }
+        if (r) return r;
+        if (!direct) DNB_CUDA(cudaMemcpyAsync(w.pinned_out, w.out, bytes, cudaMemcpyDeviceToHost, c->stream));
+        return DNB_OK;
+    });
     if (rc) return rc;
-    DNB_CUDA(cudaMemcpyAsync(w.pinned_out, w.out, bytes, cudaMemcpyDeviceToHost, c->stream));
     DNB_CUDA(nt <= 64 ? wait_short(c->stream) : cudaStreamSynchronize(c->stream));
     if ((rc = finish_checked(c, "moe_experts"))) return rc;
     memcpy(out, w.pinned_out, bytes);
@@ -1435,8 +1458,8 @@ int dnb_expert_rows_dev(dnb_ctx* c, int layer, const float* x_rows_dev, const in
     const bool umma = c->use_umma && w.op_ok && rows >= 16;
     if (!use_shared) {
         // every row is one (token, slot): a "chunk" of `rows` tokens with one selected expert each and weight 1
-        if (umma && tc_routed) return experts_dev_umma(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, 1, M.shard_count, 0);
-        return experts_dev(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, 1, M.shard_count, 0);
+        if (umma && tc_routed) return experts_dev_umma(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, nullptr, 1, M.shard_count, 0);
+        return experts_dev(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, nullptr, 1, M.shard_count, 0);
     }
     return shared_rows(c, layer, x_rows_dev, rows, false, h_rows_dev);
 }
@@ -1472,19 +1495,8 @@ int dnb_moe_stack_dev(dnb_ctx* c, float* h_dev, int nt) {
     if (rc) return rc;
     return run_graphed(c, GraphKey{4, 0, nt, h_dev, nullptr}, [&]() -> int {
         for (int l = 0; l < M.n_layer; ++l) {
-            if (nt == 1 && c->decode_fast) {
-                const int rd = block_dev_decode(c, l, h_dev, h_dev, h_dev);
-                if (rd == DNB_OK) continue;
-                if (rd != DNB_DECLINED) return rd;
-            }
-            if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !mm_eligible(c, M.layers[l]) && !umma_eligible(c, M.layers[l], nt)) {
-                const int rd = block_dev_decode_batch(c, l, h_dev, nt, h_dev, h_dev);
-                if (rd == DNB_OK) continue;
-                if (rd != DNB_DECLINED) return rd;
-            }
-            int r = block_dev(c, l, h_dev, nt, c->ws.out);
+            const int r = block_dev(c, l, h_dev, nt, h_dev, h_dev);
             if (r) return r;
-            if ((r = launch_add_inplace(c, c->stream, h_dev, c->ws.out, (size_t)nt * M.e))) return r;
         }
         return DNB_OK;
     });

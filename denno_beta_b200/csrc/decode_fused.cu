@@ -65,6 +65,8 @@ extern "C" int dnb_probe_timeline(void* dst) { return (int)cudaMemcpyFromSymbol(
 #define DNB_STAMP(i) do { } while (0)
 #endif
 
+#include "route_topk.cuh"
+
 namespace dnb {
 
 constexpr int kFdUnits = 2;                         // down units (8 output rows) per CTA
@@ -75,7 +77,6 @@ constexpr int kFdSegs = 2 * kFdPairs;
 constexpr int kFdPad = 8;                           // halves of padding per activation row (bank spread)
 constexpr int kFdHeader = 256;                      // 16 mbarriers, then flags
 constexpr int kFdRouterRows = 4;                    // router rows a CTA can hold (ROUTED)
-constexpr int kFdCand = 64;                         // entries the parallel ranking of the top-k takes
 static_assert(kFdWarps >= kGmGroups * kGmKs, "the gate/up phase needs its warps");
 
 struct FusedArgs {
@@ -114,25 +115,6 @@ struct FusedArgs {
     float* xn_out;             // [e] normalised row, or null
 };
 
-// Shared memory of the routing phase (ROUTED).
-struct RouteSmem {
-    float probs[1024];
-    uint32_t tmax[128];
-    int wcnt[4];
-    uint32_t cand_k[kFdCand];
-    int cand_x[kFdCand];
-    float red[128];
-    float cmax[4];
-    float bcast;
-    float inv;
-    int nan_any;
-    int total;
-    int sel[32];
-    float pv[32];
-    int ssel[32];
-    float spv[32];
-};
-
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -161,201 +143,10 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs& A, bool wait) {
     return pass;
 }
 
-__device__ __forceinline__ uint32_t order_key(float v) {  // larger float -> larger key; never 0 for a probability
-    const uint32_t ub = __float_as_uint(v);
-    return (ub & 0x80000000u) ? ~ub : (ub | 0x80000000u);
-}
-
-// softmax + top-k + renorm of the ne logits in global memory (written by all CTAs before the
-// barrier), by the whole CTA.  Leaves the selection ascending in R.ssel, the routing weights in
-// wts_s[0..k).  Every thread of the CTA must call it (it contains CTA-wide barriers).
 // Barrier of the four routing warps (named barrier 6; 1-5 belong to the gate/up groups).
-__device__ __forceinline__ void route_sync() { asm volatile("bar.sync 6, 128;" ::: "memory"); }
-
-// Softmax, top-k and renorm of one token's logits by threads 0..127 of the CTA (the other warps wait at
-// the CTA barrier that follows the call).  Thread v holds entries v, v + 128, ...; every value that
-// depends on evaluation order is computed as in topk_block (moe_kernels.cu), so a token gets the same
-// routing bits as on the other paths.  Six 128-thread barriers: what only one warp did before (the
-// sum's tree, the threshold) every warp now does for itself instead of waiting for a broadcast.
-__device__ __forceinline__ void route_topk(RouteSmem& R, const float* __restrict__ logits, int ne, int k, int norm_topk,
-                                           float* wts_s) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float p[8];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int idx = j * 128 + tid;
-        p[j] = idx < ne ? __ldcg(logits + idx) : -INFINITY;
-        mx = fmaxf(mx, p[j]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) R.cmax[warp] = mx;
-    if (tid == 0) R.nan_any = 0;
-    DNB_STAMP(16);
-    route_sync();
-    mx = fmaxf(fmaxf(R.cmax[0], R.cmax[1]), fmaxf(R.cmax[2], R.cmax[3]));
-    {
-        float part = 0.f;
-        bool any_nan = false;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (j * 128 + tid < ne) {
-                p[j] = expf(p[j] - mx);
-                part += p[j];
-                any_nan |= (p[j] != p[j]);
-            }
-        }
-        R.red[tid] = part;
-        if (any_nan) R.nan_any = 1;
-    }
-    DNB_STAMP(17);
-    route_sync();
-    // the tree of topk_block; the xor butterfly leaves the same bits in every lane of every warp
-    float sum = (R.red[lane] + R.red[lane + 64]) + (R.red[lane + 32] + R.red[lane + 96]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const bool has_nan = R.nan_any != 0;
-    uint32_t key[8];
-    uint32_t km = 0u;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int idx = j * 128 + tid;
-        key[j] = 0u;
-        if (idx < ne) {
-            p[j] = sum > 0.f ? p[j] / sum : p[j];
-            R.probs[idx] = p[j];
-            key[j] = order_key(p[j]);
-            km = max(km, key[j]);
-        }
-    }
-    R.tmax[tid] = km;
-    DNB_STAMP(18);
-    route_sync();
-    // ---- selection ----
-    // Fast form (no NaN): the entries fall into 32 classes by index mod 32 (= lane); t = the k-th largest
-    // of the class maxima.  At least k entries reach t, so every one of the top k does; the entries that
-    // reach it (a dozen or two) are ranked among themselves by (value descending, index ascending) -- the
-    // CPU scan's rule.
-    bool fast = !has_nan && k <= 32;
-    int total = 0;
-    if (fast) {
-        const uint32_t v = max(max(R.tmax[lane], R.tmax[lane + 32]), max(R.tmax[lane + 64], R.tmax[lane + 96]));
-        int above = 0;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) above += (__shfl_sync(0xffffffffu, v, j) > v) ? 1 : 0;
-        uint32_t t = __reduce_min_sync(0xffffffffu, (above < k && v != 0u) ? v : 0xffffffffu);
-        const int have = __popc(__ballot_sync(0xffffffffu, v != 0u));
-        if (have < k) t = 1u;  // fewer maxima than selections: every entry is a candidate
-        uint32_t smask = 0u;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) smask |= (key[j] != 0u && key[j] >= t) ? (1u << j) : 0u;
-        const int cnt = __popc(smask);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) R.wcnt[warp] = incl;
-        DNB_STAMP(19);
-        route_sync();
-        int before = incl - cnt;
-        for (int w2 = 0; w2 < 4; ++w2) {
-            const int c = R.wcnt[w2];
-            if (w2 < warp) before += c;
-            total += c;
-        }
-        fast = total >= k && total <= kFdCand;
-        if (fast) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if ((smask >> j) & 1u) {
-                    R.cand_k[before] = key[j];
-                    R.cand_x[before] = j * 128 + tid;
-                    ++before;
-                }
-        }
-        DNB_STAMP(20);
-        route_sync();
-        if (fast && tid < total) {
-            const uint32_t ck = R.cand_k[tid];
-            const int cx = R.cand_x[tid];
-            int rank = 0;
-            for (int j = 0; j < total; ++j) {
-                const uint32_t ok = R.cand_k[j];
-                const int ox = R.cand_x[j];
-                rank += (ok > ck || (ok == ck && ox < cx)) ? 1 : 0;
-            }
-            if (rank < k) {
-                R.sel[rank] = cx;
-                R.pv[rank] = R.probs[cx];
-            }
-        }
-    }
-    if (!fast) {
-        // General form, warp 0: k rounds of the CPU scan (moe.rs:256-279) with the entries dealt to
-        // the lanes.  A strictly larger value wins, ties go to the lower index, and a NaN is taken
-        // only when it is the first unused entry.
-        if (warp == 0) {
-            uint32_t used = 0u;  // bit m: entry 32 m + lane
-            for (int round = 0; round < k; ++round) {
-                float best = -INFINITY;
-                int best_i = 0x7fffffff, first = 0x7fffffff;
-                for (int m = 0; 32 * m + lane < ne; ++m) {
-                    if ((used >> m) & 1u) continue;
-                    const int idx = 32 * m + lane;
-                    first = min(first, idx);
-                    const float v = R.probs[idx];
-                    if (v == v && (best_i == 0x7fffffff || v > best)) {
-                        best = v;
-                        best_i = idx;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-                    first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-                    if (oi != 0x7fffffff && (best_i == 0x7fffffff || ov > best || (ov == best && oi < best_i))) {
-                        best = ov;
-                        best_i = oi;
-                    }
-                }
-                int win = best_i;
-                if (has_nan || best_i == 0x7fffffff) {
-                    const float fv = first != 0x7fffffff ? R.probs[first] : 0.f;
-                    if (fv != fv || best_i == 0x7fffffff) win = first;
-                }
-                if ((win & 31) == lane) used |= 1u << (win >> 5);
-                if (lane == 0) {
-                    R.sel[round] = win;
-                    R.pv[round] = R.probs[win];
-                }
-            }
-        }
-    }
-    DNB_STAMP(21);
-    route_sync();
-    if (tid < k) {
-        const int mine = R.sel[tid];
-        int rank = 0;
-        for (int j = 0; j < k; ++j) rank += (R.sel[j] < mine) ? 1 : 0;
-        R.ssel[rank] = mine;
-        R.spv[rank] = R.pv[tid];
-    }
-    route_sync();
-    if (tid < k) {
-        float s = 0.f;  // the selected probabilities in ascending expert index, one add at a time
-        for (int j = 0; j < k; ++j) s = __fadd_rn(s, R.spv[j]);
-        float w;
-        if (!norm_topk) w = R.spv[tid];
-        else if (isfinite(s) && s > 0.f) w = R.spv[tid] / s;
-        else w = 1.0f / (float)k;
-        wts_s[tid] = w;
-    }
-    DNB_STAMP(22);
-}
+struct RouteSync {
+    __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 6, 128;" ::: "memory"); }
+};
 
 // Dynamic shared memory:
 // [16 mbarriers | flags, pad to 256][codebook 32 KB][gate/up rows][down rows][x fp32][x bf16 x3]
@@ -507,7 +298,7 @@ __global__ void __maxnreg__(ROUTED ? 80 : 64) decode_fused_kernel(const FusedArg
         ready = flags[1] != 0 && ready;
         // Every CTA ranks the logits itself.  (After a failed wait the host discards the call; the
         // selection below then runs on whatever is there, and every index stays in range.)
-        if (tid < 128) route_topk(*R, A.logits + (size_t)(blockIdx.x % kActRep) * A.ne, A.ne, A.k, A.norm_topk, ws);
+        if (tid < 128) route_topk(*R, A.logits + (size_t)(blockIdx.x % kActRep) * A.ne, A.ne, A.k, A.norm_topk, ws, tid, RouteSync());
         DNB_STAMP(7);
         if (tid < A.k) {
             int ex = R->ssel[tid];

@@ -274,6 +274,8 @@ int launch_prep(dnb_ctx* c, cudaStream_t st, const float* h, const float* w, flo
 int launch_prep_operand(dnb_ctx* c, cudaStream_t st, int type, const float* h, const float* w, float eps, int nt, int e, float* out, uint16_t* x3,
                         size_t x3_part, uint16_t* op);
 int launch_add_inplace(dnb_ctx* c, cudaStream_t st, float* h, const float* d, size_t n);
+int launch_stage_routed(dnb_ctx* c, cudaStream_t st, const float* x_pinned, float* x, size_t n, const int32_t* sels_pinned, int32_t* sels,
+                        const float* wts_pinned, float* wts, size_t pairs);
 int launch_stage_in(dnb_ctx* c, cudaStream_t st, const float* host_pinned, float* dst, size_t n);  // DNB_DECLINED: use a copy
 int launch_stall(dnb_ctx* c, cudaStream_t st, float ms);
 int launch_fill_u32(dnb_ctx* c, cudaStream_t st, uint32_t* dst, uint32_t v, size_t n);
@@ -313,6 +315,11 @@ int launch_seg_gemv_m1(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool x
                        PermOut perm = PermOut());
 int launch_decode_batch_tables(dnb_ctx* c, cudaStream_t st, const int32_t* sels, int nt, int k, const Layer& L,
                                Workspace& ws, bool fold_shared);
+// Routing of a decode batch in two launches (route_small.cu).
+bool route_small_handles(int nt, int e, int ne, int k);
+int launch_router_batch(dnb_ctx* c, cudaStream_t st, const float* h, int nt, const Model& M, const Layer& L, Workspace& w);
+int launch_topk_tables(dnb_ctx* c, cudaStream_t st, bool logits, int nt, int k, int ne, int norm_topk, int32_t* sels, float* wts, const Layer& L,
+                       Workspace& w, bool fold_shared);
 int launch_topk(dnb_ctx* c, cudaStream_t st, const float* logits, int nt, int ne, int k, int norm_topk, int32_t* sels,
                 float* wts, float* rowsum, int nsplit = 1, const float* bias = nullptr);
 // Builds, from sels[nt][k], the expert-major row space: counts, segment
@@ -320,7 +327,7 @@ int launch_topk(dnb_ctx* c, cudaStream_t st, const float* logits, int nt, int ne
 // fold_shared: the shared expert becomes one more segment (m = nt) whose packed rows
 // follow the routed rows (row nt*k + t reads token t).
 int launch_route_tables(dnb_ctx* c, cudaStream_t st, const int32_t* sels, int nt, int k, int ne, const Layer& L,
-                        Workspace& ws, bool fold_shared = false);
+                        Workspace& ws, bool fold_shared = false, bool pdl = true);
 // The opt-in dynamic shared memory limit is an attribute of a kernel PER DEVICE: what was
 // granted is remembered per device, so a process that drives several GPUs sets it on each.
 struct SmemGrant { size_t got[64] = {0}; };
@@ -395,8 +402,8 @@ int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const S
 // The shared expert of a layer on `rows` fp32 rows (api.cu); op_ready: their operand rows are in the workspace already.
 int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, float* out);
 int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t* pos, const float* wts, int nt,
-                   int k, int e, const float* sh, const float* shcoef, float* out);
-int launch_shared_coef(dnb_ctx* c, cudaStream_t st, const float* x, const float* row, int nt, int e, float* coef);
+                   int k, int e, const float* sh, const float* shcoef, float* out, const float* residual = nullptr, bool pdl = true);
+int launch_shared_coef(dnb_ctx* c, cudaStream_t st, const float* x, const float* row, int nt, int e, float* coef, bool pdl = true);
 int launch_synth_blocks(dnb_ctx* c, cudaStream_t st, int type, uint64_t seed, uint64_t tensor_id, uint8_t* dst,
                         uint64_t n_blocks, uint64_t first_block = 0);
 int launch_synth_normal(dnb_ctx* c, cudaStream_t st, uint64_t seed, uint64_t tensor_id, float sigma, float* dst,

@@ -5,6 +5,7 @@
 #include "formats.cuh"
 #include "tc_ptx.cuh"
 #include "operand_rows.cuh"
+#include "route_topk.cuh"
 
 namespace dnb {
 
@@ -30,6 +31,8 @@ __global__ void __launch_bounds__(128)
 prep_kernel(const float* __restrict__ h, const float* __restrict__ w, float eps, int e, float* __restrict__ out,
             SegDesc* sh_gu, SegDesc* sh_dn, const uint8_t* sg, const uint8_t* su, const uint8_t* sdn, uint32_t nt,
             uint16_t* __restrict__ x3, size_t x3_part) {
+    pdl_wait();
+    pdl_launch_dependents();
     if (blockIdx.x == 0 && threadIdx.x == 0 && sh_gu) {
         sh_gu[0] = SegDesc{sg, su, nt, 0u};
         sh_dn[0] = SegDesc{sdn, nullptr, nt, 0u};
@@ -65,6 +68,8 @@ prep_operand_kernel(const float* __restrict__ h, const float* __restrict__ w, fl
     __shared__ uint32_t redm[4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const float* xr = h + (size_t)blockIdx.x * e;
+    pdl_wait();
+    pdl_launch_dependents();
     const float inv = rms_inv_128(xr, e, eps, red);
     float* o = out + (size_t)blockIdx.x * e;
     uint16_t* p3 = x3 ? x3 + (size_t)blockIdx.x * e : nullptr;
@@ -111,9 +116,10 @@ prep_operand_kernel(const float* __restrict__ h, const float* __restrict__ w, fl
 
 int launch_rmsnorm(dnb_ctx* c, cudaStream_t st, const float* h, const float* w, float eps, int nt, int e, float* out) {
     ProfScope prof_(c, st, "rmsnorm");
-    prep_kernel<<<nt, 128, 0, st>>>(h, w, eps, e, out, nullptr, nullptr, nullptr, nullptr, nullptr, 0u, nullptr, 0);
+    const uint8_t* none = nullptr;
+    DNB_CUDA(launch_k(prep_kernel, dim3(nt), dim3(128), 0, st, c->use_pdl, h, w, eps, e, out, (SegDesc*)nullptr, (SegDesc*)nullptr, none, none, none,
+                      0u, (uint16_t*)nullptr, (size_t)0));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -122,9 +128,8 @@ int launch_prep_operand(dnb_ctx* c, cudaStream_t st, int type, const float* h, c
     if (e % 256 || (type != T_Q4_K && type != T_IQ3_XXS)) return DNB_DECLINED;
     ProfScope prof_(c, st, "prep_rmsnorm");
     auto kern = type == T_Q4_K ? prep_operand_kernel<T_Q4_K> : prep_operand_kernel<T_IQ3_XXS>;
-    kern<<<nt, 128, 0, st>>>(h, w, eps, e, out, x3, x3_part, op);
+    DNB_CUDA(launch_k(kern, dim3(nt), dim3(128), 0, st, c->use_pdl, h, w, eps, e, out, x3, x3_part, op));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -132,9 +137,9 @@ int launch_prep(dnb_ctx* c, cudaStream_t st, const float* h, const float* w, flo
                 SegDesc* sh_gu, SegDesc* sh_dn, const uint8_t* sg, const uint8_t* su, const uint8_t* sdn, uint16_t* x3,
                 size_t x3_part) {
     ProfScope prof_(c, st, "prep_rmsnorm");
-    prep_kernel<<<nt, 128, 0, st>>>(h, w, eps, e, out, sh_gu, sh_dn, sg, su, sdn, (uint32_t)nt, w ? x3 : nullptr, x3_part);
+    DNB_CUDA(launch_k(prep_kernel, dim3(nt), dim3(128), 0, st, c->use_pdl, h, w, eps, e, out, sh_gu, sh_dn, sg, su, sdn, (uint32_t)nt,
+                      w ? x3 : (uint16_t*)nullptr, x3_part));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -150,6 +155,8 @@ __global__ void __launch_bounds__(RROWS * 32)
 router_logits_kernel(const float* __restrict__ x, int nt, int e, const float* __restrict__ w_r,
                      const float* __restrict__ bias, int ne, float* __restrict__ logits) {
     extern __shared__ __align__(16) float xs[];  // [RT][e]
+    pdl_wait();
+    pdl_launch_dependents();
     const int t0 = blockIdx.y * RT;
     const int ntok = min(RT, nt - t0);
     const int e4 = e >> 2;
@@ -240,301 +247,32 @@ int launch_router_logits(dnb_ctx* c, cudaStream_t st, const float* x, int nt, in
     if (rc) return rc;
     dim3 grid((ne + RROWS * RW - 1) / (RROWS * RW), (nt + RT - 1) / RT);
     ProfScope prof_(c, st, "router_logits");
-    router_logits_kernel<<<grid, RROWS * 32, smem, st>>>(x, nt, e, w_r, bias, ne, logits);
+    DNB_CUDA(launch_k(router_logits_kernel, grid, dim3(RROWS * 32), smem, st, c->use_pdl, x, nt, e, w_r, bias, ne, logits));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
-// ---- softmax + top-k + renorm (tensor.rs:1171-1183; moe.rs:188-279;
-// qwen4exp.rs:11802-11821; GPU form kernels_router225.cu:36-171) -----------------
-// One CTA of 128 threads per token, ne <= 1024, k <= 32.  Thread v holds entries
-// v, v+128, ...  Everything that depends on evaluation order is fixed:
-//   softmax denominator: per-thread partials in ascending index, then the tree
-//     ((s[l]+s[l+64]) + (s[l+32]+s[l+96])) followed by a 32-lane xor tree;
-//   selection: the CPU scan's rule (moe.rs:256-279) -- a strictly larger value
-//     wins, ties go to the lower index, and a NaN is taken only when it is the
-//     first unused entry;
-//   renorm: the selected probabilities summed in ascending expert index, one add
-//     at a time, as on the CPU.
-// The same function serves the per-token kernel and the tail of the fused decode
-// router, so a token gets the same routing bits on either path.
-struct TopkSmem {
-    uint32_t keys[1024];
-    uint32_t cand_k[32];
-    int cand_x[32];
-    float red[128];
-    float cand_v[4];
-    int cand_i[4];
-    int cand_first[4];
-    float bcast;
-    int ibcast;
-    int sel[32];
-    float pv[32];
-    int ssel[32];
-    float spv[32];
+// ---- softmax + top-k + renorm (route_topk.cuh) ----------------------------------
+// One CTA of 128 threads per token, ne <= 1024, k <= 32.
+struct CtaSync {
+    __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
-
-// nsplit > 1: logit_row points at the first of nsplit partial sums of the row, split_stride floats apart (the
-// tensor-core router's K splits); they are added in ascending order, then the bias: the sequence of adds of
-// router_reduce_kernel, so the logits are the same bits whether that kernel ran or not.
-__device__ __forceinline__ void topk_block(const float* __restrict__ logit_row, int ne, int k, int norm_topk,
-                                           TopkSmem& sm, int32_t* __restrict__ sels_out, float* __restrict__ wts_out,
-                                           float* __restrict__ rowsum_out, int nsplit = 1, size_t split_stride = 0,
-                                           const float* __restrict__ bias = nullptr) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float p[8];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int idx = j * 128 + tid;
-        float v = -INFINITY;
-        if (idx < ne) {
-            v = __ldcg(logit_row + idx);  // L2: other CTAs of this launch may have written them
-            if (nsplit > 1) {
-                float part[kRouterSplitMax];  // all requested before the first is used
-#pragma unroll
-                for (int s = 1; s < kRouterSplitMax; ++s)
-                    part[s] = s < nsplit ? __ldcg(logit_row + (size_t)s * split_stride + idx) : 0.f;
-#pragma unroll
-                for (int s = 1; s < kRouterSplitMax; ++s)
-                    if (s < nsplit) v = __fadd_rn(v, part[s]);
-                if (bias) v = __fadd_rn(v, bias[idx]);
-            }
-        }
-        p[j] = v;
-        mx = fmaxf(mx, p[j]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) sm.cand_v[warp] = mx;
-    __syncthreads();
-    mx = fmaxf(fmaxf(sm.cand_v[0], sm.cand_v[1]), fmaxf(sm.cand_v[2], sm.cand_v[3]));
-    float part = 0.f;
-    bool any_nan = false;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (j * 128 + tid < ne) {
-            p[j] = expf(p[j] - mx);
-            part += p[j];
-            any_nan |= (p[j] != p[j]);
-        }
-    }
-    sm.red[tid] = part;
-    const int nan_block = __syncthreads_or(any_nan ? 1 : 0);
-    if (warp == 0) {
-        float a = (sm.red[lane] + sm.red[lane + 64]) + (sm.red[lane + 32] + sm.red[lane + 96]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) sm.bcast = a;
-    }
-    __syncthreads();
-    const float sum = sm.bcast;
-    if (sum > 0.f) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (j * 128 + tid < ne) p[j] = p[j] / sum;  // (the -inf padding would take the division's slow path)
-    }
-    uint32_t used = 0;
-    if (!nan_block) {
-        // Fast path (no NaN anywhere): values map to order-preserving integer keys, the
-        // warp finds the maximum and the lowest index holding it with two redux
-        // instructions, and only the lane that owned the winner rescans its entries.
-        // Same rule: larger value first, ties to the lower index.
-        // The keys go to shared memory and warp 0 selects alone: no block barrier inside
-        // the k rounds.
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t ub = __float_as_uint(p[j]);
-            if (j * 128 + tid < ne) sm.keys[j * 128 + tid] = (ub & 0x80000000u) ? ~ub : (ub | 0x80000000u);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t key[32];  // entry 32 * m + lane
-#pragma unroll
-            for (int m = 0; m < 32; ++m) key[m] = (32 * m + lane < ne) ? sm.keys[32 * m + lane] : 0u;
-            // a lane's best: maximum by a pairwise tree (depth 5, not a 32-step chain), then
-            // the lowest entry holding it
-            auto lane_best = [&](uint32_t& bk, int& bm) {
-                uint32_t t[16];
-#pragma unroll
-                for (int m = 0; m < 16; ++m) t[m] = max(key[2 * m], key[2 * m + 1]);
-#pragma unroll
-                for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-                    for (int m = 0; m < w; ++m) t[m] = max(t[m], t[m + w]);
-                bk = t[0];
-                uint32_t hit = 0u;
-#pragma unroll
-                for (int m = 0; m < 32; ++m) hit |= (key[m] == bk ? 1u : 0u) << m;
-                bm = bk ? __ffs((int)hit) - 1 : -1;
-            };
-            uint32_t bk;
-            int bm;
-            lane_best(bk, bm);
-            // Shortcut without rounds.  t = the k-th largest of the 32 lane maxima: at least k
-            // entries reach t, so every one of the top k does.  When no more than 32 entries
-            // reach t (the usual case: a dozen or two), each goes to one lane, which ranks it
-            // among the others by value and index; rank r < k is selection r.
-            bool done = false;
-            if (k <= 32) {
-                int above = 0;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) above += (__shfl_sync(0xffffffffu, bk, j) > bk) ? 1 : 0;
-                const uint32_t t = __reduce_min_sync(0xffffffffu, above < k ? bk : 0xffffffffu);
-                uint32_t surv = 0u;
-#pragma unroll
-                for (int m = 0; m < 32; ++m) surv |= ((key[m] >= t && key[m] != 0u) ? 1u : 0u) << m;
-                const int mine = __popc(surv);
-                int incl = mine;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                if (total <= 32 && total >= k) {
-                    int pos = incl - mine;
-                    while (surv) {
-                        const int m = __ffs((int)surv) - 1;
-                        surv &= surv - 1u;
-                        sm.cand_k[pos] = sm.keys[32 * m + lane];
-                        sm.cand_x[pos] = 32 * m + lane;
-                        ++pos;
-                    }
-                    __syncwarp();
-                    const uint32_t ck = lane < total ? sm.cand_k[lane] : 0u;
-                    const int cx = lane < total ? sm.cand_x[lane] : 0x7fffffff;
-                    int rank = 0;
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const uint32_t ok = __shfl_sync(0xffffffffu, ck, j);
-                        const int ox = __shfl_sync(0xffffffffu, cx, j);
-                        rank += (ok > ck || (ok == ck && ox < cx)) ? 1 : 0;
-                    }
-                    if (lane < total && rank < k) {
-                        sm.sel[rank] = cx;
-                        sm.pv[rank] = __uint_as_float((ck & 0x80000000u) ? (ck ^ 0x80000000u) : ~ck);
-                    }
-                    done = true;
-                }
-            }
-            for (int round = 0; round < k && !done; ++round) {
-                const uint32_t wm = __reduce_max_sync(0xffffffffu, bk);
-                const uint32_t wi = __reduce_min_sync(0xffffffffu, (bk == wm && bm >= 0) ? (uint32_t)(32 * bm + lane) : 0x7fffffffu);
-                if (lane == 0) {
-                    sm.sel[round] = (int)wi;
-                    sm.pv[round] = __uint_as_float((wm & 0x80000000u) ? (wm ^ 0x80000000u) : ~wm);
-                }
-                if ((int)(wi & 31u) == lane) {  // the owner drops the winner and rescans its entries
-#pragma unroll
-                    for (int m = 0; m < 32; ++m)
-                        if (m == (int)(wi >> 5)) key[m] = 0u;
-                    lane_best(bk, bm);
-                }
-            }
-        }
-        __syncthreads();
-    } else
-    for (int round = 0; round < k; ++round) {
-        float best = -INFINITY;
-        int best_i = 0x7fffffff, first = 0x7fffffff;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int idx = j * 128 + tid;
-            if (idx < ne && !((used >> j) & 1u)) {
-                first = min(first, idx);
-                const float v = p[j];
-                if (v == v && (best_i == 0x7fffffff || v > best)) {
-                    best = v;
-                    best_i = idx;
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-            first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-            if (oi != 0x7fffffff && (best_i == 0x7fffffff || ov > best || (ov == best && oi < best_i))) {
-                best = ov;
-                best_i = oi;
-            }
-        }
-        if (lane == 0) {
-            sm.cand_v[warp] = best;
-            sm.cand_i[warp] = best_i;
-            sm.cand_first[warp] = first;
-        }
-        __syncthreads();
-        float bv = sm.cand_v[0];
-        int bi = sm.cand_i[0], gfirst = sm.cand_first[0];
-#pragma unroll
-        for (int w = 1; w < 4; ++w) {
-            const float ov = sm.cand_v[w];
-            const int oi = sm.cand_i[w];
-            gfirst = min(gfirst, sm.cand_first[w]);
-            if (oi != 0x7fffffff && (bi == 0x7fffffff || ov > bv || (ov == bv && oi < bi))) {
-                bv = ov;
-                bi = oi;
-            }
-        }
-        int win = bi;
-        if (nan_block) {  // rare path: does the scan's first unused entry hold a NaN?
-            if ((gfirst & 127) == tid) {
-                float fv = 0.f;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (j == (gfirst >> 7)) fv = p[j];
-                sm.ibcast = (fv != fv) ? 1 : 0;
-            }
-            __syncthreads();
-            if (sm.ibcast || bi == 0x7fffffff) win = gfirst;
-        }
-        if ((win & 127) == tid) {
-            used |= 1u << (win >> 7);
-            float wv = 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j == (win >> 7)) wv = p[j];
-            sm.sel[round] = win;
-            sm.pv[round] = wv;
-        }
-        __syncthreads();
-    }
-    if (tid < k) {
-        const int mine = sm.sel[tid];
-        int rank = 0;
-        for (int j = 0; j < k; ++j) rank += (sm.sel[j] < mine) ? 1 : 0;
-        sm.ssel[rank] = mine;
-        sm.spv[rank] = sm.pv[tid];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        float s = 0.f;
-        for (int j = 0; j < k; ++j) s = __fadd_rn(s, sm.spv[j]);
-        sm.bcast = s;
-    }
-    __syncthreads();
-    const float s = sm.bcast;
-    if (tid < k) {
-        float w;
-        if (!norm_topk) w = sm.spv[tid];
-        else if (isfinite(s) && s > 0.f) w = sm.spv[tid] / s;
-        else w = 1.0f / (float)k;
-        sels_out[tid] = sm.ssel[tid];
-        wts_out[tid] = w;
-    }
-    if (rowsum_out && tid == 0) *rowsum_out = s;
-}
 
 __global__ void __launch_bounds__(128)
 topk_kernel(const float* __restrict__ logits, int nt, int ne, int k, int norm_topk, int32_t* __restrict__ sels,
             float* __restrict__ wts, float* __restrict__ rowsum, int nsplit, const float* __restrict__ bias) {
-    __shared__ TopkSmem sm;
+    __shared__ RouteSmem sm;
+    __shared__ float w_s[32];
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x;
-    topk_block(logits + (size_t)t * ne, ne, k, norm_topk, sm, sels + (size_t)t * k, wts + (size_t)t * k,
-               rowsum ? rowsum + t : nullptr, nsplit, (size_t)nt * ne, bias);
+    route_topk(sm, logits + (size_t)t * ne, ne, k, norm_topk, w_s, threadIdx.x, CtaSync(), rowsum ? rowsum + t : nullptr, nsplit,
+               (size_t)nt * ne, bias);
+    __syncthreads();
+    if (threadIdx.x < k) {
+        sels[(size_t)t * k + threadIdx.x] = sm.ssel[threadIdx.x];
+        wts[(size_t)t * k + threadIdx.x] = w_s[threadIdx.x];
+    }
 }
 
 // nsplit > 1: `logits` is [nsplit][nt][ne] partial sums (router_tc.cu), added here with `bias`.
@@ -546,9 +284,9 @@ int launch_topk(dnb_ctx* c, cudaStream_t st, const float* logits, int nt, int ne
         return DNB_DECLINED;
     }
     ProfScope prof_(c, st, "router_topk");
-    topk_kernel<<<nt, 128, 0, st>>>(logits, nt, ne, k, norm_topk, sels, wts, rowsum, nsplit, nsplit > 1 ? bias : nullptr);
+    DNB_CUDA(launch_k(topk_kernel, dim3(nt), dim3(128), 0, st, c->use_pdl, logits, nt, ne, k, norm_topk, sels, wts, rowsum, nsplit,
+                      nsplit > 1 ? bias : (const float*)nullptr));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -574,7 +312,8 @@ router_decode_kernel(const float* __restrict__ h, const float* __restrict__ norm
     extern __shared__ __align__(16) float xs[];  // [e]
     __shared__ float red[4];
     __shared__ int is_last;
-    __shared__ TopkSmem sm;
+    __shared__ RouteSmem sm;
+    __shared__ float w_s[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row = blockIdx.x * 4 + warp;
     // The router rows are constants of the layer: fetch this warp's row before
@@ -648,9 +387,11 @@ router_decode_kernel(const float* __restrict__ h, const float* __restrict__ norm
         for (int i = tid; i < e; i += 128) o[slot_index(gate_type, i, e >> 5)] = xs[i];
     }
     if (!is_last) return;
-    topk_block(logits, ne, k, norm_topk, sm, sels, wts, nullptr);
+    route_topk(sm, logits, ne, k, norm_topk, w_s, tid, CtaSync());
     __syncthreads();
     if (tid < k) {
+        sels[tid] = sm.ssel[tid];
+        wts[tid] = w_s[tid];
         // Expert parallel: only experts [shard_first, shard_first + shard_count) are resident here (indexed from
         // 0 in the local tensors); the other slots become empty segments, which the GEMV kernels skip.
         const int li = sm.ssel[tid] - shard_first;
@@ -826,6 +567,8 @@ route_tables_kernel(const int32_t* __restrict__ sels, int nt, int k, int ne, con
     for (int i = tid; i < RTE * words; i += RTE * 32) bits[i] = 0;
     for (int i = tid; i < ne; i += RTE * 32) counts[i] = 0;
     __syncthreads();
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int RTB = 8;  // selections a thread requests before it uses the first (the loop is bound by their latency)
     for (int i0 = tid; i0 < nt * k; i0 += RTE * 32 * RTB) {
         int ev[RTB];
@@ -936,7 +679,7 @@ route_tables_kernel(const int32_t* __restrict__ sels, int nt, int k, int ne, con
 }
 
 int launch_route_tables(dnb_ctx* c, cudaStream_t st, const int32_t* sels, int nt, int k, int ne, const Layer& L,
-                        Workspace& ws, bool fold_shared) {
+                        Workspace& ws, bool fold_shared, bool pdl) {
     const int words = (nt + 31) >> 5;
     const size_t smem = ((size_t)2 * RTE * words + (size_t)ne) * 4;
     if (smem > 200 * 1024 || (uint64_t)nt * k * k >= (1ull << 32) || (uint64_t)ne * ((ne + RTE - 1) / RTE) >= (1ull << 32)) {
@@ -946,12 +689,11 @@ int launch_route_tables(dnb_ctx* c, cudaStream_t st, const int32_t* sels, int nt
     static SmemGrant grant;
     DNB_CUDA(grant_smem(grant, c->device, route_tables_kernel, smem));
     ProfScope prof_(c, st, "route_tables");
-    route_tables_kernel<<<(ne + RTE - 1) / RTE, RTE * 32, smem, st>>>(
-        sels, nt, k, ne, L.m[0].dev, L.m[1].dev, L.m[2].dev, L.m[0].expert_bytes, L.m[1].expert_bytes,
-        L.m[2].expert_bytes, fold_shared ? L.m[3].dev : nullptr, fold_shared ? L.m[4].dev : nullptr,
-        fold_shared ? L.m[5].dev : nullptr, ws.seg_gu, ws.seg_dn, ws.row_token, ws.pos, ws.nseg, ws.counts);
+    DNB_CUDA(launch_k(route_tables_kernel, dim3((ne + RTE - 1) / RTE), dim3(RTE * 32), smem, st, c->use_pdl && pdl, sels, nt, k, ne,
+                      (const uint8_t*)L.m[0].dev, (const uint8_t*)L.m[1].dev, (const uint8_t*)L.m[2].dev, L.m[0].expert_bytes, L.m[1].expert_bytes,
+                      L.m[2].expert_bytes, (const uint8_t*)(fold_shared ? L.m[3].dev : nullptr), (const uint8_t*)(fold_shared ? L.m[4].dev : nullptr),
+                      (const uint8_t*)(fold_shared ? L.m[5].dev : nullptr), ws.seg_gu, ws.seg_dn, ws.row_token, ws.pos, ws.nseg, ws.counts));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -993,10 +735,12 @@ int launch_decode_batch_tables(dnb_ctx* c, cudaStream_t st, const int32_t* sels,
 // ---- weighted combine (kernels_dec_epi.cu:28-46 dno_dec_exp_sum;
 // moe_grouped_gpu.rs:540-565 scatter; qwen4exp.rs:12126-12216) --------------------
 // out[t][j] = sum over slots in ascending order of w[t][s] * h[pos[t][s]][j]
-// (separate multiply and add, as on the CPU), then + coef * sh[t][j].
+// (separate multiply and add, as on the CPU), then + coef * sh[t][j], then residual[t][j] + that (residual may be out).
 __global__ void __launch_bounds__(256)
 combine_kernel(const float* __restrict__ hrow, const int32_t* __restrict__ pos, const float* __restrict__ wts, int k,
-               int e, const float* __restrict__ sh, const float* __restrict__ shcoef, float* __restrict__ out) {
+               int e, const float* __restrict__ sh, const float* __restrict__ shcoef, const float* residual, float* out) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x;
     __shared__ int32_t prow[32];
     __shared__ float pw[32];
@@ -1006,9 +750,9 @@ combine_kernel(const float* __restrict__ hrow, const int32_t* __restrict__ pos, 
     }
     __syncthreads();
     if ((e & 3) == 0) {
-        // four columns per thread; the rows of up to eight slots are requested before the
-        // first is used (the sum itself stays one slot after the other, ascending)
-        for (int j = threadIdx.x * 4; j < e; j += 1024) {
+        // four columns per thread, a quarter of a 4096-column row per CTA (a batch of eight tokens would otherwise be eight CTAs); the
+        // rows of up to eight slots are requested before the first is used (the sum stays one slot after the other, ascending)
+        for (int j = (blockIdx.y * 256 + threadIdx.x) * 4; j < e; j += gridDim.y * 1024) {
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int s0 = 0; s0 < k; s0 += 8) {
                 float4 v[8];
@@ -1040,27 +784,34 @@ combine_kernel(const float* __restrict__ hrow, const int32_t* __restrict__ pos, 
                     acc.w = __fadd_rn(acc.w, v.w);
                 }
             }
+            if (residual) {
+                const float4 v = *reinterpret_cast<const float4*>(residual + (size_t)t * e + j);
+                acc.x = __fadd_rn(v.x, acc.x);
+                acc.y = __fadd_rn(v.y, acc.y);
+                acc.z = __fadd_rn(v.z, acc.z);
+                acc.w = __fadd_rn(v.w, acc.w);
+            }
             *reinterpret_cast<float4*>(out + (size_t)t * e + j) = acc;
         }
         return;
     }
-    for (int j = threadIdx.x; j < e; j += 256) {
+    for (int j = blockIdx.y * 256 + threadIdx.x; j < e; j += gridDim.y * 256) {
         float acc = 0.f;
         for (int s = 0; s < k; ++s) acc = __fadd_rn(acc, __fmul_rn(pw[s], hrow[(size_t)prow[s] * e + j]));
         if (sh) {
             const float v = sh[(size_t)t * e + j];
             acc = __fadd_rn(acc, shcoef ? __fmul_rn(v, shcoef[t]) : v);
         }
+        if (residual) acc = __fadd_rn(residual[(size_t)t * e + j], acc);
         out[(size_t)t * e + j] = acc;
     }
 }
 
 int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t* pos, const float* wts, int nt,
-                   int k, int e, const float* sh, const float* shcoef, float* out) {
+                   int k, int e, const float* sh, const float* shcoef, float* out, const float* residual, bool pdl) {
     ProfScope prof_(c, st, "combine");
-    combine_kernel<<<nt, 256, 0, st>>>(hrow, pos, wts, k, e, sh, shcoef, out);
+    DNB_CUDA(launch_k(combine_kernel, dim3(nt, (e + 1023) / 1024), dim3(256), 0, st, c->use_pdl && pdl, hrow, pos, wts, k, e, sh, shcoef, residual, out));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -1068,6 +819,8 @@ int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t
 __global__ void __launch_bounds__(128)
 shared_coef_kernel(const float* __restrict__ x, const float* __restrict__ row, int nt, int e, float* __restrict__ coef) {
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_wait();
+    pdl_launch_dependents();
     if (t >= nt) return;
     float acc = 0.f;
     for (int i = lane; i < e; i += 32) acc = fmaf(row[i], x[(size_t)t * e + i], acc);
@@ -1076,11 +829,10 @@ shared_coef_kernel(const float* __restrict__ x, const float* __restrict__ row, i
     if (lane == 0) coef[t] = 1.0f / (1.0f + expf(-acc));
 }
 
-int launch_shared_coef(dnb_ctx* c, cudaStream_t st, const float* x, const float* row, int nt, int e, float* coef) {
+int launch_shared_coef(dnb_ctx* c, cudaStream_t st, const float* x, const float* row, int nt, int e, float* coef, bool pdl) {
     ProfScope prof_(c, st, "shared_coef");
-    shared_coef_kernel<<<(nt + 3) / 4, 128, 0, st>>>(x, row, nt, e, coef);
+    DNB_CUDA(launch_k(shared_coef_kernel, dim3((nt + 3) / 4), dim3(128), 0, st, c->use_pdl && pdl, x, row, nt, e, coef));
     c->launches++;
-    DNB_CUDA(cudaGetLastError());
     return DNB_OK;
 }
 
@@ -1113,6 +865,30 @@ int launch_stage_in(dnb_ctx* c, cudaStream_t st, const float* host_pinned, float
     ProfScope prof_(c, st, "stage_in");
     DNB_CUDA(launch_k(stage_in_kernel, dim3((n4 + 511) / 512), dim3(512), 0, st, c->use_pdl,
                       reinterpret_cast<const float4*>(host_pinned), reinterpret_cast<float4*>(dst), n4));
+    c->launches++;
+    return DNB_OK;
+}
+
+// The same for rows that come with their routing: pairs selections and weights beside n floats.
+__global__ void __launch_bounds__(512)
+stage_routed_kernel(const float4* __restrict__ src, float4* __restrict__ dst, int n4, const int32_t* __restrict__ sels_src, int32_t* __restrict__ sels,
+                    const float* __restrict__ wts_src, float* __restrict__ wts, int pairs) {
+    pdl_launch_dependents();
+    pdl_wait();  // the kernels in front may still read the routing that this one replaces
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) dst[i] = src[i];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
+        sels[i] = sels_src[i];
+        wts[i] = wts_src[i];
+    }
+}
+
+int launch_stage_routed(dnb_ctx* c, cudaStream_t st, const float* x_pinned, float* x, size_t n, const int32_t* sels_pinned, int32_t* sels,
+                        const float* wts_pinned, float* wts, size_t pairs) {
+    if (n % 4 || n / 4 > (1u << 20) || pairs > (1u << 20)) return DNB_DECLINED;
+    const int n4 = (int)(n / 4);
+    ProfScope prof_(c, st, "stage_in");
+    DNB_CUDA(launch_k(stage_routed_kernel, dim3((n4 + 511) / 512), dim3(512), 0, st, c->use_pdl, reinterpret_cast<const float4*>(x_pinned),
+                      reinterpret_cast<float4*>(x), n4, sels_pinned, sels, wts_pinned, wts, (int)pairs));
     c->launches++;
     return DNB_OK;
 }

@@ -88,6 +88,8 @@ router_tc_kernel(const __grid_constant__ Maps maps, int nt, int ne, int kchunks,
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
+    pdl_wait();
+    pdl_launch_dependents();
 
     if (warp == 0) {
         // ---------------- TMA ----------------
@@ -265,10 +267,9 @@ int launch_router_logits_tc(dnb_ctx* c, cudaStream_t st, const float* x, int nt,
     const dim3 grid((ne + rt::TM - 1) / rt::TM, (nt + rt::TN - 1) / rt::TN, nsplit);
     {
         ProfScope prof_(c, st, "router_logits_tc");
-        rt::router_tc_kernel<<<grid, rt::NTHREADS, smem, st>>>(maps, nt, ne, e / rt::BK / nsplit, L.router_bias,
-                                                              nsplit == 1 ? logits : w.rpart, c->status);
+        DNB_CUDA(launch_k(rt::router_tc_kernel, grid, dim3(rt::NTHREADS), smem, st, c->use_pdl, maps, nt, ne, e / rt::BK / nsplit,
+                          (const float*)L.router_bias, nsplit == 1 ? logits : w.rpart, c->status));
         c->launches++;
-        DNB_CUDA(cudaGetLastError());
     }
     if (nsplit > 1 && reduce) {
         ProfScope prof_(c, st, "router_reduce");
