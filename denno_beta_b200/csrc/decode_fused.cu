@@ -457,23 +457,14 @@ __global__ void __maxnreg__(ROUTED ? 80 : 64) decode_fused_kernel(const FusedArg
             const uint16_t* xb = acts + ((size_t)((which ? sb : sa) * kGmSplit + (n < kGmSplit ? n : 0))) * arow + 8 * t;
             const int nblk = ff >> 8, b0 = kh * (nblk >> 1), b1 = b0 + (nblk >> 1);
             float acc = 0.f;
-            for (int b = b0; b < b1; ++b) {
-                const uint8_t* ba = ra + b * 98;
-                const uint8_t* bb = rbp + b * 98;
-                const float da = h2f(ld16(ba)) * 0.25f, db = h2f(ld16(bb)) * 0.25f;
-#pragma unroll 2
-                for (int ib = 0; ib < 8; ++ib) {
-                    uint4 y = make_uint4(0u, 0u, 0u, 0u);
-                    if (has_col) y = *reinterpret_cast<const uint4*>(xb + (b * 8 + ib) * 32);
-                    float c[4];
-                    uint32_t auxa, auxb;
-                    iq3_subblock_mma(ba, bb, ib, t, lutp, y, c, auxa, auxb);
-                    // lanes t = 0, 1 keep the first expert's columns (rows 0-7), t = 2, 3 the second's (rows 8-15)
-                    const float mine = t < 2 ? c[0] + c[1] : c[2] + c[3];
-                    const float sc = t < 2 ? iq3_scale(da, auxa) : iq3_scale(db, auxb);
-                    acc = fmaf(sc, mine, acc);
-                }
-            }
+            for (int b = b0; b < b1; ++b)
+                iq3_block_mma(
+                    ra + b * 98, rbp + b * 98, t, lutp,
+                    [&](int ib) { return has_col ? *reinterpret_cast<const uint4*>(xb + (b * 8 + ib) * 32) : make_uint4(0u, 0u, 0u, 0u); },
+                    [&](const float (&c)[4], float sa, float sb) {
+                        // lanes t = 0, 1 keep the first expert's columns (rows 0-7), t = 2, 3 the second's (rows 8-15)
+                        acc = fmaf(t < 2 ? sa : sb, t < 2 ? c[0] + c[1] : c[2] + c[3], acc);
+                    });
             acc += __shfl_xor_sync(0xffffffffu, acc, 1);
             float* hq = hp + (size_t)(u * 2 + kh) * kFdSegs * 8;
             if (t == 0) hq[sa * 8 + g] = acc;

@@ -1,0 +1,114 @@
+"""The edges of the expert kernels' tiles and of the rules that choose between them, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from helpers import SEED, check_block, make_layer, rel_err
+from test_hyper import hc_weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def ctx():
+    from denno_beta_b200 import cuda as cu
+
+    c = cu.CudaCtx(0)
+    yield c
+    assert c.device_status() == 0
+    c.close()
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("k,n", [(256, 32), (768, 288), (2304, 544)])
+def test_grouped_mma(orc, ctx, name, k, n):
+    """grouped_mma.cu: row counts around its 8-token tiles, rows that end inside a 16-row tile group, K of 1, 3 and 9 blocks."""
+    from denno_beta_b200 import cuda as cu
+
+    ty, ne = orc.TYPE_BY_NAME[name], 6
+    assert ctx.moe_config(1, k, n, ne, 2)
+    w = orc.synth_blocks(ty, SEED, 40 + ty, ne * n * k // orc.blck_size(ty))
+    assert ctx.register_experts(0, cu.GATE, ty, k, n, ne, w)
+    segs, at = [], 0
+    for ex, m in ((4, 17), (0, 9), (5, 8), (2, 7), (1, 1)):
+        segs.append([ex, m, at, at])
+        at += m
+    segs = np.array(segs, np.uint32)
+    x = orc.synth_normal(SEED, 41, 1.0, at * k).reshape(at, k)
+    x[3] *= 1e-6  # rows are scaled one by one
+    x[4] = 0.0
+    got = cu.moe_grouped_gemm_layer(ctx, 0, cu.GATE, segs, x, n)
+    want = orc.grouped_gemm(ty, w, k, n, segs, x)
+    for lo, hi in ((0, 3), (3, 4), (5, at)):
+        assert rel_err(got[lo:hi], want[lo:hi]) <= 2e-5
+    assert not got[4].any()
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "IQ3_XXS"])
+@pytest.mark.parametrize("e,ff,ne,k", [(256, 256, 8, 2), (768, 512, 16, 3), (2304, 256, 4, 1), (512, 1280, 24, 4)])
+def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
+    """Token counts on both sides of every hand-over (routing in two launches to 15, tensor-core router from 16, tcgen05 from 48),
+    with experts of one token to a full 32-token tile and more; K of 1 to 9 blocks."""
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.TYPE_BY_NAME[name], e, ff, ne, k, bias=True, gate_row=True)
+    for nt in (2, 9, 15, 16, 47, 48, 49, 97):
+        h = orc.synth_normal(SEED, 50 + nt, 1.0, nt * e).reshape(nt, e)
+        out, sels, wts = ctx.moe_block(0, h, want_routing=True)
+        err, _ = check_block(orc, L, h, out, sels, wts)
+        assert err <= (5e-5 if nt < 16 else 2e-4), "nt %d: %.3g" % (nt, err)
+        assert np.array_equal(out.view(np.uint32), ctx.moe_block(0, h).view(np.uint32)), "nt %d: bits of a replay" % nt
+
+
+@pytest.mark.parametrize("up,down,e,ff", [("Q5_K", "Q8_0", 768, 288), ("Q4_K", "Q6_K", 512, 768), ("IQ3_XXS", "Q4_K", 512, 256)])
+def test_experts_given_mixed(orc, ctx, up, down, e, ff):
+    """A selection of the caller's own and two formats in a layer, one with an expert width (288) that the mma kernel leaves alone."""
+    ne, k = 40, 5
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.TYPE_BY_NAME[up], e, ff, ne, k, ty_down=orc.TYPE_BY_NAME[down])
+    rng = np.random.RandomState(3)
+    for nt in (1, 4, 8, 9, 15, 16, 50):
+        x = orc.synth_normal(SEED, 60 + nt, 1.0, nt * e).reshape(nt, e)
+        sels = np.sort(np.argsort(rng.rand(nt, ne), axis=1)[:, :k], axis=1).astype(np.int32)
+        wts = rng.rand(nt, k).astype(np.float32)
+        for _ in range(3):  # the third one replays
+            out = ctx.moe_experts(0, x, sels, wts)
+            assert rel_err(out, orc.moe_experts_given(L, x, sels, wts)) <= 5e-5
+            sels, wts = np.ascontiguousarray(sels[::-1]), np.ascontiguousarray(wts[::-1])
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("k,n,nvec", [(256, 1, 1), (768, 15, 2), (2304, 17, 3), (512, 2369, 8), (4096, 33, 1)])
+def test_gemv_edges(orc, ctx, name, k, n, nvec):
+    ty = orc.TYPE_BY_NAME[name]
+    w = orc.synth_blocks(ty, SEED, 70 + ty, n * k // orc.blck_size(ty))
+    x = orc.synth_normal(SEED, 71, 1.0, nvec * k).reshape(nvec, k)
+    out = np.full((nvec + 1, n), 7.0, np.float32)
+    dw, dx, do = ctx.dev_alloc(w.nbytes), ctx.dev_alloc(x.nbytes), ctx.dev_alloc(out.nbytes)
+    try:
+        ctx.upload(dw, w)
+        ctx.upload(dx, x)
+        ctx.upload(do, out)
+        assert ctx.gemv_dev(ty, dw, k, n, dx, do, nvec)
+        got = ctx.download(do, np.empty_like(out))
+    finally:
+        for p in (dw, dx, do):
+            ctx.dev_free(p)
+    assert np.all(got[nvec] == 7.0), "wrote behind the last row"
+    want = np.stack([orc.gemv_scalar(ty, w, k, n, v) for v in x])
+    assert rel_err(got[:nvec], want) <= 2e-5
+
+
+@pytest.mark.parametrize("hc,lr,nts", [(1, 8, (1, 9)), (2, 33, (1, 8)), (3, 320, (2, 17))])
+def test_hyper_edges(orc, ctx, hc, lr, nts):
+    """Streams, ranks that end inside a CTA's rows, and more tokens than a CTA takes at once."""
+    e, ff, ne, k = 512, 256, 8, 2
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.IQ3_XXS, e, ff, ne, k, norm=False)
+    w_norm, w_down, w_up = hc_weights(orc, hc, e, lr, 1)
+    ctx.register_hc(0, hc, lr, w_norm, w_down, w_up)
+    for nt in nts:
+        res = orc.synth_normal(SEED, 80 + nt, 1.0, nt * hc * e).reshape(nt, hc, e)
+        mix = [orc.hc_mix(r, w_norm, w_down, w_up, lr, 1e-6)[:2] for r in res]
+        blk = orc.moe_block(L, np.stack([m.reshape(-1) for m, _ in mix]))[0]
+        want = np.stack([orc.hc_combine(r, b, inj) for r, b, (_, inj) in zip(res, blk, mix)])
+        for _ in range(3):
+            assert rel_err(ctx.hc_moe_block(0, res), want) <= 5e-5
