@@ -127,7 +127,10 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
             }
         }
     } else if constexpr (T == T_IQ3_XXS) {
-        const float da = h2f(ld16(ra)) * 0.25f, db = h2f(ld16(rb)) * 0.25f;
+        // (d / 4) * (2 s + 1) (kquant.rs:667) = 8 d v - 7.75 d with v = 1 + s / 16 read off the bits: exact, d has 11 significant bits
+        // (a conversion from integer would be a quarter-rate instruction)
+        const float da = h2f(ld16(ra)), db = h2f(ld16(rb));
+        const float ma8 = 8.f * da, na = -7.75f * da, mb8 = 8.f * db, nbs = -7.75f * db;
         // the eight sub-block words of a row as aligned words, shifted into place (a block starts on any even byte)
         const uint32_t ma = (tcp::s32(ra) + 2u) & 2u, mb = (tcp::s32(rb) + 2u) & 2u;
         const uint32_t* wa = reinterpret_cast<const uint32_t*>(ra + 66 - ma);
@@ -140,15 +143,15 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
 #pragma unroll
         for (int ib = 0; ib < 8; ++ib) {
             // the ninth word belongs to the row only where the words are shifted
-            const uint32_t na = wa[ib < 7 ? ib + 1 : 7 + (ma >> 1)], nbw = wb[ib < 7 ? ib + 1 : 7 + (mb >> 1)];
-            const uint32_t xa = __funnelshift_r(la, na, sa), xb = __funnelshift_r(lb, nbw, sb);
-            la = na;
+            const uint32_t naw = wa[ib < 7 ? ib + 1 : 7 + (ma >> 1)], nbw = wb[ib < 7 ? ib + 1 : 7 + (mb >> 1)];
+            const uint32_t xa = __funnelshift_r(la, naw, sa), xb = __funnelshift_r(lb, nbw, sb);
+            la = naw;
             lb = nbw;
             uint32_t p[4], q[4];
             iq3_pairs_h(gl, sl, ld16(ia + 8 * ib), __funnelshift_r(xa, xa, st), p);
             iq3_pairs_h(gl, sl, ld16(ibp + 8 * ib), __funnelshift_r(xb, xb, st), q);
-            // d * (0.5 + s) * 0.5 = (d / 4) * (2 s + 1) (kquant.rs:667)
-            const float fa = fmaf((float)(xa >> 28), da + da, da), fb = fmaf((float)(xb >> 28), db + db, db);
+            const float fa = fmaf(__uint_as_float(((xa >> 9) & 0x00780000u) | 0x3f800000u), ma8, na);
+            const float fb = fmaf(__uint_as_float(((xb >> 9) & 0x00780000u) | 0x3f800000u), mb8, nbs);
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 if (NT == 1 || n < nt) {
@@ -240,6 +243,7 @@ struct MmArgs {
     float* out;                // [packed row][n_out]
     int ks, nst;               // warps that split K, stages of a warp's ring
     int col_stride;            // bytes between B columns
+    int skip;                  // row groups' time that a tile's activations take
     uint32_t smem;             // bytes of dynamic shared memory
     int* status;
 };
@@ -340,14 +344,17 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
     const uint32_t gl = tcp::s32(book) + 8 * (lane & (kLutRep - 1)), sl = tcp::s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
     int par = 0;
-    // this CTA's share of all (tile, row group) pairs: a range of pairs in a row, so that every CTA gets the same number
-    const long total = (long)pre[nseg] * n_rg;
-    const long at1 = total * (blockIdx.x + 1) / gridDim.x;
+    // This CTA's share of all (tile, row group) pairs: a range of pairs in a row.  Another tile means another set of activations,
+    // which takes as long as A.skip row groups: each tile is that much longer, and a CTA that has two gets so much less of them.
+    const int span = n_rg + A.skip, total = pre[nseg] * span;
+    const int share = total / (int)gridDim.x, extra = total - share * (int)gridDim.x;
+    const int at1 = share * ((int)blockIdx.x + 1) + min((int)blockIdx.x + 1, extra);
 
-    for (long at = total * blockIdx.x / gridDim.x; at < at1; par ^= 1) {
-        const int gtile = (int)(at / n_rg), rg_begin = (int)(at - (long)gtile * n_rg);
-        const int rg_end = (int)min((long)n_rg, rg_begin + (at1 - at));
-        at += rg_end - rg_begin;
+    for (int at = share * (int)blockIdx.x + min((int)blockIdx.x, extra); at < at1; par ^= 1) {
+        const int gtile = at / span, in = at - gtile * span;
+        const int rg_begin = max(in - A.skip, 0), rg_end = min(in + (at1 - at), span) - A.skip;
+        at += span - in;
+        if (rg_end <= rg_begin) { par ^= 1; continue; }
         int lo = 0, hi = nseg;  // the segment: pre[lo] <= gtile < pre[lo + 1]
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -664,6 +671,9 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
             const size_t smem = base + A.nst * stage;
             A.smem = (uint32_t)smem;
             A.status = c->status;
+            // activations of a tile 2.5 - 3 us, a row group 1.1 us at K = 2048 and a quarter of that at K = 512 (measured, IQ3_XXS)
+            A.skip = std::max(1, 5120 / n_in);
+            if ((double)(nseg_max + (rows + nt * tpt - 1) / (nt * tpt)) * (n_rg + A.skip) > 2e9) return DNB_DECLINED;
             const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, std::max<long>(1, tiles * n_rg * ks / kMmWarps));
             switch (type) {
                 case T_Q4_K: return mm_launch_type<T_Q4_K>(c, st, fused, parts, nt, A, smem, grid, name);
