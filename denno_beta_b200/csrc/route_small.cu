@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(1024) topk_tables_kernel(const TableArgs A) {
     __shared__ float wt[8][32];
     __shared__ uint32_t tok[1024];                                         // tokens of an expert, a bit each
     __shared__ int active[kRsTok * 32], first[kRsTok * 32];                // the active experts in ascending order, their first rows
-    __shared__ int n_active, wsum[32];
+    __shared__ __align__(16) int key[kRsTok * 32 + 4];
+    __shared__ int wsum[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = tid >> 7;
     tok[tid] = 0u;
     pdl_wait();
@@ -169,24 +170,22 @@ __global__ void __launch_bounds__(1024) topk_tables_kernel(const TableArgs A) {
     const uint32_t bal = __ballot_sync(0xffffffffu, on);
     if (lane == 0) wsum[warp] = __popc(bal);
     __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < 32; ++w) {
-        const int c = wsum[w];
-        before += w < warp ? c : 0;
-        total += c;
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? wsum[lane] : 0), n_active = __reduce_add_sync(0xffffffffu, wsum[lane]);
+    // An expert's key: larger = earlier among the segments (more tokens, then the lower index).
+    if (on) {
+        const int a = before + __popc(bal & ((1u << lane) - 1u));
+        active[a] = tid;
+        key[a] = __popc(tok[tid]) << 10 | (1023 - a);
     }
-    if (on) active[before + __popc(bal & ((1u << lane) - 1u))] = tid;
-    if (tid == 0) n_active = total;
+    if (tid < 4) key[n_active + tid] = 0;  // (read in fours)
     __syncthreads();
     if (tid < n_active) {
-        const int ex = active[tid], c = __popc(tok[ex]);
+        const int ex = active[tid], mine = key[tid], c = mine >> 10;
         int rank = 0, row = 0;
-        for (int o = 0; o < n_active; ++o) {
-            const int co = __popc(tok[active[o]]);
-            if (co > c || (co == c && o < tid)) {
-                rank++;
-                row += co;
-            }
+        for (int o = 0; o < n_active; o += 4) {
+            const int4 k4 = *reinterpret_cast<const int4*>(key + o);
+            rank += (k4.x > mine) + (k4.y > mine) + (k4.z > mine) + (k4.w > mine);
+            row += (k4.x > mine ? k4.x >> 10 : 0) + (k4.y > mine ? k4.y >> 10 : 0) + (k4.z > mine ? k4.z >> 10 : 0) + (k4.w > mine ? k4.w >> 10 : 0);
         }
         A.seg_gu[rank] = SegDesc{A.gate + (size_t)ex * A.eb_g, A.up + (size_t)ex * A.eb_u, (uint32_t)c, (uint32_t)row};
         A.seg_dn[rank] = SegDesc{A.down + (size_t)ex * A.eb_d, nullptr, (uint32_t)c, (uint32_t)row};
