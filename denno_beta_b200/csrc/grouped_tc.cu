@@ -24,6 +24,7 @@
 //   * four groups of four producer warps, (even or odd stages) x (tile), a thread one row: decodes 64 weights into registers, THEN
 //     waits for a ring slot (tensor memory holds only four stages; with the decoding inside its turn-around a stage took 1,100
 //     cycles) and stores them.  The block's scales go to a small ring, its mins to shared memory of the thread's own.
+//     A stage has one full barrier for both operands, on which producers and B copies arrive (a second wait a stage: 2 to 3 % more time).
 //   * one MMA thread; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
 //     once per K step.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
@@ -241,7 +242,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm vol
 template <int T> struct Layout {
     static constexpr int RSTAGES = 3;
     static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
-    static constexpr int BARS = 3 * STAGES + BSTAGES + 2 * (RSTAGES + NB);
+    static constexpr int BARS = 2 * BSTAGES + 2 * (RSTAGES + NB);
     static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
     static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
     static constexpr int MINS = T == T_Q4_K ? PWARPS * 32 * 8 * 10 : 0;  // 8 + 2 bytes per block and producer thread
@@ -272,9 +273,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (s32(smem_raw) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(base);
-    uint64_t* bfull = full + STAGES;
-    uint64_t* empty = bfull + BSTAGES;        // one per B slot, two per A slot
-    uint64_t* rfull = empty + 2 * STAGES;
+    uint64_t* empty = full + BSTAGES;         // both: one per B slot, two per A slot
+    uint64_t* rfull = empty + BSTAGES;
     uint64_t* rempty = rfull + L::RSTAGES;
     uint64_t* tfull = rempty + L::RSTAGES;
     uint64_t* tfree = tfull + NB;
@@ -301,9 +301,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < STAGES; ++i) mb_init(&full[i], 8);                 // two producer groups' warps, a tile each
-        for (int i = 0; i < BSTAGES; ++i) mb_init(&bfull[i], BWARPS * 32);     // the B warps' lanes
-        for (int i = 0; i < 2 * STAGES; ++i) mb_init(&empty[i], 1);            // a commit
+        for (int i = 0; i < BSTAGES; ++i) mb_init(&full[i], 8 + BWARPS * 32);  // two producer groups' warps, a tile each, and the B warps' lanes
+        for (int i = 0; i < BSTAGES; ++i) mb_init(&empty[i], 1);               // a commit
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
         for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
         fence_mbarrier_init();
@@ -456,7 +455,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive(&full[q.slot()]);
+            if (lane == 0) mb_arrive(&full[q.q]);
         };
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
@@ -570,7 +569,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (i < steps) cp_async16(d + i * 1024, src[i] + off);
-                cp_async_arrive(&bfull[q.q]);
+                cp_async_arrive(&full[q.q]);
                 q.advance(1);
             };
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
@@ -605,7 +604,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         ok = mb_wait(&tfree[buf], pf, A.status, 6);
                         const uint32_t d = tmem_base + (uint32_t)(buf * BUF_COLS);
                         for (int c = 0; c < stages && ok; ++c) {
-                            ok = mb_wait(&bfull[q.q], q.turn, A.status, 5) && mb_wait(&full[q.slot()], q.q < STAGES ? 0u : 1u, A.status, 5);
+                            ok = mb_wait(&full[q.q], q.turn, A.status, 5);
                             if (!ok) break;
                             tc_fence_after();    // A: written to tensor memory by the producers
                             fence_async_smem();  // B: written to shared memory by the B warps' copies
