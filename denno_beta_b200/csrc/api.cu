@@ -358,7 +358,10 @@ static int tc_type(const Layer& L, int first, int last) {
         if (!L.m[i].dev || L.m[i].type != ty) return -1;
     return ty;
 }
-// Tokens from which a chunk or decode batch leaves the mma.sync kernel for the tcgen05 grouped GEMM.
+// Tokens from which a chunk or decode batch leaves the mma.sync kernel for the tcgen05 grouped GEMM.  A stage of the latter costs the
+// same for one token as for 32, so the line depends on how many tokens share an expert, which the host does not know.  us per layer at
+// 2048 x 512, top 10 of 512, mma.sync / tcgen05: Q4_K evenly routed 173 / 222 at 32 tokens, 216 / 275 at 48, 250 / 304 at 64; under a
+// skewed router 106 / 96, 129 / 100, 155 / 103.  At 48 either choice loses the same factor at worst (1.27).
 constexpr int kTcMin = 48;
 static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMin : c->exact_min_nt; }
 

@@ -5,15 +5,15 @@
 //
 //   route (local)                                  existing kernels
 //   plan      counts per expert, row order         ep_plan_kernel      -> peers' cnt + flag
-//   dispatch  x rows -> bf16 hi/lo, stored straight into the OWNER rank's operand buffers
-//             (the B operand the tcgen05 kernel reads by TMA from its own memory)
+//   dispatch  x rows -> fp16 hi/lo operand rows, stored straight into the OWNER rank's buffers
+//             (the tcgen05 kernel reads them from its own memory)
 //                                                  ep_dispatch_kernel  -> peers' data flag
 //   build     wait for every source's counts and rows (bounded), segment table per
 //             (source, expert), destination pointer of every received row
 //                                                  ep_build_kernel
-//   gate/up   grouped tcgen05 GEMM + SwiGLU        grouped_q4k_umma_kernel<2>
+//   gate/up   grouped tcgen05 GEMM + SwiGLU        grouped_tc_kernel<T, false>
 //   down      grouped tcgen05 GEMM whose epilogue stores each row into the (token, slot)
-//             row of the rank that owns the token  grouped_q4k_umma_kernel<1>, row_dst
+//             row of the rank that owns the token  grouped_tc_kernel<T, true>, row_dst
 //   signal / wait   release flags to the sources, wait for every owner's flag (bounded)
 //   combine   ascending slot order, as on one GPU  combine_kernel
 //

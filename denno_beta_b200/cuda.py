@@ -165,11 +165,11 @@ class CudaCtx:
         check(self.lib.dnb_set_gemv_impl(self.h, impl))
 
     def set_tc_min_tokens(self, iq3_xxs_min_tokens):
-        """IQ3_XXS layers: token count from which a batch takes the exact-weight tcgen05 grouped GEMM."""
+        """IQ3_XXS layers: token count from which a batch takes the tcgen05 grouped GEMM (default 48)."""
         check(self.lib.dnb_set_tc_min_tokens(self.h, iq3_xxs_min_tokens))
 
     def set_q4k_int(self, on):
-        """Q4_K chunks: three-product bf16 tcgen05 kernel (default, on=False) or the integer-weight kernel (more exact, slower)."""
+        """Accepted and without effect: the tcgen05 kernel of Q4_K chunks always has exact integer weights."""
         check(self.lib.dnb_set_q4k_int(self.h, int(on)))
 
     def set_router_tc(self, on):

@@ -151,16 +151,12 @@ int dnb_gemv_dev(dnb_ctx* ctx, int ggml_type, const void* w_dev, int k, int n, c
  * the fused one.  5: as 0, but the router of a one-token IQ3_XXS block runs as a
  * kernel of its own in front of the fused gate/up + down kernel instead of inside it. */
 int dnb_set_gemv_impl(dnb_ctx* ctx, int impl);
-/* IQ3_XXS layers: the token count from which a chunk or decode batch leaves the one-token kernels for the
- * exact-weight tcgen05 grouped GEMM (default 16, where it measured level with the one-token kernels and
- * 1.7x / 2.1x faster at 64 / 194 tokens; Q4_K layers switch to their tcgen05 kernel at 16 too).  A tuning
- * and A/B knob with no reference counterpart; results stay within the path's tolerance either way. */
+/* IQ3_XXS layers: the token count from which a chunk or decode batch leaves the mma.sync kernel for the tcgen05 grouped
+ * GEMM (default 48, as for Q4_K layers: evenly routed batches are faster on the first beyond 96 tokens, skewed ones on the
+ * second from 24).  A tuning and A/B knob with no reference counterpart; results stay within the path's tolerance either way. */
 int dnb_set_tc_min_tokens(dnb_ctx* ctx, int iq3_xxs_min_tokens);
-/* Q4_K chunks on tcgen05: on = 0 (default) the kernel that folds the scales into bf16 hi / lo weights (three
- * products per element); on = 1 the kernel with integer fp16 weights (sc * q, exact) and the block scales d,
- * dmin * m applied after the tensor-core sum, where the shape fits (n_embd, n_ff <= 2048, multiples of 256): a
- * sixth of the error (1e-5 against 7e-5 of the output RMS) at 1.2x the time of a 512-token chunk.  Both are far
- * inside the path's tolerance of the CPU reference; an A/B knob with no reference counterpart. */
+/* Accepted and without effect: the tcgen05 kernel of Q4_K chunks always has integer fp16 weights (sc * q, exact) with the
+ * block scales d, dmin * m applied after the tensor-core sum (1e-5 of the output RMS). */
 int dnb_set_q4k_int(dnb_ctx* ctx, int on);
 /* Router logits of calls of 16 tokens or more (cuda.rs:48695 pf_router_dev_topk over kernels_elem.cu:1085
  * dno_gemm_f32_mt): on = 1 (default) the tcgen05 kernel -- both operands as three bf16 parts, six products,
@@ -356,8 +352,9 @@ int dnb_moe_combine_dev(dnb_ctx* ctx, int layer, const float* h_slots_dev, const
  *       them with any host-side all-gather); maps the peers' arenas.
  *   dnb_ep_block_dev: one MoE block for this rank's nt tokens, h_dev/out_dev device
  *       [nt][n_embd].  Every rank of the group must make the same sequence of calls
- *       (same layer; nt may differ per rank).  The result equals the single-GPU block
- *       bit for bit: same operands, same accumulation order, same combine order. */
+ *       (same layer; nt may differ per rank).  The result equals the single-GPU block of
+ *       48 tokens or more (the tcgen05 path) bit for bit: same operands, same accumulation
+ *       order, same combine order; smaller single-GPU blocks agree to rounding. */
 int dnb_ep_init(dnb_ctx* ctx, int rank, int world, int max_tokens, void* handle_out);
 int dnb_ep_connect(dnb_ctx* ctx, const void* handles);
 int dnb_ep_block_dev(dnb_ctx* ctx, int layer, const float* h_dev, int nt, float* out_dev);
