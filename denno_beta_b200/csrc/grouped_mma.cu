@@ -24,6 +24,10 @@
 // 256-element block of the 16 rows each) without any CTA-wide barrier.  Few row groups for the chip (small models, single
 // matrices): KS warps share a row group, each takes a part of K, and their sums are added in a fixed order.
 // A row's result depends on nothing but the row: not on the tile, the column or the split of the launch.
+//
+// Measured, us per layer of 2048 x 512, top 10 of 512, against one-row GEMVs (to 15 tokens) and tiled fp32 or bf16 tensor-core kernels:
+// 8 tokens, IQ3_XXS 140 -> 95; 32 tokens 502 -> 204; 77 tokens under a skewed router, Q4_K with Q6_K down 895 -> 255.  Issue slots are
+// 0.53 to 0.64 used, DRAM 0.12 to 0.20.
 #include <algorithm>
 
 #include "dnb_common.cuh"
@@ -694,6 +698,8 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
 // work); a warp takes every ks-th block of K of 16 rows and asks for its first stages before it waits for the kernel in front of
 // it, whose output the vector may be; it converts its own blocks of the vector, each with a power of two of its own, so that no
 // CTA-wide step stands between vector and math; the warps' partial sums meet once per 16 rows, in a fixed order.
+// Measured back to back, us, register-decode GEMV before: 4096 x 4096 Q4_K 8.4 -> 5.7, IQ3_XXS 10.3 -> 6.4, Q8_0 8.9 -> 6.5; 65536 x
+// 4096 Q8_0 103 -> 69 (4.1 TB/s), Q4_K 84 -> 47, IQ3_XXS 99 -> 56; two vectors of IQ3_XXS 62034 x 5632 466 -> 94.
 constexpr int kGvWarps = 8;
 constexpr int kGvPart = 576;  // bytes of a part of a block: 512, its sub-block sums (16), and padding that spreads neighbouring parts over the banks
 

@@ -29,6 +29,10 @@
 //     once per K step.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
 // Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
+//
+// Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, us gate/up + down as bracketed by events: Q4_K 174 + 90 (three
+// bf16 products) -> 131 + 84, IQ3_XXS 343 + 180 -> 154 + 90.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
+// commit; without the decoding a copy of the kernel was only 7 % faster.
 #include <cuda.h>
 #include <cuda_fp16.h>
 

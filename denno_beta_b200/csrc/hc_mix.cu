@@ -37,6 +37,7 @@ __device__ __forceinline__ float hc_sigmoid(float v) { return 1.0f / (1.0f + exp
 
 // One token's mix is three dependent kernels over 21 MB of fp32 weights, and a call of one token is their latencies: each kernel
 // therefore starts while its predecessor still runs (programmatic launch) and holds its first weights in registers before it waits.
+// A call of one token (hc 4, n_embd 2048, rank 320, host buffers, the block included): 100 -> 57 us.
 
 // one CTA of 128 threads per (token, stream): the summation tree of rms_inv_128 (moe_kernels.cu).  `res` may be pinned host memory;
 // then res_dev (else null) receives a copy for the combine, and the row crosses the bus once.

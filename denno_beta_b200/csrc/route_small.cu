@@ -5,7 +5,7 @@
 // What bounds it: latencies.  As four kernels (RMSNorm, logits by 16 CTAs, a CTA per token, a CTA per eight experts) the routing of
 // eight tokens took 34 us of a 109 us layer, most of it launches, cold first loads and half-empty chips; the 4 MB of router rows are
 // 0.7 us.  Here a warp holds its router row in registers before it waits for the kernel in front, and the tables are built where the
-// selections are.
+// selections are: a layer of eight tokens 109 -> 96 us.
 #include <algorithm>
 
 #include "dnb_common.cuh"
