@@ -28,10 +28,10 @@
 //   * one MMA thread; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
 //     once per K step.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
-// Persistent, one CTA per SM; items (segment, 32-token tile, 128 rows x 2) dealt round-robin.
+// Persistent, one CTA per SM; items (segment, 32- or 64-token tile, 128 rows x 2) dealt round-robin.
 //
 // Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, us gate/up + down as bracketed by events: Q4_K 174 + 90 (three
-// bf16 products) -> 131 + 84, IQ3_XXS 343 + 180 -> 154 + 90.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
+// bf16 products) -> 131 + 84, IQ3_XXS 343 + 180 -> 135 + 76.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
 // commit; without the decoding a copy of the kernel was only 7 % faster.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -47,25 +47,32 @@ using namespace tcp;
 
 constexpr int BK = 64;                  // K of a stage: one 128-byte swizzle row of fp16
 constexpr int TILE_M = 128;
-constexpr int NT = 32;                  // tokens of an item
 constexpr int A_COLS = BK / 2;          // tensor-memory columns of an A tile (two fp16 each)
-constexpr int B_STAGE = 2 * NT * BK * 2;// hi and lo rows: 8 KB
-constexpr int NB = 2;                   // accumulator buffers
-constexpr int BUF_COLS = 2 * 2 * NT;    // two tiles x (hi, lo) x tokens
 constexpr int EWARPS = 8, PWARPS = 16, RWARPS = 4, BWARPS = 2;
 constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;
 constexpr int NTHREADS = 1024;          // 32 warps, the last one idle
-// Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
-constexpr int REG_EPI = 96, REG_PROD = 64, REG_RAW = 24, REG_MISC = 40;
-static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
+// What depends on the tokens of an item.  64 tokens a weight tile halve the decoding of an expert with many, but there is room for one
+// accumulator buffer only (the tensor core waits while a block's sums are read) and for four B tiles instead of eight.
+template <int NT> struct Tok {
+    static constexpr int B_STAGE = 2 * NT * BK * 2;  // hi and lo rows: 8 or 16 KB
+    static constexpr int NB = 64 / NT;               // accumulator buffers
+    static constexpr int BUF_COLS = 2 * 2 * NT;      // two tiles x (hi, lo) x tokens
+    static constexpr int BSLOTS = 256 / NT;          // ring of B in shared memory (its copies take over a microsecond)
+    // Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
+    static constexpr int REG_EPI = NT == 64 ? 112 : 96, REG_PROD = NT == 64 ? 56 : 64, REG_RAW = 24, REG_MISC = 40;
+    static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
+};
+constexpr int B_BYTES = 65536;          // of the B ring
 static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA == 30, "roles fill warpgroups");
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
-constexpr int STAGES = 4, BSTAGES = 8;  // rings of A (tensor memory) and of B (shared memory: its copies take over a microsecond)
-constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + STAGES * 2 * A_COLS;
-static_assert(BSTAGES == 2 * STAGES, "a stage number names its B slot");
+constexpr int STAGES = 4, BSTAGES = 2 * STAGES;  // ring of A (tensor memory); barriers of a stage, which is known by its number mod BSTAGES
+constexpr int A_COL0 = 256, TMEM_COLS = A_COL0 + STAGES * 2 * A_COLS;
+static_assert(Tok<32>::NB * Tok<32>::BUF_COLS == A_COL0 && Tok<64>::NB * Tok<64>::BUF_COLS == A_COL0, "accumulators");
+static_assert(Tok<32>::BSLOTS * Tok<32>::B_STAGE == B_BYTES && Tok<64>::BSLOTS * Tok<64>::B_STAGE == B_BYTES, "B ring");
+static_assert(Tok<32>::BSLOTS == BSTAGES && Tok<64>::BSLOTS == STAGES, "a B slot is freed by the stage BSTAGES or STAGES earlier");
 static_assert(TMEM_COLS == 512, "tensor memory");
-constexpr int SCL = 8;                  // ring of block scales: producers are at most NB + 3 blocks ahead of the epilogue
+constexpr int SCL = 8;                  // ring of block scales: producers are at most five blocks ahead of the epilogue
 constexpr uint32_t kMinScaleH = 0x4C004C00u;  // the mins' A values are 16 times the mins: their low halves then lose nothing that matters
 constexpr float kMinScale = 16.f;             // (2^-28 absolute), and a min may still be as large as 4,000
 
@@ -74,11 +81,11 @@ template <int T> constexpr int kBB = T == T_Q4_K ? 144 : 98;
 struct Item {
     const uint8_t* pa;  // tile 0, first row
     const uint8_t* pb;  // tile 1
-    int prow, m;        // first packed row, tokens (1..NT)
+    int prow, m;        // first packed row, tokens
     int r0, pad;        // first output row
 };
 
-template <bool PAIR>
+template <bool PAIR, int NT>
 __device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int nseg, const int* pre, const SegDesc* __restrict__ seg) {
     const int tile = item / row_tiles, rt = item - tile * row_tiles;
     int lo = 0, hi = nseg;  // pre[lo] <= tile < pre[lo + 1]
@@ -98,8 +105,8 @@ __device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int
     return it;
 }
 
-// Tokens of the B tile: the smallest of 8, 16, 32 that holds the item.
-__device__ __forceinline__ int tile_tokens(int m) { return m <= 8 ? 8 : m <= 16 ? 16 : 32; }
+// Tokens of the B tile: the smallest of 8, 16, 32, 64 that holds the item.
+__device__ __forceinline__ int tile_tokens(int m) { return m <= 8 ? 8 : m <= 16 ? 16 : m <= 32 ? 32 : 64; }
 
 // An item's stages: for every eight blocks (or the rest) their 64-element stages, then those of the mins (Q4_K): with up to four
 // blocks one stage holds the hi parts of the up to 32 mins in its first 32 columns and the lo parts in the others (the operand row
@@ -246,7 +253,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm vol
 template <int T> struct Layout {
     static constexpr int RSTAGES = 3;
     static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
-    static constexpr int BARS = 2 * BSTAGES + 2 * (RSTAGES + NB);
+    static constexpr int BARS = 2 * BSTAGES + 2 * (RSTAGES + 2);
     static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
     static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
     static constexpr int MINS = T == T_Q4_K ? PWARPS * 32 * 8 * 10 : 0;  // 8 + 2 bytes per block and producer thread
@@ -270,10 +277,12 @@ struct StageCount {
     }
 };
 
-template <int T, bool PAIR>  // PAIR: both tiles from seg.wa (256 rows, fp32 results); else gate and up rows, silu(g) * u
+template <int T, bool PAIR, int NT>  // NT: tokens of an item; PAIR: both tiles from seg.wa (256 rows, fp32 results); else gate and up rows, silu(g) * u
 __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     using L = Layout<T>;
     using R = Raw<T>;
+    using K = Tok<NT>;
+    constexpr int NB = K::NB, BUF_COLS = K::BUF_COLS, B_STAGE = K::B_STAGE;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (s32(smem_raw) & 1023u)) & 1023u);
     uint64_t* full = reinterpret_cast<uint64_t*>(base);
@@ -287,7 +296,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     Item* itab = reinterpret_cast<Item*>((reinterpret_cast<uintptr_t>(pre + kMaxSeg + 1) + 7) & ~(uintptr_t)7);
     float* scl = reinterpret_cast<float*>(base + L::HEAD);  // [SCL][2][128]
     uint8_t* b_ring = base + L::LOW;
-    uint8_t* p = b_ring + BSTAGES * B_STAGE;
+    uint8_t* p = b_ring + B_BYTES;
     uint8_t* book = p;
     if constexpr (T == T_IQ3_XXS) {
         book += (kMmBookAlign - (s32(p) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
@@ -345,16 +354,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     const int n_items = nseg > 0 ? pre[nseg] * row_tiles : 0;
     const int GR = gridDim.x;
     const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + GR - 1) / GR : 0;
-    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, pre, A.seg);
+    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR, NT>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, pre, A.seg);
     __syncthreads();
     auto item = [&](int k) {
-        return k < kLocalItems ? itab[k] : decode_item<PAIR>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, pre, A.seg);
+        return k < kLocalItems ? itab[k] : decode_item<PAIR, NT>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, pre, A.seg);
     };
     bool ok = true;
 
     if (warp < EWARPS) {
         // ---------------- epilogue: TMEM lane = weight row ----------------
-        reg_inc<REG_EPI>();
+        reg_inc<K::REG_EPI>();
         const int quad = warp & 3, hsel = warp >> 2;
         const int r = quad * 32 + lane;
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -372,11 +381,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             const int nte = tile_tokens(it.m), half = nte >> 1;
             const float rs = rs_next;
             rs_next = k + 1 < my_items ? row_scale(k + 1) : 0.f;
-            float acc[2][16];
+            float acc[2][NT / 2];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) acc[mt][j] = 0.f;
+                for (int j = 0; j < NT / 2; ++j) acc[mt][j] = 0.f;
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
                 for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0); ++b) {  // the last one: the mins
@@ -391,13 +400,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     }
                     const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * nte);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {  // eight tokens a load; 32-token tiles have sixteen per warp
-                        if (h == 0 || nte == 32) {
+                    for (int h = 0; h < NT / 16; ++h) {  // eight tokens a load; a warp has half of the tile's
+                        if (h == 0 || 16 * h < nte) {
                             uint32_t v[2][16];
                             tmem_ld16(col + 16 * h, v[0]);
                             tmem_ld16(col + 2 * NT + 16 * h, v[1]);
                             tmem_ld_wait();
-                            if (h == 1 || nte != 32) {  // read: hand the buffer back before the arithmetic
+                            if (16 * h + 16 >= nte) {  // read: hand the buffer back before the arithmetic
                                 tc_fence_before();
                                 __syncwarp();
                                 if (lane == 0) mb_arrive(&tfree[buf]);
@@ -417,7 +426,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             const int t0 = hsel * half, cnt = min(half, it.m - t0);
             float* o = A.out + (size_t)(it.prow + t0) * A.n_out + it.r0 + r;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {  // all results first (independent chains), then the stores
+            for (int j = 0; j < NT / 2; ++j) {  // all results first (independent chains), then the stores
                 const float f = __shfl_sync(0xffffffffu, rs, j);
                 acc[0][j] *= f;
                 acc[1][j] *= f;
@@ -425,7 +434,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
             if (PAIR && A.row_dst) {  // expert parallel: the owner's (token, slot) row
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
+                for (int j = 0; j < NT / 2; ++j)
                     if (j < cnt) {
                         float* d = A.row_dst[it.prow + t0 + j] + it.r0 + r;
                         d[0] = acc[0][j];
@@ -433,7 +442,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j, o += A.n_out)
+                for (int j = 0; j < NT / 2; ++j, o += A.n_out)
                     if (j < cnt) {
                         o[0] = acc[0][j];
                         if constexpr (PAIR) o[TILE_M] = acc[1][j];
@@ -442,7 +451,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         }
     } else if (warp < W_RAW) {
         // ---------------- producers ----------------
-        reg_dec<REG_PROD>();
+        reg_dec<K::REG_PROD>();
         const int pw = warp - EWARPS, odd = pw >> 3, tile = (pw >> 2) & 1, r = (pw & 3) * 32 + lane;
         const uint32_t tlane = tmem_base + A_COL0 + (uint32_t)(tile * A_COLS) + ((uint32_t)((pw & 3) * 32) << 16);
         const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
@@ -511,7 +520,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
     } else if (warp < W_B) {
-        reg_dec<REG_RAW>();
+        reg_dec<K::REG_RAW>();
         // ---------------- raw rows: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
         const int rw = warp - W_RAW, c16 = (lane & 7) * 16, row0 = (rw & 1) * (TILE_M / 2);  // half a tile per warp
         int rst = 0;
@@ -549,7 +558,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         }
         cp_async_wait_all();
     } else {
-        reg_dec<REG_MISC>();
+        reg_dec<K::REG_MISC>();
         if (warp < W_MMA) {
         // ---------------- B tiles: rows 2 t, 2 t + 1 = hi and lo of token t; lane = unit lane % 8 of row lane / 8 (+ 8 per step, the
         // other warp takes the four between) ----------------
@@ -559,20 +568,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             const int steps = tile_tokens(it.m) / 4;  // 8 rows each
-            const uint16_t* src[8];  // operand array rows of this lane's B rows
+            uint32_t src[NT / 4];  // operand array rows of this lane's B rows, in 16-byte units
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < NT / 4; ++i) {
                 const int br = 8 * i + brow, pr = it.prow + min(br >> 1, it.m - 1);
                 const uint32_t orow = i < steps ? (uint32_t)(A.row_token ? A.row_token[pr] : pr) : 0u;
-                src[i] = A.op + (size_t)(2u * orow + (br & 1)) * pitch + 8 * (lane & 7);
+                src[i] = (2u * orow + (br & 1)) * (uint32_t)(pitch >> 3) + (lane & 7);
             }
-            auto stage = [&](int off) {  // off: elements from src
-                ok = warp_all(mb_wait(&empty[q.q], q.turn ^ 1u, A.status, 4));  // BSTAGES stages earlier
+            auto stage = [&](int off) {  // off: elements from the row's start
+                ok = warp_all(NT == 64 ? q.wait(empty, A.status, 4) : mb_wait(&empty[q.q], q.turn ^ 1u, A.status, 4));
                 if (!ok) return;
-                uint8_t* d = b_ring + q.q * B_STAGE + at;
+                uint8_t* d = b_ring + (NT == 64 ? q.slot() : q.q) * B_STAGE + at;
+                const uint16_t* from = A.op + off;
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (i < steps) cp_async16(d + i * 1024, src[i] + off);
+                for (int i = 0; i < NT / 4; ++i)
+                    if (i < steps) cp_async16(d + i * 1024, from + (size_t)src[i] * 8);
                 cp_async_arrive(&full[q.q]);
                 q.advance(1);
             };
@@ -580,11 +590,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                 const int bn = min(8, nblk - b0);
                 for (int b = 0; b < bn && ok; ++b) {
 #pragma unroll 1
-                    for (int c = 0; c < 4 && ok; ++c) stage(c * BK);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) src[i] += 256;
+                    for (int c = 0; c < 4 && ok; ++c) stage((b0 + b) * 256 + c * BK);
                 }
-                const int sums = A.n_in - 256 * (b0 + bn) + 8 * b0;  // the mins read the sums behind the row
+                const int sums = A.n_in + 8 * b0;  // the mins read the sums behind the row
                 for (int u = 0; u < min_stages<T>(bn) && ok; ++u) stage(sums);
             }
         }
@@ -612,7 +620,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                             if (!ok) break;
                             tc_fence_after();    // A: written to tensor memory by the producers
                             fence_async_smem();  // B: written to shared memory by the B warps' copies
-                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(q.slot() * 2 * A_COLS), b_lo = b_lo0 + (uint32_t)(q.q * (B_STAGE >> 4));
+                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(q.slot() * 2 * A_COLS), b_lo = b_lo0 + (uint32_t)((NT == 64 ? q.slot() : q.q) * (B_STAGE >> 4));
                             uint32_t acc = c == 0 ? 0u : 1u;
 #pragma unroll
                             for (int ks = 0; ks < 4; ++ks) {
@@ -722,15 +730,15 @@ bool tc_handles(int type, int n_in, int n_out, bool fused) {
     return (type == T_Q4_K || type == T_IQ3_XXS) && n_in % 256 == 0 && n_out % (fused ? tg::TILE_M : 2 * tg::TILE_M) == 0;
 }
 
-template <int T, bool PAIR>
+template <int T, bool PAIR, int NT>
 static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
     using L = tg::Layout<T>;
-    size_t at = kMmSmemBase + L::LOW + tg::BSTAGES * tg::B_STAGE;
+    size_t at = kMmSmemBase + L::LOW + tg::B_BYTES;
     if (T == T_IQ3_XXS) at = (at + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign + sizeof(MmCodebook);
     const size_t smem = at + L::TAIL - kMmSmemBase;
     static_assert(L::BARS * 8 + 16 + (tg::kMaxSeg + 1) * 4 + 8 + tg::kLocalItems * sizeof(tg::Item) <= L::HEAD, "head too small");
     A.smem = (uint32_t)smem;
-    auto kern = tg::grouped_tc_kernel<T, PAIR>;
+    auto kern = tg::grouped_tc_kernel<T, PAIR, NT>;
     static SmemGrant grant;
     DNB_CUDA(grant_smem(grant, c->device, kern, smem));
     ProfScope prof_(c, st, PAIR ? "tc_down" : "tc_gate_up");
@@ -740,15 +748,23 @@ static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
 }
 
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
-                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst) {
+                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst, int tokens, int rows) {
     if (!tc_handles(type, n_in, n_out, fused) || nseg_max > tg::kMaxSeg) return DNB_DECLINED;
     int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
     if (rc) return rc;
     tg::Args A = {};
     A.seg = seg; A.nseg_dev = nseg_dev; A.nseg_max = nseg_max; A.n_in = n_in; A.n_out = n_out; A.rb = (int)row_bytes(type, n_in);
     A.op = op; A.row_token = row_token; A.out = out; A.row_dst = row_dst; A.status = c->status;
-    if (type == T_Q4_K) return fused ? launch_tc_t<T_Q4_K, false>(c, st, A) : launch_tc_t<T_Q4_K, true>(c, st, A);
-    return fused ? launch_tc_t<T_IQ3_XXS, false>(c, st, A) : launch_tc_t<T_IQ3_XXS, true>(c, st, A);
+    // Items of 64 tokens where hot experts have several tiles.  us a layer, 32 / 64 tokens an item, 2048 x 512 under a skewed router:
+    // IQ3_XXS from 256 tokens: 512 experts top 10, 512 tokens 287 / 254; 128 experts top 8, 512 tokens 243 / 213; 128 top 4 (1024 x 768), 300
+    // tokens 94 / 94; 128 top 10, 150 tokens 144 / 157.  Q4_K, whose decoding is cheaper, waits for the single accumulator and the shorter
+    // B ring (gate and up of the first chunk 131 / 138), so only with 96 rows a segment: 64 top 10, 700 tokens 303 / 292, 512 tokens 242 / 241.
+    const bool wide = type == T_IQ3_XXS ? tokens >= 256 : rows / nseg_max >= 96;
+#define DNB_TC(TY, PAIR) return wide ? launch_tc_t<TY, PAIR, 64>(c, st, A) : launch_tc_t<TY, PAIR, 32>(c, st, A)
+    if (type == T_Q4_K) { if (fused) DNB_TC(T_Q4_K, false); DNB_TC(T_Q4_K, true); }
+    if (fused) DNB_TC(T_IQ3_XXS, false);
+    DNB_TC(T_IQ3_XXS, true);
+#undef DNB_TC
 }
 
 }  // namespace dnb

@@ -46,11 +46,11 @@ def test_grouped_mma(orc, ctx, name, k, n):
 @pytest.mark.parametrize("name", ["Q4_K", "IQ3_XXS"])
 @pytest.mark.parametrize("e,ff,ne,k", [(256, 256, 8, 2), (768, 512, 16, 3), (2304, 256, 4, 1), (512, 1280, 24, 4)])
 def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
-    """Token counts on both sides of every hand-over (routing in two launches to 15, tensor-core router from 16, tcgen05 from 48),
-    with experts of one token to a full 32-token tile and more; K of 1 to 9 blocks."""
+    """Token counts on both sides of every hand-over (routing in two launches to 15, tensor-core router from 16, tcgen05 from 48, its
+    64-token items from 256 or with 96 rows an expert), with experts of one token to several full tiles; K of 1 to 9 blocks."""
     assert ctx.moe_config(1, e, ff, ne, k)
     L = make_layer(orc, ctx, 0, orc.TYPE_BY_NAME[name], e, ff, ne, k, bias=True, gate_row=True)
-    for nt in (2, 9, 15, 16, 47, 48, 49, 97):
+    for nt in (2, 9, 15, 16, 47, 48, 49, 97, 256, 257):
         h = orc.synth_normal(SEED, 50 + nt, 1.0, nt * e).reshape(nt, e)
         out, sels, wts = ctx.moe_block(0, h, want_routing=True)
         err, _ = check_block(orc, L, h, out, sels, wts)
