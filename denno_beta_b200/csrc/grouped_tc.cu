@@ -8,8 +8,9 @@
 //   Q4_K    : w = sc * q <= 945, s_b = d, and the mins: X = the sum of the sub-block's 32 activations
 //   IQ3_XXS : w = codebook magnitude * sign * (2 s + 1) <= 1922, s_b = d / 4
 // Every w is an integer below 2048 and exact in fp16, so a weight costs its decoding and nothing is rounded.  The mins are one
-// more block of K = sub-blocks: A = -(dmin * m) * 2^10 as fp16 hi and lo, B = X.  An activation is fp16 hi + lo (22 bits) of the
-// row times a power of two that puts its largest element into [512, 1024).
+// more block of K = sub-blocks: A = -(dmin * m) as fp16 hi and lo, times a power of two of the row's own that fits its largest
+// dmin into fp16's range whatever its size, B = X.  An activation is fp16 hi + lo (22 bits) of the row times a power of two that
+// puts its largest element into [512, 1024).
 //
 // What bounds it: a 64-element stage of two 128-row tiles is about 900 warp instructions of decoding (Q4_K; 1.7 per weight) on
 // four schedulers and 8 MMAs of N = 2 x tokens, the same order of time at 32 tokens; everything else has to stay out of the
@@ -72,9 +73,7 @@ static_assert(Tok<32>::NB * Tok<32>::BUF_COLS == A_COL0 && Tok<64>::NB * Tok<64>
 static_assert(Tok<32>::BSLOTS * Tok<32>::B_STAGE == B_BYTES && Tok<64>::BSLOTS * Tok<64>::B_STAGE == B_BYTES, "B ring");
 static_assert(Tok<32>::BSLOTS == BSTAGES && Tok<64>::BSLOTS == STAGES, "a B slot is freed by the stage BSTAGES or STAGES earlier");
 static_assert(TMEM_COLS == 512, "tensor memory");
-constexpr int SCL = 8;                  // ring of block scales: producers are at most five blocks ahead of the epilogue
-constexpr uint32_t kMinScaleH = 0x4C004C00u;  // the mins' A values are 16 times the mins: their low halves then lose nothing that matters
-constexpr float kMinScale = 16.f;             // (2^-28 absolute), and a min may still be as large as 4,000
+constexpr int SCL = 8;                  // ring of block scales (the mins count as a block): producers are at most five blocks ahead of the epilogue
 
 template <int T> constexpr int kBB = T == T_Q4_K ? 144 : 98;
 
@@ -221,9 +220,13 @@ __device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int, uint3
     }
 }
 // Stage u of the mins of one Q4_K row.  mm, dd: the last eight mins bytes of each block's header and its dmin, as the thread saved
-// them (PWARPS * 32 entries from block to block).
-__device__ __forceinline__ void mins_stage(const uint2* mm, const uint16_t* dd, int blocks, int u, uint32_t (&o)[32]) {
+// them (PWARPS * 32 entries from block to block); top: the bits of the largest |dmin|, in the upper half.  Returns what undoes the
+// scaling: with e the exponent field of the largest |dmin| < 2^(e - 14), dmin times 2^(24 - e) (2^15 at most) is below 2^10 and
+// dmin * m <= 63 * dmin below fp16's largest number.
+__device__ __forceinline__ float mins_stage(const uint2* mm, const uint16_t* dd, int blocks, int u, uint32_t top, uint32_t (&o)[32]) {
     const bool both = blocks <= 4;
+    const uint32_t ex = min(30u, 39u - (top >> 26));  // exponent field of the scale, a power of two
+    const uint32_t neg = ((ex << 10) | 0x8000u) * 0x10001u;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {  // the eight sub-blocks of a block: four columns
         const bool low = both ? c >= 4 : u != 0;
@@ -231,7 +234,7 @@ __device__ __forceinline__ void mins_stage(const uint2* mm, const uint16_t* dd, 
         const bool live = blk < blocks;
         const uint2 h = mm[(live ? blk : 0) * PWARPS * 32];
         const uint32_t d = live ? dd[blk * PWARPS * 32] : 0u;
-        const uint32_t dm = h2mul(d * 0x10001u, kMinScaleH ^ 0x80008000u);  // -16 * dmin
+        const uint32_t dm = h2mul(d * 0x10001u, neg);  // -scale * dmin
         const uint32_t mn[2] = {h.x & 0x3f3f3f3fu, ((h.y >> 4) & 0x0f0f0f0fu) | ((h.x >> 2) & 0x30303030u)};  // kquant.rs:878-887
 #pragma unroll
         for (int k = 0; k < 4; ++k) {  // sub-blocks 2 k, 2 k + 1: dmin * m rounded, or exactly what that left over
@@ -240,6 +243,7 @@ __device__ __forceinline__ void mins_stage(const uint2* mm, const uint16_t* dd, 
             o[4 * c + k] = low ? h2fma(dm, m2, hi ^ 0x80008000u) : hi;
         }
     }
+    return __uint_as_float((142u - ex) << 23);  // 2^-(ex - 15)
 }
 
 __device__ __forceinline__ float swiglu_fast(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
@@ -392,12 +396,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     ok = warp_all(mb_wait(&tfull[buf], pb, A.status, 3));
                     if (!ok) break;
                     tc_fence_after();
-                    float s[2] = {1.f / kMinScale, 1.f / kMinScale};
-                    if (b < bn) {
-                        s[0] = scl[(sc * 2) * TILE_M + r];
-                        s[1] = scl[(sc * 2 + 1) * TILE_M + r];
-                        sc = (sc + 1) & (SCL - 1);
-                    }
+                    const float s[2] = {scl[(sc * 2) * TILE_M + r], scl[(sc * 2 + 1) * TILE_M + r]};
+                    sc = (sc + 1) & (SCL - 1);
                     const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * nte);
 #pragma unroll
                     for (int h = 0; h < NT / 16; ++h) {  // eight tokens a load; a warp has half of the tile's
@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             if constexpr (T == T_IQ3_XXS) off = (uint32_t)(uintptr_t)(tile ? it.pb : it.pa) + (uint32_t)r * A.rb;
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
+                uint32_t top = 0u;
                 for (int b = 0; b < bn; ++b) {
                     ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
                     if (!ok) break;
@@ -491,6 +492,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                                 sc = (sc + 1) & (SCL - 1);
                             }
                             if constexpr (T == T_Q4_K) {
+                                top = max(top, in.h.x & 0x7fff0000u);
                                 mm[b * PWARPS * 32] = make_uint2(in.h.z, in.h.w);
                                 dd[b * PWARPS * 32] = (uint16_t)(in.h.x >> 16);
                             }
@@ -512,9 +514,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                     const int nm = min_stages<T>(bn);
                     if (odd < nm) {
                         uint32_t o[32];
-                        mins_stage(mm, dd, bn, odd, o);
+                        const float s = mins_stage(mm, dd, bn, odd, top, o);
+                        if (!odd) scl[(sc * 2 + tile) * TILE_M + r] = s;
                         hand_over(o);
                     }
+                    sc = (sc + 1) & (SCL - 1);
                     q.advance(nm);
                 }
             }

@@ -6,8 +6,9 @@ SEED = 0xD3770B200
 
 
 def make_layer(orc, ctx, layer, ty, e, ff, ne, k, *, shared=True, bias=False, gate_row=False, norm=True, seed=SEED,
-               ty_down=None):
-    """Generates the layer on the host, registers it and returns the oracle's Layer."""
+               ty_down=None, edit=None):
+    """Generates the layer on the host, registers it and returns the oracle's Layer.  edit(name, blocks): changes the bytes of
+    "gate", "up" or "down" in place before they are registered."""
     from denno_beta_b200 import cuda as cu
 
     ty_down = ty if ty_down is None else ty_down
@@ -17,6 +18,9 @@ def make_layer(orc, ctx, layer, ty, e, ff, ne, k, *, shared=True, bias=False, ga
     gate = orc.synth_blocks(ty, seed, tid + 0, nb_gu)
     up = orc.synth_blocks(ty, seed, tid + 1, nb_gu)
     down = orc.synth_blocks(ty_down, seed, tid + 2, nb_d)
+    if edit:
+        for name, blocks in (("gate", gate), ("up", up), ("down", down)):
+            edit(name, blocks)
     assert ctx.register_experts(layer, cu.GATE, ty, e, ff, ne, gate)
     assert ctx.register_experts(layer, cu.UP, ty, e, ff, ne, up)
     assert ctx.register_experts(layer, cu.DOWN, ty_down, ff, e, ne, down)

@@ -112,3 +112,27 @@ def test_hyper_edges(orc, ctx, hc, lr, nts):
         want = np.stack([orc.hc_combine(r, b, inj) for r, b, (_, inj) in zip(res, blk, mix)])
         for _ in range(3):
             assert rel_err(ctx.hc_moe_block(0, res), want) <= 5e-5
+
+
+@pytest.mark.parametrize("e,ff", [(512, 256), (1280, 1280), (2304, 512)])
+@pytest.mark.parametrize("nt", [33, 64, 300])
+def test_q4k_mins_of_any_size(orc, ctx, e, ff, nt):
+    """Q4_K blocks whose dmin is fp16's largest number, or subnormal: dmin * m reaches 4e6, far outside fp16, in rows of all three
+    matrices, on both expert kernels of a chunk and with one and two stages of mins.  The other rows do not feel it."""
+    ne, k, row = 4, 2, 7
+
+    def edit(name, blocks):
+        n_out, n_in = (e, ff) if name == "down" else (ff, e)
+        b = blocks.reshape(ne, n_out, n_in // 256, 144)
+        b[:, row, :, 2:4] = np.array([65504.0], np.float16).view(np.uint8)
+        b[:, row + 1, 0, 2:4] = np.array([65504.0], np.float16).view(np.uint8)  # beside blocks of ordinary size
+        b[:, row + 2, :, 2:4] = np.array([6e-8], np.float16).view(np.uint8)
+
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.Q4_K, e, ff, ne, k, edit=edit)
+    h = orc.synth_normal(SEED, 90 + nt, 1.0, nt * e).reshape(nt, e)
+    out, sels, wts = ctx.moe_block(0, h, want_routing=True)
+    assert np.isfinite(out).all()
+    want = orc.moe_experts_given(L, orc.rmsnorm(h, np.ones(e, np.float32)), sels, wts)
+    for rows in (slice(row, row + 2), slice(row + 2, e)):
+        assert rel_err(out[:, rows], want[:, rows]) <= 2e-4

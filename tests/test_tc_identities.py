@@ -42,6 +42,37 @@ def _q4k_fields(blocks, n_blocks):
     return d, dmin, sc, m, q.reshape(n_blocks, 256)
 
 
+def _mins_operand(dmin, m):
+    """The A operand of the mins as csrc/grouped_tc.cu forms it for one row: dmin [blocks] fp16, m [blocks, 8] -> (hi, lo) fp16
+    and the power of two both carry.  Each step is one fp16 operation."""
+    ex = min(30, 39 - int(np.max(dmin.view(np.uint16) & 0x7FFF) >> 10))
+    scale = np.float16(2.0 ** (ex - 15))
+    dm = dmin * -scale
+    prod = dm.astype(np.float64)[:, None] * m
+    hi = prod.astype(np.float16)
+    return hi, (prod - hi.astype(np.float64)).astype(np.float16), float(scale)  # the fma rounds the exact remainder once
+
+
+def test_q4k_mins_of_any_size_fit_fp16():
+    """Every exponent of the largest dmin of a row, up to fp16's largest number: nothing overflows; the product is exact where the
+    scaled dmin is a normal number, and off by 2^-35 of the row's largest min where it is not."""
+    rng = np.random.RandomState(4)
+    m = np.tile(np.array([0, 1, 2, 31, 32, 61, 62, 63]), (8, 1))
+    for top in range(31):
+        for _ in range(50):
+            bits = ((rng.randint(0, top + 1, 8) << 10) | rng.randint(0, 1024, 8) | (rng.randint(0, 2, 8) << 15)).astype(np.uint16)
+            bits[rng.randint(8)] = (top << 10) | 0x3FF
+            dmin = bits.view(np.float16)
+            with np.errstate(over="raise"):
+                hi, lo, scale = _mins_operand(dmin, m)
+            assert np.isfinite(hi).all() and np.isfinite(lo).all()
+            want = -(dmin.astype(np.float64)[:, None] * m)
+            err = np.abs((hi.astype(np.float64) + lo.astype(np.float64)) / scale - want)
+            normal = (np.abs(dmin.astype(np.float64)) * scale >= 2.0 ** -14) | (scale >= 1.0)
+            assert not err[normal].any()
+            assert err.max() <= 2.0 ** -35 * 64 * np.abs(dmin.astype(np.float64)).max()
+
+
 def test_q4k_integer_weight_decomposition(orc):
     k, n = 1024, 24
     nb = k // 256
@@ -62,11 +93,10 @@ def test_q4k_integer_weight_decomposition(orc):
     assert np.array_equal(c.astype(np.float64), -1024.0 * sc)   # six bits times 2^10: exact
     fma = (big.astype(np.float64) * sc[:, :, None] + c.astype(np.float64)[:, :, None]).astype(np.float16)  # rounds once
     assert np.array_equal(fma.astype(np.int64), iw)
-    # (2) -(dmin * m) as fp16 hi + lo is exact
+    # (2) -(dmin * m) times the row's power of two is exact as fp16 hi + lo
     v = -(dmin[:, None].astype(np.float64) * m)
-    hi = v.astype(np.float16)
-    lo = (v - hi.astype(np.float64)).astype(np.float16)
-    assert np.array_equal(hi.astype(np.float64) + lo.astype(np.float64), v)
+    hi, lo, scale = _mins_operand(dmin.astype(np.float16), m)
+    assert np.array_equal((hi.astype(np.float64) + lo.astype(np.float64)) / scale, v)
     # (3) the decomposition: block sums scaled by d, minus the offsets against the sub-block sums of x
     xs = x.astype(np.float64).reshape(nb, 8, 32)
     main = np.einsum("rbsi,bsi->rb", iw.reshape(n, nb, 8, 32).astype(np.float64), xs) * d.reshape(n, nb)
