@@ -31,8 +31,8 @@
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
 // Persistent, one CTA per SM; items (segment, 32- or 64-token tile, 128 rows x 2) dealt round-robin.
 //
-// Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, us gate/up + down as bracketed by events: Q4_K 174 + 90 (three
-// bf16 products) -> 131 + 84, IQ3_XXS 343 + 180 -> 135 + 76.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
+// Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, us gate/up + down as bracketed by events: Q4_K 175 + 84 (three
+// bf16 products, a seventh of the accuracy) -> 122 + 83, IQ3_XXS 343 + 180 -> 122 + 73.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
 // commit; without the decoding a copy of the kernel was only 7 % faster.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -220,12 +220,9 @@ __device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int, uint3
     }
 }
 // Stage u of the mins of one Q4_K row.  mm, dd: the last eight mins bytes of each block's header and its dmin, as the thread saved
-// them (PWARPS * 32 entries from block to block); top: the bits of the largest |dmin|, in the upper half.  Returns what undoes the
-// scaling: with e the exponent field of the largest |dmin| < 2^(e - 14), dmin times 2^(24 - e) (2^15 at most) is below 2^10 and
-// dmin * m <= 63 * dmin below fp16's largest number.
-__device__ __forceinline__ float mins_stage(const uint2* mm, const uint16_t* dd, int blocks, int u, uint32_t top, uint32_t (&o)[32]) {
+// them (PWARPS * 32 entries from block to block); ex: exponent field of the scale, a power of two.
+__device__ __forceinline__ void mins_stage(const uint2* mm, const uint16_t* dd, int blocks, int u, uint32_t ex, uint32_t (&o)[32]) {
     const bool both = blocks <= 4;
-    const uint32_t ex = min(30u, 39u - (top >> 26));  // exponent field of the scale, a power of two
     const uint32_t neg = ((ex << 10) | 0x8000u) * 0x10001u;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {  // the eight sub-blocks of a block: four columns
@@ -243,7 +240,6 @@ __device__ __forceinline__ float mins_stage(const uint2* mm, const uint16_t* dd,
             o[4 * c + k] = low ? h2fma(dm, m2, hi ^ 0x80008000u) : hi;
         }
     }
-    return __uint_as_float((142u - ex) << 23);  // 2^-(ex - 15)
 }
 
 __device__ __forceinline__ float swiglu_fast(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
@@ -312,7 +308,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         return;
     }
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // The warp's number, told to be the same for its lanes: what depends on it leaves the 64 registers a thread.  Spills in bytes, stores +
+    // loads: Q4_K 48 + 88 -> 0 at 32 tokens, 112 + 148 -> 72 + 68 at 64; IQ3_XXS at 64 64 + 100 -> 36 + 28.  us gate/up + down, 64 experts top 10,
+    // 1024 tokens evenly routed: Q4_K at 64 166 + 106 -> 145 + 103, IQ3_XXS 160 + 97 -> 150 + 97.  IQ3_XXS down at 32 never spilled and loses:
+    // 128 -> 135.
+    constexpr bool kUniform = !(T == T_IQ3_XXS && PAIR && NT == 32);
+    const int tid = threadIdx.x, warp = kUniform ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
     const int nblk = A.n_in / 256;
     const int row_tiles = A.n_out / (PAIR ? 2 * TILE_M : TILE_M);
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             if constexpr (T == T_IQ3_XXS) off = (uint32_t)(uintptr_t)(tile ? it.pb : it.pa) + (uint32_t)r * A.rb;
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
-                uint32_t top = 0u;
+                uint32_t top = 0u;  // bits of the largest |dmin|, in the upper half
                 for (int b = 0; b < bn; ++b) {
                     ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
                     if (!ok) break;
@@ -513,12 +514,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                 if constexpr (T == T_Q4_K) {
                     const int nm = min_stages<T>(bn);
                     if (odd < nm) {
+                        // e = top >> 26, the exponent field of the largest |dmin| < 2^(e - 14): times 2^(24 - e) (2^15 at most) it is below
+                        // 2^10, and dmin * m <= 63 * dmin below fp16's largest number
+                        const uint32_t ex = min(30u, 39u - (top >> 26));
+                        if (!odd) {
+                            scl[(sc * 2 + tile) * TILE_M + r] = __uint_as_float((142u - ex) << 23);  // 2^-(ex - 15): undoes the scale
+                            sc = (sc + 1) & (SCL - 1);
+                        }
                         uint32_t o[32];
-                        const float s = mins_stage(mm, dd, bn, odd, top, o);
-                        if (!odd) scl[(sc * 2 + tile) * TILE_M + r] = s;
+                        mins_stage(mm, dd, bn, odd, ex, o);
                         hand_over(o);
                     }
-                    sc = (sc + 1) & (SCL - 1);
                     q.advance(nm);
                 }
             }
