@@ -765,11 +765,20 @@ int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const S
     tg::Args A = {};
     A.seg = seg; A.nseg_dev = nseg_dev; A.nseg_max = nseg_max; A.n_in = n_in; A.n_out = n_out; A.rb = (int)row_bytes(type, n_in);
     A.op = op; A.row_token = row_token; A.out = out; A.row_dst = row_dst; A.status = c->status;
-    // Items of 64 tokens where hot experts have several tiles.  us a layer, 32 / 64 tokens an item, 2048 x 512 under a skewed router:
-    // IQ3_XXS from 256 tokens: 512 experts top 10, 512 tokens 287 / 254; 128 experts top 8, 512 tokens 243 / 213; 128 top 4 (1024 x 768), 300
-    // tokens 94 / 94; 128 top 10, 150 tokens 144 / 157.  Q4_K, whose decoding is cheaper, waits for the single accumulator and the shorter
-    // B ring (gate and up of the first chunk 131 / 138), so only with 96 rows a segment: 64 top 10, 700 tokens 303 / 292, 512 tokens 242 / 241.
-    const bool wide = type == T_IQ3_XXS ? tokens >= 256 : rows / nseg_max >= 96;
+    // Items of 64 tokens, or of 32.  Where no expert has more than 32 tokens, 64 save no decoding and cost a second accumulator and half of
+    // the B ring: 11 to 14 % of a layer (Q4_K), 5 to 8 % (IQ3_XXS); where experts have more, they gain up to 30 %.  That depends on how the
+    // tokens spread, which the host does not know.  With 40 rows a segment (IQ3_XXS: 24) 64 are the better choice either way; with fewer Q4_K
+    // stays at 32, while IQ3_XXS, which loses little where 64 do not help, takes them from 256 tokens on.  us a layer, 32 / 64 tokens an
+    // item, even routing, and skewed by -1.1 ln rank, 2048 x 512:
+    //   Q4_K, 512 experts top 10: 512 tokens (11 rows a segment) 431 / 493, 248 / 238; 1024 tokens (22) 490 / 558, 416 / 364
+    //         128 experts top 8: 384 tokens (27) 163 / 190, 181 / 179; 512 (36) 210 / 205, 211 / 197; 700 (49) 270 / 220, 256 / 238
+    //         64 experts top 10: 200 tokens (34) 139 / 132, 144 / 156; 1024 (173) 381 / 315, 381 / 317
+    //   IQ3_XXS, 512 experts top 10: 200 tokens 438 / 474, 166 / 151; 256 tokens 440 / 477, 176 / 160; 512 tokens 479 / 511, 275 / 238
+    //         128 experts top 8: 200 tokens (14) 166 / 177, 139 / 144; 384 (27) 179 / 191, 199 / 179; 512 (36) 234 / 201, 233 / 199
+    // Over six such shapes and 48 to 1024 tokens the rule is 0.1 % / 1.7 % (Q4_K, even / skewed) and 1.6 % / 1.0 % (IQ3_XXS) behind the better.
+    // (Tried: the choice on the device, from the segments' token counts.  Both kernels launched, one without items: 1.5 us each.  One
+    // kernel with both bodies, or with items of either size: 7 to 15 % slower, in registers and code.)
+    const bool q4 = type == T_Q4_K, wide = rows >= (q4 ? 40 : 24) * nseg_max || (!q4 && tokens >= 256);
 #define DNB_TC(TY, PAIR) return wide ? launch_tc_t<TY, PAIR, 64>(c, st, A) : launch_tc_t<TY, PAIR, 32>(c, st, A)
     if (type == T_Q4_K) { if (fused) DNB_TC(T_Q4_K, false); DNB_TC(T_Q4_K, true); }
     if (fused) DNB_TC(T_IQ3_XXS, false);

@@ -47,7 +47,8 @@ def test_grouped_mma(orc, ctx, name, k, n):
 @pytest.mark.parametrize("e,ff,ne,k", [(256, 256, 8, 2), (768, 512, 16, 3), (2304, 256, 4, 1), (512, 1280, 24, 4)])
 def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
     """Token counts on both sides of every hand-over (routing in two launches to 15, tensor-core router from 16, tcgen05 from 48, its
-    64-token items from 256 or with 96 rows an expert), with experts of one token to several full tiles; K of 1 to 9 blocks."""
+    64-token items with 24 or 32 rows an expert or from 256 or 640 tokens), with experts of one token to several full tiles; K of 1 to 9
+    blocks.  From 48 tokens on a token's bits do not depend on the size of its chunk."""
     assert ctx.moe_config(1, e, ff, ne, k)
     L = make_layer(orc, ctx, 0, orc.TYPE_BY_NAME[name], e, ff, ne, k, bias=True, gate_row=True)
     for nt in (2, 9, 15, 16, 47, 48, 49, 97, 256, 257):
@@ -56,6 +57,9 @@ def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
         err, _ = check_block(orc, L, h, out, sels, wts)
         assert err <= (5e-5 if nt < 16 else 2e-4), "nt %d: %.3g" % (nt, err)
         assert np.array_equal(out.view(np.uint32), ctx.moe_block(0, h).view(np.uint32)), "nt %d: bits of a replay" % nt
+        if nt >= 256:
+            part = ctx.moe_block(0, h[5:53])
+            assert np.array_equal(part.view(np.uint32), out[5:53].view(np.uint32)), "nt %d: bits of a chunk of 48" % nt
 
 
 @pytest.mark.parametrize("up,down,e,ff", [("Q5_K", "Q8_0", 768, 288), ("Q4_K", "Q6_K", 512, 768), ("IQ3_XXS", "Q4_K", 512, 256)])
