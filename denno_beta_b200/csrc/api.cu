@@ -363,11 +363,11 @@ static int tc_type(const Layer& L, int first, int last) {
 // 2048 x 512, top 10 of 512, mma.sync / tcgen05: Q4_K evenly routed 173 / 222 at 32 tokens, 216 / 275 at 48, 250 / 304 at 64; under a
 // skewed router 106 / 96, 129 / 100, 155 / 103.  At 48 either choice loses the same factor at worst (1.27).
 constexpr int kTcMin = 48;
-static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMin : c->exact_min_nt; }
+static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMin : c->tc_min_iq3; }
 
-static bool umma_eligible(const dnb_ctx* c, const Layer& L, int nt) {
+static bool tc_eligible(const dnb_ctx* c, const Layer& L, int nt) {
     const Model& M = c->model;
-    if (!c->use_umma || !c->ws.op_ok) return false;
+    if (!c->use_tc || !c->ws.op_ok) return false;
     const int ty = tc_type(L, 0, 3);
     if (ty < 0 || nt < tc_min_tokens(c, ty) || !tc_handles(ty, M.e, M.ff, true) || !tc_handles(ty, M.ff, M.e, false)) return false;
     if (L.has_shared()) {  // the shared expert rides in the same launches as one more segment
@@ -377,7 +377,7 @@ static bool umma_eligible(const dnb_ctx* c, const Layer& L, int nt) {
 }
 
 // op_ready: the operand rows of x are in the workspace (written with the RMSNorm).
-static int experts_dev_umma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts,
+static int experts_dev_tc(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts,
                             float* out, const float* residual = nullptr, int k = -1, int ne = -1, int with_shared = -1, bool op_ready = false) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
@@ -474,8 +474,8 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out, 
         rc = block_dev_decode(c, layer, h, out, residual);
         if (rc != DNB_DECLINED) return rc;
     }
-    const bool mma = nt > 1 && mm_eligible(c, L) && !umma_eligible(c, L, nt);
-    if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !mma && !umma_eligible(c, L, nt)) {
+    const bool mma = nt > 1 && mm_eligible(c, L) && !tc_eligible(c, L, nt);
+    if (nt > 1 && nt <= kDecodeBatchMax && c->decode_fast && !mma && !tc_eligible(c, L, nt)) {
         rc = block_dev_decode_batch(c, layer, h, nt, out, residual);
         if (rc != DNB_DECLINED) return rc;
     }
@@ -488,7 +488,7 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out, 
         if (rc != DNB_DECLINED) return rc;
     }
     // the RMSNorm kernel writes the router's operand (three bf16 parts of the normalised rows) and the experts' in the same pass
-    const bool umma = umma_eligible(c, L, nt), split_in_prep = L.norm_w && router_tc_eligible(c, L, nt), op_in_prep = L.norm_w && umma;
+    const bool on_tc = tc_eligible(c, L, nt), split_in_prep = L.norm_w && router_tc_eligible(c, L, nt), op_in_prep = L.norm_w && on_tc;
     if (op_in_prep) {
         if ((rc = launch_prep_operand(c, st, L.m[0].type, h, L.norm_w, M.eps, nt, M.e, w.xn, split_in_prep ? w.x3 : nullptr, w.x3_part, w.op_x)))
             return rc;
@@ -500,7 +500,7 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out, 
     }
     const float* x = L.norm_w ? w.xn : h;
     if ((rc = router_topk_dev(c, st, x, nt, L, w.sels, w.wts, nullptr, split_in_prep))) return rc;
-    if (umma) return experts_dev_umma(c, layer, x, nt, w.sels, w.wts, out, residual, -1, -1, -1, op_in_prep);
+    if (on_tc) return experts_dev_tc(c, layer, x, nt, w.sels, w.wts, out, residual, -1, -1, -1, op_in_prep);
     if (mma) {
         rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, nt >= 16 && tc_type(L, 0, 3) >= 0 ? 2 : 3, residual);
         if (rc != DNB_DECLINED) return rc;
@@ -517,7 +517,7 @@ int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, 
     int rc;
     if ((rc = launch_prep(c, st, x, nullptr, M.eps, rows, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev, L.m[4].dev, L.m[5].dev))) return rc;
     const int sff = L.m[3].n_out, ty = sff == M.ff ? tc_type(L, 3, 6) : -1;
-    if (c->use_umma && w.op_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
+    if (c->use_tc && w.op_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
         if (!op_ready)
             if ((rc = launch_operand_rows(c, st, ty, x, M.e, rows, M.e, w.op_x, "operand_rows_x"))) return rc;
         if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, nullptr, w.act, nullptr, rows, rows))) return rc;
@@ -820,7 +820,7 @@ int dnb_set_tc_min_tokens(dnb_ctx* c, int iq3_xxs_min_tokens) {
     if (!c || iq3_xxs_min_tokens < 1) return DNB_ERR_ARG;
     DNB_CUDA(cudaDeviceSynchronize());
     drop_graphs(c);
-    c->exact_min_nt = iq3_xxs_min_tokens;
+    c->tc_min_iq3 = iq3_xxs_min_tokens;
     return DNB_OK;
 }
 
@@ -845,7 +845,7 @@ int dnb_set_gemv_impl(dnb_ctx* c, int impl) {
     drop_graphs(c);
     c->gemv_impl = impl == 1 ? 1 : 0;
     c->decode_fast = impl != 2;
-    c->use_umma = impl != 2;
+    c->use_tc = impl != 2;
     c->gemv_mma = impl != 3;
     c->decode_fused = impl != 3 && impl != 4;
     c->decode_routed = impl != 5;
@@ -1215,14 +1215,14 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
     // Matrices of the model's own shapes with enough rows per segment go to the tcgen05 grouped GEMM, the others to the mma.sync
     // kernel (four rows per segment: where decoding a weight once per 32 tokens starts to pay for the 128-row tiles).
     const bool in_e = t.n_in == M.e, in_ff = t.n_in == M.ff;
-    bool umma = c->use_umma && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(t.type, t.n_in, t.n_out, false);
-    if (umma) {
+    bool on_tc = c->use_tc && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(t.type, t.n_in, t.n_out, false);
+    if (on_tc) {
         if ((rc = ensure_ws(c, (int)((row + M.k) / (M.k + 1))))) return rc;
-        umma = c->ws.op_ok;
+        on_tc = c->ws.op_ok;
     }
     DNB_CUDA(cudaMemcpyAsync(dx, xs, row * t.n_in * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     DNB_CUDA(cudaMemcpyAsync(dsd, sd.data(), nseg * sizeof(SegDesc), cudaMemcpyHostToDevice, c->stream));
-    if (umma) {
+    if (on_tc) {
         Workspace& w = c->ws;
         DNB_CUDA(cudaMemcpyAsync(dnseg, &nseg, sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
         uint16_t* op = in_e ? w.op_x : w.op_act;
@@ -1458,10 +1458,10 @@ int dnb_expert_rows_dev(dnb_ctx* c, int layer, const float* x_rows_dev, const in
     if (rc) return rc;
     Workspace& w = c->ws;
     const bool tc_routed = !use_shared && tc_type(L, 0, 3) >= 0 && tc_handles(L.m[0].type, M.e, M.ff, true) && tc_handles(L.m[2].type, M.ff, M.e, false);
-    const bool umma = c->use_umma && w.op_ok && rows >= 16;
+    const bool on_tc = c->use_tc && w.op_ok && rows >= 16;
     if (!use_shared) {
         // every row is one (token, slot): a "chunk" of `rows` tokens with one selected expert each and weight 1
-        if (umma && tc_routed) return experts_dev_umma(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, nullptr, 1, M.shard_count, 0);
+        if (on_tc && tc_routed) return experts_dev_tc(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, nullptr, 1, M.shard_count, 0);
         return experts_dev(c, layer, x_rows_dev, rows, local_ids_dev, nullptr, h_rows_dev, nullptr, 1, M.shard_count, 0);
     }
     return shared_rows(c, layer, x_rows_dev, rows, false, h_rows_dev);

@@ -170,8 +170,8 @@ struct dnb_ctx {
     bool gemv_mma = true;               // one-token IQ3_XXS kernels on mma.sync (gemv_mma.cu, decode_fused.cu) where the shape fits
     bool decode_fused = true;           // gate/up + down of a one-token IQ3_XXS block as one kernel (decode_fused.cu)
     bool decode_routed = true;          // ... with the router folded into the same kernel (one launch per block)
-    int exact_min_nt = 48;              // IQ3_XXS layers: tokens from which a batch takes the tcgen05 kernel
-    bool use_umma = true;               // prefill chunks of Q4_K and IQ3_XXS layers take the tcgen05 grouped GEMM
+    int tc_min_iq3 = 48;                // IQ3_XXS layers: tokens from which a batch takes the tcgen05 kernel
+    bool use_tc = true;                 // prefill chunks of Q4_K and IQ3_XXS layers take the tcgen05 grouped GEMM
     void* ep = nullptr;                 // dnb::EpState of the peer-memory expert-parallel path (ep_p2p.cu)
     void* hc = nullptr;                 // dnb::HcState: hyper-connection mix weights and scratch (hc_mix.cu)
     void* epd = nullptr;                // dnb::EpdState of the expert-parallel decode path (ep_decode.cu)
@@ -373,8 +373,6 @@ int router_logits(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const Lay
 // Router logits + softmax / top-k / renorm of a call (w.logits and, on the tensor-core path, w.rpart are its scratch).
 int router_topk_dev(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const Layer& L, int32_t* sels, float* wts,
                     float* rowsum, bool x_is_split = false);
-// One tensor map: [rows][cols] bf16 row-major, box = 64 columns x box_rows rows, 128-byte swizzle.  map: 128 bytes.
-int tc_make_map(void* map, void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 // Grouped dequant matmul for few tokens per expert on mma.sync (grouped_mma.cu): fused = gate/up with silu(g) * u, else one
 // matrix; parts = fp16 numbers per activation (3: all bits of an fp32, 2: 22 bits).  fp32 rows in (row_token names a packed

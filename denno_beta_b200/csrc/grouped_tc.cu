@@ -34,7 +34,6 @@
 // Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, us gate/up + down as bracketed by events: Q4_K 175 + 84 (three
 // bf16 products, a seventh of the accuracy) -> 122 + 83, IQ3_XXS 343 + 180 -> 122 + 73.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
 // commit; without the decoding a copy of the kernel was only 7 % faster.
-#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include "dnb_common.cuh"
@@ -686,43 +685,6 @@ __global__ void __launch_bounds__(256) operand_rows_kernel(const float* __restri
     operand_tail<T>(up, K, pitch, lane, hi);
 }
 }  // namespace tg
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
-    }
-    return fn;
-}
-
-// [rows][cols] 16-bit row-major, box = 64 columns x box_rows rows, 128-byte swizzle.
-int tc_make_map(void* m, void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) {
-        set_error("cuTensorMapEncodeTiled is not available from this driver");
-        return DNB_ERR_CUDA;
-    }
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * 2};
-    const cuuint32_t box[2] = {64, box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(reinterpret_cast<CUtensorMap*>(m), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        set_error("cuTensorMapEncodeTiled failed (%d) for %llu x %llu box %u", (int)r, (unsigned long long)rows,
-                  (unsigned long long)cols, box_rows);
-        return DNB_ERR_CUDA;
-    }
-    return DNB_OK;
-}
 
 size_t tc_row_pitch(int n_in) { return (size_t)tg::row_pitch(n_in); }
 

@@ -211,6 +211,43 @@ static int launch_split3(dnb_ctx* c, cudaStream_t st, const float* x, size_t n, 
     return DNB_OK;
 }
 
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = (EncodeTiledFn)p;
+    }
+    return fn;
+}
+
+// One tensor map: [rows][cols] bf16 row-major, box = 64 columns x box_rows rows, 128-byte swizzle.  m: 128 bytes.
+static int make_map(void* m, void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) {
+        set_error("cuTensorMapEncodeTiled is not available from this driver");
+        return DNB_ERR_CUDA;
+    }
+    const cuuint64_t dims[2] = {cols, rows};
+    const cuuint64_t strides[1] = {cols * 2};
+    const cuuint32_t box[2] = {64, box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(reinterpret_cast<CUtensorMap*>(m), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed (%d) for %llu x %llu box %u", (int)r, (unsigned long long)rows,
+                  (unsigned long long)cols, box_rows);
+        return DNB_ERR_CUDA;
+    }
+    return DNB_OK;
+}
+
 // Once per layer, after the router matrix is resident: its three bf16 parts and their tensor maps.
 int router_tc_prepare(dnb_ctx* c, Layer& L, int ne, int e) {
     L.router_tc = false;
@@ -224,7 +261,7 @@ int router_tc_prepare(dnb_ctx* c, Layer& L, int ne, int e) {
     DNB_CUDA(cudaStreamSynchronize(c->stream));
     CUtensorMap* m = reinterpret_cast<CUtensorMap*>(&L.rmaps);
     for (int p = 0; p < 3; ++p)
-        if (tc_make_map(&m[p], L.router_w3 + p * part, (uint64_t)ne, (uint64_t)e, rt::TM) != DNB_OK) return DNB_OK;
+        if (make_map(&m[p], L.router_w3 + p * part, (uint64_t)ne, (uint64_t)e, rt::TM) != DNB_OK) return DNB_OK;
     L.router_tc = true;
     return DNB_OK;
 }
@@ -240,7 +277,7 @@ int router_tc_workspace(dnb_ctx* c, Workspace& w, int cap, int ne, int e) {
     if (nsplit > 1) DNB_CUDA(cudaMalloc((void**)&w.rpart, (size_t)nsplit * cap * ne * sizeof(float)));
     CUtensorMap* m = reinterpret_cast<CUtensorMap*>(&w.xmaps);
     for (int p = 0; p < 3; ++p)
-        if (tc_make_map(&m[p], w.x3 + p * rows * e, rows, (uint64_t)e, rt::TN) != DNB_OK) return DNB_OK;
+        if (make_map(&m[p], w.x3 + p * rows * e, rows, (uint64_t)e, rt::TN) != DNB_OK) return DNB_OK;
     w.x3_part = rows * e;
     w.router_tc = true;
     return DNB_OK;
