@@ -67,7 +67,7 @@ def test_expert_parallel_equals_single_gpu():
 def test_peer_memory_path_on_one_gpu(ty_name):
     """World of one: the dispatch, the tables, the down epilogue's row destinations and the
     flags all run against the rank's own arena.  The block must equal the ordinary
-    single-GPU block bit for bit (Q4_K: three-product tcgen05 kernel; IQ3_XXS: exact-weight kernel)."""
+    single-GPU block bit for bit: 50 tokens, so that both take the tcgen05 kernel."""
     import numpy as np
 
     import oracle as orc

@@ -42,8 +42,9 @@ def test_block_small(orc, small, layer, nt):
 def test_batch_equals_token_by_token(orc, small):
     """qwen4exp.rs:28259 (batch prefill == sequential).  A token's routing never depends
     on its neighbours; its values agree across chunk sizes and kernel families (one-token
-    decode kernels, tiled fp32 kernels, tcgen05 grouped GEMM) to rounding, and are
-    bit-identical when the same kernels run (fp32 tiled path, any chunk composition)."""
+    decode kernels, mma.sync grouped kernel with three or two parts per activation, tcgen05
+    grouped GEMM) to rounding, and are bit-identical when the same kernels run (any batch
+    composition)."""
     c, layers = small
     nt = 21
     for layer in (0, 1):
@@ -56,46 +57,49 @@ def test_batch_equals_token_by_token(orc, small):
             assert np.array_equal(osel[0], bsel[t]) and np.array_equal(ow[0].view(np.uint32), bw[t].view(np.uint32))
             assert rel_err(one[0], batch[t]) <= 5e-4
     h = orc.synth_normal(SEED, 952, 1.0, nt * layers[0].e).reshape(nt, -1)
-    batch = c.moe_block(0, h[:13])  # IQ3_XXS layer, 13 and 4 tokens: the decode kernels over one-row segments both times
+    batch = c.moe_block(0, h[:13])  # IQ3_XXS layer, 13 and 4 tokens: the mma.sync kernel with three parts both times
     sub = c.moe_block(0, h[[5, 3, 12, 11]])
     assert np.array_equal(sub.view(np.uint32), batch[[5, 3, 12, 11]].view(np.uint32))
-    big = c.moe_block(0, np.concatenate([h, h]))  # 42 and 21 tokens: the tiled fp32 kernels both times
+    big = c.moe_block(0, np.concatenate([h, h]))  # 42 and 21 tokens: the mma.sync kernel with two parts both times
     assert np.array_equal(big[:nt].view(np.uint32), c.moe_block(0, h).view(np.uint32))
+    big = c.moe_block(0, np.concatenate([h] * 6))  # 126 and 63 tokens: the tcgen05 kernel both times
+    assert np.array_equal(big[:3 * nt].view(np.uint32), c.moe_block(0, np.concatenate([h] * 3)).view(np.uint32))
 
 
-@pytest.mark.parametrize("int_weights", [True, False])
-def test_tcgen05_grouped_gemm_matches_fp32_kernels(orc, small, int_weights):
-    """Q4_K prefill chunks on the tensor cores, both kernels: scales folded into bf16 hi / lo weights (three MMAs per
-    product, the default), and integer fp16 weights sc * q with the block scales applied after the sum.
-    The result must stay at fp32-kernel accuracy, far inside the 1e-3 bar, for ragged chunk sizes that
-    exercise every N tile width, one and several token tiles per expert and tiles with one token."""
+def test_tcgen05_grouped_gemm_matches_fp32_kernels(orc, small):
+    """Q4_K prefill chunks on the tensor cores: integer fp16 weights sc * q, the block scales and the mins applied in
+    fp32.  The result must stay at fp32-kernel accuracy, far inside the 1e-3 bar, for ragged chunk sizes from the smallest
+    that takes the kernel, which exercise every N tile width, one and several token tiles per expert and tiles with one
+    token.  set_q4k_int is accepted and changes nothing."""
     c, layers = small
     L = layers[1]
-    c.set_q4k_int(int_weights)
-    try:
-        for nt in (16, 17, 33, 40, 100, 130, 300):
-            h = orc.synth_normal(SEED, 1300 + nt, 1.0, nt * L.e).reshape(nt, L.e)
-            tc, tsel, tw = c.moe_block(1, h, want_routing=True)
-            c.set_gemv_impl(2)
-            try:
-                fp = c.moe_block(1, h)
-            finally:
-                c.set_gemv_impl(0)
-            print("nt=%d tcgen05 (%s) vs fp32 kernels: %.3g" % (nt, "integer" if int_weights else "bf16 x 3", rel_err(tc, fp)))
-            assert rel_err(tc, fp) <= 5e-4, "nt=%d: tcgen05 vs fp32 kernels %.3g" % (nt, rel_err(tc, fp))
-            idx = sorted({0, nt // 3, nt - 1})
-            err, _ = check_block(orc, L, h[idx], tc[idx], tsel[idx], tw[idx])
-            assert err <= 5e-4, "nt=%d: %.3g vs oracle" % (nt, err)
+    for nt in (48, 49, 64, 77, 100, 130, 300):
+        h = orc.synth_normal(SEED, 1300 + nt, 1.0, nt * L.e).reshape(nt, L.e)
+        c.profile(True)
+        tc, tsel, tw = c.moe_block(1, h, want_routing=True)
+        launched = c.profile_read()
+        c.profile(False)
+        assert "tc_gate_up" in launched and "tc_down" in launched, sorted(launched)
+        c.set_gemv_impl(2)
+        try:
+            fp = c.moe_block(1, h)
+        finally:
+            c.set_gemv_impl(0)
+        print("nt=%d tcgen05 vs fp32 kernels: %.3g" % (nt, rel_err(tc, fp)))
+        assert rel_err(tc, fp) <= 5e-4, "nt=%d: tcgen05 vs fp32 kernels %.3g" % (nt, rel_err(tc, fp))
+        idx = sorted({0, nt // 3, nt - 1})
+        err, _ = check_block(orc, L, h[idx], tc[idx], tsel[idx], tw[idx])
+        assert err <= 5e-4, "nt=%d: %.3g vs oracle" % (nt, err)
+        for on in (True, False):
+            c.set_q4k_int(on)
             again = c.moe_block(1, h)
             assert np.array_equal(tc.view(np.uint32), again.view(np.uint32)), "tcgen05 path not bit-identical run to run"
-        assert c.device_status() == 0
-    finally:
-        c.set_q4k_int(False)
+    assert c.device_status() == 0
 
 
 def test_exact_weight_tcgen05_kernel_matches_fp32_kernels(orc, small):
-    """IQ3_XXS chunks and decode batches from the threshold up (lowered to 2 here): exact bf16 weights on the tensor cores, sub-block scales
-    applied by the epilogue.  Ragged sizes cover one and several 32-token tiles per expert and tiles with one token;
+    """IQ3_XXS chunks and decode batches from the threshold up (lowered to 2 here): exact integer fp16 weights on the tensor cores, block
+    scales applied by the epilogue.  Ragged sizes cover one and several 32-token tiles per expert and tiles with one token;
     a batch's rows do not depend on their companions."""
     c, layers = small
     L = layers[0]
@@ -120,9 +124,9 @@ def test_exact_weight_tcgen05_kernel_matches_fp32_kernels(orc, small):
                 part = c.moe_block(0, h[nt // 2:])
                 assert np.array_equal(part.view(np.uint32), tc[nt // 2:].view(np.uint32)), "a row depends on its companions"
     finally:
-        c.set_tc_min_tokens(16)
-    # the default threshold: 15 tokens stay on the one-token kernels, 16 take the tensor cores; both within the bar
-    for nt in (15, 16):
+        c.set_tc_min_tokens(48)
+    # the default threshold: 47 tokens stay on the mma.sync kernel, 48 take the tcgen05 kernel; both within the bar
+    for nt in (47, 48):
         h = orc.synth_normal(SEED, 1450 + nt, 1.0, nt * L.e).reshape(nt, L.e)
         tc, tsel, tw = c.moe_block(0, h, want_routing=True)
         err, _ = check_block(orc, L, h[:4], tc[:4], tsel[:4], tw[:4])

@@ -1,11 +1,14 @@
 """The arithmetic identities the tensor-core kernels rest on, checked on the CPU against the oracle's block decode
 (no GPU, no product code): what must hold for the kernels' operand formats to be EXACT.
 
-* Q4_K with integer weights (csrc/grouped_q4k_int.cu): w = d * sc * q - dmin * m (kquant.rs:505-526), so
+* Q4_K with integer weights (csrc/grouped_tc.cu, csrc/grouped_mma.cu): w = d * sc * q - dmin * m (kquant.rs:505-526), so
   W . x = sum_blocks d * [sum (sc * q) * x] - sum_subblocks (dmin * m) * X with X the sub-block sums of x;
-  sc * q <= 945 is exact in fp16 and one fp16 fma (1024 + q) * sc - 1024 * sc produces it; -(dmin * m) is exact as
-  fp16 hi + lo.
-* IQ3_XXS with exact weights (csrc/grouped_exact.cu): w = db * (grid magnitude) * sign, magnitudes exact in bf16.
+  sc * q <= 945 is exact in fp16 and one fp16 fma (1024 + q) * sc - 1024 * sc produces it; -(dmin * m) times a power of
+  two of the row is exact as fp16 hi + lo.
+* IQ3_XXS with exact weights: w = d / 4 * (grid magnitude) * sign * (2 s + 1), the product of the last three an integer exact
+  in fp16 (csrc/grouped_tc.cu); the magnitude alone exact in fp16 (csrc/grouped_mma.cu) and in bf16 (csrc/iq3_mma.cuh).
+* Activations of those kernels: a row times a power of two as two or three fp16 numbers (csrc/operand_rows.cuh,
+  csrc/grouped_mma.cu).
 * Router operands (csrc/router_tc.cu): an fp32 value is the exact sum of three bf16 numbers (round, round, round).
 """
 import numpy as np
@@ -106,38 +109,46 @@ def test_q4k_integer_weight_decomposition(orc):
     assert np.max(np.abs(got - want)) <= 2e-6 * rms   # the oracle's own fp32 rounding
 
 
-def test_activation_rows_as_scaled_fp16_pairs(orc):
-    """Rows scaled by a power of two so that the largest element is in [256, 512): hi + lo fp16 carry 22 bits of every
-    element that matters and the sub-block sums (<= 32 * 512) stay inside fp16's range."""
+def test_activation_rows_as_scaled_fp16_parts(orc):
+    """Rows scaled by a power of two so that the largest element is in [512, 1024): two fp16 parts carry 22 bits, three all bits of
+    the elements above 1/1024 of the largest and 2^-34 of the largest below; the sub-block sums stay inside fp16's range."""
     x = orc.synth_normal(SEED, 903, 37.5, 4096).astype(np.float32)
     x[7] = 3.1e4      # an outlier, as SwiGLU outputs have
     x[11] = 1e-7
-    mx = float(np.max(np.abs(x)))
-    e = int(np.frexp(mx)[1])
-    up = np.float32(2.0 ** (9 - e))
-    xs = x * up
-    assert 256 <= np.max(np.abs(xs)) < 512
-    hi = xs.astype(np.float16)
-    lo = (xs - hi.astype(np.float32)).astype(np.float16)
-    err = np.abs(hi.astype(np.float64) + lo.astype(np.float64) - xs.astype(np.float64))
-    assert np.max(err) <= 2.0 ** -13 * 2.0 ** -11 * 512 + 2.0 ** -25   # 2^-22 of the row's scale (+ the subnormal floor)
-    sums = xs.reshape(-1, 32).astype(np.float64).sum(axis=1)
-    assert np.max(np.abs(sums)) < 65504
+    for row in (x, x[1024:2048]):  # with the outlier, and without
+        mx = np.max(np.abs(row))
+        up = np.uint32((127 + 9 - (int(mx.view(np.uint32) >> 23) - 127)) << 23).view(np.float32)
+        xs = row * up
+        assert 512 <= np.max(np.abs(xs)) < 1024
+        rest, parts = xs.copy(), []
+        for _ in range(3):
+            parts.append(rest.astype(np.float16))
+            rest = rest - parts[-1].astype(np.float32)  # exact
+        xs64 = xs.astype(np.float64)
+        two = parts[0].astype(np.float64) + parts[1].astype(np.float64)
+        assert np.max(np.abs(two - xs64)) <= 2.0 ** -22 * 1024 + 2.0 ** -25
+        three = two + parts[2].astype(np.float64)
+        large = np.abs(xs64) >= 1.0
+        assert large.any() and np.array_equal(three[large], xs64[large])
+        assert np.max(np.abs(three - xs64)) <= 2.0 ** -25  # 2^-34 of 512
+        assert np.max(np.abs(xs64.reshape(-1, 32).sum(axis=1))) < 65504
 
 
-def test_iq3xxs_magnitudes_are_exact_in_bf16(orc):
+def test_iq3xxs_integers_are_exact(orc):
     k = 512
     w = orc.synth_blocks(orc.IQ3_XXS, SEED, 904, k // 256)
     row = orc.dequant_row(orc.IQ3_XXS, w, k).astype(np.float64)
     b = np.frombuffer(w, np.uint8).reshape(-1, 98)
     d = b[:, 0:2].copy().view(np.float16).astype(np.float64).reshape(-1)
-    aux = b[:, 66:98].copy().view(np.uint32).reshape(-1, 8)          # one 32-bit word per 32-element sub-block
-    db = d[:, None] * (0.5 + (aux >> 28)) * 0.5
-    mag = row.reshape(-1, 8, 32) / db[:, :, None]                     # grid magnitude x sign
+    s = (b[:, 66:98].copy().view(np.uint32).reshape(-1, 8) >> 28).astype(np.int64)  # of the word of each 32-element sub-block
+    mag = row.reshape(-1, 8, 32) / (d[:, None] * (0.5 + s) * 0.5)[:, :, None]         # grid magnitude x sign
     assert np.allclose(mag, np.round(mag), atol=1e-3)
-    mag = np.round(mag).astype(np.float32)
+    mag = np.round(mag)
     assert np.max(np.abs(mag)) <= 62
-    assert np.array_equal(_bf16_rn(mag), mag)
+    assert np.array_equal(_bf16_rn(mag), mag) and np.array_equal(mag.astype(np.float16).astype(np.float64), mag)
+    iw = mag * (2 * s + 1)[:, :, None]
+    assert np.max(np.abs(iw)) <= 62 * 31 and np.array_equal(iw.astype(np.float16).astype(np.float64), iw)
+    assert np.allclose((d / 4)[:, None, None] * iw, row.reshape(-1, 8, 32), rtol=1e-6, atol=0)
 
 
 def test_three_bf16_parts_carry_an_fp32_exactly(orc):
