@@ -430,10 +430,10 @@ static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const 
     const int nseg_max = (nt * k < ne ? nt * k : ne) + (shared ? 1 : 0);
     // experts that nt tokens reach when each picks k of ne at random
     const int est = std::min(nseg_max, (int)(ne * (1.0 - pow(1.0 - (double)k / ne, nt)) + 1.5));
-    if ((rc = launch_mm(c, st, L.m[0].type, true, parts, w.seg_gu, w.nseg, nseg_max, est, rows, M.e, M.ff, x, M.e, w.row_token, w.act, nullptr,
+    if ((rc = launch_mm(c, st, L.m[0].type, true, parts, nt < kTcMin, w.seg_gu, w.nseg, nseg_max, est, rows, M.e, M.ff, x, M.e, w.row_token, w.act, nullptr,
                         "mm_gate_up")))
         return rc;
-    if ((rc = launch_mm(c, st, L.m[2].type, false, parts, w.seg_dn, w.nseg, nseg_max, est, rows, M.ff, M.e, w.act, M.ff, nullptr, w.hrow, nullptr,
+    if ((rc = launch_mm(c, st, L.m[2].type, false, parts, nt < kTcMin, w.seg_dn, w.nseg, nseg_max, est, rows, M.ff, M.e, w.act, M.ff, nullptr, w.hrow, nullptr,
                         "mm_down")))
         return rc;
     if (shared && L.shared_gate_row)
@@ -863,7 +863,7 @@ static int gemv_dev(dnb_ctx* c, int type, const uint8_t* w, int k, int n, const 
     const SegDesc sd{w, nullptr, (uint32_t)nvec, 0u};
     if (c->decode_fast) {
         int rc = launch_gemv_mma(c, c->stream, type, w, k, n, x, out, nvec);
-        if (rc == DNB_DECLINED) rc = launch_mm(c, c->stream, type, false, 3, nullptr, nullptr, 1, 1, nvec, k, n, x, k, nullptr, out, &sd, "mm_vectors");
+        if (rc == DNB_DECLINED) rc = launch_mm(c, c->stream, type, false, 3, false, nullptr, nullptr, 1, 1, nvec, k, n, x, k, nullptr, out, &sd, "mm_vectors");
         if (rc != DNB_DECLINED) return rc;
     }
     if (nvec == 1 && c->decode_fast && (((uintptr_t)w) & 15) == 0) {
@@ -1230,7 +1230,7 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
             rc = launch_grouped_tc(c, c->stream, t.type, false, dsd, dnseg, nseg, t.n_in, t.n_out, op, nullptr,
                                    dout);
     } else {
-        rc = c->decode_fast ? launch_mm(c, c->stream, t.type, false, tc_type_ok(t.type) && row >= 64 ? 2 : 3, dsd, nullptr, nseg, nseg, (int)row,
+        rc = c->decode_fast ? launch_mm(c, c->stream, t.type, false, tc_type_ok(t.type) && row >= 64 ? 2 : 3, false, dsd, nullptr, nseg, nseg, (int)row,
                                         t.n_in, t.n_out, dx, t.n_in, nullptr, dout, nullptr, "mm_grouped")
                             : DNB_DECLINED;
         if (rc == DNB_DECLINED)

@@ -357,8 +357,10 @@ int launch_decode_block(dnb_ctx* c, cudaStream_t st, const Model& M, const Layer
 
 // Router logits of chunks of kRouterTcMin tokens or more on tcgen05 (router_tc.cu)
 constexpr int kRouterSplitMax = 8;  // K splits of the tensor-core router at most (the top-k kernel adds that many partial sums)
-constexpr int kRouterTcMin = 16;   // the token count from which the tensor-core expert kernels take a call, too: a token's bits then do not
-                                  // depend on the size of its chunk or on how an expert-parallel group split it
+// Calls below take the fp32 kernel in the one-token router's order of adds, and three parts per activation; a token's bits do not
+// depend on its batch within 2 to 15 tokens, within 16 to 47 (mma.sync, three and two parts) and from 48 on (tcgen05; a layer of mixed
+// formats stays on mma.sync, whose sums are then split by the call's size).
+constexpr int kRouterTcMin = 16;
 int router_tc_prepare(dnb_ctx* c, Layer& L, int ne, int e);
 int router_tc_workspace(dnb_ctx* c, Workspace& w, int cap, int ne, int e);
 bool router_tc_eligible(const dnb_ctx* c, const Layer& L, int nt);
@@ -375,11 +377,12 @@ int router_topk_dev(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const L
                     float* rowsum, bool x_is_split = false);
 
 // Grouped dequant matmul for few tokens per expert on mma.sync (grouped_mma.cu): fused = gate/up with silu(g) * u, else one
-// matrix; parts = fp16 numbers per activation (3: all bits of an fp32, 2: 22 bits).  fp32 rows in (row_token names a packed
+// matrix; parts = fp16 numbers per activation (3: an fp32 to 2^-34 of its row's largest, 2: 22 bits); batch = sums in an order
+// that does not depend on the launch's size.  fp32 rows in (row_token names a packed
 // row's input row, null: itself), fp32 packed rows out.  rows, nseg_est: token rows and active segments (an estimate where the
 // device counts them; it only steers the split of the work).  DNB_DECLINED = type or shape not covered, nothing launched.
 bool mm_handles(int type, int n_in);
-int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
+int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name);
 

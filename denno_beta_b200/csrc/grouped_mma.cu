@@ -12,7 +12,7 @@
 //     Q8_0: q; IQ3_XXS: the codebook magnitude <= 62 with its sign), so no weight is rounded;
 //   * the scales multiply the fp32 sums of a 256-element block (Q4_K, Q5_K: d; their mins are one more K step of
 //     m against the sub-block sums of the activations), of a 32-element block (Q8_0, IQ3_XXS) or of 16 elements (Q6_K);
-//   * an activation is P fp16 numbers in P columns of B (P = 3 carries the 24 bits of an fp32; P = 2 carries 22 and is
+//   * an activation is P fp16 numbers in P columns of B (P = 3 carries an fp32 to 2^-34 of the row's largest; P = 2 carries 22 bits and is
 //     used where a call of this size had 16 before), of the row times a power of two that puts its largest element into
 //     [512, 1024), so that nothing overflows and sub-block sums fit, too;
 //   * K is walked in the order in which the packed bytes yield elements; the activations are staged in that order.
@@ -21,9 +21,9 @@
 // Work: an item is (segment, token tile, block of row groups); a row group is 16 A rows: 16 rows of one matrix, or 8 gate
 // and 8 up rows of the same indices, whose results meet in one lane for silu(g) * u.  A persistent CTA of 16 warps stages
 // an item's activations once; a warp then streams its row groups through a private ring of cp.async stages (one
-// 256-element block of the 16 rows each) without any CTA-wide barrier.  Few row groups for the chip (small models, single
-// matrices): KS warps share a row group, each takes a part of K, and their sums are added in a fixed order.
-// A row's result depends on nothing but the row: not on the tile, the column or the split of the launch.
+// 256-element block of the 16 rows each) without any CTA-wide barrier.  Few row groups for the chip: KS warps share a row
+// group, each takes a part of K, and their sums are added in a fixed order.  A row's result depends on the row, on P and on KS, not on
+// the tile, the column or the CTA; for decode batches KS is a constant of the shape, so that a token's bits do not depend on its batch.
 //
 // Measured, us per layer of 2048 x 512, top 10 of 512, against one-row GEMVs (to 15 tokens) and tiled fp32 or bf16 tensor-core kernels:
 // 8 tokens, IQ3_XXS 140 -> 95; 32 tokens 502 -> 204; 77 tokens under a skewed router, Q4_K with Q6_K down 895 -> 255.  Issue slots are
@@ -260,7 +260,8 @@ __device__ __forceinline__ float mm_row_scale(uint32_t amax_bits) {
     const int s = ex == 0 ? 0 : max(-126, min(126, 9 - (ex - 127)));
     return __uint_as_float((uint32_t)(s + 127) << 23);
 }
-// Two values as P fp16 pairs whose sums are the values (P = 3: every bit of an fp32; P = 2: 22 bits).
+// Two values as P fp16 pairs whose sums are the values.  P = 2: 22 bits of the row's (one matrix: the block's) largest element; P = 3: every
+// bit of the elements above 1/1024 of the largest, and 2^-34 of the largest below, where the third part meets fp16's smallest number.
 template <int P>
 __device__ __forceinline__ void mm_split(float a, float b, uint32_t (&h)[P]) {
 #pragma unroll
@@ -630,8 +631,8 @@ static int mm_launch_type(dnb_ctx* c, cudaStream_t st, bool fused, int parts, in
 #undef DNB_MM
 }
 
-// rows: token rows of the launch in total; nseg_est: segments that will have rows (an estimate when the device counts them).
-int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
+// batch: K is split as a constant of the shape.  rows: token rows of the launch in total; nseg_est: segments that will have rows (an estimate when the device counts them).
+int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name) {
     if (!mm_handles(type, n_in) || n_out < 1 || (fused && n_out % 8) || nseg_max < 1 || nseg_max > kMmSegMax || rows < 1) return DNB_DECLINED;
@@ -661,10 +662,15 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, cons
     for (;; nt /= 2) {
         const long tiles = std::max(nseg_est, (rows + nt * tpt - 1) / (nt * tpt));
         // A CTA's row groups go round its slots of `ks` warps; the last round is partly empty, so K is split until there are
-        // about six rounds (at most eight ways: each split costs an exchange of the sums).
+        // about six rounds (at most eight ways: each split costs an exchange of the sums).  A decode batch: two ways from four blocks on,
+        // else not at all.  us a layer, gate/up of 2048 x 512, top 10 of 512, IQ3_XXS, 1 / 2 / 4 / 8 ways: 2 tokens 48.8 / 45.2 / 45.1 / 45.2,
+        // 8 tokens 94.3 / 92.8 / 93.9 / 96.0, 32 tokens 206.8 / 204.1 / 213.1 / 222.7; down (two blocks) 1 / 2 ways: 8 tokens 93.1 / 93.8, 32 tokens
+        // 206.6 / 209.8.  (Two sums in one warp, added like two warps' sums, would let K go unsplit with the same bits from 48 tokens on: 16 more
+        // registers or as much shared memory, 10 to 20 % of a prompt's time.)
         const long per_cta = tiles * n_rg / c->sm_count;
-        int ks = 1;
-        while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
+        int ks = batch && nb >= 4 ? 2 : 1;
+        if (!batch)
+            while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
         A.ks = ks;
         size_t base = fixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 4 * 32 * 4 : 0) + (size_t)nt * tpt * parts * A.col_stride;
         if (type == T_IQ3_XXS)  // the tables behind the activations, on their boundary (dynamic shared memory starts at kMmSmemBase)

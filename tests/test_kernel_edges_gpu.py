@@ -62,6 +62,30 @@ def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
             assert np.array_equal(part.view(np.uint32), out[5:53].view(np.uint32)), "nt %d: bits of a chunk of 48" % nt
 
 
+@pytest.mark.parametrize("up,down", [("IQ3_XXS", "IQ3_XXS"), ("Q4_K", "Q4_K"), ("Q4_K", "Q6_K")])
+def test_bits_do_not_depend_on_the_batch(orc, ctx, up, down):
+    """Wide enough that a split of K pays for few tokens and not for many: a token has the same bits in every batch of 2 to 15, of
+    16 to 47 and, unless formats are mixed, from 48 on, routed by the layer or by the caller."""
+    from denno_beta_b200 import cuda as cu
+
+    e, ff, ne, k = 2048, 1024, 64, 8
+    up, down = orc.TYPE_BY_NAME[up], orc.TYPE_BY_NAME[down]
+    assert ctx.moe_config(1, e, ff, ne, k)
+    for m, ty, ni, no, n in ((cu.GATE, up, e, ff, ne), (cu.UP, up, e, ff, ne), (cu.DOWN, down, ff, e, ne), (cu.SHARED_GATE, up, e, ff, 1),
+                             (cu.SHARED_UP, up, e, ff, 1), (cu.SHARED_DOWN, down, ff, e, 1)):
+        assert ctx.synth_experts(0, m, ty, ni, no, n, SEED)
+    ctx.register_router(0, orc.synth_normal(SEED, 6, 0.02, ne * e).reshape(ne, e), None, np.ones(e, np.float32), None)
+    h = orc.synth_normal(SEED, 95, 1.0, 96 * e).reshape(96, e)
+    for large, small in ((15, 2), (9, 4), (47, 16)) + (((96, 48),) if up == down else ()):
+        out, part = ctx.moe_block(0, h[:large]), ctx.moe_block(0, h[large - small:large])
+        assert np.array_equal(out[large - small:].view(np.uint32), part.view(np.uint32)), (large, small)
+    rng = np.random.RandomState(5)
+    sels = np.sort(np.argsort(rng.rand(40, ne), axis=1)[:, :k], axis=1).astype(np.int32)
+    wts = rng.rand(40, k).astype(np.float32)
+    out, part = ctx.moe_experts(0, h[:40], sels, wts), ctx.moe_experts(0, h[7:8], sels[7:8], wts[7:8])
+    assert np.array_equal(out[7:8].view(np.uint32), part.view(np.uint32))
+
+
 @pytest.mark.parametrize("up,down,e,ff", [("Q5_K", "Q8_0", 768, 288), ("Q4_K", "Q6_K", 512, 768), ("IQ3_XXS", "Q4_K", 512, 256)])
 def test_experts_given_mixed(orc, ctx, up, down, e, ff):
     """A selection of the caller's own and two formats in a layer, one with an expert width (288) that the mma kernel leaves alone."""
