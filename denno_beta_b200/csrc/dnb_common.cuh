@@ -358,8 +358,8 @@ int launch_decode_block(dnb_ctx* c, cudaStream_t st, const Model& M, const Layer
 // Router logits of chunks of kRouterTcMin tokens or more on tcgen05 (router_tc.cu)
 constexpr int kRouterSplitMax = 8;  // K splits of the tensor-core router at most (the top-k kernel adds that many partial sums)
 // Calls below take the fp32 kernel in the one-token router's order of adds, and three parts per activation; a token's bits do not
-// depend on its batch within 2 to 15 tokens, within 16 to 47 (mma.sync, three and two parts) and from 48 on (tcgen05; a layer of mixed
-// formats stays on mma.sync, whose sums are then split by the call's size).
+// depend on its batch within 2 to 15 tokens, within 16 to 47 (mma.sync, three and two parts) and from 48 on (tcgen05; layers that it
+// does not take stay on mma.sync, whose sums are then split by the call's size).
 constexpr int kRouterTcMin = 16;
 int router_tc_prepare(dnb_ctx* c, Layer& L, int ne, int e);
 int router_tc_workspace(dnb_ctx* c, Workspace& w, int cap, int ne, int e);

@@ -705,7 +705,7 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
 // it, whose output the vector may be; it converts its own blocks of the vector, each with a power of two of its own, so that no
 // CTA-wide step stands between vector and math; the warps' partial sums meet once per 16 rows, in a fixed order.
 // Measured back to back, us, register-decode GEMV before: 4096 x 4096 Q4_K 8.4 -> 5.7, IQ3_XXS 10.3 -> 6.4, Q8_0 8.9 -> 6.5; 65536 x
-// 4096 Q8_0 103 -> 69 (4.1 TB/s), Q4_K 84 -> 47, IQ3_XXS 99 -> 56; two vectors of IQ3_XXS 62034 x 5632 466 -> 94.
+// 4096 Q8_0 103 -> 71 (4.0 TB/s), Q4_K 84 -> 47, IQ3_XXS 99 -> 56; two vectors of IQ3_XXS 62034 x 5632 466 -> 94.
 constexpr int kGvWarps = 8;
 constexpr int kGvPart = 576;  // bytes of a part of a block: 512, its sub-block sums (16), and padding that spreads neighbouring parts over the banks
 

@@ -87,7 +87,7 @@ uint64_t dnb_launch_count(dnb_ctx* ctx);
  *   24       expert-parallel decode: a peer's result rows did not arrive
  *   23       grid barrier of the fused one-token kernel
  *   25       the tensor-core router GEMM of a prefill chunk (stage or accumulator barrier)
- *   26       no wait: the mma.sync grouped kernel found its shared memory laid out otherwise than it asked for
+ *   26       no wait: a grouped kernel (mma.sync or tcgen05) found its shared memory laid out otherwise than it asked for
  * What the reference promises for a GPU call that did not complete -- "false: out
  * untouched, the caller recomputes" (cuda.rs:21024-21027, 8785-8788) -- holds here too:
  * every host-buffer entry point reads the word after its stream synchronisation and, when
@@ -231,6 +231,9 @@ int dnb_load_gguf_layer(dnb_ctx* ctx, const dnb_gguf* g, int layer, int gguf_lay
  *   prefill: qwen4exp.rs:17921 moe_ffn_quant_batch_full -> cuda.rs:48695
  *            pf_router_dev_topk + cuda.rs:10919 moe_experts_iq_pf_layer /
  *            cuda.rs:7065 moe_grouped_gemm_layer + moe_grouped_gpu.rs:540 scatter
+ * A token's bits do not depend on the other tokens of the call, nor on their number within 2 to 15 tokens, within
+ * 16 to 47 and from 48 on; across those lines other kernels run and a token agrees to rounding.  (Layers
+ * other than Q4_K or IQ3_XXS throughout: from 48 tokens on to rounding only.)
  * h, out: host [nt][n_embd].  sels_out [nt][k] / wts_out [nt][k] may be NULL. */
 int dnb_moe_block(dnb_ctx* ctx, int layer, const float* h, int nt, float* out, int32_t* sels_out, float* wts_out);
 /* Same with device pointers; nothing is copied and the call does not synchronise. */

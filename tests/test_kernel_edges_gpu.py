@@ -65,7 +65,7 @@ def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
 @pytest.mark.parametrize("up,down", [("IQ3_XXS", "IQ3_XXS"), ("Q4_K", "Q4_K"), ("Q4_K", "Q6_K")])
 def test_bits_do_not_depend_on_the_batch(orc, ctx, up, down):
     """Wide enough that a split of K pays for few tokens and not for many: a token has the same bits in every batch of 2 to 15, of
-    16 to 47 and, unless formats are mixed, from 48 on, routed by the layer or by the caller."""
+    16 to 47 and, in a layer of one format, from 48 on, routed by the layer or by the caller."""
     from denno_beta_b200 import cuda as cu
 
     e, ff, ne, k = 2048, 1024, 64, 8
