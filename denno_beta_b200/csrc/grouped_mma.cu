@@ -659,6 +659,7 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
     while (nt < max_nt && avg > 0.75f * nt * tpt) nt *= 2;
     const int n_rg = fused ? n_out / 8 : (n_out + 15) / 16, nb = n_in / 256;
     const size_t fixed = ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
+    int split = batch && nb >= 4 ? 2 : 1;  // of a batch
     for (;; nt /= 2) {
         const long tiles = std::max(nseg_est, (rows + nt * tpt - 1) / (nt * tpt));
         // A CTA's row groups go round its slots of `ks` warps; the last round is partly empty, so K is split until there are
@@ -668,7 +669,7 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
         // 206.6 / 209.8.  (Two sums in one warp, added like two warps' sums, would let K go unsplit with the same bits from 48 tokens on: 16 more
         // registers or as much shared memory, 10 to 20 % of a prompt's time.)
         const long per_cta = tiles * n_rg / c->sm_count;
-        int ks = batch && nb >= 4 ? 2 : 1;
+        int ks = split;
         if (!batch)
             while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
         A.ks = ks;
@@ -693,7 +694,10 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
                 default: return mm_launch_type<T_IQ3_XXS>(c, st, fused, parts, nt, A, smem, grid, name);
             }
         }
-        if (nt == 1) return DNB_DECLINED;
+        if (nt > 1) continue;
+        if (split == 1) return DNB_DECLINED;
+        split = 1;  // K so long that the exchange has no room beside it
+        nt = 2;
     }
 }
 

@@ -86,6 +86,21 @@ def test_bits_do_not_depend_on_the_batch(orc, ctx, up, down):
     assert np.array_equal(out[7:8].view(np.uint32), part.view(np.uint32))
 
 
+def test_batch_with_a_long_k(orc, ctx):
+    """Q8_0 rows of 6144: two warps' sums have no room beside the activations, so one warp takes all of K."""
+    e, ff, ne, k, nt = 6144, 256, 4, 2, 9
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.Q8_0, e, ff, ne, k)
+    h = orc.synth_normal(SEED, 97, 1.0, nt * e).reshape(nt, e)
+    ctx.profile(True)
+    out, sels, wts = ctx.moe_block(0, h, want_routing=True)
+    launched = ctx.profile_read()
+    ctx.profile(False)
+    assert launched["mm_gate_up"]["launches"] == 1 and "combine" in launched
+    assert check_block(orc, L, h, out, sels, wts)[0] <= 5e-5
+    assert np.array_equal(ctx.moe_block(0, h[3:5]).view(np.uint32), out[3:5].view(np.uint32))
+
+
 @pytest.mark.parametrize("up,down,e,ff", [("Q5_K", "Q8_0", 768, 288), ("Q4_K", "Q6_K", 512, 768), ("IQ3_XXS", "Q4_K", 512, 256)])
 def test_experts_given_mixed(orc, ctx, up, down, e, ff):
     """A selection of the caller's own and two formats in a layer, one with an expert width (288) that the mma kernel leaves alone."""
