@@ -411,7 +411,7 @@ static bool mm_eligible(const dnb_ctx* c, const Layer& L) {
 }
 
 // The experts on the mma.sync grouped kernel: tables, gate/up, down, combine.  The shared expert is one more segment.
-static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts, float* out, int parts,
+static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const int32_t* sels, const float* wts, float* out,
                            const float* residual = nullptr, int k = -1, int ne = -1, int with_shared = -1, bool tables_ready = false) {
     const Model& M = c->model;
     const Layer& L = M.layers[layer];
@@ -430,10 +430,10 @@ static int experts_dev_mma(dnb_ctx* c, int layer, const float* x, int nt, const 
     const int nseg_max = (nt * k < ne ? nt * k : ne) + (shared ? 1 : 0);
     // experts that nt tokens reach when each picks k of ne at random
     const int est = std::min(nseg_max, (int)(ne * (1.0 - pow(1.0 - (double)k / ne, nt)) + 1.5));
-    if ((rc = launch_mm(c, st, L.m[0].type, true, parts, nt < kTcMin, w.seg_gu, w.nseg, nseg_max, est, rows, M.e, M.ff, x, M.e, w.row_token, w.act, nullptr,
+    if ((rc = launch_mm(c, st, L.m[0].type, true, nt < kTcMin, w.seg_gu, w.nseg, nseg_max, est, rows, M.e, M.ff, x, M.e, w.row_token, w.act, nullptr,
                         "mm_gate_up")))
         return rc;
-    if ((rc = launch_mm(c, st, L.m[2].type, false, parts, nt < kTcMin, w.seg_dn, w.nseg, nseg_max, est, rows, M.ff, M.e, w.act, M.ff, nullptr, w.hrow, nullptr,
+    if ((rc = launch_mm(c, st, L.m[2].type, false, nt < kTcMin, w.seg_dn, w.nseg, nseg_max, est, rows, M.ff, M.e, w.act, M.ff, nullptr, w.hrow, nullptr,
                         "mm_down")))
         return rc;
     if (shared && L.shared_gate_row)
@@ -484,7 +484,7 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out, 
         // a decode batch: routing in two launches (route_small.cu), the block in five
         rc = launch_router_batch(c, st, h, nt, M, L, w);
         if (rc == DNB_OK) rc = launch_topk_tables(c, st, true, nt, M.k, M.ne, M.norm_topk, w.sels, w.wts, L, w, shared);
-        if (rc == DNB_OK) rc = experts_dev_mma(c, layer, L.norm_w ? w.xn : h, nt, w.sels, w.wts, out, 3, residual, -1, -1, -1, true);
+        if (rc == DNB_OK) rc = experts_dev_mma(c, layer, L.norm_w ? w.xn : h, nt, w.sels, w.wts, out, residual, -1, -1, -1, true);
         if (rc != DNB_DECLINED) return rc;
     }
     // the RMSNorm kernel writes the router's operand (three bf16 parts of the normalised rows) and the experts' in the same pass
@@ -502,7 +502,7 @@ static int block_dev(dnb_ctx* c, int layer, const float* h, int nt, float* out, 
     if ((rc = router_topk_dev(c, st, x, nt, L, w.sels, w.wts, nullptr, split_in_prep))) return rc;
     if (on_tc) return experts_dev_tc(c, layer, x, nt, w.sels, w.wts, out, residual, -1, -1, -1, op_in_prep);
     if (mma) {
-        rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, nt >= 16 && tc_type(L, 0, 3) >= 0 ? 2 : 3, residual);
+        rc = experts_dev_mma(c, layer, x, nt, w.sels, w.wts, out, residual);
         if (rc != DNB_DECLINED) return rc;
     }
     return experts_dev(c, layer, x, nt, w.sels, w.wts, out, residual);
@@ -863,7 +863,7 @@ static int gemv_dev(dnb_ctx* c, int type, const uint8_t* w, int k, int n, const 
     const SegDesc sd{w, nullptr, (uint32_t)nvec, 0u};
     if (c->decode_fast) {
         int rc = launch_gemv_mma(c, c->stream, type, w, k, n, x, out, nvec);
-        if (rc == DNB_DECLINED) rc = launch_mm(c, c->stream, type, false, 3, false, nullptr, nullptr, 1, 1, nvec, k, n, x, k, nullptr, out, &sd, "mm_vectors");
+        if (rc == DNB_DECLINED) rc = launch_mm(c, c->stream, type, false, false, nullptr, nullptr, 1, 1, nvec, k, n, x, k, nullptr, out, &sd, "mm_vectors");
         if (rc != DNB_DECLINED) return rc;
     }
     if (nvec == 1 && c->decode_fast && (((uintptr_t)w) & 15) == 0) {
@@ -1132,7 +1132,7 @@ int dnb_moe_experts(dnb_ctx* c, int layer, const float* x, int nt, const int32_t
             DNB_CUDA(cudaMemcpyAsync(w.wts, w.pinned_wts, rows * 4, cudaMemcpyHostToDevice, c->stream));
         }
         float* o = direct ? w.pinned_out : w.out;
-        r = mm_eligible(c, L) ? experts_dev_mma(c, layer, w.hin, nt, w.sels, w.wts, o, 3) : DNB_DECLINED;
+        r = mm_eligible(c, L) ? experts_dev_mma(c, layer, w.hin, nt, w.sels, w.wts, o) : DNB_DECLINED;
         if (r == DNB_DECLINED) {
             if (L.has_shared())
                 if ((r = launch_prep(c, c->stream, w.hin, nullptr, M.eps, nt, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev, L.m[4].dev, L.m[5].dev)))
@@ -1230,7 +1230,7 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
             rc = launch_grouped_tc(c, c->stream, t.type, false, dsd, dnseg, nseg, t.n_in, t.n_out, op, nullptr,
                                    dout);
     } else {
-        rc = c->decode_fast ? launch_mm(c, c->stream, t.type, false, tc_type_ok(t.type) && row >= 64 ? 2 : 3, false, dsd, nullptr, nseg, nseg, (int)row,
+        rc = c->decode_fast ? launch_mm(c, c->stream, t.type, false, false, dsd, nullptr, nseg, nseg, (int)row,
                                         t.n_in, t.n_out, dx, t.n_in, nullptr, dout, nullptr, "mm_grouped")
                             : DNB_DECLINED;
         if (rc == DNB_DECLINED)

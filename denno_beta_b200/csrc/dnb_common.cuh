@@ -377,12 +377,11 @@ int router_topk_dev(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const L
                     float* rowsum, bool x_is_split = false);
 
 // Grouped dequant matmul for few tokens per expert on mma.sync (grouped_mma.cu): fused = gate/up with silu(g) * u, else one
-// matrix; parts = fp16 numbers per activation (3: an fp32 to 2^-34 of its row's largest, 2: 22 bits); batch = sums in an order
-// that does not depend on the launch's size.  fp32 rows in (row_token names a packed
+// matrix; batch = sums in an order that does not depend on the launch's size.  fp32 rows in (row_token names a packed
 // row's input row, null: itself), fp32 packed rows out.  rows, nseg_est: token rows and active segments (an estimate where the
 // device counts them; it only steers the split of the work).  DNB_DECLINED = type or shape not covered, nothing launched.
 bool mm_handles(int type, int n_in);
-int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
+int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name);
 

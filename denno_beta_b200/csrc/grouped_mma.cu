@@ -1,50 +1,54 @@
 // Grouped dequant matmul for few tokens per expert: decode batches, short prompts, caller-given selections, single
-// matrices with a few vectors.  Q4_K, Q5_K, Q6_K, Q8_0 and IQ3_XXS on mma.sync.m16n8k16 (fp16, fp32 accumulators).
+// matrices with a few vectors.  Q4_K, Q5_K, Q6_K, Q8_0 and IQ3_XXS on mma.sync with bytes (s8 or u8 x s8, integer sums).
 //
 // Reference kernels of this role: kernels_seg_k.cu:201-241, kernels_exp_iq_v2.cu:259-319 (one warp per row, fp32 FMA);
 // block layouts kquant.rs:341-887.
 //
 // What bounds a call like this is instructions, not bytes: at HBM speed an SM has about four lane-instructions per weight
 // of a 4-bit format, and an FMA kernel spends two (convert, multiply) per weight AND token.  Here a weight costs its
-// decoding only, whatever the number of tokens:
-//   * a lane turns packed bytes into the fp16 A fragment in registers; the quantised value is an integer and exact
-//     (Q4_K, Q5_K: sc * q <= 63 * 31 = 1953 < 2048, formed by one fp16 fma on the 1024 + q bit pattern; Q6_K: q - 32;
+// decoding only, whatever the number of tokens, and it is decoded no further than to a byte:
+//   * a lane turns packed bytes into the A fragment in registers (Q4_K: q, or 16 q where the nibble lies; Q5_K: q; Q6_K: 4 (q - 32);
 //     Q8_0: q; IQ3_XXS: the codebook magnitude <= 62 with its sign), so no weight is rounded;
-//   * the scales multiply the fp32 sums of a 256-element block (Q4_K, Q5_K: d; their mins are one more K step of
-//     m against the sub-block sums of the activations), of a 32-element block (Q8_0, IQ3_XXS) or of 16 elements (Q6_K);
-//   * an activation is P fp16 numbers in P columns of B (P = 3 carries an fp32 to 2^-34 of the row's largest; P = 2 carries 22 bits and is
-//     used where a call of this size had 16 before), of the row times a power of two that puts its largest element into
-//     [512, 1024), so that nothing overflows and sub-block sums fit, too;
-//   * K is walked in the order in which the packed bytes yield elements; the activations are staged in that order.
-// A B column costs an mma per 16 weights of a lane's two rows and half a 16-byte shared-memory read.
+//   * the integer scales multiply the integer sums of a sub-block (Q4_K, Q5_K: sc, IQ3_XXS: 2 s + 1, 32 elements; Q6_K: 16 elements) and
+//     add up over a 256-element block without rounding; d then multiplies in fp32.  (Q8_0 has a d per 32 elements.)  The mins of Q4_K
+//     and Q5_K are one fp16 K step of m against the sub-block sums of the activations;
+//   * an activation is an integer of 31 bits, of its 256-element block times a power of two, as four digits in base 256 in
+//     four columns of B: 2^-31 of the block's largest.
+// Why bytes: the logic and byte-permute instructions, fp16x2 and integer multiplies take two issue cycles of a scheduler here (FFMA and
+// integer adds one), and an mma.sync of bytes (K = 32) eight, as one of fp16 (K = 16) does.  With fp16 weights a Q4_K weight pair was 2.3
+// logic instructions and one fp16x2 multiply, now 0.6; 16 weights of an IQ3_XXS lane 34, now 25, and 12 instead of 18 shared-memory wavefronts.
 //
 // Work: an item is (segment, token tile, block of row groups); a row group is 16 A rows: 16 rows of one matrix, or 8 gate
 // and 8 up rows of the same indices, whose results meet in one lane for silu(g) * u.  A persistent CTA of 16 warps stages
 // an item's activations once; a warp then streams its row groups through a private ring of cp.async stages (one
 // 256-element block of the 16 rows each) without any CTA-wide barrier.  Few row groups for the chip: KS warps share a row
-// group, each takes a part of K, and their sums are added in a fixed order.  A row's result depends on the row, on P and on KS, not on
+// group, each takes a part of K, and their sums are added in a fixed order.  A row's result depends on the row and on KS, not on
 // the tile, the column or the CTA; for decode batches KS is a constant of the shape, so that a token's bits do not depend on its batch.
 //
-// Measured, us per layer of 2048 x 512, top 10 of 512, against one-row GEMVs (to 15 tokens) and tiled fp32 or bf16 tensor-core kernels:
-// 8 tokens, IQ3_XXS 140 -> 95; 32 tokens 502 -> 204; 77 tokens under a skewed router, Q4_K with Q6_K down 895 -> 255.  Issue slots are
-// 0.53 to 0.64 used, DRAM 0.12 to 0.20.
+// Measured, us per pass, fp16 operands in two or three parts -> bytes: six layers of 2048 x 512, top 10 of 512, one of Q4_K and five of
+// IQ3_XXS, 8 tokens 547 -> 491, 32 tokens 1185 -> 1112; two layers of Q4_K with Q6_K down, 77 tokens under a skewed router, 502 -> 404.  Distance
+// from the 64-bit result, five formats, normal and heavy-tailed inputs: 0.43 of what it was.
 #include <algorithm>
 
 #include "dnb_common.cuh"
 #include "formats.cuh"
 #include "tc_ptx.cuh"
-#include "iq3_f16.cuh"
+#include "dnb_iq_tables.h"
 
 namespace dnb {
 
 constexpr int kMmWarps = 16;
 constexpr int kMmThreads = kMmWarps * 32;
 constexpr int kMmSegMax = 1088;  // segments of a launch at most
+constexpr int kMmFixed = ((kMmSegMax + 4 + 16) * 4 + 127) / 128 * 128;  // bytes of the segment table in shared memory
+constexpr uint32_t kMmBookAlign = 32768;  // IQ3_XXS tables
+constexpr uint32_t kMmSmemBase = 1024;    // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
+constexpr int kMmTok = 2;        // tokens of a column tile: eight columns, four digits a token
 
 // 256 elements of a row: bytes, 16-byte units of a stage row (blocks that are not 16-byte sized start anywhere in their first
-// unit), and the unit stride of a stage row (chosen so that the eight rows a warp reads at once fall on different banks).
+// unit), and the stride of a stage row (chosen so that rows read together fall on different banks; Q5_K and Q8_0: as far as the ring's size allows).
 template <int T> struct Mq;
-template <> struct Mq<T_Q4_K> { static constexpr int BB = 144, UNITS = 9, RS = 144; static constexpr bool ALIGNED = true; };
+template <> struct Mq<T_Q4_K> { static constexpr int BB = 144, UNITS = 9, RS = 160; static constexpr bool ALIGNED = true; };
 template <> struct Mq<T_Q5_K> { static constexpr int BB = 176, UNITS = 11, RS = 176; static constexpr bool ALIGNED = true; };
 template <> struct Mq<T_Q6_K> { static constexpr int BB = 210, UNITS = 14, RS = 240; static constexpr bool ALIGNED = false; };
 template <> struct Mq<T_IQ3_XXS> { static constexpr int BB = 98, UNITS = 7, RS = 112; static constexpr bool ALIGNED = false; };
@@ -52,13 +56,15 @@ template <> struct Mq<T_Q8_0> { static constexpr int BB = 272, UNITS = 17, RS = 
 
 template <int T> constexpr bool mq_mins = (T == T_Q4_K || T == T_Q5_K);
 
-// First element (of 256) of the two groups of four that unit u = 0..7 of lane t takes; `swap`: a group's order is 0, 2, 1, 3.
+// ---- activations -----------------------------------------------------------------------------------------------------------
+// A 256-element block of one token: [4 digits][256 bytes, unit u and lane t at 32 u + 8 t, kXDigit bytes apart: four digits of a
+// lane's eight bytes fall on different banks][3 parts][8] sub-block sums as fp16 (formats with mins), then what undoes the scaling.
+constexpr int kXDigit = 288, kXSums = 4 * kXDigit, kXInv = kXSums + 48, kXBlock = kXInv + 16;
+
+// First element (of 256) of the two groups of four that unit u = 0..7 of lane t takes.
 template <int T>
 __device__ __forceinline__ void mm_unit_elems(int u, int t, int& e0, int& e1) {
-    if constexpr (mq_mins<T>) {
-        e0 = 64 * t + 4 * u;
-        e1 = e0 + 32;
-    } else if constexpr (T == T_Q6_K) {
+    if constexpr (T == T_Q6_K) {
         e0 = (u >> 2) * 128 + (u & 1) * 32 + ((u >> 1) & 1) * 16 + 4 * t;
         e1 = e0 + 64;
     } else {
@@ -66,11 +72,98 @@ __device__ __forceinline__ void mm_unit_elems(int u, int t, int& e0, int& e1) {
         e1 = e0 + 4;
     }
 }
+// The digits of four elements: d[j] = byte j of each.
+__device__ __forceinline__ void mm_digits(const int (&v)[4], uint32_t (&d)[4]) {
+    const uint32_t a = __byte_perm(v[0], v[1], 0x5140), b = __byte_perm(v[2], v[3], 0x5140);
+    const uint32_t c = __byte_perm(v[0], v[1], 0x7362), e = __byte_perm(v[2], v[3], 0x7362);
+    d[0] = __byte_perm(a, b, 0x5410);
+    d[1] = __byte_perm(a, b, 0x7632);
+    d[2] = __byte_perm(c, e, 0x5410);
+    d[3] = __byte_perm(c, e, 0x7632);
+}
+// Two values as three fp16 pairs whose sums are the values: every bit of the elements above 1/1024 of the block's largest, and 2^-34 of the
+// largest below, where the third part meets fp16's smallest number.
+__device__ __forceinline__ void mm_split(float a, float b, uint32_t (&h)[3]) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const __half2 v = __floats2half2_rn(a, b);
+        h[p] = *reinterpret_cast<const uint32_t*>(&v);
+        if (p < 2) {
+            const float2 f = __half22float2(v);
+            a -= f.x;
+            b -= f.y;
+        }
+    }
+}
+__device__ __forceinline__ float mm_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
 
-__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// One warp: a token's 256 elements at xr into their place in shared memory.  The block times 2^s is below 2^30 and rounded to an integer; its
+// four digits in base 256 are balanced (-128 .. 127), so that sum_j 256^j * d_j is the integer.
+template <int T>
+__device__ __forceinline__ void mm_stage_block(const float* __restrict__ xr, uint8_t* dst, int lane) {
+    const int u = lane >> 2, t = lane & 3;
+    int e0, e1;
+    mm_unit_elems<T>(u, t, e0, e1);
+    const float4 f0 = *reinterpret_cast<const float4*>(xr + e0), f1 = *reinterpret_cast<const float4*>(xr + e1);
+    float x[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    uint32_t mx = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mx = max(mx, __float_as_uint(fabsf(x[i])));
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    const int ex = (int)(mx >> 23);  // biased exponent of the largest |x|; s puts it into [2^29, 2^30)
+    const int s = ex == 0 ? 0 : min(149, 156 - ex), s1 = min(s, 120);
+    const float up = mm_pow2(s1);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] *= up;
+    if (s > s1) {  // a block below 2^-90 throughout: a second power of two
+        const float up2 = mm_pow2(s - s1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] *= up2;
+    }
+    if constexpr (mq_mins<T>) {  // a sub-block is a unit: its sum over the four lanes, in units of 2^20
+        float a = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        a += __shfl_xor_sync(0xffffffffu, a, 2);
+        a *= 0x1p-20f;
+        const float b = __shfl_xor_sync(0xffffffffu, a, 4);
+        uint32_t h[3];
+        mm_split(a, b, h);
+        if ((lane & 7) == 0) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint32_t*>(dst + kXSums + p * 16 + (lane >> 3) * 4) = h[p];
+        }
+    }
+    int v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = (int)(((uint32_t)__float2int_rn(x[i]) + 0x00808080u) ^ 0x00808080u);
+    uint32_t d0[4], d1[4];
+    mm_digits({v[0], v[1], v[2], v[3]}, d0);
+    mm_digits({v[4], v[5], v[6], v[7]}, d1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<uint2*>(dst + j * kXDigit + lane * 8) = make_uint2(d0[j], d1[j]);
+    // 2^-s for the low two digits, 2^(16 - s) for the high two; a block with an infinity or a NaN makes a NaN of every sum
+    if (lane < 2) {
+        const int e = 16 * lane - s;
+        reinterpret_cast<float*>(dst + kXInv)[lane] = ex == 255 ? __uint_as_float(0x7fc00000u) : e >= -126 ? mm_pow2(e) : __uint_as_float(1u << (149 + e));
+    }
+}
+
+// ---- integer products --------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void mma_u8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(0));
+}
+template <int C0>  // every element of C
+__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint2 b) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b.x), "r"(b.y), "r"(C0));
+}
+__device__ __forceinline__ void mma_s8_k16(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(a0), "r"(a1), "r"(b), "r"(0));
 }
 __device__ __forceinline__ void mma_f16_z(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
@@ -79,42 +172,233 @@ __device__ __forceinline__ void mma_f16_z(float (&c)[4], uint32_t a0, uint32_t a
 }
 __device__ __forceinline__ uint32_t ld32u(const uint8_t* p) { return ld16(p) | (ld16(p + 2) << 16); }  // 2-byte aligned
 
+// Q4_K / Q5_K header of a row: d, dmin, the eight scales (a byte each) and the pair of mins of sub-blocks 2 t, 2 t + 1 (kquant.rs:878-887).
+struct MmK { float d, dmin; uint32_t sc[2], mm; };
+__device__ __forceinline__ MmK mm_k_header(const uint8_t* row, int t) {
+    const uint4 h = *reinterpret_cast<const uint4*>(row);
+    MmK r;
+    r.d = h2f((uint16_t)h.x);
+    r.dmin = h2f((uint16_t)(h.x >> 16));
+    r.sc[0] = h.y & 0x3f3f3f3fu;
+    r.sc[1] = (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u);
+    const int sh = 16 * (t & 1);
+    const uint32_t mn = (t < 2 ? h.z & 0x3f3f3f3fu : ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u)) >> sh;
+    r.mm = h2sub(__byte_perm(mn, 0x64646464u, 0x4140u), 0x64006400u);
+    return r;
+}
+
+// IQ3_XXS tables in shared memory, a copy per bank (a lane reads copy `lane`: no conflicts), 128 bytes from entry to entry:
+//   grid: the four magnitudes of a codebook entry, a byte each
+//   sgn : the signs of a 7-bit code (the eighth makes their number even): weight i at bit 8 i, weight 4 + i at bit 8 i + 1
+// The tables sit on a 32 KB boundary of the shared-memory address space: an entry's address is a shift and one and-or.
+struct MmTables { uint32_t grid[256 * 32]; uint32_t sgn[128 * 32]; };
+static __device__ __align__(16) MmTables g_mm_s8;
+static bool g_mm_s8_up[64] = {false};
+
+static int upload_mm_s8(int device) {
+    if (device < 0 || device >= 64) return DNB_ERR_ARG;
+    if (g_mm_s8_up[device]) return DNB_OK;
+    static MmTables tb;
+    for (int e = 0; e < 256; ++e)
+        for (int r = 0; r < 32; ++r) tb.grid[e * 32 + r] = dnb_iq3xxs_grid[e];
+    for (uint32_t code = 0; code < 128; ++code) {
+        const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
+        uint32_t u = 0;
+        for (int i = 0; i < 4; ++i) u |= ((sg >> i) & 1u) << (8 * i) | ((sg >> (4 + i)) & 1u) << (8 * i + 1);
+        for (int r = 0; r < 32; ++r) tb.sgn[code * 32 + r] = u;
+    }
+    DNB_CUDA(cudaMemcpyToSymbol(g_mm_s8, &tb, sizeof(tb)));
+    g_mm_s8_up[device] = true;
+    return DNB_OK;
+}
+
+// Eight weights of an IQ3_XXS sub-block as signed bytes.  gl, sl: shared addresses of the lane's copies; idx: the two codebook indices; code:
+// the sub-block word rotated so that the quarter's 7-bit sign code starts at bit 7.  A negative byte is ~v + 1 (v >= 4: nothing carries).
+__device__ __forceinline__ void iq3_s8(uint32_t gl, uint32_t sl, uint32_t idx, uint32_t code, uint32_t& p0, uint32_t& p1) {
+    uint32_t u, g0, g1;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"((code & 0x3f80u) | sl));  // constant tables: plain asm, free to move
+    asm("ld.shared.u32 %0, [%1];" : "=r"(g0) : "r"(((idx << 7) & 0x7f80u) | gl));
+    asm("ld.shared.u32 %0, [%1];" : "=r"(g1) : "r"(((idx >> 1) & 0x7f80u) | gl));
+    const uint32_t o0 = u & 0x01010101u, o1 = (u >> 1) & 0x01010101u;
+    p0 = (g0 ^ (o0 * 255u)) + o0;
+    p1 = (g1 ^ (o1 * 255u)) + o1;
+}
+
 // One 256-element block of 16 rows (this lane: rows `ra` and `rb`) against NT column tiles; bp[i]: the lane's B column of tile
-// i at this block; nt: tiles in use.  acc += scales * sums.
+// i at this block; inv, sumw: of the token whose columns the lane's accumulators hold, and of its B column; nt: tiles in use.
+// acc[i] += scales * sums: rows `ra` and `rb`, digits 0 and 1 of a token (t even) or 2 and 3 (t odd).
 template <int T, int NT>
 __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, uint32_t gl, uint32_t sl, const uint8_t* const (&bp)[NT],
-                                         const uint32_t (&sumw)[NT], int nt, float (&acc)[NT][4]) {
-    if constexpr (mq_mins<T>) {
-        const KScales sa = k_scales(ra, t), sb = k_scales(rb, t);
-        constexpr bool FIVE = T == T_Q5_K;
-        constexpr int QS = FIVE ? 48 : 16;
-        float D[NT][4];
+                                         const uint32_t (&sumw)[NT], const float (&inv)[NT], int nt, float (&acc)[NT][2]) {
+    if constexpr (T == T_Q8_0) {
+        float s[NT][2];
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
+        for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) D[i][c] = 0.f;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const uint4 qa = *reinterpret_cast<const uint4*>(ra + QS + 32 * t + 16 * half);
-            const uint4 qb = *reinterpret_cast<const uint4*>(rb + QS + 32 * t + 16 * half);
-            uint4 ha = make_uint4(0, 0, 0, 0), hb = ha;
-            if constexpr (FIVE) {
-                ha = *reinterpret_cast<const uint4*>(ra + 16 + 16 * half);
-                hb = *reinterpret_cast<const uint4*>(rb + 16 + 16 * half);
+        for (int ib = 0; ib < 8; ++ib) {
+            // the bytes start 2 or 4 bytes behind an aligned word
+            uint32_t p[2], q[2];
+            const uint8_t *a = ra + 34 * ib + 8 * t, *b = rb + 34 * ib + 8 * t;
+            if (ib & 1) {
+                p[0] = *reinterpret_cast<const uint32_t*>(a + 2);
+                p[1] = *reinterpret_cast<const uint32_t*>(a + 6);
+                q[0] = *reinterpret_cast<const uint32_t*>(b + 2);
+                q[1] = *reinterpret_cast<const uint32_t*>(b + 6);
+            } else {
+                const uint32_t a0 = *reinterpret_cast<const uint32_t*>(a), a1 = *reinterpret_cast<const uint32_t*>(a + 4), a2 = *reinterpret_cast<const uint32_t*>(a + 8);
+                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(b), b1 = *reinterpret_cast<const uint32_t*>(b + 4), b2 = *reinterpret_cast<const uint32_t*>(b + 8);
+                p[0] = __byte_perm(a0, a1, 0x5432);
+                p[1] = __byte_perm(a1, a2, 0x5432);
+                q[0] = __byte_perm(b0, b1, 0x5432);
+                q[1] = __byte_perm(b1, b2, 0x5432);
             }
-            const uint32_t wa[4] = {qa.x, qa.y, qa.z, qa.w}, wb[4] = {qb.x, qb.y, qb.z, qb.w};
-            const uint32_t fa[4] = {ha.x, ha.y, ha.z, ha.w}, fb[4] = {hb.x, hb.y, hb.z, hb.w};
+            const float fa = h2f(ld16(ra + 34 * ib)), fb = h2f(ld16(rb + 34 * ib));
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t p[4], q[4];
-                k_word<FIVE>(wa[i], fa[i] >> (2 * t), sa, p);
-                k_word<FIVE>(wb[i], fb[i] >> (2 * t), sb, q);
+            for (int n = 0; n < NT; ++n) {
+                if (NT == 1 || n < nt) {
+                    // sums start at the bits of 1.5 * 2^23, so that they are floats as they stand (|sum| <= 2^19)
+                    int D[4];
+                    mma_s8<0x4B400000>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
+                    const float m = 12582912.f;
+                    s[n][0] = fmaf(fa, fmaf(256.f, __int_as_float(D[1]) - m, __int_as_float(D[0]) - m), s[n][0]);
+                    s[n][1] = fmaf(fb, fmaf(256.f, __int_as_float(D[3]) - m, __int_as_float(D[2]) - m), s[n][1]);
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            if (NT == 1 || n < nt) {
+                acc[n][0] = fmaf(s[n][0], inv[n], acc[n][0]);
+                acc[n][1] = fmaf(s[n][1], inv[n], acc[n][1]);
+            }
+        }
+    } else {
+        int c[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) c[n][i] = 0;
+        // one sub-block: its sums times its scales
+        auto add = [&](int n, const int (&D)[4], int fa, int fb) {
+            c[n][0] += fa * D[0];
+            c[n][1] += fa * D[1];
+            c[n][2] += fb * D[2];
+            c[n][3] += fb * D[3];
+        };
+        float da, db, dma = 0.f, dmb = 0.f;
+        uint32_t mma = 0u, mmb = 0u;
+        if constexpr (mq_mins<T>) {
+            // bounds of a block's sums: Q4_K 8 * 16 * 63 * 32 * 15 * 128 < 2^29 (see below for the 16), Q5_K 8 * 63 * 32 * 31 * 128 < 2^26
+            const MmK ka = mm_k_header(ra, t), kb = mm_k_header(rb, t);
+            da = ka.d; db = kb.d; dma = ka.dmin; dmb = kb.dmin; mma = ka.mm; mmb = kb.mm;
+            constexpr bool FIVE = T == T_Q5_K;
+            uint2 ha = make_uint2(0u, 0u), hb = ha;
+            if constexpr (FIVE) {
+                ha = *reinterpret_cast<const uint2*>(ra + 16 + 8 * t);
+                hb = *reinterpret_cast<const uint2*>(rb + 16 + 8 * t);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {  // sub-blocks 2 j (low nibbles) and 2 j + 1 (high)
+                const uint2 qa = *reinterpret_cast<const uint2*>(ra + (FIVE ? 48 : 16) + 32 * j + 8 * t);
+                const uint2 qb = *reinterpret_cast<const uint2*>(rb + (FIVE ? 48 : 16) + 32 * j + 8 * t);
+                const uint32_t wa = ka.sc[j >> 1] >> (16 * (j & 1)), wb = kb.sc[j >> 1] >> (16 * (j & 1));
+                int fa[2] = {(int)(wa & 0xffu), (int)((wa >> 8) & 0xffu)}, fb[2] = {(int)(wb & 0xffu), (int)((wb >> 8) & 0xffu)};
+                uint32_t a[2][2], b[2][2];
+                if constexpr (FIVE) {
+                    auto fifth = [&](uint32_t h, int u) { return (u < 4 ? h << (4 - u) : h >> (u - 4)) & 0x10101010u; };
+                    a[0][0] = (qa.x & 0x0f0f0f0fu) | fifth(ha.x, 2 * j);
+                    a[0][1] = (qa.y & 0x0f0f0f0fu) | fifth(ha.y, 2 * j);
+                    b[0][0] = (qb.x & 0x0f0f0f0fu) | fifth(hb.x, 2 * j);
+                    b[0][1] = (qb.y & 0x0f0f0f0fu) | fifth(hb.y, 2 * j);
+                    a[1][0] = ((qa.x >> 4) & 0x0f0f0f0fu) | fifth(ha.x, 2 * j + 1);
+                    a[1][1] = ((qa.y >> 4) & 0x0f0f0f0fu) | fifth(ha.y, 2 * j + 1);
+                    b[1][0] = ((qb.x >> 4) & 0x0f0f0f0fu) | fifth(hb.x, 2 * j + 1);
+                    b[1][1] = ((qb.y >> 4) & 0x0f0f0f0fu) | fifth(hb.y, 2 * j + 1);
+                } else {  // the high nibbles stay where they are, 16 times too large, and the even sub-blocks' scales take the 16, too
+                    a[0][0] = qa.x & 0x0f0f0f0fu; a[0][1] = qa.y & 0x0f0f0f0fu;
+                    b[0][0] = qb.x & 0x0f0f0f0fu; b[0][1] = qb.y & 0x0f0f0f0fu;
+                    a[1][0] = qa.x & 0xf0f0f0f0u; a[1][1] = qa.y & 0xf0f0f0f0u;
+                    b[1][0] = qb.x & 0xf0f0f0f0u; b[1][1] = qb.y & 0xf0f0f0f0u;
+                    fa[0] *= 16;
+                    fb[0] *= 16;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        if (NT == 1 || n < nt) {
+                            int D[4];
+                            mma_u8(D, a[h][0], b[h][0], a[h][1], b[h][1], *reinterpret_cast<const uint2*>(bp[n] + (2 * j + h) * 32));
+                            add(n, D, fa[h], fb[h]);
+                        }
+                    }
+            }
+            if constexpr (!FIVE) {
+                da *= 0.0625f;
+                db *= 0.0625f;
+            }
+        } else if constexpr (T == T_IQ3_XXS) {  // (d / 4) * (2 s + 1) (kquant.rs:667); sums: 8 * 31 * 32 * 62 * 128 < 2^26
+            da = 0.25f * h2f(ld16(ra));
+            db = 0.25f * h2f(ld16(rb));
+            // the eight sub-block words of a row as aligned words, shifted into place (a block starts on any even byte)
+            const uint32_t ma = (tcp::s32(ra) + 2u) & 2u, mb = (tcp::s32(rb) + 2u) & 2u;
+            const uint32_t* wa = reinterpret_cast<const uint32_t*>(ra + 66 - ma);
+            const uint32_t* wb = reinterpret_cast<const uint32_t*>(rb + 66 - mb);
+            const uint32_t sa = ma * 8u, sb = mb * 8u;
+            const uint8_t* ia = ra + 2 + 2 * t;
+            const uint8_t* ib2 = rb + 2 + 2 * t;
+            const int st = (7 * t + 25) & 31;
+            uint32_t la = wa[0], lb = wb[0];
+#pragma unroll
+            for (int ib = 0; ib < 8; ++ib) {
+                // the ninth word belongs to the row only where the words are shifted
+                const uint32_t naw = wa[ib < 7 ? ib + 1 : 7 + (ma >> 1)], nbw = wb[ib < 7 ? ib + 1 : 7 + (mb >> 1)];
+                const uint32_t xa = __funnelshift_r(la, naw, sa), xb = __funnelshift_r(lb, nbw, sb);
+                la = naw;
+                lb = nbw;
+                uint32_t p[2], q[2];
+                iq3_s8(gl, sl, ld16(ia + 8 * ib), __funnelshift_r(xa, xa, st), p[0], p[1]);
+                iq3_s8(gl, sl, ld16(ib2 + 8 * ib), __funnelshift_r(xb, xb, st), q[0], q[1]);
+                const int fa = (int)(2u * (xa >> 28) + 1u), fb = (int)(2u * (xb >> 28) + 1u);
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
                     if (NT == 1 || n < nt) {
-                        const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + (half * 4 + i) * 64);
-                        mma_f16(D[n], p[0], q[0], p[1], q[1], y.x, y.y);
-                        mma_f16(D[n], p[2], q[2], p[3], q[3], y.z, y.w);
+                        int D[4];
+                        mma_s8<0>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
+                        add(n, D, fa, fb);
+                    }
+                }
+            }
+        } else {  // Q6_K: a K step is one 16-element group of one scale; bytes are 4 * (q - 32), sums 16 * 128 * 16 * 128 * 128 < 2^30
+            da = 0.25f * h2f(ld16(ra + 208));
+            db = 0.25f * h2f(ld16(rb + 208));
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {  // (half, is)
+                const int half = g >> 1, is = g & 1;
+                // the upper bit of each pair inverted: q - 32 in two's complement
+                const uint32_t ha = ld32u(ra + 128 + 32 * half + 16 * is + 4 * t) ^ 0xaaaaaaaau, hb = ld32u(rb + 128 + 32 * half + 16 * is + 4 * t) ^ 0xaaaaaaaau;
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const uint32_t qa = ld32u(ra + 64 * half + 32 * w + 16 * is + 4 * t), qb = ld32u(rb + 64 * half + 32 * w + 16 * is + 4 * t);
+                    uint2 y[NT];
+#pragma unroll
+                    for (int n = 0; n < NT; ++n)
+                        if (NT == 1 || n < nt) y[n] = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 32);
+#pragma unroll
+                    for (int hi = 0; hi < 2; ++hi) {
+                        const int sh = 6 - 2 * w - 4 * hi;  // the pair of bits to the top of its byte
+                        const uint32_t va = ((hi ? qa >> 2 : qa << 2) & 0x3c3c3c3cu) | ((ha << sh) & 0xc0c0c0c0u);
+                        const uint32_t vb = ((hi ? qb >> 2 : qb << 2) & 0x3c3c3c3cu) | ((hb << sh) & 0xc0c0c0c0u);
+                        const int sc = 192 + 8 * half + is + 2 * w + 4 * hi;
+                        const int fa = *reinterpret_cast<const int8_t*>(ra + sc), fb = *reinterpret_cast<const int8_t*>(rb + sc);
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            if (NT == 1 || n < nt) {
+                                int D[4];
+                                mma_s8_k16(D, va, vb, hi ? y[n].y : y[n].x);
+                                add(n, D, fa, fb);
+                            }
+                        }
                     }
                 }
             }
@@ -122,114 +406,16 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
             if (NT == 1 || n < nt) {
-                float M[4];
-                mma_f16_z(M, sa.mm, sb.mm, 0u, 0u, sumw[n], 0u);
-                acc[n][0] = fmaf(-sa.dmin, M[0], fmaf(sa.d, D[n][0], acc[n][0]));
-                acc[n][1] = fmaf(-sa.dmin, M[1], fmaf(sa.d, D[n][1], acc[n][1]));
-                acc[n][2] = fmaf(-sb.dmin, M[2], fmaf(sb.d, D[n][2], acc[n][2]));
-                acc[n][3] = fmaf(-sb.dmin, M[3], fmaf(sb.d, D[n][3], acc[n][3]));
-            }
-        }
-    } else if constexpr (T == T_IQ3_XXS) {
-        // (d / 4) * (2 s + 1) (kquant.rs:667) = 8 d v - 7.75 d with v = 1 + s / 16 read off the bits: exact, d has 11 significant bits
-        // (a conversion from integer would be a quarter-rate instruction)
-        const float da = h2f(ld16(ra)), db = h2f(ld16(rb));
-        const float ma8 = 8.f * da, na = -7.75f * da, mb8 = 8.f * db, nbs = -7.75f * db;
-        // the eight sub-block words of a row as aligned words, shifted into place (a block starts on any even byte)
-        const uint32_t ma = (tcp::s32(ra) + 2u) & 2u, mb = (tcp::s32(rb) + 2u) & 2u;
-        const uint32_t* wa = reinterpret_cast<const uint32_t*>(ra + 66 - ma);
-        const uint32_t* wb = reinterpret_cast<const uint32_t*>(rb + 66 - mb);
-        const uint32_t sa = ma * 8u, sb = mb * 8u;
-        const uint8_t* ia = ra + 2 + 2 * t;
-        const uint8_t* ibp = rb + 2 + 2 * t;
-        const int st = (7 * t + 26) & 31;
-        uint32_t la = wa[0], lb = wb[0];
-#pragma unroll
-        for (int ib = 0; ib < 8; ++ib) {
-            // the ninth word belongs to the row only where the words are shifted
-            const uint32_t naw = wa[ib < 7 ? ib + 1 : 7 + (ma >> 1)], nbw = wb[ib < 7 ? ib + 1 : 7 + (mb >> 1)];
-            const uint32_t xa = __funnelshift_r(la, naw, sa), xb = __funnelshift_r(lb, nbw, sb);
-            la = naw;
-            lb = nbw;
-            uint32_t p[4], q[4];
-            iq3_pairs_h(gl, sl, ld16(ia + 8 * ib), __funnelshift_r(xa, xa, st), p);
-            iq3_pairs_h(gl, sl, ld16(ibp + 8 * ib), __funnelshift_r(xb, xb, st), q);
-            const float fa = fmaf(__uint_as_float(((xa >> 9) & 0x00780000u) | 0x3f800000u), ma8, na);
-            const float fb = fmaf(__uint_as_float(((xb >> 9) & 0x00780000u) | 0x3f800000u), mb8, nbs);
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                if (NT == 1 || n < nt) {
-                    const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + ib * 64);
-                    float D[4];
-                    mma_f16_z(D, p[0], q[0], p[1], q[1], y.x, y.y);
-                    mma_f16(D, p[2], q[2], p[3], q[3], y.z, y.w);
-                    acc[n][0] = fmaf(fa, D[0], acc[n][0]);
-                    acc[n][1] = fmaf(fa, D[1], acc[n][1]);
-                    acc[n][2] = fmaf(fb, D[2], acc[n][2]);
-                    acc[n][3] = fmaf(fb, D[3], acc[n][3]);
+                float va = da * fmaf(256.f, (float)c[n][1], (float)c[n][0]), vb = db * fmaf(256.f, (float)c[n][3], (float)c[n][2]);
+                if constexpr (mq_mins<T>) {
+                    float M[4];
+                    mma_f16_z(M, mma, mmb, 0u, 0u, sumw[n], 0u);
+                    const float k = (t & 1) ? 16.f : 0x1p20f;  // columns 0, 1 of a token stand beside its low digits, column 2 beside the high ones
+                    va = fmaf(-dma, (M[0] + M[1]) * k, va);
+                    vb = fmaf(-dmb, (M[2] + M[3]) * k, vb);
                 }
-            }
-        }
-    } else if constexpr (T == T_Q8_0) {
-        const uint32_t bias = 0x64806480u;  // 1024 + 128
-#pragma unroll 4
-        for (int ib = 0; ib < 8; ++ib) {
-            const float fa = h2f(ld16(ra + 34 * ib)), fb = h2f(ld16(rb + 34 * ib));
-            uint32_t p[4], q[4];
-#pragma unroll
-            for (int v = 0; v < 2; ++v) {
-                const uint32_t wa = ld32u(ra + 34 * ib + 2 + 8 * t + 4 * v) ^ 0x80808080u;
-                const uint32_t wb = ld32u(rb + 34 * ib + 2 + 8 * t + 4 * v) ^ 0x80808080u;
-                p[2 * v] = h2sub(__byte_perm(wa, 0x64646464u, 0x5140u), bias);
-                p[2 * v + 1] = h2sub(__byte_perm(wa, 0x64646464u, 0x7362u), bias);
-                q[2 * v] = h2sub(__byte_perm(wb, 0x64646464u, 0x5140u), bias);
-                q[2 * v + 1] = h2sub(__byte_perm(wb, 0x64646464u, 0x7362u), bias);
-            }
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                if (NT == 1 || n < nt) {
-                    const uint4 y = *reinterpret_cast<const uint4*>(bp[n] + ib * 64);
-                    float D[4];
-                    mma_f16_z(D, p[0], q[0], p[1], q[1], y.x, y.y);
-                    mma_f16(D, p[2], q[2], p[3], q[3], y.z, y.w);
-                    acc[n][0] = fmaf(fa, D[0], acc[n][0]);
-                    acc[n][1] = fmaf(fa, D[1], acc[n][1]);
-                    acc[n][2] = fmaf(fb, D[2], acc[n][2]);
-                    acc[n][3] = fmaf(fb, D[3], acc[n][3]);
-                }
-            }
-        }
-    } else {  // Q6_K: a K step is one 16-element group of one scale
-        const float da = h2f(ld16(ra + 208)), db = h2f(ld16(rb + 208));
-        const uint32_t bias = 0x64206420u;  // 1024 + 32
-#pragma unroll 2
-        for (int g = 0; g < 4; ++g) {  // (half, is)
-            const int half = g >> 1, is = g & 1;
-            const uint32_t ha = ld32u(ra + 128 + 32 * half + 16 * is + 4 * t), hb = ld32u(rb + 128 + 32 * half + 16 * is + 4 * t);
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const uint32_t qa = ld32u(ra + 64 * half + 32 * w + 16 * is + 4 * t), qb = ld32u(rb + 64 * half + 32 * w + 16 * is + 4 * t);
-#pragma unroll
-                for (int hi = 0; hi < 2; ++hi) {
-                    const uint32_t va = ((qa >> (4 * hi)) & 0x0f0f0f0fu) | (((ha >> (2 * w + 4 * hi)) & 0x03030303u) << 4);
-                    const uint32_t vb = ((qb >> (4 * hi)) & 0x0f0f0f0fu) | (((hb >> (2 * w + 4 * hi)) & 0x03030303u) << 4);
-                    const uint32_t p0 = h2sub(__byte_perm(va, 0x64646464u, 0x5140u), bias), p1 = h2sub(__byte_perm(va, 0x64646464u, 0x7362u), bias);
-                    const uint32_t q0 = h2sub(__byte_perm(vb, 0x64646464u, 0x5140u), bias), q1 = h2sub(__byte_perm(vb, 0x64646464u, 0x7362u), bias);
-                    const int sc = 192 + 8 * half + is + 2 * w + 4 * hi;
-                    const float fa = da * (float)(int)*reinterpret_cast<const int8_t*>(ra + sc), fb = db * (float)(int)*reinterpret_cast<const int8_t*>(rb + sc);
-#pragma unroll
-                    for (int n = 0; n < NT; ++n) {
-                        if (NT == 1 || n < nt) {
-                            const uint2 y = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 64 + 8 * hi);
-                            float D[4];
-                            mma_f16_z(D, p0, q0, p1, q1, y.x, y.y);
-                            acc[n][0] = fmaf(fa, D[0], acc[n][0]);
-                            acc[n][1] = fmaf(fa, D[1], acc[n][1]);
-                            acc[n][2] = fmaf(fb, D[2], acc[n][2]);
-                            acc[n][3] = fmaf(fb, D[3], acc[n][3]);
-                        }
-                    }
-                }
+                acc[n][0] = fmaf(va, inv[n], acc[n][0]);
+                acc[n][1] = fmaf(vb, inv[n], acc[n][1]);
             }
         }
     }
@@ -246,7 +432,6 @@ struct MmArgs {
     const int32_t* row_token;  // packed row -> x row, or null
     float* out;                // [packed row][n_out]
     int ks, nst;               // warps that split K, stages of a warp's ring
-    int col_stride;            // bytes between B columns
     int skip;                  // row groups' time that a tile's activations take
     uint32_t smem;             // bytes of dynamic shared memory
     int* status;
@@ -254,47 +439,24 @@ struct MmArgs {
 
 __device__ __forceinline__ void mm_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
-// Scale of a row: the power of two that puts its largest element into [512, 1024).
-__device__ __forceinline__ float mm_row_scale(uint32_t amax_bits) {
-    const int ex = (int)(amax_bits >> 23);  // biased exponent of the largest |x|
-    const int s = ex == 0 ? 0 : max(-126, min(126, 9 - (ex - 127)));
-    return __uint_as_float((uint32_t)(s + 127) << 23);
-}
-// Two values as P fp16 pairs whose sums are the values.  P = 2: 22 bits of the row's (one matrix: the block's) largest element; P = 3: every
-// bit of the elements above 1/1024 of the largest, and 2^-34 of the largest below, where the third part meets fp16's smallest number.
-template <int P>
-__device__ __forceinline__ void mm_split(float a, float b, uint32_t (&h)[P]) {
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
-        const __half2 v = __floats2half2_rn(a, b);
-        h[p] = *reinterpret_cast<const uint32_t*>(&v);
-        if (p + 1 < P) {
-            const float2 f = __half22float2(v);
-            a -= f.x;
-            b -= f.y;
-        }
-    }
-}
-
-template <int T, bool FUSED, int P, int NT>
+template <int T, bool FUSED, int NT>
 __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     using Q = Mq<T>;
-    constexpr int TPT = P == 3 ? 2 : 4;  // tokens of a column tile (P = 3: columns 3 and 7 are copies nobody adds)
-    constexpr int TT = NT * TPT;         // tokens of an item
+    constexpr int TT = NT * kMmTok;  // tokens of an item
     constexpr int STAGE = 16 * Q::RS;
     extern __shared__ __align__(128) uint8_t smem[];
     int* pre = reinterpret_cast<int*>(smem);                            // [kMmSegMax + 1] first token tile of a segment
     int* wsum = pre + kMmSegMax + 4;                                    // [16]
-    uint32_t* amax = reinterpret_cast<uint32_t*>(wsum + 16);            // [2][16]
-    uint8_t* p0 = smem + ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
-    float* red = reinterpret_cast<float*>(p0);                          // [2][16 warps][NT * 4][32] when ks > 1
-    if (A.ks > 1) p0 += 2 * kMmWarps * NT * 4 * 32 * sizeof(float);
-    uint8_t* acts = p0;
-    p0 += (size_t)TT * P * A.col_stride;
+    uint8_t* p0 = smem + kMmFixed;
+    float* red = reinterpret_cast<float*>(p0);                          // [2][16 warps][NT * 2][32] when ks > 1
+    if (A.ks > 1) p0 += 2 * kMmWarps * NT * 2 * 32 * sizeof(float);
+    const int nb = A.n_in >> 8;
+    uint8_t* acts = p0;                                                 // [TT tokens][nb blocks][kXBlock]
+    p0 += (size_t)TT * nb * kXBlock;
     uint8_t* book = p0;
     if constexpr (T == T_IQ3_XXS) {
         book += (kMmBookAlign - (tcp::s32(p0) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
-        p0 = book + sizeof(MmCodebook);
+        p0 = book + sizeof(MmTables);
     }
     uint8_t* ring = p0;
     if (T == T_IQ3_XXS && (uint32_t)(ring - smem) + kMmWarps * A.nst * STAGE > A.smem) {  // only if shared memory started elsewhere
@@ -305,12 +467,11 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     ring += (size_t)warp * A.nst * STAGE;
     if constexpr (T == T_IQ3_XXS) {
-        for (int i = tid; i < (int)(sizeof(MmCodebook) / 16); i += kMmThreads)
-            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_codebook) + 16 * i);
+        for (int i = tid; i < (int)(sizeof(MmTables) / 16); i += kMmThreads)
+            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_s8) + 16 * i);
         tcp::cp_async_commit();
         tcp::cp_async_wait_all();
     }
-    if (tid < 32) amax[tid] = 0u;
     pdl_wait();
     pdl_launch_dependents();
 
@@ -343,23 +504,21 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
         if (tid == kMmThreads - 1) pre[nseg] = at;
         __syncthreads();
     }
-    const int nb = A.n_in >> 8;
     const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
     const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
     const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
-    const uint32_t gl = tcp::s32(book) + 8 * (lane & (kLutRep - 1)), sl = tcp::s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
-    int par = 0;
+    const uint32_t gl = tcp::s32(book) + 4 * lane, sl = gl + (uint32_t)sizeof(uint32_t) * 256 * 32;
     // This CTA's share of all (tile, row group) pairs: a range of pairs in a row.  Another tile means another set of activations,
     // which takes as long as A.skip row groups: each tile is that much longer, and a CTA that has two gets so much less of them.
     const int span = n_rg + A.skip, total = pre[nseg] * span;
     const int share = total / (int)gridDim.x, extra = total - share * (int)gridDim.x;
     const int at1 = share * ((int)blockIdx.x + 1) + min((int)blockIdx.x + 1, extra);
 
-    for (int at = share * (int)blockIdx.x + min((int)blockIdx.x, extra); at < at1; par ^= 1) {
+    for (int at = share * (int)blockIdx.x + min((int)blockIdx.x, extra); at < at1;) {
         const int gtile = at / span, in = at - gtile * span;
         const int rg_begin = max(in - A.skip, 0), rg_end = min(in + (at1 - at), span) - A.skip;
         at += span - in;
-        if (rg_end <= rg_begin) { par ^= 1; continue; }
+        if (rg_end <= rg_begin) continue;
         int lo = 0, hi = nseg;  // the segment: pre[lo] <= gtile < pre[lo + 1]
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -427,71 +586,23 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
         };
         for (int i = 1; i < A.nst; ++i) prefetch();
 
-        // ---- activations: largest element of each row, then the split into P columns ----
-        for (int gi = warp; gi < m * nb; gi += kMmWarps) {  // one 256-element block of one token per warp
-            const int tok = gi / nb, b = gi - tok * nb;
-            const uint32_t pr = row0 + tok;
-            const float* xr = A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256;
-            const float4 v0 = *reinterpret_cast<const float4*>(xr + 4 * lane), v1 = *reinterpret_cast<const float4*>(xr + 128 + 4 * lane);
-            uint32_t mx = max(max(__float_as_uint(fabsf(v0.x)), __float_as_uint(fabsf(v0.y))), max(__float_as_uint(fabsf(v0.z)), __float_as_uint(fabsf(v0.w))));
-            mx = max(mx, max(max(__float_as_uint(fabsf(v1.x)), __float_as_uint(fabsf(v1.y))), max(__float_as_uint(fabsf(v1.z)), __float_as_uint(fabsf(v1.w)))));
-            mx = __reduce_max_sync(0xffffffffu, mx);
-            if (lane == 0) atomicMax(&amax[par * 16 + tok], mx);  // a maximum: any order gives the same
-        }
-        __syncthreads();
+        // ---- activations: a 256-element block of a token per warp ----
         for (int gi = warp; gi < m * nb; gi += kMmWarps) {
             const int tok = gi / nb, b = gi - tok * nb;
             const uint32_t pr = row0 + tok;
-            const float* xr = A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256;
-            const float s = mm_row_scale(amax[par * 16 + tok]);
-            int e0, e1;
-            mm_unit_elems<T>(g, t, e0, e1);  // lane = 4 * unit + quarter
-            float4 v0 = *reinterpret_cast<const float4*>(xr + e0), v1 = *reinterpret_cast<const float4*>(xr + e1);
-            v0.x *= s; v0.y *= s; v0.z *= s; v0.w *= s;
-            v1.x *= s; v1.y *= s; v1.z *= s; v1.w *= s;
-            uint32_t h[4][P];
-            if constexpr (mq_mins<T>) {
-                mm_split<P>(v0.x, v0.z, h[0]);
-                mm_split<P>(v0.y, v0.w, h[1]);
-                mm_split<P>(v1.x, v1.z, h[2]);
-                mm_split<P>(v1.y, v1.w, h[3]);
-            } else {
-                mm_split<P>(v0.x, v0.y, h[0]);
-                mm_split<P>(v0.z, v0.w, h[1]);
-                mm_split<P>(v1.x, v1.y, h[2]);
-                mm_split<P>(v1.z, v1.w, h[3]);
-            }
-            uint8_t* col = acts + (size_t)tok * P * A.col_stride;
-#pragma unroll
-            for (int p = 0; p < P; ++p)
-                *reinterpret_cast<uint4*>(col + (size_t)p * A.col_stride + b * 512 + lane * 16) = make_uint4(h[0][p], h[1][p], h[2][p], h[3][p]);
-            if constexpr (mq_mins<T>) {  // sums of the lane's two sub-blocks, over the eight units
-                float a = (v0.x + v0.y) + (v0.z + v0.w), c = (v1.x + v1.y) + (v1.z + v1.w);
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    a += __shfl_xor_sync(0xffffffffu, a, o);
-                    c += __shfl_xor_sync(0xffffffffu, c, o);
-                }
-                uint32_t sp[P];
-                mm_split<P>(a, c, sp);
-                if (g == 0) {
-#pragma unroll
-                    for (int p = 0; p < P; ++p) *reinterpret_cast<uint32_t*>(col + (size_t)p * A.col_stride + A.n_in * 2 + b * 16 + t * 4) = sp[p];
-                }
-            }
+            mm_stage_block<T>(A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256, acts + (size_t)gi * kXBlock, lane);
         }
-        if (tid < 16) amax[(par ^ 1) * 16 + tid] = 0u;
         __syncthreads();
 
         // ---- the row groups ----
-        const int nt = (m + TPT - 1) / TPT;
-        const uint8_t* colb[NT];
+        const int nt = (m + kMmTok - 1) / kMmTok;
+        const uint8_t *colb[NT], *colv[NT];  // the token of this lane's B column, and of its accumulators
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            const int tok = min(n * TPT + (P == 3 ? g >> 2 : g >> 1), m - 1), part = P == 3 ? min(g & 3, 2) : g & 1;
-            colb[n] = acts + (size_t)(tok * P + part) * A.col_stride;
+            colb[n] = acts + (size_t)min(n * kMmTok + (g >> 2), m - 1) * nb * kXBlock;
+            colv[n] = acts + (size_t)min(n * kMmTok + (t >> 1), m - 1) * nb * kXBlock + kXInv + (t & 1) * 4;
         }
-        float acc[NT][4];
+        float acc[NT][2];
         int q_s = 0, q_b = 0, round = 0;
         uint32_t offa = 0, offb = 0;  // where a row's block starts (only the position inside 16 bytes matters)
         for (int q = 0; q < nstage; ++q) {
@@ -516,42 +627,43 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
             }
             if (q_b == 0) {
 #pragma unroll
-                for (int n = 0; n < NT; ++n)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[n][c] = 0.f;
+                for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = 0.f;
             }
             const uint8_t* bp[NT];
             uint32_t sumw[NT];
+            float inv[NT];
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                bp[n] = colb[n] + (kb0 + q_b) * 512 + t * 16;
-                sumw[n] = 0u;
+                const int at_b = (kb0 + q_b) * kXBlock;
+                bp[n] = colb[n] + at_b + (g & 3) * kXDigit + t * 8;
+                inv[n] = *reinterpret_cast<const float*>(colv[n] + at_b);
+                sumw[n] = 0u;  // the fourth column of a token takes no sums
                 if constexpr (mq_mins<T>) {
-                    if (n < nt) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + A.n_in * 2 + (kb0 + q_b) * 16 + t * 4);
+                    if (n < nt && (g & 3) < 3) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + at_b + kXSums + (g & 3) * 16 + t * 4);
                 }
             }
-            mm_block<T, NT>(ra, rb, t, gl, sl, bp, sumw, nt, acc);
+            mm_block<T, NT>(ra, rb, t, gl, sl, bp, sumw, inv, nt, acc);
             if (++q_s == A.nst) q_s = 0;
             if (++q_b == kbn) {
                 q_b = 0;
                 bool mine = true;
                 if (A.ks > 1) {  // the warps of the row group meet; the first adds the others' sums in order
-                    float* rp = red + ((size_t)(round & 1) * kMmWarps + warp) * NT * 4 * 32 + lane;
+                    float* rp = red + ((size_t)(round & 1) * kMmWarps + warp) * NT * 2 * 32 + lane;
                     mine = kpart == 0;
                     if (!mine) {
 #pragma unroll
                         for (int n = 0; n < NT; ++n)
 #pragma unroll
-                            for (int c = 0; c < 4; ++c) rp[(n * 4 + c) * 32] = acc[n][c];
+                            for (int c = 0; c < 2; ++c) rp[(n * 2 + c) * 32] = acc[n][c];
                     }
                     mm_barrier(1 + slot, A.ks * 32);
                     if (mine) {
                         for (int k2 = 1; k2 < A.ks; ++k2) {
-                            rp += NT * 4 * 32;
+                            rp += NT * 2 * 32;
 #pragma unroll
                             for (int n = 0; n < NT; ++n)
 #pragma unroll
-                                for (int c = 0; c < 4; ++c) acc[n][c] += rp[(n * 4 + c) * 32];
+                                for (int c = 0; c < 2; ++c) acc[n][c] += rp[(n * 2 + c) * 32];
                         }
                     }
                 }
@@ -559,31 +671,19 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
                         if (NT == 1 || n < nt) {
-                            float a, b;  // this row of both halves of the tile, one token
-                            int tok;
-                            if constexpr (P == 3) {
-                                a = (t & 1) ? acc[n][0] : acc[n][0] + acc[n][1];
-                                b = (t & 1) ? acc[n][2] : acc[n][2] + acc[n][3];
-                                a += __shfl_xor_sync(0xffffffffu, a, 1);
-                                b += __shfl_xor_sync(0xffffffffu, b, 1);
-                                tok = n * TPT + (t >> 1);
-                            } else {
-                                a = acc[n][0] + acc[n][1];
-                                b = acc[n][2] + acc[n][3];
-                                tok = n * TPT + t;
-                            }
+                            // the low two digits' sums and the high two's meet: both lanes have both rows of the token
+                            float a = acc[n][0], b = acc[n][1];
+                            a += __shfl_xor_sync(0xffffffffu, a, 1);
+                            b += __shfl_xor_sync(0xffffffffu, b, 1);
+                            const int tok = n * kMmTok + (t >> 1);
                             if (tok < m) {
-                                const float s = mm_row_scale(amax[par * 16 + tok]);
-                                const float inv = __uint_as_float((254u << 23) - __float_as_uint(s));  // 1 / 2^s: exponent 254 - e
-                                a *= inv;
-                                b *= inv;
                                 float* o = A.out + (size_t)(row0 + tok) * A.n_out;
                                 if constexpr (FUSED) {
-                                    if (P == 2 || !(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
+                                    if (!(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
                                 } else {
                                     const int r = rg * 16 + g;
-                                    if ((P == 2 || !(t & 1)) && r < A.n_out) o[r] = a;
-                                    if ((P == 2 || (t & 1)) && r + 8 < A.n_out) o[r + 8] = b;
+                                    if (!(t & 1) && r < A.n_out) o[r] = a;
+                                    if ((t & 1) && r + 8 < A.n_out) o[r + 8] = b;
                                 }
                             }
                         }
@@ -598,9 +698,9 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     }
 }
 
-template <int T, bool FUSED, int P, int NT>
+template <int T, bool FUSED, int NT>
 static int launch_mm_t(dnb_ctx* c, cudaStream_t st, MmArgs A, size_t smem, int grid, const char* name) {
-    auto kern = mm_kernel<T, FUSED, P, NT>;
+    auto kern = mm_kernel<T, FUSED, NT>;
     static SmemGrant grant;
     DNB_CUDA(grant_smem(grant, c->device, kern, smem));
     ProfScope prof_(c, st, name);
@@ -614,32 +714,23 @@ bool mm_handles(int type, int n_in) {
 }
 
 template <int T>
-static int mm_launch_type(dnb_ctx* c, cudaStream_t st, bool fused, int parts, int nt, MmArgs& A, size_t smem, int grid, const char* name) {
-#define DNB_MM(F, P, N) return launch_mm_t<T, F, P, N>(c, st, A, smem, grid, name)
-    if (parts == 2) {
-        if constexpr (T == T_Q4_K || T == T_IQ3_XXS) {
-            if (fused) { if (nt == 1) DNB_MM(true, 2, 1); DNB_MM(true, 2, 2); }
-            if (nt == 1) DNB_MM(false, 2, 1);
-            DNB_MM(false, 2, 2);
-        }
-        return DNB_DECLINED;
-    }
-    if (fused) { if (nt == 1) DNB_MM(true, 3, 1); if (nt == 2) DNB_MM(true, 3, 2); DNB_MM(true, 3, 4); }
-    if (nt == 1) DNB_MM(false, 3, 1);
-    if (nt == 2) DNB_MM(false, 3, 2);
-    DNB_MM(false, 3, 4);
+static int mm_launch_type(dnb_ctx* c, cudaStream_t st, bool fused, int nt, MmArgs& A, size_t smem, int grid, const char* name) {
+#define DNB_MM(F, N) return launch_mm_t<T, F, N>(c, st, A, smem, grid, name)
+    if (fused) { if (nt == 1) DNB_MM(true, 1); if (nt == 2) DNB_MM(true, 2); DNB_MM(true, 4); }
+    if (nt == 1) DNB_MM(false, 1);
+    if (nt == 2) DNB_MM(false, 2);
+    DNB_MM(false, 4);
 #undef DNB_MM
 }
 
 // batch: K is split as a constant of the shape.  rows: token rows of the launch in total; nseg_est: segments that will have rows (an estimate when the device counts them).
-int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
+int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name) {
     if (!mm_handles(type, n_in) || n_out < 1 || (fused && n_out % 8) || nseg_max < 1 || nseg_max > kMmSegMax || rows < 1) return DNB_DECLINED;
     if (!seg && !single) return DNB_ERR_ARG;
     if ((((uintptr_t)x) & 15) || ldx % 4 || (single && ((((uintptr_t)single->wa) & 15) || (fused && (((uintptr_t)single->wb) & 15))))) return DNB_DECLINED;
-    if (type != T_Q4_K && type != T_IQ3_XXS) parts = 3;
-    int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
+    int rc = type == T_IQ3_XXS ? upload_mm_s8(c->device) : DNB_OK;
     if (rc) return rc;
     const int bb = type == T_Q4_K ? 144 : type == T_Q5_K ? 176 : type == T_Q6_K ? 210 : type == T_Q8_0 ? 272 : 98;
     const int rs = type == T_Q4_K ? Mq<T_Q4_K>::RS : type == T_Q5_K ? Mq<T_Q5_K>::RS : type == T_Q6_K ? Mq<T_Q6_K>::RS
@@ -649,16 +740,13 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
     if (single) A.single = *single;
     A.n_in = n_in; A.n_out = n_out; A.rb = bb * (n_in / 256);
     A.x = x; A.ldx = ldx; A.row_token = row_token; A.out = out;
-    // columns 64 bytes apart modulo 128: the two columns a quarter-warp reads together fall on different banks
-    A.col_stride = n_in * 2 + (n_in / 16 + 127) / 128 * 128 + 64;
     // Column tiles: the fewest that hold an average segment (a wider instance costs registers and shared memory, a narrower
     // one decodes a segment's weights once more per tile).
-    const int tpt = parts == 3 ? 2 : 4, max_nt = parts == 3 ? 4 : 2;
+    constexpr int tpt = kMmTok, max_nt = 4;
     const float avg = (float)rows / (float)std::max(1, nseg_est);
     int nt = 1;
     while (nt < max_nt && avg > 0.75f * nt * tpt) nt *= 2;
     const int n_rg = fused ? n_out / 8 : (n_out + 15) / 16, nb = n_in / 256;
-    const size_t fixed = ((kMmSegMax + 4 + 16 + 32) * 4 + 127) / 128 * 128;
     int split = batch && nb >= 4 ? 2 : 1;  // of a batch
     for (;; nt /= 2) {
         const long tiles = std::max(nseg_est, (rows + nt * tpt - 1) / (nt * tpt));
@@ -673,9 +761,9 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
         if (!batch)
             while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
         A.ks = ks;
-        size_t base = fixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 4 * 32 * 4 : 0) + (size_t)nt * tpt * parts * A.col_stride;
+        size_t base = kMmFixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 2 * 32 * 4 : 0) + (size_t)nt * tpt * nb * kXBlock;
         if (type == T_IQ3_XXS)  // the tables behind the activations, on their boundary (dynamic shared memory starts at kMmSmemBase)
-            base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmCodebook);
+            base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmTables);
         const size_t stage = (size_t)kMmWarps * 16 * rs, cap = 225 * 1024;
         for (A.nst = 4; A.nst >= 2 && base + A.nst * stage > cap; --A.nst) {}
         if (A.nst >= 2) {
@@ -687,11 +775,11 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
             if ((double)(nseg_max + (rows + nt * tpt - 1) / (nt * tpt)) * (n_rg + A.skip) > 2e9) return DNB_DECLINED;
             const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, std::max<long>(1, tiles * n_rg * ks / kMmWarps));
             switch (type) {
-                case T_Q4_K: return mm_launch_type<T_Q4_K>(c, st, fused, parts, nt, A, smem, grid, name);
-                case T_Q5_K: return mm_launch_type<T_Q5_K>(c, st, fused, parts, nt, A, smem, grid, name);
-                case T_Q6_K: return mm_launch_type<T_Q6_K>(c, st, fused, parts, nt, A, smem, grid, name);
-                case T_Q8_0: return mm_launch_type<T_Q8_0>(c, st, fused, parts, nt, A, smem, grid, name);
-                default: return mm_launch_type<T_IQ3_XXS>(c, st, fused, parts, nt, A, smem, grid, name);
+                case T_Q4_K: return mm_launch_type<T_Q4_K>(c, st, fused, nt, A, smem, grid, name);
+                case T_Q5_K: return mm_launch_type<T_Q5_K>(c, st, fused, nt, A, smem, grid, name);
+                case T_Q6_K: return mm_launch_type<T_Q6_K>(c, st, fused, nt, A, smem, grid, name);
+                case T_Q8_0: return mm_launch_type<T_Q8_0>(c, st, fused, nt, A, smem, grid, name);
+                default: return mm_launch_type<T_IQ3_XXS>(c, st, fused, nt, A, smem, grid, name);
             }
         }
         if (nt > 1) continue;
@@ -708,10 +796,9 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, int parts, bool
 // work); a warp takes every ks-th block of K of 16 rows and asks for its first stages before it waits for the kernel in front of
 // it, whose output the vector may be; it converts its own blocks of the vector, each with a power of two of its own, so that no
 // CTA-wide step stands between vector and math; the warps' partial sums meet once per 16 rows, in a fixed order.
-// Measured back to back, us, register-decode GEMV before: 4096 x 4096 Q4_K 8.4 -> 5.7, IQ3_XXS 10.3 -> 6.4, Q8_0 8.9 -> 6.5; 65536 x
-// 4096 Q8_0 103 -> 71 (4.0 TB/s), Q4_K 84 -> 47, IQ3_XXS 99 -> 56; two vectors of IQ3_XXS 62034 x 5632 466 -> 94.
+// Measured back to back, us, with fp16 operands -> with bytes: 4096 x 4096 Q4_K 5.6 -> 4.7; 65536 x 4096 Q8_0 71.8 -> 64.1 (4.45 TB/s).  (The
+// register-decode GEMV before took 8.4 and 103.)
 constexpr int kGvWarps = 8;
-constexpr int kGvPart = 576;  // bytes of a part of a block: 512, its sub-block sums (16), and padding that spreads neighbouring parts over the banks
 
 struct GvArgs {
     const uint8_t* w;
@@ -726,20 +813,19 @@ struct GvArgs {
 template <int T, int TOK>
 __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const GvArgs A) {
     using Q = Mq<T>;
-    constexpr int STAGE = 16 * Q::RS, XB = TOK * 3 * kGvPart;  // bytes of a converted block
+    constexpr int STAGE = 16 * Q::RS, XB = TOK * kXBlock;  // bytes of a converted block
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int nb = A.k >> 8, nslot = kGvWarps / A.ks, slot = warp / A.ks, kw = warp - slot * A.ks;
     const int kbn = (nb - kw + A.ks - 1) / A.ks, kb_max = (nb + A.ks - 1) / A.ks;  // this warp's blocks: kw, kw + ks, ...
     float* red = reinterpret_cast<float*>(smem);                                   // [2][8 warps][16 rows][TOK]
-    float* inv = red + 2 * kGvWarps * 16 * TOK + warp * kb_max * TOK;              // [blocks][TOK] what undoes a block's scaling
-    uint8_t* p = smem + ((2 * kGvWarps * 16 * TOK + kGvWarps * kb_max * TOK) * 4 + 127) / 128 * 128;
+    uint8_t* p = smem + 2 * kGvWarps * 16 * TOK * 4;
     uint8_t* xs = p + (size_t)warp * kb_max * XB;
     p += (size_t)kGvWarps * kb_max * XB;
     uint8_t* book = p;
     if constexpr (T == T_IQ3_XXS) {
         book += (kMmBookAlign - (tcp::s32(p) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
-        p = book + sizeof(MmCodebook);
+        p = book + sizeof(MmTables);
     }
     if (T == T_IQ3_XXS && (uint32_t)(p - smem) + kGvWarps * A.nst * STAGE > A.smem) {  // only if shared memory started elsewhere
         if (tid == 0) status_set(A.status, 26);
@@ -794,8 +880,8 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
     };
     for (int i = 1; i < A.nst; ++i) prefetch();
     if constexpr (T == T_IQ3_XXS) {  // in the last of those groups' shadow: waited for with the first stage
-        for (int i = tid; i < (int)(sizeof(MmCodebook) / 16); i += kGvWarps * 32)
-            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_codebook) + 16 * i);
+        for (int i = tid; i < (int)(sizeof(MmTables) / 16); i += kGvWarps * 32)
+            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_s8) + 16 * i);
         tcp::cp_async_commit();
     }
     pdl_wait();
@@ -806,45 +892,7 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
     for (int i = 0; i < kbn; ++i) {
 #pragma unroll
         for (int q = 0; q < TOK; ++q) {
-            const float* xr = A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (kw + i * A.ks) * 256;
-            int e0, e1;
-            mm_unit_elems<T>(g, t, e0, e1);  // lane = 4 * unit + quarter
-            float4 xa = *reinterpret_cast<const float4*>(xr + e0), xb = *reinterpret_cast<const float4*>(xr + e1);
-            uint32_t mx = max(max(__float_as_uint(fabsf(xa.x)), __float_as_uint(fabsf(xa.y))), max(__float_as_uint(fabsf(xa.z)), __float_as_uint(fabsf(xa.w))));
-            mx = max(mx, max(max(__float_as_uint(fabsf(xb.x)), __float_as_uint(fabsf(xb.y))), max(__float_as_uint(fabsf(xb.z)), __float_as_uint(fabsf(xb.w)))));
-            const float s = mm_row_scale(__reduce_max_sync(0xffffffffu, mx));
-            if (lane == 0) inv[i * TOK + q] = __uint_as_float((254u << 23) - __float_as_uint(s));
-            xa.x *= s; xa.y *= s; xa.z *= s; xa.w *= s;
-            xb.x *= s; xb.y *= s; xb.z *= s; xb.w *= s;
-            uint32_t h[4][3];
-            if constexpr (mq_mins<T>) {
-                mm_split<3>(xa.x, xa.z, h[0]);
-                mm_split<3>(xa.y, xa.w, h[1]);
-                mm_split<3>(xb.x, xb.z, h[2]);
-                mm_split<3>(xb.y, xb.w, h[3]);
-            } else {
-                mm_split<3>(xa.x, xa.y, h[0]);
-                mm_split<3>(xa.z, xa.w, h[1]);
-                mm_split<3>(xb.x, xb.y, h[2]);
-                mm_split<3>(xb.z, xb.w, h[3]);
-            }
-            uint8_t* col = xs + i * XB + q * 3 * kGvPart;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) *reinterpret_cast<uint4*>(col + c * kGvPart + lane * 16) = make_uint4(h[0][c], h[1][c], h[2][c], h[3][c]);
-            if constexpr (mq_mins<T>) {
-                float a = (xa.x + xa.y) + (xa.z + xa.w), b = (xb.x + xb.y) + (xb.z + xb.w);
-#pragma unroll
-                for (int o = 4; o < 32; o <<= 1) {
-                    a += __shfl_xor_sync(0xffffffffu, a, o);
-                    b += __shfl_xor_sync(0xffffffffu, b, o);
-                }
-                uint32_t sp[3];
-                mm_split<3>(a, b, sp);
-                if (g == 0) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(col + c * kGvPart + 512 + t * 4) = sp[c];
-                }
-            }
+            mm_stage_block<T>(A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (kw + i * A.ks) * 256, xs + i * XB + q * kXBlock, lane);
         }
     }
     if constexpr (T == T_IQ3_XXS) {  // the tables came in parts from all threads
@@ -854,11 +902,11 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
     __syncwarp();
 
     // ---- the row groups ----
-    const uint32_t gl = tcp::s32(book) + 8 * (lane & (kLutRep - 1)), sl = tcp::s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
-    const uint8_t* colb = xs + ((TOK == 2 ? (g >> 2) : 0) * 3 + min(g & 3, 2)) * kGvPart;
+    const uint32_t gl = tcp::s32(book) + 4 * lane, sl = gl + (uint32_t)sizeof(uint32_t) * 256 * 32;
+    const uint8_t *colb = xs + (TOK == 2 ? g >> 2 : 0) * kXBlock, *colv = xs + (TOK == 2 ? t >> 1 : 0) * kXBlock + kXInv + (t & 1) * 4;
     int q_s = 0, rg = rg0;
     for (int rd = 0; rd < rounds; ++rd, rg += rg_step) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        float acc[1][2] = {{0.f, 0.f}};
         if (rd < nrg) {
             uint32_t offa = 0, offb = 0;
             if constexpr (!Q::ALIGNED) {
@@ -879,18 +927,15 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
                     offa += A.ks * Q::BB;
                     offb += A.ks * Q::BB;
                 }
-                const uint8_t* const bp[1] = {colb + i * XB + t * 16};
-                const uint32_t sumw[1] = {mq_mins<T> ? *reinterpret_cast<const uint32_t*>(colb + i * XB + 512 + t * 4) : 0u};
-                float c[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-                mm_block<T, 1>(ra, rb, t, gl, sl, bp, sumw, 1, c);
-                const float f = inv[i * TOK + (TOK == 2 ? t >> 1 : 0)];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[j] = fmaf(f, c[0][j], acc[j]);
+                const uint8_t* const bp[1] = {colb + i * XB + (g & 3) * kXDigit + t * 8};
+                const uint32_t sumw[1] = {mq_mins<T> && (g & 3) < 3 ? *reinterpret_cast<const uint32_t*>(colb + i * XB + kXSums + (g & 3) * 16 + t * 4) : 0u};
+                const float inv[1] = {*reinterpret_cast<const float*>(colv + i * XB)};
+                mm_block<T, 1>(ra, rb, t, gl, sl, bp, sumw, inv, 1, acc);
                 if (++q_s == A.nst) q_s = 0;
             }
         }
-        // columns 0-2 (lanes t = 0, 1) are the first vector's parts, 4-6 (t = 2, 3) the second's
-        float a = (t & 1) ? acc[0] : acc[0] + acc[1], b = (t & 1) ? acc[2] : acc[2] + acc[3];
+        // lanes t = 0, 1 hold the first vector's low and high digits, t = 2, 3 the second's
+        float a = acc[0][0], b = acc[0][1];
         a += __shfl_xor_sync(0xffffffffu, a, 1);
         b += __shfl_xor_sync(0xffffffffu, b, 1);
         float* rp = red + ((rd & 1) * kGvWarps + warp) * 16 * TOK;
@@ -914,8 +959,8 @@ static int launch_gv_t(dnb_ctx* c, cudaStream_t st, GvArgs A) {
     int ks = 1;
     while (ks < kGvWarps && ks * 2 <= nb) ks *= 2;
     const int kb_max = (nb + ks - 1) / ks;
-    size_t base = ((2 * kGvWarps * 16 * TOK + kGvWarps * kb_max * TOK) * 4 + 127) / 128 * 128 + (size_t)kGvWarps * kb_max * TOK * 3 * kGvPart;
-    if (T == T_IQ3_XXS) base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmCodebook);
+    size_t base = 2 * kGvWarps * 16 * TOK * 4 + (size_t)kGvWarps * kb_max * TOK * kXBlock;
+    if (T == T_IQ3_XXS) base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmTables);
     const size_t stage = (size_t)kGvWarps * 16 * rs, two = 113 * 1024, cap = 225 * 1024;  // two CTAs per SM where they fit
     A.ks = ks;
     for (A.nst = 4; A.nst > 2 && base + A.nst * stage > two; --A.nst) {}
@@ -939,7 +984,7 @@ static int launch_gv_t(dnb_ctx* c, cudaStream_t st, GvArgs A) {
 
 int launch_gemv_mma(dnb_ctx* c, cudaStream_t st, int type, const uint8_t* w, int k, int n, const float* x, float* out, int nvec) {
     if (!mm_handles(type, k) || n < 1 || nvec < 1 || (((uintptr_t)w) & 15) || (((uintptr_t)x) & 15)) return DNB_DECLINED;
-    const int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
+    const int rc = type == T_IQ3_XXS ? upload_mm_s8(c->device) : DNB_OK;
     if (rc) return rc;
     GvArgs A = {};
     A.w = w; A.x = x; A.out = out; A.k = k; A.n = n; A.nvec = nvec; A.rb = (int)row_bytes(type, k);

@@ -197,7 +197,7 @@ __device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint32
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             uint32_t p[4];
-            k_word<false>(w[i], 0u, s, p);
+            k_word(w[i], s, p);
 #pragma unroll
             for (int j = 0; j < 4; ++j) o[16 * h + 4 * i + j] = p[j];
         }

@@ -1,6 +1,6 @@
-// Packed quants into exact fp16 pairs, for the tensor-core kernels whose scales follow the sum (grouped_mma.cu on mma.sync,
-// grouped_tc.cu on tcgen05): Q4_K / Q5_K words as sc * q, IQ3_XXS codebook entries with their signs.  Each translation unit
-// that includes this header owns a copy of the IQ3_XXS tables and uploads it once per device.
+// Packed quants into exact fp16 pairs, for the tensor-core kernel whose scales follow the sum (grouped_tc.cu): Q4_K words as
+// sc * q, IQ3_XXS codebook entries with their signs.  Each translation unit that includes this header owns a copy of the
+// IQ3_XXS tables and uploads it once per device.
 #pragma once
 #include "dnb_common.cuh"
 #include "formats.cuh"
@@ -8,55 +8,13 @@
 
 namespace dnb {
 
-__device__ __forceinline__ uint32_t h2fma(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2sub(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t h2mul(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-// Q4_K / Q5_K: a lane's scales of one row of a block.  s0 / s1: the scale of its even / odd sub-block in both halves,
-// k0 / k1: -1024 * s0 and -64 * s1, mm: the pair of mins.
-struct KScales { float d, dmin; uint32_t s0, s1, k0, k1, mm; };
-__device__ __forceinline__ KScales k_scales(const uint8_t* row, int t) {
-    const uint4 h = *reinterpret_cast<const uint4*>(row);
-    const int sh = 16 * (t & 1);
-    const uint32_t a = h.y >> sh, b = h.z >> sh, c = h.w >> sh;
-    const bool low = t < 2;  // kquant.rs:878-887
-    const uint32_t sc = low ? (a & 0x3f3fu) : ((c & 0x0f0fu) | ((a >> 2) & 0x3030u));
-    const uint32_t mn = low ? (b & 0x3f3fu) : (((c >> 4) & 0x0f0fu) | ((b >> 2) & 0x3030u));
-    KScales r;
-    r.d = h2f((uint16_t)h.x);
-    r.dmin = h2f((uint16_t)(h.x >> 16));
-    r.s0 = h2sub(__byte_perm(sc, 0x64646464u, 0x4040u), 0x64006400u);
-    r.s1 = h2sub(__byte_perm(sc, 0x64646464u, 0x4141u), 0x64006400u);
-    r.k0 = h2mul(r.s0, 0xE400E400u);  // * -1024
-    r.k1 = h2mul(r.s1, 0xD400D400u);  // * -64
-    r.mm = h2sub(__byte_perm(mn, 0x64646464u, 0x4140u), 0x64006400u);
-    return r;
-}
-// Word i of a lane's 32 bytes: low nibbles are the even sub-block, high nibbles the odd one.  hq (Q5_K): the word of fifth
-// bits shifted so that bit 0 of a byte belongs to the low and bit 1 to the high nibble.
-template <bool FIVE>
-__device__ __forceinline__ void k_word(uint32_t w, uint32_t hq, const KScales& s, uint32_t (&p)[4]) {
+// Q4_K: the scales of two sub-blocks.  s0 / s1: of the even / odd one in both halves, k0 / k1: -1024 * s0 and -64 * s1.
+struct KScales { uint32_t s0, s1, k0, k1; };
+// A word of packed bytes: low nibbles are the even sub-block, high nibbles the odd one.
+__device__ __forceinline__ void k_word(uint32_t w, const KScales& s, uint32_t (&p)[4]) {
     const uint32_t w8 = w >> 8;
-    uint32_t a = (w & 0x000f000fu) | 0x64006400u, b = (w8 & 0x000f000fu) | 0x64006400u;    // 1024 + q
-    uint32_t c = (w & 0x00f000f0u) | 0x54005400u, d = (w8 & 0x00f000f0u) | 0x54005400u;    // 64 + q
-    if constexpr (FIVE) {
-        const uint32_t h8 = hq >> 8;
-        a |= (hq << 4) & 0x00100010u;
-        b |= (h8 << 4) & 0x00100010u;
-        c |= (hq << 7) & 0x01000100u;
-        d |= (h8 << 7) & 0x01000100u;
-    }
+    const uint32_t a = (w & 0x000f000fu) | 0x64006400u, b = (w8 & 0x000f000fu) | 0x64006400u;    // 1024 + q
+    const uint32_t c = (w & 0x00f000f0u) | 0x54005400u, d = (w8 & 0x00f000f0u) | 0x54005400u;    // 64 + q
     p[0] = h2fma(a, s.s0, s.k0);
     p[1] = h2fma(b, s.s0, s.k0);
     p[2] = h2fma(c, s.s1, s.k1);

@@ -179,3 +179,42 @@ def test_q4k_mins_of_any_size(orc, ctx, e, ff, nt):
     want = orc.moe_experts_given(L, orc.rmsnorm(h, np.ones(e, np.float32)), sels, wts)
     for rows in (slice(row, row + 2), slice(row + 2, e)):
         assert rel_err(out[:, rows], want[:, rows]) <= 2e-4
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("nvec", [1, 2, 5])
+def test_activations_of_any_size(orc, ctx, name, nvec):
+    """Activations are integers of their 256-element block: blocks from 1e-37 to 1e30, an element 2^20 times its neighbours, a block of
+    zeros, and blocks with an infinity or a NaN, whose vector alone feels it."""
+    ty, k, n = orc.TYPE_BY_NAME[name], 1024, 48
+    w = orc.synth_blocks(ty, SEED, 110 + ty, n * k // orc.blck_size(ty))
+    x = orc.synth_normal(SEED, 111, 1.0, 8 * nvec * k).reshape(8, nvec, k)
+    for i, f in enumerate((1e-37, 1e-30, 1.0, 1e30)):
+        x[i] *= np.float32(f)
+    x[3, :, 256:512] = 0.0
+    x[4, :, :256] *= np.float32(1e-20)
+    x[5, :, 300] *= np.float32(2.0 ** 20)
+    x[6, 0, 700] = np.inf
+    x[7, 0, 5] = np.nan
+    dw, dx, do = ctx.dev_alloc(w.nbytes), ctx.dev_alloc(x.nbytes), ctx.dev_alloc(8 * nvec * n * 4)
+    try:
+        ctx.upload(dw, w)
+        ctx.upload(dx, x)
+        for i in range(8):
+            assert ctx.gemv_dev(ty, dw, k, n, dx + 4 * i * nvec * k, do + 4 * i * nvec * n, nvec)
+        got = ctx.download(do, np.empty((8, nvec, n), np.float32))
+    finally:
+        for p in (dw, dx, do):
+            ctx.dev_free(p)
+    deq = orc.dequant_row(ty, w, n * k).reshape(n, k).astype(np.float64)
+    for i in range(8):
+        first = 1 if i > 5 else 0
+        if first:
+            assert not np.isfinite(got[i, 0]).any()
+            if nvec == 1:
+                continue
+        want = x[i, first:].astype(np.float64) @ deq.T
+        # 2^-30 of a block's largest element a term, and fp32 sums; 1e-37: an fp32 below 2^-126 keeps 2^-149
+        tiny = k * 2.0 ** -149 * np.abs(deq).max() if i == 0 else 0.0
+        bound = 2.0 ** -20 * np.sqrt((x[i, first:].astype(np.float64) ** 2) @ (deq ** 2).T) + 2.0 ** -28 * np.abs(x[i, first:]).max() * np.abs(deq).sum(1) + tiny
+        assert np.all(np.abs(got[i, first:] - want) <= bound), (i, np.max(np.abs(got[i, first:] - want) / bound))

@@ -1,17 +1,18 @@
 """The arithmetic identities the tensor-core kernels rest on, checked on the CPU against the oracle's block decode
 (no GPU, no product code): what must hold for the kernels' operand formats to be EXACT.
 
-* Q4_K with integer weights (csrc/grouped_tc.cu, csrc/grouped_mma.cu): w = d * sc * q - dmin * m (kquant.rs:505-526), so
+* Q4_K with integer weights (csrc/grouped_tc.cu): w = d * sc * q - dmin * m (kquant.rs:505-526), so
   W . x = sum_blocks d * [sum (sc * q) * x] - sum_subblocks (dmin * m) * X with X the sub-block sums of x;
   sc * q <= 945 is exact in fp16 and one fp16 fma (1024 + q) * sc - 1024 * sc produces it; -(dmin * m) times a power of
   two of the row is exact as fp16 hi + lo.
 * IQ3_XXS with exact weights: w = d / 4 * (grid magnitude) * sign * (2 s + 1), the product of the last three an integer exact
-  in fp16 (csrc/grouped_tc.cu); the magnitude alone exact in fp16 (csrc/grouped_mma.cu) and in bf16 (csrc/iq3_mma.cuh).
-* Activations of those kernels: a row times a power of two as two or three fp16 numbers (csrc/operand_rows.cuh,
-  csrc/grouped_mma.cu).
+  in fp16 (csrc/grouped_tc.cu); the magnitude alone exact in bf16 (csrc/iq3_mma.cuh) and a signed byte (csrc/grouped_mma.cu).
+* Activations of those kernels: a row times a power of two as two fp16 numbers (csrc/operand_rows.cuh), three for the
+  sub-block sums of csrc/grouped_mma.cu, whose activations are four digits in base 256 of a block; its integer sums fit.
 * Router operands (csrc/router_tc.cu): an fp32 value is the exact sum of three bf16 numbers (round, round, round).
 """
 import numpy as np
+import pytest
 
 SEED = 0xD3770B200
 
@@ -162,3 +163,37 @@ def test_three_bf16_parts_carry_an_fp32_exactly(orc):
     assert np.array_equal(r2.astype(np.float64), r1.astype(np.float64) - mid.astype(np.float64))
     lo = _bf16_rn(r2)
     assert np.array_equal(hi.astype(np.float64) + mid.astype(np.float64) + lo.astype(np.float64), x.astype(np.float64))
+
+
+def _digits(x):
+    """Four digits in base 256, -128 .. 127, of a block times the power of two that puts its largest element into [2^29, 2^30)."""
+    ex = int(np.max(np.abs(x)).view(np.uint32) >> 23)
+    v = np.rint(np.ldexp(x.astype(np.float64), 156 - ex)).astype(np.int64)
+    b = ((v + 0x00808080) ^ 0x00808080).astype(np.int32).view(np.uint32)
+    return np.stack([(b >> (8 * j)).astype(np.uint8).view(np.int8) for j in range(4)]).astype(np.int64), v, 156 - ex
+
+
+@pytest.mark.parametrize("spread", [0.0, 3.0])
+def test_activation_blocks_as_four_digits(orc, spread):
+    rng = np.random.RandomState(8)
+    for _ in range(50):
+        x = (rng.randn(256) * np.exp(spread * rng.randn(256))).astype(np.float32)
+        x[rng.randint(256)] *= -1.999
+        d, v, s = _digits(x)
+        assert d.min() >= -128 and d.max() <= 127
+        assert np.array_equal(sum(256 ** j * d[j] for j in range(4)), v)
+        assert np.max(np.abs(np.ldexp(v.astype(np.float64), -s) - x)) <= 2.0 ** -30 * np.max(np.abs(x))  # half a unit of 2^-29 of it
+
+
+def test_integer_block_sums_fit(orc):
+    """Largest sums of a 256-element block against a digit of 128: below 2^31, as the kernel's comments bound them; the byte forms of the
+    weights are the weights."""
+    n = 32 * 128
+    assert 8 * 16 * 63 * 15 * n < 2 ** 29 and 4 * 63 * (16 * 15 + 240) * n < 2 ** 29      # Q4_K: scales or nibbles 16 times as large
+    assert 8 * 63 * 31 * n < 2 ** 26 and 8 * 31 * 62 * n < 2 ** 26                         # Q5_K, IQ3_XXS
+    assert 16 * 128 * 16 * 128 * 128 < 2 ** 30 and 32 * 128 * 128 < 2 ** 22                # Q6_K; Q8_0 beside 1.5 * 2^23
+    q = np.arange(64, dtype=np.uint32)                                                     # Q6_K: the upper pair of bits inverted in its upper bit
+    byte = ((q & 15) << 2) | ((((q >> 4) ^ 2) & 3) << 6)
+    assert np.array_equal(byte.astype(np.uint8).view(np.int8).astype(int), 4 * (q.astype(int) - 32))
+    v = np.arange(4, 63, dtype=np.uint32)                                                  # IQ3_XXS: a negative byte is ~v + 1
+    assert np.array_equal(((v ^ 255) + 1).astype(np.uint8).view(np.int8).astype(int), -v.astype(int))
