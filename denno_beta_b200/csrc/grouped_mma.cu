@@ -25,10 +25,14 @@
 // group, each takes a part of K, and their sums are added in a fixed order.  A row's result depends on the row and on KS, not on
 // the tile, the column or the CTA; for decode batches KS is a constant of the shape, so that a token's bits do not depend on its batch.
 //
-// Measured, us per pass, fp16 operands in two or three parts -> bytes: six layers of 2048 x 512, top 10 of 512, one of Q4_K and five of
-// IQ3_XXS, 8 tokens 547 -> 491, 32 tokens 1185 -> 1112; two layers of Q4_K with Q6_K down, 77 tokens under a skewed router, 502 -> 404.  Distance
-// from the 64-bit result, five formats, normal and heavy-tailed inputs: 0.43 of what it was.
+// Measured, us of a launch, gate/up + down of 2048 x 512, top 10 of 512: fp16 operands in two or three parts -> bytes -> two blocks a stage and a
+// loop for each number of column tiles.  8 tokens: IQ3_XXS 49 + 31 -> 44 + 29 -> 41 + 27, Q4_K 44 + 28 -> 33 + 23 -> 32 + 21; 32 tokens: IQ3_XXS
+// 115 + 68 -> 108 + 66 -> 101 + 62, Q4_K 98 + 56 -> 75 + 45 -> 71 + 42, Q8_0 151 + 92 -> 134 + 74 -> 111 + 64; 200 tokens under a skewed router: Q4_K
+// and Q6_K 302 + 175 -> 263 + 119 -> 154 + 120, Q8_0 395 + 169 -> 249 + 135 -> 176 + 103.  (One loop with unused column tiles switched off took the
+// time of all of them, or not, as the compiler chose.)  Decoding alone is 30 (Q4_K) to 66 (IQ3_XXS) cycles of a scheduler for 16 rows x 32
+// elements; bytes from HBM take 50 and 34.  Distance from the 64-bit result, five formats, normal and heavy-tailed inputs: 0.43 of what it was.
 #include <algorithm>
+#include <type_traits>
 
 #include "dnb_common.cuh"
 #include "formats.cuh"
@@ -40,19 +44,18 @@ namespace dnb {
 constexpr int kMmWarps = 16;
 constexpr int kMmThreads = kMmWarps * 32;
 constexpr int kMmSegMax = 1088;  // segments of a launch at most
-constexpr int kMmFixed = ((kMmSegMax + 4 + 16) * 4 + 127) / 128 * 128;  // bytes of the segment table in shared memory
-constexpr uint32_t kMmBookAlign = 32768;  // IQ3_XXS tables
+constexpr int kMmFixed = ((kMmSegMax + 4 + 16) * 4 + 127) / 128 * 128;  // segment table in shared memory
 constexpr uint32_t kMmSmemBase = 1024;    // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
 constexpr int kMmTok = 2;        // tokens of a column tile: eight columns, four digits a token
 
-// 256 elements of a row: bytes, 16-byte units of a stage row (blocks that are not 16-byte sized start anywhere in their first
-// unit), and the stride of a stage row (chosen so that rows read together fall on different banks; Q5_K and Q8_0: as far as the ring's size allows).
+// 256 elements of a row: bytes, and the pitch of a stage's rows with one and with two of them (a multiple of 16; a format whose blocks are
+// not may start anywhere in its first 16 bytes).  The rows that are read together fall on different banks.
 template <int T> struct Mq;
-template <> struct Mq<T_Q4_K> { static constexpr int BB = 144, UNITS = 9, RS = 160; static constexpr bool ALIGNED = true; };
-template <> struct Mq<T_Q5_K> { static constexpr int BB = 176, UNITS = 11, RS = 176; static constexpr bool ALIGNED = true; };
-template <> struct Mq<T_Q6_K> { static constexpr int BB = 210, UNITS = 14, RS = 240; static constexpr bool ALIGNED = false; };
-template <> struct Mq<T_IQ3_XXS> { static constexpr int BB = 98, UNITS = 7, RS = 112; static constexpr bool ALIGNED = false; };
-template <> struct Mq<T_Q8_0> { static constexpr int BB = 272, UNITS = 17, RS = 272; static constexpr bool ALIGNED = true; };
+template <> struct Mq<T_Q4_K> { static constexpr int BB = 144, P1 = 160, P2 = 288; static constexpr bool ALIGNED = true; };
+template <> struct Mq<T_Q5_K> { static constexpr int BB = 176, P1 = 176, P2 = 352; static constexpr bool ALIGNED = true; };
+template <> struct Mq<T_Q6_K> { static constexpr int BB = 210, P1 = 240, P2 = 464; static constexpr bool ALIGNED = false; };
+template <> struct Mq<T_IQ3_XXS> { static constexpr int BB = 98, P1 = 112, P2 = 240; static constexpr bool ALIGNED = false; };
+template <> struct Mq<T_Q8_0> { static constexpr int BB = 272, P1 = 272, P2 = 544; static constexpr bool ALIGNED = true; };
 
 template <int T> constexpr bool mq_mins = (T == T_Q4_K || T == T_Q5_K);
 
@@ -67,6 +70,9 @@ __device__ __forceinline__ void mm_unit_elems(int u, int t, int& e0, int& e1) {
     if constexpr (T == T_Q6_K) {
         e0 = (u >> 2) * 128 + (u & 1) * 32 + ((u >> 1) & 1) * 16 + 4 * t;
         e1 = e0 + 64;
+    } else if constexpr (T == T_Q8_0) {
+        e0 = 32 * u + 4 * t;
+        e1 = e0 + 16;
     } else {
         e0 = 32 * u + 8 * t;
         e1 = e0 + 4;
@@ -187,11 +193,11 @@ __device__ __forceinline__ MmK mm_k_header(const uint8_t* row, int t) {
     return r;
 }
 
-// IQ3_XXS tables in shared memory, a copy per bank (a lane reads copy `lane`: no conflicts), 128 bytes from entry to entry:
-//   grid: the four magnitudes of a codebook entry, a byte each
-//   sgn : the signs of a 7-bit code (the eighth makes their number even): weight i at bit 8 i, weight 4 + i at bit 8 i + 1
-// The tables sit on a 32 KB boundary of the shared-memory address space: an entry's address is a shift and one and-or.
-struct MmTables { uint32_t grid[256 * 32]; uint32_t sgn[128 * 32]; };
+// IQ3_XXS tables in shared memory, 128 bytes from entry to entry, so that a lane's copies are on banks of its own:
+//   grid: the four magnitudes of a codebook entry, a byte each (lane i reads copy i)
+//   sgn : the signs of a 7-bit code (the eighth makes their number even) as 0 or 1 in a byte each: weights 0-3, 4-7 (copy i mod 16)
+// They are the first thing in shared memory, an address that the instructions hold.
+struct MmTables { uint32_t grid[256 * 32]; uint2 sgn[128 * 16]; };
 static __device__ __align__(16) MmTables g_mm_s8;
 static bool g_mm_s8_up[64] = {false};
 
@@ -203,74 +209,148 @@ static int upload_mm_s8(int device) {
         for (int r = 0; r < 32; ++r) tb.grid[e * 32 + r] = dnb_iq3xxs_grid[e];
     for (uint32_t code = 0; code < 128; ++code) {
         const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
-        uint32_t u = 0;
-        for (int i = 0; i < 4; ++i) u |= ((sg >> i) & 1u) << (8 * i) | ((sg >> (4 + i)) & 1u) << (8 * i + 1);
-        for (int r = 0; r < 32; ++r) tb.sgn[code * 32 + r] = u;
+        uint2 u = make_uint2(0u, 0u);
+        for (int i = 0; i < 4; ++i) {
+            u.x |= ((sg >> i) & 1u) << (8 * i);
+            u.y |= ((sg >> (4 + i)) & 1u) << (8 * i);
+        }
+        for (int r = 0; r < 16; ++r) tb.sgn[code * 16 + r] = u;
     }
     DNB_CUDA(cudaMemcpyToSymbol(g_mm_s8, &tb, sizeof(tb)));
     g_mm_s8_up[device] = true;
     return DNB_OK;
 }
 
-// Eight weights of an IQ3_XXS sub-block as signed bytes.  gl, sl: shared addresses of the lane's copies; idx: the two codebook indices; code:
+// Eight weights of an IQ3_XXS sub-block as signed bytes.  gl, sl: where the lane's copies are in an entry; idx: the two codebook indices; code:
 // the sub-block word rotated so that the quarter's 7-bit sign code starts at bit 7.  A negative byte is ~v + 1 (v >= 4: nothing carries).
 __device__ __forceinline__ void iq3_s8(uint32_t gl, uint32_t sl, uint32_t idx, uint32_t code, uint32_t& p0, uint32_t& p1) {
-    uint32_t u, g0, g1;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"((code & 0x3f80u) | sl));  // constant tables: plain asm, free to move
-    asm("ld.shared.u32 %0, [%1];" : "=r"(g0) : "r"(((idx << 7) & 0x7f80u) | gl));
-    asm("ld.shared.u32 %0, [%1];" : "=r"(g1) : "r"(((idx >> 1) & 0x7f80u) | gl));
-    const uint32_t o0 = u & 0x01010101u, o1 = (u >> 1) & 0x01010101u;
+    uint32_t o0, o1, g0, g1;  // constant tables: plain asm, free to move
+    asm("ld.shared.v2.u32 {%0, %1}, [%2 + %3];" : "=r"(o0), "=r"(o1) : "r"((code & 0x3f80u) | sl), "n"(kMmSmemBase + 256 * 32 * 4));
+    asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(g0) : "r"(((idx << 7) & 0x7f80u) | gl), "n"(kMmSmemBase));
+    asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(g1) : "r"(((idx >> 1) & 0x7f80u) | gl), "n"(kMmSmemBase));
     p0 = (g0 ^ (o0 * 255u)) + o0;
     p1 = (g1 ^ (o1 * 255u)) + o1;
 }
+// A CTA's copy of the tables; complete after the caller's barrier.
+__device__ __forceinline__ void mm_tables_in(uint8_t* dst, int tid, int threads) {
+    for (int i = tid; i < (int)(sizeof(MmTables) / 16); i += threads)
+        tcp::cp_async16<false>(dst + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_s8) + 16 * i);
+    tcp::cp_async_commit();
+}
+
+// ---- weights ---------------------------------------------------------------------------------------------------------------------
+// A warp's ring of stages: one or two blocks of each of 16 rows, in 16-byte copies: a lane copies unit lane % 8 (+ 8, 16, ..) of rows
+// lane / 8 + 0, 4, 8, 12.  Two blocks a stage halve what is spent on addresses and counters, and lift what copies alone reach from 4.6 to 5.7
+// TB/s.  What a copy costs is its cache lines: four lanes to a row, with half the addresses, are 10 % slower, and so is one copy of all rows' last
+// units where a block leaves one over (Q8_0 by 10 %).  (Bulk copies per row reach 5.6 TB/s, but each costs the warp a turn of a loop of a dozen
+// instructions, a request of sixteen rows as many as decoding a block.)
+struct MmRing { int nst, bps, pitch; };
+template <int T>
+struct MmStream {
+    using Q = Mq<T>;
+    uint8_t* mem;  // of this warp
+    int nst, bps, pitch;
+    uint32_t at;   // of this lane in a stage
+    int lane, in = 0, out = 0;  // slots that are filled and read next
+    const uint8_t *sa, *sb;       // rows lane / 8 and lane / 8 + 8
+    uint32_t o1, o3;              // from there to rows lane / 8 + 4 and + 12
+    __device__ __forceinline__ MmStream(uint8_t* m, const MmRing& r, int ln)
+        : mem(m), nst(r.nst), bps(r.bps), pitch(r.pitch), at((ln >> 3) * r.pitch + (ln & 7) * 16), lane(ln), sa(nullptr), sb(nullptr), o1(0), o3(0) {}
+    // the next requests are for rows r, r + 1, ... of w, or (pair) eight rows from r on of wa and of wb; no row beyond `last`
+    template <bool PAIR>
+    __device__ __forceinline__ void point(const uint8_t* wa, const uint8_t* wb, int r, int last, uint32_t rb) {
+        const int q = lane >> 3;
+        if constexpr (PAIR) {
+            const size_t off = (size_t)(r + q) * rb;
+            sa = wa + off;
+            sb = wb + off;
+            o1 = o3 = 4u * rb;
+        } else {
+            const int r0 = min(r + q, last), r2 = min(r + q + 8, last);
+            sa = wa + (size_t)r0 * rb;
+            sb = wa + (size_t)r2 * rb;
+            o1 = (uint32_t)(min(r + q + 4, last) - r0) * rb;
+            o3 = (uint32_t)(min(r + q + 12, last) - r2) * rb;
+        }
+    }
+    __device__ __forceinline__ void request(int n) {  // n blocks of them; an empty request keeps the count of groups
+        if (n > 0) {
+            const int c16 = (lane & 7) * 16;
+            uint8_t* dst = mem + in * 16 * pitch + at;
+#pragma unroll
+            for (int j = 0; j < 4; ++j, dst += 4 * pitch) {
+                const uint8_t* src = (j < 2 ? sa : sb) + (j == 1 ? o1 : j == 3 ? o3 : 0u);
+                int bytes = n * Q::BB;
+                if constexpr (!Q::ALIGNED) {
+                    bytes += (int)((uintptr_t)src & 15);
+                    src = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
+                }
+#pragma unroll
+                for (int cc = 0; cc < 2 * Q::BB + (Q::ALIGNED ? 0 : 14); cc += 128)
+                    if (cc + 128 <= Q::BB || cc + c16 < bytes) tcp::cp_async16(dst + cc, src + c16 + cc);
+            }
+            sa += n * Q::BB;
+            sb += n * Q::BB;
+            if (++in == nst) in = 0;
+        }
+        tcp::cp_async_commit();
+    }
+    __device__ __forceinline__ void skip(int bytes) {  // between requests
+        sa += bytes;
+        sb += bytes;
+    }
+    __device__ __forceinline__ const uint8_t* wait() {  // rows 0-15 of the next stage; every lane has left the one before
+        if (nst == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        else if (nst == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 2;" ::: "memory");
+        __syncwarp();
+        return mem + out * 16 * pitch;
+    }
+    __device__ __forceinline__ void next() {
+        if (++out == nst) out = 0;
+    }
+};
 
 // One 256-element block of 16 rows (this lane: rows `ra` and `rb`) against NT column tiles; bp[i]: the lane's B column of tile
-// i at this block; inv, sumw: of the token whose columns the lane's accumulators hold, and of its B column; nt: tiles in use.
+// i at this block; inv, sumw: of the token whose columns the lane's accumulators hold, and of its B column.
 // acc[i] += scales * sums: rows `ra` and `rb`, digits 0 and 1 of a token (t even) or 2 and 3 (t odd).
 template <int T, int NT>
 __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, uint32_t gl, uint32_t sl, const uint8_t* const (&bp)[NT],
-                                         const uint32_t (&sumw)[NT], const float (&inv)[NT], int nt, float (&acc)[NT][2]) {
+                                         const uint32_t (&sumw)[NT], const float (&inv)[NT], float (&acc)[NT][2]) {
     if constexpr (T == T_Q8_0) {
         float s[NT][2];
 #pragma unroll
         for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = 0.f;
 #pragma unroll
         for (int ib = 0; ib < 8; ++ib) {
-            // the bytes start 2 or 4 bytes behind an aligned word
+            // the bytes start 2 or 4 bytes behind an aligned word; a lane takes words t and t + 4 of them
             uint32_t p[2], q[2];
-            const uint8_t *a = ra + 34 * ib + 8 * t, *b = rb + 34 * ib + 8 * t;
-            if (ib & 1) {
-                p[0] = *reinterpret_cast<const uint32_t*>(a + 2);
-                p[1] = *reinterpret_cast<const uint32_t*>(a + 6);
-                q[0] = *reinterpret_cast<const uint32_t*>(b + 2);
-                q[1] = *reinterpret_cast<const uint32_t*>(b + 6);
-            } else {
-                const uint32_t a0 = *reinterpret_cast<const uint32_t*>(a), a1 = *reinterpret_cast<const uint32_t*>(a + 4), a2 = *reinterpret_cast<const uint32_t*>(a + 8);
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(b), b1 = *reinterpret_cast<const uint32_t*>(b + 4), b2 = *reinterpret_cast<const uint32_t*>(b + 8);
-                p[0] = __byte_perm(a0, a1, 0x5432);
-                p[1] = __byte_perm(a1, a2, 0x5432);
-                q[0] = __byte_perm(b0, b1, 0x5432);
-                q[1] = __byte_perm(b1, b2, 0x5432);
+            const uint8_t *a = ra + 34 * ib + 4 * t, *b = rb + 34 * ib + 4 * t;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (ib & 1) {
+                    p[h] = *reinterpret_cast<const uint32_t*>(a + 2 + 16 * h);
+                    q[h] = *reinterpret_cast<const uint32_t*>(b + 2 + 16 * h);
+                } else {
+                    p[h] = __byte_perm(*reinterpret_cast<const uint32_t*>(a + 16 * h), *reinterpret_cast<const uint32_t*>(a + 16 * h + 4), 0x5432);
+                    q[h] = __byte_perm(*reinterpret_cast<const uint32_t*>(b + 16 * h), *reinterpret_cast<const uint32_t*>(b + 16 * h + 4), 0x5432);
+                }
             }
             const float fa = h2f(ld16(ra + 34 * ib)), fb = h2f(ld16(rb + 34 * ib));
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                if (NT == 1 || n < nt) {
-                    // sums start at the bits of 1.5 * 2^23, so that they are floats as they stand (|sum| <= 2^19)
-                    int D[4];
-                    mma_s8<0x4B400000>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
-                    const float m = 12582912.f;
-                    s[n][0] = fmaf(fa, fmaf(256.f, __int_as_float(D[1]) - m, __int_as_float(D[0]) - m), s[n][0]);
-                    s[n][1] = fmaf(fb, fmaf(256.f, __int_as_float(D[3]) - m, __int_as_float(D[2]) - m), s[n][1]);
-                }
+                // sums start at the bits of 1.5 * 2^23, so that they are floats as they stand (|sum| <= 2^19)
+                int D[4];
+                mma_s8<0x4B400000>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
+                const float m = 12582912.f;
+                s[n][0] = fmaf(fa, fmaf(256.f, __int_as_float(D[1]) - m, __int_as_float(D[0]) - m), s[n][0]);
+                s[n][1] = fmaf(fb, fmaf(256.f, __int_as_float(D[3]) - m, __int_as_float(D[2]) - m), s[n][1]);
             }
         }
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            if (NT == 1 || n < nt) {
-                acc[n][0] = fmaf(s[n][0], inv[n], acc[n][0]);
-                acc[n][1] = fmaf(s[n][1], inv[n], acc[n][1]);
-            }
+            acc[n][0] = fmaf(s[n][0], inv[n], acc[n][0]);
+            acc[n][1] = fmaf(s[n][1], inv[n], acc[n][1]);
         }
     } else {
         int c[NT][4];
@@ -326,11 +406,9 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
                     for (int n = 0; n < NT; ++n) {
-                        if (NT == 1 || n < nt) {
-                            int D[4];
-                            mma_u8(D, a[h][0], b[h][0], a[h][1], b[h][1], *reinterpret_cast<const uint2*>(bp[n] + (2 * j + h) * 32));
-                            add(n, D, fa[h], fb[h]);
-                        }
+                        int D[4];
+                        mma_u8(D, a[h][0], b[h][0], a[h][1], b[h][1], *reinterpret_cast<const uint2*>(bp[n] + (2 * j + h) * 32));
+                        add(n, D, fa[h], fb[h]);
                     }
             }
             if constexpr (!FIVE) {
@@ -362,11 +440,9 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                 const int fa = (int)(2u * (xa >> 28) + 1u), fb = (int)(2u * (xb >> 28) + 1u);
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    if (NT == 1 || n < nt) {
-                        int D[4];
-                        mma_s8<0>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
-                        add(n, D, fa, fb);
-                    }
+                    int D[4];
+                    mma_s8<0>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
+                    add(n, D, fa, fb);
                 }
             }
         } else {  // Q6_K: a K step is one 16-element group of one scale; bytes are 4 * (q - 32), sums 16 * 128 * 16 * 128 * 128 < 2^30
@@ -383,7 +459,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                     uint2 y[NT];
 #pragma unroll
                     for (int n = 0; n < NT; ++n)
-                        if (NT == 1 || n < nt) y[n] = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 32);
+                        y[n] = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 32);
 #pragma unroll
                     for (int hi = 0; hi < 2; ++hi) {
                         const int sh = 6 - 2 * w - 4 * hi;  // the pair of bits to the top of its byte
@@ -393,11 +469,9 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                         const int fa = *reinterpret_cast<const int8_t*>(ra + sc), fb = *reinterpret_cast<const int8_t*>(rb + sc);
 #pragma unroll
                         for (int n = 0; n < NT; ++n) {
-                            if (NT == 1 || n < nt) {
-                                int D[4];
-                                mma_s8_k16(D, va, vb, hi ? y[n].y : y[n].x);
-                                add(n, D, fa, fb);
-                            }
+                            int D[4];
+                            mma_s8_k16(D, va, vb, hi ? y[n].y : y[n].x);
+                            add(n, D, fa, fb);
                         }
                     }
                 }
@@ -405,18 +479,16 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
         }
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-            if (NT == 1 || n < nt) {
-                float va = da * fmaf(256.f, (float)c[n][1], (float)c[n][0]), vb = db * fmaf(256.f, (float)c[n][3], (float)c[n][2]);
-                if constexpr (mq_mins<T>) {
-                    float M[4];
-                    mma_f16_z(M, mma, mmb, 0u, 0u, sumw[n], 0u);
-                    const float k = (t & 1) ? 16.f : 0x1p20f;  // columns 0, 1 of a token stand beside its low digits, column 2 beside the high ones
-                    va = fmaf(-dma, (M[0] + M[1]) * k, va);
-                    vb = fmaf(-dmb, (M[2] + M[3]) * k, vb);
-                }
-                acc[n][0] = fmaf(va, inv[n], acc[n][0]);
-                acc[n][1] = fmaf(vb, inv[n], acc[n][1]);
+            float va = da * fmaf(256.f, (float)c[n][1], (float)c[n][0]), vb = db * fmaf(256.f, (float)c[n][3], (float)c[n][2]);
+            if constexpr (mq_mins<T>) {
+                float M[4];
+                mma_f16_z(M, mma, mmb, 0u, 0u, sumw[n], 0u);
+                const float k = (t & 1) ? 16.f : 0x1p20f;  // columns 0, 1 of a token stand beside its low digits, column 2 beside the high ones
+                va = fmaf(-dma, (M[0] + M[1]) * k, va);
+                vb = fmaf(-dmb, (M[2] + M[3]) * k, vb);
             }
+            acc[n][0] = fmaf(va, inv[n], acc[n][0]);
+            acc[n][1] = fmaf(vb, inv[n], acc[n][1]);
         }
     }
 }
@@ -431,9 +503,9 @@ struct MmArgs {
     int ldx;
     const int32_t* row_token;  // packed row -> x row, or null
     float* out;                // [packed row][n_out]
-    int ks, nst;               // warps that split K, stages of a warp's ring
+    int ks;                    // warps that split K
+    MmRing ring;
     int skip;                  // row groups' time that a tile's activations take
-    uint32_t smem;             // bytes of dynamic shared memory
     int* status;
 };
 
@@ -443,33 +515,25 @@ template <int T, bool FUSED, int NT>
 __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     using Q = Mq<T>;
     constexpr int TT = NT * kMmTok;  // tokens of an item
-    constexpr int STAGE = 16 * Q::RS;
     extern __shared__ __align__(128) uint8_t smem[];
-    int* pre = reinterpret_cast<int*>(smem);                            // [kMmSegMax + 1] first token tile of a segment
+    uint8_t* p0 = smem + (T == T_IQ3_XXS ? sizeof(MmTables) : 0);
+    int* pre = reinterpret_cast<int*>(p0);                              // [kMmSegMax + 1] first token tile of a segment
     int* wsum = pre + kMmSegMax + 4;                                    // [16]
-    uint8_t* p0 = smem + kMmFixed;
+    p0 += kMmFixed;
     float* red = reinterpret_cast<float*>(p0);                          // [2][16 warps][NT * 2][32] when ks > 1
     if (A.ks > 1) p0 += 2 * kMmWarps * NT * 2 * 32 * sizeof(float);
     const int nb = A.n_in >> 8;
     uint8_t* acts = p0;                                                 // [TT tokens][nb blocks][kXBlock]
     p0 += (size_t)TT * nb * kXBlock;
-    uint8_t* book = p0;
-    if constexpr (T == T_IQ3_XXS) {
-        book += (kMmBookAlign - (tcp::s32(p0) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
-        p0 = book + sizeof(MmTables);
-    }
-    uint8_t* ring = p0;
-    if (T == T_IQ3_XXS && (uint32_t)(ring - smem) + kMmWarps * A.nst * STAGE > A.smem) {  // only if shared memory started elsewhere
+    if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
     }
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    ring += (size_t)warp * A.nst * STAGE;
+    MmStream<T> W(p0 + (size_t)warp * A.ring.nst * 16 * A.ring.pitch, A.ring, lane);
     if constexpr (T == T_IQ3_XXS) {
-        for (int i = tid; i < (int)(sizeof(MmTables) / 16); i += kMmThreads)
-            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_s8) + 16 * i);
-        tcp::cp_async_commit();
+        mm_tables_in(smem, tid, kMmThreads);
         tcp::cp_async_wait_all();
     }
     pdl_wait();
@@ -507,7 +571,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
     const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
     const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
-    const uint32_t gl = tcp::s32(book) + 4 * lane, sl = gl + (uint32_t)sizeof(uint32_t) * 256 * 32;
+    const uint32_t gl = 4 * lane, sl = 8 * (lane & 15);
     // This CTA's share of all (tile, row group) pairs: a range of pairs in a row.  Another tile means another set of activations,
     // which takes as long as A.skip row groups: each tile is that much longer, and a CTA that has two gets so much less of them.
     const int span = n_rg + A.skip, total = pre[nseg] * span;
@@ -530,61 +594,27 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
         const uint32_t row0 = sd.row0 + tile * TT;
         int rg = rg_begin + slot;
         const int nrg = rg < rg_end ? (rg_end - rg + nslot - 1) / nslot : 0;
-        const int nstage = nrg * kbn;
 
-        // ---- the warp's weight stream: the next block of the next row group goes to ring slot pf_s ----
-        // A lane copies unit `lane & 7` (+ 8, 16) of rows lane / 8 + 4 j; a format with one unit over has 16 lanes copy that one.
-        int pf_rg = rg, pf_b = 0, pf_s = 0, pf_n = 0;
-        const int r_in = lane >> 3, c16 = (lane & 7) * 16;
-        constexpr bool TAIL = Q::ALIGNED && Q::UNITS % 8 == 1;
-        const uint8_t *sa = nullptr, *sb = nullptr, *stl = nullptr;
-        uint32_t o1 = 4u * A.rb, o2 = 0, o3 = 0;
-        auto point = [&]() {  // row group pf_rg, first block
-            const uint32_t boff = (uint32_t)kb0 * Q::BB;
-            if constexpr (FUSED) {
-                const size_t off = (size_t)(pf_rg * 8 + r_in) * A.rb + boff;
-                sa = sd.wa + off;
-                sb = sd.wb + off;
-                if constexpr (TAIL) stl = (lane < 8 ? sd.wa : sd.wb) + (size_t)(pf_rg * 8 + (lane & 7)) * A.rb + boff + (Q::UNITS - 1) * 16;
-            } else {
-                const int row = pf_rg * 16 + r_in, last = A.n_out - 1;
-                const int r0 = min(row, last);
-                sa = sd.wa + (size_t)r0 * A.rb + boff;
-                o1 = (uint32_t)(min(row + 4, last) - r0) * A.rb;
-                o2 = (uint32_t)(min(row + 8, last) - r0) * A.rb;
-                o3 = (uint32_t)(min(row + 12, last) - r0) * A.rb;
-                if constexpr (TAIL) stl = sd.wa + (size_t)min(pf_rg * 16 + (lane & 15), last) * A.rb + boff + (Q::UNITS - 1) * 16;
-            }
-        };
-        if (nstage > 0) point();
+        // ---- the warp's weight stream: the next blocks of the next row group ----
+        int pf_rg = rg, pf_b = 0;
+        const int rg_stop = rg + nrg * nslot;
         auto prefetch = [&]() {
-            if (pf_n < nstage) {
-                uint8_t* dst = ring + pf_s * STAGE + r_in * Q::RS + c16;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint8_t* src = FUSED ? (j >= 2 ? sb : sa) + ((j & 1) ? o1 : 0u) : sa + (j == 0 ? 0u : j == 1 ? o1 : j == 2 ? o2 : o3);
-                    if constexpr (!Q::ALIGNED) src = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
-#pragma unroll
-                    for (int cc = 0; cc < (TAIL ? Q::UNITS - 1 : Q::UNITS); cc += 8)
-                        if (cc + 8 <= Q::UNITS || cc * 16 + c16 < Q::UNITS * 16) tcp::cp_async16(dst + j * 4 * Q::RS + cc * 16, src + cc * 16 + c16);
+            int n = 0;
+            if (pf_rg < rg_stop) {
+                if (pf_b == 0) {
+                    const uint32_t boff = (uint32_t)kb0 * Q::BB;
+                    W.template point<FUSED>(sd.wa + boff, FUSED ? sd.wb + boff : nullptr, pf_rg * (FUSED ? 8 : 16), A.n_out - 1, (uint32_t)A.rb);
                 }
-                if constexpr (TAIL) {
-                    if (lane < 16) tcp::cp_async16(ring + pf_s * STAGE + lane * Q::RS + (Q::UNITS - 1) * 16, stl);
-                    stl += Q::BB;
-                }
-                ++pf_n;
-                sa += Q::BB;
-                if constexpr (FUSED) sb += Q::BB;
-                if (++pf_b == kbn) {
+                n = min(W.bps, kbn - pf_b);
+                pf_b += n;
+                if (pf_b == kbn) {
                     pf_b = 0;
                     pf_rg += nslot;
-                    if (pf_n < nstage) point();
                 }
-                if (++pf_s == A.nst) pf_s = 0;
             }
-            tcp::cp_async_commit();
+            W.request(n);
         };
-        for (int i = 1; i < A.nst; ++i) prefetch();
+        for (int i = 1; i < W.nst; ++i) prefetch();
 
         // ---- activations: a 256-element block of a token per warp ----
         for (int gi = warp; gi < m * nb; gi += kMmWarps) {
@@ -595,73 +625,68 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
         __syncthreads();
 
         // ---- the row groups ----
-        const int nt = (m + kMmTok - 1) / kMmTok;
-        const uint8_t *colb[NT], *colv[NT];  // the token of this lane's B column, and of its accumulators
+        auto row_groups = [&](auto tiles) {  // N column tiles: one, two or four, those behind the last token repeat it
+            constexpr int N = decltype(tiles)::value;
+            const uint8_t *colb[N], *colv[N];  // the token of this lane's B column, and of its accumulators
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            colb[n] = acts + (size_t)min(n * kMmTok + (g >> 2), m - 1) * nb * kXBlock;
-            colv[n] = acts + (size_t)min(n * kMmTok + (t >> 1), m - 1) * nb * kXBlock + kXInv + (t & 1) * 4;
-        }
-        float acc[NT][2];
-        int q_s = 0, q_b = 0, round = 0;
-        uint32_t offa = 0, offb = 0;  // where a row's block starts (only the position inside 16 bytes matters)
-        for (int q = 0; q < nstage; ++q) {
-            if (A.nst == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
-            else if (A.nst == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-            else asm volatile("cp.async.wait_group 2;" ::: "memory");
-            __syncwarp();  // the stage is complete for every lane, and every lane has left the slot that is filled next
-            prefetch();
-            const uint8_t* st = ring + q_s * STAGE;
-            const uint8_t* ra = st + g * Q::RS;
-            const uint8_t* rb = st + (g + 8) * Q::RS;
-            if constexpr (!Q::ALIGNED) {
-                if (q_b == 0) {
+            for (int n = 0; n < N; ++n) {
+                colb[n] = acts + (size_t)min(n * kMmTok + (g >> 2), m - 1) * nb * kXBlock;
+                colv[n] = acts + (size_t)min(n * kMmTok + (t >> 1), m - 1) * nb * kXBlock + kXInv + (t & 1) * 4;
+            }
+            float acc[N][2];
+            for (int round = 0; round < nrg; ++round, rg += nslot) {
+                // where a row's blocks start (only the position inside 16 bytes matters)
+                uint32_t offa = 0, offb = 0;
+                if constexpr (!Q::ALIGNED) {
                     const uint32_t r0 = FUSED ? rg * 8 + g : min(rg * 16 + g, A.n_out - 1), r1 = FUSED ? r0 : (uint32_t)min(rg * 16 + 8 + g, A.n_out - 1);
                     offa = r0 * (uint32_t)A.rb + (uint32_t)kb0 * Q::BB;
                     offb = r1 * (uint32_t)A.rb + (uint32_t)kb0 * Q::BB;
                 }
-                ra += offa & 15u;
-                rb += offb & 15u;
-                offa += Q::BB;
-                offb += Q::BB;
-            }
-            if (q_b == 0) {
 #pragma unroll
-                for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = 0.f;
-            }
-            const uint8_t* bp[NT];
-            uint32_t sumw[NT];
-            float inv[NT];
+                for (int n = 0; n < N; ++n) acc[n][0] = acc[n][1] = 0.f;
+#pragma unroll 1
+                for (int b = 0; b < kbn;) {
+                    const uint8_t* st = W.wait();  // and every lane has left the slot that is filled next
+                    prefetch();
+                    const uint8_t *ra = st + g * W.pitch + (Q::ALIGNED ? 0u : offa & 15u), *rb = st + (g + 8) * W.pitch + (Q::ALIGNED ? 0u : offb & 15u);
+                    const int stop = min(b + W.bps, kbn);
+                    offa += (stop - b) * Q::BB;
+                    offb += (stop - b) * Q::BB;
+#pragma unroll 1
+                    for (; b < stop; ++b, ra += Q::BB, rb += Q::BB) {
+                        const uint8_t* bp[N];
+                        uint32_t sumw[N];
+                        float inv[N];
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                const int at_b = (kb0 + q_b) * kXBlock;
-                bp[n] = colb[n] + at_b + (g & 3) * kXDigit + t * 8;
-                inv[n] = *reinterpret_cast<const float*>(colv[n] + at_b);
-                sumw[n] = 0u;  // the fourth column of a token takes no sums
-                if constexpr (mq_mins<T>) {
-                    if (n < nt && (g & 3) < 3) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + at_b + kXSums + (g & 3) * 16 + t * 4);
+                        for (int n = 0; n < N; ++n) {
+                            const int at_b = (kb0 + b) * kXBlock;
+                            bp[n] = colb[n] + at_b + (g & 3) * kXDigit + t * 8;
+                            inv[n] = *reinterpret_cast<const float*>(colv[n] + at_b);
+                            sumw[n] = 0u;  // the fourth column of a token takes no sums
+                            if constexpr (mq_mins<T>) {
+                                if ((g & 3) < 3) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + at_b + kXSums + (g & 3) * 16 + t * 4);
+                            }
+                        }
+                        mm_block<T, N>(ra, rb, t, gl, sl, bp, sumw, inv, acc);
+                    }
+                    W.next();
                 }
-            }
-            mm_block<T, NT>(ra, rb, t, gl, sl, bp, sumw, inv, nt, acc);
-            if (++q_s == A.nst) q_s = 0;
-            if (++q_b == kbn) {
-                q_b = 0;
                 bool mine = true;
                 if (A.ks > 1) {  // the warps of the row group meet; the first adds the others' sums in order
-                    float* rp = red + ((size_t)(round & 1) * kMmWarps + warp) * NT * 2 * 32 + lane;
+                    float* rp = red + ((size_t)(round & 1) * kMmWarps + warp) * N * 2 * 32 + lane;
                     mine = kpart == 0;
                     if (!mine) {
 #pragma unroll
-                        for (int n = 0; n < NT; ++n)
+                        for (int n = 0; n < N; ++n)
 #pragma unroll
                             for (int c = 0; c < 2; ++c) rp[(n * 2 + c) * 32] = acc[n][c];
                     }
                     mm_barrier(1 + slot, A.ks * 32);
                     if (mine) {
                         for (int k2 = 1; k2 < A.ks; ++k2) {
-                            rp += NT * 2 * 32;
+                            rp += N * 2 * 32;
 #pragma unroll
-                            for (int n = 0; n < NT; ++n)
+                            for (int n = 0; n < N; ++n)
 #pragma unroll
                                 for (int c = 0; c < 2; ++c) acc[n][c] += rp[(n * 2 + c) * 32];
                         }
@@ -669,33 +694,32 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
                 }
                 if (mine) {
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) {
-                        if (NT == 1 || n < nt) {
-                            // the low two digits' sums and the high two's meet: both lanes have both rows of the token
-                            float a = acc[n][0], b = acc[n][1];
-                            a += __shfl_xor_sync(0xffffffffu, a, 1);
-                            b += __shfl_xor_sync(0xffffffffu, b, 1);
-                            const int tok = n * kMmTok + (t >> 1);
-                            if (tok < m) {
-                                float* o = A.out + (size_t)(row0 + tok) * A.n_out;
-                                if constexpr (FUSED) {
-                                    if (!(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
-                                } else {
-                                    const int r = rg * 16 + g;
-                                    if (!(t & 1) && r < A.n_out) o[r] = a;
-                                    if ((t & 1) && r + 8 < A.n_out) o[r + 8] = b;
-                                }
+                    for (int n = 0; n < N; ++n) {
+                        // the low two digits' sums and the high two's meet: both lanes have both rows of the token
+                        float a = acc[n][0], b = acc[n][1];
+                        a += __shfl_xor_sync(0xffffffffu, a, 1);
+                        b += __shfl_xor_sync(0xffffffffu, b, 1);
+                        const int tok = n * kMmTok + (t >> 1);
+                        if (tok < m) {
+                            float* o = A.out + (size_t)(row0 + tok) * A.n_out;
+                            if constexpr (FUSED) {
+                                if (!(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
+                            } else {
+                                const int r = rg * 16 + g;
+                                if (!(t & 1) && r < A.n_out) o[r] = a;
+                                if ((t & 1) && r + 8 < A.n_out) o[r + 8] = b;
                             }
                         }
                     }
                 }
-                rg += nslot;
-                ++round;
             }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        };
+        if (NT >= 4 && m > 2 * kMmTok) row_groups(std::integral_constant<int, NT >= 4 ? 4 : 1>());
+        else if (NT >= 2 && m > kMmTok) row_groups(std::integral_constant<int, NT >= 2 ? 2 : 1>());
+        else row_groups(std::integral_constant<int, 1>());
         __syncthreads();  // every warp has left the activations
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 template <int T, bool FUSED, int NT>
@@ -723,6 +747,26 @@ static int mm_launch_type(dnb_ctx* c, cudaStream_t st, bool fused, int nt, MmArg
 #undef DNB_MM
 }
 
+// The ring of each of `warps` warps that fits beside `base` bytes: two blocks a stage where a warp has that many, three stages, then two; else one
+// block, four stages to two.  Bytes of shared memory in all, or 0.
+static size_t mm_ring(int type, int blocks, int warps, size_t base, size_t cap, MmRing& r) {
+    static const int form[5][2] = {{2, 3}, {2, 2}, {1, 4}, {1, 3}, {1, 2}};
+    for (const auto& f : form) {
+        if (f[0] > blocks) continue;
+        r.bps = f[0];
+        r.nst = f[1];
+        switch (type) {
+#define DNB_P(TT) case TT: r.pitch = f[0] == 2 ? Mq<TT>::P2 : Mq<TT>::P1; break;
+            DNB_P(T_Q4_K) DNB_P(T_Q5_K) DNB_P(T_Q6_K) DNB_P(T_Q8_0) DNB_P(T_IQ3_XXS)
+#undef DNB_P
+            default: return 0;
+        }
+        const size_t smem = base + (size_t)warps * r.nst * 16 * r.pitch;
+        if (smem <= cap) return smem;
+    }
+    return 0;
+}
+
 // batch: K is split as a constant of the shape.  rows: token rows of the launch in total; nseg_est: segments that will have rows (an estimate when the device counts them).
 int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
@@ -733,8 +777,6 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, con
     int rc = type == T_IQ3_XXS ? upload_mm_s8(c->device) : DNB_OK;
     if (rc) return rc;
     const int bb = type == T_Q4_K ? 144 : type == T_Q5_K ? 176 : type == T_Q6_K ? 210 : type == T_Q8_0 ? 272 : 98;
-    const int rs = type == T_Q4_K ? Mq<T_Q4_K>::RS : type == T_Q5_K ? Mq<T_Q5_K>::RS : type == T_Q6_K ? Mq<T_Q6_K>::RS
-                 : type == T_Q8_0 ? Mq<T_Q8_0>::RS : Mq<T_IQ3_XXS>::RS;
     MmArgs A = {};
     A.seg = seg; A.nseg_dev = nseg_dev; A.nseg_max = nseg_max;
     if (single) A.single = *single;
@@ -762,13 +804,9 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, con
             while (ks < 8 && ks * 2 <= nb && per_cta * ks < 6 * kMmWarps) ks *= 2;
         A.ks = ks;
         size_t base = kMmFixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 2 * 32 * 4 : 0) + (size_t)nt * tpt * nb * kXBlock;
-        if (type == T_IQ3_XXS)  // the tables behind the activations, on their boundary (dynamic shared memory starts at kMmSmemBase)
-            base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmTables);
-        const size_t stage = (size_t)kMmWarps * 16 * rs, cap = 225 * 1024;
-        for (A.nst = 4; A.nst >= 2 && base + A.nst * stage > cap; --A.nst) {}
-        if (A.nst >= 2) {
-            const size_t smem = base + A.nst * stage;
-            A.smem = (uint32_t)smem;
+        if (type == T_IQ3_XXS) base += sizeof(MmTables);
+        const size_t smem = mm_ring(type, nb / ks, kMmWarps, base, 225 * 1024, A.ring);
+        if (smem) {
             A.status = c->status;
             // activations of a tile 2.5 - 3 us, a row group 1.1 us at K = 2048 and a quarter of that at K = 512 (measured, IQ3_XXS)
             A.skip = std::max(1, 5120 / n_in);
@@ -796,105 +834,76 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, con
 // work); a warp takes every ks-th block of K of 16 rows and asks for its first stages before it waits for the kernel in front of
 // it, whose output the vector may be; it converts its own blocks of the vector, each with a power of two of its own, so that no
 // CTA-wide step stands between vector and math; the warps' partial sums meet once per 16 rows, in a fixed order.
-// Measured back to back, us, with fp16 operands -> with bytes: 4096 x 4096 Q4_K 5.6 -> 4.7; 65536 x 4096 Q8_0 71.8 -> 64.1 (4.45 TB/s).  (The
-// register-decode GEMV before took 8.4 and 103.)
+// Measured back to back, us, with fp16 operands -> with bytes: 4096 x 4096 Q4_K 5.6 -> 4.7; 65536 x 4096 Q8_0 71.8 -> 61 (4.7 TB/s), Q4_K 54 -> 38, IQ3_XXS
+// 64 -> 57.  (The register-decode GEMV before took 8.4 for the small one, 103 for Q8_0.)
 constexpr int kGvWarps = 8;
 
 struct GvArgs {
     const uint8_t* w;
     const float* x;      // [tok][k]
     float* out;          // [tok][n]
-    int k, n, rb, ks, nst;
+    int k, n, rb, ks;
+    MmRing ring;
     int nvec;            // a grid row takes TOK of them
-    uint32_t smem;
     int* status;
 };
 
 template <int T, int TOK>
 __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const GvArgs A) {
     using Q = Mq<T>;
-    constexpr int STAGE = 16 * Q::RS, XB = TOK * kXBlock;  // bytes of a converted block
+    constexpr int XB = TOK * kXBlock;  // bytes of a converted block
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int nb = A.k >> 8, nslot = kGvWarps / A.ks, slot = warp / A.ks, kw = warp - slot * A.ks;
-    const int kbn = (nb - kw + A.ks - 1) / A.ks, kb_max = (nb + A.ks - 1) / A.ks;  // this warp's blocks: kw, kw + ks, ...
-    float* red = reinterpret_cast<float*>(smem);                                   // [2][8 warps][16 rows][TOK]
-    uint8_t* p = smem + 2 * kGvWarps * 16 * TOK * 4;
+    // this warp's blocks: every ks-th stage of K, so that neighbours ask for neighbouring bytes at the same time
+    const int bps = A.ring.bps, units = (nb + bps - 1) / bps, nst = (units - kw + A.ks - 1) / A.ks, kb_max = (units + A.ks - 1) / A.ks * bps;
+    auto first = [&](int i) { return (kw + i * A.ks) * bps; };         // block of stage i
+    auto count = [&](int i) { return min(bps, nb - first(i)); };
+    uint8_t* p = smem + (T == T_IQ3_XXS ? sizeof(MmTables) : 0);
+    float* red = reinterpret_cast<float*>(p);                                      // [2][8 warps][16 rows][TOK]
+    p += 2 * kGvWarps * 16 * TOK * 4;
     uint8_t* xs = p + (size_t)warp * kb_max * XB;
     p += (size_t)kGvWarps * kb_max * XB;
-    uint8_t* book = p;
-    if constexpr (T == T_IQ3_XXS) {
-        book += (kMmBookAlign - (tcp::s32(p) & (kMmBookAlign - 1))) & (kMmBookAlign - 1);
-        p = book + sizeof(MmTables);
-    }
-    if (T == T_IQ3_XXS && (uint32_t)(p - smem) + kGvWarps * A.nst * STAGE > A.smem) {  // only if shared memory started elsewhere
+    if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right
         if (tid == 0) status_set(A.status, 26);
         return;
     }
-    uint8_t* ring = p + (size_t)warp * A.nst * STAGE;
+    MmStream<T> W(p + (size_t)warp * A.ring.nst * 16 * A.ring.pitch, A.ring, lane);
     const int n_rg = (A.n + 15) / 16, last = A.n - 1, rg_step = gridDim.x * nslot;
     const int rounds = (n_rg - (int)blockIdx.x * nslot + rg_step - 1) / rg_step;  // of the CTA; a slot's last one may be empty
     const int rg0 = blockIdx.x * nslot + slot;
-    const int nrg = rg0 < n_rg ? (n_rg - rg0 + rg_step - 1) / rg_step : 0, nstage = nrg * kbn;
+    const int nrg = rg0 < n_rg ? (n_rg - rg0 + rg_step - 1) / rg_step : 0;
 
     // ---- weight stream (as in mm_kernel) ----
-    int pf_rg = rg0, pf_b = 0, pf_s = 0, pf_n = 0;
-    const int r_in = lane >> 3, c16 = (lane & 7) * 16;
-    constexpr bool TAIL = Q::ALIGNED && Q::UNITS % 8 == 1;
-    const uint8_t *sa = nullptr, *stl = nullptr;
-    uint32_t o1 = 0, o2 = 0, o3 = 0;
-    auto point = [&]() {
-        const int row = pf_rg * 16 + r_in, r0 = min(row, last);
-        sa = A.w + (size_t)r0 * A.rb + (uint32_t)kw * Q::BB;
-        o1 = (uint32_t)(min(row + 4, last) - r0) * A.rb;
-        o2 = (uint32_t)(min(row + 8, last) - r0) * A.rb;
-        o3 = (uint32_t)(min(row + 12, last) - r0) * A.rb;
-        if constexpr (TAIL) stl = A.w + (size_t)min(pf_rg * 16 + (lane & 15), last) * A.rb + (uint32_t)kw * Q::BB + (Q::UNITS - 1) * 16;
-    };
-    if (nstage > 0) point();
+    int pf_rg = rg0, pf_i = 0;
+    const int rg_stop = rg0 + nrg * rg_step;
     auto prefetch = [&]() {
-        if (pf_n < nstage) {
-            uint8_t* dst = ring + pf_s * STAGE + r_in * Q::RS + c16;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint8_t* src = sa + (j == 0 ? 0u : j == 1 ? o1 : j == 2 ? o2 : o3);
-                if constexpr (!Q::ALIGNED) src = reinterpret_cast<const uint8_t*>((uintptr_t)src & ~(uintptr_t)15);
-#pragma unroll
-                for (int cc = 0; cc < (TAIL ? Q::UNITS - 1 : Q::UNITS); cc += 8)
-                    if (cc + 8 <= Q::UNITS || cc * 16 + c16 < Q::UNITS * 16) tcp::cp_async16(dst + j * 4 * Q::RS + cc * 16, src + cc * 16 + c16);
-            }
-            if constexpr (TAIL) {
-                if (lane < 16) tcp::cp_async16(ring + pf_s * STAGE + lane * Q::RS + (Q::UNITS - 1) * 16, stl);
-                stl += A.ks * Q::BB;
-            }
-            ++pf_n;
-            sa += A.ks * Q::BB;
-            if (++pf_b == kbn) {
-                pf_b = 0;
-                pf_rg += rg_step;
-                if (pf_n < nstage) point();
-            }
-            if (++pf_s == A.nst) pf_s = 0;
+        int n = 0;
+        if (pf_rg < rg_stop) {
+            if (pf_i == 0) W.template point<false>(A.w + (uint32_t)first(0) * Q::BB, nullptr, pf_rg * 16, last, (uint32_t)A.rb);
+            n = count(pf_i);
         }
-        tcp::cp_async_commit();
+        W.request(n);
+        if (n > 0) {
+            W.skip((A.ks - 1) * bps * Q::BB);
+            if (++pf_i == nst) {
+                pf_i = 0;
+                pf_rg += rg_step;
+            }
+        }
     };
-    for (int i = 1; i < A.nst; ++i) prefetch();
-    if constexpr (T == T_IQ3_XXS) {  // in the last of those groups' shadow: waited for with the first stage
-        for (int i = tid; i < (int)(sizeof(MmTables) / 16); i += kGvWarps * 32)
-            tcp::cp_async16<false>(book + 16 * i, reinterpret_cast<const uint8_t*>(&g_mm_s8) + 16 * i);
-        tcp::cp_async_commit();
-    }
+    for (int i = 1; i < W.nst; ++i) prefetch();
+    if constexpr (T == T_IQ3_XXS) mm_tables_in(smem, tid, kGvWarps * 32);
     pdl_wait();
     pdl_launch_dependents();
 
     // ---- this warp's blocks of the vectors ----
     const int v0 = blockIdx.y * TOK;
-    for (int i = 0; i < kbn; ++i) {
+    for (int i = 0; i < nst; ++i)
+        for (int j = 0; j < count(i); ++j)
 #pragma unroll
-        for (int q = 0; q < TOK; ++q) {
-            mm_stage_block<T>(A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (kw + i * A.ks) * 256, xs + i * XB + q * kXBlock, lane);
-        }
-    }
+            for (int q = 0; q < TOK; ++q)
+                mm_stage_block<T>(A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (first(i) + j) * 256, xs + (i * bps + j) * XB + q * kXBlock, lane);
     if constexpr (T == T_IQ3_XXS) {  // the tables came in parts from all threads
         tcp::cp_async_wait_all();
         __syncthreads();
@@ -902,36 +911,33 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
     __syncwarp();
 
     // ---- the row groups ----
-    const uint32_t gl = tcp::s32(book) + 4 * lane, sl = gl + (uint32_t)sizeof(uint32_t) * 256 * 32;
+    const uint32_t gl = 4 * lane, sl = 8 * (lane & 15);
     const uint8_t *colb = xs + (TOK == 2 ? g >> 2 : 0) * kXBlock, *colv = xs + (TOK == 2 ? t >> 1 : 0) * kXBlock + kXInv + (t & 1) * 4;
-    int q_s = 0, rg = rg0;
-    for (int rd = 0; rd < rounds; ++rd, rg += rg_step) {
+    for (int rd = 0, rg = rg0; rd < rounds; ++rd, rg += rg_step) {
         float acc[1][2] = {{0.f, 0.f}};
         if (rd < nrg) {
             uint32_t offa = 0, offb = 0;
             if constexpr (!Q::ALIGNED) {
-                offa = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + g, last) * A.rb + (uint32_t)kw * Q::BB;
-                offb = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + 8 + g, last) * A.rb + (uint32_t)kw * Q::BB;
+                offa = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + g, last) * A.rb + (uint32_t)first(0) * Q::BB;
+                offb = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + 8 + g, last) * A.rb + (uint32_t)first(0) * Q::BB;
             }
-            for (int i = 0; i < kbn; ++i) {
-                if (A.nst == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
-                else if (A.nst == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-                else asm volatile("cp.async.wait_group 2;" ::: "memory");
-                __syncwarp();
+#pragma unroll 1
+            for (int i = 0; i < nst; ++i) {
+                const uint8_t* st = W.wait();
                 prefetch();
-                const uint8_t* st = ring + q_s * STAGE;
-                const uint8_t *ra = st + g * Q::RS, *rb = st + (g + 8) * Q::RS;
-                if constexpr (!Q::ALIGNED) {
-                    ra += offa & 15u;
-                    rb += offb & 15u;
-                    offa += A.ks * Q::BB;
-                    offb += A.ks * Q::BB;
+                const uint8_t *ra = st + g * W.pitch + (Q::ALIGNED ? 0u : offa & 15u), *rb = st + (g + 8) * W.pitch + (Q::ALIGNED ? 0u : offb & 15u);
+                offa += A.ks * bps * Q::BB;
+                offb += A.ks * bps * Q::BB;
+                const int n = count(i);
+#pragma unroll 1
+                for (int j = 0; j < n; ++j, ra += Q::BB, rb += Q::BB) {
+                    const int b = i * bps + j;
+                    const uint8_t* const bp[1] = {colb + b * XB + (g & 3) * kXDigit + t * 8};
+                    const uint32_t sumw[1] = {mq_mins<T> && (g & 3) < 3 ? *reinterpret_cast<const uint32_t*>(colb + b * XB + kXSums + (g & 3) * 16 + t * 4) : 0u};
+                    const float inv[1] = {*reinterpret_cast<const float*>(colv + b * XB)};
+                    mm_block<T, 1>(ra, rb, t, gl, sl, bp, sumw, inv, acc);
                 }
-                const uint8_t* const bp[1] = {colb + i * XB + (g & 3) * kXDigit + t * 8};
-                const uint32_t sumw[1] = {mq_mins<T> && (g & 3) < 3 ? *reinterpret_cast<const uint32_t*>(colb + i * XB + kXSums + (g & 3) * 16 + t * 4) : 0u};
-                const float inv[1] = {*reinterpret_cast<const float*>(colv + i * XB)};
-                mm_block<T, 1>(ra, rb, t, gl, sl, bp, sumw, inv, 1, acc);
-                if (++q_s == A.nst) q_s = 0;
+                W.next();
             }
         }
         // lanes t = 0, 1 hold the first vector's low and high digits, t = 2, 3 the second's
@@ -955,18 +961,17 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
 
 template <int T, int TOK>
 static int launch_gv_t(dnb_ctx* c, cudaStream_t st, GvArgs A) {
-    const int nb = A.k / 256, rs = Mq<T>::RS;
+    const int nb = A.k / 256;
     int ks = 1;
     while (ks < kGvWarps && ks * 2 <= nb) ks *= 2;
-    const int kb_max = (nb + ks - 1) / ks;
-    size_t base = 2 * kGvWarps * 16 * TOK * 4 + (size_t)kGvWarps * kb_max * TOK * kXBlock;
-    if (T == T_IQ3_XXS) base = (base + kMmSmemBase + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign - kMmSmemBase + sizeof(MmTables);
-    const size_t stage = (size_t)kGvWarps * 16 * rs, two = 113 * 1024, cap = 225 * 1024;  // two CTAs per SM where they fit
+    // a warp's share of the vectors: at most one block more than nb / ks (a ring of two blocks a stage: two)
+    size_t base = 2 * kGvWarps * 16 * TOK * 4 + (size_t)kGvWarps * ((nb + 2 * ks - 1) / (2 * ks) * 2) * TOK * kXBlock;
+    if (T == T_IQ3_XXS) base += sizeof(MmTables);
+    const size_t two = 113 * 1024;  // two CTAs per SM where they fit
     A.ks = ks;
-    for (A.nst = 4; A.nst > 2 && base + A.nst * stage > two; --A.nst) {}
-    const size_t smem = base + A.nst * stage;
-    if (smem > cap) return DNB_DECLINED;
-    A.smem = (uint32_t)smem;
+    size_t smem = mm_ring(T, nb / ks, kGvWarps, base, two, A.ring);
+    if (!smem) smem = mm_ring(T, nb / ks, kGvWarps, base, 225 * 1024, A.ring);
+    if (!smem) return DNB_DECLINED;
     A.status = c->status;
     auto kern = gemv_mma_single_kernel<T, TOK>;
     static SmemGrant grant;
