@@ -393,9 +393,9 @@ static int experts_dev_tc(dnb_ctx* c, int layer, const float* x, int nt, const i
     const int ty = L.m[0].type;
     if (!op_ready)
         if ((rc = launch_operand_rows(c, st, ty, x, M.e, nt, M.e, w.op_x, "operand_rows_x"))) return rc;
-    if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, w.op_x, w.row_token, w.act, nullptr, nt, rows))) return rc;
+    if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_gu, w.nseg, nseg_max, M.e, M.ff, w.op_x, w.row_token, w.act))) return rc;
     if ((rc = launch_operand_rows(c, st, ty, w.act, M.ff, rows, M.ff, w.op_act, "operand_rows_act"))) return rc;
-    if ((rc = launch_grouped_tc(c, st, ty, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, w.op_act, nullptr, w.hrow, nullptr, nt, rows))) return rc;
+    if ((rc = launch_grouped_tc(c, st, ty, false, w.seg_dn, w.nseg, nseg_max, M.ff, M.e, w.op_act, nullptr, w.hrow))) return rc;
     if (shared && L.shared_gate_row)
         if ((rc = launch_shared_coef(c, st, x, L.shared_gate_row, nt, M.e, w.shcoef))) return rc;
     return launch_combine(c, st, w.hrow, w.pos, wts, nt, k, M.e, shared ? w.hrow + (size_t)nt * k * M.e : nullptr,
@@ -520,9 +520,9 @@ int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, 
     if (c->use_tc && w.op_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
         if (!op_ready)
             if ((rc = launch_operand_rows(c, st, ty, x, M.e, rows, M.e, w.op_x, "operand_rows_x"))) return rc;
-        if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, nullptr, w.act, nullptr, rows, rows))) return rc;
+        if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, nullptr, w.act))) return rc;
         if ((rc = launch_operand_rows(c, st, ty, w.act, M.ff, rows, M.ff, w.op_act, "operand_rows_act"))) return rc;
-        return launch_grouped_tc(c, st, ty, false, w.seg_sh_dn, w.one, 1, M.ff, M.e, w.op_act, nullptr, out, nullptr, rows, rows);
+        return launch_grouped_tc(c, st, ty, false, w.seg_sh_dn, w.one, 1, M.ff, M.e, w.op_act, nullptr, out);
     }
     if ((rc = launch_seg_matmul(c, st, L.m[3].type, true, w.seg_sh_gu, nullptr, 1, M.e, sff, x, M.e, nullptr, w.sact, rows))) return rc;
     return launch_seg_matmul(c, st, L.m[5].type, false, w.seg_sh_dn, nullptr, 1, sff, M.e, w.sact, sff, nullptr, out, rows);

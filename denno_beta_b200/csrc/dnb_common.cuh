@@ -398,7 +398,7 @@ int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, i
 // fused: seg[].wa / wb = gate / up, out = silu(g) * u; otherwise seg[].wa.  fp32 packed rows out, or where row_dst says (expert
 // parallel).  row_token: packed row -> operand row, null: itself.  tokens, rows: of the call, choose the items' size (0: small).
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
-                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst = nullptr, int tokens = 0, int rows = 0);
+                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst = nullptr);
 // The shared expert of a layer on `rows` fp32 rows (api.cu); op_ready: their operand rows are in the workspace already.
 int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, float* out);
 int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t* pos, const float* wts, int nt,

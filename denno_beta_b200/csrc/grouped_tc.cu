@@ -12,29 +12,35 @@
 // dmin into fp16's range whatever its size, B = X.  An activation is fp16 hi + lo (22 bits) of the row times a power of two that
 // puts its largest element into [512, 1024).
 //
-// What bounds it: a 64-element stage of two 128-row tiles is about 900 warp instructions of decoding (Q4_K; 1.7 per weight) on
-// four schedulers and 8 MMAs of N = 2 x tokens, the same order of time at 32 tokens; everything else has to stay out of the
-// way of both.  Shared memory is the tightest: with A tiles in it (32 KB written and 32 KB read per stage, B read once per tile) a
-// stage took 840 cycles, all of them shared-memory bandwidth.  So A goes from the producers' registers to tensor memory
-// (tcgen05.st, thread = row = lane) and the MMA takes it from there.  One role per warp, each with a ring of its own in front:
-//   * four warps copy packed rows (a 256-element block of all 256 rows: 9 or 7 neighbouring lanes per row) into a raw ring.  (A
-//     thread that fetches its own row's bytes touches 32 cache lines per instruction; that alone took 0.5 us per stage.)
-//   * two warps copy the tokens' hi and lo rows into swizzled B tiles, a stage each in turn, gathered from the token-major rows:
-//     no packed copy of the activations.  (TMA row gathers took 80 cycles per four rows; a proxy fence in the copying warp
-//     waits for the copies still on their way, so it is the MMA thread that executes it.)
+// What bounds it: instructions.  A 64-element stage of two 128-row tiles is 900 to 1,500 warp instructions of decoding on four schedulers, a
+// copy, a wait or a hand-over of some warp as much again, and 16 MMAs of N = tokens (8 N cycles in all); 0.7 of the issue slots are taken.
+// Shared memory is next: with A tiles in it (32 KB written and 32 KB read per stage, B read once per tile) a stage took 840 cycles, all of
+// them shared-memory bandwidth.  So A goes from the producers' registers to tensor memory (tcgen05.st, thread = row = lane) and the MMA
+// takes it from there.  One role per warp, each with a ring of its own in front:
+//   * two warps copy packed rows (a 256-element block of all 256 rows, a tile a warp: 9 or 7 neighbouring lanes per row) into a raw ring.
+//     (A thread that fetches its own row's bytes touches 32 cache lines per instruction; that alone took 0.5 us per stage.)
+//   * four warps copy the tokens' lo (two) and hi rows into swizzled B tiles, two stages at a time, gathered from the token-major rows: no
+//     packed copy of the activations.  (TMA row gathers took 80 cycles per four rows; a proxy fence in the copying warp waits for the copies
+//     still on their way, so it is the MMA thread that executes it.  Two warps were behind the others in IQ3_XXS.)
 //   * four groups of four producer warps, (even or odd stages) x (tile), a thread one row: decodes 64 weights into registers, THEN
-//     waits for a ring slot (tensor memory holds only four stages; with the decoding inside its turn-around a stage took 1,100
+//     waits for its slot (tensor memory holds only a block; with the decoding inside its turn-around a stage took 1,100
 //     cycles) and stores them.  The block's scales go to a small ring, its mins to shared memory of the thread's own.
-//     A stage has one full barrier for both operands, on which producers and B copies arrive (a second wait a stage: 2 to 3 % more time).
-//   * one MMA thread; hi and lo rows of a token are neighbours in the B tile (N = 2 x tokens) and in TMEM, so a weight tile is read
-//     once per K step.
+//   * two MMA threads, a tile each.  A block's weights stay in tensor memory while they are multiplied with the lo rows and then with the hi
+//     rows, into the same columns: with 64 tokens there are two accumulator buffers (with sums of hi and lo apart there was room for
+//     one, and the tensor core waited 350 cycles of a stage's 1,060 while it was read), and as lo comes first, the sums are rounded as often
+//     as those of hi alone: the distance from 64 bits is what it was (0.998 of it over 48 forms).  A wait, a fence and a commit are some 200
+//     cycles of a thread's time, so two stages share them, and one thread for both tiles would be the bottleneck.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
-// Persistent, one CTA per SM; items (segment, 32- or 64-token tile, 128 rows x 2) dealt round-robin.
+// Persistent, one CTA per SM; items (segment, up to 64 tokens, 128 rows x 2) dealt round-robin.
+// The code of all roles has to stay small: eight warps of a scheduler run five different loops.  Waiting loops that the compiler
+// had unrolled made 150 KB of it, and no_instruction was a stall as frequent as the arithmetic pipes' (75 KB: Q4_K 434 -> 409 us a pass of the
+// below); one copy of the decoding instead of two, and one of the MMA loop, 493 -> 434.
 //
-// Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, us gate/up + down as bracketed by events: Q4_K 175 + 84 (three
-// bf16 products, a seventh of the accuracy) -> 122 + 83, IQ3_XXS 343 + 180 -> 122 + 73.  A stage takes about 950 cycles: the issuing thread's waits, fence, issue and
-// commit; without the decoding a copy of the kernel was only 7 % faster.
+// Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, two layers, us a pass: items of 32 (Q4_K) or 64 tokens with hi and lo
+// sums apart -> these: Q4_K 501 -> 409, IQ3_XXS 473 -> 429; a prompt of 14,018 tokens 6,865 -> 5,684.
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "dnb_common.cuh"
 #include "tc_ptx.cuh"
@@ -48,31 +54,27 @@ using namespace tcp;
 constexpr int BK = 64;                  // K of a stage: one 128-byte swizzle row of fp16
 constexpr int TILE_M = 128;
 constexpr int A_COLS = BK / 2;          // tensor-memory columns of an A tile (two fp16 each)
-constexpr int EWARPS = 8, PWARPS = 16, RWARPS = 4, BWARPS = 2;
-constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;
-constexpr int NTHREADS = 1024;          // 32 warps, the last one idle
-// What depends on the tokens of an item.  64 tokens a weight tile halve the decoding of an expert with many, but there is room for one
-// accumulator buffer only (the tensor core waits while a block's sums are read) and for four B tiles instead of eight.
-template <int NT> struct Tok {
-    static constexpr int B_STAGE = 2 * NT * BK * 2;  // hi and lo rows: 8 or 16 KB
-    static constexpr int NB = 64 / NT;               // accumulator buffers
-    static constexpr int BUF_COLS = 2 * 2 * NT;      // two tiles x (hi, lo) x tokens
-    static constexpr int BSLOTS = 256 / NT;          // ring of B in shared memory (its copies take over a microsecond)
-    // Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
-    static constexpr int REG_EPI = NT == 64 ? 112 : 96, REG_PROD = NT == 64 ? 56 : 64, REG_RAW = 24, REG_MISC = 40;
-    static_assert(2 * REG_EPI + 4 * REG_PROD + REG_RAW + REG_MISC <= 8 * 64, "register split");
-};
-constexpr int B_BYTES = 65536;          // of the B ring
-static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 4 && W_MMA == 30, "roles fill warpgroups");
+constexpr int EWARPS = 8, PWARPS = 16, RWARPS = 2, BWARPS = 4;
+constexpr int W_RAW = EWARPS + PWARPS, W_B = W_RAW + RWARPS, W_MMA = W_B + BWARPS;  // two warps, a tile each
+constexpr int NTHREADS = 1024;
+// Tokens of an item at most; N of its MMAs follows it in sixteens.  Against items of up to 32 (or, from some rows a segment on, 64), us a layer of
+// 2048 x 512, evenly routed and skewed by -1.1 ln rank: Q4_K, 64 experts top 10, 512 tokens 212, 212 -> 186, 188; 128 top 8, 700 tokens 223, 239 ->
+// 183, 207; 512 top 10, 512 tokens 434, 253 -> 439, 207; 64 tokens 306, 103 -> 307, 105.  IQ3_XXS 215, 214 -> 195, 195; 217, 240 -> 192, 218;
+// 510, 242 -> 452, 217; 331, 106 -> 319, 108.
+constexpr int NT = 64;
+constexpr int NB = 2, BUF_COLS = 2 * NT;  // accumulator buffers: two tiles x tokens
+constexpr int SLOTS = 4;                // of A (tensor memory) and of each half of B: stage c of a block has slot c
+constexpr int PAIRS = SLOTS / 2;        // two stages have a barrier in common
+constexpr int B_SLOT = NT * BK * 2, B_BYTES = 2 * SLOTS * B_SLOT;  // lo rows, then hi rows
+// Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
+constexpr int REG_EPI = 112, REG_PROD = 56, REG_COPY = 32;
+static_assert(2 * REG_EPI + 4 * REG_PROD + 2 * REG_COPY <= 8 * 64, "register split");
+static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS + BWARPS == 6 && W_MMA == 30, "roles fill warpgroups");
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
-constexpr int STAGES = 4, BSTAGES = 2 * STAGES;  // ring of A (tensor memory); barriers of a stage, which is known by its number mod BSTAGES
-constexpr int A_COL0 = 256, TMEM_COLS = A_COL0 + STAGES * 2 * A_COLS;
-static_assert(Tok<32>::NB * Tok<32>::BUF_COLS == A_COL0 && Tok<64>::NB * Tok<64>::BUF_COLS == A_COL0, "accumulators");
-static_assert(Tok<32>::BSLOTS * Tok<32>::B_STAGE == B_BYTES && Tok<64>::BSLOTS * Tok<64>::B_STAGE == B_BYTES, "B ring");
-static_assert(Tok<32>::BSLOTS == BSTAGES && Tok<64>::BSLOTS == STAGES, "a B slot is freed by the stage BSTAGES or STAGES earlier");
+constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + SLOTS * 2 * A_COLS;
 static_assert(TMEM_COLS == 512, "tensor memory");
-constexpr int SCL = 8;                  // ring of block scales (the mins count as a block): producers are at most five blocks ahead of the epilogue
+constexpr int SCL = 8;                  // ring of block scales (the mins count as a block): producers are at most three blocks ahead of the epilogue
 
 template <int T> constexpr int kBB = T == T_Q4_K ? 144 : 98;
 
@@ -83,7 +85,7 @@ struct Item {
     int r0, pad;        // first output row
 };
 
-template <bool PAIR, int NT>
+template <bool PAIR>
 __device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int nseg, const int* pre, const SegDesc* __restrict__ seg) {
     const int tile = item / row_tiles, rt = item - tile * row_tiles;
     int lo = 0, hi = nseg;  // pre[lo] <= tile < pre[lo + 1]
@@ -103,8 +105,8 @@ __device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int
     return it;
 }
 
-// Tokens of the B tile: the smallest of 8, 16, 32, 64 that holds the item.
-__device__ __forceinline__ int tile_tokens(int m) { return m <= 8 ? 8 : m <= 16 ? 16 : m <= 32 ? 32 : 64; }
+// Tokens of the B tile, N of its MMAs: the item's in sixteens.
+__device__ __forceinline__ int tile_tokens(int m) { return (m + 15) & ~15; }
 
 // An item's stages: for every eight blocks (or the rest) their 64-element stages, then those of the mins (Q4_K): with up to four
 // blocks one stage holds the hi parts of the up to 32 mins in its first 32 columns and the lo parts in the others (the operand row
@@ -172,6 +174,14 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+template <int N> using Int = std::integral_constant<int, N>;
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 // D (+)= A * B with A in tensor memory.
 __device__ __forceinline__ void mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
@@ -252,41 +262,22 @@ template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm vol
 template <int T> struct Layout {
     static constexpr int RSTAGES = 3;
     static constexpr int RAW_TILE = TILE_M * Raw<T>::RS, RAW_STAGE = 2 * RAW_TILE;
-    static constexpr int BARS = 2 * BSTAGES + 2 * (RSTAGES + 2);
+    static constexpr int BARS = 8 * PAIRS + 2 * (RSTAGES + NB);
     static constexpr int HEAD = (BARS * 8 + 16 + (kMaxSeg + 1) * 4 + 8 + kLocalItems * (int)sizeof(Item) + 127) / 128 * 128;
     static constexpr int LOW = (HEAD + SCL * 2 * TILE_M * 4 + 1023) / 1024 * 1024;  // where the B ring starts
     static constexpr int MINS = T == T_Q4_K ? PWARPS * 32 * 8 * 10 : 0;  // 8 + 2 bytes per block and producer thread
     static constexpr int TAIL = RSTAGES * RAW_STAGE + MINS;
 };
 
-// A stage number as its user sees it.  A group's stages are up to six apart and the groups may be a block apart from one another:
-// with one `empty` barrier per slot a group could look at a slot whose last but one stage is still in use and take its parity for
-// the last one's.  Stage n therefore commits to barrier n mod 2 * STAGES, and its slot's next user waits for exactly that commit.
-struct StageCount {
-    int q;          // stage number mod 2 * STAGES
-    uint32_t turn;  // parity of its turn
-    __device__ __forceinline__ explicit StageCount(int first) : q(first), turn(0u) {}
-    __device__ __forceinline__ void advance(int n) {
-        q += n;
-        if (q >= 2 * STAGES) { q -= 2 * STAGES; turn ^= 1u; }
-    }
-    __device__ __forceinline__ int slot() const { return q & (STAGES - 1); }
-    __device__ __forceinline__ bool wait(uint64_t* empty, int* status, int code) const {  // the stage STAGES earlier is done with its slot
-        return q < STAGES ? mb_wait(&empty[q + STAGES], turn ^ 1u, status, code) : mb_wait(&empty[q - STAGES], turn, status, code);
-    }
-};
-
-template <int T, bool PAIR, int NT>  // NT: tokens of an item; PAIR: both tiles from seg.wa (256 rows, fp32 results); else gate and up rows, silu(g) * u
+template <int T, bool PAIR>  // PAIR: both tiles from seg.wa (256 rows, fp32 results); else gate and up rows, silu(g) * u
 __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     using L = Layout<T>;
     using R = Raw<T>;
-    using K = Tok<NT>;
-    constexpr int NB = K::NB, BUF_COLS = K::BUF_COLS, B_STAGE = K::B_STAGE;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* base = smem_raw + ((1024u - (s32(smem_raw) & 1023u)) & 1023u);
-    uint64_t* full = reinterpret_cast<uint64_t*>(base);
-    uint64_t* empty = full + BSTAGES;         // both: one per B slot, two per A slot
-    uint64_t* rfull = empty + BSTAGES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(base);  // [tile][PAIRS] A and the lo rows of B, [PAIRS] the hi rows
+    uint64_t* empty = full + 4 * PAIRS;                  // [tile][PAIRS] the lo rows of B, [PAIRS] A and the hi rows
+    uint64_t* rfull = empty + 4 * PAIRS;
     uint64_t* rempty = rfull + L::RSTAGES;
     uint64_t* tfull = rempty + L::RSTAGES;
     uint64_t* tfree = tfull + NB;
@@ -307,21 +298,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         return;
     }
 
-    // The warp's number, told to be the same for its lanes: what depends on it leaves the 64 registers a thread.  Spills in bytes, stores +
-    // loads: Q4_K 48 + 88 -> 0 at 32 tokens, 112 + 148 -> 72 + 68 at 64; IQ3_XXS at 64 64 + 100 -> 36 + 28.  us gate/up + down, 64 experts top 10,
-    // 1024 tokens evenly routed: Q4_K at 64 166 + 106 -> 145 + 103, IQ3_XXS 160 + 97 -> 150 + 97.  IQ3_XXS down at 32 never spilled and loses:
-    // 128 -> 135.
-    constexpr bool kUniform = !(T == T_IQ3_XXS && PAIR && NT == 32);
-    const int tid = threadIdx.x, warp = kUniform ? __shfl_sync(0xffffffffu, tid >> 5, 0) : tid >> 5, lane = tid & 31;
+    // The warp's number, told to be the same for its lanes: what depends on it leaves the 64 registers a thread.
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nblk = A.n_in / 256;
     const int row_tiles = A.n_out / (PAIR ? 2 * TILE_M : TILE_M);
     const int pitch = row_pitch(A.n_in), scale_col = A.n_in + x_cols(A.n_in);
 
     if (tid == 0) {
-        for (int i = 0; i < BSTAGES; ++i) mb_init(&full[i], 8 + BWARPS * 32);  // two producer groups' warps, a tile each, and the B warps' lanes
-        for (int i = 0; i < BSTAGES; ++i) mb_init(&empty[i], 1);               // a commit
+        for (int i = 0; i < 4 * PAIRS; ++i) {
+            mb_init(&full[i], (i & PAIRS ? 0 : PWARPS / 2) + BWARPS / 2 * 32);  // a tile's producers, and the lanes of two B warps
+            mb_init(&empty[i], 1);                                              // a commit
+        }
         for (int i = 0; i < L::RSTAGES; ++i) { mb_init(&rfull[i], RWARPS * 32); mb_init(&rempty[i], PWARPS); }
-        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 1); mb_init(&tfree[i], EWARPS); }
+        for (int i = 0; i < NB; ++i) { mb_init(&tfull[i], 2); mb_init(&tfree[i], EWARPS); }
         fence_mbarrier_init();
     }
     if constexpr (T == T_IQ3_XXS) {
@@ -354,20 +343,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const int n_items = nseg > 0 ? pre[nseg] * row_tiles : 0;
     const int GR = gridDim.x;
     const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + GR - 1) / GR : 0;
-    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR, NT>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, pre, A.seg);
+    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, pre, A.seg);
     __syncthreads();
     auto item = [&](int k) {
-        return k < kLocalItems ? itab[k] : decode_item<PAIR, NT>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, pre, A.seg);
+        return k < kLocalItems ? itab[k] : decode_item<PAIR>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, pre, A.seg);
     };
     bool ok = true;
 
     if (warp < EWARPS) {
         // ---------------- epilogue: TMEM lane = weight row ----------------
-        reg_inc<K::REG_EPI>();
+        reg_inc<REG_EPI>();
         const int quad = warp & 3, hsel = warp >> 2;
         const int r = quad * 32 + lane;
         const uint32_t tlane = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -380,45 +369,46 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             return *reinterpret_cast<const float*>(A.op + (size_t)(2 * orow) * pitch + scale_col);
         };
         float rs_next = my_items > 0 ? row_scale(0) : 0.f;
+#pragma unroll 1
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             const int nte = tile_tokens(it.m), half = nte >> 1;
             const float rs = rs_next;
             rs_next = k + 1 < my_items ? row_scale(k + 1) : 0.f;
-            float acc[2][NT / 2];
+            float acc[2][NT / 2];  // the tile's first or second half of the tokens
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                 for (int j = 0; j < NT / 2; ++j) acc[mt][j] = 0.f;
+#pragma unroll 1
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
+#pragma unroll 1
                 for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0); ++b) {  // the last one: the mins
                     ok = warp_all(mb_wait(&tfull[buf], pb, A.status, 3));
                     if (!ok) break;
                     tc_fence_after();
                     const float s[2] = {scl[(sc * 2) * TILE_M + r], scl[(sc * 2 + 1) * TILE_M + r]};
                     sc = (sc + 1) & (SCL - 1);
-                    const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * nte);
-#pragma unroll
-                    for (int h = 0; h < NT / 16; ++h) {  // eight tokens a load; a warp has half of the tile's
-                        if (h == 0 || 16 * h < nte) {
-                            uint32_t v[2][16];
-                            tmem_ld16(col + 16 * h, v[0]);
-                            tmem_ld16(col + 2 * NT + 16 * h, v[1]);
-                            tmem_ld_wait();
-                            if (16 * h + 16 >= nte) {  // read: hand the buffer back before the arithmetic
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) mb_arrive(&tfree[buf]);
-                            }
-#pragma unroll
-                            for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    acc[mt][8 * h + j] =
-                                        fmaf(s[mt], __uint_as_float(v[mt][2 * j]) + __uint_as_float(v[mt][2 * j + 1]), acc[mt][8 * h + j]);
+                    const uint32_t col = tlane + (uint32_t)(buf * BUF_COLS + hsel * half);
+                    auto sums = [&](auto at, auto width) {  // of `width` tokens; the last of them hand the buffer back before the arithmetic
+                        constexpr int O = decltype(at)::value, W = decltype(width)::value;
+                        uint32_t v[2][W];
+                        tmem_ld(col + O, v[0]);
+                        tmem_ld(col + NT + O, v[1]);
+                        tmem_ld_wait();
+                        if (O + W >= half) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mb_arrive(&tfree[buf]);
                         }
-                    }
+#pragma unroll
+                        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                            for (int j = 0; j < W; ++j) acc[mt][O + j] = fmaf(s[mt], __uint_as_float(v[mt][j]), acc[mt][O + j]);
+                    };
+                    if (half == 8) sums(Int<0>(), Int<8>()); else sums(Int<0>(), Int<16>());
+                    if (half == 24) sums(Int<16>(), Int<8>()); else if (half == 32) sums(Int<16>(), Int<16>());
                     if (++buf == NB) { buf = 0; pb ^= 1u; }
                 }
             }
@@ -426,32 +416,36 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             const int t0 = hsel * half, cnt = min(half, it.m - t0);
             float* o = A.out + (size_t)(it.prow + t0) * A.n_out + it.r0 + r;
 #pragma unroll
-            for (int j = 0; j < NT / 2; ++j) {  // all results first (independent chains), then the stores
-                const float f = __shfl_sync(0xffffffffu, rs, j);
-                acc[0][j] *= f;
-                acc[1][j] *= f;
-                if constexpr (!PAIR) acc[0][j] = swiglu_fast(acc[0][j], acc[1][j]);
-            }
-            if (PAIR && A.row_dst) {  // expert parallel: the owner's (token, slot) row
+            for (int j0 = 0; j0 < NT / 2; j0 += 8) {
+                if (j0 >= cnt) break;
 #pragma unroll
-                for (int j = 0; j < NT / 2; ++j)
-                    if (j < cnt) {
-                        float* d = A.row_dst[it.prow + t0 + j] + it.r0 + r;
-                        d[0] = acc[0][j];
-                        d[TILE_M] = acc[1][j];
-                    }
-            } else {
+                for (int j = j0; j < j0 + 8; ++j) {  // eight results first (independent chains), then the stores
+                    const float f = __shfl_sync(0xffffffffu, rs, j);
+                    acc[0][j] *= f;
+                    acc[1][j] *= f;
+                    if constexpr (!PAIR) acc[0][j] = swiglu_fast(acc[0][j], acc[1][j]);
+                }
+                if (PAIR && A.row_dst) {  // expert parallel: the owner's (token, slot) row
 #pragma unroll
-                for (int j = 0; j < NT / 2; ++j, o += A.n_out)
-                    if (j < cnt) {
-                        o[0] = acc[0][j];
-                        if constexpr (PAIR) o[TILE_M] = acc[1][j];
-                    }
+                    for (int j = j0; j < j0 + 8; ++j)
+                        if (j < cnt) {
+                            float* d = A.row_dst[it.prow + t0 + j] + it.r0 + r;
+                            d[0] = acc[0][j];
+                            d[TILE_M] = acc[1][j];
+                        }
+                } else {
+#pragma unroll
+                    for (int j = j0; j < j0 + 8; ++j, o += A.n_out)
+                        if (j < cnt) {
+                            o[0] = acc[0][j];
+                            if constexpr (PAIR) o[TILE_M] = acc[1][j];
+                        }
+                }
             }
         }
     } else if (warp < W_RAW) {
         // ---------------- producers ----------------
-        reg_dec<K::REG_PROD>();
+        reg_dec<REG_PROD>();
         const int pw = warp - EWARPS, odd = pw >> 3, tile = (pw >> 2) & 1, r = (pw & 3) * 32 + lane;
         const uint32_t tlane = tmem_base + A_COL0 + (uint32_t)(tile * A_COLS) + ((uint32_t)((pw & 3) * 32) << 16);
         const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
@@ -459,30 +453,37 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         uint16_t* dd = reinterpret_cast<uint16_t*>(raw_base + L::RSTAGES * L::RAW_STAGE + PWARPS * 32 * 8 * 8) + pw * 32 + lane;
         int rst = 0, sc = 0;
         uint32_t rph = 0u;
-        StageCount q(odd);
-        auto hand_over = [&](const uint32_t (&o)[32]) {  // into the ring slot of stage q
-            ok = warp_all(q.wait(empty, A.status, 2));
+        uint32_t turn = ~0u;  // parities of the pairs
+        auto claim = [&](int h) {  // slot odd + 2 h
+            ok = warp_all(mb_wait(&empty[(2 * tile + 1) * PAIRS + h], (turn >> h) & 1u, A.status, 2));
+            turn ^= 1u << h;
+        };
+        auto hand_over = [&](const uint32_t (&o)[32], int h) {
+            claim(h);
             if (!ok) return;
             tc_fence_after();
-            tmem_st32(tlane + q.slot() * (2 * A_COLS), o);
+            tmem_st32(tlane + (odd + 2 * h) * (2 * A_COLS), o);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mb_arrive(&full[q.q]);
+            if (lane == 0) mb_arrive(&full[2 * tile * PAIRS + h]);
         };
+#pragma unroll 1
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
             uint32_t off = 0;  // where the row's block starts within 16 bytes
             if constexpr (T == T_IQ3_XXS) off = (uint32_t)(uintptr_t)(tile ? it.pb : it.pa) + (uint32_t)r * A.rb;
+#pragma unroll 1
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
                 uint32_t top = 0u;  // bits of the largest |dmin|, in the upper half
+#pragma unroll 1
                 for (int b = 0; b < bn; ++b) {
                     ok = warp_all(mb_wait(&rfull[rst], rph, A.status, 7));
                     if (!ok) break;
                     const uint8_t* raw = raw_base + rst * L::RAW_STAGE + tile * L::RAW_TILE + r * R::RS + (off & 15u);
                     if constexpr (T == T_IQ3_XXS) off += kBB<T>;
-#pragma unroll
+#pragma unroll 1
                     for (int h = 0; h < 2; ++h) {
                         R in;
                         in.load(raw, odd + 2 * h);
@@ -503,16 +504,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         }
                         uint32_t o[32];
                         decode_stage(in, odd + 2 * h, o, gl, sl);
-                        hand_over(o);
+                        hand_over(o, h);
                         if (!ok) break;
-                        q.advance(2);
                     }
                     if (!ok) break;
                 }
                 if (!ok) break;
                 if constexpr (T == T_Q4_K) {
-                    const int nm = min_stages<T>(bn);
-                    if (odd < nm) {
+                    if (odd < min_stages<T>(bn)) {
                         // e = top >> 26, the exponent field of the largest |dmin| < 2^(e - 14): times 2^(24 - e) (2^15 at most) it is below
                         // 2^10, and dmin * m <= 63 * dmin below fp16's largest number
                         const uint32_t ex = min(30u, 39u - (top >> 26));
@@ -522,32 +521,37 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         }
                         uint32_t o[32];
                         mins_stage(mm, dd, bn, odd, ex, o);
-                        hand_over(o);
+                        hand_over(o, 0);
+                    } else {
+                        claim(0);
+                        if (ok && lane == 0) mb_arrive(&full[2 * tile * PAIRS]);
                     }
-                    q.advance(nm);
                 }
             }
         }
     } else if (warp < W_B) {
-        reg_dec<K::REG_RAW>();
-        // ---------------- raw rows: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
-        const int rw = warp - W_RAW, c16 = (lane & 7) * 16, row0 = (rw & 1) * (TILE_M / 2);  // half a tile per warp
+        reg_dec<REG_COPY>();
+        // ---------------- raw rows, a tile per warp: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
+        const int rw = warp - W_RAW, c16 = (lane & 7) * 16;
         int rst = 0;
         uint32_t rph = 1u;
+#pragma unroll 1
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
-            const uint8_t* half = ((rw & 2) ? it.pb : it.pa) + (size_t)row0 * A.rb;
+            const uint8_t* tile = rw ? it.pb : it.pa;
+#pragma unroll 1
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
+#pragma unroll 1
                 for (int b = 0; b < bn; ++b) {
                     ok = warp_all(mb_wait(&rempty[rst], rph, A.status, 8));
                     if (!ok) break;
-                    uint8_t* dst = raw_base + rst * L::RAW_STAGE + ((rw & 2) ? L::RAW_TILE : 0) + row0 * R::RS;
+                    uint8_t* dst = raw_base + rst * L::RAW_STAGE + (rw ? L::RAW_TILE : 0);
                     const uint32_t step = 4u * A.rb;
-                    const uint8_t* src = half + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
+                    const uint8_t* src = tile + (size_t)(lane >> 3) * A.rb + (size_t)(b0 + b) * kBB<T>;
                     uint8_t* d = dst + (lane >> 3) * R::RS + c16;
 #pragma unroll
-                    for (int i = 0; i < TILE_M / 8; ++i, src += step) {
+                    for (int i = 0; i < TILE_M / 4; ++i, src += step) {
                         if constexpr (T == T_Q4_K) {
                             cp_async16(d + i * 4 * R::RS, src + c16);
                         } else {
@@ -556,9 +560,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                         }
                     }
                     if constexpr (T == T_Q4_K) {
-                        const uint8_t* s9 = half + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
+                        const uint8_t* s9 = tile + (size_t)lane * A.rb + (size_t)(b0 + b) * kBB<T> + 128;
 #pragma unroll
-                        for (int i = 0; i < TILE_M / 64; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
+                        for (int i = 0; i < TILE_M / 32; ++i) cp_async16(dst + (lane + 32 * i) * R::RS + 128, s9 + (size_t)(32 * i) * A.rb);
                     }
                     cp_async_arrive(&rfull[rst]);
                     if (++rst == L::RSTAGES) { rst = 0; rph ^= 1u; }
@@ -567,84 +571,113 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         }
         cp_async_wait_all();
     } else {
-        reg_dec<K::REG_MISC>();
+        reg_dec<REG_COPY>();
         if (warp < W_MMA) {
-        // ---------------- B tiles: rows 2 t, 2 t + 1 = hi and lo of token t; lane = unit lane % 8 of row lane / 8 (+ 8 per step, the
-        // other warp takes the four between) ----------------
-        StageCount q(0);
-        const int brow = 4 * (warp - W_B) + (lane >> 3);
-        const uint32_t at = chunk_off(brow, lane & 7);  // rows r and r + 8 swizzle alike
+        // ---------------- B tiles: two warps the tokens' lo rows, two the hi rows; lane = unit lane % 8 of row lane / 8 (+ 8 per step, the
+        // half's other warp takes the four between) ----------------
+        const int hi = (warp - W_B) >> 1, brow = 4 * ((warp - W_B) & 1) + (lane >> 3);
+        const uint32_t at = hi * SLOTS * B_SLOT + chunk_off(brow, lane & 7);  // rows r and r + 8 swizzle alike
+        uint32_t turn = ~0u;  // parities of the pairs
+#pragma unroll 1
         for (int k = 0; k < my_items && ok; ++k) {
             const Item it = item(k);
-            const int steps = tile_tokens(it.m) / 4;  // 8 rows each
-            uint32_t src[NT / 4];  // operand array rows of this lane's B rows, in 16-byte units
+            const int steps = (it.m - 4 * ((warp - W_B) & 1) + 7) >> 3;  // columns of B behind the item's tokens may hold anything: nobody reads their sums
+            uint32_t src[NT / 8];  // operand array rows of this lane's B rows, in 16-byte units
 #pragma unroll
-            for (int i = 0; i < NT / 4; ++i) {
-                const int br = 8 * i + brow, pr = it.prow + min(br >> 1, it.m - 1);
+            for (int i = 0; i < NT / 8; ++i) {
+                const int pr = it.prow + min(8 * i + brow, it.m - 1);
                 const uint32_t orow = i < steps ? (uint32_t)(A.row_token ? A.row_token[pr] : pr) : 0u;
-                src[i] = (2u * orow + (br & 1)) * (uint32_t)(pitch >> 3) + (lane & 7);
+                src[i] = (2u * orow + 1u - hi) * (uint32_t)(pitch >> 3) + (lane & 7);
             }
-            auto stage = [&](int off) {  // off: elements from the row's start
-                ok = warp_all(NT == 64 ? q.wait(empty, A.status, 4) : mb_wait(&empty[q.q], q.turn ^ 1u, A.status, 4));
+            auto pair = [&](int off, int h, int stages, int next) {  // off: elements from the row's start; next: from one stage to the other
+                const uint32_t t = (turn >> h) & 1u;
+                ok = warp_all(mb_wait(&empty[hi * PAIRS + h], t, A.status, 4) && mb_wait(&empty[(2 + hi) * PAIRS + h], t, A.status, 4));
                 if (!ok) return;
-                uint8_t* d = b_ring + (NT == 64 ? q.slot() : q.q) * B_STAGE + at;
+                turn ^= 1u << h;
+                uint8_t* d = b_ring + 2 * h * B_SLOT + at;
                 const uint16_t* from = A.op + off;
 #pragma unroll
-                for (int i = 0; i < NT / 4; ++i)
-                    if (i < steps) cp_async16(d + i * 1024, from + (size_t)src[i] * 8);
-                cp_async_arrive(&full[q.q]);
-                q.advance(1);
+                for (int i = 0; i < NT / 8; ++i)
+                    if (i < steps) {
+                        const uint16_t* row = from + (size_t)src[i] * 8;
+                        cp_async16(d + i * 1024, row);
+                        if (stages > 1) cp_async16(d + B_SLOT + i * 1024, row + next);
+                    }
+                cp_async_arrive(&full[hi * PAIRS + h]);
+                cp_async_arrive(&full[(2 + hi) * PAIRS + h]);
             };
+#pragma unroll 1
             for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                 const int bn = min(8, nblk - b0);
+#pragma unroll 1
                 for (int b = 0; b < bn && ok; ++b) {
 #pragma unroll 1
-                    for (int c = 0; c < 4 && ok; ++c) stage((b0 + b) * 256 + c * BK);
+                    for (int h = 0; h < PAIRS && ok; ++h) pair((b0 + b) * 256 + h * 2 * BK, h, 2, BK);
                 }
-                const int sums = A.n_in + 8 * b0;  // the mins read the sums behind the row
-                for (int u = 0; u < min_stages<T>(bn) && ok; ++u) stage(sums);
+                if (T == T_Q4_K && ok) pair(A.n_in + 8 * b0, 0, min_stages<T>(bn), 0);  // the mins read the sums behind the row
             }
         }
         cp_async_wait_all();
-        } else if (warp == W_MMA && elect_one()) {
-            // ---------------- MMA issue: one thread ----------------
-            const uint32_t b_lo0 = desc_lo(s32(b_ring));
-            StageCount q(0);
+        } else if (elect_one()) {
+            // ---------------- MMA issue: a thread per tile ----------------
+            const int tile = warp - W_MMA;
+            const uint32_t b_lo0 = desc_lo(s32(b_ring)), d0 = tmem_base + (uint32_t)(tile * NT), ta0 = tmem_base + A_COL0 + (uint32_t)(tile * A_COLS);
+            uint32_t turn = 0u;  // parities
+            uint64_t *fu = full + tile * 2 * PAIRS, *em = empty + tile * 2 * PAIRS;
             int buf = 0;
             uint32_t pf = 1u;
+#pragma unroll 1
             for (int k = 0; k < my_items && ok; ++k) {
-                const int nte = tile_tokens(item(k).m);
-                const uint32_t idesc = (1u << 4) | ((uint32_t)((2 * nte) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
+                const uint32_t idesc = (1u << 4) | ((uint32_t)(tile_tokens(item(k).m) >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);  // fp16 x fp16 -> fp32
+                auto begin = [&]() { return mb_wait(&tfree[buf], pf, A.status, 6); };
+                auto end = [&]() {
+                    mma_commit(&tfull[buf]);
+                    if (++buf == NB) { buf = 0; pf ^= 1u; }
+                };
+                // two stages against the lo (p < PAIRS) or hi rows; acc: of the first K step
+                auto pair = [&](int p, uint32_t acc, auto mins, int steps, int hop) {
+                    ok = mb_wait(&fu[p], (turn >> p) & 1u, A.status, 5);
+                    if (!ok) return;
+                    turn ^= 1u << p;
+                    tc_fence_after();    // A: written to tensor memory by the producers
+                    fence_async_smem();  // B: written to shared memory by the B warps' copies
+                    const uint32_t d = d0 + (uint32_t)(buf * BUF_COLS);
+                    const uint32_t ta = ta0 + (uint32_t)((p % PAIRS) * 4 * A_COLS), b_lo = b_lo0 + (uint32_t)(p * (2 * B_SLOT >> 4));
+                    if constexpr (!decltype(mins)::value) {
+#pragma unroll
+                        for (int ks = 0; ks < 8; ++ks)
+                            mma_f16_ta(d, ta + (uint32_t)(ks >> 2) * 2 * A_COLS + 8u * (ks & 3), desc_of(b_lo + (uint32_t)(ks >> 2) * (B_SLOT >> 4) + 2u * (ks & 3)), idesc,
+                                       ks == 0 ? acc : 1u);
+                    } else {  // `steps` K steps of hi mins, then of lo mins: `hop` further on
+#pragma unroll 1
+                        for (int i = 0; i < 2 * steps; ++i) {
+                            const int ks = i < steps ? i : hop + i - steps;
+                            mma_f16_ta(d, ta + (uint32_t)(ks >> 2) * 2 * A_COLS + 8u * (ks & 3), desc_of(b_lo + (uint32_t)(ks >> 2) * (B_SLOT >> 4) + 2u * (ks & 3)), idesc,
+                                       i == 0 ? acc : 1u);
+                        }
+                    }
+                    mma_commit(&em[p]);
+                };
+#pragma unroll 1
                 for (int b0 = 0; b0 < nblk && ok; b0 += 8) {
                     const int bn = min(8, nblk - b0);
-                    for (int b = 0; b < bn + (T == T_Q4_K ? 1 : 0) && ok; ++b) {
-                        // a block's four stages; or those of the mins, whose K steps without sub-blocks are left out (hi and lo side
-                        // by side when both fit into one stage)
-                        const bool mins = b == bn, pair = mins && bn <= 4;
-                        const int stages = mins ? min_stages<T>(bn) : 4, live = mins ? (bn * 8 + 15) / 16 : 4;
-                        ok = mb_wait(&tfree[buf], pf, A.status, 6);
-                        const uint32_t d = tmem_base + (uint32_t)(buf * BUF_COLS);
-                        for (int c = 0; c < stages && ok; ++c) {
-                            ok = mb_wait(&full[q.q], q.turn, A.status, 5);
-                            if (!ok) break;
-                            tc_fence_after();    // A: written to tensor memory by the producers
-                            fence_async_smem();  // B: written to shared memory by the B warps' copies
-                            const uint32_t ta = tmem_base + A_COL0 + (uint32_t)(q.slot() * 2 * A_COLS), b_lo = b_lo0 + (uint32_t)((NT == 64 ? q.slot() : q.q) * (B_STAGE >> 4));
-                            uint32_t acc = c == 0 ? 0u : 1u;
-#pragma unroll
-                            for (int ks = 0; ks < 4; ++ks) {
-                                if ((pair ? ks & 1 : ks) >= live) continue;
-                                mma_f16_ta(d, ta + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
-                                mma_f16_ta(d + 2 * NT, ta + A_COLS + 8u * ks, desc_of(b_lo + 2u * ks), idesc, acc);
-                                acc = 1u;
-                            }
-                            mma_commit(&empty[q.q]);
-                            q.advance(1);
-                        }
+#pragma unroll 1
+                    for (int b = 0; b < bn && ok; ++b) {
+                        ok = begin();
                         if (!ok) break;
-                        mma_commit(&tfull[buf]);
-                        if (++buf == NB) { buf = 0; pf ^= 1u; }
+                        // everything against the lo rows, then against the hi rows: the hi sums are rounded as often as alone
+#pragma unroll 1
+                        for (int p = 0; p < 2 * PAIRS && ok; ++p)
+                            pair(p, p ? 1u : 0u, Int<0>(), 0, 0);
+                        if (ok) end();
                     }
+                    if (T != T_Q4_K || !ok) continue;
+                    // The mins: K steps without sub-blocks are left out (hi and lo side by side when both fit into one stage).
+                    const int steps = (bn * 8 + 15) / 16, hop = min_stages<T>(bn) == 1 ? 2 : 4;
+                    ok = begin();
+                    if (ok) pair(0, 0u, Int<1>(), steps, hop);
+                    if (ok) pair(PAIRS, 1u, Int<1>(), steps, hop);
+                    if (ok) end();
                 }
             }
         }
@@ -702,7 +735,7 @@ bool tc_handles(int type, int n_in, int n_out, bool fused) {
     return (type == T_Q4_K || type == T_IQ3_XXS) && n_in % 256 == 0 && n_out % (fused ? tg::TILE_M : 2 * tg::TILE_M) == 0;
 }
 
-template <int T, bool PAIR, int NT>
+template <int T, bool PAIR>
 static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
     using L = tg::Layout<T>;
     size_t at = kMmSmemBase + L::LOW + tg::B_BYTES;
@@ -710,7 +743,7 @@ static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
     const size_t smem = at + L::TAIL - kMmSmemBase;
     static_assert(L::BARS * 8 + 16 + (tg::kMaxSeg + 1) * 4 + 8 + tg::kLocalItems * sizeof(tg::Item) <= L::HEAD, "head too small");
     A.smem = (uint32_t)smem;
-    auto kern = tg::grouped_tc_kernel<T, PAIR, NT>;
+    auto kern = tg::grouped_tc_kernel<T, PAIR>;
     static SmemGrant grant;
     DNB_CUDA(grant_smem(grant, c->device, kern, smem));
     ProfScope prof_(c, st, PAIR ? "tc_down" : "tc_gate_up");
@@ -720,32 +753,15 @@ static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
 }
 
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
-                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst, int tokens, int rows) {
+                      int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst) {
     if (!tc_handles(type, n_in, n_out, fused) || nseg_max > tg::kMaxSeg) return DNB_DECLINED;
     int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
     if (rc) return rc;
     tg::Args A = {};
     A.seg = seg; A.nseg_dev = nseg_dev; A.nseg_max = nseg_max; A.n_in = n_in; A.n_out = n_out; A.rb = (int)row_bytes(type, n_in);
     A.op = op; A.row_token = row_token; A.out = out; A.row_dst = row_dst; A.status = c->status;
-    // Items of 64 tokens, or of 32.  Where no expert has more than 32 tokens, 64 save no decoding and cost a second accumulator and half of
-    // the B ring: 11 to 14 % of a layer (Q4_K), 5 to 8 % (IQ3_XXS); where experts have more, they gain up to 30 %.  That depends on how the
-    // tokens spread, which the host does not know.  With 40 rows a segment (IQ3_XXS: 24) 64 are the better choice either way; with fewer Q4_K
-    // stays at 32, while IQ3_XXS, which loses little where 64 do not help, takes them from 256 tokens on.  us a layer, 32 / 64 tokens an
-    // item, even routing, and skewed by -1.1 ln rank, 2048 x 512:
-    //   Q4_K, 512 experts top 10: 512 tokens (11 rows a segment) 431 / 493, 248 / 238; 1024 tokens (22) 490 / 558, 416 / 364
-    //         128 experts top 8: 384 tokens (27) 163 / 190, 181 / 179; 512 (36) 210 / 205, 211 / 197; 700 (49) 270 / 220, 256 / 238
-    //         64 experts top 10: 200 tokens (34) 139 / 132, 144 / 156; 1024 (173) 381 / 315, 381 / 317
-    //   IQ3_XXS, 512 experts top 10: 200 tokens 438 / 474, 166 / 151; 256 tokens 440 / 477, 176 / 160; 512 tokens 479 / 511, 275 / 238
-    //         128 experts top 8: 200 tokens (14) 166 / 177, 139 / 144; 384 (27) 179 / 191, 199 / 179; 512 (36) 234 / 201, 233 / 199
-    // Over six such shapes and 48 to 1024 tokens the rule is 0.1 % / 1.7 % (Q4_K, even / skewed) and 1.6 % / 1.0 % (IQ3_XXS) behind the better.
-    // (Tried: the choice on the device, from the segments' token counts.  Both kernels launched, one without items: 1.5 us each.  One
-    // kernel with both bodies, or with items of either size: 7 to 15 % slower, in registers and code.)
-    const bool q4 = type == T_Q4_K, wide = rows >= (q4 ? 40 : 24) * nseg_max || (!q4 && tokens >= 256);
-#define DNB_TC(TY, PAIR) return wide ? launch_tc_t<TY, PAIR, 64>(c, st, A) : launch_tc_t<TY, PAIR, 32>(c, st, A)
-    if (type == T_Q4_K) { if (fused) DNB_TC(T_Q4_K, false); DNB_TC(T_Q4_K, true); }
-    if (fused) DNB_TC(T_IQ3_XXS, false);
-    DNB_TC(T_IQ3_XXS, true);
-#undef DNB_TC
+    if (type == T_Q4_K) return fused ? launch_tc_t<T_Q4_K, false>(c, st, A) : launch_tc_t<T_Q4_K, true>(c, st, A);
+    return fused ? launch_tc_t<T_IQ3_XXS, false>(c, st, A) : launch_tc_t<T_IQ3_XXS, true>(c, st, A);
 }
 
 }  // namespace dnb

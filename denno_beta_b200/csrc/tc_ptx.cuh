@@ -30,8 +30,10 @@ __device__ __forceinline__ bool mb_try(uint64_t* b, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded: after 2^15 polls (half a second or so) the wait gives up, records `code` in the status word and returns false.
+// Bounded: after 2^15 polls (half a second or so) the wait gives up, records `code` in the status word and returns false.  Not unrolled: a
+// kernel has dozens of these, and instruction caches to fill.
 __device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, int* status, int code) {
+#pragma unroll 1
     for (int i = 0; i < (1 << 15); ++i)
         if (mb_try(b, parity)) return true;
     status_set(status, code);

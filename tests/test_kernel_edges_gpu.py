@@ -218,3 +218,34 @@ def test_activations_of_any_size(orc, ctx, name, nvec):
         tiny = k * 2.0 ** -149 * np.abs(deq).max() if i == 0 else 0.0
         bound = 2.0 ** -20 * np.sqrt((x[i, first:].astype(np.float64) ** 2) @ (deq ** 2).T) + 2.0 ** -28 * np.abs(x[i, first:]).max() * np.abs(deq).sum(1) + tiny
         assert np.all(np.abs(got[i, first:] - want) <= bound), (i, np.max(np.abs(got[i, first:] - want) / bound))
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "IQ3_XXS"])
+@pytest.mark.parametrize("k,n", [(256, 256), (1024, 512), (1280, 256), (2304, 256)])
+def test_tcgen05_items(orc, ctx, name, k, n):
+    """grouped_tc.cu: experts whose tokens end on either side of 16, 32, 48 and 64 columns (N of the MMAs, loads of the sums) and of a second
+    item, K of 1, 4, 5 and 9 blocks (the mins in one stage, in two, and a second time for the ninth).  Bound: an activation is 22 bits of its
+    row's largest, a block's sum is rounded 16 times in 24 bits, rows of K / 256 blocks are summed in fp32: 2e-6 of the result's rms each, and up
+    to 4 sigma of it over a row."""
+    from denno_beta_b200 import cuda as cu
+
+    ty, sizes = orc.TYPE_BY_NAME[name], (129, 128, 80, 65, 64, 63, 49, 48, 47, 33, 32, 31, 24, 17, 16, 15, 9, 8, 4, 1)
+    ne = len(sizes)
+    assert ctx.moe_config(1, k, n, ne, 1)
+    w = orc.synth_blocks(ty, SEED, 140 + ty, ne * n * k // orc.blck_size(ty))
+    assert ctx.register_experts(0, cu.GATE, ty, k, n, ne, w)
+    at = np.concatenate([[0], np.cumsum(sizes)])
+    segs = np.array([[ne - 1 - i, m, at[i], at[i]] for i, m in enumerate(sizes)], np.uint32)
+    x = orc.synth_normal(SEED, 141, 1.0, int(at[-1]) * k).reshape(-1, k)
+    x[5] *= 1e-6  # rows are scaled one by one
+    x[6] = 0.0
+    ctx.profile(True)
+    got = cu.moe_grouped_gemm_layer(ctx, 0, cu.GATE, segs, x, n)
+    launched = ctx.profile_read()
+    ctx.profile(False)
+    assert "tc_down" in launched, sorted(launched)
+    want = orc.grouped_gemm(ty, w, k, n, segs, x)
+    for i, m in enumerate(sizes):
+        rows = slice(at[i] + (7 if i == 0 else 0), at[i + 1])
+        assert rel_err(got[rows], want[rows]) <= 2e-5, m
+    assert rel_err(got[5:6], want[5:6]) <= 2e-5 and not got[6].any()
