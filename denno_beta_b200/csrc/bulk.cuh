@@ -31,8 +31,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: gives up after ~2^22 polls (tens of milliseconds), records the
-// failure in *status and reports false; the caller then skips its math.
+// failure in *status and reports false; the caller then skips its math.  Not unrolled: code has to be fetched.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* status) {
+#pragma unroll 1
     for (int i = 0; i < (1 << 22); ++i)
         if (mbar_try_wait(bar, parity)) return true;
     status_set(status, 1);

@@ -7,6 +7,10 @@
 //                    softmax / top-k / renorm (every CTA ranks the logits itself), then
 //                    the half above -- one launch per block, no table in global memory
 //
+// Code: a CTA runs through nearly all of it once, so what it fetches of it is on the critical path.  Waiting loops, and loops of one or two
+// turns, that the compiler had unrolled made 89 KB of it, now 70: a stack of ten such layers and two of Q4_K 280 -> 274 us.  The sub-blocks of
+// the K loops stay unrolled by four (one, two and eight: 282, 278 and 280).
+//
 // Why one kernel: with two, the down kernel's CTAs cannot all be resident beside the
 // gate/up kernel (registers, shared memory), so a good part of the down weights is
 // requested only after gate/up has ended and their arrival (~1 us) plus the launch
@@ -138,6 +142,7 @@ __device__ __forceinline__ bool grid_barrier(const FusedArgs& A, bool wait) {
     if (!wait) return false;
     const unsigned long long target = (ticket / gridDim.x + 1ull) * gridDim.x + A.barrier_bias;
     bool pass = ticket + 1ull == target;
+#pragma unroll 1
     for (int i = 0; i < A.barrier_polls && !pass; ++i) pass = ld_acquire_u64(A.gbar) >= target;  // ~0.2 s at most by default
     if (!pass) status_set(A.status, 23);
     return pass;
@@ -240,6 +245,7 @@ __global__ void __maxnreg__(ROUTED ? 80 : 64) decode_fused_kernel(const FusedArg
         {
             // every thread evaluates the same expression on the same four partial sums: no broadcast, no second barrier
             const float inv = A.norm_w ? 1.0f / sqrtf(((R->red[0] + R->red[1]) + (R->red[2] + R->red[3])) / (float)e + A.eps) : 1.0f;
+#pragma unroll 1
             for (int i = 2 * tid; i < e; i += 2 * kFdThreads) {
                 float2 v = *reinterpret_cast<const float2*>(hbuf + i);
                 if (A.norm_w) {
@@ -457,6 +463,7 @@ __global__ void __maxnreg__(ROUTED ? 80 : 64) decode_fused_kernel(const FusedArg
             const uint16_t* xb = acts + ((size_t)((which ? sb : sa) * kGmSplit + (n < kGmSplit ? n : 0))) * arow + 8 * t;
             const int nblk = ff >> 8, b0 = kh * (nblk >> 1), b1 = b0 + (nblk >> 1);
             float acc = 0.f;
+#pragma unroll 1
             for (int b = b0; b < b1; ++b)
                 iq3_block_mma(
                     ra + b * 98, rbp + b * 98, t, lutp,

@@ -151,6 +151,7 @@ __device__ __forceinline__ void split3(float v, uint32_t (&h)[kGmSplit]) {
 __device__ __forceinline__ void gate_up_warp(const uint8_t* rowg, const uint8_t* rowu, const Iq3Lane& lutp,
                                              const uint16_t* xb, bool has_col, int b0, int b1, int t, float& accg,
                                              float& accu) {
+#pragma unroll 1
     for (int b = b0; b < b1; ++b)
         iq3_block_mma(
             rowg + b * 98, rowu + b * 98, t, lutp,

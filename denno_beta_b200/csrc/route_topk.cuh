@@ -184,9 +184,11 @@ __device__ __forceinline__ void route_topk(RouteSmem& R, const float* __restrict
         // only when it is the first unused entry.
         if (warp == 0) {
             uint32_t used = 0u;  // bit m: entry 32 m + lane
+#pragma unroll 1
             for (int round = 0; round < k; ++round) {
                 float best = -INFINITY;
                 int best_i = 0x7fffffff, first = 0x7fffffff;
+#pragma unroll 1
                 for (int m = 0; 32 * m + lane < ne; ++m) {
                     if ((used >> m) & 1u) continue;
                     const int idx = 32 * m + lane;
