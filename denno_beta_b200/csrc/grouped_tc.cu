@@ -5,7 +5,7 @@
 // kernels_exp_iq_tc.cu (bf16 wmma); block layouts kquant.rs:505-526, :659-680.
 //
 //     W . x  =  sum over 256-element blocks b of  s_b * [ sum_i w_i * x_i ]   ( - sum over sub-blocks of (dmin * m) * X )
-//   Q4_K    : w = sc * q <= 945, s_b = d, and the mins: X = the sum of the sub-block's 32 activations
+//   Q4_K    : w = sc * q <= 945 (times 2^-14, which s_b takes back), s_b = d, and the mins: X = the sum of the sub-block's 32 activations
 //   IQ3_XXS : w = codebook magnitude * sign * (2 s + 1) <= 1922, s_b = d / 4
 // Every w is an integer below 2048 and exact in fp16, so a weight costs its decoding and nothing is rounded.  The mins are one
 // more block of K = sub-blocks: A = -(dmin * m) as fp16 hi and lo, times a power of two of the row's own that fits its largest
@@ -37,7 +37,8 @@
 // below); one copy of the decoding instead of two, and one of the MMA loop, 493 -> 434.
 //
 // Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, two layers, us a pass: items of 32 (Q4_K) or 64 tokens with hi and lo
-// sums apart -> these: Q4_K 501 -> 409, IQ3_XXS 473 -> 429; a prompt of 14,018 tokens 6,865 -> 5,684.
+// sums apart -> these -> the shared expert's items first, nibbles as numbers below the normal ones, 32 copies of the signs: Q4_K 501 -> 409 -> 384,
+// IQ3_XXS 473 -> 429 -> 421; a prompt of 14,018 tokens 6,865 -> 5,684 -> 5,300.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -86,9 +87,13 @@ struct Item {
 };
 
 template <bool PAIR>
-__device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int nseg, const int* pre, const SegDesc* __restrict__ seg) {
-    const int tile = item / row_tiles, rt = item - tile * row_tiles;
+__device__ __forceinline__ Item decode_item(int item, int row_tiles, int rb, int nseg, int first, const int* pre, const SegDesc* __restrict__ seg) {
+    int tile = item / row_tiles;
+    const int rt = item - tile * row_tiles;
+    tile += first;
+    if (tile >= pre[nseg]) tile -= pre[nseg];
     int lo = 0, hi = nseg;  // pre[lo] <= tile < pre[lo + 1]
+#pragma unroll 1
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (pre[mid] <= tile) lo = mid; else hi = mid;
@@ -142,7 +147,7 @@ template <> struct Raw<T_Q4_K> {
         a = *reinterpret_cast<const uint4*>(p + 16 + 32 * c);
         b = *reinterpret_cast<const uint4*>(p + 32 + 32 * c);
     }
-    __device__ __forceinline__ float scale() const { return h2f((uint16_t)h.x); }
+    __device__ __forceinline__ float scale() const { return 16384.0f * h2f((uint16_t)h.x); }  // the weights are 2^-14 of theirs
 };
 template <> struct Raw<T_IQ3_XXS> {  // 16 index bytes and two sub-block words from the aligned words around them
     static constexpr int UNITS = 7, RS = 112;
@@ -196,10 +201,8 @@ __device__ __forceinline__ void decode_stage(const Raw<T_Q4_K>& R, int c, uint32
     const uint32_t a = R.h.y >> sh, cc = R.h.w >> sh;
     const uint32_t sc = c < 2 ? (a & 0x3f3fu) : ((cc & 0x0f0fu) | ((a >> 2) & 0x3030u));  // kquant.rs:878-887
     KScales s;
-    s.s0 = h2sub(__byte_perm(sc, 0x64646464u, 0x4040u), 0x64006400u);
-    s.s1 = h2sub(__byte_perm(sc, 0x64646464u, 0x4141u), 0x64006400u);
-    s.k0 = h2mul(s.s0, 0xE400E400u);
-    s.k1 = h2mul(s.s1, 0xD400D400u);
+    s.s0 = h2mul(h2sub(__byte_perm(sc, 0x64646464u, 0x4040u), 0x64006400u), 0x64006400u);
+    s.s1 = h2mul(h2sub(__byte_perm(sc, 0x64646464u, 0x4141u), 0x64006400u), 0x54005400u);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const uint4 q = h ? R.b : R.a;
@@ -222,7 +225,7 @@ __device__ __forceinline__ void decode_stage(const Raw<T_IQ3_XXS>& R, int, uint3
         for (int q = 0; q < 4; ++q) {
             const uint32_t iw = __funnelshift_r(R.i[2 * hb + (q >> 1)], R.i[2 * hb + (q >> 1) + 1], R.sh) >> (16 * (q & 1));
             uint32_t p[4];
-            iq3_pairs_h(gl, sl, iw, q == 0 ? aux << 6 : aux >> (7 * q - 6), p);
+            iq3_pairs_h(gl, sl, iw, q == 0 ? aux << 7 : aux >> (7 * q - 7), p);
 #pragma unroll
             for (int j = 0; j < 4; ++j) o[16 * hb + 4 * q + j] = h2mul(p[j], s2);
         }
@@ -345,12 +348,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const int n_items = nseg > 0 ? pre[nseg] * row_tiles : 0;
+    // The segments come by descending tokens, but for the shared expert's, which is the last: the largest has to be dealt first, not into the
+    // last round of items.
+    const int first = nseg > 1 && A.seg[nseg - 1].m > A.seg[0].m ? pre[nseg - 1] : 0;
     const int GR = gridDim.x;
     const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + GR - 1) / GR : 0;
-    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, pre, A.seg);
+    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, first, pre, A.seg);
     __syncthreads();
     auto item = [&](int k) {
-        return k < kLocalItems ? itab[k] : decode_item<PAIR>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, pre, A.seg);
+        return k < kLocalItems ? itab[k] : decode_item<PAIR>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, first, pre, A.seg);
     };
     bool ok = true;
 
@@ -448,7 +454,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         reg_dec<REG_PROD>();
         const int pw = warp - EWARPS, odd = pw >> 3, tile = (pw >> 2) & 1, r = (pw & 3) * 32 + lane;
         const uint32_t tlane = tmem_base + A_COL0 + (uint32_t)(tile * A_COLS) + ((uint32_t)((pw & 3) * 32) << 16);
-        const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * (lane & (kLutRep - 1));
+        const uint32_t gl = s32(book) + 8 * (lane & (kLutRep - 1)), sl = s32(book) + (uint32_t)sizeof(uint2) * 256 * kLutRep + 4 * lane;
         uint2* mm = reinterpret_cast<uint2*>(raw_base + L::RSTAGES * L::RAW_STAGE) + pw * 32 + lane;
         uint16_t* dd = reinterpret_cast<uint16_t*>(raw_base + L::RSTAGES * L::RAW_STAGE + PWARPS * 32 * 8 * 8) + pw * 32 + lane;
         int rst = 0, sc = 0;

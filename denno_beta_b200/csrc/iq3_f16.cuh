@@ -8,25 +8,27 @@
 
 namespace dnb {
 
-// Q4_K: the scales of two sub-blocks.  s0 / s1: of the even / odd one in both halves, k0 / k1: -1024 * s0 and -64 * s1.
-struct KScales { uint32_t s0, s1, k0, k1; };
-// A word of packed bytes: low nibbles are the even sub-block, high nibbles the odd one.
+// Q4_K: the scales of two sub-blocks in both halves, 2^10 sc of the even one (64,512 at most), 2^6 sc of the odd one.
+struct KScales { uint32_t s0, s1; };
+// A word of packed bytes as 2^-14 sc * q: low nibbles are the even sub-block, high nibbles the odd one.  A nibble where it lies is the fp16
+// number 2^-24 q or 2^-20 q below the normal ones, which multiplies like any other, and the product is exact and normal: a mask and a
+// multiplication a pair.  (As 1024 + q and 64 + q, with a multiply-add, the mask and the exponent took two logic instructions, for want of
+// registers for the constants: 58.8 M warp instructions of a launch -> 53.2 M.)
 __device__ __forceinline__ void k_word(uint32_t w, const KScales& s, uint32_t (&p)[4]) {
     const uint32_t w8 = w >> 8;
-    const uint32_t a = (w & 0x000f000fu) | 0x64006400u, b = (w8 & 0x000f000fu) | 0x64006400u;    // 1024 + q
-    const uint32_t c = (w & 0x00f000f0u) | 0x54005400u, d = (w8 & 0x00f000f0u) | 0x54005400u;    // 64 + q
-    p[0] = h2fma(a, s.s0, s.k0);
-    p[1] = h2fma(b, s.s0, s.k0);
-    p[2] = h2fma(c, s.s1, s.k1);
-    p[3] = h2fma(d, s.s1, s.k1);
+    p[0] = h2mul(w & 0x000f000fu, s.s0);
+    p[1] = h2mul(w8 & 0x000f000fu, s.s0);
+    p[2] = h2mul(w & 0x00f000f0u, s.s1);
+    p[3] = h2mul(w8 & 0x00f000f0u, s.s1);
 }
 
 // IQ3_XXS tables in shared memory, kLutRep copies each (a lane reads copy lane % kLutRep: no bank conflicts).
 //   grid: the codebook as fp16 pairs, 128 bytes from entry to entry
-//   sgn : the eight signs of a 7-bit code (the eighth makes their number even): pair q of the eight weights at bits 15 - q and
+//   sgn : the eight signs of a 7-bit code (the eighth makes their number even), 32 copies (half as many and two lanes of most reads meet on
+//         a bank: a chunk of 512 tokens 426 -> 421 us): pair q of the eight weights at bits 15 - q and
 //         31 - q, so that a shift by q and a mask give the sign bits of a pair
 // The tables sit on a 32 KB boundary of the shared-memory address space: an entry's address is a shift and one and-or.
-struct MmCodebook { uint2 grid[256 * kLutRep]; uint32_t sgn[128 * kLutRep]; };
+struct MmCodebook { uint2 grid[256 * kLutRep]; uint32_t sgn[128 * 32]; };
 constexpr uint32_t kMmBookAlign = 32768;
 constexpr uint32_t kMmSmemBase = 1024;  // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
 static __device__ __align__(16) MmCodebook g_mm_codebook;
@@ -45,7 +47,7 @@ static int upload_mm_tables(int device) {
         const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
         uint32_t u = 0;
         for (int q = 0; q < 4; ++q) u |= ((sg >> (2 * q)) & 1u) << (15 - q) | ((sg >> (2 * q + 1)) & 1u) << (31 - q);
-        for (int r = 0; r < kLutRep; ++r) tb.sgn[code * kLutRep + r] = u;
+        for (int r = 0; r < 32; ++r) tb.sgn[code * 32 + r] = u;
     }
     DNB_CUDA(cudaMemcpyToSymbol(g_mm_codebook, &tb, sizeof(tb)));
     g_mm_tables[device] = true;
@@ -53,10 +55,10 @@ static int upload_mm_tables(int device) {
 }
 
 // Eight weights of an IQ3_XXS sub-block as four signed fp16 pairs.  gl, sl: shared addresses of the lane's copies; idx: the two
-// codebook indices; code: the sub-block word rotated so that the quarter's 7-bit sign code starts at bit 6.
+// codebook indices; code: the sub-block word rotated so that the quarter's 7-bit sign code starts at bit 7.
 __device__ __forceinline__ void iq3_pairs_h(uint32_t gl, uint32_t sl, uint32_t idx, uint32_t code, uint32_t (&p)[4]) {
     uint32_t u, g0, g1, g2, g3;
-    asm("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"((code & 0x1fc0u) | sl));  // constant tables: plain asm, free to move
+    asm("ld.shared.u32 %0, [%1];" : "=r"(u) : "r"((code & 0x3f80u) | sl));  // constant tables: plain asm, free to move
     asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(g0), "=r"(g1) : "r"(((idx << 7) & 0x7f80u) | gl));
     asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(g2), "=r"(g3) : "r"(((idx >> 1) & 0x7f80u) | gl));
     p[0] = g0 ^ (u & 0x80008000u);

@@ -3,8 +3,8 @@
 
 * Q4_K with integer weights (csrc/grouped_tc.cu): w = d * sc * q - dmin * m (kquant.rs:505-526), so
   W . x = sum_blocks d * [sum (sc * q) * x] - sum_subblocks (dmin * m) * X with X the sub-block sums of x;
-  sc * q <= 945 is exact in fp16 and one fp16 fma (1024 + q) * sc - 1024 * sc produces it; -(dmin * m) times a power of
-  two of the row is exact as fp16 hi + lo.
+  sc * q <= 945 is exact in fp16, and so is 2^-14 sc * q, the fp16 product of a nibble's bits (2^-24 q or 2^-20 q) and 2^10 sc or 2^6 sc;
+  -(dmin * m) times a power of two of the row is exact as fp16 hi + lo.
 * IQ3_XXS with exact weights: w = d / 4 * (grid magnitude) * sign * (2 s + 1), the product of the last three an integer exact
   in fp16 (csrc/grouped_tc.cu); the magnitude alone exact in bf16 (csrc/iq3_mma.cuh) and a signed byte (csrc/grouped_mma.cu).
 * Activations of those kernels: a row times a power of two as two fp16 numbers (csrc/operand_rows.cuh), three for the
@@ -97,6 +97,13 @@ def test_q4k_integer_weight_decomposition(orc):
     assert np.array_equal(c.astype(np.float64), -1024.0 * sc)   # six bits times 2^10: exact
     fma = (big.astype(np.float64) * sc[:, :, None] + c.astype(np.float64)[:, :, None]).astype(np.float16)  # rounds once
     assert np.array_equal(fma.astype(np.int64), iw)
+    # the same times 2^-14, without a constant to add: the bits of a nibble as a number below the normal ones, times a power of two of sc
+    for shift in (0, 4):
+        bits = (q.reshape(-1, 8, 32) << shift).astype(np.uint16).view(np.float16)
+        by = (2.0 ** (10 - shift) * sc).astype(np.float16)
+        assert np.array_equal(by.astype(np.float64), 2.0 ** (10 - shift) * sc)
+        prod = bits * by[:, :, None]  # fp16 x fp16, rounded once
+        assert np.array_equal(prod.astype(np.float64) * 2.0 ** 14, iw) and np.all((prod == 0) | (prod >= 2.0 ** -14))
     # (2) -(dmin * m) times the row's power of two is exact as fp16 hi + lo
     v = -(dmin[:, None].astype(np.float64) * m)
     hi, lo, scale = _mins_operand(dmin.astype(np.float16), m)
