@@ -38,7 +38,7 @@
 //
 // Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, two layers, us a pass: items of 32 (Q4_K) or 64 tokens with hi and lo
 // sums apart -> these -> the shared expert's items first, nibbles as numbers below the normal ones, 32 copies of the signs: Q4_K 501 -> 409 -> 384,
-// IQ3_XXS 473 -> 429 -> 421; a prompt of 14,018 tokens 6,865 -> 5,684 -> 5,300.
+// IQ3_XXS 473 -> 429 -> 421; a prompt of 14,018 tokens 6,865 -> 5,684 -> 5,330.
 #include <cuda_fp16.h>
 
 #include <type_traits>

@@ -249,3 +249,16 @@ def test_tcgen05_items(orc, ctx, name, k, n):
         rows = slice(at[i] + (7 if i == 0 else 0), at[i + 1])
         assert rel_err(got[rows], want[rows]) <= 2e-5, m
     assert rel_err(got[5:6], want[5:6]) <= 2e-5 and not got[6].any()
+
+
+@pytest.mark.parametrize("k", [1, 8, 9, 12, 13, 25])
+@pytest.mark.parametrize("nt", [5, 300])
+def test_combine_slots(orc, ctx, k, nt):
+    """combine_kernel: slots around the eight (large grids) and twelve (small ones) that are requested together, with a shared expert, its
+    gate row and the residual of a block."""
+    e, ff, ne = 256, 256, 32
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.Q4_K, e, ff, ne, k, bias=True, gate_row=True)
+    h = orc.synth_normal(SEED, 160 + nt, 1.0, nt * e).reshape(nt, e)
+    out, sels, wts = ctx.moe_block(0, h, want_routing=True)
+    assert check_block(orc, L, h, out, sels, wts)[0] <= (5e-5 if nt < 16 else 2e-4)
