@@ -40,7 +40,7 @@ def test_config0_other_formats_4096(orc, name):
 
 @pytest.mark.parametrize("ty_name,seam", [("Q4_K", 32), ("IQ3_XXS", 64)])
 def test_config2_every_token(orc, ty_name, seam):
-    """Config 2 (Q4_K: 32-token tiles of the tcgen05 kernel) and the same chunk with IQ3_XXS experts (64-token tiles):
+    """Config 2 (Q4_K) and the same chunk with IQ3_XXS experts on the tcgen05 kernel (items of 64 tokens; 32 is inside one):
     every token against the fp32 kernels, a sample that covers the hottest expert's tile seams against the oracle."""
     from denno_beta_b200 import cuda as cu
 

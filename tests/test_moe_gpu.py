@@ -42,7 +42,7 @@ def test_block_small(orc, small, layer, nt):
 def test_batch_equals_token_by_token(orc, small):
     """qwen4exp.rs:28259 (batch prefill == sequential).  A token's routing never depends
     on its neighbours; its values agree across chunk sizes and kernel families (one-token
-    decode kernels, mma.sync grouped kernel with three or two parts per activation, tcgen05
+    decode kernels, mma.sync grouped kernel, tcgen05
     grouped GEMM) to rounding, and are bit-identical when the same kernels run (any batch
     composition)."""
     c, layers = small
@@ -99,7 +99,7 @@ def test_tcgen05_grouped_gemm_matches_fp32_kernels(orc, small):
 
 def test_exact_weight_tcgen05_kernel_matches_fp32_kernels(orc, small):
     """IQ3_XXS chunks and decode batches from the threshold up (lowered to 2 here): exact integer fp16 weights on the tensor cores, block
-    scales applied by the epilogue.  Ragged sizes cover one and several 32-token tiles per expert and tiles with one token;
+    scales applied by the epilogue.  Ragged sizes cover one and several items per expert and tiles with one token;
     a batch's rows do not depend on their companions."""
     c, layers = small
     L = layers[0]
