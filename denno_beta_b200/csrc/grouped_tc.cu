@@ -38,7 +38,7 @@
 //
 // Measured, 512 tokens of 2048 x 512, top 10 of 512 under a skewed router, two layers, us a pass: items of 32 (Q4_K) or 64 tokens with hi and lo
 // sums apart -> these -> the shared expert's items first, nibbles as numbers below the normal ones, 32 copies of the signs: Q4_K 501 -> 409 -> 384,
-// IQ3_XXS 473 -> 429 -> 421; a prompt of 14,018 tokens 6,865 -> 5,684 -> 5,330.
+// IQ3_XXS 473 -> 429 -> 421; a prompt of 14,018 tokens 6,865 -> 5,684 -> 5,285; the last round dealt backwards: 381, 416 and 5,216.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -352,8 +352,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
     // last round of items.
     const int first = nseg > 1 && A.seg[nseg - 1].m > A.seg[0].m ? pre[nseg - 1] : 0;
     const int GR = gridDim.x;
-    const int my_items = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + GR - 1) / GR : 0;
-    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR>((int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, first, pre, A.seg);
+    // Items are dealt round by round, the last round backwards, so that the CTAs that get one more are those that had the smaller ones: 1.4 % of
+    // the passes below.  (Beyond the table, where a round is one of forty, straight on: what it took to know the last one there cost registers and
+    // more than it gave, Q4_K 383 -> 412 us.)
+    const int last = (n_items + GR - 1) / GR - 1, tail = last * GR + GR - 1 - (int)blockIdx.x;
+    const bool back = last < kLocalItems;
+    const int my_items = back ? last + (tail < n_items ? 1 : 0) : (n_items - (int)blockIdx.x + GR - 1) / GR;
+    if (tid < min(my_items, kLocalItems)) itab[tid] = decode_item<PAIR>(back && tid == last ? tail : (int)blockIdx.x + tid * GR, row_tiles, A.rb, nseg, first, pre, A.seg);
     __syncthreads();
     auto item = [&](int k) {
         return k < kLocalItems ? itab[k] : decode_item<PAIR>((int)blockIdx.x + k * GR, row_tiles, A.rb, nseg, first, pre, A.seg);

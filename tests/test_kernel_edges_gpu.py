@@ -46,8 +46,8 @@ def test_grouped_mma(orc, ctx, name, k, n):
 @pytest.mark.parametrize("name", ["Q4_K", "IQ3_XXS"])
 @pytest.mark.parametrize("e,ff,ne,k", [(256, 256, 8, 2), (768, 512, 16, 3), (2304, 256, 4, 1), (512, 1280, 24, 4)])
 def test_block_between_kernels(orc, ctx, name, e, ff, ne, k):
-    """Token counts on both sides of every hand-over (routing in two launches to 15, tensor-core router from 16, tcgen05 from 48, its
-    64-token items with 24 or 32 rows an expert or from 256 or 640 tokens), with experts of one token to several full tiles; K of 1 to 9
+    """Token counts on both sides of every hand-over (routing in two launches to 15, tensor-core router from 16, tcgen05 from 48),
+    with experts of one token to several full tiles; K of 1 to 9
     blocks.  From 48 tokens on a token's bits do not depend on the size of its chunk."""
     assert ctx.moe_config(1, e, ff, ne, k)
     L = make_layer(orc, ctx, 0, orc.TYPE_BY_NAME[name], e, ff, ne, k, bias=True, gate_row=True)
@@ -262,3 +262,22 @@ def test_combine_slots(orc, ctx, k, nt):
     h = orc.synth_normal(SEED, 160 + nt, 1.0, nt * e).reshape(nt, e)
     out, sels, wts = ctx.moe_block(0, h, want_routing=True)
     assert check_block(orc, L, h, out, sels, wts)[0] <= (5e-5 if nt < 16 else 2e-4)
+
+
+@pytest.mark.parametrize("name,segments", [("Q4_K", 48), ("IQ3_XXS", 47)])
+def test_tcgen05_many_items(orc, ctx, name, segments):
+    """grouped_tc.cu: more items than a CTA has in its table (40 on 148 SMs), in a last round that is full or not; the same experts in turn."""
+    from denno_beta_b200 import cuda as cu
+
+    ty, k, n, m = orc.TYPE_BY_NAME[name], 256, 32768, 4
+    assert ctx.moe_config(1, k, n, 2, 1)
+    w = orc.synth_blocks(ty, SEED, 150 + ty, 2 * n * k // orc.blck_size(ty))
+    assert ctx.register_experts(0, cu.GATE, ty, k, n, 2, w)
+    segs = np.array([[i % 2, m, i * m, i * m] for i in range(segments)], np.uint32)
+    x = orc.synth_normal(SEED, 151, 1.0, segments * m * k).reshape(-1, k)
+    ctx.profile(True)
+    got = cu.moe_grouped_gemm_layer(ctx, 0, cu.GATE, segs, x, n)
+    launched = ctx.profile_read()
+    ctx.profile(False)
+    assert "tc_down" in launched, sorted(launched)
+    assert rel_err(got, orc.grouped_gemm(ty, w, k, n, segs, x)) <= 2e-5
