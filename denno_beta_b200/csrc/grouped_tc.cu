@@ -70,7 +70,8 @@ constexpr int B_SLOT = NT * BK * 2, B_BYTES = 2 * SLOTS * B_SLOT;  // lo rows, t
 // Registers per thread of the warpgroups once their roles are known; launched with 64, and no more than that in sum.
 constexpr int REG_EPI = 112, REG_PROD = 56, REG_COPY = 32;
 static_assert(2 * REG_EPI + 4 * REG_PROD + 2 * REG_COPY <= 8 * 64, "register split");
-static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS + BWARPS == 6 && W_MMA == 30, "roles fill warpgroups");
+static_assert(EWARPS % 4 == 0 && W_RAW % 4 == 0 && (W_MMA + 2) * 32 == NTHREADS, "a register split falls between warpgroups");
+static_assert(EWARPS == 8 && PWARPS == 16 && RWARPS == 2 && BWARPS == 4, "what the roles' index arithmetic and the register split are written for");
 constexpr int kMaxSeg = 1055;
 constexpr int kLocalItems = 40;
 constexpr int A_COL0 = NB * BUF_COLS, TMEM_COLS = A_COL0 + SLOTS * 2 * A_COLS;
@@ -540,8 +541,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
                 }
             }
         }
-    } else if (warp < W_B) {
-        reg_dec<REG_COPY>();
+    } else {
+        reg_dec<REG_COPY>();  // one instruction for both warpgroups, above the roles: all warps of a warpgroup execute the same setmaxnreg
+        if (warp < W_B) {
         // ---------------- raw rows, a tile per warp: lane = unit lane % 8 of row lane / 8 (+ 4 per step); Q4_K: the ninth units afterwards ----------------
         const int rw = warp - W_RAW, c16 = (lane & 7) * 16;
         int rst = 0;
@@ -581,9 +583,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
             }
         }
         cp_async_wait_all();
-    } else {
-        reg_dec<REG_COPY>();
-        if (warp < W_MMA) {
+        } else if (warp < W_MMA) {
         // ---------------- B tiles: two warps the tokens' lo rows, two the hi rows; lane = unit lane % 8 of row lane / 8 (+ 8 per step, the
         // half's other warp takes the four between) ----------------
         const int hi = (warp - W_B) >> 1, brow = 4 * ((warp - W_B) & 1) + (lane >> 3);

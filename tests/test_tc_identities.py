@@ -11,6 +11,9 @@
   sub-block sums of csrc/grouped_mma.cu, whose activations are four digits in base 256 of a block; its integer sums fit.
 * Router operands (csrc/router_tc.cu): an fp32 value is the exact sum of three bf16 numbers (round, round, round).
 """
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -204,3 +207,23 @@ def test_integer_block_sums_fit(orc):
     assert np.array_equal(byte.astype(np.uint8).view(np.int8).astype(int), 4 * (q.astype(int) - 32))
     v = np.arange(4, 63, dtype=np.uint32)                                                  # IQ3_XXS: a negative byte is ~v + 1
     assert np.array_equal(((v ^ 255) + 1).astype(np.uint8).view(np.int8).astype(int), -v.astype(int))
+
+
+def test_register_splits_fall_between_warpgroups():
+    """csrc/grouped_tc.cu: setmaxnreg stands directly behind a condition on the warp's number that is the same for all four warps of a
+    warpgroup, as PTX asks of it."""
+    import denno_beta_b200
+
+    with open(os.path.join(os.path.dirname(denno_beta_b200.__file__), "csrc", "grouped_tc.cu")) as f:
+        src = f.read()
+    value = {}
+    for line in re.findall(r"^constexpr int ([A-Z_]+ = .*?);", src, re.M):
+        for name, expr in re.findall(r"([A-Z_]+) = ([^,]+)", line):
+            if re.fullmatch(r"[A-Z_0-9 +*]+", expr):
+                value[name] = eval(expr, {}, value)
+    calls = len(re.findall(r"^\s*reg_(?:inc|dec)<", src, re.M))
+    sites = re.findall(r"if \(warp < ([A-Z_]+)\) \{\s*(?://[^\n]*\n\s*)*reg_(?:inc|dec)<", src)
+    last = len(re.findall(r"\} else \{\s*(?://[^\n]*\n\s*)*reg_(?:inc|dec)<", src))
+    assert calls >= 3 and last <= 1 and len(sites) + last == calls
+    assert [value[s] for s in sites] == sorted(value[s] for s in sites)
+    assert all(value[s] % 4 == 0 for s in sites), [(s, value[s]) for s in sites]
