@@ -12,8 +12,9 @@
 //   * the integer scales multiply the integer sums of a sub-block (Q4_K, Q5_K: sc, IQ3_XXS: 2 s + 1, 32 elements; Q6_K: 16 elements) and
 //     add up over a 256-element block without rounding; d then multiplies in fp32.  (Q8_0 has a d per 32 elements.)  The mins of Q4_K
 //     and Q5_K are one fp16 K step of m against the sub-block sums of the activations;
-//   * an activation is an integer of 31 bits, of its 256-element block times a power of two, as four digits in base 256 in
-//     four columns of B: 2^-31 of the block's largest.
+//   * an activation is an integer of 32 bits, of its 256-element block times a power of two, as four digits in base 256 in
+//     four columns of B: rounded to 2^-31 of the block's largest.  Where that could be felt, in a block whose elements are of very
+//     different size, what is left over is one more digit, of one more column tile.
 // Why bytes: the logic and byte-permute instructions, fp16x2 and integer multiplies take two issue cycles of a scheduler here (FFMA and
 // integer adds one), and an mma.sync of bytes (K = 32) eight, as one of fp16 (K = 16) does.  With fp16 weights a Q4_K weight pair was 2.3
 // logic instructions and one fp16x2 multiply, now 0.6; 16 weights of an IQ3_XXS lane 34, now 25, and 12 instead of 18 shared-memory wavefronts.
@@ -30,7 +31,7 @@
 // 115 + 68 -> 108 + 66 -> 101 + 62, Q4_K 98 + 56 -> 75 + 45 -> 71 + 42, Q8_0 151 + 92 -> 134 + 74 -> 111 + 64; 200 tokens under a skewed router: Q4_K
 // and Q6_K 302 + 175 -> 263 + 119 -> 154 + 120, Q8_0 395 + 169 -> 249 + 135 -> 176 + 103.  (One loop with unused column tiles switched off took the
 // time of all of them, or not, as the compiler chose.)  Decoding alone is 30 (Q4_K) to 66 (IQ3_XXS) cycles of a scheduler for 16 rows x 32
-// elements; bytes from HBM take 50 and 34.  Distance from the 64-bit result, five formats, normal and heavy-tailed inputs: 0.43 of what it was.
+// elements; bytes from HBM take 50 and 34.  Distance from the 64-bit result: see mm_stage_block.
 #include <algorithm>
 #include <type_traits>
 
@@ -44,7 +45,7 @@ namespace dnb {
 constexpr int kMmWarps = 16;
 constexpr int kMmThreads = kMmWarps * 32;
 constexpr int kMmSegMax = 1088;  // segments of a launch at most
-constexpr int kMmFixed = ((kMmSegMax + 4 + 16) * 4 + 127) / 128 * 128;  // segment table in shared memory
+constexpr int kMmFixed = ((kMmSegMax + 4 + 16) * 4 + 127) / 128 * 128;  // segment table and the like in shared memory
 constexpr uint32_t kMmSmemBase = 1024;    // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
 constexpr int kMmTok = 2;        // tokens of a column tile: eight columns, four digits a token
 
@@ -61,8 +62,10 @@ template <int T> constexpr bool mq_mins = (T == T_Q4_K || T == T_Q5_K);
 
 // ---- activations -----------------------------------------------------------------------------------------------------------
 // A 256-element block of one token: [4 digits][256 bytes, unit u and lane t at 32 u + 8 t, kXDigit bytes apart: four digits of a
-// lane's eight bytes fall on different banks][3 parts][8] sub-block sums as fp16 (formats with mins), then what undoes the scaling.
-constexpr int kXDigit = 288, kXSums = 4 * kXDigit, kXInv = kXSums + 48, kXBlock = kXInv + 16;
+// lane's eight bytes fall on different banks; the 32 bytes between them: what is left over (mm_left_at)][3 parts][8] sub-block sums as fp16
+// (formats with mins), then what undoes the scaling (two floats), and whether the block is wide.
+constexpr int kXDigit = 288, kXSums = 4 * kXDigit, kXInv = kXSums + 48, kXWide = kXInv + 8, kXBlock = kXInv + 16;
+__device__ __forceinline__ int mm_left_at(int u, int t) { return (u >> 1) * kXDigit + 256 + (u & 1) * 16 + 4 * t; }
 
 // First element (of 256) of the two groups of four that unit u = 0..7 of lane t takes.
 template <int T>
@@ -103,21 +106,33 @@ __device__ __forceinline__ void mm_split(float a, float b, uint32_t (&h)[3]) {
 }
 __device__ __forceinline__ float mm_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
 
-// One warp: a token's 256 elements at xr into their place in shared memory.  The block times 2^s is below 2^30 and rounded to an integer; its
-// four digits in base 256 are balanced (-128 .. 127), so that sum_j 256^j * d_j is the integer.
+// One warp: a token's 256 elements at xr into their place in shared memory.  The block times 2^s, which puts its largest element into [2^30,
+// 2^31), or into half of that where it would be above 0x7f7f7f7f, is rounded to integers; their four digits in base 256 are balanced (-128 ..
+// 127), so that sum_j 256^j * d_j is the integer.
+// That rounds elements below 2^24 (2^-7 to 2^-6 of the block's largest) to 2^-31 of the largest, which is less than what the sums are rounded
+// by, unless hardly any weight hears the large elements.  So a block is called wide, and four more bits are kept of what the rounding left
+// over, if fewer than 8 of its 32 lanes hold an element of 2^24 or more, or none of some unit's four (the 32 elements of a scale, which may be
+// zero for the others), and other lanes are not zero.  Relative error against 64 bits with one element 2^j times the others in each block that
+// no weight hears, Q8_0, K = 2048, in 1e-7, three fp16 parts of a row (as this kernel had before) / integers of 31 bits / these, j = 6: 0.91 /
+// 0.88 / 0.83; 8: 0.91 / 1.6 / 0.82; 10: 0.97 / 5.6 / 0.84; 12: 1.7 / 22 / 1.05; 16: 22 / 354 / 12.  Over five formats, K of 512 to 4096, normal and
+// heavy-tailed inputs, such outliers and small sub-blocks: at most 0.97 of the fp16 parts' error in any.
+// Normal inputs have no wide blocks; of what the down projection meets, none or, behind a Q4_K or Q5_K layer whose mins drive most of a
+// token's gates negative, a few in a hundred.  An item that has one costs a fifth more: a batch of 8 469 -> 472 us a pass, of 32 1,041 -> 1,050, a
+// prompt of 77 357 -> 372 (before there were rests: 461, 1,023, 348).
+// Returns whether the block is wide.
 template <int T>
-__device__ __forceinline__ void mm_stage_block(const float* __restrict__ xr, uint8_t* dst, int lane) {
+__device__ __forceinline__ bool mm_stage_block(const float* __restrict__ xr, uint8_t* dst, int lane) {
     const int u = lane >> 2, t = lane & 3;
     int e0, e1;
     mm_unit_elems<T>(u, t, e0, e1);
     const float4 f0 = *reinterpret_cast<const float4*>(xr + e0), f1 = *reinterpret_cast<const float4*>(xr + e1);
     float x[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-    uint32_t mx = 0u;
+    uint32_t mine = 0u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) mx = max(mx, __float_as_uint(fabsf(x[i])));
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    const int ex = (int)(mx >> 23);  // biased exponent of the largest |x|; s puts it into [2^29, 2^30)
-    const int s = ex == 0 ? 0 : min(149, 156 - ex), s1 = min(s, 120);
+    for (int i = 0; i < 8; ++i) mine = max(mine, __float_as_uint(fabsf(x[i])));
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, mine);
+    const int ex = (int)((mx + 0x10101u) >> 23);  // biased exponent of the largest |x|, one more where its mantissa is too large
+    const int s = ex == 0 ? 0 : min(149, 157 - ex), s1 = min(s, 120);
     const float up = mm_pow2(s1);
 #pragma unroll
     for (int i = 0; i < 8; ++i) x[i] *= up;
@@ -126,11 +141,15 @@ __device__ __forceinline__ void mm_stage_block(const float* __restrict__ xr, uin
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] *= up2;
     }
-    if constexpr (mq_mins<T>) {  // a sub-block is a unit: its sum over the four lanes, in units of 2^20
+    // lanes that have an element of 2^24 or more, lanes that have one at all; a unit is four lanes
+    const uint32_t large = __ballot_sync(0xffffffffu, mine >= (uint32_t)(151 - s) << 23), some = __ballot_sync(0xffffffffu, mine != 0u);
+    const uint32_t large4 = large | large >> 1 | large >> 2 | large >> 3, some4 = some | some >> 1 | some >> 2 | some >> 3;
+    const bool wide = (some4 & ~large4 & 0x11111111u) != 0u || (__popc(large) < 8 && large != some);
+    if constexpr (mq_mins<T>) {  // a sub-block is a unit: its sum over the four lanes, in units of 2^21
         float a = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
         a += __shfl_xor_sync(0xffffffffu, a, 1);
         a += __shfl_xor_sync(0xffffffffu, a, 2);
-        a *= 0x1p-20f;
+        a *= 0x1p-21f;
         const float b = __shfl_xor_sync(0xffffffffu, a, 4);
         uint32_t h[3];
         mm_split(a, b, h);
@@ -150,8 +169,18 @@ __device__ __forceinline__ void mm_stage_block(const float* __restrict__ xr, uin
     // 2^-s for the low two digits, 2^(16 - s) for the high two; a block with an infinity or a NaN makes a NaN of every sum
     if (lane < 2) {
         const int e = 16 * lane - s;
-        reinterpret_cast<float*>(dst + kXInv)[lane] = ex == 255 ? __uint_as_float(0x7fc00000u) : e >= -126 ? mm_pow2(e) : __uint_as_float(1u << (149 + e));
+        reinterpret_cast<float*>(dst + kXInv)[lane] = mx >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : e >= -126 ? mm_pow2(e) : __uint_as_float(1u << (149 + e));
     }
+    if (lane == 2) *reinterpret_cast<uint32_t*>(dst + kXWide) = wide ? 1u : 0u;
+    if (__builtin_expect(wide, 0)) {
+        // what is left over in fifteenths, -7 .. 7 (not to -8: with a bias, weights that are all positive would add it up); elements 4 .. 7 in the
+        // lower nibbles of the bytes, 0 .. 3 in the upper
+        uint32_t left = 0u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) left |= ((uint32_t)max(-7, min(7, __float2int_rn((x[i] - rintf(x[i])) * 15.f))) & 15u) << (8 * (i & 3) + (i < 4 ? 4 : 0));
+        *reinterpret_cast<uint32_t*>(dst + mm_left_at(u, t)) = left;
+    }
+    return wide;
 }
 
 // ---- integer products --------------------------------------------------------------------------------------------------------
@@ -311,12 +340,13 @@ struct MmStream {
     }
 };
 
-// One 256-element block of 16 rows (this lane: rows `ra` and `rb`) against NT column tiles; bp[i]: the lane's B column of tile
+// One 256-element block of 16 rows (this lane: rows `ra` and `rb`) against NT column tiles; bq(i, u): unit u of the lane's B column of tile
 // i at this block; inv, sumw: of the token whose columns the lane's accumulators hold, and of its B column.
 // acc[i] += scales * sums: rows `ra` and `rb`, digits 0 and 1 of a token (t even) or 2 and 3 (t odd).
-template <int T, int NT>
-__device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, uint32_t gl, uint32_t sl, const uint8_t* const (&bp)[NT],
-                                         const uint32_t (&sumw)[NT], const float (&inv)[NT], float (&acc)[NT][2]) {
+// REST: one more column tile, NT, whose columns are eight tokens; left: rows `ra` and `rb` of columns 2 t, 2 t + 1, without an `inv`.
+template <int T, int NT, bool REST, class B>
+__device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, int t, uint32_t gl, uint32_t sl, const B& bq, const uint32_t (&sumw)[NT], const float (&inv)[NT], float (&acc)[NT][2], float (&left)[2][2]) {
+    constexpr int N1 = NT + (REST ? 1 : 0);
     if constexpr (T == T_Q8_0) {
         float s[NT][2];
 #pragma unroll
@@ -338,11 +368,18 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
             }
             const float fa = h2f(ld16(ra + 34 * ib)), fb = h2f(ld16(rb + 34 * ib));
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
+            for (int n = 0; n < N1; ++n) {
                 // sums start at the bits of 1.5 * 2^23, so that they are floats as they stand (|sum| <= 2^19)
                 int D[4];
-                mma_s8<0x4B400000>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
+                mma_s8<0x4B400000>(D, p[0], q[0], p[1], q[1], bq(n, ib));
                 const float m = 12582912.f;
+                if (REST && n == NT) {
+                    left[0][0] = fmaf(fa, __int_as_float(D[0]) - m, left[0][0]);
+                    left[0][1] = fmaf(fa, __int_as_float(D[1]) - m, left[0][1]);
+                    left[1][0] = fmaf(fb, __int_as_float(D[2]) - m, left[1][0]);
+                    left[1][1] = fmaf(fb, __int_as_float(D[3]) - m, left[1][1]);
+                    continue;
+                }
                 s[n][0] = fmaf(fa, fmaf(256.f, __int_as_float(D[1]) - m, __int_as_float(D[0]) - m), s[n][0]);
                 s[n][1] = fmaf(fb, fmaf(256.f, __int_as_float(D[3]) - m, __int_as_float(D[2]) - m), s[n][1]);
             }
@@ -353,9 +390,9 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
             acc[n][1] = fmaf(s[n][1], inv[n], acc[n][1]);
         }
     } else {
-        int c[NT][4];
+        int c[N1][4];
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < N1; ++n)
 #pragma unroll
             for (int i = 0; i < 4; ++i) c[n][i] = 0;
         // one sub-block: its sums times its scales
@@ -405,9 +442,9 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) {
+                    for (int n = 0; n < N1; ++n) {
                         int D[4];
-                        mma_u8(D, a[h][0], b[h][0], a[h][1], b[h][1], *reinterpret_cast<const uint2*>(bp[n] + (2 * j + h) * 32));
+                        mma_u8(D, a[h][0], b[h][0], a[h][1], b[h][1], bq(n, 2 * j + h));
                         add(n, D, fa[h], fb[h]);
                     }
             }
@@ -439,9 +476,9 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                 iq3_s8(gl, sl, ld16(ib2 + 8 * ib), __funnelshift_r(xb, xb, st), q[0], q[1]);
                 const int fa = (int)(2u * (xa >> 28) + 1u), fb = (int)(2u * (xb >> 28) + 1u);
 #pragma unroll
-                for (int n = 0; n < NT; ++n) {
+                for (int n = 0; n < N1; ++n) {
                     int D[4];
-                    mma_s8<0>(D, p[0], q[0], p[1], q[1], *reinterpret_cast<const uint2*>(bp[n] + ib * 32));
+                    mma_s8<0>(D, p[0], q[0], p[1], q[1], bq(n, ib));
                     add(n, D, fa, fb);
                 }
             }
@@ -456,10 +493,10 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
                     const uint32_t qa = ld32u(ra + 64 * half + 32 * w + 16 * is + 4 * t), qb = ld32u(rb + 64 * half + 32 * w + 16 * is + 4 * t);
-                    uint2 y[NT];
+                    uint2 y[N1];
 #pragma unroll
-                    for (int n = 0; n < NT; ++n)
-                        y[n] = *reinterpret_cast<const uint2*>(bp[n] + (2 * g + w) * 32);
+                    for (int n = 0; n < N1; ++n)
+                        y[n] = bq(n, 2 * g + w);
 #pragma unroll
                     for (int hi = 0; hi < 2; ++hi) {
                         const int sh = 6 - 2 * w - 4 * hi;  // the pair of bits to the top of its byte
@@ -468,7 +505,7 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
                         const int sc = 192 + 8 * half + is + 2 * w + 4 * hi;
                         const int fa = *reinterpret_cast<const int8_t*>(ra + sc), fb = *reinterpret_cast<const int8_t*>(rb + sc);
 #pragma unroll
-                        for (int n = 0; n < NT; ++n) {
+                        for (int n = 0; n < N1; ++n) {
                             int D[4];
                             mma_s8_k16(D, va, vb, hi ? y[n].y : y[n].x);
                             add(n, D, fa, fb);
@@ -483,12 +520,19 @@ __device__ __forceinline__ void mm_block(const uint8_t* ra, const uint8_t* rb, i
             if constexpr (mq_mins<T>) {
                 float M[4];
                 mma_f16_z(M, mma, mmb, 0u, 0u, sumw[n], 0u);
-                const float k = (t & 1) ? 16.f : 0x1p20f;  // columns 0, 1 of a token stand beside its low digits, column 2 beside the high ones
+                const float k = (t & 1) ? 32.f : 0x1p21f;  // columns 0, 1 of a token stand beside its low digits, column 2 beside the high ones
                 va = fmaf(-dma, (M[0] + M[1]) * k, va);
                 vb = fmaf(-dmb, (M[2] + M[3]) * k, vb);
             }
             acc[n][0] = fmaf(va, inv[n], acc[n][0]);
             acc[n][1] = fmaf(vb, inv[n], acc[n][1]);
+        }
+        if constexpr (REST) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                left[0][i] = da * (float)c[NT][i];
+                left[1][i] = db * (float)c[NT][2 + i];
+            }
         }
     }
 }
@@ -511,27 +555,253 @@ struct MmArgs {
 
 __device__ __forceinline__ void mm_barrier(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 
+// What a warp does of an item.
+struct MmItem {
+    const uint8_t *wa, *wb;    // the segment's matrices
+    const uint8_t* acts;       // [m tokens][nb blocks][kXBlock]
+    float* red;                // [2][16 warps][tiles * 2][32] when ks > 1
+    float* out;                // the first token's results
+    int m, nb, kb0, kbn;       // tokens; blocks of K, first and number of this warp's
+    int rg, nrg, nslot;        // first row group and number of them, every nslot-th
+    int n_out, rb, ks, slot, kpart;
+};
+
+// The warp's weight stream: the next blocks of the next row group.
+template <int T, bool FUSED>
+struct MmFeed {
+    MmStream<T> w;
+    int rg, b;
+    __device__ __forceinline__ void prefetch(const MmItem& I) {
+        int n = 0;
+        if (rg < I.rg + I.nrg * I.nslot) {
+            if (b == 0) {
+                const uint32_t boff = (uint32_t)I.kb0 * Mq<T>::BB;
+                w.template point<FUSED>(I.wa + boff, FUSED ? I.wb + boff : nullptr, rg * (FUSED ? 8 : 16), I.n_out - 1, (uint32_t)I.rb);
+            }
+            n = min(w.bps, I.kbn - b);
+            b += n;
+            if (b == I.kbn) {
+                b = 0;
+                rg += I.nslot;
+            }
+        }
+        w.request(n);
+    }
+};
+
+// One block of the 16 rows with what is left over of the wide ones among the tokens: one more column tile, token g's bytes are sixteen
+// times the fifteenths.  token(k): token k's block.
+template <int T, int N, class Token>
+__device__ __forceinline__ void mm_block_wide(const uint8_t* ra, const uint8_t* rb, int lane, const Token& token, const uint8_t* const (&bp)[N],
+                                              const uint32_t (&sumw)[N], const float (&inv)[N], float (&acc)[N][2]) {
+    const int g = lane >> 2, t = lane & 3;
+    auto is_wide = [&](int k) { return *reinterpret_cast<const uint32_t*>(token(k) + kXWide) != 0u; };
+    const uint8_t* rest = token(g) + mm_left_at(0, t);
+    const uint32_t mask = is_wide(g) ? 0xf0f0f0f0u : 0u;
+    auto column = [&](int n, int u) {
+        if (n < N) return *reinterpret_cast<const uint2*>(bp[n < N ? n : 0] + u * 32);
+        const uint32_t v = *reinterpret_cast<const uint32_t*>(rest + mm_left_at(u, 0) - mm_left_at(0, 0));
+        return make_uint2(v & mask, (v << 4) & mask);
+    };
+    float left[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    mm_block<T, N, true>(ra, rb, t, 4 * lane, 8 * (lane & 15), column, sumw, inv, acc, left);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {  // from lane t = n to the lanes that hold the low digits' sums of tokens 2 n, 2 n + 1
+        const bool add = !(t & 1) && is_wide(n * kMmTok + (t >> 1));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float v0 = __shfl_sync(0xffffffffu, left[h][0], (g << 2) + n), v1 = __shfl_sync(0xffffffffu, left[h][1], (g << 2) + n);
+            if (add) acc[n][h] = fmaf(t ? v1 : v0, (1.f / 240.f) * inv[n], acc[n][h]);
+        }
+    }
+}
+
+// The item's row groups with N column tiles (those behind the last token repeat it); REST: with what is left over of wide blocks, too.
+template <int T, bool FUSED, int N, bool REST>
+__device__ __forceinline__ void mm_row_groups(const MmItem& I, MmFeed<T, FUSED>& F) {
+    using Q = Mq<T>;
+    const int lane = F.w.lane, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t gl = 4 * lane, sl = 8 * (lane & 15);
+    auto token = [&](int k) { return I.acts + (size_t)min(k, I.m - 1) * I.nb * kXBlock; };
+    const uint8_t *colb[N], *colv[N];  // the token of this lane's B column, and of its accumulators
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        colb[n] = token(n * kMmTok + (g >> 2));
+        colv[n] = token(n * kMmTok + (t >> 1)) + kXInv + (t & 1) * 4;
+    }
+    float acc[N][2];
+    for (int round = 0, rg = I.rg; round < I.nrg; ++round, rg += I.nslot) {
+        // where a row's blocks start (only the position inside 16 bytes matters)
+        uint32_t offa = 0, offb = 0;
+        if constexpr (!Q::ALIGNED) {
+            const uint32_t r0 = FUSED ? rg * 8 + g : min(rg * 16 + g, I.n_out - 1), r1 = FUSED ? r0 : (uint32_t)min(rg * 16 + 8 + g, I.n_out - 1);
+            offa = r0 * (uint32_t)I.rb + (uint32_t)I.kb0 * Q::BB;
+            offb = r1 * (uint32_t)I.rb + (uint32_t)I.kb0 * Q::BB;
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[n][0] = acc[n][1] = 0.f;
+#pragma unroll 1
+        for (int b = 0; b < I.kbn;) {
+            const uint8_t* st = F.w.wait();  // and every lane has left the slot that is filled next
+            F.prefetch(I);
+            const uint8_t *ra = st + g * F.w.pitch + (Q::ALIGNED ? 0u : offa & 15u), *rb = st + (g + 8) * F.w.pitch + (Q::ALIGNED ? 0u : offb & 15u);
+            const int stop = min(b + F.w.bps, I.kbn);
+            offa += (stop - b) * Q::BB;
+            offb += (stop - b) * Q::BB;
+#pragma unroll 1
+            for (; b < stop; ++b, ra += Q::BB, rb += Q::BB) {
+                const uint8_t* bp[N];
+                uint32_t sumw[N];
+                float inv[N];
+                const int at_b = (I.kb0 + b) * kXBlock;
+#pragma unroll
+                for (int n = 0; n < N; ++n) {
+                    bp[n] = colb[n] + at_b + (g & 3) * kXDigit + t * 8;
+                    inv[n] = *reinterpret_cast<const float*>(colv[n] + at_b);
+                    sumw[n] = 0u;  // the fourth column of a token takes no sums
+                    if constexpr (mq_mins<T>) {
+                        if ((g & 3) < 3) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + at_b + kXSums + (g & 3) * 16 + t * 4);
+                    }
+                }
+                if constexpr (!REST) {
+                    float none[2][2];
+                    mm_block<T, N, false>(ra, rb, t, gl, sl, [&](int n, int u) { return *reinterpret_cast<const uint2*>(bp[n] + u * 32); }, sumw, inv, acc, none);
+                } else {
+                    mm_block_wide<T, N>(ra, rb, lane, [&](int k) { return token(k) + at_b; }, bp, sumw, inv, acc);
+                }
+            }
+            F.w.next();
+        }
+        bool mine = true;
+        if (I.ks > 1) {  // the warps of the row group meet; the first adds the others' sums in order
+            float* rp = I.red + ((size_t)(round & 1) * kMmWarps + warp) * N * 2 * 32 + lane;
+            mine = I.kpart == 0;
+            if (!mine) {
+#pragma unroll
+                for (int n = 0; n < N; ++n)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) rp[(n * 2 + c) * 32] = acc[n][c];
+            }
+            mm_barrier(1 + I.slot, I.ks * 32);
+            if (mine) {
+                for (int k2 = 1; k2 < I.ks; ++k2) {
+                    rp += N * 2 * 32;
+#pragma unroll
+                    for (int n = 0; n < N; ++n)
+#pragma unroll
+                        for (int c = 0; c < 2; ++c) acc[n][c] += rp[(n * 2 + c) * 32];
+                }
+            }
+        }
+        if (mine) {
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                // the low two digits' sums and the high two's meet: both lanes have both rows of the token
+                float a = acc[n][0], b = acc[n][1];
+                a += __shfl_xor_sync(0xffffffffu, a, 1);
+                b += __shfl_xor_sync(0xffffffffu, b, 1);
+                const int tok = n * kMmTok + (t >> 1);
+                if (tok < I.m) {
+                    float* o = I.out + (size_t)tok * I.n_out;
+                    if constexpr (FUSED) {
+                        if (!(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
+                    } else {
+                        const int r = rg * 16 + g;
+                        if (!(t & 1) && r < I.n_out) o[r] = a;
+                        if ((t & 1) && r + 8 < I.n_out) o[r + 8] = b;
+                    }
+                }
+            }
+        }
+    }
+}
+// Where things are in a CTA's shared memory, behind the IQ3_XXS tables.
+struct MmShared {
+    int* pre;        // [kMmSegMax + 1] first token tile of a segment
+    int* wsum;       // [16]
+    float* red;      // [2][16 warps][NT * 2][32] when ks > 1
+    uint8_t* acts;   // [tokens of an item][blocks][kXBlock]
+    uint8_t* ring;   // of the warp
+};
+template <int T, int NT>
+__device__ __forceinline__ MmShared mm_shared(uint8_t* smem, const MmArgs& A) {
+    MmShared S;
+    uint8_t* p = smem + (T == T_IQ3_XXS ? sizeof(MmTables) : 0);
+    S.pre = reinterpret_cast<int*>(p);
+    S.wsum = S.pre + kMmSegMax + 4;
+    p += kMmFixed;
+    S.red = reinterpret_cast<float*>(p);
+    if (A.ks > 1) p += 2 * kMmWarps * NT * 2 * 32 * sizeof(float);
+    S.acts = p;
+    S.ring = p + (size_t)NT * kMmTok * (A.n_in >> 8) * kXBlock + (size_t)(threadIdx.x >> 5) * A.ring.nst * 16 * A.ring.pitch;
+    return S;
+}
+
+// The CTA's items.
+template <int T, bool FUSED, int NT>
+__device__ __forceinline__ void mm_items(const MmArgs& A, const MmShared& S, int nseg) {
+    constexpr int TT = NT * kMmTok;  // tokens of an item
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = A.n_in >> 8;
+    MmFeed<T, FUSED> F{MmStream<T>(S.ring, A.ring, lane), 0, 0};
+    const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
+    const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
+    const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
+    // This CTA's share of all (tile, row group) pairs: a range of pairs in a row.  Another tile means another set of activations,
+    // which takes as long as A.skip row groups: each tile is that much longer, and a CTA that has two gets so much less of them.
+    const int span = n_rg + A.skip, total = S.pre[nseg] * span;
+    const int share = total / (int)gridDim.x, extra = total - share * (int)gridDim.x;
+    const int at1 = share * ((int)blockIdx.x + 1) + min((int)blockIdx.x + 1, extra);
+    for (int at = share * (int)blockIdx.x + min((int)blockIdx.x, extra); at < at1;) {
+        const int gtile = at / span, in = at - gtile * span;
+        const int rg_begin = max(in - A.skip, 0), rg_end = min(in + (at1 - at), span) - A.skip;
+        at += span - in;
+        if (rg_end <= rg_begin) continue;
+        int lo = 0, hi = nseg;  // the segment: pre[lo] <= gtile < pre[lo + 1]
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (S.pre[mid] <= gtile) lo = mid; else hi = mid;
+        }
+        const SegDesc sd = A.seg ? A.seg[lo] : A.single;
+        const int tile = gtile - S.pre[lo];
+        const int m = min(TT, (int)sd.m - tile * TT);
+        const uint32_t row0 = sd.row0 + tile * TT;
+        const int rg = rg_begin + slot;
+        const MmItem I = {sd.wa, sd.wb, S.acts, S.red, A.out + (size_t)row0 * A.n_out, m, nb, kb0, kbn, rg, rg < rg_end ? (rg_end - rg + nslot - 1) / nslot : 0, nslot,
+                          A.n_out, A.rb, A.ks, slot, kpart};
+        F.rg = rg;
+        F.b = 0;
+        for (int i = 1; i < F.w.nst; ++i) F.prefetch(I);
+
+        // ---- activations: a 256-element block of a token per warp ----
+        bool wide = false;
+        for (int gi = warp; gi < m * nb; gi += kMmWarps) {
+            const int tok = gi / nb, b = gi - tok * nb;
+            const uint32_t pr = row0 + tok;
+            wide |= mm_stage_block<T>(A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256, S.acts + (size_t)gi * kXBlock, lane);
+        }
+        if (__builtin_expect(__syncthreads_or(wide), 0)) {
+            mm_row_groups<T, FUSED, NT, true>(I, F);
+        } else if (NT >= 4 && m > 2 * kMmTok) {
+            mm_row_groups<T, FUSED, NT >= 4 ? 4 : 1, false>(I, F);
+        } else if (NT >= 2 && m > kMmTok) {
+            mm_row_groups<T, FUSED, NT >= 2 ? 2 : 1, false>(I, F);
+        } else {
+            mm_row_groups<T, FUSED, 1, false>(I, F);
+        }
+        __syncthreads();  // every warp has left the activations
+    }
+    tcp::cp_async_wait_all();
+}
 template <int T, bool FUSED, int NT>
 __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
-    using Q = Mq<T>;
     constexpr int TT = NT * kMmTok;  // tokens of an item
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* p0 = smem + (T == T_IQ3_XXS ? sizeof(MmTables) : 0);
-    int* pre = reinterpret_cast<int*>(p0);                              // [kMmSegMax + 1] first token tile of a segment
-    int* wsum = pre + kMmSegMax + 4;                                    // [16]
-    p0 += kMmFixed;
-    float* red = reinterpret_cast<float*>(p0);                          // [2][16 warps][NT * 2][32] when ks > 1
-    if (A.ks > 1) p0 += 2 * kMmWarps * NT * 2 * 32 * sizeof(float);
-    const int nb = A.n_in >> 8;
-    uint8_t* acts = p0;                                                 // [TT tokens][nb blocks][kXBlock]
-    p0 += (size_t)TT * nb * kXBlock;
     if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
     }
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    MmStream<T> W(p0 + (size_t)warp * A.ring.nst * 16 * A.ring.pitch, A.ring, lane);
+    const MmShared S = mm_shared<T, NT>(smem, A);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if constexpr (T == T_IQ3_XXS) {
         mm_tables_in(smem, tid, kMmThreads);
         tcp::cp_async_wait_all();
@@ -554,172 +824,21 @@ __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
             const int v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += v;
         }
-        if (lane == 31) wsum[warp] = incl;
+        if (lane == 31) S.wsum[warp] = incl;
         __syncthreads();
         int at = incl - sum;
-        for (int w = 0; w < warp; ++w) at += wsum[w];
+        for (int w = 0; w < warp; ++w) at += S.wsum[w];
         for (int j = 0; j < per; ++j) {
             const int s = tid * per + j;
             if (s < nseg) {
-                pre[s] = at;
+                S.pre[s] = at;
                 at += (int)(((A.seg ? A.seg[s].m : A.single.m) + TT - 1) / TT);
             }
         }
-        if (tid == kMmThreads - 1) pre[nseg] = at;
+        if (tid == kMmThreads - 1) S.pre[nseg] = at;
         __syncthreads();
     }
-    const int nslot = kMmWarps / A.ks, slot = warp / A.ks, kpart = warp - slot * A.ks;
-    const int kb0 = nb * kpart / A.ks, kbn = nb * (kpart + 1) / A.ks - kb0;
-    const int n_rg = FUSED ? A.n_out / 8 : (A.n_out + 15) / 16;
-    const uint32_t gl = 4 * lane, sl = 8 * (lane & 15);
-    // This CTA's share of all (tile, row group) pairs: a range of pairs in a row.  Another tile means another set of activations,
-    // which takes as long as A.skip row groups: each tile is that much longer, and a CTA that has two gets so much less of them.
-    const int span = n_rg + A.skip, total = pre[nseg] * span;
-    const int share = total / (int)gridDim.x, extra = total - share * (int)gridDim.x;
-    const int at1 = share * ((int)blockIdx.x + 1) + min((int)blockIdx.x + 1, extra);
-
-    for (int at = share * (int)blockIdx.x + min((int)blockIdx.x, extra); at < at1;) {
-        const int gtile = at / span, in = at - gtile * span;
-        const int rg_begin = max(in - A.skip, 0), rg_end = min(in + (at1 - at), span) - A.skip;
-        at += span - in;
-        if (rg_end <= rg_begin) continue;
-        int lo = 0, hi = nseg;  // the segment: pre[lo] <= gtile < pre[lo + 1]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (pre[mid] <= gtile) lo = mid; else hi = mid;
-        }
-        const SegDesc sd = A.seg ? A.seg[lo] : A.single;
-        const int tile = gtile - pre[lo];
-        const int m = min(TT, (int)sd.m - tile * TT);
-        const uint32_t row0 = sd.row0 + tile * TT;
-        int rg = rg_begin + slot;
-        const int nrg = rg < rg_end ? (rg_end - rg + nslot - 1) / nslot : 0;
-
-        // ---- the warp's weight stream: the next blocks of the next row group ----
-        int pf_rg = rg, pf_b = 0;
-        const int rg_stop = rg + nrg * nslot;
-        auto prefetch = [&]() {
-            int n = 0;
-            if (pf_rg < rg_stop) {
-                if (pf_b == 0) {
-                    const uint32_t boff = (uint32_t)kb0 * Q::BB;
-                    W.template point<FUSED>(sd.wa + boff, FUSED ? sd.wb + boff : nullptr, pf_rg * (FUSED ? 8 : 16), A.n_out - 1, (uint32_t)A.rb);
-                }
-                n = min(W.bps, kbn - pf_b);
-                pf_b += n;
-                if (pf_b == kbn) {
-                    pf_b = 0;
-                    pf_rg += nslot;
-                }
-            }
-            W.request(n);
-        };
-        for (int i = 1; i < W.nst; ++i) prefetch();
-
-        // ---- activations: a 256-element block of a token per warp ----
-        for (int gi = warp; gi < m * nb; gi += kMmWarps) {
-            const int tok = gi / nb, b = gi - tok * nb;
-            const uint32_t pr = row0 + tok;
-            mm_stage_block<T>(A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256, acts + (size_t)gi * kXBlock, lane);
-        }
-        __syncthreads();
-
-        // ---- the row groups ----
-        auto row_groups = [&](auto tiles) {  // N column tiles: one, two or four, those behind the last token repeat it
-            constexpr int N = decltype(tiles)::value;
-            const uint8_t *colb[N], *colv[N];  // the token of this lane's B column, and of its accumulators
-#pragma unroll
-            for (int n = 0; n < N; ++n) {
-                colb[n] = acts + (size_t)min(n * kMmTok + (g >> 2), m - 1) * nb * kXBlock;
-                colv[n] = acts + (size_t)min(n * kMmTok + (t >> 1), m - 1) * nb * kXBlock + kXInv + (t & 1) * 4;
-            }
-            float acc[N][2];
-            for (int round = 0; round < nrg; ++round, rg += nslot) {
-                // where a row's blocks start (only the position inside 16 bytes matters)
-                uint32_t offa = 0, offb = 0;
-                if constexpr (!Q::ALIGNED) {
-                    const uint32_t r0 = FUSED ? rg * 8 + g : min(rg * 16 + g, A.n_out - 1), r1 = FUSED ? r0 : (uint32_t)min(rg * 16 + 8 + g, A.n_out - 1);
-                    offa = r0 * (uint32_t)A.rb + (uint32_t)kb0 * Q::BB;
-                    offb = r1 * (uint32_t)A.rb + (uint32_t)kb0 * Q::BB;
-                }
-#pragma unroll
-                for (int n = 0; n < N; ++n) acc[n][0] = acc[n][1] = 0.f;
-#pragma unroll 1
-                for (int b = 0; b < kbn;) {
-                    const uint8_t* st = W.wait();  // and every lane has left the slot that is filled next
-                    prefetch();
-                    const uint8_t *ra = st + g * W.pitch + (Q::ALIGNED ? 0u : offa & 15u), *rb = st + (g + 8) * W.pitch + (Q::ALIGNED ? 0u : offb & 15u);
-                    const int stop = min(b + W.bps, kbn);
-                    offa += (stop - b) * Q::BB;
-                    offb += (stop - b) * Q::BB;
-#pragma unroll 1
-                    for (; b < stop; ++b, ra += Q::BB, rb += Q::BB) {
-                        const uint8_t* bp[N];
-                        uint32_t sumw[N];
-                        float inv[N];
-#pragma unroll
-                        for (int n = 0; n < N; ++n) {
-                            const int at_b = (kb0 + b) * kXBlock;
-                            bp[n] = colb[n] + at_b + (g & 3) * kXDigit + t * 8;
-                            inv[n] = *reinterpret_cast<const float*>(colv[n] + at_b);
-                            sumw[n] = 0u;  // the fourth column of a token takes no sums
-                            if constexpr (mq_mins<T>) {
-                                if ((g & 3) < 3) sumw[n] = *reinterpret_cast<const uint32_t*>(colb[n] + at_b + kXSums + (g & 3) * 16 + t * 4);
-                            }
-                        }
-                        mm_block<T, N>(ra, rb, t, gl, sl, bp, sumw, inv, acc);
-                    }
-                    W.next();
-                }
-                bool mine = true;
-                if (A.ks > 1) {  // the warps of the row group meet; the first adds the others' sums in order
-                    float* rp = red + ((size_t)(round & 1) * kMmWarps + warp) * N * 2 * 32 + lane;
-                    mine = kpart == 0;
-                    if (!mine) {
-#pragma unroll
-                        for (int n = 0; n < N; ++n)
-#pragma unroll
-                            for (int c = 0; c < 2; ++c) rp[(n * 2 + c) * 32] = acc[n][c];
-                    }
-                    mm_barrier(1 + slot, A.ks * 32);
-                    if (mine) {
-                        for (int k2 = 1; k2 < A.ks; ++k2) {
-                            rp += N * 2 * 32;
-#pragma unroll
-                            for (int n = 0; n < N; ++n)
-#pragma unroll
-                                for (int c = 0; c < 2; ++c) acc[n][c] += rp[(n * 2 + c) * 32];
-                        }
-                    }
-                }
-                if (mine) {
-#pragma unroll
-                    for (int n = 0; n < N; ++n) {
-                        // the low two digits' sums and the high two's meet: both lanes have both rows of the token
-                        float a = acc[n][0], b = acc[n][1];
-                        a += __shfl_xor_sync(0xffffffffu, a, 1);
-                        b += __shfl_xor_sync(0xffffffffu, b, 1);
-                        const int tok = n * kMmTok + (t >> 1);
-                        if (tok < m) {
-                            float* o = A.out + (size_t)(row0 + tok) * A.n_out;
-                            if constexpr (FUSED) {
-                                if (!(t & 1)) o[rg * 8 + g] = a / (1.0f + expf(-a)) * b;
-                            } else {
-                                const int r = rg * 16 + g;
-                                if (!(t & 1) && r < A.n_out) o[r] = a;
-                                if ((t & 1) && r + 8 < A.n_out) o[r + 8] = b;
-                            }
-                        }
-                    }
-                }
-            }
-        };
-        if (NT >= 4 && m > 2 * kMmTok) row_groups(std::integral_constant<int, NT >= 4 ? 4 : 1>());
-        else if (NT >= 2 && m > kMmTok) row_groups(std::integral_constant<int, NT >= 2 ? 2 : 1>());
-        else row_groups(std::integral_constant<int, 1>());
-        __syncthreads();  // every warp has left the activations
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    mm_items<T, FUSED, NT>(A, S, nseg);
 }
 
 template <int T, bool FUSED, int NT>
@@ -899,11 +1018,12 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
 
     // ---- this warp's blocks of the vectors ----
     const int v0 = blockIdx.y * TOK;
+    bool wide = false;
     for (int i = 0; i < nst; ++i)
         for (int j = 0; j < count(i); ++j)
 #pragma unroll
             for (int q = 0; q < TOK; ++q)
-                mm_stage_block<T>(A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (first(i) + j) * 256, xs + (i * bps + j) * XB + q * kXBlock, lane);
+                wide |= mm_stage_block<T>(A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (first(i) + j) * 256, xs + (i * bps + j) * XB + q * kXBlock, lane);
     if constexpr (T == T_IQ3_XXS) {  // the tables came in parts from all threads
         tcp::cp_async_wait_all();
         __syncthreads();
@@ -921,24 +1041,34 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
                 offa = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + g, last) * A.rb + (uint32_t)first(0) * Q::BB;
                 offb = (uint32_t)(uintptr_t)A.w + (uint32_t)min(rg * 16 + 8 + g, last) * A.rb + (uint32_t)first(0) * Q::BB;
             }
+            auto all_of_k = [&](auto rest) {
 #pragma unroll 1
-            for (int i = 0; i < nst; ++i) {
-                const uint8_t* st = W.wait();
-                prefetch();
-                const uint8_t *ra = st + g * W.pitch + (Q::ALIGNED ? 0u : offa & 15u), *rb = st + (g + 8) * W.pitch + (Q::ALIGNED ? 0u : offb & 15u);
-                offa += A.ks * bps * Q::BB;
-                offb += A.ks * bps * Q::BB;
-                const int n = count(i);
+                for (int i = 0; i < nst; ++i) {
+                    const uint8_t* st = W.wait();
+                    prefetch();
+                    const uint8_t *ra = st + g * W.pitch + (Q::ALIGNED ? 0u : offa & 15u), *rb = st + (g + 8) * W.pitch + (Q::ALIGNED ? 0u : offb & 15u);
+                    offa += A.ks * bps * Q::BB;
+                    offb += A.ks * bps * Q::BB;
+                    const int n = count(i);
 #pragma unroll 1
-                for (int j = 0; j < n; ++j, ra += Q::BB, rb += Q::BB) {
-                    const int b = i * bps + j;
-                    const uint8_t* const bp[1] = {colb + b * XB + (g & 3) * kXDigit + t * 8};
-                    const uint32_t sumw[1] = {mq_mins<T> && (g & 3) < 3 ? *reinterpret_cast<const uint32_t*>(colb + b * XB + kXSums + (g & 3) * 16 + t * 4) : 0u};
-                    const float inv[1] = {*reinterpret_cast<const float*>(colv + b * XB)};
-                    mm_block<T, 1>(ra, rb, t, gl, sl, bp, sumw, inv, acc);
+                    for (int j = 0; j < n; ++j, ra += Q::BB, rb += Q::BB) {
+                        const int b = i * bps + j;
+                        const uint8_t* bp = colb + b * XB + (g & 3) * kXDigit + t * 8;
+                        const uint32_t sumw[1] = {mq_mins<T> && (g & 3) < 3 ? *reinterpret_cast<const uint32_t*>(colb + b * XB + kXSums + (g & 3) * 16 + t * 4) : 0u};
+                        const float inv[1] = {*reinterpret_cast<const float*>(colv + b * XB)};
+                        if constexpr (decltype(rest)::value) {
+                            const uint8_t* const columns[1] = {bp};
+                            mm_block_wide<T, 1>(ra, rb, lane, [&](int k) { return xs + b * XB + min(k, TOK - 1) * kXBlock; }, columns, sumw, inv, acc);
+                        } else {
+                            float none[2][2];
+                            mm_block<T, 1, false>(ra, rb, t, gl, sl, [&](int, int u) { return *reinterpret_cast<const uint2*>(bp + u * 32); }, sumw, inv, acc, none);
+                        }
+                    }
+                    W.next();
                 }
-                W.next();
-            }
+            };
+            if (__builtin_expect(wide, 0)) all_of_k(std::true_type());
+            else all_of_k(std::false_type());
         }
         // lanes t = 0, 1 hold the first vector's low and high digits, t = 2, 3 the second's
         float a = acc[0][0], b = acc[0][1];

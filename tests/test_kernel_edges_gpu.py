@@ -214,10 +214,103 @@ def test_activations_of_any_size(orc, ctx, name, nvec):
             if nvec == 1:
                 continue
         want = x[i, first:].astype(np.float64) @ deq.T
-        # 2^-30 of a block's largest element a term, and fp32 sums; 1e-37: an fp32 below 2^-126 keeps 2^-149
+        # fp32 sums, and what three fp16 parts would leave over of a block's largest element; 1e-37: an fp32 below 2^-126 keeps 2^-149
         tiny = k * 2.0 ** -149 * np.abs(deq).max() if i == 0 else 0.0
-        bound = 2.0 ** -20 * np.sqrt((x[i, first:].astype(np.float64) ** 2) @ (deq ** 2).T) + 2.0 ** -28 * np.abs(x[i, first:]).max() * np.abs(deq).sum(1) + tiny
+        bound = 2.0 ** -20 * np.sqrt((x[i, first:].astype(np.float64) ** 2) @ (deq ** 2).T) + 2.0 ** -34 * np.abs(x[i, first:]).max() * np.abs(deq).sum(1) + tiny
         assert np.all(np.abs(got[i, first:] - want) <= bound), (i, np.max(np.abs(got[i, first:] - want) / bound))
+
+
+def _deaf(name, w):
+    """Blocks of 256 elements whose weights do not hear element 37: zero, or (IQ3_XXS, which has no zero) the same as element 45's."""
+    b = w.reshape(-1, {"Q4_K": 144, "Q5_K": 176, "Q6_K": 210, "Q8_0": 272, "IQ3_XXS": 98}[name])
+    if name in ("Q4_K", "Q5_K"):
+        b[:, 9] &= 0xC0  # the min of its sub-block
+        b[:, (21 if name == "Q4_K" else 53)] &= 0x0F
+        if name == "Q5_K":
+            b[:, 21] &= 0xFD
+    elif name == "Q6_K":
+        b[:, 37] &= 0xF0
+        b[:, 133] = (b[:, 133] & 0xF3) | 8
+    elif name == "Q8_0":
+        b[:, 41] = 0
+    else:
+        b[:, 12:14] = b[:, 10:12]
+        signs = b[:, 70:74].copy().view(np.uint32)
+        b[:, 70:74] = ((signs & ~np.uint32(0x3F80)) | ((signs & np.uint32(0x7F)) << np.uint32(7))).view(np.uint8)
+    return w
+
+
+def _beside_outliers(name, x, ratio):
+    """x with element 37 of every block `ratio` times the others' size (IQ3_XXS: and element 45 its negative)."""
+    x = x.copy()
+    b = x.reshape(-1, 256)
+    b[:, 37] = ratio * (1.0 + np.arange(len(b)) % 7 / 7.0)
+    if name == "IQ3_XXS":
+        b[:, 45] = -b[:, 37]
+    return x
+
+
+def _small_elements_bound(name, x, deq):
+    """fp32 sums of what is heard, and 2^-34 of the row's largest element from each weight, as three fp16 parts of a row would have it."""
+    y = x.astype(np.float64).reshape(len(x), -1, 256).copy()
+    y[:, :, 37] = 0.0
+    if name == "IQ3_XXS":
+        y[:, :, 45] = 0.0
+    norm = np.sqrt((deq ** 2).sum(1))
+    return 2.0 ** -20 * np.sqrt((y.reshape(len(x), -1) ** 2) @ (deq ** 2).T) + 4 * 2.0 ** -34 * np.abs(x).max(1)[:, None] * norm
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("k,nvec", [(1024, 1), (1024, 2), (4352, 1), (768, 5)])
+def test_small_elements_beside_large_ones_gemv(orc, ctx, name, k, nvec):
+    """Blocks of x with an element far above the others that no weight hears: the others are as exact as three fp16 parts would hold them."""
+    ty, n = orc.TYPE_BY_NAME[name], 48
+    w = _deaf(name, np.array(orc.synth_blocks(ty, SEED, 170 + ty, n * k // orc.blck_size(ty))))
+    deq = orc.dequant_row(ty, w, n * k).reshape(n, k).astype(np.float64)
+    x = orc.synth_normal(SEED, 171, 1.0, nvec * k).reshape(nvec, k)
+    dw, dx, do = ctx.dev_alloc(w.nbytes), ctx.dev_alloc(x.nbytes), ctx.dev_alloc(nvec * n * 4)
+    try:
+        ctx.upload(dw, w)
+        for j in (8, 12, 16, 20):
+            xs = _beside_outliers(name, x, 2.0 ** j)
+            if j == 16:
+                xs[0] = x[0]  # one vector without
+            ctx.upload(dx, xs)
+            assert ctx.gemv_dev(ty, dw, k, n, dx, do, nvec)
+            got = ctx.download(do, np.empty((nvec, n), np.float32))
+            off = np.abs(got - xs.astype(np.float64) @ deq.T) / _small_elements_bound(name, xs, deq)
+            assert off.max() <= 1.0, (j, off.max())
+    finally:
+        for p in (dw, dx, do):
+            ctx.dev_free(p)
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("sizes", [(1, 1, 2, 1, 1, 1), (3, 2, 4, 2, 1, 2), (1, 17, 8, 5, 3, 7)])
+def test_small_elements_beside_large_ones_grouped(orc, ctx, name, sizes):
+    """The same for items of one, two and four column tiles; tokens that have no such blocks do not feel their neighbours that do."""
+    from denno_beta_b200 import cuda as cu
+
+    ty, k, n, ne = orc.TYPE_BY_NAME[name], 768, 96, len(sizes)
+    assert ctx.moe_config(1, k, n, ne, 2)
+    w = _deaf(name, np.array(orc.synth_blocks(ty, SEED, 180 + ty, ne * n * k // orc.blck_size(ty))))
+    assert ctx.register_experts(0, cu.GATE, ty, k, n, ne, w)
+    deq = orc.dequant_row(ty, w, ne * n * k).reshape(ne, n, k).astype(np.float64)
+    at = np.concatenate([[0], np.cumsum(sizes)])
+    segs = np.array([[ne - 1 - i, m, at[i], at[i]] for i, m in enumerate(sizes)], np.uint32)
+    x = orc.synth_normal(SEED, 181, 1.0, int(at[-1]) * k).reshape(-1, k)
+    plain = cu.moe_grouped_gemm_layer(ctx, 0, cu.GATE, segs, x, n)
+    for j in (8, 12, 16, 20):
+        xs = _beside_outliers(name, x, 2.0 ** j)
+        xs[1::3] = x[1::3]
+        xs[2::5, 256:] = x[2::5, 256:]  # one wide block of three
+        got = cu.moe_grouped_gemm_layer(ctx, 0, cu.GATE, segs, xs, n)
+        same = np.all(xs == x, axis=1)
+        assert np.array_equal(got[same].view(np.uint32), plain[same].view(np.uint32)), j
+        for i, m in enumerate(sizes):
+            rows, d = slice(at[i], at[i + 1]), deq[ne - 1 - i]
+            off = np.abs(got[rows] - xs[rows].astype(np.float64) @ d.T) / _small_elements_bound(name, xs[rows], d)
+            assert off.max() <= 1.0, (j, i, off.max())
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "IQ3_XXS"])

@@ -8,7 +8,8 @@
 * IQ3_XXS with exact weights: w = d / 4 * (grid magnitude) * sign * (2 s + 1), the product of the last three an integer exact
   in fp16 (csrc/grouped_tc.cu); the magnitude alone exact in bf16 (csrc/iq3_mma.cuh) and a signed byte (csrc/grouped_mma.cu).
 * Activations of those kernels: a row times a power of two as two fp16 numbers (csrc/operand_rows.cuh), three for the
-  sub-block sums of csrc/grouped_mma.cu, whose activations are four digits in base 256 of a block; its integer sums fit.
+  sub-block sums of csrc/grouped_mma.cu, whose activations are four digits in base 256 of a block and, of a wide one, what they leave over;
+  its integer sums fit.
 * Router operands (csrc/router_tc.cu): an fp32 value is the exact sum of three bf16 numbers (round, round, round).
 """
 import os
@@ -176,23 +177,65 @@ def test_three_bf16_parts_carry_an_fp32_exactly(orc):
 
 
 def _digits(x):
-    """Four digits in base 256, -128 .. 127, of a block times the power of two that puts its largest element into [2^29, 2^30)."""
-    ex = int(np.max(np.abs(x)).view(np.uint32) >> 23)
-    v = np.rint(np.ldexp(x.astype(np.float64), 156 - ex)).astype(np.int64)
+    """Four digits in base 256, -128 .. 127, of a block times the power of two that puts its largest element into [2^30, 2^31), or into half of it
+    where four digits do not reach; and what that leaves over, in fifteenths, -7 .. 7."""
+    s = 157 - ((int(np.max(np.abs(x)).view(np.uint32)) + 0x10101) >> 23)
+    scaled = np.ldexp(x.astype(np.float64), s)
+    v = np.rint(scaled).astype(np.int64)
     b = ((v + 0x00808080) ^ 0x00808080).astype(np.int32).view(np.uint32)
-    return np.stack([(b >> (8 * j)).astype(np.uint8).view(np.int8) for j in range(4)]).astype(np.int64), v, 156 - ex
+    digits = np.stack([(b >> (8 * j)).astype(np.uint8).view(np.int8) for j in range(4)]).astype(np.int64)
+    return digits, v, np.clip(np.rint((scaled - v) * 15), -7, 7), s
+
+
+def _wide(x):
+    """Blocks [n, 256] of which fewer than 8 lanes (of eight elements each) have one that is exact as an integer (2^24 or more after the scaling),
+    or none of some four lanes, and other lanes are not zero."""
+    ex = (np.max(np.abs(x), axis=1).view(np.uint32) + 0x10101) >> 23
+    v = np.abs(np.ldexp(x.astype(np.float64), 157 - ex.astype(np.int64)[:, None])).reshape(len(x), 8, 4, 8)
+    large, some = (v >= 2.0 ** 24).any(3), (v > 0).any(3)
+    return (some.any(2) & ~large.any(2)).any(1) | ((large.sum((1, 2)) < 8) & (large != some).any((1, 2)))
 
 
 @pytest.mark.parametrize("spread", [0.0, 3.0])
 def test_activation_blocks_as_four_digits(orc, spread):
     rng = np.random.RandomState(8)
-    for _ in range(50):
+    tops = np.array([0x7EFEFE, 0x7EFEFF, 0x7FFFFF, 0], np.uint32)  # mantissas around the largest that four digits hold
+    seen = []
+    for i in range(50):
         x = (rng.randn(256) * np.exp(spread * rng.randn(256))).astype(np.float32)
         x[rng.randint(256)] *= -1.999
-        d, v, s = _digits(x)
+        at = np.argmax(np.abs(x))
+        x[at] = np.copysign(((x[at:at + 1].view(np.uint32) & 0x7F800000) | tops[i % 4]).view(np.float32)[0], x[at])
+        d, v, rest, s = _digits(x)
         assert d.min() >= -128 and d.max() <= 127
         assert np.array_equal(sum(256 ** j * d[j] for j in range(4)), v)
-        assert np.max(np.abs(np.ldexp(v.astype(np.float64), -s) - x)) <= 2.0 ** -30 * np.max(np.abs(x))  # half a unit of 2^-29 of it
+        left = x.astype(np.float64) - np.ldexp(v.astype(np.float64), -s)
+        unit = 2.0 ** -30 * 1.01 * np.max(np.abs(x))  # at most, of it (or of 0.996 * 2^30)
+        assert np.max(np.abs(left)) <= unit / 2
+        left -= np.ldexp(rest / 15, -s)
+        assert np.max(np.abs(left)) <= unit / 30
+        seen.append(left / unit)
+    assert abs(np.mean(seen)) < 4 * np.std(seen) / np.sqrt(50 * 256)  # no bias, which weights of one sign would add up
+
+
+def test_which_activation_blocks_are_wide(orc):
+    """Those with an outlier of 2^8 times the others or more, or with small sub-blocks; not normal ones, nor what the down projection meets
+    (silu of one number times another, with half of them next to nothing where the first are large)."""
+    rng = np.random.RandomState(9)
+    f = lambda a: np.ascontiguousarray(a, np.float32)
+    silu = lambda a: a / (1 + np.exp(-a))
+    g, u = rng.randn(4000, 256), rng.randn(4000, 256)
+    for x in (g, g + 3, silu(g) * u, silu(10 * g) * u, silu(100 * g) * u):
+        assert _wide(f(x)).mean() < 1e-3
+    for j, lo, hi in ((5, 0.0, 0.0), (8, 0.99, 1.0), (9, 1.0, 1.0), (20, 1.0, 1.0)):
+        x = g.copy()
+        x[:, 37] = 2.0 ** j * 1.5
+        assert lo <= _wide(f(x)).mean() <= hi, j
+    x = g.reshape(-1, 8, 32).copy()
+    x[:, 5] *= 2.0 ** -8
+    assert _wide(f(x.reshape(-1, 256))).mean() > 0.99
+    x[:, 5] = 0.0
+    assert not _wide(f(x.reshape(-1, 256))).any()  # zeros are exact
 
 
 def test_integer_block_sums_fit(orc):
