@@ -22,6 +22,7 @@ SIGNATURES = {
     "dnb_device_status": (_i, [_vp, C.POINTER(C.c_int)]),
     "dnb_clear_status": (_i, [_vp]),
     "dnb_set_wait_limits": (_i, [_vp, _i, _i, _i]),
+    "dnb_set_smem_base": (_i, [_vp, _i]),
     "dnb_timer_start": (_i, [_vp]),
     "dnb_timer_stop": (_i, [_vp, _fp]),
     "dnb_use_graphs": (_i, [_vp, _i]),

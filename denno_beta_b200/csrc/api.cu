@@ -189,11 +189,18 @@ static cudaError_t wait_short(cudaStream_t st) {
 // copied to the caller, the word is cleared so that the next call is judged on its own, and
 // the call reports DNB_DECLINED ("did not run, out untouched": cuda.rs:21024-21027,
 // 8785-8788).  A grid barrier that ran out (23) also retires the one-kernel decode form
-// for this context: the two-launch form has no inter-CTA wait.
+// for this context: the two-launch form has no inter-CTA wait.  Shared memory that did not start
+// where the context has it (26) retires the kernels that depend on it, so that a retry takes others.
+static void retire_smem_base(dnb_ctx* c, int st) {
+    if (st != 26 || !c->smem_base) return;
+    c->smem_base = 0;
+    drop_graphs(c);
+}
 static int finish_checked(dnb_ctx* c, const char* what) {
     const int st = *reinterpret_cast<volatile int*>(c->status_host);
     if (st == 0) return DNB_OK;
     *reinterpret_cast<volatile int*>(c->status_host) = 0;
+    retire_smem_base(c, st);
     if (st == 23 && c->decode_fused) {
         c->decode_fused = false;
         drop_graphs(c);
@@ -369,7 +376,7 @@ static bool tc_eligible(const dnb_ctx* c, const Layer& L, int nt) {
     const Model& M = c->model;
     if (!c->use_tc || !c->ws.op_ok) return false;
     const int ty = tc_type(L, 0, 3);
-    if (ty < 0 || nt < tc_min_tokens(c, ty) || !tc_handles(ty, M.e, M.ff, true) || !tc_handles(ty, M.ff, M.e, false)) return false;
+    if (ty < 0 || nt < tc_min_tokens(c, ty) || !tc_handles(c, ty, M.e, M.ff, true) || !tc_handles(c, ty, M.ff, M.e, false)) return false;
     if (L.has_shared()) {  // the shared expert rides in the same launches as one more segment
         if (tc_type(L, 3, 6) != ty || L.m[3].n_out != M.ff) return false;
     }
@@ -405,7 +412,7 @@ static int experts_dev_tc(dnb_ctx* c, int layer, const float* x, int nt, const i
 // Layers that the mma.sync grouped kernel takes (grouped_mma.cu): its five formats, the shared expert like the routed ones.
 static bool mm_eligible(const dnb_ctx* c, const Layer& L) {
     const Model& M = c->model;
-    if (!c->decode_fast || L.m[0].type != L.m[1].type || !mm_handles(L.m[0].type, M.e) || !mm_handles(L.m[2].type, M.ff)) return false;
+    if (!c->decode_fast || L.m[0].type != L.m[1].type || !mm_handles(c, L.m[0].type, M.e) || !mm_handles(c, L.m[2].type, M.ff)) return false;
     if (!L.has_shared()) return true;
     return L.m[3].type == L.m[0].type && L.m[4].type == L.m[1].type && L.m[5].type == L.m[2].type && L.m[3].n_out == M.ff;
 }
@@ -517,7 +524,7 @@ int shared_rows(dnb_ctx* c, int layer, const float* x, int rows, bool op_ready, 
     int rc;
     if ((rc = launch_prep(c, st, x, nullptr, M.eps, rows, M.e, nullptr, w.seg_sh_gu, w.seg_sh_dn, L.m[3].dev, L.m[4].dev, L.m[5].dev))) return rc;
     const int sff = L.m[3].n_out, ty = sff == M.ff ? tc_type(L, 3, 6) : -1;
-    if (c->use_tc && w.op_ok && rows >= 16 && ty >= 0 && tc_handles(ty, M.e, M.ff, true) && tc_handles(ty, M.ff, M.e, false)) {
+    if (c->use_tc && w.op_ok && rows >= 16 && ty >= 0 && tc_handles(c, ty, M.e, M.ff, true) && tc_handles(c, ty, M.ff, M.e, false)) {
         if (!op_ready)
             if ((rc = launch_operand_rows(c, st, ty, x, M.e, rows, M.e, w.op_x, "operand_rows_x"))) return rc;
         if ((rc = launch_grouped_tc(c, st, ty, true, w.seg_sh_gu, w.one, 1, M.e, M.ff, w.op_x, nullptr, w.act))) return rc;
@@ -564,6 +571,7 @@ int dnb_init(int device, dnb_ctx** out) {
     dnb_ctx* c = new dnb_ctx();
     c->device = device;
     c->sm_count = prop.multiProcessorCount;
+    DNB_CUDA(cudaDeviceGetAttribute(&c->smem_base, cudaDevAttrReservedSharedMemoryPerBlock, device));
     DNB_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     DNB_CUDA(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
     DNB_CUDA(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
@@ -650,6 +658,7 @@ int dnb_sync(dnb_ctx* c) {
     DNB_CUDA(cudaStreamSynchronize(c->side));
     const int st = *reinterpret_cast<volatile int*>(c->status_host);
     if (st != 0) {  // sticky until dnb_clear_status: the device-pointer calls since then cannot be trusted
+        retire_smem_base(c, st);
         set_error("sync: a bounded device wait gave up (status %d) since the status was last cleared", st);
         return DNB_DECLINED;
     }
@@ -684,6 +693,15 @@ int dnb_set_wait_limits(dnb_ctx* c, int barrier_polls, int flag_polls, int barri
     c->barrier_polls = barrier_polls;
     c->flag_polls = flag_polls;
     c->barrier_bias = (unsigned int)barrier_bias;
+    return DNB_OK;
+}
+
+int dnb_set_smem_base(dnb_ctx* c, int bytes) {
+    if (!c || bytes < 0) return DNB_ERR_ARG;
+    DNB_CUDA(cudaSetDevice(c->device));
+    DNB_CUDA(cudaDeviceSynchronize());
+    c->smem_base = bytes;
+    drop_graphs(c);
     return DNB_OK;
 }
 
@@ -1215,7 +1233,7 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
     // Matrices of the model's own shapes with enough rows per segment go to the tcgen05 grouped GEMM, the others to the mma.sync
     // kernel (four rows per segment: where decoding a weight once per 32 tokens starts to pay for the 128-row tiles).
     const bool in_e = t.n_in == M.e, in_ff = t.n_in == M.ff;
-    bool on_tc = c->use_tc && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(t.type, t.n_in, t.n_out, false);
+    bool on_tc = c->use_tc && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(c, t.type, t.n_in, t.n_out, false);
     if (on_tc) {
         if ((rc = ensure_ws(c, (int)((row + M.k) / (M.k + 1))))) return rc;
         on_tc = c->ws.op_ok;
@@ -1457,7 +1475,7 @@ int dnb_expert_rows_dev(dnb_ctx* c, int layer, const float* x_rows_dev, const in
     int rc = ensure_ws(c, rows);
     if (rc) return rc;
     Workspace& w = c->ws;
-    const bool tc_routed = !use_shared && tc_type(L, 0, 3) >= 0 && tc_handles(L.m[0].type, M.e, M.ff, true) && tc_handles(L.m[2].type, M.ff, M.e, false);
+    const bool tc_routed = !use_shared && tc_type(L, 0, 3) >= 0 && tc_handles(c, L.m[0].type, M.e, M.ff, true) && tc_handles(c, L.m[2].type, M.ff, M.e, false);
     const bool on_tc = c->use_tc && w.op_ok && rows >= 16;
     if (!use_shared) {
         // every row is one (token, slot): a "chunk" of `rows` tokens with one selected expert each and weight 1

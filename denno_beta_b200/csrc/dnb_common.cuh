@@ -155,6 +155,7 @@ struct dnb_ctx {
     dnb::Scratch gemv_x, gemv_out, gemv_host;   // gemv_host: pinned host staging of dnb_gemv's result
     dnb::Scratch gg_x, gg_out, gg_seg;           // grow-only buffers of dnb_grouped_gemm
     int sm_count = 148;
+    int smem_base = 0;                  // where a CTA's dynamic shared memory starts (what the system keeps per CTA); 0: not known
     int* status = nullptr;              // status word the kernels write when a bounded wait gave up: pinned host memory, device address
     int* status_host = nullptr;         // the same word as the host reads it (valid after a stream synchronisation)
     int barrier_polls = 400000;         // polls of the fused decode kernel's grid barrier before it gives up (~0.2 s)
@@ -380,7 +381,7 @@ int router_topk_dev(dnb_ctx* c, cudaStream_t st, const float* x, int nt, const L
 // matrix; batch = sums in an order that does not depend on the launch's size.  fp32 rows in (row_token names a packed
 // row's input row, null: itself), fp32 packed rows out.  rows, nseg_est: token rows and active segments (an estimate where the
 // device counts them; it only steers the split of the work).  DNB_DECLINED = type or shape not covered, nothing launched.
-bool mm_handles(int type, int n_in);
+bool mm_handles(const dnb_ctx* c, int type, int n_in);
 int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name);
@@ -392,7 +393,7 @@ int launch_gemv_mma(dnb_ctx* c, cudaStream_t st, int type, const uint8_t* w, int
 // tc_row_pitch(n_in) numbers each, one after the other.  launch_operand_rows makes them from fp32 rows; rows_dev (optional): the
 // device's count of rows, at most `rows`.
 size_t tc_row_pitch(int n_in);
-bool tc_handles(int type, int n_in, int n_out, bool fused);
+bool tc_handles(const dnb_ctx* c, int type, int n_in, int n_out, bool fused);
 int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, int ldx, int rows, int n_in, uint16_t* op, const char* name,
                         const int32_t* rows_dev = nullptr);
 // fused: seg[].wa / wb = gate / up, out = silu(g) * u; otherwise seg[].wa.  fp32 packed rows out, or where row_dst says (expert

@@ -46,7 +46,9 @@ constexpr int kMmWarps = 16;
 constexpr int kMmThreads = kMmWarps * 32;
 constexpr int kMmSegMax = 1088;  // segments of a launch at most
 constexpr int kMmFixed = ((kMmSegMax + 4 + 16) * 4 + 127) / 128 * 128;  // segment table and the like in shared memory
-constexpr uint32_t kMmSmemBase = 1024;    // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
+// Where dynamic shared memory has to start for IQ3_XXS, whose tables' address is part of the instructions (as a register it costs 1.5 to 2 % of a
+// batch).  The context knows where it starts (smem_base), and elsewhere mm_handles leaves the format to other kernels.
+constexpr uint32_t kMmSmemBase = 1024;
 constexpr int kMmTok = 2;        // tokens of a column tile: eight columns, four digits a token
 
 // 256 elements of a row: bytes, and the pitch of a stage's rows with one and with two of them (a multiple of 16; a format whose blocks are
@@ -796,7 +798,7 @@ template <int T, bool FUSED, int NT>
 __global__ void __launch_bounds__(kMmThreads, 1) mm_kernel(const MmArgs A) {
     constexpr int TT = NT * kMmTok;  // tokens of an item
     extern __shared__ __align__(128) uint8_t smem[];
-    if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right
+    if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right: the context was told wrong
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
     }
@@ -852,8 +854,9 @@ static int launch_mm_t(dnb_ctx* c, cudaStream_t st, MmArgs A, size_t smem, int g
     return DNB_OK;
 }
 
-bool mm_handles(int type, int n_in) {
-    return (type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_Q8_0 || type == T_IQ3_XXS) && n_in % 256 == 0 && n_in > 0;
+bool mm_handles(const dnb_ctx* c, int type, int n_in) {
+    return (type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_Q8_0 || (type == T_IQ3_XXS && c->smem_base == (int)kMmSmemBase)) && n_in % 256 == 0 &&
+           n_in > 0;
 }
 
 template <int T>
@@ -890,7 +893,7 @@ static size_t mm_ring(int type, int blocks, int warps, size_t base, size_t cap, 
 int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max,
               int nseg_est, int rows, int n_in, int n_out, const float* x, int ldx, const int32_t* row_token, float* out,
               const SegDesc* single, const char* name) {
-    if (!mm_handles(type, n_in) || n_out < 1 || (fused && n_out % 8) || nseg_max < 1 || nseg_max > kMmSegMax || rows < 1) return DNB_DECLINED;
+    if (!mm_handles(c, type, n_in) || n_out < 1 || (fused && n_out % 8) || nseg_max < 1 || nseg_max > kMmSegMax || rows < 1) return DNB_DECLINED;
     if (!seg && !single) return DNB_ERR_ARG;
     if ((((uintptr_t)x) & 15) || ldx % 4 || (single && ((((uintptr_t)single->wa) & 15) || (fused && (((uintptr_t)single->wb) & 15))))) return DNB_DECLINED;
     int rc = type == T_IQ3_XXS ? upload_mm_s8(c->device) : DNB_OK;
@@ -983,7 +986,7 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
     p += 2 * kGvWarps * 16 * TOK * 4;
     uint8_t* xs = p + (size_t)warp * kb_max * XB;
     p += (size_t)kGvWarps * kb_max * XB;
-    if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right
+    if (T == T_IQ3_XXS && tcp::s32(smem) != kMmSmemBase) {  // the tables' addresses would not be right: the context was told wrong
         if (tid == 0) status_set(A.status, 26);
         return;
     }
@@ -1118,7 +1121,7 @@ static int launch_gv_t(dnb_ctx* c, cudaStream_t st, GvArgs A) {
 }
 
 int launch_gemv_mma(dnb_ctx* c, cudaStream_t st, int type, const uint8_t* w, int k, int n, const float* x, float* out, int nvec) {
-    if (!mm_handles(type, k) || n < 1 || nvec < 1 || (((uintptr_t)w) & 15) || (((uintptr_t)x) & 15)) return DNB_DECLINED;
+    if (!mm_handles(c, type, k) || n < 1 || nvec < 1 || (((uintptr_t)w) & 15) || (((uintptr_t)x) & 15)) return DNB_DECLINED;
     const int rc = type == T_IQ3_XXS ? upload_mm_s8(c->device) : DNB_OK;
     if (rc) return rc;
     GvArgs A = {};

@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) grouped_tc_kernel(const Args A) {
         p = book + sizeof(MmCodebook);
     }
     uint8_t* raw_base = p;
-    if ((uint32_t)(raw_base + L::TAIL - smem_raw) > A.smem) {  // only if shared memory started elsewhere
+    if ((uint32_t)(raw_base + L::TAIL - smem_raw) > A.smem) {  // only if shared memory starts elsewhere than the context was told
         if (threadIdx.x == 0) status_set(A.status, 26);
         return;
     }
@@ -742,16 +742,17 @@ int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, i
     return DNB_OK;
 }
 
-bool tc_handles(int type, int n_in, int n_out, bool fused) {
-    return (type == T_Q4_K || type == T_IQ3_XXS) && n_in % 256 == 0 && n_out % (fused ? tg::TILE_M : 2 * tg::TILE_M) == 0;
+bool tc_handles(const dnb_ctx* c, int type, int n_in, int n_out, bool fused) {
+    return c->smem_base > 0 && (type == T_Q4_K || type == T_IQ3_XXS) && n_in % 256 == 0 && n_out % (fused ? tg::TILE_M : 2 * tg::TILE_M) == 0;
 }
 
 template <int T, bool PAIR>
 static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
     using L = tg::Layout<T>;
-    size_t at = kMmSmemBase + L::LOW + tg::B_BYTES;
+    const size_t base = c->smem_base;  // the parts are on 1 KB and 32 KB boundaries of the address space, wherever the CTA's part of it starts
+    size_t at = (base + 1023) / 1024 * 1024 + L::LOW + tg::B_BYTES;
     if (T == T_IQ3_XXS) at = (at + kMmBookAlign - 1) / kMmBookAlign * kMmBookAlign + sizeof(MmCodebook);
-    const size_t smem = at + L::TAIL - kMmSmemBase;
+    const size_t smem = at + L::TAIL - base;
     static_assert(L::BARS * 8 + 16 + (tg::kMaxSeg + 1) * 4 + 8 + tg::kLocalItems * sizeof(tg::Item) <= L::HEAD, "head too small");
     A.smem = (uint32_t)smem;
     auto kern = tg::grouped_tc_kernel<T, PAIR>;
@@ -765,7 +766,7 @@ static int launch_tc_t(dnb_ctx* c, cudaStream_t st, tg::Args& A) {
 
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
                       int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst) {
-    if (!tc_handles(type, n_in, n_out, fused) || nseg_max > tg::kMaxSeg) return DNB_DECLINED;
+    if (!tc_handles(c, type, n_in, n_out, fused) || nseg_max > tg::kMaxSeg) return DNB_DECLINED;
     int rc = type == T_IQ3_XXS ? upload_mm_tables(c->device) : DNB_OK;
     if (rc) return rc;
     tg::Args A = {};

@@ -30,7 +30,6 @@ __device__ __forceinline__ void k_word(uint32_t w, const KScales& s, uint32_t (&
 // The tables sit on a 32 KB boundary of the shared-memory address space: an entry's address is a shift and one and-or.
 struct MmCodebook { uint2 grid[256 * kLutRep]; uint32_t sgn[128 * 32]; };
 constexpr uint32_t kMmBookAlign = 32768;
-constexpr uint32_t kMmSmemBase = 1024;  // where dynamic shared memory starts (what the system keeps of an SM's shared memory per CTA)
 static __device__ __align__(16) MmCodebook g_mm_codebook;
 static bool g_mm_tables[64] = {false};
 

@@ -97,6 +97,9 @@ class CudaCtx:
     def set_wait_limits(self, barrier_polls=400000, flag_polls=1 << 21, barrier_bias=0):
         check(self.lib.dnb_set_wait_limits(self.h, barrier_polls, flag_polls, barrier_bias))
 
+    def set_smem_base(self, nbytes):
+        check(self.lib.dnb_set_smem_base(self.h, nbytes))
+
     def launch_count(self):
         return int(self.lib.dnb_launch_count(self.h))
 

@@ -87,13 +87,14 @@ uint64_t dnb_launch_count(dnb_ctx* ctx);
  *   24       expert-parallel decode: a peer's result rows did not arrive
  *   23       grid barrier of the fused one-token kernel
  *   25       the tensor-core router GEMM of a prefill chunk (stage or accumulator barrier)
- *   26       no wait: a grouped kernel (mma.sync or tcgen05) found its shared memory laid out otherwise than it asked for
+ *   26       no wait: a grouped kernel (mma.sync or tcgen05) found its shared memory to start elsewhere than the context has it
  * What the reference promises for a GPU call that did not complete -- "false: out
  * untouched, the caller recomputes" (cuda.rs:21024-21027, 8785-8788) -- holds here too:
  * every host-buffer entry point reads the word after its stream synchronisation and, when
  * it is non-zero, copies nothing to the caller, clears the word and returns DNB_DECLINED
  * (after a 23 the context also stops using the one-kernel decode form: the two-launch
- * form has no inter-CTA wait).  Device-pointer entry points are asynchronous; for them the
+ * form has no inter-CTA wait; after a 26 the kernels that depend on where shared memory
+ * starts, so that a retry is served by others).  Device-pointer entry points are asynchronous; for them the
  * word stays set until dnb_clear_status, dnb_device_status reads it and dnb_sync returns
  * DNB_DECLINED while it is non-zero. */
 int dnb_device_status(dnb_ctx* ctx, int* status);
@@ -104,6 +105,11 @@ int dnb_clear_status(dnb_ctx* ctx);
  * the barrier unreachable and the time-out path can be exercised without faulting or
  * hanging anything; 0 in production. */
 int dnb_set_wait_limits(dnb_ctx* ctx, int barrier_polls, int flag_polls, int barrier_bias);
+/* Where a CTA's own shared memory starts, in bytes: what the system keeps of an SM's shared memory per CTA.
+ * dnb_init asks the device for it.  The mma.sync kernels serve IQ3_XXS only where it is 1024 (the address of
+ * their tables is part of the instructions); 0, or after a status 26: neither those nor the tcgen05 kernel are used
+ * (other kernels serve every call).  A test hook. */
+int dnb_set_smem_base(dnb_ctx* ctx, int bytes);
 /* Device-side timing on the context's stream: start, ... calls ..., stop -> ms. */
 int dnb_timer_start(dnb_ctx* ctx);
 int dnb_timer_stop(dnb_ctx* ctx, float* ms);

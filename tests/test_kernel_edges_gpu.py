@@ -140,6 +140,37 @@ def test_gemv_edges(orc, ctx, name, k, n, nvec):
     assert rel_err(got[:nvec], want) <= 2e-5
 
 
+@pytest.mark.parametrize("base", [0, 2048])
+def test_shared_memory_that_starts_elsewhere(orc, ctx, base):
+    """IQ3_XXS where the tables of the mma.sync kernels would not be where their instructions look for them: other kernels serve every call.  A
+    context that is told wrong learns it from the first tcgen05 call, which is declined, and the second one is served."""
+    from denno_beta_b200 import cuda as cu
+
+    e, ff, ne, k = 512, 256, 8, 2
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, orc.IQ3_XXS, e, ff, ne, k)
+    w = orc.synth_blocks(orc.IQ3_XXS, SEED, 190, 300 * e // 256)
+    assert ctx.register_matrix(190, orc.IQ3_XXS, w, e, 300)
+    h = orc.synth_normal(SEED, 191, 1.0, 64 * e).reshape(64, e)
+    ctx.set_smem_base(base)
+    ctx.profile(True)
+    for nt in (1, 2, 9, 24):
+        for _ in range(3):  # the third one replays
+            out, sels, wts = ctx.moe_block(0, h[:nt], want_routing=True)
+            assert check_block(orc, L, h[:nt], out, sels, wts)[0] <= 2e-4
+    out = ctx.moe_experts(0, h[:4], sels[:4], wts[:4])
+    assert rel_err(out, orc.moe_experts_given(L, h[:4], sels[:4], wts[:4])) <= 5e-5
+    got = np.empty(300, np.float32)
+    assert ctx.gemv(190, h[0], got)
+    assert rel_err(got, orc.gemv_scalar(orc.IQ3_XXS, w, e, 300, h[0])) <= 2e-5
+    assert not [n for n in ctx.profile_read() if n.startswith(("mm_", "gemv_mma"))]
+    ctx.profile(False)
+    if base:
+        assert ctx.moe_block(0, h) is None
+    out, sels, wts = ctx.moe_block(0, h, want_routing=True)
+    assert check_block(orc, L, h, out, sels, wts)[0] <= 2e-4
+
+
 @pytest.mark.parametrize("hc,lr,nts", [(1, 8, (1, 9)), (2, 33, (1, 8)), (3, 320, (2, 17))])
 def test_hyper_edges(orc, ctx, hc, lr, nts):
     """Streams, ranks that end inside a CTA's rows, and more tokens than a CTA takes at once."""
