@@ -27,8 +27,8 @@
 //     cycles) and stores them.  The block's scales go to a small ring, its mins to shared memory of the thread's own.
 //   * two MMA threads, a tile each.  A block's weights stay in tensor memory while they are multiplied with the lo rows and then with the hi
 //     rows, into the same columns: with 64 tokens there are two accumulator buffers (with sums of hi and lo apart there was room for
-//     one, and the tensor core waited 350 cycles of a stage's 1,060 while it was read), and as lo comes first, the sums are rounded as often
-//     as those of hi alone: the distance from 64 bits is what it was (0.998 of it over 48 forms).  A wait, a fence and a commit are some 200
+//     one, and the tensor core waited 350 cycles of a stage's 1,060 while it was read), and as lo comes first, the sums are rounded once more
+//     than those of hi alone (what that costs is in operand_rows.cuh, and why the result is no less exact).  A wait, a fence and a commit are some 200
 //     cycles of a thread's time, so two stages share them, and one thread for both tiles would be the bottleneck.
 //   * eight epilogue warps, two accumulator buffers (thread = weight row, half of the token columns of both tiles).
 // Persistent, one CTA per SM; items (segment, up to 64 tokens, 128 rows x 2) dealt round-robin.
