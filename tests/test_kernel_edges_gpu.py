@@ -119,8 +119,10 @@ def test_experts_given_mixed(orc, ctx, up, down, e, ff):
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
-@pytest.mark.parametrize("k,n,nvec", [(256, 1, 1), (768, 15, 2), (2304, 17, 3), (512, 2369, 8), (4096, 33, 1)])
+@pytest.mark.parametrize("k,n,nvec", [(256, 1, 1), (768, 15, 2), (2304, 17, 3), (512, 2369, 8), (4096, 33, 1), (4352, 33, 1), (4864, 17, 2), (8448, 15, 1)])
 def test_gemv_edges(orc, ctx, name, k, n, nvec):
+    """Rows that end inside a group of 16, vectors in pairs and an odd one, K of 1 to 33 blocks: 17, 19 and 33 are two a stage with a last stage of
+    one."""
     ty = orc.TYPE_BY_NAME[name]
     w = orc.synth_blocks(ty, SEED, 70 + ty, n * k // orc.blck_size(ty))
     x = orc.synth_normal(SEED, 71, 1.0, nvec * k).reshape(nvec, k)
@@ -342,6 +344,26 @@ def test_small_elements_beside_large_ones_grouped(orc, ctx, name, sizes):
             rows, d = slice(at[i], at[i + 1]), deq[ne - 1 - i]
             off = np.abs(got[rows] - xs[rows].astype(np.float64) @ d.T) / _small_elements_bound(name, xs[rows], d)
             assert off.max() <= 1.0, (j, i, off.max())
+
+
+@pytest.mark.parametrize("up,down", [("Q4_K", "Q6_K"), ("Q5_K", "Q8_0"), ("IQ3_XXS", "IQ3_XXS"), ("Q8_0", "Q4_K")])
+def test_block_with_outliers(orc, ctx, up, down):
+    """Tokens with an element far above the others in a block on the fused gate/up kernel; the other tokens do not feel them."""
+    e, ff, ne, k = 1024, 512, 16, 3
+    up, down = orc.TYPE_BY_NAME[up], orc.TYPE_BY_NAME[down]
+    assert ctx.moe_config(1, e, ff, ne, k)
+    L = make_layer(orc, ctx, 0, up, e, ff, ne, k, ty_down=down)
+    for nt in (2, 9, 15, 40):
+        h = orc.synth_normal(SEED, 210 + nt, 1.0, nt * e).reshape(nt, e)
+        plain = ctx.moe_block(0, h)
+        loud = h.copy()
+        for i, at in ((1, 300), (4, 37), (7, 1000)):
+            if i < nt:
+                loud[i, at] = 2.0 ** (8 + 3 * i)
+        out, sels, wts = ctx.moe_block(0, loud, want_routing=True)
+        assert check_block(orc, L, loud, out, sels, wts)[0] <= 5e-5
+        same = np.all(loud == h, axis=1)
+        assert np.array_equal(out[same].view(np.uint32), plain[same].view(np.uint32)), nt
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "IQ3_XXS"])
