@@ -6,8 +6,10 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 #include <stddef.h>
+#include <atomic>
 #include <functional>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -339,6 +341,22 @@ inline cudaError_t grant_smem(SmemGrant& g, int device, K kern, size_t bytes) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess) g.got[device] = bytes;
     return e;
+}
+
+// A translation unit's constant tables, copied to a device by the first call that needs them.  A copy from pageable memory may return before
+// it has reached the device, and the contexts' streams do not wait for the legacy stream that it is in: it is waited for before any call goes
+// on.  Contexts of several threads may come at once: one copies, the others wait.
+struct TablesOnce { std::mutex mutex; std::atomic<bool> up[64] = {}; };
+template <class F>  // copy(): cudaMemcpyToSymbol calls, DNB_OK or an error
+inline int tables_once(TablesOnce& t, int device, F copy) {
+    if (device < 0 || device >= 64) return DNB_ERR_ARG;
+    if (t.up[device].load(std::memory_order_acquire)) return DNB_OK;
+    std::lock_guard<std::mutex> lock(t.mutex);
+    if (t.up[device].load(std::memory_order_relaxed)) return DNB_OK;
+    if (const int rc = copy()) return rc;
+    DNB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    t.up[device].store(true, std::memory_order_release);
+    return DNB_OK;
 }
 
 // One-token IQ3_XXS gate/up GEMV on mma.sync (gemv_mma.cu); DNB_DECLINED when the shape does not fit.

@@ -24,16 +24,15 @@ namespace dnb {
 // The IQ3_XXS codebook in the replicated layout of IqLut, ready to be bulk-copied into a
 // CTA's shared memory (a constant of the library: requested before any wait on other kernels).
 __device__ __align__(16) uint32_t g_grid3xxs_rep[256 * kLutRep];
-static bool g_tables_b[64] = {false};
+static TablesOnce g_tables_b;
 
 static int upload_tables_b(int device) {
-    if (device < 0 || device >= 64) return DNB_ERR_ARG;
-    if (g_tables_b[device]) return DNB_OK;
-    static uint32_t rep[256 * kLutRep];
-    for (int i = 0; i < 256 * kLutRep; ++i) rep[i] = dnb_iq3xxs_grid[i / kLutRep];
-    DNB_CUDA(cudaMemcpyToSymbol(g_grid3xxs_rep, rep, sizeof(rep)));
-    g_tables_b[device] = true;
-    return DNB_OK;
+    return tables_once(g_tables_b, device, [] {
+        static uint32_t rep[256 * kLutRep];
+        for (int i = 0; i < 256 * kLutRep; ++i) rep[i] = dnb_iq3xxs_grid[i / kLutRep];
+        DNB_CUDA(cudaMemcpyToSymbol(g_grid3xxs_rep, rep, sizeof(rep)));
+        return DNB_OK;
+    });
 }
 
 __device__ __forceinline__ float silu_b(float v) { return v / (1.0f + expf(-v)); }

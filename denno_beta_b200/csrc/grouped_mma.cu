@@ -230,26 +230,25 @@ __device__ __forceinline__ MmK mm_k_header(const uint8_t* row, int t) {
 // They are the first thing in shared memory, an address that the instructions hold.
 struct MmTables { uint32_t grid[256 * 32]; uint2 sgn[128 * 16]; };
 static __device__ __align__(16) MmTables g_mm_s8;
-static bool g_mm_s8_up[64] = {false};
+static TablesOnce g_mm_s8_up;
 
 static int upload_mm_s8(int device) {
-    if (device < 0 || device >= 64) return DNB_ERR_ARG;
-    if (g_mm_s8_up[device]) return DNB_OK;
-    static MmTables tb;
-    for (int e = 0; e < 256; ++e)
-        for (int r = 0; r < 32; ++r) tb.grid[e * 32 + r] = dnb_iq3xxs_grid[e];
-    for (uint32_t code = 0; code < 128; ++code) {
-        const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
-        uint2 u = make_uint2(0u, 0u);
-        for (int i = 0; i < 4; ++i) {
-            u.x |= ((sg >> i) & 1u) << (8 * i);
-            u.y |= ((sg >> (4 + i)) & 1u) << (8 * i);
+    return tables_once(g_mm_s8_up, device, [] {
+        static MmTables tb;
+        for (int e = 0; e < 256; ++e)
+            for (int r = 0; r < 32; ++r) tb.grid[e * 32 + r] = dnb_iq3xxs_grid[e];
+        for (uint32_t code = 0; code < 128; ++code) {
+            const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
+            uint2 u = make_uint2(0u, 0u);
+            for (int i = 0; i < 4; ++i) {
+                u.x |= ((sg >> i) & 1u) << (8 * i);
+                u.y |= ((sg >> (4 + i)) & 1u) << (8 * i);
+            }
+            for (int r = 0; r < 16; ++r) tb.sgn[code * 16 + r] = u;
         }
-        for (int r = 0; r < 16; ++r) tb.sgn[code * 16 + r] = u;
-    }
-    DNB_CUDA(cudaMemcpyToSymbol(g_mm_s8, &tb, sizeof(tb)));
-    g_mm_s8_up[device] = true;
-    return DNB_OK;
+        DNB_CUDA(cudaMemcpyToSymbol(g_mm_s8, &tb, sizeof(tb)));
+        return DNB_OK;
+    });
 }
 
 // Eight weights of an IQ3_XXS sub-block as signed bytes.  gl, sl: where the lane's copies are in an entry; idx: the two codebook indices; code:

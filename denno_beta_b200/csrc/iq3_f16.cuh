@@ -31,26 +31,25 @@ __device__ __forceinline__ void k_word(uint32_t w, const KScales& s, uint32_t (&
 struct MmCodebook { uint2 grid[256 * kLutRep]; uint32_t sgn[128 * 32]; };
 constexpr uint32_t kMmBookAlign = 32768;
 static __device__ __align__(16) MmCodebook g_mm_codebook;
-static bool g_mm_tables[64] = {false};
+static TablesOnce g_mm_tables;
 
 static int upload_mm_tables(int device) {
-    if (device < 0 || device >= 64) return DNB_ERR_ARG;
-    if (g_mm_tables[device]) return DNB_OK;
-    static MmCodebook tb;
-    for (int e = 0; e < 256; ++e) {
-        uint32_t h[4];
-        for (int j = 0; j < 4; ++j) h[j] = __half_as_ushort(__float2half((float)((dnb_iq3xxs_grid[e] >> (8 * j)) & 0xFFu)));
-        for (int r = 0; r < kLutRep; ++r) tb.grid[e * kLutRep + r] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-    }
-    for (uint32_t code = 0; code < 128; ++code) {
-        const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
-        uint32_t u = 0;
-        for (int q = 0; q < 4; ++q) u |= ((sg >> (2 * q)) & 1u) << (15 - q) | ((sg >> (2 * q + 1)) & 1u) << (31 - q);
-        for (int r = 0; r < 32; ++r) tb.sgn[code * 32 + r] = u;
-    }
-    DNB_CUDA(cudaMemcpyToSymbol(g_mm_codebook, &tb, sizeof(tb)));
-    g_mm_tables[device] = true;
-    return DNB_OK;
+    return tables_once(g_mm_tables, device, [] {
+        static MmCodebook tb;
+        for (int e = 0; e < 256; ++e) {
+            uint32_t h[4];
+            for (int j = 0; j < 4; ++j) h[j] = __half_as_ushort(__float2half((float)((dnb_iq3xxs_grid[e] >> (8 * j)) & 0xFFu)));
+            for (int r = 0; r < kLutRep; ++r) tb.grid[e * kLutRep + r] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+        }
+        for (uint32_t code = 0; code < 128; ++code) {
+            const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
+            uint32_t u = 0;
+            for (int q = 0; q < 4; ++q) u |= ((sg >> (2 * q)) & 1u) << (15 - q) | ((sg >> (2 * q + 1)) & 1u) << (31 - q);
+            for (int r = 0; r < 32; ++r) tb.sgn[code * 32 + r] = u;
+        }
+        DNB_CUDA(cudaMemcpyToSymbol(g_mm_codebook, &tb, sizeof(tb)));
+        return DNB_OK;
+    });
 }
 
 // Eight weights of an IQ3_XXS sub-block as four signed fp16 pairs.  gl, sl: shared addresses of the lane's copies; idx: the two

@@ -28,32 +28,31 @@ struct Iq3Tables {
     uint32_t sgn[128 * kLutRep];
 };
 static __device__ __align__(16) Iq3Tables g_iq3_tables;
-static bool g_tables_m[64] = {false};
+static TablesOnce g_tables_m;
 
 static int upload_tables_m(int device) {
-    if (device < 0 || device >= 64) return DNB_ERR_ARG;
-    if (g_tables_m[device]) return DNB_OK;
-    static Iq3Tables tb;
-    for (int e = 0; e < 256; ++e) {
-        const uint32_t w = dnb_iq3xxs_grid[e];
-        uint32_t h[4];
-        for (int j = 0; j < 4; ++j) {
-            const float f = (float)((w >> (8 * j)) & 0xFFu);  // <= 62: its fp32 pattern has nothing below bit 16
-            uint32_t bits;
-            memcpy(&bits, &f, 4);
-            h[j] = bits >> 16;
+    return tables_once(g_tables_m, device, [] {
+        static Iq3Tables tb;
+        for (int e = 0; e < 256; ++e) {
+            const uint32_t w = dnb_iq3xxs_grid[e];
+            uint32_t h[4];
+            for (int j = 0; j < 4; ++j) {
+                const float f = (float)((w >> (8 * j)) & 0xFFu);  // <= 62: its fp32 pattern has nothing below bit 16
+                uint32_t bits;
+                memcpy(&bits, &f, 4);
+                h[j] = bits >> 16;
+            }
+            for (int r = 0; r < kLutRep; ++r) tb.grid[e * kLutRep + r] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
         }
-        for (int r = 0; r < kLutRep; ++r) tb.grid[e * kLutRep + r] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-    }
-    for (uint32_t code = 0; code < 128; ++code) {
-        const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
-        uint32_t u = 0;
-        for (int q = 0; q < 4; ++q) u |= ((sg >> (2 * q)) & 1u) << (15 - q) | ((sg >> (2 * q + 1)) & 1u) << (31 - q);
-        for (int r = 0; r < kLutRep; ++r) tb.sgn[code * kLutRep + r] = u;
-    }
-    DNB_CUDA(cudaMemcpyToSymbol(g_iq3_tables, &tb, sizeof(tb)));
-    g_tables_m[device] = true;
-    return DNB_OK;
+        for (uint32_t code = 0; code < 128; ++code) {
+            const uint32_t sg = code | ((uint32_t)(__builtin_popcount(code) & 1) << 7);
+            uint32_t u = 0;
+            for (int q = 0; q < 4; ++q) u |= ((sg >> (2 * q)) & 1u) << (15 - q) | ((sg >> (2 * q + 1)) & 1u) << (31 - q);
+            for (int r = 0; r < kLutRep; ++r) tb.sgn[code * kLutRep + r] = u;
+        }
+        DNB_CUDA(cudaMemcpyToSymbol(g_iq3_tables, &tb, sizeof(tb)));
+        return DNB_OK;
+    });
 }
 // A lane's view of the tables in shared memory: the addresses of its own copies
 struct Iq3Lane {

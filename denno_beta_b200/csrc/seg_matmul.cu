@@ -21,17 +21,16 @@ __constant__ uint32_t c_iq3xxs_grid[256];
 __constant__ uint32_t c_iq3s_grid[512];
 __constant__ unsigned long long c_iq2s_grid[1024];
 __constant__ int8_t c_kvalues_iq4nl[16];
-static bool g_tables_uploaded[64] = {false};
+static TablesOnce g_tables_uploaded;
 
 static int upload_tables(int device) {
-    if (device < 0 || device >= 64) return DNB_ERR_ARG;
-    if (g_tables_uploaded[device]) return DNB_OK;
-    DNB_CUDA(cudaMemcpyToSymbol(c_iq3xxs_grid, dnb_iq3xxs_grid, sizeof(c_iq3xxs_grid)));
-    DNB_CUDA(cudaMemcpyToSymbol(c_iq3s_grid, dnb_iq3s_grid, sizeof(c_iq3s_grid)));
-    DNB_CUDA(cudaMemcpyToSymbol(c_iq2s_grid, dnb_iq2s_grid, sizeof(c_iq2s_grid)));
-    DNB_CUDA(cudaMemcpyToSymbol(c_kvalues_iq4nl, dnb_kvalues_iq4nl, sizeof(c_kvalues_iq4nl)));
-    g_tables_uploaded[device] = true;
-    return DNB_OK;
+    return tables_once(g_tables_uploaded, device, [] {
+        DNB_CUDA(cudaMemcpyToSymbol(c_iq3xxs_grid, dnb_iq3xxs_grid, sizeof(c_iq3xxs_grid)));
+        DNB_CUDA(cudaMemcpyToSymbol(c_iq3s_grid, dnb_iq3s_grid, sizeof(c_iq3s_grid)));
+        DNB_CUDA(cudaMemcpyToSymbol(c_iq2s_grid, dnb_iq2s_grid, sizeof(c_iq2s_grid)));
+        DNB_CUDA(cudaMemcpyToSymbol(c_kvalues_iq4nl, dnb_kvalues_iq4nl, sizeof(c_kvalues_iq4nl)));
+        return DNB_OK;
+    });
 }
 
 // The CTA's copy of the format's codebook, behind the one pointer decode_unit takes.

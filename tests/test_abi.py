@@ -95,3 +95,17 @@ def test_product_never_touches_the_oracle():
                 if re.search(r"\boracle\b|dnb_oracle|orc_", text):
                     bad.append(os.path.join(dirpath, f))
     assert not bad, "library files that mention the oracle: %s" % bad
+
+
+def test_constant_tables_are_there_before_any_call_goes_on():
+    """A device's constant tables are copied under a lock, and the copy is waited for before another call may take them as present: contexts of
+    several threads share them, and no stream of theirs waits for the stream of the copy."""
+    csrc = os.path.join(ROOT, "denno_beta_b200", "csrc")
+    text = {f: open(os.path.join(csrc, f)).read() for f in os.listdir(csrc) if f.endswith((".cu", ".cuh"))}
+    helper = re.search(r"inline int tables_once\(.*?\n\}\n", text["dnb_common.cuh"], re.S)
+    assert helper, "no helper"
+    steps = [helper.group(0).find(s) for s in ("lock_guard", "copy()", "cudaStreamSynchronize", "store(true")]
+    assert -1 not in steps and steps == sorted(steps)
+    for f, s in text.items():
+        guarded = re.findall(r"return tables_once\(.*?\n    \}\);\n", s, re.S)
+        assert s.count("cudaMemcpyToSymbol(") == sum(g.count("cudaMemcpyToSymbol(") for g in guarded), f

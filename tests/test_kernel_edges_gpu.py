@@ -452,3 +452,45 @@ def test_tcgen05_many_items(orc, ctx, name, segments):
     ctx.profile(False)
     assert "tc_down" in launched, sorted(launched)
     assert rel_err(got, orc.grouped_gemm(ty, w, k, n, segs, x)) <= 2e-5
+
+
+FIRST_CALLS = """
+import threading
+import numpy as np
+from denno_beta_b200 import cuda as cu
+
+k, n, threads = 1024, 512, 6
+rng = np.random.default_rng(1)
+w = rng.integers(0, 256, n * k // 256 * 98, dtype=np.uint8)
+w.reshape(-1, 98)[:, :2] = np.array([0.01], np.float16).view(np.uint8)
+x = rng.standard_normal(k).astype(np.float32)
+start, got = threading.Barrier(threads), [None] * threads
+
+def first_call(i):
+    c = cu.CudaCtx(0)
+    assert c.register_matrix(1, cu.IQ3_XXS, w, k, n)
+    start.wait()
+    outs = []
+    for _ in range(2):
+        outs.append(np.empty(n, np.float32))
+        assert c.gemv(1, x, outs[-1])
+    got[i] = outs
+    c.close()
+
+workers = [threading.Thread(target=first_call, args=(i,)) for i in range(threads)]
+for t in workers:
+    t.start()
+for t in workers:
+    t.join()
+assert all(np.array_equal(o, got[0][1]) for outs in got for o in outs) and np.abs(got[0][1]).min() > 0
+print("same")
+"""
+
+
+def test_first_calls_of_several_threads():
+    """A process whose first IQ3_XXS calls come from several contexts at once: each finds the tables in place."""
+    import subprocess
+    import sys
+
+    out = subprocess.run([sys.executable, "-c", FIRST_CALLS], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and out.stdout.strip() == "same", out.stderr[-2000:]
