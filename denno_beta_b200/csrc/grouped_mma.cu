@@ -134,7 +134,7 @@ __device__ __forceinline__ bool mm_stage_block(const float* __restrict__ xr, uin
     for (int i = 0; i < 8; ++i) mine = max(mine, __float_as_uint(fabsf(x[i])));
     const uint32_t mx = __reduce_max_sync(0xffffffffu, mine);
     const int ex = (int)((mx + 0x10101u) >> 23);  // biased exponent of the largest |x|, one more where its mantissa is too large
-    const int s = ex == 0 ? 0 : min(149, 157 - ex), s1 = min(s, 120);
+    const int s = min(149, 157 - ex), s1 = min(s, 120);  // 149: every fp32 is an integer, subnormal ones too
     const float up = mm_pow2(s1);
 #pragma unroll
     for (int i = 0; i < 8; ++i) x[i] *= up;

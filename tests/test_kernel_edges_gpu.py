@@ -253,6 +253,33 @@ def test_activations_of_any_size(orc, ctx, name, nvec):
         assert np.all(np.abs(got[i, first:] - want) <= bound), (i, np.max(np.abs(got[i, first:] - want) / bound))
 
 
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("nvec", [1, 2, 5])
+def test_subnormal_activations(orc, ctx, name, nvec):
+    """Blocks whose elements are all below fp32's normal numbers are as exact as any: alone, beside zeros and beside small normal blocks."""
+    ty, k, n = orc.TYPE_BY_NAME[name], 1024, 48
+    w = orc.synth_blocks(ty, SEED, 120 + ty, n * k // orc.blck_size(ty))
+    x = (orc.synth_normal(SEED, 121, 1.0, nvec * k).astype(np.float64) * 2e-39).reshape(nvec, 4, 256)
+    x[-1, 1] = 0.0
+    x[-1, 2] *= 3e4
+    x = x.reshape(nvec, k).astype(np.float32)
+    assert 0 < np.abs(x[0, :256]).max() < 2.0 ** -126
+    dw, dx, do = ctx.dev_alloc(w.nbytes), ctx.dev_alloc(x.nbytes), ctx.dev_alloc(nvec * n * 4)
+    try:
+        ctx.upload(dw, w)
+        ctx.upload(dx, x)
+        assert ctx.gemv_dev(ty, dw, k, n, dx, do, nvec)
+        got = ctx.download(do, np.empty((nvec, n), np.float32))
+    finally:
+        for p in (dw, dx, do):
+            ctx.dev_free(p)
+    deq = orc.dequant_row(ty, w, n * k).reshape(n, k).astype(np.float64)
+    x64 = x.astype(np.float64)
+    # fp32 sums; sums below the normal numbers round to 2^-149: four blocks, of a sum each for low and high digits, and their meeting
+    bound = 2.0 ** -20 * np.sqrt((x64 ** 2) @ (deq ** 2).T) + 16 * 2.0 ** -149
+    assert np.all(np.abs(got - x64 @ deq.T) <= bound), np.max(np.abs(got - x64 @ deq.T) / bound)
+
+
 def _deaf(name, w):
     """Blocks of 256 elements whose weights do not hear element 37: zero, or (IQ3_XXS, which has no zero) the same as element 45's."""
     b = w.reshape(-1, {"Q4_K": 144, "Q5_K": 176, "Q6_K": 210, "Q8_0": 272, "IQ3_XXS": 98}[name])
