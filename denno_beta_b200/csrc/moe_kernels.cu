@@ -818,9 +818,12 @@ combine_kernel(const float* __restrict__ hrow, const int32_t* __restrict__ pos, 
 int launch_combine(dnb_ctx* c, cudaStream_t st, const float* hrow, const int32_t* pos, const float* wts, int nt,
                    int k, int e, const float* sh, const float* shcoef, float* out, const float* residual, bool pdl) {
     ProfScope prof_(c, st, "combine");
-    // Twelve slots' rows at once cost registers, and with them CTAs of an SM: the better choice while there are few.
+    // Twelve slots' rows at once cost registers, and with them CTAs of an SM: the better choice while there are few, and where it saves a round
+    // of loads.  us as bracketed by events, eight / twelve, two CTAs a token of 2048: top 10, 8 tokens 8.3 / 7.6, 64 8.7 / 8.6, 128 8.7 / 8.7, 256 8.8 /
+    // 10.7, 512 12.8 / 14.6; top 8, 64 tokens 7.6 / 8.7; top 4, 8 tokens 6.7 / 7.3, 64 6.9 / 8.6, 128 7.1 / 8.6.
     const dim3 grid(nt, (e + 1023) / 1024);
-    auto kern = (int)(grid.x * grid.y) <= 2 * c->sm_count ? combine_kernel<12> : combine_kernel<8>;
+    const bool few = (int)(grid.x * grid.y) <= 2 * c->sm_count, fewer_rounds = (k + 11) / 12 < (k + 7) / 8;
+    auto kern = few && fewer_rounds ? combine_kernel<12> : combine_kernel<8>;
     DNB_CUDA(launch_k(kern, grid, dim3(256), 0, st, c->use_pdl && pdl, hrow, pos, wts, k, e, sh, shcoef, residual, out));
     c->launches++;
     return DNB_OK;
