@@ -365,10 +365,13 @@ static int tc_type(const Layer& L, int first, int last) {
         if (!L.m[i].dev || L.m[i].type != ty) return -1;
     return ty;
 }
-// Tokens from which a chunk or decode batch leaves the mma.sync kernel for the tcgen05 grouped GEMM.  A stage of the latter costs the
-// same for one token as for 32, so the line depends on how many tokens share an expert, which the host does not know.  us per layer at
-// 2048 x 512, top 10 of 512, mma.sync / tcgen05: Q4_K evenly routed 173 / 222 at 32 tokens, 216 / 275 at 48, 250 / 304 at 64; under a
-// skewed router 106 / 96, 129 / 100, 155 / 103.  At 48 either choice loses the same factor at worst (1.27).
+// Tokens from which a chunk or decode batch leaves the mma.sync kernel for the tcgen05 grouped GEMM.  A stage of the latter costs nearly
+// the same for one token as for 64, so the line depends on how many tokens share an expert, which the host does not know.  us per layer at
+// 2048 x 512, top 10 of 512, mma.sync / tcgen05, 32, 40, 48, 64 tokens: Q4_K evenly routed 136 / 195, 178 / 217, 194 / 241, 220 / 270, skewed by
+// -1.1 ln rank 106 / 85, 107 / 86, 117 / 87, 140 / 93; IQ3_XXS 183 / 220, 231 / 246, 250 / 273, 285 / 309, skewed 141 / 93, 131 / 93, 142 / 95, 172 /
+// 100.  At 48 the wrong choice costs a factor of 1.24 or 1.35 (Q4_K), 1.09 or 1.50 (IQ3_XXS).  The line was drawn for earlier forms of both kernels,
+// where it was 1.27 either way; with these the factors meet at about 40 and 24 tokens.  A token's bits change at the line, so it stays until that is
+// worth it.
 constexpr int kTcMin = 48;
 static int tc_min_tokens(const dnb_ctx* c, int ty) { return ty == T_Q4_K ? kTcMin : c->tc_min_iq3; }
 
@@ -1231,7 +1234,11 @@ int dnb_grouped_gemm(dnb_ctx* c, int layer, int matrix, const uint32_t* segs, in
     int32_t* dnseg = (int32_t*)((uint8_t*)c->gg_seg.p + (size_t)nseg * sizeof(SegDesc));
     const Model& M = c->model;
     // Matrices of the model's own shapes with enough rows per segment go to the tcgen05 grouped GEMM, the others to the mma.sync
-    // kernel (four rows per segment: where decoding a weight once per 32 tokens starts to pay for the 128-row tiles).
+    // kernel.  us, operand rows and tcgen05 / mma.sync, segments of 4, 6, 8, 12, 16, 32 rows, 128 of them: Q4_K 2048 x 512 48 / 37, 49 / 49, 50 /
+    // 51, 52 / 74, 53 / 80, 63 / 140, 512 x 2048 49 / 31, 51 / 41, 50 / 41, 51 / 62, 51 / 70, 58 / 129, IQ3_XXS 54 / 44, 55 / 55, 55 / 56, 59 / 88, 60 /
+    // 94, 69 / 172; 16 of them: Q4_K 2048 x 512 32 / 15, 32 / 17, 32 / 17, 32 / 23, 32 / 25, 34 / 35, 512 x 2048 22 / 14, 22 / 15, 22 / 15, 22 / 21, 22 /
+    // 21, 23 / 31.  Four rows was the line of earlier forms of both kernels; with these it is six to eight, and 16 to 32 where there are few segments.
+    // The sums' rounding differs between the kernels, so it stays until that is worth it.
     const bool in_e = t.n_in == M.e, in_ff = t.n_in == M.ff;
     bool on_tc = c->use_tc && row >= 64 && row >= (size_t)4 * nseg && (in_e || in_ff) && tc_handles(c, t.type, t.n_in, t.n_out, false);
     if (on_tc) {

@@ -376,9 +376,9 @@ int launch_decode_block(dnb_ctx* c, cudaStream_t st, const Model& M, const Layer
 
 // Router logits of chunks of kRouterTcMin tokens or more on tcgen05 (router_tc.cu)
 constexpr int kRouterSplitMax = 8;  // K splits of the tensor-core router at most (the top-k kernel adds that many partial sums)
-// Calls below take the fp32 kernel in the one-token router's order of adds, and three parts per activation; a token's bits do not
-// depend on its batch within 2 to 15 tokens, within 16 to 47 (mma.sync, three and two parts) and from 48 on (tcgen05; layers that it
-// does not take stay on mma.sync, whose sums are then split by the call's size).
+// Calls below take the fp32 kernel in the one-token router's order of adds; a token's bits do not depend on its batch within 2 to 15
+// tokens, within 16 to 47 (both on mma.sync) and from 48 on (tcgen05; layers that it does not take stay on mma.sync, whose sums are then
+// split by the call's size).
 constexpr int kRouterTcMin = 16;
 int router_tc_prepare(dnb_ctx* c, Layer& L, int ne, int e);
 int router_tc_workspace(dnb_ctx* c, Workspace& w, int cap, int ne, int e);
@@ -415,7 +415,7 @@ bool tc_handles(const dnb_ctx* c, int type, int n_in, int n_out, bool fused);
 int launch_operand_rows(dnb_ctx* c, cudaStream_t st, int type, const float* x, int ldx, int rows, int n_in, uint16_t* op, const char* name,
                         const int32_t* rows_dev = nullptr);
 // fused: seg[].wa / wb = gate / up, out = silu(g) * u; otherwise seg[].wa.  fp32 packed rows out, or where row_dst says (expert
-// parallel).  row_token: packed row -> operand row, null: itself.  tokens, rows: of the call, choose the items' size (0: small).
+// parallel).  row_token: packed row -> operand row, null: itself.
 int launch_grouped_tc(dnb_ctx* c, cudaStream_t st, int type, bool fused, const SegDesc* seg, const int32_t* nseg_dev, int nseg_max, int n_in,
                       int n_out, const uint16_t* op, const int32_t* row_token, float* out, float* const* row_dst = nullptr);
 // The shared expert of a layer on `rows` fp32 rows (api.cu); op_ready: their operand rows are in the workspace already.

@@ -929,7 +929,10 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, con
         const size_t smem = mm_ring(type, nb / ks, kMmWarps, base, 225 * 1024, A.ring);
         if (smem) {
             A.status = c->status;
-            // activations of a tile 2.5 - 3 us, a row group 1.1 us at K = 2048 and a quarter of that at K = 512 (measured, IQ3_XXS)
+            // Activations of a tile 2.5 - 3 us, a row group 1.1 us at K = 2048 and a quarter of that at K = 512 (IQ3_XXS).  us a layer of 2048 x 512, top
+            // 10 of 512, with this many row groups / half / twice / four times as many: 8 tokens IQ3_XXS 80.1 / 82.0 / 79.7 / 83.0, Q4_K 67.9 / 69.5 / 68.0 /
+            // 68.7, Q8_0 87.8 / 90.2 / 86.8 / 88.0; 32 tokens IQ3_XXS 182.5 / 183.0 / 182.7 / 185.9, Q4_K 135.8 / 136.5 / 136.6 / 136.3; Q4_K and Q6_K 77
+            // tokens skewed 187.6 / 188.8 / 187.9 / 191.6, 200 even 482 / 485 / 484 / 486; 1024 x 768, 8 tokens Q4_K 58.0 / 59.1 / 57.7 / 58.5.
             A.skip = std::max(1, 5120 / n_in);
             if ((double)(nseg_max + (rows + nt * tpt - 1) / (nt * tpt)) * (n_rg + A.skip) > 2e9) return DNB_DECLINED;
             const int grid = nseg_dev ? c->sm_count : (int)std::min<long>(c->sm_count, std::max<long>(1, tiles * n_rg * ks / kMmWarps));

@@ -253,6 +253,59 @@ def test_activations_of_any_size(orc, ctx, name, nvec):
         assert np.all(np.abs(got[i, first:] - want) <= bound), (i, np.max(np.abs(got[i, first:] - want) / bound))
 
 
+def _largest_weights(orc, name, n_blocks):
+    """Blocks whose integers are as large as the format has them, of one sign."""
+    if name == "Q8_0":
+        b = np.full((n_blocks * 8, 34), 0x80, np.uint8)
+        b[:, 0:2] = np.array([0.5], np.float16).view(np.uint8)
+        return b
+    b = np.full((n_blocks, {"Q4_K": 144, "Q5_K": 176, "Q6_K": 210, "IQ3_XXS": 98}[name]), 0xFF, np.uint8)
+    if name in ("Q4_K", "Q5_K"):
+        b[:, 0:4] = np.array([0.5, 0.25], np.float16).view(np.uint8)
+    elif name == "Q6_K":
+        b[:, :192] = 0     # q = -32
+        b[:, 192:208] = 0x80
+        b[:, 208:210] = np.array([0.5], np.float16).view(np.uint8)
+    else:
+        b[:, 0:2] = np.array([0.5], np.float16).view(np.uint8)
+        b[:, 66:] = np.array([15 << 28], np.uint32).view(np.uint8).reshape(1, 4).repeat(8, 0).reshape(-1)
+        sums = []
+        for code in range(256):
+            b[0, 2:66] = code
+            sums.append(orc.dequant_row(orc.IQ3_XXS, b[0].copy(), 256).sum())
+        b[:, 2:66] = int(np.argmax(sums))
+    return b
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
+@pytest.mark.parametrize("nvec", [1, 2, 5])
+def test_largest_integer_sums(orc, ctx, name, nvec):
+    """Weights of the largest integers and scales against activations of the largest digits, all of one sign: 0x7e7f7f80 is the digits -128, -128,
+    -128, 127 in base 256, -0x808080 in a block with one large element -128, -128, -128, 0.  Nothing leaves 32 bits."""
+    ty, k, n = orc.TYPE_BY_NAME[name], 1024, 32
+    w = _largest_weights(orc, name, n * k // 256)
+    deq = orc.dequant_row(ty, w.reshape(-1), n * k).reshape(n, k).astype(np.float64)
+    x = np.empty((3, nvec, 4, 256), np.float32)
+    x[0] = 0x7E7F7F80 * 2.0 ** -23
+    x[1] = -0x7E7F7F80 * 2.0 ** -23
+    x[2] = -0x808080 * 2.0 ** -23
+    x[2, ..., 100] = -128.0
+    x = x.reshape(3, nvec, k)
+    dw, dx, do = ctx.dev_alloc(w.nbytes), ctx.dev_alloc(x.nbytes), ctx.dev_alloc(3 * nvec * n * 4)
+    try:
+        ctx.upload(dw, w)
+        ctx.upload(dx, x)
+        for i in range(3):
+            assert ctx.gemv_dev(ty, dw, k, n, dx + 4 * i * nvec * k, do + 4 * i * nvec * n, nvec)
+        got = ctx.download(do, np.empty((3, nvec, n), np.float32))
+    finally:
+        for p in (dw, dx, do):
+            ctx.dev_free(p)
+    want = x.astype(np.float64) @ deq.T
+    # at most a few dozen roundings of 2^-24 of sums of one sign; the mins (Q4_K, Q5_K) are a part of them
+    assert np.all(np.abs(got - want) <= 40 * 2.0 ** -24 * np.abs(want)), np.max(np.abs(got / want - 1.0))
+
+
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
 @pytest.mark.parametrize("nvec", [1, 2, 5])
 def test_subnormal_activations(orc, ctx, name, nvec):

@@ -57,7 +57,7 @@ def test_batch_equals_token_by_token(orc, small):
             assert np.array_equal(osel[0], bsel[t]) and np.array_equal(ow[0].view(np.uint32), bw[t].view(np.uint32))
             assert rel_err(one[0], batch[t]) <= 5e-4
     h = orc.synth_normal(SEED, 952, 1.0, nt * layers[0].e).reshape(nt, -1)
-    batch = c.moe_block(0, h[:13])  # IQ3_XXS layer, 13 and 4 tokens: the mma.sync kernel with three parts both times
+    batch = c.moe_block(0, h[:13])  # IQ3_XXS layer, 13 and 4 tokens: the mma.sync kernel both times
     sub = c.moe_block(0, h[[5, 3, 12, 11]])
     assert np.array_equal(sub.view(np.uint32), batch[[5, 3, 12, 11]].view(np.uint32))
     big = c.moe_block(0, np.concatenate([h, h]))  # 42 and 21 tokens: the mma.sync kernel with two parts both times

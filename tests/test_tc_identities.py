@@ -239,8 +239,8 @@ def test_which_activation_blocks_are_wide(orc):
 
 
 def test_integer_block_sums_fit(orc):
-    """Largest sums of a 256-element block against a digit of 128: below 2^31, as the kernel's comments bound them; the byte forms of the
-    weights are the weights."""
+    """Largest sums of a 256-element block against a digit of 128: the arithmetic of the kernel's comments (test_largest_integer_sums runs such
+    blocks through the kernels); the byte forms of the weights are the weights."""
     n = 32 * 128
     assert 8 * 16 * 63 * 15 * n < 2 ** 29 and 4 * 63 * (16 * 15 + 240) * n < 2 ** 29      # Q4_K: scales or nibbles 16 times as large
     assert 8 * 63 * 31 * n < 2 ** 26 and 8 * 31 * 62 * n < 2 ** 26                         # Q5_K, IQ3_XXS
