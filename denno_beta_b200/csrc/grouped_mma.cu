@@ -108,7 +108,16 @@ __device__ __forceinline__ void mm_split(float a, float b, uint32_t (&h)[3]) {
 }
 __device__ __forceinline__ float mm_pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
 
-// One warp: a token's 256 elements at xr into their place in shared memory.  The block times 2^s, which puts its largest element into [2^30,
+// A lane's eight of the 256 elements at xr.
+struct MmIn { float4 a, b; };
+template <int T>
+__device__ __forceinline__ MmIn mm_load_block(const float* xr, int lane) {
+    int e0, e1;
+    mm_unit_elems<T>(lane >> 2, lane & 3, e0, e1);
+    return {*reinterpret_cast<const float4*>(xr + e0), *reinterpret_cast<const float4*>(xr + e1)};
+}
+
+// One warp: a token's 256 elements into their place in shared memory.  The block times 2^s, which puts its largest element into [2^30,
 // 2^31), or into half of that where it would be above 0x7f7f7f7f, is rounded to integers; their four digits in base 256 are balanced (-128 ..
 // 127), so that sum_j 256^j * d_j is the integer.
 // That rounds elements below 2^24 (2^-7 to 2^-6 of the block's largest) to 2^-31 of the largest, which is less than what the sums are rounded
@@ -123,12 +132,9 @@ __device__ __forceinline__ float mm_pow2(int e) { return __uint_as_float((uint32
 // prompt of 77 357 -> 372 (before there were rests: 461, 1,023, 348).
 // Returns whether the block is wide.
 template <int T>
-__device__ __forceinline__ bool mm_stage_block(const float* __restrict__ xr, uint8_t* dst, int lane) {
+__device__ __forceinline__ bool mm_stage_block(const MmIn& in, uint8_t* dst, int lane) {
     const int u = lane >> 2, t = lane & 3;
-    int e0, e1;
-    mm_unit_elems<T>(u, t, e0, e1);
-    const float4 f0 = *reinterpret_cast<const float4*>(xr + e0), f1 = *reinterpret_cast<const float4*>(xr + e1);
-    float x[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+    float x[8] = {in.a.x, in.a.y, in.a.z, in.a.w, in.b.x, in.b.y, in.b.z, in.b.w};
     uint32_t mine = 0u;
 #pragma unroll
     for (int i = 0; i < 8; ++i) mine = max(mine, __float_as_uint(fabsf(x[i])));
@@ -778,7 +784,8 @@ __device__ __forceinline__ void mm_items(const MmArgs& A, const MmShared& S, int
         for (int gi = warp; gi < m * nb; gi += kMmWarps) {
             const int tok = gi / nb, b = gi - tok * nb;
             const uint32_t pr = row0 + tok;
-            wide |= mm_stage_block<T>(A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256, S.acts + (size_t)gi * kXBlock, lane);
+            const float* xr = A.x + (size_t)(A.row_token ? A.row_token[pr] : (int32_t)pr) * A.ldx + b * 256;
+            wide |= mm_stage_block<T>(mm_load_block<T>(xr, lane), S.acts + (size_t)gi * kXBlock, lane);
         }
         if (__builtin_expect(__syncthreads_or(wide), 0)) {
             mm_row_groups<T, FUSED, NT, true>(I, F);
@@ -868,9 +875,9 @@ static int mm_launch_type(dnb_ctx* c, cudaStream_t st, bool fused, int nt, MmArg
 #undef DNB_MM
 }
 
-// The ring of each of `warps` warps that fits beside `base` bytes: two blocks a stage where a warp has that many, three stages, then two; else one
-// block, four stages to two.  Bytes of shared memory in all, or 0.
-static size_t mm_ring(int type, int blocks, int warps, size_t base, size_t cap, MmRing& r) {
+// The ring of each of `warps` warps that fits beside `base` bytes (`base_two`: with two blocks a stage): two blocks a stage where a warp has that many,
+// three stages, then two; else one block, four stages to two.  Bytes of shared memory in all, or 0.
+static size_t mm_ring(int type, int blocks, int warps, size_t base, size_t base_two, size_t cap, MmRing& r) {
     static const int form[5][2] = {{2, 3}, {2, 2}, {1, 4}, {1, 3}, {1, 2}};
     for (const auto& f : form) {
         if (f[0] > blocks) continue;
@@ -882,7 +889,7 @@ static size_t mm_ring(int type, int blocks, int warps, size_t base, size_t cap, 
 #undef DNB_P
             default: return 0;
         }
-        const size_t smem = base + (size_t)warps * r.nst * 16 * r.pitch;
+        const size_t smem = (f[0] == 2 ? base_two : base) + (size_t)warps * r.nst * 16 * r.pitch;
         if (smem <= cap) return smem;
     }
     return 0;
@@ -926,7 +933,7 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, con
         A.ks = ks;
         size_t base = kMmFixed + (ks > 1 ? (size_t)2 * kMmWarps * nt * 2 * 32 * 4 : 0) + (size_t)nt * tpt * nb * kXBlock;
         if (type == T_IQ3_XXS) base += sizeof(MmTables);
-        const size_t smem = mm_ring(type, nb / ks, kMmWarps, base, 225 * 1024, A.ring);
+        const size_t smem = mm_ring(type, nb / ks, kMmWarps, base, base, 225 * 1024, A.ring);
         if (smem) {
             A.status = c->status;
             // Activations of a tile 2.5 - 3 us, a row group 1.1 us at K = 2048 and a quarter of that at K = 512 (IQ3_XXS).  us a layer of 2048 x 512, top
@@ -1024,11 +1031,27 @@ __global__ void __launch_bounds__(kGvWarps * 32, 2) gemv_mma_single_kernel(const
     // ---- this warp's blocks of the vectors ----
     const int v0 = blockIdx.y * TOK;
     bool wide = false;
-    for (int i = 0; i < nst; ++i)
-        for (int j = 0; j < count(i); ++j)
+    // A block's elements are asked for before the one in front of it is converted, those of two vectors together: what a conversion stores keeps
+    // the compiler from doing so.  us, one after the other -> so: 2816 x 649, two vectors, Q4_K 4.9 -> 3.8, Q8_0 5.4 -> 4.2; 4096 x 4096 Q4_K 4.83 -> 4.78.
+    // (In mm_kernel, where a warp rarely has two of them, it costs registers and 1 to 2 %.)
+    {
+        const int mine = (nst - 1) * bps + count(nst - 1);
+        auto load = [&](int n, MmIn (&in)[TOK]) {
+            const float* xr = A.x + (first(n >> (bps - 1)) + (n & (bps - 1))) * 256;
 #pragma unroll
-            for (int q = 0; q < TOK; ++q)
-                wide |= mm_stage_block<T>(A.x + (size_t)min(v0 + q, A.nvec - 1) * A.k + (first(i) + j) * 256, xs + (i * bps + j) * XB + q * kXBlock, lane);
+            for (int q = 0; q < TOK; ++q) in[q] = mm_load_block<T>(xr + (size_t)min(v0 + q, A.nvec - 1) * A.k, lane);
+        };
+        MmIn now[TOK], next[TOK];
+        load(0, next);
+#pragma unroll 1
+        for (int n = 0; n < mine; ++n) {
+#pragma unroll
+            for (int q = 0; q < TOK; ++q) now[q] = next[q];
+            if (n + 1 < mine) load(n + 1, next);
+#pragma unroll
+            for (int q = 0; q < TOK; ++q) wide |= mm_stage_block<T>(now[q], xs + n * XB + q * kXBlock, lane);
+        }
+    }
     if constexpr (T == T_IQ3_XXS) {  // the tables came in parts from all threads
         tcp::cp_async_wait_all();
         __syncthreads();
@@ -1099,20 +1122,27 @@ static int launch_gv_t(dnb_ctx* c, cudaStream_t st, GvArgs A) {
     const int nb = A.k / 256;
     int ks = 1;
     while (ks < kGvWarps && ks * 2 <= nb) ks *= 2;
-    // a warp's share of the vectors: at most one block more than nb / ks (a ring of two blocks a stage: two)
-    size_t base = 2 * kGvWarps * 16 * TOK * 4 + (size_t)kGvWarps * ((nb + 2 * ks - 1) / (2 * ks) * 2) * TOK * kXBlock;
-    if (T == T_IQ3_XXS) base += sizeof(MmTables);
+    // room for a warp's share of the vectors: whole stages of the form that is taken (2048 x 2048 IQ3_XXS with four vectors is two CTAs an SM, 4.4 us;
+    // with room for two blocks where there is one it was one, and the call went to mm_kernel, 8.4 us)
+    const size_t fixed = 2 * kGvWarps * 16 * TOK * 4 + (T == T_IQ3_XXS ? sizeof(MmTables) : 0), share = (size_t)kGvWarps * TOK * kXBlock;
+    const size_t base = fixed + share * ((nb + ks - 1) / ks), base_two = fixed + share * ((nb + 2 * ks - 1) / (2 * ks) * 2);
     const size_t two = 113 * 1024;  // two CTAs per SM where they fit
     A.ks = ks;
-    size_t smem = mm_ring(T, nb / ks, kGvWarps, base, two, A.ring);
-    if (!smem) smem = mm_ring(T, nb / ks, kGvWarps, base, 225 * 1024, A.ring);
+    const int nslot = kGvWarps / ks, n_rg = (A.n + 15) / 16, ctas = (n_rg + nslot - 1) / nslot, rows = (A.nvec + TOK - 1) / TOK;
+    // Two blocks a stage give the warps whole stages of K.  Where that makes the longest share longer (18 to 24 blocks: four instead of three)
+    // and no SM has more than one CTA, whose longest share is then the time, it is one.  us, two / one: 1024 x 20 blocks Q4_K 5.5 / 4.5, 649 x 20, two
+    // vectors, Q8_0 6.1 / 5.0, Q6_K 6.4 / 5.7, IQ3_XXS 6.8 / 6.1; with CTAs enough not always: 65536 x 20 blocks Q4_K 55 / 57, 24 blocks 59 / 66, 19 57 /
+    // 55, other formats alike; and where the shares are as long: 1024 x 16 blocks 3.5 / 3.7, 65536 x 16 41 / 49.
+    const int units = (nb + 1) / 2, longest_one = (nb + ks - 1) / ks, longest_two = (units + ks - 1) / ks * 2 - ((units - 1) % ks == 0 ? nb & 1 : 0);
+    const int blocks = longest_two > longest_one && (long)ctas * rows <= c->sm_count ? 1 : nb / ks;
+    size_t smem = mm_ring(T, blocks, kGvWarps, base, base_two, two, A.ring);
+    if (!smem) smem = mm_ring(T, blocks, kGvWarps, base, base_two, 225 * 1024, A.ring);
     if (!smem) return DNB_DECLINED;
     A.status = c->status;
     auto kern = gemv_mma_single_kernel<T, TOK>;
     static SmemGrant grant;
     DNB_CUDA(grant_smem(grant, c->device, kern, smem));
-    const int nslot = kGvWarps / ks, n_rg = (A.n + 15) / 16;
-    const int room = (smem <= two ? 2 : 1) * c->sm_count, ctas = (n_rg + nslot - 1) / nslot, rows = (A.nvec + TOK - 1) / TOK;
+    const int room = (smem <= two ? 2 : 1) * c->sm_count;
     // more vectors in grid rows of their own, each decoding the weights again: while they only fill SMs that would idle
     if (rows > 1 && (long)ctas * rows > room) return DNB_DECLINED;
     const int grid = std::min(ctas, room);

@@ -119,10 +119,11 @@ def test_experts_given_mixed(orc, ctx, up, down, e, ff):
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K", "Q6_K", "Q8_0", "IQ3_XXS"])
-@pytest.mark.parametrize("k,n,nvec", [(256, 1, 1), (768, 15, 2), (2304, 17, 3), (512, 2369, 8), (4096, 33, 1), (4352, 33, 1), (4864, 17, 2), (8448, 15, 1)])
+@pytest.mark.parametrize("k,n,nvec", [(256, 1, 1), (768, 15, 2), (2304, 17, 3), (512, 2369, 8), (4096, 33, 1), (4352, 33, 1), (4864, 17, 2), (4864, 2400, 1),
+                                      (5632, 371, 8), (8448, 15, 1), (2048, 2048, 4)])
 def test_gemv_edges(orc, ctx, name, k, n, nvec):
-    """Rows that end inside a group of 16, vectors in pairs and an odd one, K of 1 to 33 blocks: 17, 19 and 33 are two a stage with a last stage of
-    one."""
+    """Rows that end inside a group of 16, vectors in pairs and an odd one, K of 1 to 33 blocks: 17, 33 and (with more CTAs than SMs) 19 are two a stage
+    with a last stage of one, 19 and 22 with few CTAs one a stage; 2048 x 2048 with four vectors is two CTAs an SM."""
     ty = orc.TYPE_BY_NAME[name]
     w = orc.synth_blocks(ty, SEED, 70 + ty, n * k // orc.blck_size(ty))
     x = orc.synth_normal(SEED, 71, 1.0, nvec * k).reshape(nvec, k)
@@ -140,6 +141,22 @@ def test_gemv_edges(orc, ctx, name, k, n, nvec):
     assert np.all(got[nvec] == 7.0), "wrote behind the last row"
     want = np.stack([orc.gemv_scalar(ty, w, k, n, v) for v in x])
     assert rel_err(got[:nvec], want) <= 2e-5
+
+
+def test_four_vectors_of_a_small_matrix(orc, ctx):
+    """2048 x 2048 of IQ3_XXS: two CTAs fit an SM, so the two pairs of vectors are grid rows of the GEMV."""
+    w = orc.synth_blocks(orc.IQ3_XXS, SEED, 75, 2048 * 8)
+    dw, dx, do = ctx.dev_alloc(w.nbytes), ctx.dev_alloc(4 * 2048 * 4), ctx.dev_alloc(4 * 2048 * 4)
+    try:
+        ctx.upload(dw, w)
+        ctx.upload(dx, orc.synth_normal(SEED, 76, 1.0, 4 * 2048))
+        ctx.profile(True)
+        assert ctx.gemv_dev(orc.IQ3_XXS, dw, 2048, 2048, dx, do, 4)
+        assert list(ctx.profile_read()) == ["gemv_mma"]
+        ctx.profile(False)
+    finally:
+        for p in (dw, dx, do):
+            ctx.dev_free(p)
 
 
 @pytest.mark.parametrize("base", [0, 2048])
