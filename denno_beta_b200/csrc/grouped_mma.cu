@@ -27,9 +27,10 @@
 // the tile, the column or the CTA; for decode batches KS is a constant of the shape, so that a token's bits do not depend on its batch.
 //
 // Measured, us of a launch, gate/up + down of 2048 x 512, top 10 of 512: fp16 operands in two or three parts -> bytes -> two blocks a stage and a
-// loop for each number of column tiles.  8 tokens: IQ3_XXS 49 + 31 -> 44 + 29 -> 41 + 27, Q4_K 44 + 28 -> 33 + 23 -> 32 + 21; 32 tokens: IQ3_XXS
-// 115 + 68 -> 108 + 66 -> 101 + 62, Q4_K 98 + 56 -> 75 + 45 -> 71 + 42, Q8_0 151 + 92 -> 134 + 74 -> 111 + 64; 200 tokens under a skewed router: Q4_K
-// and Q6_K 302 + 175 -> 263 + 119 -> 154 + 120, Q8_0 395 + 169 -> 249 + 135 -> 176 + 103.  (One loop with unused column tiles switched off took the
+// loop for each number of column tiles -> 32 bits an activation and the remainders of wide blocks.  8 tokens: IQ3_XXS 49 + 31 -> 44 + 29 -> 41 + 27 -> 41 +
+// 27, Q4_K 44 + 28 -> 33 + 23 -> 32 + 21 -> 32 + 23; 32 tokens: IQ3_XXS 115 + 68 -> 108 + 66 -> 101 + 62 -> 104 + 64, Q4_K 98 + 56 -> 75 + 45 -> 71 + 42 -> 71 + 49,
+// Q8_0 151 + 92 -> 134 + 74 -> 111 + 64 -> 113 + 65; 200 tokens under a skewed router: Q4_K and Q6_K 302 + 175 -> 263 + 119 -> 154 + 120 -> 157 + 138, Q8_0 395 +
+// 169 -> 249 + 135 -> 176 + 103 -> 189 + 105.  (One loop with unused column tiles switched off took the
 // time of all of them, or not, as the compiler chose.)  Decoding alone is 30 (Q4_K) to 66 (IQ3_XXS) cycles of a scheduler for 16 rows x 32
 // elements; bytes from HBM take 50 and 34.  Distance from the 64-bit result: see mm_stage_block.
 #include <algorithm>
@@ -965,8 +966,8 @@ int launch_mm(dnb_ctx* c, cudaStream_t st, int type, bool fused, bool batch, con
 // work); a warp takes every ks-th block of K of 16 rows and asks for its first stages before it waits for the kernel in front of
 // it, whose output the vector may be; it converts its own blocks of the vector, each with a power of two of its own, so that no
 // CTA-wide step stands between vector and math; the warps' partial sums meet once per 16 rows, in a fixed order.
-// Measured back to back, us, with fp16 operands -> with bytes: 4096 x 4096 Q4_K 5.6 -> 4.7; 65536 x 4096 Q8_0 71.8 -> 61 (4.7 TB/s), Q4_K 54 -> 38, IQ3_XXS
-// 64 -> 57.  (The register-decode GEMV before took 8.4 for the small one, 103 for Q8_0.)
+// Measured back to back, us, with fp16 operands -> with bytes: 4096 x 4096 Q4_K 5.6 -> 4.7; 65536 x 4096 Q8_0 71.8 -> 61 (4.7 TB/s), Q4_K 54 -> 37, IQ3_XXS
+// 64 -> 55.  (The register-decode GEMV before took 8.4 for the small one, 103 for Q8_0.)
 constexpr int kGvWarps = 8;
 
 struct GvArgs {
